@@ -47,3 +47,21 @@ def test_one_launch_delta_prefill_matches_oracle_and_per_token_path(ctx, tmp_pat
     assert outs[1][1] < outs[0][1], "one launch per DeltaNet layer instead of one per token"
     g1, g0 = bf16_to_f32(outs[1][0][0]), bf16_to_f32(outs[0][0][0])
     assert np.abs(g1 - g0).max() <= 0.02 * np.abs(g0).max() + 1e-3
+
+
+@pytest.mark.parametrize("kind,groups,portions", [("qwen-hybrid", 2, (4, 9, 1, 5, 8)), ("qwen-hybrid-512", 4, (33, 4, 7))])
+def test_scan_prefill_in_portions_matches_oracle(ctx, tmp_path, kind, groups, portions):
+    """Passes of 4 tokens and more: blocks of 8 tokens that are not full, a pass whose conv window starts in the state left by the one
+    before it, several v heads per k head; the same bound as the whole-model logit checks."""
+    spec = synth.tiny(kind)
+    assert spec.dn_num_groups == groups
+    path = synth.write_model(spec, tmp_path / "m", seed=31)
+    prompt = np.random.default_rng(12).integers(0, spec.vocab_size, sum(portions))
+    ref = OracleModel(path, max_context=256)
+    with B.Engine(ctx, path, max_context_length=256, use_cuda_graph=False) as eng:
+        at = 0
+        for n in portions:
+            for t in prompt[at:at + n]:
+                lr = ref.forward([t])
+            _logit_check(eng.forward(prompt[at:at + n]), lr, f"portion of {n} at {at}")
+            at += n

@@ -116,8 +116,13 @@ bool dense_umma_applicable(const uzu_dense_linear_args& a);
 // tensor-core prefill attention (attention_prefill.cu, opt-in), tried first by uzu_attention_single_pass_encode
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a);
 
-// multi-token DeltaNet recurrence in one launch (deltanet_prefill.cu, opt-in), tried by the engine's batched hybrid prefill
-bool encode_delta_net_prefill(uzu_command_buffer* cmd, const uzu_delta_net_fused_update_args& f, uint32_t rows, uint32_t in_stride, uint32_t out_stride);
+// multi-token DeltaNet recurrence (deltanet_prefill.cu), tried by the engine's batched hybrid prefill; scratch may be 0 (then only passes of 2
+// and 3 tokens are taken)
+bool encode_delta_net_prefill(uzu_command_buffer* cmd, const uzu_delta_net_fused_update_args& f, uint32_t rows, uint32_t in_stride, uint32_t out_stride,
+                              uint64_t scratch);
+size_t delta_net_prefill_scratch_bytes(uint32_t rows, uint32_t key_dim, uint32_t value_dim, uint32_t v_heads);
+// the token-by-token scan of uzu_gated_delta_encode over prepared rows (gated_delta.cu); prep.taps = 1: no convolution ring is advanced
+void launch_gated_delta_scan(uzu_command_buffer* cmd, const uzu_gated_delta_args& a);
 
 // The launch stream belongs to the context's device: make that device current on the calling thread (another context, or the
 // host program, may have switched it since start_encoding).

@@ -641,7 +641,7 @@ struct uzu_engine {
     // scratch arena
     Buf shortcut2;   // fused decode path: the residual ping-pongs between `shortcut` and `shortcut2`
     bool fused_ok = false;
-    Buf token_ids, hidden_a, hidden_b, shortcut, qkv, queries, attn_out, gate, fused_up, gated, mixer_out, in_proj, delta_out, normed_out,
+    Buf token_ids, hidden_a, hidden_b, shortcut, qkv, queries, attn_out, gate, fused_up, gated, mixer_out, in_proj, delta_out, delta_scratch, normed_out,
         logits, sampled, seeds, tp_parts, tp_sums, tp_maxs;
     Buf host_ring;        // pinned u32[TOKEN_RING]
     Buf host_tokens;      // pinned u32[MAX_ROWS] upload staging
@@ -1184,6 +1184,7 @@ static void create_state_and_scratch(uzu_engine* e) {
     const bool sparse = (uzu_context_device_capabilities(e->ctx) & UZU_CAP_SPARSE_BUFFERS) != 0;
     e->state.resize(e->runs.size());
     uint32_t max_qkv = 0, max_qd = 0, max_f = 0, max_proj = 0, max_vd = 0, max_heads = 0, max_hd = 0;
+    size_t scan_bytes = 0;
     for (size_t i = 0; i < e->runs.size(); ++i) {
         Layer& L = e->layers[e->runs[i]];
         alloc_layer_state(e, L, e->state[i], rows_total, sparse, false);
@@ -1198,6 +1199,7 @@ static void create_state_and_scratch(uzu_engine* e) {
             const DeltaNetLayer& D = L.dn;
             max_proj = std::max(max_proj, D.total_proj_dim);
             max_vd = std::max(max_vd, D.value_dim);
+            scan_bytes = std::max(scan_bytes, delta_net_prefill_scratch_bytes(MAX_ROWS, D.key_dim, D.value_dim, D.num_heads));
         }
     }
     auto dev = [&](size_t bytes) { return make_buf(e, std::max<size_t>(bytes, 256), UZU_BUFFER_DEVICE); };
@@ -1216,6 +1218,7 @@ static void create_state_and_scratch(uzu_engine* e) {
     e->gated = dev((size_t)MAX_ROWS * max_f * 2);
     e->in_proj = dev((size_t)MAX_ROWS * max_proj * 2);
     e->delta_out = dev((size_t)MAX_ROWS * max_vd * 2);
+    if (scan_bytes) e->delta_scratch = dev(scan_bytes);      // q, k, v, read-outs and gates of a prompt pass (f32 rows)
     e->logits = dev((size_t)e->logits_rows * V * 2);
     if (e->tp_sharded) {
         e->tp_partial = dev((size_t)MAX_ROWS * H * 4);
@@ -1491,7 +1494,7 @@ static uint64_t encode_delta_net(uzu_engine* e, uzu_command_buffer* cmd, const L
     // Kernels::DeltaNetChunkedPrefill, evaluates the same recurrence in a different summation order; not restated here.)
     encode_linear(cmd, D.in_proj, hidden, m, e->in_proj.ptr());
     bool whole_pass = false;
-    if (m > 1) {   // opt-in: the m-token recurrence of this layer in ONE launch (deltanet_prefill.cu), state kept on chip across tokens
+    if (m > 1) {   // the m-token recurrence of this layer in a few launches (deltanet_prefill.cu), state kept on chip across tokens
         uzu_delta_net_fused_update_args f0{};
         f0.conv.conv_weight = D.conv_weight.ptr(); f0.conv.bias = D.conv_bias.ptr(); f0.conv.in_out = e->in_proj.ptr(); f0.conv.state = S.conv_state.ptr();
         f0.conv.kernel_size = D.kernel_size; f0.conv.conv_dim = D.conv_dim; f0.conv.state_stride = D.kernel_size - 1; f0.conv.has_bias = D.conv_has_bias;
@@ -1499,7 +1502,7 @@ static uint64_t encode_delta_net(uzu_engine* e, uzu_command_buffer* cmd, const L
         f0.update.state = S.ssm_state.ptr(); f0.update.out = e->delta_out.ptr();
         f0.update.num_v_heads = D.num_heads; f0.update.num_k_heads = D.num_groups; f0.update.head_v_dim = D.value_head_dim; f0.update.key_dim = D.key_dim;
         f0.update.value_dim = D.value_dim; f0.update.norm_epsilon = D.norm_epsilon; f0.update.head_k_dim = D.head_dim;
-        whole_pass = encode_delta_net_prefill(cmd, f0, m, D.total_proj_dim, D.value_dim);
+        whole_pass = encode_delta_net_prefill(cmd, f0, m, D.total_proj_dim, D.value_dim, e->delta_scratch.ptr());
     }
     for (uint32_t t = 0; t < m && !whole_pass; ++t) {
         const uint64_t row = e->in_proj.ptr() + (size_t)t * D.total_proj_dim * 2;

@@ -545,6 +545,16 @@ static void by_key_size(uint32_t dim, F&& f) {
     else f(std::integral_constant<int, 32>{}, std::integral_constant<int, 8>{});
 }
 
+void launch_gated_delta_scan(uzu_command_buffer* cmd, const uzu_gated_delta_args& a) {
+    by_key_size(a.prep.dim, [&](auto l_c, auto nv_c) {
+        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GD_WARPS * (32 / L), BATCH = gd_batch<L, NV>();
+        constexpr size_t smem = ((size_t)4 * BATCH * L * NV * 4 + (size_t)2 * BATCH * CC + 4 * BATCH) * sizeof(float);
+        static std::atomic<uint64_t> done{0};
+        if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, gated_delta_kernel<L, NV>, (int)smem, done);
+        launch(cmd, "gated_delta_kernel", gated_delta_kernel<L, NV>, dim3((a.prep.vdim + CC - 1) / CC, a.prep.heads), dim3(GD_WARPS * 32), smem, a);
+    });
+}
+
 }  // namespace uzu
 
 extern "C" {
@@ -586,13 +596,7 @@ void uzu_gated_delta_encode(uzu_command_buffer* cmd, const uzu_gated_delta_args*
         return;
     }
     if (a->prep.rows == 0) return;
-    by_key_size(a->prep.dim, [&](auto l_c, auto nv_c) {
-        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GD_WARPS * (32 / L), BATCH = gd_batch<L, NV>();
-        constexpr size_t smem = ((size_t)4 * BATCH * L * NV * 4 + (size_t)2 * BATCH * CC + 4 * BATCH) * sizeof(float);
-        static std::atomic<uint64_t> done{0};
-        if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, gated_delta_kernel<L, NV>, (int)smem, done);
-        launch(cmd, "gated_delta_kernel", gated_delta_kernel<L, NV>, dim3((a->prep.vdim + CC - 1) / CC, a->prep.heads), dim3(GD_WARPS * 32), smem, *a);
-    });
+    launch_gated_delta_scan(cmd, *a);
 }
 
 void uzu_gated_delta_step_encode(uzu_command_buffer* cmd, const uzu_gated_delta_step_args* a) {
