@@ -269,6 +269,25 @@ def test_general_delta_kernel(ctx, rows, heads, dim):
         close(got_state, ref_state, 1e-5, "generalized delta state")
 
 
+@pytest.mark.parametrize("rows,heads,dim,extra", [(4, 2, 4, 0), (9, 1, 33, 3), (17, 2, 64, 1), (8, 1, 65, 0), (31, 2, 128, 4), (15, 1, 200, 0), (5, 1, 300, 4)])
+def test_general_delta_scan(ctx, rows, heads, dim, extra):
+    """Passes that form their vectors up front: full and partial batches of tokens, head sizes at both sides of a lane layout's range, rows
+    with and without 16-byte alignment (`extra` elements of stride). Sums of at most 300 f32 products: 1e-5 as for the other form."""
+    rng = np.random.default_rng(rows * dim)
+    hd, ld = heads * dim, heads * dim + extra
+    r, k, v, rate, decay = (rng.standard_normal((rows, ld), dtype=np.float32) for _ in range(5))
+    rate_b, decay_b = rng.standard_normal(hd, dtype=np.float32), rng.standard_normal(hd, dtype=np.float32)
+    state = rng.standard_normal((heads, dim, dim), dtype=np.float32)
+    ref, ref_state = general_delta_plain(*(np.ascontiguousarray(x[:, :hd]) for x in (r, k, v, rate, decay)), rate_b, decay_b, state, heads, dim)
+    bufs = [ctx.upload(x) for x in (r, k, v, rate, decay, rate_b, decay_b, state, np.zeros((rows, hd), np.float32), np.zeros((rows, hd), np.float32))]
+    a = B.GeneralDeltaArgs(r=bufs[0].ptr, k=bufs[1].ptr, v=bufs[2].ptr, rate_logit=bufs[3].ptr, decay_logit=bufs[4].ptr, rate_bias=bufs[5].ptr,
+                           decay_bias=bufs[6].ptr, state=bufs[7].ptr, unit=bufs[8].ptr, out=bufs[9].ptr, r_stride=ld, k_stride=ld, v_stride=ld,
+                           rate_stride=ld, decay_stride=ld, rows=rows, heads=heads, dim=dim)
+    run(ctx, "uzu_general_delta_encode", C.byref(a))
+    close(bufs[9].numpy(np.float32, (rows, hd)), ref, 1e-5, "scan output")
+    close(bufs[7].numpy(np.float32, state.shape), ref_state, 1e-5, "scan state")
+
+
 def test_general_delta_one_launch_equals_token_by_token(ctx):
     rng = np.random.default_rng(11)
     rows, heads, dim = 24, 2, 40

@@ -1,23 +1,24 @@
 // Generalized delta rule (per head a dim x dim f32 state S, key channel x value channel):
 //     S <- diag(d) S - (a * u)(u^T S) + k v^T,   out = S^T r
 // with decay d = exp(-e^-1/2 * sigmoid(.)), removal rate a = sigmoid(.), unit key u = k / sqrt(sum k^2 + 1e-6), all formed in f32 here
-// from the raw projections. One launch walks the `rows` tokens of a pass in order with the state on chip: the value columns of a head are
-// independent (u^T S is a per-column dot product), so the grid is (column blocks of 32, heads) and a CTA keeps its dim x 32 slice of
-// the state in registers -- warp p owns PART key channels [PART p, PART p + PART), lane c owns column c (PART is chosen per head size
-// so that a CTA has about 16 warps). Per token the CTA puts the head's vectors in shared memory, every thread contributes a partial
-// of u^T S and of S^T r, and partials meet in shared memory in warp order (a fixed order: one token at a time or a thousand in one
-// launch give the same bits). A token's inputs are requested three tokens ahead. Passes of >= 4 tokens that bring a scratch form decay,
-// rate * unit key and unit key for all tokens in one parallel launch first (general_delta_prepare_kernel), which takes the exponentials
-// and the key norm out of the token-by-token chain. The same kernel is the decode step (rows = 1).
+// from the raw projections. The value columns of a head are independent (u^T S is a per-column dot product).
+//   general_delta_scan_kernel   passes of >= 4 tokens that bring a scratch: decay, rate * unit key and unit key of all tokens are formed in one
+//                               parallel launch first (general_delta_prepare_kernel), then L lanes own a column and walk the tokens, two dot
+//                               products and an update each, no barrier between tokens; the five vectors of a token come from shared memory,
+//                               a batch of tokens ahead by cp.async. Bound: the chain of tokens.
+//   general_delta_kernel        the decode step and short passes: a CTA keeps a dim x 32 slice of the state in registers -- warp p owns PART
+//                               key channels, lane c owns column c; partial sums meet in shared memory in warp order (a fixed order: one
+//                               token at a time or several in one launch give the same bits).
 #include <cstdlib>
+#include <type_traits>
 
+#include "column_scan.cuh"
 #include "common.cuh"
 
 namespace uzu {
 
 
-// PREP: decay, rate * unit key and unit key arrive ready-made (general_delta_prepare_kernel) in decay_logit, rate_logit and `unit`.
-template <bool PREP, int PART>
+template <int PART>
 __global__ void __launch_bounds__(1024) general_delta_kernel(const uzu_general_delta_args a) {
     pdl_launch_dependents();
     pdl_wait();
@@ -47,18 +48,16 @@ __global__ void __launch_bounds__(1024) general_delta_kernel(const uzu_general_d
     const bool prep = tid < dim;
     const float rate_b = (prep && a.rate_bias) ? reinterpret_cast<const float*>(a.rate_bias)[hc + tid] : 0.0f;
     const float decay_b = (prep && a.decay_bias) ? reinterpret_cast<const float*>(a.decay_bias)[hc + tid] : 0.0f;
-    const float* pu = reinterpret_cast<const float*>(a.unit);
     // a token's inputs are requested three tokens ahead: the token-by-token chain never waits for memory
-    struct Inputs { float k, r, a, d, u, v; };
+    struct Inputs { float k, r, a, d, v; };
     auto request = [&](uint32_t t) {
-        Inputs q{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        Inputs q{0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
         if (t < a.rows) {
             if (prep) {
                 q.k = pk[(size_t)t * a.k_stride + hc + tid];
                 q.r = pr[(size_t)t * a.r_stride + hc + tid];
                 q.a = pa[(size_t)t * a.rate_stride + hc + tid];
                 q.d = pd[(size_t)t * a.decay_stride + hc + tid];
-                if constexpr (PREP) q.u = pu[(size_t)t * a.heads * dim + hc + tid];
             }
             if (col_ok) q.v = pv[(size_t)t * a.v_stride + hc + col];
         }
@@ -73,17 +72,8 @@ __global__ void __launch_bounds__(1024) general_delta_kernel(const uzu_general_d
         q0 = q1;
         q1 = q2;
         q2 = request(t + 3);
-        const float kk = cur.k, rr = cur.r, raw_a = cur.a, raw_d = cur.d, vv = cur.v, uu = cur.u;
+        const float kk = cur.k, rr = cur.r, raw_a = cur.a, raw_d = cur.d, vv = cur.v;
         const float al = raw_a + rate_b, dl = raw_d + decay_b;
-        if constexpr (PREP) {
-            if (prep) {
-                vd[tid] = raw_d;
-                vau[tid] = raw_a;
-                vu[tid] = uu;
-                vk[tid] = kk;
-                vr[tid] = rr;
-            }
-        } else {
         const float sq = warp_sum(prep ? kk * kk : 0.0f);
         if (lane == 0) ssq[b * 32 + warp] = sq;
         __syncthreads();
@@ -98,7 +88,6 @@ __global__ void __launch_bounds__(1024) general_delta_kernel(const uzu_general_d
             vu[tid] = u;
             vk[tid] = kk;
             vr[tid] = rr;
-        }
         }
         __syncthreads();
         float zp = 0.0f;
@@ -158,6 +147,152 @@ __global__ void __launch_bounds__(128) general_delta_prepare_kernel(const uzu_ge
     }
 }
 
+// The tokens of a pass in order over ready-made vectors (decay in decay_logit, rate * unit key in rate_logit, unit key in `unit`): 4 warps per CTA,
+// 32 / L columns per warp, grid (column blocks, heads). Bound: the chain of a token (dot product over the lane's channels, log2 L shuffles, the
+// update). 1024 tokens, 16 heads of 128: 0.37 ms against 1.70 ms as a CTA per 32 columns with three barriers a token.
+constexpr int GS_WARPS = 4;
+template <int L, int NV>
+constexpr int gs_batch() { return L * NV * 4 <= 128 ? 8 : (L * NV * 4 <= 256 ? 4 : 2); }
+
+template <int L, int NV>
+__global__ void __launch_bounds__(GS_WARPS * 32) general_delta_scan_kernel(const uzu_general_delta_args a, uint32_t vec) {
+    constexpr int ROWF = L * NV * 4, BATCH = gs_batch<L, NV>(), CC = GS_WARPS * (32 / L);
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float gs_smem[];
+    float* vecs = gs_smem;                           // [2][BATCH][5][ROWF]: d, a * u, u, k, r
+    float* vs = vecs + 2 * BATCH * 5 * ROWF;         // [2][BATCH][CC]
+    const uint32_t dim = a.dim, h = blockIdx.y, hc = h * dim;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = lane % L;
+    const uint32_t cl = warp * (32 / L) + lane / L, col0 = blockIdx.x * CC, col = col0 + cl;
+    const bool col_ok = col < dim;
+    const float* src[5] = {reinterpret_cast<const float*>(a.decay_logit) + hc, reinterpret_cast<const float*>(a.rate_logit) + hc,
+                           reinterpret_cast<const float*>(a.unit) + hc, reinterpret_cast<const float*>(a.k) + hc, reinterpret_cast<const float*>(a.r) + hc};
+    const uint32_t stride[5] = {a.decay_stride, a.rate_stride, a.heads * dim, a.k_stride, a.r_stride};
+    const float* pv = reinterpret_cast<const float*>(a.v) + hc + col0;
+    auto stage = [&](uint32_t tb, uint32_t buf) {
+        const uint32_t nb = tb < a.rows ? min((uint32_t)BATCH, a.rows - tb) : 0u;
+        float* dst = vecs + buf * BATCH * 5 * ROWF;
+        if (vec) {                                   // rows and head offsets on 16-byte boundaries, dim a multiple of 4
+            const uint32_t pieces = dim / 4;
+#pragma unroll
+            for (int w = 0; w < 5; ++w)
+                for (uint32_t i = tid; i < nb * pieces; i += GS_WARPS * 32) {
+                    const uint32_t r = i / pieces, c = (i - r * pieces) * 4;
+                    gd_cp_async16(dst + (r * 5 + w) * ROWF + c, src[w] + (size_t)(tb + r) * stride[w] + c);
+                }
+        } else {
+#pragma unroll
+            for (int w = 0; w < 5; ++w)
+                for (uint32_t i = tid; i < nb * dim; i += GS_WARPS * 32) {
+                    const uint32_t r = i / dim, c = i - r * dim;
+                    gd_cp_async4(dst + (r * 5 + w) * ROWF + c, src[w] + (size_t)(tb + r) * stride[w] + c);
+                }
+        }
+        for (uint32_t i = tid; i < nb * CC; i += GS_WARPS * 32) {
+            const uint32_t r = i / CC, c = i % CC;
+            if (col0 + c < dim) gd_cp_async4(vs + (buf * BATCH + r) * CC + c, pv + (size_t)(tb + r) * a.v_stride + c);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (dim < (uint32_t)ROWF) {                      // channels past the head stay zero in both buffers
+        const uint32_t tail = ROWF - dim;
+        for (uint32_t i = tid; i < 2 * BATCH * 5 * tail; i += GS_WARPS * 32) vecs[i / tail * ROWF + dim + i % tail] = 0.0f;
+    }
+    stage(0, 0);
+    float4 S[NV];
+    float* state = reinterpret_cast<float*>(a.state) + (size_t)h * dim * dim + (col_ok ? col : 0u);
+    auto at = [&](int i, int j) { return 4u * (i * L + part) + j; };
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+        float s[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[j] = (col_ok && at(i, j) < dim) ? state[(size_t)at(i, j) * dim] : 0.0f;
+        S[i] = make_float4(s[0], s[1], s[2], s[3]);
+    }
+    float* out = reinterpret_cast<float*>(a.out) + hc + col;
+    const uint32_t out_stride = a.heads * dim;
+    uint32_t buf = 0;
+    for (uint32_t tb = 0; tb < a.rows; tb += BATCH, buf ^= 1) {
+        const uint32_t nb = min((uint32_t)BATCH, a.rows - tb);
+        stage(tb + BATCH, buf ^ 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const float* row = vecs + buf * BATCH * 5 * ROWF + part * 4;
+        const float* v = vs + buf * BATCH * CC + cl;
+        auto load_row = [&](float4 (&x)[NV], uint32_t r, int w) {
+#pragma unroll
+            for (int i = 0; i < NV; ++i) x[i] = *reinterpret_cast<const float4*>(row + (r * 5 + w) * ROWF + i * L * 4);
+        };
+        auto token = [&](uint32_t r) {               // one token; the lane's part of its read-out
+            float4 u[NV], d[NV], au[NV], k[NV], rr[NV];
+            load_row(u, r, 2);
+            load_row(d, r, 0);
+            load_row(au, r, 1);
+            load_row(k, r, 3);
+            load_row(rr, r, 4);
+            const float vv = v[r * CC];
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {           // what does not wait for the dot product: d S + k v
+                d[i].x = fmaf(k[i].x, vv, d[i].x * S[i].x);
+                d[i].y = fmaf(k[i].y, vv, d[i].y * S[i].y);
+                d[i].z = fmaf(k[i].z, vv, d[i].z * S[i].z);
+                d[i].w = fmaf(k[i].w, vv, d[i].w * S[i].w);
+            }
+            const float z = gd_lane_sum<L>(gd_dot<NV>(S, u));
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                S[i].x = fmaf(-au[i].x, z, d[i].x);
+                S[i].y = fmaf(-au[i].y, z, d[i].y);
+                S[i].z = fmaf(-au[i].z, z, d[i].z);
+                S[i].w = fmaf(-au[i].w, z, d[i].w);
+            }
+            return gd_dot<NV>(S, rr);
+        };
+        if (nb == BATCH) {                           // straight-line code; the read-outs of the batch meet over the lanes all at once
+            float o[BATCH];
+#pragma unroll
+            for (int j = 0; j < BATCH; ++j) o[j] = token(j);
+            gd_transpose_sum<BATCH, L>(o, part);
+            if (col_ok && part % (L / BATCH) == 0) out[(size_t)(tb + part / (L / BATCH)) * out_stride] = o[0];
+        } else {
+            for (uint32_t r = 0; r < nb; ++r) {
+                const float o = gd_lane_sum<L>(token(r));
+                if (part == 0 && col_ok) out[(size_t)(tb + r) * out_stride] = o;
+            }
+        }
+        __syncthreads();
+    }
+    if (col_ok) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const float s[4] = {S[i].x, S[i].y, S[i].z, S[i].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (at(i, j) < dim) state[(size_t)at(i, j) * dim] = s[j];
+        }
+    }
+}
+
+static void launch_general_delta_scan(uzu_command_buffer* cmd, const uzu_general_delta_args& a) {
+    // 16-byte copies where every row of every vector starts on a 16-byte boundary
+    const uint32_t vec = !((a.decay_logit | a.rate_logit | a.unit | a.k | a.r) & 15u) &&
+                         !((a.decay_stride | a.rate_stride | a.k_stride | a.r_stride | a.dim) & 3u);
+    auto go = [&](auto l_c, auto nv_c) {
+        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GS_WARPS * (32 / L), BATCH = gs_batch<L, NV>();
+        constexpr size_t smem = ((size_t)2 * BATCH * 5 * L * NV * 4 + (size_t)2 * BATCH * CC) * sizeof(float);
+        static std::atomic<uint64_t> done{0};
+        if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, general_delta_scan_kernel<L, NV>, (int)smem, done);
+        launch(cmd, "general_delta_scan_kernel", general_delta_scan_kernel<L, NV>, dim3((a.dim + CC - 1) / CC, a.heads), dim3(GS_WARPS * 32), smem, a, vec);
+    };
+    auto l8 = std::integral_constant<int, 8>{};
+    if (a.dim <= 32) go(l8, std::integral_constant<int, 1>{});
+    else if (a.dim <= 64) go(l8, std::integral_constant<int, 2>{});
+    else if (a.dim <= 128) go(l8, std::integral_constant<int, 4>{});
+    else if (a.dim <= 256) go(std::integral_constant<int, 16>{}, std::integral_constant<int, 4>{});
+    else go(std::integral_constant<int, 32>{}, std::integral_constant<int, 4>{});
+}
+
 // one warp per (row, head)
 // WIDE: a CTA per (row, head) instead of a warp: long heads (a norm over all heads at once)
 template <bool WIDE>
@@ -207,10 +342,11 @@ void uzu_general_delta_encode(uzu_command_buffer* cmd, const uzu_general_delta_a
     }
     if (a->rows == 0) return;
     // passes of several tokens with a scratch for the unit keys: the per-token vectors are formed for all tokens at once first
-    const bool prepared = a->unit != 0 && a->rows >= 4;
-    if (prepared) {
+    if (a->unit != 0 && a->rows >= 4) {
         const uint32_t units = a->rows * a->heads;
         launch(cmd, "general_delta_prepare_kernel", general_delta_prepare_kernel, dim3((units + 3) / 4), dim3(128), 0, *a);
+        launch_general_delta_scan(cmd, *a);
+        return;
     }
     // key channels per warp: about 16 warps per CTA whatever the head size (4 channels up to 64, 8 at 128, ...), so that a thread's
     // token-by-token chain is short and the schedulers have other warps to issue from. Measured, 1024 tokens, 16 heads: head 128: 2.95 ms
@@ -227,11 +363,11 @@ void uzu_general_delta_encode(uzu_command_buffer* cmd, const uzu_general_delta_a
         if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, kernel, (int)smem, done);
         launch(cmd, "general_delta_kernel", kernel, grid, block, smem, *a);
     };
-    static std::atomic<uint64_t> done[8];
-    if (part == 4) prepared ? go(general_delta_kernel<true, 4>, done[0]) : go(general_delta_kernel<false, 4>, done[1]);
-    else if (part == 8) prepared ? go(general_delta_kernel<true, 8>, done[2]) : go(general_delta_kernel<false, 8>, done[3]);
-    else if (part == 16) prepared ? go(general_delta_kernel<true, 16>, done[4]) : go(general_delta_kernel<false, 16>, done[5]);
-    else prepared ? go(general_delta_kernel<true, 32>, done[6]) : go(general_delta_kernel<false, 32>, done[7]);
+    static std::atomic<uint64_t> done[4];
+    if (part == 4) go(general_delta_kernel<4>, done[0]);
+    else if (part == 8) go(general_delta_kernel<8>, done[1]);
+    else if (part == 16) go(general_delta_kernel<16>, done[2]);
+    else go(general_delta_kernel<32>, done[3]);
 }
 
 void uzu_head_norm_gate_encode(uzu_command_buffer* cmd, const uzu_head_norm_gate_args* a) {
