@@ -412,3 +412,36 @@ def test_runtime_buffers_copy_fill_sparse(ctx):
         assert (dst.numpy(np.uint8) == 0xAB).all()
         assert ctx.lib.uzu_sparse_buffer_unmap(h, pages, 2) == 0
         ctx.lib.uzu_sparse_buffer_destroy(h)
+
+
+@pytest.mark.parametrize("V", [1, 9, 1023, 8192, 70001, 131072])
+@pytest.mark.parametrize("kw", [dict(top_k=1), dict(top_k=37), dict(top_k=500000, min_p=0.02), dict(top_p=0.9), dict(top_p=1.0, top_k=5), dict(min_p=0.3),
+                                dict(top_p=0.6, top_k=200, temperature=0.7, min_p=0.001)])
+def test_sampling_filters_count_values(ctx, V, kw):
+    """Many equal logits (values on a grid of 1/4, so the kept set ends inside a group of equals), masked entries, both zeros, slices of a few
+    elements and of none: the kept set of the counting kernel is the oracle's."""
+    rng = np.random.default_rng(V)
+    rows = 4
+    x = np.round(rng.standard_normal((rows, V)) * 8).astype(np.float32) / 4
+    x[:, ::3] *= -1.0                                   # -0 beside +0
+    logits = f32_to_bf16(x)
+    mask = rng.integers(0, 2 ** 32, (rows, (V + 31) // 32), dtype=np.uint32) | np.uint32(1)
+    seeds = rng.integers(0, 2 ** 63, rows).astype(np.uint64)
+    for bitmask in (None, mask):
+        ref = O.unified_sampling(logits, seeds=seeds, bitmask=bitmask, **kw)
+        got = G.unified_sampling(ctx, logits, seeds=seeds, bitmask=bitmask, **kw)
+        assert np.array_equal(ref, got)
+        ref = O.unified_sampling(logits, bitmask=bitmask, **kw)
+        assert np.array_equal(ref, G.unified_sampling(ctx, logits, bitmask=bitmask, **kw))
+
+
+def test_sampling_filters_rows_without_finite_logits(ctx):
+    """Everything masked, infinities of both signs: the candidate walk answers as the oracle does."""
+    V = 300
+    x = np.random.default_rng(3).standard_normal((4, V)).astype(np.float32)
+    x[0] = -np.inf
+    x[1, 17] = np.inf
+    x[2, 5:] = -np.inf
+    logits = f32_to_bf16(x)
+    for kw in (dict(top_k=3), dict(top_k=7, min_p=0.1)):
+        assert np.array_equal(O.unified_sampling(logits, **kw), G.unified_sampling(ctx, logits, **kw))

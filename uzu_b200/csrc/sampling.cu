@@ -7,12 +7,15 @@
 // Two code paths:
 //   * no filters (greedy, or temperature + Gumbel): multi-CTA argmax over a packed (value, ~index)
 //     64-bit key, last CTA (ticket) merges -> one launch, ~V*2 bytes read at HBM/L2 speed;
-//   * with top-k / top-p / min-p: the kept set is a prefix of the (value desc, index asc) order and each
-//     condition is monotone along that order, so "kept" is a per-element predicate on (rank, mass before,
-//     value). One CTA per row iterates candidates: take the best post-noise element of the current set,
-//     compute its rank / preceding mass in one pass, accept if it passes the filters, otherwise shrink the
-//     set to the elements ranked before it (same idea as the reference's Metal kernel,
-//     metal/kernel/sampling/unified_sampling.metal:154-238).
+//   * with top-k / top-p / min-p: the kept set is a prefix of the (value desc, index asc) order, and equal values are equally likely, so
+//     what is kept follows from how often each of the 65536 bf16 values occurs. A cluster of 8 CTAs per row counts them in shared memory
+//     (a slice of the row per CTA, 16-bit counts), CTA c adds up the counts of an eighth of the values over distributed shared memory,
+//     and the cluster finds the one value at which the kept set ends and how many elements of that value are kept. Noise is then drawn
+//     for kept elements only. Sums of probabilities are f64 over exact counts: the same whatever the order of the atomics.
+//     Rows whose largest logit is not finite (everything masked, infinities, NaN) walk the candidates one by one instead
+//     (sampling_walk: take the best post-noise element of the current set, accept it if its rank and the mass before it pass, otherwise
+//     shrink the set to the elements ranked before it; metal/kernel/sampling/unified_sampling.metal:154-238), as does a vocabulary
+//     whose slice does not fit 16-bit counts.
 #include "common.cuh"
 
 namespace uzu {
@@ -122,14 +125,15 @@ __global__ void __launch_bounds__(1024) sampling_argmax_kernel(const uzu_unified
 // "ranked before c": strictly better in (value desc, index asc)
 __device__ __forceinline__ bool ranked_before(float lj, uint32_t j, float lc, uint32_t c) { return lj > lc || (lj == lc && j < c); }
 
-__global__ void __launch_bounds__(1024) sampling_filtered_kernel(const uzu_unified_sampling_args a) {
+// one CTA of 1024 threads: the candidates of row `row` one by one
+__device__ __noinline__ void sampling_walk(const uzu_unified_sampling_args& a, uint32_t row) {
     __shared__ float redf[32];
     __shared__ unsigned long long redk[32];
     __shared__ unsigned int redc[32];
     __shared__ unsigned long long s_key;
     __shared__ float s_f;
     __shared__ unsigned int s_c;
-    const uint32_t row = blockIdx.x, V = a.vocab_size;
+    const uint32_t V = a.vocab_size;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const __nv_bfloat16* logits = reinterpret_cast<const __nv_bfloat16*>(a.logits) + (size_t)row * V;
     const uint32_t* bitmask = a.has_bitmask ? reinterpret_cast<const uint32_t*>(a.bitmask) + (size_t)row * ((V + 31) / 32) : nullptr;
@@ -226,6 +230,239 @@ __global__ void __launch_bounds__(1024) sampling_filtered_kernel(const uzu_unifi
     if (threadIdx.x == 0) reinterpret_cast<uint32_t*>(a.output)[row] = result;
 }
 
+__global__ void __launch_bounds__(1024) sampling_walk_kernel(const uzu_unified_sampling_args a) { sampling_walk(a, blockIdx.x); }
+
+// order-preserving 16-bit key of a bf16 logit; -0 counts as +0 (they compare equal)
+__device__ __forceinline__ uint32_t bf16_key(uint16_t bits) {
+    if (bits == 0x8000u) bits = 0;
+    return (bits & 0x8000u) ? (uint32_t)(uint16_t)~bits : (uint32_t)bits | 0x8000u;
+}
+__device__ __forceinline__ float key_value(uint32_t key) {
+    return bf16_bits_to_f32((key & 0x8000u) ? (uint16_t)(key & 0x7FFFu) : (uint16_t)~key);
+}
+
+constexpr uint32_t SF_CTAS = 8, SF_THREADS = 1024;
+constexpr uint32_t SF_KEYS = 65536, SF_OWNED = SF_KEYS / SF_CTAS, SF_PER = SF_OWNED / SF_THREADS;    // keys per CTA and per thread when they are added up
+constexpr size_t SF_SMEM = SF_KEYS * sizeof(uint16_t);
+static_assert(SF_PER == 8, "a thread adds up eight neighbouring keys: one 16-byte read per CTA");
+
+// Bound: latency (a few cluster barriers, one pass over a 128 KB count table); the logits are read twice, the second time from L2.
+// 8 rows of 128256 logits, temperature, top-k 50, top-p 0.95: 40 us a call (268 us as one CTA per row walking the candidates).
+__global__ void __cluster_dims__(SF_CTAS, 1, 1) __launch_bounds__(SF_THREADS, 1) sampling_filtered_kernel(const uzu_unified_sampling_args a) {
+    extern __shared__ __align__(16) uint16_t sf_counts[];
+    // what the CTAs of the cluster tell one another, slot = the sender
+    __shared__ uint32_t x_top[SF_CTAS], x_n[SF_CTAS], x_edge[SF_CTAS], x_kept[SF_CTAS], x_same[SF_CTAS], x_bad[SF_CTAS];
+    __shared__ double x_mass[SF_CTAS];
+    __shared__ unsigned long long x_best[SF_CTAS];
+    __shared__ double red_d[32];
+    __shared__ uint32_t red_u[32];
+    __shared__ unsigned long long red_k[32];
+    pdl_launch_dependents();
+    pdl_wait();
+    const uint32_t V = a.vocab_size, row = blockIdx.y, rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint16_t* logits = reinterpret_cast<const uint16_t*>(a.logits) + (size_t)row * V;
+    const uint32_t* bitmask = a.has_bitmask ? reinterpret_cast<const uint32_t*>(a.bitmask) + (size_t)row * ((V + 31) / 32) : nullptr;
+    const float recip_t = a.has_temperature ? 1.0f / a.temperature : 1.0f;
+    const uint32_t slice = (V + SF_CTAS - 1) / SF_CTAS, lo = min(rank * slice, V), hi = min(lo + slice, V);
+    auto masked_bits = [&](uint32_t i) -> uint16_t {
+        const bool off = bitmask && ((bitmask[i >> 5] >> (i & 31)) & 1u) == 0u;
+        return off ? (uint16_t)0xFF80u : logits[i];
+    };
+    auto cluster_sync = [] { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); };
+    auto remote = [](const void* p, uint32_t cta) {
+        uint32_t r;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
+        return r;
+    };
+    auto tell_u32 = [&](uint32_t* slots, uint32_t v) {      // thread c < SF_CTAS tells CTA c
+        if (tid < SF_CTAS) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote(slots + rank, tid)), "r"(v) : "memory");
+    };
+    auto tell_u64 = [&](void* slot, unsigned long long v) {
+        if (tid < SF_CTAS) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote(slot, tid)), "l"(v) : "memory");
+    };
+    auto block_max_u = [&](uint32_t v) {
+        v = __reduce_max_sync(0xffffffffu, v);
+        __syncthreads();
+        if (lane == 0) red_u[warp] = v;
+        __syncthreads();
+        return __reduce_max_sync(0xffffffffu, red_u[lane]);
+    };
+    // exclusive sum over the threads AFTER this one (keys rise with the thread, ranks with falling keys) and the total
+    auto suffix_u = [&](uint32_t v, uint32_t& total) {
+        uint32_t s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_down_sync(0xffffffffu, s, o); if (lane + o < 32) s += t; }
+        __syncthreads();
+        if (lane == 0) red_u[warp] = s;
+        __syncthreads();
+        uint32_t w = red_u[lane], ws = w;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_down_sync(0xffffffffu, ws, o); if (lane + o < 32) ws += t; }
+        total = __shfl_sync(0xffffffffu, ws, 0);
+        return s - v + __shfl_sync(0xffffffffu, ws - w, warp);
+    };
+    auto suffix_d = [&](double v, double& total) {
+        double s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const double t = __shfl_down_sync(0xffffffffu, s, o); if (lane + o < 32) s += t; }
+        const double after = __shfl_down_sync(0xffffffffu, s, 1);
+        __syncthreads();
+        if (lane == 0) red_d[warp] = s;
+        __syncthreads();
+        double ws = red_d[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const double t = __shfl_down_sync(0xffffffffu, ws, o); if (lane + o < 32) ws += t; }
+        total = __shfl_sync(0xffffffffu, ws, 0);
+        const double warps_after = __shfl_down_sync(0xffffffffu, ws, 1);      // lane w: sum of the warps after w
+        const double mine = __shfl_sync(0xffffffffu, lane == 31 ? 0.0 : warps_after, warp);
+        return (lane == 31 ? 0.0 : after) + mine;
+    };
+
+    // 1. count the values of this CTA's slice
+    for (uint32_t i = tid; i < SF_KEYS / 8; i += SF_THREADS) reinterpret_cast<uint4*>(sf_counts)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    uint32_t bad = 0;
+    for (uint32_t i = lo + tid; i < hi; i += SF_THREADS) {
+        const uint16_t bits = masked_bits(i);
+        bad |= (uint32_t)((bits & 0x7FFFu) > 0x7F80u) | (uint32_t)(bits == 0x7F80u);       // NaN, +inf
+        const uint32_t key = bf16_key(bits);
+        atomicAdd(reinterpret_cast<uint32_t*>(sf_counts) + (key >> 1), (key & 1u) ? 0x10000u : 1u);
+    }
+    bad = (uint32_t)__syncthreads_or((int)bad);
+    cluster_sync();
+    // 2. add up the eight keys this thread owns over the CTAs' tables
+    uint32_t n[SF_PER];
+#pragma unroll
+    for (uint32_t j = 0; j < SF_PER; ++j) n[j] = 0;
+    const uint32_t key0 = rank * SF_OWNED + tid * SF_PER;
+#pragma unroll
+    for (uint32_t c = 0; c < SF_CTAS; ++c) {
+        uint4 v;
+        asm volatile("ld.shared::cluster.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(remote(sf_counts + key0, c)));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { n[2 * j] += w[j] & 0xFFFFu; n[2 * j + 1] += w[j] >> 16; }
+    }
+    uint32_t top = 0, mine = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < SF_PER; ++j) {
+        if (n[j]) top = key0 + j;
+        mine += n[j];
+    }
+    uint32_t cta_n;
+    const uint32_t after_n = suffix_u(mine, cta_n);
+    top = block_max_u(top);
+    tell_u32(x_top, top);
+    tell_u32(x_n, cta_n);
+    tell_u32(x_bad, bad);
+    cluster_sync();
+    top = 0;
+    uint32_t rank0 = after_n;                        // elements with a larger key than this thread's
+    for (uint32_t c = 0; c < SF_CTAS; ++c) {
+        top = max(top, x_top[c]);
+        bad |= x_bad[c];
+        if (c > rank) rank0 += x_n[c];
+    }
+    const float lmax = key_value(top) * recip_t;
+    // not finite, or a temperature that could make different values equal: the general walk
+    if (bad || !(fabsf(lmax) < INFINITY) || !(recip_t > 1.52587890625e-5f && recip_t < 65536.0f)) {
+        if (rank == 0) sampling_walk(a, row);
+        return;                                      // (uniform over the cluster; no CTA reads another's memory any more)
+    }
+    // 3. probabilities: f64 sums of counts * exp(l - lmax)
+    double e[SF_PER], mass = 0.0;
+#pragma unroll
+    for (uint32_t j = 0; j < SF_PER; ++j) {
+        e[j] = n[j] ? (double)expf(key_value(key0 + j) * recip_t - lmax) : 0.0;
+        mass += (double)n[j] * e[j];
+    }
+    double cta_mass;
+    double mass0 = suffix_d(mass, cta_mass);
+    tell_u64(x_mass + rank, (unsigned long long)__double_as_longlong(cta_mass));
+    cluster_sync();
+    double norm = 0.0;
+    for (uint32_t c = 0; c < SF_CTAS; ++c) {
+        norm += x_mass[c];
+        if (c > rank) mass0 += x_mass[c];
+    }
+    // 4. the kept elements of each value: those of rank < top_k, mass before < top_p, value >= min_p threshold. The kept set ends at the
+    //    largest key that is not kept as a whole.
+    const float min_p_thr = a.has_min_p ? lmax + logf(a.min_p) : -INFINITY;
+    const double limit = (double)a.top_p * norm;
+    uint32_t edge = 0, kept_at_edge = 0;             // edge = key + 1, 0 = none
+#pragma unroll
+    for (int j = (int)SF_PER - 1; j >= 0; --j) {
+        if (n[j] && !edge) {
+            uint32_t q = n[j];
+            if (a.has_top_k) q = rank0 >= a.top_k ? 0u : min(q, a.top_k - rank0);
+            if (a.has_top_p) {                       // element i of this value is kept while mass0 + i e < limit
+                const double room = limit - mass0;
+                if (!(room > 0.0)) q = 0;
+                else if (e[j] > 0.0 && room < e[j] * (double)q) q = min(q, (uint32_t)ceil(room / e[j]));
+            }
+            if (a.has_min_p && key_value(key0 + j) * recip_t < min_p_thr) q = 0;
+            if (q < n[j]) { edge = key0 + j + 1; kept_at_edge = q; }
+        }
+        rank0 += n[j];
+        mass0 += (double)n[j] * e[j];
+    }
+    const uint32_t cta_edge = block_max_u(edge);
+    __syncthreads();                                 // all have read red_u
+    if (cta_edge && edge == cta_edge) red_u[0] = kept_at_edge;       // (one thread owns the key)
+    __syncthreads();
+    kept_at_edge = red_u[0];
+    tell_u32(x_edge, cta_edge);
+    tell_u32(x_kept, kept_at_edge);
+    cluster_sync();
+    edge = 0;
+    uint32_t quota = 0;
+    for (uint32_t c = 0; c < SF_CTAS; ++c)
+        if (x_edge[c] > edge) { edge = x_edge[c]; quota = x_kept[c]; }
+    // 5. elements of the edge value are kept by rising index: the slices before this CTA's come first
+    const uint32_t edge_key = edge - 1;              // (edge = 0: every element is kept)
+    tell_u32(x_same, edge ? (uint32_t)sf_counts[edge_key] : 0u);
+    cluster_sync();
+    for (uint32_t c = 0; c < rank; ++c) quota -= min(quota, x_same[c]);
+    const uint64_t seed = a.is_stochastic ? reinterpret_cast<const unsigned long long*>(a.seeds)[row] : 0ull;
+    unsigned long long best = 0ull;
+    auto offer = [&](uint32_t i, uint16_t bits) {
+        float v = bf16_bits_to_f32(bits) * recip_t;
+        if (a.is_stochastic) v += gumbel_noise(seed, i, V);
+        const unsigned long long k = pack_key(v, i);
+        best = k > best ? k : best;
+    };
+    const bool count_equal = edge != 0 && quota != 0 && quota < sf_counts[edge_key];     // (uniform over the CTA)
+    for (uint32_t i0 = lo; i0 < hi; i0 += SF_THREADS) {
+        const uint32_t i = i0 + tid;
+        const uint16_t bits = i < hi ? masked_bits(i) : (uint16_t)0xFF80u;
+        const uint32_t key = i < hi ? bf16_key(bits) + 1u : 0u;
+        bool keep = i < hi && key > edge;
+        const bool equal = edge != 0 && key == edge;
+        if (count_equal) {
+            const uint32_t b = __ballot_sync(0xffffffffu, equal);
+            __syncthreads();
+            if (lane == 0) red_u[warp] = (uint32_t)__popc(b);
+            __syncthreads();
+            const uint32_t w = red_u[lane];
+            const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u) + (uint32_t)__popc(b & ((1u << lane) - 1u));
+            const uint32_t all = __reduce_add_sync(0xffffffffu, w);
+            if (equal && before < quota) keep = true;
+            quota -= min(quota, all);
+        } else if (equal && quota != 0) keep = true;
+        if (keep) offer(i, bits);
+    }
+    best = warp_max_u64(best);
+    if (lane == 0) red_k[warp] = best;
+    __syncthreads();
+    best = warp_max_u64(red_k[lane]);
+    if (tid == 0) asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(remote(x_best + rank, 0)), "l"(best) : "memory");
+    cluster_sync();
+    if (rank == 0 && warp == 0) {
+        best = warp_max_u64(lane < SF_CTAS ? x_best[lane] : 0ull);
+        if (lane == 0) reinterpret_cast<uint32_t*>(a.output)[row] = best ? 0xFFFFFFFFu - (uint32_t)(best & 0xFFFFFFFFull) : 0u;   // nothing kept: index 0
+    }
+}
+
 }  // namespace uzu
 
 extern "C" {
@@ -240,8 +477,20 @@ void uzu_unified_sampling_encode(uzu_command_buffer* cmd, const uzu_unified_samp
     if (a->batch_size == 0) return;
     uzu_context* ctx = cmd->ctx;
     if (a->has_top_k || a->has_top_p || a->has_min_p) {
-        uzu::sampling_filtered_kernel<<<a->batch_size, 1024, 0, ctx->stream>>>(*a);
-        uzu::after_launch(cmd, "sampling_filtered_kernel");
+        if (a->vocab_size > uzu::SF_CTAS * 65535u) {         // 16-bit counts per slice
+            uzu::sampling_walk_kernel<<<a->batch_size, 1024, 0, ctx->stream>>>(*a);
+            uzu::after_launch(cmd, "sampling_walk_kernel");
+            return;
+        }
+        static std::atomic<uint64_t> smem_opt_in{0};
+        uzu::opt_in_dynamic_smem(cmd, uzu::sampling_filtered_kernel, (int)uzu::SF_SMEM, smem_opt_in);
+        for (uint32_t row0 = 0; row0 < a->batch_size; row0 += 65535u) {      // (rows are the grid's y axis)
+            uzu_unified_sampling_args b = *a;
+            b.logits += (uint64_t)row0 * a->vocab_size * 2; b.output += (uint64_t)row0 * 4; b.seeds += a->is_stochastic ? (uint64_t)row0 * 8 : 0;
+            b.bitmask += a->has_bitmask ? (uint64_t)row0 * ((a->vocab_size + 31) / 32) * 4 : 0;
+            b.batch_size = std::min(65535u, a->batch_size - row0);
+            uzu::launch(cmd, "sampling_filtered_kernel", uzu::sampling_filtered_kernel, dim3(uzu::SF_CTAS, b.batch_size), dim3(uzu::SF_THREADS), uzu::SF_SMEM, b);
+        }
         return;
     }
     uint32_t nblocks = std::min(uzu::SAMPLING_MAX_BLOCKS, (a->vocab_size + 8191u) / 8192u);
