@@ -59,3 +59,28 @@ def test_prefill_attention_token_major_cache_matches_decode_kernel(prefill_attn)
     ctx.lib.uzu_debug_set_prefill_attention(1)
     assert_bf16_close(got, base, max_ulp=1, min_exact=0.9, what="tensor-core vs split-KV kernel")
     assert_bf16_close(got, O.attention_single_pass(q, k, v, **kw), max_ulp=1, min_exact=0.95, what="vs oracle")
+
+
+@pytest.mark.parametrize("H,Hkv,prefix,suffix,D", [(8, 2, 0, 64, 256), (8, 2, 700, 33, 256), (3, 1, 130, 21, 64), (12, 2, 65, 5, 128), (32, 8, 1500, 16, 128), (4, 4, 63, 4, 256), (2, 1, 0, 31, 64)])
+@pytest.mark.parametrize("trie", [False, True])
+def test_rows_of_grouped_heads(ctx, H, Hkv, prefix, suffix, D, trie):
+    """Rows of (token, head) pairs: tiles that end inside a token's heads, head counts that do not divide a tile, 256 channels, few rows over
+    many keys (a cluster shares them, some of its CTAs without a tile), and a trie's masks; the cache behind the last key is NaN."""
+    rng = np.random.default_rng(H + prefix + suffix)
+    n, G_ = prefix + suffix, H // Hkv
+    if trie and suffix > 16:
+        suffix, n = 16, prefix + 16
+    q = f32_to_bf16(rng.standard_normal((H, suffix, D)).astype(np.float32))
+    k, v = (f32_to_bf16(rng.standard_normal((n + 64, Hkv * D)).astype(np.float32)) for _ in range(2))
+    k[n:], v[n:] = 0x7FC0, 0x7FC0
+    kw = dict(head_dim=D, gqa_factor=G_, sequence_length=n, k_head_stride=D, k_seq_stride=Hkv * D, v_head_stride=D, v_seq_stride=Hkv * D,
+              scale=float(D ** -0.5), num_heads=H, suffix_length=suffix, is_causal=True)
+    if trie:
+        heights = [0]
+        for _ in range(suffix - 1):
+            heights.append(int(rng.integers(1, heights[-1] + 2)))
+        ends = [max(j for j in range(i, suffix) if all(heights[x] > heights[i] for x in range(i + 1, j + 1))) for i in range(suffix)]
+        kw["trie"] = np.array([[i, ends[i], heights[i]] for i in range(suffix)], dtype=np.uint32)
+    ref = O.attention_single_pass(q, k, v, **kw)
+    got = G.attention_single_pass(ctx, q, k, v, **kw)
+    assert_bf16_close(got, ref, max_ulp=1, min_exact=0.95, what="grouped rows vs oracle")

@@ -1,22 +1,23 @@
-// Prefill attention on tensor cores (suffix >= 16 query tokens): flash-attention-style tiling over the token-major KV cache.
-//
-//   OPT-IN (UZU_PREFILL_ATTN=1). Written after round 1's GPU budget was spent; its only hardware run so far is tools/prefill_attn_probe.py
-//   (3 shapes within one bf16 step of a float64 softmax, profiles/r1_prefill_attention_probe.txt). Until tests/test_prefill_attention_gpu.py
-//   (oracle ulp comparison, enabled with UZU_TEST_PREFILL_ATTN=1) and the engine tests have run through it, the default prefill path stays
-//   the split-KV decode kernel applied per query token (attention.cu).
+// Attention of several query tokens on the tensor cores: prompt chunks, short portions and speculation passes over the token-major KV cache.
 //
 // Semantic spec: backends/cpu/kernel/attention/attention_single_pass.rs:49-126 (online softmax per query over the visible keys, q scaled by
 // `scale`, GQA kv_head = h / gqa, output [suffix, heads, D] cast after the division by the sum), mask.rs:3-62 restricted to the plain causal /
-// non-causal case (no ring, trie, sliding window, sinks: those keep the decode kernel).
+// non-causal case and the trie (no ring, sliding window, sinks: those keep the split-KV kernel of attention.cu).
 //
-// One CTA = 16 query tokens x one KV head; its G = heads-per-KV-head warps each own one query head and share the K / V tiles:
-//   * S = Q K^T with mma.sync.m16n8k16 (bf16 x bf16 products are exact, f32 accumulate), Q fragments live in registers, the K tile
-//     (64 keys x D, rows padded to D + 8 so the 32-bit fragment loads are bank-conflict free) arrives by cp.async, double buffered;
-//   * online softmax in f32 registers (expf, like the reference), the row statistics reduced over the 4 lanes of a quad;
+// One CTA = 64 rows of one KV head, a row being one (query token, query head) pair: the heads that share a KV head read its keys and values
+// once, and a speculation pass of 16 nodes x 4 heads is one tile. Four warps of 16 rows:
+//   * S = Q K^T with mma.sync.m16n8k16 (bf16 x bf16 products are exact, f32 accumulate), Q, K and V fragments by ldmatrix from shared memory
+//     (64 keys x D, rows padded to D + 8: conflict-free);
+//   * online softmax in f32 registers, row statistics over the 4 lanes of a quad; O is rescaled only when some row's maximum moved;
 //   * O += P V with P split into two bf16 planes (hi = bf16(p), lo = bf16(p - hi)): a single rounded plane would put 2^-9 on every
-//     probability, the same budget argument as the prefill GEMM's weight planes; V fragments come from ldmatrix.trans.
-// Causal blocks past the CTA's last query are never loaded. Work per CTA grows with the query index; CTAs are launched in reverse
-// (longest first) so the tail is short.
+//     probability; V fragments come from ldmatrix.trans.
+// The next key tile is requested when S is done (it arrives during P V), the next value tile when P V is done: one buffer each, so that two or
+// three CTAs share an SM and fill one another's waits. Causal tiles past the CTA's last query are never loaded, and tiles every row of a
+// warp sees whole are not masked. CTAs with the most keys start first.
+// Where rows x KV heads do not fill the chip a cluster of up to 8 CTAs shares the keys of a tile and merges its partial results over
+// distributed shared memory in rank order.
+// Bound: shared-memory reads and mma.sync issue. 8 heads of 256 channels (2 KV heads), 1024 rows behind 1024: 0.10 ms against 1.11 ms one query
+// token at a time on the split-KV kernel.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -25,7 +26,7 @@
 
 namespace uzu {
 
-constexpr int PA_BM = 16;   // query rows per CTA (one m16 tile per warp)
+constexpr int PA_BM = 64;   // rows per CTA
 constexpr int PA_BN = 64;   // keys per K / V tile
 
 __device__ __forceinline__ void pa_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -33,200 +34,299 @@ __device__ __forceinline__ void pa_mma(float (&d)[4], const uint32_t (&a)[4], ui
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void pa_ldmatrix_x2_trans(uint32_t& r0, uint32_t& r1, const void* smem_ptr) {
-    const uint32_t addr = (uint32_t)__cvta_generic_to_shared(smem_ptr);
-    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r0), "=r"(r1) : "r"(addr));
+__device__ __forceinline__ void pa_ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-__device__ __forceinline__ void pa_cp16(void* dst_smem, const void* src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst_smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(valid ? 16u : 0u) : "memory");
+__device__ __forceinline__ void pa_ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void pa_cp16(uint32_t dst_smem, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(valid ? 16u : 0u) : "memory");
 }
 __device__ __forceinline__ uint32_t pa_pack(float lo_elem, float hi_elem) {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo_elem, hi_elem);
     return *reinterpret_cast<uint32_t*>(&v);
 }
+__device__ __forceinline__ void pa_cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float pa_remote(uint32_t addr, uint32_t rank) {
+    uint32_t remote;
+    float x;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote) : "memory");
+    return x;
+}
 
-template <int D, int G>
-__global__ void __launch_bounds__(G * 32) attn_prefill_kernel(const uzu_attention_args a) {
-    constexpr int LD = D + 8;                       // padded tile row (elements): 16-byte aligned rows, conflict-free fragment loads
-    constexpr int TILE = PA_BN * LD;
-    constexpr int CH = D / 8;                       // 16-byte chunks per row
+template <int D>
+__global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(const uzu_attention_args a, const uint32_t splits) {
+    constexpr uint32_t LD = D + 8;                  // padded tile row (elements): 16-byte aligned rows, conflict-free ldmatrix
+    constexpr uint32_t TILE = PA_BN * LD * 2;       // bytes
+    constexpr uint32_t CH = D / 8;                  // 16-byte chunks per row
+    constexpr float kLog2e = 1.4426950408889634f;
     extern __shared__ __align__(16) uint8_t pa_smem[];
-    __nv_bfloat16* sk = reinterpret_cast<__nv_bfloat16*>(pa_smem);   // [2][TILE]
-    __nv_bfloat16* sv = sk + 2 * TILE;                                // [2][TILE]
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = lane >> 2, tq = lane & 3;
-    const uint32_t m = a.suffix_length, seq = a.sequence_length, prefix = seq - m;
-    const uint32_t qblk = gridDim.x - 1u - blockIdx.x;              // longest (latest queries) first
-    const uint32_t q0 = qblk * PA_BM, kvh = blockIdx.y, h = kvh * G + (uint32_t)warp;
-    const uint32_t q_hi = min(q0 + (uint32_t)PA_BM, m);
-    const uint32_t kend = a.is_causal ? prefix + q_hi : seq;        // keys [0, kend) can be visible to some row of this CTA
-    const uint32_t nblocks = (kend + PA_BN - 1) / PA_BN;
+    const uint32_t sq = (uint32_t)__cvta_generic_to_shared(pa_smem), sk = sq + TILE, sv = sk + TILE;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = lane >> 2, tq = lane & 3;
+    const uint32_t G = a.gqa_factor, m = a.suffix_length, seq = a.sequence_length, prefix = seq - m, rows = m * G;
+    const uint32_t rank = splits > 1 ? blockIdx.x % splits : 0u;
+    const uint32_t tile = gridDim.x / splits - 1u - blockIdx.x / splits;      // the rows with the most keys first
+    const uint32_t row0 = tile * PA_BM, kvh = blockIdx.y;
+    const bool causal = a.is_causal != 0;
+    const uint32_t q_last = min(row0 + (uint32_t)PA_BM, rows) - 1u;           // last row of the CTA
+    // keys [0, kend) can be visible to some row of this CTA (a trie node may be seen by any later node: all suffix keys)
+    const uint32_t kend = causal && !a.is_trie ? prefix + q_last / G + 1u : seq;
+    const uint32_t all_tiles = (kend + PA_BN - 1) / PA_BN, per = (all_tiles + splits - 1) / splits;
+    const uint32_t t_begin = min(rank * per, all_tiles), t_end = min(t_begin + per, all_tiles);
     const __nv_bfloat16* kbase = reinterpret_cast<const __nv_bfloat16*>(a.keys) + (size_t)kvh * a.k_head_stride;
     const __nv_bfloat16* vbase = reinterpret_cast<const __nv_bfloat16*>(a.values) + (size_t)kvh * a.v_head_stride;
 
-    // ---- Q fragments (A operand, row-major 16 x 16 per k step): a0 (row g, k 2t..), a1 (row g+8), a2 (row g, k 2t+8..), a3 (row g+8) ----
-    uint32_t qf[D / 16][4];
-    {
-        const __nv_bfloat16* qh = reinterpret_cast<const __nv_bfloat16*>(a.queries) + (size_t)h * m * D;
-        const uint32_t r0 = q0 + quad, r1 = r0 + 8;
-#pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-            const int c0 = ks * 16 + 2 * tq;
-            qf[ks][0] = r0 < m ? *reinterpret_cast<const uint32_t*>(qh + (size_t)r0 * D + c0) : 0u;
-            qf[ks][1] = r1 < m ? *reinterpret_cast<const uint32_t*>(qh + (size_t)r1 * D + c0) : 0u;
-            qf[ks][2] = r0 < m ? *reinterpret_cast<const uint32_t*>(qh + (size_t)r0 * D + c0 + 8) : 0u;
-            qf[ks][3] = r1 < m ? *reinterpret_cast<const uint32_t*>(qh + (size_t)r1 * D + c0 + 8) : 0u;
-        }
-    }
-
-    auto load_tiles = [&](uint32_t kb, int stage) {
-        __nv_bfloat16* dk = sk + stage * TILE;
-        __nv_bfloat16* dv = sv + stage * TILE;
-        for (int c = threadIdx.x; c < PA_BN * CH; c += G * 32) {
-            const int key = c / CH, ch = c % CH;
-            const uint32_t kg = kb * PA_BN + (uint32_t)key;
+    auto load_tile = [&](uint32_t dst, const __nv_bfloat16* src, size_t stride, uint32_t t) {
+#pragma unroll 4
+        for (uint32_t c = tid; c < PA_BN * CH; c += 128) {
+            const uint32_t key = c / CH, ch = c % CH, kg = t * PA_BN + key;
             const bool ok = kg < kend;                               // rows past the visible range may be unmapped cache pages: never read
-            const size_t row = ok ? kg : 0u;
-            pa_cp16(dk + key * LD + ch * 8, kbase + row * a.k_seq_stride + ch * 8, ok);
-            pa_cp16(dv + key * LD + ch * 8, vbase + row * a.v_seq_stride + ch * 8, ok);
+            pa_cp16(dst + (key * LD + ch * 8) * 2, src + (size_t)(ok ? kg : 0u) * stride + ch * 8, ok);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    for (uint32_t c = tid; c < PA_BM * CH; c += 128) {               // row r of the tile: token r / G, head r % G of the group
+        const uint32_t r = c / CH, ch = c % CH, row = row0 + r;
+        const bool ok = row < rows;
+        const uint32_t token = ok ? row / G : 0u, head = kvh * G + (ok ? row % G : 0u);
+        pa_cp16(sq + (r * LD + ch * 8) * 2, reinterpret_cast<const __nv_bfloat16*>(a.queries) + ((size_t)head * m + token) * D + ch * 8, ok);
+    }
+    if (t_begin < t_end) load_tile(sk, kbase, a.k_seq_stride, t_begin);      // (one group with the queries)
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    if (t_begin < t_end) load_tile(sv, vbase, a.v_seq_stride, t_begin);
 
     float o[D / 8][4];
 #pragma unroll
     for (int nd = 0; nd < D / 8; ++nd) o[nd][0] = o[nd][1] = o[nd][2] = o[nd][3] = 0.0f;
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;     // running max / sum of rows (quad) and (quad + 8)
-    const uint32_t qr0 = q0 + quad, qr1 = qr0 + 8;
-    // exclusive key bound per row: causal -> keys up to and including the query's own position
-    const uint32_t lim0 = qr0 < m ? (a.is_causal ? prefix + qr0 + 1 : seq) : 0u;
-    const uint32_t lim1 = qr1 < m ? (a.is_causal ? prefix + qr1 + 1 : seq) : 0u;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.0f, l1 = 0.0f;     // running max (in units of ln 2) / sum of rows r0 and r0 + 8
+    const uint32_t r0 = row0 + warp * 16 + quad, r1 = r0 + 8;
+    // exclusive key bound per row: causal -> keys up to and including the query's own position; trie: the prefix, suffix keys by their node's range
+    const uint32_t n0 = r0 / G, n1 = r1 / G;
+    const uint32_t lim0 = r0 < rows ? (!causal ? seq : a.is_trie ? prefix : prefix + n0 + 1) : 0u;
+    const uint32_t lim1 = r1 < rows ? (!causal ? seq : a.is_trie ? prefix : prefix + n1 + 1) : 0u;
+    const uint32_t w_first = row0 + warp * 16, w_last = w_first + 15;        // every row of the warp sees keys below `whole`
+    const uint32_t whole = w_last >= rows ? 0u : (!causal ? seq : a.is_trie ? prefix : prefix + w_first / G + 1);
+    const bool trie = causal && a.is_trie;
+    const uzu_trie_node* nodes = reinterpret_cast<const uzu_trie_node*>(a.trie);
+    auto sees = [&](uint32_t key, uint32_t lim, uint32_t node, bool row_ok) {
+        if (key < lim) return true;
+        if (!trie || !row_ok || key < prefix || key >= seq) return false;
+        const uzu_trie_node& n = nodes[key - prefix];
+        return node >= n.trie_start && node <= n.trie_end;
+    };
+    const float scale2 = a.scale * kLog2e;
+    // ldmatrix rows of this lane: Q (16 rows x 16 d): row lane & 15, d half lane >> 4; K (two 8-key tiles): key (lane >> 4) * 8 + (lane & 7), d half
+    // (lane >> 3) & 1; V (16 keys x two 8-d tiles): key lane & 15, d half lane >> 4
+    const uint32_t q_addr = sq + ((warp * 16 + (lane & 15)) * LD + (lane >> 4) * 8) * 2;
+    const uint32_t k_addr = sk + (((lane >> 4) * 8 + (lane & 7)) * LD + ((lane >> 3) & 1) * 8) * 2;
+    const uint32_t v_addr = sv + ((lane & 15) * LD + (lane >> 4) * 8) * 2;
 
-    if (nblocks > 0) load_tiles(0, 0);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    for (uint32_t kb = 0; kb < nblocks; ++kb) {
-        const int stage = kb & 1;
-        if (kb + 1 < nblocks) load_tiles(kb + 1, stage ^ 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 1;" ::: "memory");        // tile kb has landed (tile kb + 1 may be in flight)
+    for (uint32_t t = t_begin; t < t_end; ++t) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");        // this tile's keys (and the queries) have landed
         __syncthreads();
-        const __nv_bfloat16* kt = sk + stage * TILE;
-        const __nv_bfloat16* vt = sv + stage * TILE;
-
-        // ---- S = Q K^T: B fragment b0 = K[key = nt*8 + g][d = ks*16 + 2t .. +1], b1 = same key, d + 8 ----
+        // ---- S = Q K^T ----
         float s[PA_BN / 8][4];
 #pragma unroll
         for (int nt = 0; nt < PA_BN / 8; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
+            uint32_t qf[4];
+            pa_ldmatrix_x4(qf, q_addr + ks * 32);
 #pragma unroll
-            for (int nt = 0; nt < PA_BN / 8; ++nt) {
-                const __nv_bfloat16* kp = kt + (nt * 8 + quad) * LD + ks * 16 + 2 * tq;
-                pa_mma(s[nt], qf[ks], *reinterpret_cast<const uint32_t*>(kp), *reinterpret_cast<const uint32_t*>(kp + 8));
+            for (int nt = 0; nt < PA_BN / 8; nt += 2) {
+                uint32_t kf[4];
+                pa_ldmatrix_x4(kf, k_addr + nt * 8 * LD * 2 + ks * 32);
+                pa_mma(s[nt], qf, kf[0], kf[1]);
+                pa_mma(s[nt + 1], qf, kf[2], kf[3]);
             }
         }
-        // ---- scale, mask, online softmax (c0,c1: row g, cols 2t, 2t+1; c2,c3: row g+8) ----
+        __syncthreads();                                            // every warp is done with the key tile
+        if (t + 1 < t_end) load_tile(sk, kbase, a.k_seq_stride, t + 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        // ---- scale, mask, online softmax (c0,c1: row r0, keys 2t, 2t+1; c2,c3: row r0 + 8) ----
+        const uint32_t key0 = t * PA_BN + 2 * tq;
         float mx0 = -INFINITY, mx1 = -INFINITY;
+        if ((t + 1) * PA_BN <= whole) {
 #pragma unroll
-        for (int nt = 0; nt < PA_BN / 8; ++nt) {
-            const uint32_t kg = kb * PA_BN + nt * 8 + 2 * tq;
-            s[nt][0] = kg < lim0 ? s[nt][0] * a.scale : -INFINITY;
-            s[nt][1] = kg + 1 < lim0 ? s[nt][1] * a.scale : -INFINITY;
-            s[nt][2] = kg < lim1 ? s[nt][2] * a.scale : -INFINITY;
-            s[nt][3] = kg + 1 < lim1 ? s[nt][3] * a.scale : -INFINITY;
-            mx0 = fmaxf(mx0, fmaxf(s[nt][0], s[nt][1]));
-            mx1 = fmaxf(mx1, fmaxf(s[nt][2], s[nt][3]));
+            for (int nt = 0; nt < PA_BN / 8; ++nt) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) s[nt][c] *= scale2;
+                mx0 = fmaxf(mx0, fmaxf(s[nt][0], s[nt][1]));
+                mx1 = fmaxf(mx1, fmaxf(s[nt][2], s[nt][3]));
+            }
+        } else {
+#pragma unroll
+            for (int nt = 0; nt < PA_BN / 8; ++nt) {
+                const uint32_t kg = key0 + nt * 8;
+                s[nt][0] = sees(kg, lim0, n0, r0 < rows) ? s[nt][0] * scale2 : -INFINITY;
+                s[nt][1] = sees(kg + 1, lim0, n0, r0 < rows) ? s[nt][1] * scale2 : -INFINITY;
+                s[nt][2] = sees(kg, lim1, n1, r1 < rows) ? s[nt][2] * scale2 : -INFINITY;
+                s[nt][3] = sees(kg + 1, lim1, n1, r1 < rows) ? s[nt][3] * scale2 : -INFINITY;
+                mx0 = fmaxf(mx0, fmaxf(s[nt][0], s[nt][1]));
+                mx1 = fmaxf(mx1, fmaxf(s[nt][2], s[nt][3]));
+            }
         }
         mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, 2));
         mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, 2));
-        const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);
-        const float c0 = n0 == -INFINITY ? 1.0f : expf(m0 - n0), c1 = n1 == -INFINITY ? 1.0f : expf(m1 - n1);   // expf(-inf) = 0
+        const float top0 = fmaxf(m0, mx0), top1 = fmaxf(m1, mx1);
+        const float base0 = top0 == -INFINITY ? 0.0f : top0, base1 = top1 == -INFINITY ? 0.0f : top1;      // (exp2(-inf - 0) = 0)
+        const float c0 = exp2f(m0 - base0), c1 = exp2f(m1 - base1);
+        const bool moved = __any_sync(0xffffffffu, top0 != m0 || top1 != m1);
         float rs0 = 0.0f, rs1 = 0.0f;
 #pragma unroll
         for (int nt = 0; nt < PA_BN / 8; ++nt) {
-            s[nt][0] = n0 == -INFINITY ? 0.0f : expf(s[nt][0] - n0);
-            s[nt][1] = n0 == -INFINITY ? 0.0f : expf(s[nt][1] - n0);
-            s[nt][2] = n1 == -INFINITY ? 0.0f : expf(s[nt][2] - n1);
-            s[nt][3] = n1 == -INFINITY ? 0.0f : expf(s[nt][3] - n1);
+            s[nt][0] = exp2f(s[nt][0] - base0);
+            s[nt][1] = exp2f(s[nt][1] - base0);
+            s[nt][2] = exp2f(s[nt][2] - base1);
+            s[nt][3] = exp2f(s[nt][3] - base1);
             rs0 += s[nt][0] + s[nt][1];
             rs1 += s[nt][2] + s[nt][3];
         }
-        rs0 += __shfl_xor_sync(0xffffffffu, rs0, 1); rs0 += __shfl_xor_sync(0xffffffffu, rs0, 2);
-        rs1 += __shfl_xor_sync(0xffffffffu, rs1, 1); rs1 += __shfl_xor_sync(0xffffffffu, rs1, 2);
-        l0 = l0 * c0 + rs0;
-        l1 = l1 * c1 + rs1;
-        m0 = n0;
-        m1 = n1;
+        if (moved) {
+            l0 *= c0;
+            l1 *= c1;
 #pragma unroll
-        for (int nd = 0; nd < D / 8; ++nd) {
-            o[nd][0] *= c0; o[nd][1] *= c0;
-            o[nd][2] *= c1; o[nd][3] *= c1;
+            for (int nd = 0; nd < D / 8; ++nd) {
+                o[nd][0] *= c0; o[nd][1] *= c0;
+                o[nd][2] *= c1; o[nd][3] *= c1;
+            }
         }
+        l0 += rs0;                                                  // (a lane's share of the row sum; the quad meets at the end)
+        l1 += rs1;
+        m0 = top0;
+        m1 = top1;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");        // this tile's values have landed
+        __syncthreads();
         // ---- O += P V: the S accumulator layout IS the A fragment layout of the next MMA (k = key) ----
 #pragma unroll
-        for (int kt2 = 0; kt2 < PA_BN / 16; ++kt2) {
+        for (int kt = 0; kt < PA_BN / 16; ++kt) {
             uint32_t ph[4], pl[4];
-            const float* e0 = s[2 * kt2];
-            const float* e1 = s[2 * kt2 + 1];
+            const float* e0 = s[2 * kt];
+            const float* e1 = s[2 * kt + 1];
             const float pv[8] = {e0[0], e0[1], e0[2], e0[3], e1[0], e1[1], e1[2], e1[3]};
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {   // a0 = (row g, k 2t..): e0[0..1]; a1 = (row g+8): e0[2..3]; a2 = (row g, k+8): e1[0..1]; a3: e1[2..3]
+            for (int r = 0; r < 4; ++r) {   // a0 = (row, k 2t..): e0[0..1]; a1 = (row + 8): e0[2..3]; a2 = (row, k + 8): e1[0..1]; a3: e1[2..3]
                 const float x = pv[2 * r], y = pv[2 * r + 1];
                 ph[r] = pa_pack(x, y);
                 pl[r] = pa_pack(x - __uint_as_float(ph[r] << 16), y - __uint_as_float(ph[r] & 0xffff0000u));
             }
 #pragma unroll
-            for (int nd = 0; nd < D / 8; ++nd) {
-                uint32_t b0, b1;   // B[k = key][n = d]: V rows are keys -> transposed 8x8 loads; lanes 0-15 address rows kt2*16 + lane
-                pa_ldmatrix_x2_trans(b0, b1, vt + (kt2 * 16 + (lane & 15)) * LD + nd * 8);
-                pa_mma(o[nd], ph, b0, b1);
-                pa_mma(o[nd], pl, b0, b1);
+            for (int nd = 0; nd < D / 8; nd += 2) {
+                uint32_t vf[4];
+                pa_ldmatrix_x4_trans(vf, v_addr + kt * 16 * LD * 2 + nd * 16);
+                pa_mma(o[nd], ph, vf[0], vf[1]);
+                pa_mma(o[nd + 1], ph, vf[2], vf[3]);
+                pa_mma(o[nd], pl, vf[0], vf[1]);
+                pa_mma(o[nd + 1], pl, vf[2], vf[3]);
             }
         }
-        __syncthreads();                                            // everyone is done with this stage before it is refilled
+        __syncthreads();                                            // every warp is done with the value tile
+        if (t + 1 < t_end) load_tile(sv, vbase, a.v_seq_stride, t + 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, 1); l1 += __shfl_xor_sync(0xffffffffu, l1, 2);
 
     // ---- out[token, head, d] = O / l, cast after the division ----
     __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out);
-    const float i0 = l0 > 0.0f ? 1.0f / l0 : 0.0f, i1 = l1 > 0.0f ? 1.0f / l1 : 0.0f;
+    auto out_row = [&](uint32_t row) { return out + ((size_t)(row / G) * a.num_heads + kvh * G + row % G) * D; };
+    if (splits == 1) {
+        const float i0 = l0 > 0.0f ? 1.0f / l0 : 0.0f, i1 = l1 > 0.0f ? 1.0f / l1 : 0.0f;
+#pragma unroll
+        for (int nd = 0; nd < D / 8; ++nd) {
+            const int d = nd * 8 + 2 * tq;
+            if (r0 < rows) *reinterpret_cast<uint32_t*>(out_row(r0) + d) = pa_pack(o[nd][0] * i0, o[nd][1] * i0);
+            if (r1 < rows) *reinterpret_cast<uint32_t*>(out_row(r1) + d) = pa_pack(o[nd][2] * i1, o[nd][3] * i1);
+        }
+        return;
+    }
+    // partial rows to shared memory (over the key and value tiles), then rank r merges rows r, r + splits, ..
+    static_assert((size_t)PA_BM * D * 4 <= 2 * (size_t)TILE, "the partial rows take the place of the key and value tiles");
+    __syncthreads();
+    float* so = reinterpret_cast<float*>(pa_smem + TILE);            // [64][D]
+    float* sml = reinterpret_cast<float*>(pa_smem);                  // [64] max, [64] sum (over the queries)
+    const uint32_t lr = warp * 16 + quad;
 #pragma unroll
     for (int nd = 0; nd < D / 8; ++nd) {
-        const int d = nd * 8 + 2 * tq;
-        if (qr0 < m) *reinterpret_cast<uint32_t*>(out + ((size_t)qr0 * a.num_heads + h) * D + d) = pa_pack(o[nd][0] * i0, o[nd][1] * i0);
-        if (qr1 < m) *reinterpret_cast<uint32_t*>(out + ((size_t)qr1 * a.num_heads + h) * D + d) = pa_pack(o[nd][2] * i1, o[nd][3] * i1);
+        *reinterpret_cast<float2*>(so + lr * D + nd * 8 + 2 * tq) = make_float2(o[nd][0], o[nd][1]);
+        *reinterpret_cast<float2*>(so + (lr + 8) * D + nd * 8 + 2 * tq) = make_float2(o[nd][2], o[nd][3]);
     }
+    if (tq == 0) {
+        sml[lr] = m0; sml[lr + 8] = m1;
+        sml[64 + lr] = l0; sml[64 + lr + 8] = l1;
+    }
+    pa_cluster_sync();
+    const uint32_t so_addr = sk, ml_addr = sq;
+    for (uint32_t r = rank + splits * warp; r < (uint32_t)PA_BM && row0 + r < rows; r += splits * 4) {
+        float top = -INFINITY;
+        for (uint32_t c = 0; c < splits; ++c) top = fmaxf(top, pa_remote(ml_addr + r * 4, c));
+        const float base = top == -INFINITY ? 0.0f : top;
+        float l = 0.0f, acc[D / 32];
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) acc[i] = 0.0f;
+        for (uint32_t c = 0; c < splits; ++c) {
+            const float w = exp2f(pa_remote(ml_addr + r * 4, c) - base);
+            l += w * pa_remote(ml_addr + (64 + r) * 4, c);
+#pragma unroll
+            for (int i = 0; i < D / 32; ++i) acc[i] += w * pa_remote(so_addr + (r * D + i * 32 + lane) * 4, c);
+        }
+        const float inv = l > 0.0f ? 1.0f / l : 0.0f;
+        __nv_bfloat16* dst = out_row(row0 + r);
+#pragma unroll
+        for (int i = 0; i < D / 32; ++i) dst[i * 32 + lane] = f2bf(acc[i] * inv);
+    }
+    pa_cluster_sync();                                              // no CTA leaves while another may still read its rows
 }
 
-template <int D, int G>
+template <int D>
 static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a) {
-    constexpr size_t smem = (size_t)4 * PA_BN * (D + 8) * sizeof(__nv_bfloat16);
+    constexpr size_t smem = (size_t)3 * PA_BN * (D + 8) * sizeof(__nv_bfloat16);
     static std::atomic<uint64_t> smem_opt_in{0};
-    opt_in_dynamic_smem(cmd, attn_prefill_kernel<D, G>, (int)((int)smem), smem_opt_in);
-    const dim3 grid((a.suffix_length + PA_BM - 1) / PA_BM, a.num_heads / G);
-    attn_prefill_kernel<D, G><<<grid, G * 32, smem, cmd->ctx->stream>>>(a);
-    after_launch(cmd, "attn_prefill_kernel");
+    opt_in_dynamic_smem(cmd, attn_prefill_kernel<D>, (int)smem, smem_opt_in);
+    const uint32_t row_tiles = (a.suffix_length * a.gqa_factor + PA_BM - 1) / PA_BM, kv_heads = a.num_heads / a.gqa_factor;
+    const uint32_t key_tiles = (a.sequence_length + PA_BN - 1) / PA_BN, room = (uint32_t)cmd->ctx->sm_count * (D == 256 ? 2u : 3u);
+    // split the keys while the chip has room for the CTAs and each keeps two tiles or more
+    uint32_t splits = 1;
+    while (splits < 8 && row_tiles * kv_heads * splits * 2 <= room && key_tiles >= splits * 4) splits *= 2;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(row_tiles * splits, kv_heads);
+    cfg.blockDim = dim3(128);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = cmd->ctx->stream;
+    cudaLaunchAttribute attr[1];
+    if (splits > 1) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = splits;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_prefill_kernel<D>, a, splits);
+    if (e != cudaSuccess) cmd->record_error(UZU_ERROR_CUDA, std::string("attn_prefill_kernel: ") + cudaGetErrorString(e));
+    cmd->launches++;
 }
 
-// true = handled. Plain causal / non-causal attention over a dense prefix only; everything else keeps the decode kernel.
+// true = handled: four query tokens and more (fewer keep the split-KV kernel, a CTA per token), dense prefix, plain mask or a causal trie.
 static int g_prefill_attn = -1;   // -1: follow UZU_PREFILL_ATTN, 0 / 1: forced by uzu_debug_set_prefill_attention
 
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a) {
-    static const bool env_enabled = [] { const char* e = getenv("UZU_PREFILL_ATTN"); return !e || atoi(e) != 0; }();   // default on (validated on B200, round 2); =0 keeps the split-KV kernel
+    static const bool env_enabled = [] { const char* e = getenv("UZU_PREFILL_ATTN"); return !e || atoi(e) != 0; }();   // =0 keeps the split-KV kernel
     if (!(g_prefill_attn < 0 ? env_enabled : g_prefill_attn != 0)) return false;
-    if (a.suffix_length < 16 || a.dynamic_position || a.has_sinks || a.is_kv_cache_ring || a.is_trie || a.is_sliding_window) return false;
-    if (a.head_dim != 64 && a.head_dim != 128) return false;
-    const uint32_t g = a.gqa_factor;
-    if ((g != 1 && g != 2 && g != 4 && g != 8) || a.num_heads % g) return false;
+    if (a.suffix_length < 4 || a.dynamic_position || a.has_sinks || a.is_kv_cache_ring || a.is_sliding_window) return false;
+    if (a.is_trie && (!a.is_causal || !a.trie)) return false;
+    if (a.head_dim != 64 && a.head_dim != 128 && a.head_dim != 256) return false;
+    if (a.gqa_factor == 0 || a.num_heads % a.gqa_factor || (uint64_t)a.suffix_length * a.gqa_factor > 0x7fffffffull) return false;
     if ((a.k_head_stride % 8) || (a.v_head_stride % 8) || (a.k_seq_stride % 8) || (a.v_seq_stride % 8)) return false;   // 16-byte cp.async rows
     if ((a.queries | a.keys | a.values | a.out) & 15u) return false;
     if (a.sequence_length < a.suffix_length) return false;
-#define UZU_PA(DD, GG) launch_attn_prefill<DD, GG>(cmd, a); return true
-    if (a.head_dim == 64) {
-        switch (g) { case 1: UZU_PA(64, 1); case 2: UZU_PA(64, 2); case 4: UZU_PA(64, 4); default: UZU_PA(64, 8); }
-    }
-    switch (g) { case 1: UZU_PA(128, 1); case 2: UZU_PA(128, 2); case 4: UZU_PA(128, 4); default: UZU_PA(128, 8); }
-#undef UZU_PA
+    if (a.head_dim == 64) launch_attn_prefill<64>(cmd, a);
+    else if (a.head_dim == 128) launch_attn_prefill<128>(cmd, a);
+    else launch_attn_prefill<256>(cmd, a);
+    return true;
 }
 
 }  // namespace uzu
