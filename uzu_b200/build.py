@@ -27,6 +27,7 @@ SOURCES = {
     "runtime.cu": [],
     "matmul.cu": [],
     "prefill_gemm.cu": [],
+    "qmm_scaled.cu": [],
     "tp.cu": [],
     "attention.cu": ["-fmad=false"],
     "attention_prefill.cu": [],

@@ -106,6 +106,12 @@ inline void launch(uzu_command_buffer* cmd, const char* what, void (*kernel)(KAr
 bool prefill_gemm_applicable(const uzu_matmul_args& a);
 void encode_prefill_gemm(uzu_command_buffer* cmd, const uzu_matmul_args& a);
 
+// quantised products of two and more rows on tcgen05, group scales applied to partial sums (qmm_scaled.cu), dispatched from encode_matmul
+bool qmm_scaled_applicable(const uzu_matmul_args& a);
+void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a);
+// the device's word for barrier waits that ran out in a tensor-memory product (dense_umma.cu; 0 = none)
+unsigned int* umma_error_word();
+
 // whether a dense product runs on the kernel that can norm its A rows as it stages them (dense_linear.cu)
 bool dense_rows_takes_norm(const uzu_dense_linear_args& a);
 // whether a dense product runs on the one-row kernel, which can take a sublayer's result into the residual as it stages its row (dense_linear.cu)

@@ -368,6 +368,12 @@ bool dense_umma_applicable(const uzu_dense_linear_args& a) {
     return true;
 }
 
+unsigned int* umma_error_word() {
+    void* err = nullptr;
+    cudaGetSymbolAddress(&err, g_dense_umma_error);
+    return (unsigned int*)err;
+}
+
 void encode_dense_umma(uzu_command_buffer* cmd, const uzu_dense_linear_args& a) {
     if (!a.a_bf16) {
         const size_t quads = (size_t)a.m * a.k / 4;
@@ -397,9 +403,7 @@ void encode_dense_umma(uzu_command_buffer* cmd, const uzu_dense_linear_args& a) 
     p.k_step = 2;
     // instruction descriptor (kind::f16): f32 accumulate @ 4, bf16 A @ 7, bf16 B @ 10, both K-major, N >> 3 @ [17,23), M >> 4 @ [24,29)
     p.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-    void* err = nullptr;
-    cudaGetSymbolAddress(&err, g_dense_umma_error);
-    p.error = (unsigned int*)err;
+    p.error = umma_error_word();
     constexpr size_t smem = (size_t)DU_STAGES * DU_STAGE_BYTES + 1024;
     auto go = [&](auto kernel, std::atomic<uint64_t>& opt_in) {
         opt_in_dynamic_smem(cmd, kernel, (int)smem, opt_in);

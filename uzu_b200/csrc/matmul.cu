@@ -2025,6 +2025,10 @@ static void launch_generic(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
 
 // returns true when the fused fast path (decode kernel) handled the call; with `fused` set and `dry_run`, only reports applicability
 static bool encode_matmul(uzu_command_buffer* cmd, uzu_context* ctx_for_query, const uzu_matmul_args& a, const uzu_fused_linear_args* fused = nullptr, bool dry_run = false) {
+    if (!fused && !dry_run && cmd && qmm_scaled_applicable(a)) {
+        encode_qmm_scaled(cmd, a);
+        return true;
+    }
     // prefill (m >= 64 tokens): tensor-core GEMM with an in-kernel dequant stage (prefill_gemm.cu)
     if (!fused && !dry_run && cmd && prefill_gemm_applicable(a)) {
         encode_prefill_gemm(cmd, a);

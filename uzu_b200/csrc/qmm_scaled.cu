@@ -1,0 +1,616 @@
+// Quantised MatmulKernel for two and more activation rows on the 5th-generation tensor cores: D[m, n] = epilogue(A[m, k] * dequant(B[n, k])^T).
+// Semantic spec: backends/cpu/kernel/matmul/kernel.rs:164-295 (caller encodable_block/linear/matmul.rs:122-148).
+//
+// Weights are turned in the kernel into TWO bf16 planes, hi = bf16(w) and lo = w - hi. For ZeroPoint / Symmetric weights w = scale * (code - zp) has
+// at most 16 significant bits, so hi + lo is w exactly; for MLX weights (scale * code + bias in f32) the remainder is below 2^-17 |w|. A single
+// rounded plane would put 2^-9 on every weight. The products are exact, the sums f32 in tensor memory.
+//
+// CTA = 128 output features x NT activation rows (the products' M and N), K in blocks of 64; warps:
+//   dequant    two or three groups of four, each takes every second or third block: a thread owns a feature row, turns its 64 codes and stores both
+//              planes to TENSOR MEMORY (tcgen05.st). The weights are the products' A operand there, so that shared memory feeds the activations
+//              only: a product that reads both operands from shared memory is capped at half of the tensor rate, and that was the bound of the
+//              kernel before this one (128 x 128 tiles; 1024 rows x 28672 x 4096 in 579 us).
+//   one warp each: TMA of the codes (128 rows x 128 bytes, 128B swizzle), TMA of the activations (NT rows x 128 k a stage), and the products
+//              (tcgen05.mma, 8 a block). What one lane issues stands behind elect.sync, which the compiler knows: behind `lane == 0` it
+//              wrapped every tcgen05 instruction in a loop over the active lanes, and the product warp was the bound.
+//   epilogue   four: finished tiles from tensor memory (a feature per lane, a row per column) to D; next to the following tile's products where
+//              tensor memory has room for two accumulators (NT <= 128).
+// CTAs stay for several tiles; where the tiles do not fill the chip (few rows, few features) a cluster of up to 8 CTAs shares a tile's k and adds
+// its partial tiles over distributed shared memory in rank order (the same bits every time).
+// (Tried instead: integer codes as one plane, group scales applied to the partial sums as they leave tensor memory. Half the products, but reading
+// 128 x NT partial sums per 64 k costs more than that: 815 us at the size above.)
+//
+// Bounds, per block and CTA: the tensor pipe 2 NT cycles; the dequant warps about 230 instructions each, four warps a block. Prompts are bound by the
+// tensor pipe (half of its rate is the most two planes can give), few rows by the codes' way: HBM, then the dequant warps' issue slots.
+// Every barrier wait is bounded (about a second): a wait that runs out sets the error word and the CTA ends its work.
+#include <cuda.h>
+
+#include <cstdlib>
+#include <type_traits>
+
+#include "common.cuh"
+
+namespace uzu {
+
+struct QsParams {
+    const __nv_bfloat16* scales;
+    const uint8_t* zero_points;      // ScaleZeroPoint
+    const __nv_bfloat16* biases;     // ScaleBias
+    void* d;
+    const __nv_bfloat16* bias;
+    unsigned int* error;
+    uint32_t m, n, k, groups, zp_stride, gshift, xor_mask, method;
+    uint32_t nkb, split_kb, splits, items, m_tiles;
+    uint32_t d_is_f32, accumulate, has_soft_cap;
+    float ab_scale, soft_cap;
+};
+
+namespace {
+
+constexpr uint32_t QS_CODE_TILE = 128 * 128;
+
+template <int NT>
+struct QsShape {
+    static constexpr int DG = NT > 64 ? 2 : 3;                               // dequant groups
+    static constexpr int ND = NT > 128 ? 1 : 2;                              // accumulators in tensor memory
+    static constexpr int AS = 4;                                             // weight blocks in tensor memory: 64 columns each (hi, lo)
+    static constexpr int BS = NT > 192 ? 2 : NT > 64 ? 3 : 4;                // activation stages of 128 k
+    static constexpr int CS = NT > 64 ? 4 : 8;                               // code tiles
+    static constexpr int THREADS = (4 + 4 * DG + 3) * 32;
+    static constexpr uint32_t ACT = NT * 256, A_COL = 256;
+    static constexpr size_t SMEM = (size_t)BS * ACT + (size_t)CS * QS_CODE_TILE + 1024;
+    static_assert(ND * NT <= 256 && AS * 64 <= 256, "tensor memory columns");
+    static_assert((size_t)NT * 512 <= (size_t)BS * ACT + (size_t)CS * QS_CODE_TILE, "the split-k exchange reuses the rings");
+};
+
+__device__ __forceinline__ uint32_t qs_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void qs_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
+__device__ __forceinline__ void qs_arrive(uint32_t bar) { asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void qs_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("{ .reg .b64 st; mbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1; }" ::"r"(bar), "r"(bytes) : "memory");
+}
+// (the thread sleeps in the barrier for up to 20 us a try: spinning warps would take the issue slots of the working ones)
+__device__ __forceinline__ bool qs_try(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000u) : "memory");
+    return ok != 0;
+}
+// false: the phase did not complete within about a second, or another role of the CTA has given up
+__device__ __noinline__ bool qs_wait_long(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up, unsigned int* error, uint32_t code) {
+    uint64_t t0 = 0;
+    for (uint32_t tries = 0; !qs_try(bar, parity); ++tries) {
+        if ((tries & 255u) != 255u) continue;                                // (reading the timer is slow)
+        if (*gave_up) return false;
+        uint64_t t1;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+        if (!t0) t0 = t1;
+        if (t1 - t0 > 1000000000ull) {
+            *gave_up = 1;
+            atomicCAS(error, 0u, code);
+            return false;
+        }
+    }
+    return true;
+}
+// all lanes of a warp wait; the answer is the warp's
+__device__ __forceinline__ bool qs_wait(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up, unsigned int* error, uint32_t code) {
+    if (__all_sync(0xffffffffu, qs_try(bar, parity))) return true;
+    return __all_sync(0xffffffffu, qs_wait_long(bar, parity, gave_up, error, code));
+}
+__device__ __forceinline__ void qs_tma_2d(uint32_t dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ bool qs_elect() {                                 // one lane of a converged warp
+    uint32_t p = 0;
+    asm volatile("{ .reg .pred q; .reg .b32 r; elect.sync r|q, 0xffffffff; @q mov.u32 %0, 1; }" : "+r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ void qs_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void qs_mma(uint32_t d, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }" ::"r"(d), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+                 : "memory");
+}
+__device__ __forceinline__ void qs_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void qs_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void qs_cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void qs_tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                 : "memory");
+}
+__device__ __forceinline__ void qs_tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]),
+          "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ __nv_bfloat162 qs_b2(uint32_t v) { return *reinterpret_cast<__nv_bfloat162*>(&v); }
+__device__ __forceinline__ uint32_t qs_u(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
+
+// d (two exact integers code - zp) -> hi = bf16(s d), lo = s d - hi, exact
+__device__ __forceinline__ void qs_planes(__nv_bfloat162 d, uint32_t s2, uint32_t& hi, uint32_t& lo) {
+    const __nv_bfloat162 h = __hmul2(qs_b2(s2), d);
+    hi = qs_u(h);
+    lo = qs_u(__hfma2(qs_b2(s2), d, __hneg2(h)));
+}
+// 8 four-bit codes (k order: nibble 0 first) -> four words of bf16 pairs per plane; z2 = (128 + zp) twice. Nibbles p and p + 4 of a word are 16 bits
+// apart: one shift and one LOP3 give the pair 128 + e, PRMT puts the pairs back into k order.
+__device__ __forceinline__ void qs_dequant4(uint32_t q, uint32_t z2, uint32_t s2, uint32_t* hi, uint32_t* lo) {
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) qs_planes(__hsub2(qs_b2(((q >> (4 * p)) & 0x000F000Fu) | 0x43004300u), qs_b2(z2)), s2, h[p], l[p]);
+    hi[0] = __byte_perm(h[0], h[1], 0x5410); hi[1] = __byte_perm(h[2], h[3], 0x5410); hi[2] = __byte_perm(h[0], h[1], 0x7632); hi[3] = __byte_perm(h[2], h[3], 0x7632);
+    lo[0] = __byte_perm(l[0], l[1], 0x5410); lo[1] = __byte_perm(l[2], l[3], 0x5410); lo[2] = __byte_perm(l[0], l[1], 0x7632); lo[3] = __byte_perm(l[2], l[3], 0x7632);
+}
+// 4 eight-bit codes -> two words per plane; a code is 16 high + low nibble, and so is its zero point: 16 (h - zh) + (l - zl) is exact (|.| <= 255)
+__device__ __forceinline__ void qs_dequant8(uint32_t q, uint32_t zh2, uint32_t zl2, uint32_t s2, uint32_t* hi, uint32_t* lo) {
+    uint32_t h[2], l[2];                                                     // bytes (0, 2) and (1, 3)
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const __nv_bfloat162 dl = __hsub2(qs_b2(((q >> (8 * p)) & 0x000F000Fu) | 0x43004300u), qs_b2(zl2));
+        const __nv_bfloat162 dh = __hsub2(qs_b2(((q >> (8 * p + 4)) & 0x000F000Fu) | 0x43004300u), qs_b2(zh2));
+        qs_planes(__hfma2(qs_b2(0x41804180u), dh, dl), s2, h[p], l[p]);
+    }
+    hi[0] = __byte_perm(h[0], h[1], 0x5410); hi[1] = __byte_perm(h[0], h[1], 0x7632);
+    lo[0] = __byte_perm(l[0], l[1], 0x5410); lo[1] = __byte_perm(l[0], l[1], 0x7632);
+}
+// MLX: the reference's scale * code + bias in f32, then the two planes
+__device__ __forceinline__ void qs_planes_f32(float w0, float w1, uint32_t& hi, uint32_t& lo) {
+    hi = qs_u(__floats2bfloat162_rn(w0, w1));
+    lo = qs_u(__floats2bfloat162_rn(w0 - __uint_as_float(hi << 16), w1 - __uint_as_float(hi & 0xFFFF0000u)));
+}
+
+}  // namespace
+
+template <int BITS, int NT>
+__global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const QsParams p) {
+    using S = QsShape<NT>;
+    constexpr int DG = S::DG, ND = S::ND, AS = S::AS, BS = S::BS, CS = S::CS, DQ_WARPS = 4 * DG;
+    constexpr uint32_t kpt = BITS == 4 ? 4u : 2u;                            // k blocks per code tile
+    extern __shared__ uint8_t qs_raw[];
+    __shared__ __align__(8) uint64_t bars[2 * CS + 2 * BS + 2 * AS + 2 * ND];
+    __shared__ uint32_t tmem_slot;
+    __shared__ volatile uint32_t gave_up;
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;     // (known to be uniform)
+    const uint32_t base = (qs_smem(qs_raw) + 1023u) & ~1023u;            // swizzle atoms sit on 1024-byte boundaries
+    const uint32_t act0 = base, code0 = base + BS * S::ACT, bar0 = qs_smem(bars);
+    auto code_full = [&](uint32_t i) { return bar0 + 8u * i; };
+    auto code_empty = [&](uint32_t i) { return bar0 + 8u * (CS + i); };
+    auto act_full = [&](uint32_t i) { return bar0 + 8u * (2 * CS + i); };
+    auto act_empty = [&](uint32_t i) { return bar0 + 8u * (2 * CS + BS + i); };
+    auto a_full = [&](uint32_t i) { return bar0 + 8u * (2 * CS + 2 * BS + i); };
+    auto a_empty = [&](uint32_t i) { return bar0 + 8u * (2 * CS + 2 * BS + AS + i); };
+    auto d_full = [&](uint32_t i) { return bar0 + 8u * (2 * CS + 2 * BS + 2 * AS + i); };
+    auto d_empty = [&](uint32_t i) { return bar0 + 8u * (2 * CS + 2 * BS + 2 * AS + ND + i); };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            for (int i = 0; i < CS; ++i) { qs_init(code_full(i), 1); qs_init(code_empty(i), DQ_WARPS); }
+            for (int i = 0; i < BS; ++i) { qs_init(act_full(i), 1); qs_init(act_empty(i), 1); }
+            for (int i = 0; i < AS; ++i) { qs_init(a_full(i), 4); qs_init(a_empty(i), 1); }
+            for (int i = 0; i < ND; ++i) { qs_init(d_full(i), 1); qs_init(d_empty(i), 4); }
+            gave_up = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        __syncwarp();
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(qs_smem(&tmem_slot)), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    pdl_launch_dependents();
+    qs_fence_before();
+    __syncthreads();
+    qs_fence_after();
+    const uint32_t tmem = tmem_slot;
+
+    // this CTA's work: items blockIdx.x / splits, then in steps of the grid; the k blocks of its rank
+    const uint32_t rank = p.splits > 1 ? blockIdx.x % p.splits : 0u, item0 = blockIdx.x / p.splits, item_step = gridDim.x / p.splits;
+    const uint32_t kb0 = rank * p.split_kb, nk = min(p.split_kb, p.nkb - kb0);       // (every rank has some)
+    const uint32_t tiles = (nk + kpt - 1) / kpt;                                     // code tiles per item
+    // neighbouring items share their weights: the row tiles of a feature tile are in flight together
+    auto item_n = [&](uint32_t item) { return item / p.m_tiles * 128u; };
+    auto item_m = [&](uint32_t item) { return item % p.m_tiles * (uint32_t)NT; };
+
+    if (warp < 4) {
+        // ================================ finished tiles ================================
+        uint32_t buf = 0, ph = 0;
+        pdl_wait();                                                      // D may be read (accumulate) and is written below
+        for (uint32_t item = item0; item < p.items; item += item_step) {
+            const uint32_t f = warp * 32u + lane, row = item_n(item) + f, t0 = item_m(item);
+            auto finish = [&](float sum, uint32_t token) {
+                if (token >= p.m || row >= p.n) return;
+                const size_t at = (size_t)token * p.n + row;
+                float val = __fmul_rn(p.ab_scale, sum);                  // separate roundings, like the reference
+                if (p.accumulate) val = __fadd_rn(val, p.d_is_f32 ? reinterpret_cast<const float*>(p.d)[at] : bf2f(reinterpret_cast<const __nv_bfloat16*>(p.d)[at]));
+                if (p.bias) val = __fadd_rn(val, bf2f(p.bias[row]));
+                if (p.has_soft_cap) val = __fmul_rn(p.soft_cap, tanhf(__fdiv_rn(val, p.soft_cap)));
+                if (p.d_is_f32) reinterpret_cast<float*>(p.d)[at] = val;
+                else reinterpret_cast<__nv_bfloat16*>(p.d)[at] = f2bf(val);
+            };
+            const bool ok = qs_wait(d_full(buf), ph, &gave_up, p.error, 0x101u);
+            qs_fence_after();
+            const uint32_t taddr = tmem + ((warp * 32u) << 16) + buf * NT, columns = min((uint32_t)NT, p.m - t0);
+            if (p.splits == 1) {
+                for (uint32_t c0 = 0; c0 < columns && ok; c0 += 16) {
+                    uint32_t v[16];
+                    qs_tmem_ld16(taddr + c0, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) finish(__uint_as_float(v[j]), t0 + c0 + j);
+                }
+                qs_fence_before();
+                __syncwarp();
+                if (lane == 0) qs_arrive(d_empty(buf));
+                if (!ok) break;
+                if (++buf == (uint32_t)ND) { buf = 0; ph ^= 1u; }
+            } else {
+                // this CTA's tile to shared memory (the rings are idle: every block has been consumed), then column shares over the cluster
+                for (uint32_t c0 = 0; c0 < columns && ok; c0 += 16) {
+                    uint32_t v[16];
+                    qs_tmem_ld16(taddr + c0, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + ((c0 + j) * 128u + f) * 4u), "r"(v[j]) : "memory");
+                }
+                qs_cluster_sync();
+                for (uint32_t j = rank; j < columns && ok; j += p.splits) {
+                    float part[8];
+#pragma unroll
+                    for (uint32_t q = 0; q < 8; ++q) {
+                        uint32_t remote;
+                        part[q] = 0.0f;
+                        if (q >= p.splits) continue;
+                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(base + (j * 128u + f) * 4u), "r"(q));
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part[q]) : "r"(remote) : "memory");
+                    }
+                    float sum = part[0];
+#pragma unroll
+                    for (int q = 1; q < 8; ++q) sum += part[q];
+                    finish(sum, t0 + j);
+                }
+                break;                                                   // (one item per cluster)
+            }
+        }
+    } else if (warp < (uint32_t)(4 + DQ_WARPS)) {
+        // ================================ codes -> two bf16 planes in tensor memory ================================
+        const uint32_t dg = (warp - 4) >> 2, lw = warp & 3u, r = lw * 32u + lane;
+        const bool mlx = p.method == UZU_QMETHOD_SCALE_BIAS, has_zp = p.method == UZU_QMETHOD_SCALE_ZERO_POINT, halves = p.gshift == 5u;
+        uint32_t turn = 0, stage = dg, a_ph = 1, slot = 0, c_ph = 0;     // whose block it is; this group's next weight block; code tile
+        bool ok = true;
+        for (uint32_t item = item0; item < p.items && ok; item += item_step) {
+            const uint32_t brow = min(item_n(item) + r, p.n - 1u);
+            const uint16_t* srow = reinterpret_cast<const uint16_t*>(p.scales) + (size_t)brow * p.groups;
+            const uint16_t* crow = reinterpret_cast<const uint16_t*>(p.biases) + (size_t)brow * p.groups;
+            const uint8_t* zrow = p.zero_points + (size_t)brow * p.zp_stride;
+            // scale | (zero point or bias) << 16 of a half block, requested a turn ahead
+            auto factor = [&](uint32_t k) -> uint32_t {
+                const uint32_t g = min(k >> p.gshift, p.groups - 1u);
+                uint32_t c = BITS == 4 ? 8u : 128u;
+                if (mlx) c = crow[g];
+                else if (has_zp) c = BITS == 4 ? (uint32_t)(zrow[g >> 1] >> (4u * (g & 1u))) & 15u : (uint32_t)zrow[g];
+                return (uint32_t)srow[g] | c << 16;
+            };
+            auto first_block = [&]() -> uint32_t { return (dg + DG - turn) % DG; };      // blocks until this group's turn
+            uint32_t f_next[2];
+            {
+                const uint32_t k0 = (kb0 + first_block()) * 64u;
+                f_next[0] = factor(k0);
+                f_next[1] = halves ? factor(k0 + 32u) : f_next[0];
+            }
+            for (uint32_t tile = 0, kb = 0; tile < tiles; ++tile) {
+                ok = qs_wait(code_full(slot), c_ph, &gave_up, p.error, 0x102u);
+                if (!ok) break;
+                const uint32_t line = code0 + slot * QS_CODE_TILE + r * 128u, blocks = min(kpt, nk - kb);
+#pragma unroll 1
+                for (uint32_t j = 0; j < blocks; ++j, ++kb) {
+                    const bool mine = turn == dg;
+                    if (++turn == (uint32_t)DG) turn = 0;
+                    if (!mine) continue;
+                    const uint32_t f_cur[2] = {f_next[0], f_next[1]};
+                    {
+                        const uint32_t k0 = (kb0 + kb + DG) * 64u;
+                        f_next[0] = factor(k0);
+                        f_next[1] = halves ? factor(k0 + 32u) : f_next[0];
+                    }
+                    const uint32_t t_col = tmem + ((lw * 32u) << 16) + S::A_COL + stage * 64u;
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; ++h) {                   // 32 k at a time
+                        uint32_t hi[16], lo[16];
+                        const uint32_t s1 = f_cur[h] & 0xFFFFu, z = f_cur[h] >> 16, s2 = s1 * 0x00010001u;
+                        if constexpr (BITS == 4) {
+                            uint32_t q[4];
+                            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(line + (((j * 2 + h) ^ (r & 7u)) << 4)));
+                            if (!mlx) {
+                                const uint32_t z2 = (0x4300u | z) * 0x00010001u;      // bf16 128 + zp
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) qs_dequant4(q[i] ^ p.xor_mask, z2, s2, hi + 4 * i, lo + 4 * i);
+                            } else {
+                                const float s = __uint_as_float(s1 << 16), c = __uint_as_float(z << 16);
+#pragma unroll
+                                for (int i = 0; i < 16; ++i) {           // pair i: nibbles 2 (i & 3), + 1 of word i / 4
+                                    const uint32_t w = (q[i >> 2] ^ p.xor_mask) >> (8 * (i & 3));
+                                    qs_planes_f32(fmaf(s, (float)(w & 15u), c), fmaf(s, (float)((w >> 4) & 15u), c), hi[i], lo[i]);
+                                }
+                            }
+                        } else {
+#pragma unroll
+                            for (uint32_t i2 = 0; i2 < 2; ++i2) {
+                                uint32_t q[4];
+                                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(line + (((j * 4 + h * 2 + i2) ^ (r & 7u)) << 4)));
+                                if (!mlx) {
+                                    const uint32_t zh2 = (0x4300u | (z >> 4)) * 0x00010001u, zl2 = (0x4300u | (z & 15u)) * 0x00010001u;
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) qs_dequant8(q[i] ^ p.xor_mask, zh2, zl2, s2, hi + 8 * i2 + 2 * i, lo + 8 * i2 + 2 * i);
+                                } else {
+                                    const float s = __uint_as_float(s1 << 16), c = __uint_as_float(z << 16);
+#pragma unroll
+                                    for (int i = 0; i < 8; ++i) {
+                                        const uint32_t w = (q[i >> 1] ^ p.xor_mask) >> (16 * (i & 1));
+                                        qs_planes_f32(fmaf(s, (float)(w & 255u), c), fmaf(s, (float)((w >> 8) & 255u), c), hi[8 * i2 + i], lo[8 * i2 + i]);
+                                    }
+                                }
+                            }
+                        }
+                        if (h == 0) {
+                            ok = qs_wait(a_empty(stage), a_ph, &gave_up, p.error, 0x103u);
+                            if (!ok) break;
+                            qs_fence_after();
+                        }
+                        qs_tmem_st16(t_col + h * 16u, hi);
+                        qs_tmem_st16(t_col + 32u + h * 16u, lo);
+                    }
+                    if (!ok) break;
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    qs_fence_before();
+                    __syncwarp();
+                    if (lane == 0) qs_arrive(a_full(stage));
+                    stage += DG;
+                    if (stage >= (uint32_t)AS) { stage -= AS; a_ph ^= 1u; }
+                }
+                if (!ok) break;
+                __syncwarp();
+                if (lane == 0) qs_arrive(code_empty(slot));
+                if (++slot == (uint32_t)CS) { slot = 0; c_ph ^= 1u; }
+            }
+        }
+        if (p.splits > 1) qs_cluster_sync();
+    } else {
+        const uint32_t role = warp - (4 + DQ_WARPS);
+        bool ok = true;
+        if (role == 0) {
+            // ================================ codes by TMA (they depend on no kernel) ================================
+            uint32_t slot = 0, ph = 1;
+            for (uint32_t item = item0; item < p.items && ok; item += item_step) {
+                const uint32_t y = item_n(item), x0 = kb0 / kpt * 128u;
+                for (uint32_t tile = 0; tile < tiles; ++tile) {
+                    ok = qs_wait(code_empty(slot), ph, &gave_up, p.error, 0x104u);
+                    if (!ok) break;
+                    if (qs_elect()) {
+                        qs_expect(code_full(slot), QS_CODE_TILE);
+                        qs_tma_2d(code0 + slot * QS_CODE_TILE, &map_w, x0 + tile * 128u, y, code_full(slot));
+                    }
+                    __syncwarp();
+                    if (++slot == (uint32_t)CS) { slot = 0; ph ^= 1u; }
+                }
+            }
+        } else if (role == 1) {
+            // ================================ activations by TMA, 128 k a stage ================================
+            uint32_t slot = 0, ph = 1;
+            pdl_wait();
+            for (uint32_t item = item0; item < p.items && ok; item += item_step) {
+                const uint32_t y = item_m(item);
+                for (uint32_t i = 0; i < nk; i += 2) {
+                    ok = qs_wait(act_empty(slot), ph, &gave_up, p.error, 0x105u);
+                    if (!ok) break;
+                    if (qs_elect()) {                                    // (a half stage behind the last k reads zeros)
+                        qs_expect(act_full(slot), S::ACT);
+                        qs_tma_2d(act0 + slot * S::ACT, &map_x, (kb0 + i) * 64u, y, act_full(slot));
+                        qs_tma_2d(act0 + slot * S::ACT + S::ACT / 2, &map_x, (kb0 + i + 1) * 64u, y, act_full(slot));
+                    }
+                    __syncwarp();
+                    if (++slot == (uint32_t)BS) { slot = 0; ph ^= 1u; }
+                }
+            }
+        } else {
+            // ================================ products ================================
+            // shared-memory descriptor: K-major SWIZZLE_128B, 1024 bytes between 8-row groups, +32 bytes per 16 k
+            constexpr uint64_t desc_hi = (uint64_t)((1024u >> 4) | (1u << 14) | (2u << 29)) << 32;
+            constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(NT >> 3) << 17) | ((128u >> 4) << 24);
+            const uint32_t desc_lo = (act0 >> 4) | (1u << 16);
+            uint32_t bs = 0, bs_ph = 0, as = 0, as_ph = 0, buf = 0, d_ph = 1;
+            for (uint32_t item = item0; item < p.items && ok; item += item_step) {
+                ok = qs_wait(d_empty(buf), d_ph, &gave_up, p.error, 0x108u);
+                const uint32_t d = tmem + buf * NT;
+                for (uint32_t i = 0; i < nk && ok; i += 2) {
+                    ok = qs_wait(act_full(bs), bs_ph, &gave_up, p.error, 0x106u);
+                    if (!ok) break;
+#pragma unroll
+                    for (uint32_t half = 0; half < 2; ++half) {
+                        if (i + half >= nk) continue;
+                        ok = qs_wait(a_full(as), as_ph, &gave_up, p.error, 0x107u);
+                        if (!ok) break;
+                        qs_fence_after();
+                        if (qs_elect()) {
+                            const uint32_t a_col = tmem + S::A_COL + as * 64u, lo = desc_lo + (bs * S::ACT + half * (S::ACT / 2) >> 4);
+#pragma unroll
+                            for (uint32_t kk = 0; kk < 4; ++kk) {
+                                qs_mma(d, a_col + kk * 8u, desc_hi | (lo + kk * 2u), idesc, (i | half | kk) != 0 ? 1u : 0u);
+                                qs_mma(d, a_col + 32u + kk * 8u, desc_hi | (lo + kk * 2u), idesc, 1u);
+                            }
+                            qs_commit(a_empty(as));
+                        }
+                        __syncwarp();
+                        if (++as == (uint32_t)AS) { as = 0; as_ph ^= 1u; }
+                    }
+                    if (!ok) break;
+                    if (qs_elect()) qs_commit(act_empty(bs));
+                    __syncwarp();
+                    if (++bs == (uint32_t)BS) { bs = 0; bs_ph ^= 1u; }
+                }
+                if (!ok) break;
+                if (qs_elect()) qs_commit(d_full(buf));
+                __syncwarp();
+                if (++buf == (uint32_t)ND) { buf = 0; d_ph ^= 1u; }
+            }
+        }
+        __syncwarp();
+        if (p.splits > 1) qs_cluster_sync();
+    }
+    // no CTA of a cluster leaves while another may still read its tile
+    if (p.splits > 1) qs_cluster_sync();
+    qs_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+        qs_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    }
+}
+
+// ---- host side -------------------------------------------------------------------------------------------------------------------------
+static decltype(&cuTensorMapEncodeTiled) tensor_map_encoder() {
+    static decltype(&cuTensorMapEncodeTiled) fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) f = nullptr;
+        cudaGetLastError();
+        return (decltype(&cuTensorMapEncodeTiled))f;
+    }();
+    return fn;
+}
+static bool tensor_map(CUtensorMap* map, CUtensorMapDataType type, uint64_t addr, uint64_t inner, uint64_t outer, uint64_t pitch, uint32_t box_inner, uint32_t box_outer) {
+    const cuuint64_t dims[2] = {inner, outer}, strides[1] = {pitch};
+    const cuuint32_t box[2] = {box_inner, box_outer}, steps[2] = {1, 1};
+    return tensor_map_encoder()(map, type, 2, (void*)addr, dims, strides, box, steps, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+bool qmm_scaled_applicable(const uzu_matmul_args& a) {
+    static const bool off = [] { const char* e = getenv("UZU_QMM_SCALED"); return e && atoi(e) == 0; }();      // 0: the kernels for other shapes (A/B runs)
+    if (off || a.m < 2) return false;
+    if (a.b_prologue == UZU_B_FULL_PRECISION || a.gather_indices || !a.b_transpose) return false;
+    if (a.input_dt != UZU_DT_BF16 || a.weights_dt != UZU_DT_BF16) return false;
+    if (a.output_dt != UZU_DT_BF16 && a.output_dt != UZU_DT_F32) return false;
+    if (a.b_mode != UZU_QMODE_U4 && a.b_mode != UZU_QMODE_U8) return false;
+    const uint32_t gs = a.b_group_size;
+    if (a.k == 0 || a.k > (1u << 18) || a.n == 0 || a.k % 64u != 0 || gs < 32 || (gs & (gs - 1)) != 0 || a.k % gs != 0) return false;
+    if ((a.a & 15u) || (a.b & 15u)) return false;            // TMA operands (their pitches are multiples of 32 bytes with k a multiple of 64)
+    // 17 .. 63 rows over a matrix of at most 2^21 weights (about a megabyte, it stays in L2): launches of 16 rows as before (matmul.cu)
+    if (a.m > 16 && a.m < 64 && (uint64_t)a.n * a.k <= (1u << 21)) return false;
+    return tensor_map_encoder() != nullptr;
+}
+
+namespace {
+
+struct QsPlan { int nt = 0; uint32_t splits = 1; float cost = 1e30f; };
+
+// Cycles of one CTA per 64 k of a tile: two planes of products take 2 NT of the tensor pipe; a dequant group's block takes `turn`, and the groups
+// work side by side.
+float qs_block_cycles(int nt, uint32_t bits, bool mlx) {
+    const float turn = mlx ? 1500.0f : bits == 4 ? 700.0f : 900.0f;
+    return std::max(2.0f * nt, turn / (nt > 64 ? 2.0f : 3.0f));
+}
+
+// Rows per tile and CTAs per tile: the shortest estimated time over the chip. A wider tile turns its codes once for more rows; a narrower one or a
+// split k fills the chip where tiles are few. Fixed cost per item: filling the pipeline and storing the tile.
+QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, uint32_t sms) {
+    QsPlan best;
+    const uint32_t n_tiles = (n + 127u) / 128u;
+    for (int nt : {16, 32, 64, 128, 192, 256}) {
+        if (nt > 16 && m <= (uint32_t)nt / 2) break;
+        if (nt < 128 && m > 2u * nt) continue;
+        const uint32_t tiles = n_tiles * ((m + nt - 1) / nt);
+        for (uint32_t splits = 1; splits <= 8; splits *= 2) {
+            const uint32_t per = ((nkb + splits - 1) / splits + 3u) & ~3u;           // whole code tiles per rank
+            if (splits > 1 && (per * (splits - 1) >= nkb || tiles * splits > sms)) break;
+            const float item = (float)std::min(per, nkb) * qs_block_cycles(nt, bits, mlx) + (nt > 128 ? 2000.0f + 10.0f * nt : 1500.0f) + (splits > 1 ? 1500.0f + 8.0f * nt : 0.0f);
+            const uint32_t waves = (tiles * splits + sms - 1) / sms;
+            const float cost = waves * item;
+            if (cost < best.cost) best = {nt, splits, cost};
+        }
+    }
+    return best;
+}
+
+template <int BITS, int NT>
+void qs_launch(uzu_command_buffer* cmd, const CUtensorMap& w, const CUtensorMap& x, const QsParams& p, uint32_t grid) {
+    static std::atomic<uint64_t> smem_opt_in{0};
+    opt_in_dynamic_smem(cmd, qmm_scaled_kernel<BITS, NT>, (int)QsShape<NT>::SMEM, smem_opt_in);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(QsShape<NT>::THREADS);
+    cfg.dynamicSmemBytes = QsShape<NT>::SMEM;
+    cfg.stream = cmd->ctx->stream;
+    cudaLaunchAttribute attr[2];
+    if (cmd->use_pdl) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.splits > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = p.splits;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, qmm_scaled_kernel<BITS, NT>, w, x, p);
+    if (e != cudaSuccess) cmd->record_error(UZU_ERROR_CUDA, std::string("matmul qmm_scaled_kernel: ") + cudaGetErrorString(e));
+    cmd->launches++;
+}
+
+}  // namespace
+
+void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
+    QsParams p{};
+    const uint32_t bits = a.b_mode == UZU_QMODE_U4 ? 4 : 8;
+    p.scales = (const __nv_bfloat16*)a.b_scales;
+    p.method = a.b_prologue == UZU_B_SCALE_BIAS_DEQUANT ? UZU_QMETHOD_SCALE_BIAS
+               : a.b_prologue == UZU_B_SCALE_ZERO_POINT_DEQUANT ? UZU_QMETHOD_SCALE_ZERO_POINT : UZU_QMETHOD_SCALE_SYMMETRIC;
+    p.zero_points = (const uint8_t*)a.b_zero_points;
+    p.biases = p.method == UZU_QMETHOD_SCALE_BIAS ? (const __nv_bfloat16*)a.b_biases : nullptr;
+    p.bias = ((a.d_transform & UZU_D_BIAS) && a.bias) ? (const __nv_bfloat16*)a.bias : nullptr;
+    p.n = a.n; p.k = a.k;
+    p.groups = a.k / a.b_group_size;
+    p.zp_stride = bits == 4 ? (p.groups + 1) / 2 : p.groups;
+    while ((1u << p.gshift) < a.b_group_size) ++p.gshift;
+    p.xor_mask = a.b_signed_codes ? (bits == 4 ? 0x88888888u : 0x80808080u) : 0u;
+    p.nkb = a.k / 64u;
+    p.d_is_f32 = a.output_dt == UZU_DT_F32;
+    p.accumulate = (a.d_transform & UZU_D_ACCUMULATE) != 0;
+    p.has_soft_cap = (a.d_transform & UZU_D_SOFT_CAP) != 0;
+    p.ab_scale = (a.d_transform & UZU_D_SCALE) ? a.ab_scale : 1.0f;
+    p.soft_cap = a.soft_cap;
+    p.error = umma_error_word();
+    p.m = a.m;
+    p.d = (void*)a.d;
+    uzu_context* ctx = cmd->ctx;
+    const QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, (uint32_t)ctx->sm_count);
+    p.splits = plan.splits;
+    p.split_kb = p.splits == 1 ? p.nkb : ((p.nkb + p.splits - 1) / p.splits + 3u) & ~3u;
+    p.m_tiles = (p.m + plan.nt - 1) / plan.nt;
+    p.items = p.m_tiles * ((a.n + 127u) / 128u);
+    CUtensorMap mw, mx;
+    if (!tensor_map(&mw, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.b, (uint64_t)a.k * bits / 8, a.n, (uint64_t)a.k * bits / 8, 128, 128) ||
+        !tensor_map(&mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, a.a, a.k, p.m, (uint64_t)a.k * 2, 64, (uint32_t)plan.nt)) {
+        cmd->record_error(UZU_ERROR_CUDA, "matmul: cuTensorMapEncodeTiled failed");
+        return;
+    }
+    const uint32_t grid = p.splits > 1 ? p.items * p.splits : std::min(p.items, (uint32_t)ctx->sm_count);
+    auto go = [&](auto bits_c) {
+        constexpr int BITS = decltype(bits_c)::value;
+        switch (plan.nt) {
+            case 16: qs_launch<BITS, 16>(cmd, mw, mx, p, grid); break;
+            case 32: qs_launch<BITS, 32>(cmd, mw, mx, p, grid); break;
+            case 64: qs_launch<BITS, 64>(cmd, mw, mx, p, grid); break;
+            case 128: qs_launch<BITS, 128>(cmd, mw, mx, p, grid); break;
+            case 192: qs_launch<BITS, 192>(cmd, mw, mx, p, grid); break;
+            default: qs_launch<BITS, 256>(cmd, mw, mx, p, grid); break;
+        }
+    };
+    if (bits == 4) go(std::integral_constant<int, 4>{});
+    else go(std::integral_constant<int, 8>{});
+}
+
+}  // namespace uzu
