@@ -61,7 +61,7 @@ def test_prefill_attention_token_major_cache_matches_decode_kernel(prefill_attn)
     assert_bf16_close(got, O.attention_single_pass(q, k, v, **kw), max_ulp=1, min_exact=0.95, what="vs oracle")
 
 
-@pytest.mark.parametrize("H,Hkv,prefix,suffix,D", [(8, 2, 0, 64, 256), (8, 2, 700, 33, 256), (3, 1, 130, 21, 64), (12, 2, 65, 5, 128), (32, 8, 1500, 16, 128), (4, 4, 63, 4, 256), (2, 1, 0, 31, 64)])
+@pytest.mark.parametrize("H,Hkv,prefix,suffix,D", [(8, 2, 0, 64, 256), (8, 2, 700, 33, 256), (3, 1, 130, 21, 64), (12, 2, 65, 9, 128), (32, 8, 1500, 16, 128), (4, 4, 63, 8, 256), (2, 1, 0, 31, 64)])
 @pytest.mark.parametrize("trie", [False, True])
 def test_rows_of_grouped_heads(ctx, H, Hkv, prefix, suffix, D, trie):
     """Rows of (token, head) pairs: tiles that end inside a token's heads, head counts that do not divide a tile, 256 channels, few rows over

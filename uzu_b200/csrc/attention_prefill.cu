@@ -310,13 +310,13 @@ static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_arg
     cmd->launches++;
 }
 
-// true = handled: four query tokens and more (fewer keep the split-KV kernel, a CTA per token), dense prefix, plain mask or a causal trie.
+// true = handled: eight query tokens and more (fewer keep the split-KV kernel, a CTA per token and split, which fills the chip as well), dense prefix, plain mask or a causal trie.
 static int g_prefill_attn = -1;   // -1: follow UZU_PREFILL_ATTN, 0 / 1: forced by uzu_debug_set_prefill_attention
 
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a) {
     static const bool env_enabled = [] { const char* e = getenv("UZU_PREFILL_ATTN"); return !e || atoi(e) != 0; }();   // =0 keeps the split-KV kernel
     if (!(g_prefill_attn < 0 ? env_enabled : g_prefill_attn != 0)) return false;
-    if (a.suffix_length < 4 || a.dynamic_position || a.has_sinks || a.is_kv_cache_ring || a.is_sliding_window) return false;
+    if (a.suffix_length < 8 || a.dynamic_position || a.has_sinks || a.is_kv_cache_ring || a.is_sliding_window) return false;
     if (a.is_trie && (!a.is_causal || !a.trie)) return false;
     if (a.head_dim != 64 && a.head_dim != 128 && a.head_dim != 256) return false;
     if (a.gqa_factor == 0 || a.num_heads % a.gqa_factor || (uint64_t)a.suffix_length * a.gqa_factor > 0x7fffffffull) return false;

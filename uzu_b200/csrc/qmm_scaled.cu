@@ -6,21 +6,21 @@
 // rounded plane would put 2^-9 on every weight. The products are exact, the sums f32 in tensor memory.
 //
 // CTA = 128 output features x NT activation rows (the products' M and N), K in blocks of 64; warps:
-//   dequant    two or three groups of four, each takes every second or third block: a thread owns a feature row, turns its 64 codes and stores both
+//   dequant    three or four groups of four, each takes every third or fourth block: a thread owns a feature row, turns its 64 codes and stores both
 //              planes to TENSOR MEMORY (tcgen05.st). The weights are the products' A operand there, so that shared memory feeds the activations
 //              only: a product that reads both operands from shared memory is capped at half of the tensor rate, and that was the bound of the
 //              kernel before this one (128 x 128 tiles; 1024 rows x 28672 x 4096 in 579 us).
 //   one warp each: TMA of the codes (128 rows x 128 bytes, 128B swizzle), TMA of the activations (NT rows x 128 k a stage), and the products
 //              (tcgen05.mma, 8 a block). What one lane issues stands behind elect.sync, which the compiler knows: behind `lane == 0` it
 //              wrapped every tcgen05 instruction in a loop over the active lanes, and the product warp was the bound.
-//   epilogue   four: finished tiles from tensor memory (a feature per lane, a row per column) to D; next to the following tile's products where
-//              tensor memory has room for two accumulators (NT <= 128).
+//   epilogue   four: finished tiles from tensor memory (a feature per lane, a row per column) to D; next to the following tile's products for NT <= 64
+//              (two accumulators).
 // CTAs stay for several tiles; where the tiles do not fill the chip (few rows, few features) a cluster of up to 8 CTAs shares a tile's k and adds
 // its partial tiles over distributed shared memory in rank order (the same bits every time).
 // (Tried instead: integer codes as one plane, group scales applied to the partial sums as they leave tensor memory. Half the products, but reading
 // 128 x NT partial sums per 64 k costs more than that: 815 us at the size above.)
 //
-// Bounds, per block and CTA: the tensor pipe 2 NT cycles; the dequant warps about 230 instructions each, four warps a block. Prompts are bound by the
+// Bounds, per block and CTA: the tensor pipe 4 NT cycles; the dequant warps about 230 instructions each, four warps a block. Prompts are bound by the
 // tensor pipe (half of its rate is the most two planes can give), few rows by the codes' way: HBM, then the dequant warps' issue slots.
 // Every barrier wait is bounded (about a second): a wait that runs out sets the error word and the CTA ends its work.
 #include <cuda.h>
@@ -41,7 +41,7 @@ struct QsParams {
     unsigned int* error;
     uint32_t m, n, k, groups, zp_stride, gshift, xor_mask, method;
     uint32_t nkb, split_kb, splits, items, m_tiles;
-    uint32_t d_is_f32, accumulate, has_soft_cap;
+    uint32_t d_is_f32, accumulate, has_soft_cap, plain;
     float ab_scale, soft_cap;
 };
 
@@ -51,15 +51,15 @@ constexpr uint32_t QS_CODE_TILE = 128 * 128;
 
 template <int NT>
 struct QsShape {
-    static constexpr int DG = NT > 64 ? 2 : 3;                               // dequant groups
-    static constexpr int ND = NT > 128 ? 1 : 2;                              // accumulators in tensor memory
-    static constexpr int AS = 4;                                             // weight blocks in tensor memory: 64 columns each (hi, lo)
+    static constexpr int DG = NT > 128 ? 3 : 4;                              // dequant groups: a block takes one about 2000 cycles, hardly a third of them issuing
+    static constexpr int ND = NT > 64 ? 1 : 2;                               // accumulators in tensor memory
+    static constexpr int AS = NT > 192 ? 4 : NT > 128 ? 5 : 6;               // weight blocks in tensor memory: 64 columns each (hi, lo)
     static constexpr int BS = NT > 192 ? 2 : NT > 64 ? 3 : 4;                // activation stages of 128 k
     static constexpr int CS = NT > 64 ? 4 : 8;                               // code tiles
     static constexpr int THREADS = (4 + 4 * DG + 3) * 32;
-    static constexpr uint32_t ACT = NT * 256, A_COL = 256;
+    static constexpr uint32_t ACT = NT * 256, A_COL = 512 - 64 * AS;
     static constexpr size_t SMEM = (size_t)BS * ACT + (size_t)CS * QS_CODE_TILE + 1024;
-    static_assert(ND * NT <= 256 && AS * 64 <= 256, "tensor memory columns");
+    static_assert(ND * NT <= (int)A_COL && DG < AS, "tensor memory columns; a group never waits for its own block");
     static_assert((size_t)NT * 512 <= (size_t)BS * ACT + (size_t)CS * QS_CODE_TILE, "the split-k exchange reuses the rings");
 };
 
@@ -235,18 +235,30 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
             const bool ok = qs_wait(d_full(buf), ph, &gave_up, p.error, 0x101u);
             qs_fence_after();
             const uint32_t taddr = tmem + ((warp * 32u) << 16) + buf * NT, columns = min((uint32_t)NT, p.m - t0);
-            if (p.splits == 1) {
+            if (p.splits == 1 && p.plain && item_n(item) + 128u <= p.n) {
+                // D is the rounded sum: a store per column (64 neighbouring bytes a warp), no more than an address step between them
+                __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.d) + (size_t)t0 * p.n + row;
+                uint32_t c0 = 0;
+                for (; c0 + 16 <= columns && ok; c0 += 16) {
+                    uint32_t v[16];
+                    qs_tmem_ld16(taddr + c0, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j, out += p.n) *out = f2bf(__uint_as_float(v[j]));
+                }
+                if (c0 < columns && ok) {
+                    uint32_t v[16];
+                    qs_tmem_ld16(taddr + c0, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j, out += p.n)
+                        if (c0 + j < columns) *out = f2bf(__uint_as_float(v[j]));
+                }
+            } else if (p.splits == 1) {
                 for (uint32_t c0 = 0; c0 < columns && ok; c0 += 16) {
                     uint32_t v[16];
                     qs_tmem_ld16(taddr + c0, v);
 #pragma unroll
                     for (int j = 0; j < 16; ++j) finish(__uint_as_float(v[j]), t0 + c0 + j);
                 }
-                qs_fence_before();
-                __syncwarp();
-                if (lane == 0) qs_arrive(d_empty(buf));
-                if (!ok) break;
-                if (++buf == (uint32_t)ND) { buf = 0; ph ^= 1u; }
             } else {
                 // this CTA's tile to shared memory (the rings are idle: every block has been consumed), then column shares over the cluster
                 for (uint32_t c0 = 0; c0 < columns && ok; c0 += 16) {
@@ -273,6 +285,11 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
                 }
                 break;                                                   // (one item per cluster)
             }
+            qs_fence_before();
+            __syncwarp();
+            if (lane == 0) qs_arrive(d_empty(buf));
+            if (!ok) break;
+            if (++buf == (uint32_t)ND) { buf = 0; ph ^= 1u; }
         }
     } else if (warp < (uint32_t)(4 + DQ_WARPS)) {
         // ================================ codes -> two bf16 planes in tensor memory ================================
@@ -497,6 +514,10 @@ bool qmm_scaled_applicable(const uzu_matmul_args& a) {
     const uint32_t gs = a.b_group_size;
     if (a.k == 0 || a.k > (1u << 18) || a.n == 0 || a.k % 64u != 0 || gs < 32 || (gs & (gs - 1)) != 0 || a.k % gs != 0) return false;
     if ((a.a & 15u) || (a.b & 15u)) return false;            // TMA operands (their pitches are multiples of 32 bytes with k a multiple of 64)
+    // up to 8 rows (MLX: 2) the rows kernel of matmul.cu reads the codes faster: a layer of an 8B model, int4, 8 rows 84 us there, 120 here; 9 rows 142
+    // and 121; int8 128 and 166, 227 and 166; MLX 2 rows 150 and 176, 4 rows 199 and 155. It needs whole 512-nibble steps of k.
+    const uint32_t bits = a.b_mode == UZU_QMODE_U4 ? 4 : 8;
+    if (a.m <= (a.b_prologue == UZU_B_SCALE_BIAS_DEQUANT ? 2u : 8u) && a.k * bits % 2048u == 0) return false;
     // 17 .. 63 rows over a matrix of at most 2^21 weights (about a megabyte, it stays in L2): launches of 16 rows as before (matmul.cu)
     if (a.m > 16 && a.m < 64 && (uint64_t)a.n * a.k <= (1u << 21)) return false;
     return tensor_map_encoder() != nullptr;
@@ -506,11 +527,11 @@ namespace {
 
 struct QsPlan { int nt = 0; uint32_t splits = 1; float cost = 1e30f; };
 
-// Cycles of one CTA per 64 k of a tile: two planes of products take 2 NT of the tensor pipe; a dequant group's block takes `turn`, and the groups
-// work side by side.
+// Cycles of one CTA per 64 k of a tile, as measured: a product takes about 64 cycles however few its rows are and the product warp's waits come on top
+// (16 rows 850, 128 rows 940), wide tiles run at the tensor pipe (256 rows 1240); MLX and 8-bit codes keep the dequant warps busier than that.
 float qs_block_cycles(int nt, uint32_t bits, bool mlx) {
-    const float turn = mlx ? 1500.0f : bits == 4 ? 700.0f : 900.0f;
-    return std::max(2.0f * nt, turn / (nt > 64 ? 2.0f : 3.0f));
+    const float products = std::max(850.0f + 0.7f * nt, 4.85f * nt), turn = mlx ? 4000.0f : bits == 4 ? 2000.0f : 2800.0f;
+    return std::max(products, turn / (nt > 128 ? 3.0f : 4.0f));
 }
 
 // Rows per tile and CTAs per tile: the shortest estimated time over the chip. A wider tile turns its codes once for more rows; a narrower one or a
@@ -525,7 +546,7 @@ QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, ui
         for (uint32_t splits = 1; splits <= 8; splits *= 2) {
             const uint32_t per = ((nkb + splits - 1) / splits + 3u) & ~3u;           // whole code tiles per rank
             if (splits > 1 && (per * (splits - 1) >= nkb || tiles * splits > sms)) break;
-            const float item = (float)std::min(per, nkb) * qs_block_cycles(nt, bits, mlx) + (nt > 128 ? 2000.0f + 10.0f * nt : 1500.0f) + (splits > 1 ? 1500.0f + 8.0f * nt : 0.0f);
+            const float item = (float)std::min(per, nkb) * qs_block_cycles(nt, bits, mlx) + 2500.0f + (nt > 64 ? 12.0f * nt : 0.0f) + (splits > 1 ? 1500.0f + 8.0f * nt : 0.0f);
             const uint32_t waves = (tiles * splits + sms - 1) / sms;
             const float cost = waves * item;
             if (cost < best.cost) best = {nt, splits, cost};
@@ -582,6 +603,7 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     p.has_soft_cap = (a.d_transform & UZU_D_SOFT_CAP) != 0;
     p.ab_scale = (a.d_transform & UZU_D_SCALE) ? a.ab_scale : 1.0f;
     p.soft_cap = a.soft_cap;
+    p.plain = !p.d_is_f32 && !p.accumulate && !p.has_soft_cap && !p.bias && p.ab_scale == 1.0f;
     p.error = umma_error_word();
     p.m = a.m;
     p.d = (void*)a.d;
