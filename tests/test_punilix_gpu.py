@@ -382,6 +382,36 @@ def latent_plain(q, kv, uk, norm_w, m, eps, prefix, cache):
     return out.numpy(), rows.numpy()
 
 
+@pytest.mark.parametrize("T,heads,rank,rot,prefix,window,extra", [(16, 2, 64, 0, 0, 0, False), (33, 3, 128, 16, 0, 0, True), (70, 16, 512, 64, 0, 0, False), (17, 5, 320, 32, 130, 0, False),
+                                                                  (64, 1, 256, 64, 63, 40, True), (100, 8, 192, 16, 200, 1, False)])
+def test_latent_attention_of_prompt_rows(ctx, T, heads, rank, rot, prefix, window, extra):
+    """The tensor-pipe form: rows that end inside a token's heads, ranks that leave column blocks of a quarter unused, windows that begin inside a tile,
+    sinks and gates; rows behind the last key are NaN. Queries and weights keep f32 precision; the bound: a score
+    of up to 60 before its scale is off by 2^-23 of that for each of up to 36 additions, times 1/8 and less, and an output of 5 times the rms by as much."""
+    rng = np.random.default_rng(T + rank)
+    w = rank + rot
+    q = rng.standard_normal((T, heads, w), dtype=np.float32)
+    n = prefix + T
+    cache = synth.f32_to_bf16_bits(rng.standard_normal((n + 70, w), dtype=np.float32))
+    cache[n:] = 0x7FC0
+    sinks, gate = rng.standard_normal(heads, dtype=np.float32), rng.standard_normal((T, heads), dtype=np.float32)
+    bq, bc, bo, bs, bg = ctx.upload(q), ctx.upload(cache), ctx.upload(np.zeros((T, heads, rank), np.float32)), ctx.upload(sinks), ctx.upload(gate)
+    a = B.LatentAttentionArgs(query=bq.ptr, cache=bc.ptr, out=bo.ptr, rows=T, heads=heads, rank=rank, rot_dim=rot, prefix=prefix, cache_dt=B.DT_BF16, scale=w ** -0.5, splits=1,
+                              window=window, sinks=bs.ptr if extra else 0, head_gate=bg.ptr if extra else 0, head_gate_stride=heads)
+    run(ctx, "uzu_latent_attention_encode", C.byref(a))
+    rows = t64(synth.st_bits_to_f32(cache[:n]))
+    pos, j = torch.arange(prefix, n)[:, None], torch.arange(n)[None, :]
+    mask = (j <= pos) & ((pos - j < window) if window else True)
+    s = torch.einsum("thw,nw->thn", t64(q), rows) * w ** -0.5
+    s = s.masked_fill(~mask[:, None, :], float("-inf"))
+    if extra:
+        s = torch.cat([s, t64(sinks)[None, :, None].expand(T, heads, 1)], -1)
+    ref = torch.softmax(s, -1)[..., :n] @ rows[:, :rank]
+    if extra:
+        ref = ref * torch.sigmoid(t64(gate))[..., None]
+    close(bo.numpy(np.float32, (T, heads, rank)), ref.numpy(), 1e-5, "latent attention of prompt rows")
+
+
 def latent_sizes(heads, dim, rot_dim, rank, dims=None, scaling=None, base=10000.0):
     return {"heads": heads, "dim": dim, "rot_dim": rot_dim, "kv_rank": rank, "scale": 0.3,
             "rot": {"dims": dims or rot_dim, "base": base, "scaling": scaling}}

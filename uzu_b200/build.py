@@ -43,6 +43,7 @@ SOURCES = {
     "residual_f32.cu": [],
     "general_delta.cu": [],
     "latent_attention.cu": [],
+    "latent_attention_mma.cu": [],
     "sigmoid_attention.cu": [],
     "window_attention.cu": [],
     "window_attention_mma.cu": [],

@@ -122,6 +122,10 @@ bool dense_umma_applicable(const uzu_dense_linear_args& a);
 // tensor-core prefill attention (attention_prefill.cu, opt-in), tried first by uzu_attention_single_pass_encode
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a);
 
+// latent attention of a prompt's rows on the tensor pipe (latent_attention_mma.cu)
+bool latent_attention_mma_applicable(const uzu_latent_attention_args& a);
+void encode_latent_attention_mma(uzu_command_buffer* cmd, const uzu_latent_attention_args& a);
+
 // multi-token DeltaNet recurrence (deltanet_prefill.cu), tried by the engine's batched hybrid prefill; scratch may be 0 (then only passes of 2
 // and 3 tokens are taken)
 bool encode_delta_net_prefill(uzu_command_buffer* cmd, const uzu_delta_net_fused_update_args& f, uint32_t rows, uint32_t in_stride, uint32_t out_stride,

@@ -368,6 +368,10 @@ void uzu_latent_attention_encode(uzu_command_buffer* cmd, const uzu_latent_atten
         return;
     }
     if (a->rows == 0) return;
+    if (latent_attention_mma_applicable(*a)) {
+        encode_latent_attention_mma(cmd, *a);
+        return;
+    }
     if (a->cache_dt == UZU_DT_BF16) dispatch_latent_attention<__nv_bfloat16>(cmd, *a);
     else dispatch_latent_attention<float>(cmd, *a);
 }
