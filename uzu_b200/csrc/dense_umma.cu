@@ -8,7 +8,7 @@
 //   warps 0..3 (128 threads): PRODUCERS. Per K block each thread copies 8 + 8 16-byte pieces (8 consecutive lanes per row: whole
 //     128-byte lines) into the K-major SWIZZLE_128B layout (8-row x 128-byte atoms, piece index XOR row-in-atom), waits for its copies
 //     of the block two iterations back, fences them to the async proxy and arrives on the stage's `full` barrier.
-//   warp 4, one lane: MMA ISSUER. Per K block 4 x tcgen05.mma.cta_group::1.kind::f16 (128 x 128 x 16) into 128 TMEM columns, then
+//   warp 4: MMA ISSUER, one lane by elect.sync (behind `lane == 0` an instruction took about 300 clk to issue). Per K block 4 x tcgen05.mma.cta_group::1.kind::f16 (128 x 128 x 16) into 128 TMEM columns, then
 //     tcgen05.commit on the stage's `empty` barrier; after the last block a commit on the accumulator barrier.
 //   warps 0..3 again: EPILOGUE. tcgen05.ld 32 lanes x 32 columns, scale / factors / bias / gelu / accumulate, 16-byte stores (f32 or bf16).
 // Row groups (routed experts): grid z is the group, its compact rows [off[z], off[z+1]) use weight block z; the producers gather the activation
@@ -78,6 +78,11 @@ __device__ __forceinline__ bool du_mbar_wait(uint32_t bar, uint32_t parity) {
     }
     return true;
 }
+__device__ __forceinline__ bool du_elect() {                     // one lane of a converged warp
+    uint32_t p = 0;
+    asm volatile("{ .reg .pred q; .reg .b32 r; elect.sync r|q, 0xffffffff; @q mov.u32 %0, 1; }" : "+r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void du_cp_async16(uint32_t dst_smem, const void* src, uint32_t src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst_smem), "l"(src), "r"(src_bytes) : "memory");
 }
@@ -121,7 +126,7 @@ __global__ void __launch_bounds__(DU_NP + 32, 1) dense_umma_kernel(const DenseUm
     __shared__ uint32_t tmem_slot;
     __shared__ uint32_t gave_up;
 
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, z = blockIdx.z;
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, z = blockIdx.z;   // (warp: uniform for the compiler too)
     constexpr uint32_t kFeatures = EPI == DuPair ? 64u : 128u;        // output features of a CTA
     const uint32_t n0 = blockIdx.x * kFeatures, m0 = blockIdx.y * 128u;
     uint32_t row_begin = 0, rows = p.m;                               // the group's compact rows
@@ -163,7 +168,7 @@ __global__ void __launch_bounds__(DU_NP + 32, 1) dense_umma_kernel(const DenseUm
         atomicCAS(p.error, 0u, code);
     };
 
-    if (tid < (uint32_t)DU_NP) {
+    if (warp < (uint32_t)DU_NP / 32u) {
         // ================================ producers ================================
         constexpr int PA = DU_STAGES - 2;                       // K blocks in flight ahead of the one being handed over
         pdl_wait();
@@ -300,15 +305,18 @@ __global__ void __launch_bounds__(DU_NP + 32, 1) dense_umma_kernel(const DenseUm
             }
         }
     } else {
-        // ================================ MMA issuer (one lane) ================================
-        if (lane == 0) {
-            uint32_t s = 0, parity = 0;
-            for (uint32_t kb = 0; kb < nkb; ++kb) {
-                if (!du_mbar_wait(full_bar(s), parity)) { fail(3); break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t a_addr = smem_base + s * DU_STAGE_BYTES, b_addr = a_addr + DU_TILE_BYTES;
-                const uint64_t hi = (uint64_t)p.desc_hi << 32;
-                const uint32_t lbo = p.desc_lbo << 16;
+        // ================================ MMA issuer ================================
+        uint32_t s = 0, parity = 0;
+        for (uint32_t kb = 0; kb < nkb; ++kb) {
+            if (__any_sync(0xffffffffu, !du_mbar_wait(full_bar(s), parity))) {
+                if (lane == 0) fail(3);
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t a_addr = smem_base + s * DU_STAGE_BYTES, b_addr = a_addr + DU_TILE_BYTES;
+            const uint64_t hi = (uint64_t)p.desc_hi << 32;
+            const uint32_t lbo = p.desc_lbo << 16;
+            if (du_elect()) {
 #pragma unroll
                 for (uint32_t kk = 0; kk < 4; ++kk) {
                     const uint64_t da = hi | (uint64_t)((((a_addr >> 4) + kk * p.k_step) & 0x3FFFu) | lbo);
@@ -319,10 +327,11 @@ __global__ void __launch_bounds__(DU_NP + 32, 1) dense_umma_kernel(const DenseUm
                                  : "memory");
                 }
                 asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(empty_bar(s)) : "memory");
-                if (++s == (uint32_t)DU_STAGES) { s = 0; parity ^= 1u; }
             }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(accum_bar) : "memory");
+            __syncwarp();
+            if (++s == (uint32_t)DU_STAGES) { s = 0; parity ^= 1u; }
         }
+        if (du_elect()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(accum_bar) : "memory");
         __syncwarp();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
