@@ -66,8 +66,11 @@ __global__ void __launch_bounds__(256) attention_prepare_kernel(const uzu_attent
 }
 
 // Eight neighbouring channels of a (token, head) per thread, 16-byte accesses; the same arithmetic (1024 tokens x 48 heads of 128 took 53 us a
-// channel at a time with a CTA per token and head).
-__global__ void __launch_bounds__(256) attention_prepare_vec_kernel(const uzu_attention_prepare_args a) {
+// channel at a time with a CTA per token and head). SEQS: row b belongs to sequence b, with its own cache, position and query row.
+struct NoSequences {};
+template <bool SEQS>
+__global__ void __launch_bounds__(256) attention_prepare_vec_kernel(const uzu_attention_prepare_args a,
+                                                                    const __grid_constant__ std::conditional_t<SEQS, AttnSequences, NoSequences> seqs) {
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t total_heads = a.has_kv ? a.num_q_heads + 2 * a.num_kv_heads : a.num_q_heads, chunks = a.head_dim / 8u;
@@ -77,9 +80,18 @@ __global__ void __launch_bounds__(256) attention_prepare_vec_kernel(const uzu_at
     const __nv_bfloat16* head = reinterpret_cast<const __nv_bfloat16*>(a.qkv) + ((size_t)b * total_heads + h) * a.head_dim;
     const bool is_query = !a.has_kv || h < a.num_q_heads, is_key = a.has_kv && h >= a.num_q_heads && h < a.num_q_heads + a.num_kv_heads;
     uint32_t row = a.kv_token_offset, rope_row = b;
-    if (a.dynamic_position) {
-        row = *reinterpret_cast<const uint32_t*>(a.dynamic_position);
-        rope_row += row;
+    uint64_t keys = a.keys, values = a.values;
+    if constexpr (SEQS) {
+        row = a.dynamic_position ? reinterpret_cast<const uint32_t*>(a.dynamic_position)[b] : seqs.prefix[b];
+        rope_row = a.dynamic_position ? row : seqs.position[b];
+        keys = seqs.keys[b];
+        values = seqs.values[b];
+    } else {
+        if (a.dynamic_position) {
+            row = *reinterpret_cast<const uint32_t*>(a.dynamic_position);
+            rope_row += row;
+        }
+        row += b;
     }
     uint4 v = *reinterpret_cast<const uint4*>(head + d);
     if (a.has_rope && d < a.rope_dim && (is_query || is_key)) {
@@ -103,9 +115,9 @@ __global__ void __launch_bounds__(256) attention_prepare_vec_kernel(const uzu_at
         }
     }
     __nv_bfloat16* dst;
-    if (is_query) dst = reinterpret_cast<__nv_bfloat16*>(a.queries) + ((size_t)h * a.batch_dim + b) * a.head_dim;
-    else if (is_key) dst = reinterpret_cast<__nv_bfloat16*>(a.keys) + ((size_t)(row + b) * a.num_kv_heads + (h - a.num_q_heads)) * a.head_dim;
-    else dst = reinterpret_cast<__nv_bfloat16*>(a.values) + ((size_t)(row + b) * a.num_kv_heads + (h - a.num_q_heads - a.num_kv_heads)) * a.head_dim;
+    if (is_query) dst = reinterpret_cast<__nv_bfloat16*>(a.queries) + (SEQS ? (size_t)b * a.num_q_heads + h : (size_t)h * a.batch_dim + b) * a.head_dim;
+    else if (is_key) dst = reinterpret_cast<__nv_bfloat16*>(keys) + ((size_t)row * a.num_kv_heads + (h - a.num_q_heads)) * a.head_dim;
+    else dst = reinterpret_cast<__nv_bfloat16*>(values) + ((size_t)row * a.num_kv_heads + (h - a.num_q_heads - a.num_kv_heads)) * a.head_dim;
     *reinterpret_cast<uint4*>(dst + d) = v;
 }
 
@@ -235,8 +247,9 @@ constexpr int ATTN_UNROLL = 2;      // key rows per lane group per round (one mo
 // loaded ATTN_UNROLL at a time with no dependency between them; (2) chunk max / exp / sum per head; (3) o += p.V with the V
 // rows streamed the same way. The running (m, l, o) is rescaled only once per chunk, so the key loop has no serial
 // softmax chain (the first version of this kernel updated (m, l, o) per key and spent most of its time waiting on loads).
-template <int D, int G>
-__global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnParams p) {
+// SEQS: grid y is a sequence with one query row and a cache of its own instead of a query row.
+template <int D, int G, bool SEQS>
+__global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnParams p, const __grid_constant__ std::conditional_t<SEQS, AttnSequences, NoSequences> seqs) {
     constexpr int EPL = (D >= 128 && G < 8) ? 16 : 8;    // elements per lane (q and o live in registers: 2 * G * EPL floats)
     constexpr int CH = (G >= 8) ? ATTN_CHUNK / 2 : ATTN_CHUNK;   // scores [G][CH] + partial outputs stay under the 48 KB static limit
     constexpr int LPK = D / EPL;              // lanes per key row
@@ -252,13 +265,20 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     pdl_wait();
     uzu_attention_args a = p.a;
     uint32_t keys_per_split = p.keys_per_split;
-    if (a.dynamic_position) {
+    if constexpr (SEQS) {
+        const uint32_t b = blockIdx.y;
+        a.sequence_length = (a.dynamic_position ? reinterpret_cast<const uint32_t*>(a.dynamic_position)[b] : seqs.prefix[b]) + 1u;
+        a.keys = seqs.keys[b];
+        a.values = seqs.values[b];
+        a.queries += (uint64_t)b * a.num_heads * D * 2u;
+        keys_per_split = ((a.sequence_length + p.nsplits - 1) / p.nsplits + 15u) & ~15u;
+    } else if (a.dynamic_position) {
         a.sequence_length = *reinterpret_cast<const uint32_t*>(a.dynamic_position) + a.suffix_length;
         keys_per_split = ((a.sequence_length + p.nsplits - 1) / p.nsplits + 15u) & ~15u;   // whole CTA steps per split
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane / LPK, li = lane % LPK, d0 = li * EPL;
-    const uint32_t head0 = blockIdx.x * G, qs = blockIdx.y, split = blockIdx.z;
+    const uint32_t head0 = blockIdx.x * G, out_row = blockIdx.y, qs = SEQS ? 0u : blockIdx.y, split = blockIdx.z;
     const uint32_t kvh = head0 / a.gqa_factor;
 
     const uint32_t prefix_length = a.sequence_length - a.suffix_length;
@@ -445,7 +465,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
 #pragma unroll
         for (int w = 0; w < ATTN_WARPS * KPW; ++w) ov += sm_o[w][h][d];
         const float lv = sm_lfin[h], gm = sm_mfin[h];
-        const size_t o_off = (size_t)qs * H + head0 + h;
+        const size_t o_off = (size_t)out_row * H + head0 + h;
         if (direct) {
             p.final_out[o_off * D + d] = f2bf(ov / lv);
         } else {
@@ -462,7 +482,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
         if (split == 0) {
             for (uint32_t blk = p.nsplits + warp; blk < p.nb; blk += ATTN_WARPS)
                 for (int h = 0; h < G; ++h) {
-                    const size_t o_off = (size_t)qs * H + head0 + h;
+                    const size_t o_off = (size_t)out_row * H + head0 + h;
                     for (int d = lane; d < D; d += 32) p.part_o[(o_off * p.nb + blk) * D + d] = 0.0f;
                     if (lane == 0) { p.part_sum[o_off * p.nb + blk] = 0.0f; p.part_max[o_off * p.nb + blk] = -1e9f; }
                 }
@@ -472,13 +492,13 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     // ---- in-kernel merge: the last CTA of this (token, head group) combines all splits (nsplits <= 32) -----------------
     __threadfence();
     __syncthreads();
-    const uint32_t cidx = qs * gridDim.x + blockIdx.x;
+    const uint32_t cidx = out_row * gridDim.x + blockIdx.x;
     if (threadIdx.x == 0) sm_ticket = atomicAdd(&p.counters[cidx], 1u);
     __syncthreads();
     if (sm_ticket != p.nsplits - 1) return;
     __threadfence();
     for (int h = warp; h < G; h += ATTN_WARPS) {        // one warp per head: split factors and the global sum
-        const size_t o_off = (size_t)qs * H + head0 + h;
+        const size_t o_off = (size_t)out_row * H + head0 + h;
         const bool has = (uint32_t)lane < p.nsplits;
         const float mymax = has ? __ldcg(&p.part_max[o_off * p.nb + lane]) : -INFINITY;
         const float gmax = warp_max(mymax);
@@ -490,7 +510,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     __syncthreads();
     for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
         const int h = idx / D, d = idx % D;
-        const size_t o_off = (size_t)qs * H + head0 + h;
+        const size_t o_off = (size_t)out_row * H + head0 + h;
         const float* po = p.part_o + (o_off * p.nb) * D + d;
         float val = 0.0f;
         float pv[32];                                   // all split partials of this output in flight at once
@@ -563,19 +583,20 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(const __nv_bfloat16* 
 // host dispatch
 // ---------------------------------------------------------------------------------------------------
 template <int D, int G>
-static void launch_attn(uzu_command_buffer* cmd, const AttnParams& p, uint32_t head_groups) {
-    dim3 grid(head_groups, p.a.suffix_length, p.nsplits);
-    launch(cmd, "attn_split_kernel", attn_split_kernel<D, G>, grid, dim3(ATTN_WARPS * 32), 0, p);
+static void launch_attn(uzu_command_buffer* cmd, const AttnParams& p, const AttnSequences* seqs, uint32_t head_groups) {
+    dim3 grid(head_groups, seqs ? seqs->count : p.a.suffix_length, p.nsplits);
+    if (seqs) launch(cmd, "attn_split_kernel", attn_split_kernel<D, G, true>, grid, dim3(ATTN_WARPS * 32), 0, p, *seqs);
+    else launch(cmd, "attn_split_kernel", attn_split_kernel<D, G, false>, grid, dim3(ATTN_WARPS * 32), 0, p, NoSequences{});
 }
 
 template <int D>
-static void launch_attn_g(uzu_command_buffer* cmd, const AttnParams& p, int g) {
+static void launch_attn_g(uzu_command_buffer* cmd, const AttnParams& p, const AttnSequences* seqs, int g) {
     const uint32_t H = p.a.num_heads;
     switch (g) {
-        case 8: launch_attn<D, 8>(cmd, p, H / 8); break;
-        case 4: launch_attn<D, 4>(cmd, p, H / 4); break;
-        case 2: launch_attn<D, 2>(cmd, p, H / 2); break;
-        default: launch_attn<D, 1>(cmd, p, H); break;
+        case 8: launch_attn<D, 8>(cmd, p, seqs, H / 8); break;
+        case 4: launch_attn<D, 4>(cmd, p, seqs, H / 4); break;
+        case 2: launch_attn<D, 2>(cmd, p, seqs, H / 2); break;
+        default: launch_attn<D, 1>(cmd, p, seqs, H); break;
     }
 }
 
@@ -610,12 +631,86 @@ static int pick_group(uint32_t gqa) {
     return 1;
 }
 
-static void dispatch_attn(uzu_command_buffer* cmd, const AttnParams& p, int g) {
+static void dispatch_attn(uzu_command_buffer* cmd, const AttnParams& p, const AttnSequences* seqs, int g) {
     switch (p.a.head_dim) {
-        case 64: launch_attn_g<64>(cmd, p, g); break;
-        case 128: launch_attn_g<128>(cmd, p, g); break;
-        default: launch_attn_g<256>(cmd, p, g); break;
+        case 64: launch_attn_g<64>(cmd, p, seqs, g); break;
+        case 128: launch_attn_g<128>(cmd, p, seqs, g); break;
+        default: launch_attn_g<256>(cmd, p, seqs, g); break;
     }
+}
+
+// the rows' keys cut over CTAs, merged by the last CTA of a (row, head group)
+static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& a, const AttnSequences* seqs) {
+    uzu_context* ctx = cmd->ctx;
+    const int g = pick_group(a.gqa_factor);
+    const uint32_t head_groups = a.num_heads / g, rows = seqs ? seqs->count : a.suffix_length;
+    // enough CTAs for ~2 waves, >= 64 keys per split, <= 32 splits, and only for short suffixes (decode)
+    uint32_t nsplits = 1;
+    if (rows <= 16) {
+        const uint32_t ctas = head_groups * rows;
+        const uint32_t want = (2u * (uint32_t)ctx->sm_count + ctas - 1) / ctas;
+        const uint32_t cap = (a.sequence_length + 63) / 64;
+        nsplits = std::max(1u, std::min(std::min(want, cap), 32u));
+    }
+    AttnParams p{};
+    p.a = a;
+    p.final_out = reinterpret_cast<__nv_bfloat16*>(a.out);
+    p.fuse_merge = 1;
+    p.nsplits = nsplits;
+    p.nb = nsplits;
+    p.keys_per_split = nsplits > 1 ? (((a.sequence_length + nsplits - 1) / nsplits + 15u) & ~15u) : a.sequence_length;
+    if (nsplits > 1) {
+        const size_t units = (size_t)rows * a.num_heads * nsplits;
+        const size_t need = units * (a.head_dim + 2) * sizeof(float);
+        if (need > ctx->attn_ws_bytes) {  // grows outside graph capture only (decode needs < 2 MiB)
+            cudaStreamSynchronize(ctx->stream);
+            cudaFree(ctx->attn_ws);
+            if (cudaMalloc(&ctx->attn_ws, need) != cudaSuccess) {
+                ctx->attn_ws = nullptr;
+                ctx->attn_ws_bytes = 0;
+                cmd->record_error(UZU_ERROR_OUT_OF_MEMORY, "attention_single_pass: workspace allocation failed");
+                return;
+            }
+            ctx->attn_ws_bytes = need;
+        }
+        if ((size_t)rows * head_groups > 65536) {
+            cmd->record_error(UZU_ERROR_UNSUPPORTED, "attention_single_pass: too many (token, head group) pairs for the split path");
+            return;
+        }
+        p.part_o = ctx->attn_ws;
+        p.part_sum = ctx->attn_ws + units * a.head_dim;
+        p.part_max = p.part_sum + units;
+        p.counters = ctx->attn_counters;
+    }
+    dispatch_attn(cmd, p, seqs, g);
+}
+
+// whole 16-byte pieces of every row, and of each half of the rotated channels
+static bool attention_prepare_whole_pieces(const uzu_attention_prepare_args& a) {
+    const uint64_t total_heads = a.has_kv ? a.num_q_heads + 2 * a.num_kv_heads : a.num_q_heads;
+    return a.head_dim % 8u == 0 && (!a.has_rope || (a.rope_dim % 16u == 0 && !((a.cosines | a.sines) & 15u))) && total_heads * a.batch_dim * (a.head_dim / 8u) < 0x80000000ull &&
+           !((a.qkv | a.queries) & 15u);
+}
+
+// Plain causal rows on caches of whole 16-byte pieces. 8 sequences x 32 heads of 128 at 200 cached rows, a layer: 19 us -- 132 us as a prepare and
+// an attention launch per sequence.
+bool attention_sequences_applicable(const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s) {
+    uint64_t caches = 0;
+    for (uint32_t b = 0; b < s.count; ++b) caches |= s.keys[b] | s.values[b];
+    return s.count && s.count <= kMaxAttnSequences && p.batch_dim == s.count && p.has_kv && a.suffix_length == 1 && !a.is_trie && !a.is_kv_cache_ring && !a.is_sliding_window &&
+           !a.has_sinks && attention_prepare_whole_pieces(p) && !(caches & 15u);
+}
+
+void encode_attention_sequences(uzu_command_buffer* cmd, const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s) {
+    if (!encodable(cmd, "attention_sequences")) return;
+    uzu_attention_args longest = a;                                  // the longest sequence decides on the cut
+    longest.keys = s.keys[0];
+    longest.values = s.values[0];
+    for (uint32_t b = 0; b < s.count; ++b) longest.sequence_length = std::max(longest.sequence_length, s.prefix[b] + 1u);
+    if (!attn_common_checks(cmd, &longest, "attention_sequences")) return;
+    const uint32_t units = (p.num_q_heads + 2 * p.num_kv_heads) * s.count * (p.head_dim / 8u);
+    launch(cmd, "attention_prepare_kernel", attention_prepare_vec_kernel<true>, dim3((units + 255u) / 256u), dim3(256), 0, p, s);
+    encode_attn_rows(cmd, longest, &s);
 }
 
 }  // namespace uzu
@@ -632,11 +727,9 @@ void uzu_attention_prepare_encode(uzu_command_buffer* cmd, const uzu_attention_p
     }
     const uint32_t total_heads = a->has_kv ? a->num_q_heads + 2 * a->num_kv_heads : a->num_q_heads;
     if (a->batch_dim == 0 || total_heads == 0) return;
-    // whole 16-byte pieces of every row, and of each half of the rotated channels
-    const uint64_t units = (uint64_t)total_heads * a->batch_dim * (a->head_dim / 8u);
-    if (a->head_dim % 8u == 0 && (!a->has_rope || (a->rope_dim % 16u == 0 && !((a->cosines | a->sines) & 15u))) && units < 0x80000000ull &&
-        !((a->qkv | a->queries | (a->has_kv ? a->keys | a->values : 0u)) & 15u)) {
-        uzu::launch(cmd, "attention_prepare_kernel", uzu::attention_prepare_vec_kernel, dim3((uint32_t)((units + 255u) / 256u)), dim3(256), 0, *a);
+    if (uzu::attention_prepare_whole_pieces(*a) && !((a->has_kv ? a->keys | a->values : 0u) & 15u)) {
+        const uint32_t units = total_heads * a->batch_dim * (a->head_dim / 8u);
+        uzu::launch(cmd, "attention_prepare_kernel", uzu::attention_prepare_vec_kernel<false>, dim3((units + 255u) / 256u), dim3(256), 0, *a, uzu::NoSequences{});
         return;
     }
     dim3 grid(total_heads, a->batch_dim);
@@ -667,49 +760,8 @@ void uzu_attention_prepare_norm_encode(uzu_command_buffer* cmd, const uzu_attent
 void uzu_attention_single_pass_encode(uzu_command_buffer* cmd, const uzu_attention_args* a) {
     if (!uzu::encodable(cmd, "attention_single_pass")) return;
     if (!uzu::attn_common_checks(cmd, a, "attention_single_pass")) return;
-    if (uzu::encode_attention_prefill(cmd, *a)) return;   // opt-in tensor-core path for suffix >= 16 (attention_prefill.cu)
-    uzu_context* ctx = cmd->ctx;
-    const int g = uzu::pick_group(a->gqa_factor);
-    const uint32_t head_groups = a->num_heads / g;
-    // enough CTAs for ~2 waves, >= 64 keys per split, <= 32 splits, and only for short suffixes (decode)
-    uint32_t nsplits = 1;
-    if (a->suffix_length <= 16) {
-        const uint32_t ctas = head_groups * a->suffix_length;
-        const uint32_t want = (2u * (uint32_t)ctx->sm_count + ctas - 1) / ctas;
-        const uint32_t cap = (a->sequence_length + 63) / 64;
-        nsplits = std::max(1u, std::min(std::min(want, cap), 32u));
-    }
-    uzu::AttnParams p{};
-    p.a = *a;
-    p.final_out = reinterpret_cast<__nv_bfloat16*>(a->out);
-    p.fuse_merge = 1;
-    p.nsplits = nsplits;
-    p.nb = nsplits;
-    p.keys_per_split = nsplits > 1 ? (((a->sequence_length + nsplits - 1) / nsplits + 15u) & ~15u) : a->sequence_length;
-    if (nsplits > 1) {
-        const size_t units = (size_t)a->suffix_length * a->num_heads * nsplits;
-        const size_t need = units * (a->head_dim + 2) * sizeof(float);
-        if (need > ctx->attn_ws_bytes) {  // grows outside graph capture only (decode needs < 2 MiB)
-            cudaStreamSynchronize(ctx->stream);
-            cudaFree(ctx->attn_ws);
-            if (cudaMalloc(&ctx->attn_ws, need) != cudaSuccess) {
-                ctx->attn_ws = nullptr;
-                ctx->attn_ws_bytes = 0;
-                cmd->record_error(UZU_ERROR_OUT_OF_MEMORY, "attention_single_pass: workspace allocation failed");
-                return;
-            }
-            ctx->attn_ws_bytes = need;
-        }
-        if ((size_t)a->suffix_length * head_groups > 65536) {
-            cmd->record_error(UZU_ERROR_UNSUPPORTED, "attention_single_pass: too many (token, head group) pairs for the split path");
-            return;
-        }
-        p.part_o = ctx->attn_ws;
-        p.part_sum = ctx->attn_ws + units * a->head_dim;
-        p.part_max = p.part_sum + units;
-        p.counters = ctx->attn_counters;
-    }
-    uzu::dispatch_attn(cmd, p, g);
+    if (uzu::encode_attention_prefill(cmd, *a)) return;   // the tensor-pipe form (attention_prefill.cu)
+    uzu::encode_attn_rows(cmd, *a, nullptr);
 }
 
 void uzu_attention_two_pass1_encode(uzu_command_buffer* cmd, const uzu_attention_args* a) {
@@ -734,7 +786,7 @@ void uzu_attention_two_pass1_encode(uzu_command_buffer* cmd, const uzu_attention
     p.nsplits = std::max(1u, std::min(std::min(want, cap), 32u));
     p.nb = 32;  // TOTAL_BLOCKS_COUNT (attention_two_pass.rs:10)
     p.keys_per_split = p.nsplits > 1 ? (((a->sequence_length + p.nsplits - 1) / p.nsplits + 15u) & ~15u) : a->sequence_length;
-    uzu::dispatch_attn(cmd, p, g);
+    uzu::dispatch_attn(cmd, p, nullptr, g);
 }
 
 void uzu_attention_two_pass2_encode(uzu_command_buffer* cmd, const uzu_attention_two_pass2_args* a) {

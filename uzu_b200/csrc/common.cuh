@@ -106,6 +106,9 @@ inline void launch(uzu_command_buffer* cmd, const char* what, void (*kernel)(KAr
 bool prefill_gemm_applicable(const uzu_matmul_args& a);
 void encode_prefill_gemm(uzu_command_buffer* cmd, const uzu_matmul_args& a);
 
+// quantised products of 2 .. 48 rows (qmm_rows.cu), dispatched from encode_matmul
+bool qmm_rows_applicable(uzu_command_buffer* cmd, const uzu_matmul_args& a);
+void encode_qmm_rows(uzu_command_buffer* cmd, const uzu_matmul_args& a);
 // quantised products of two and more rows on tcgen05, group scales applied to partial sums (qmm_scaled.cu), dispatched from encode_matmul
 bool qmm_scaled_applicable(const uzu_matmul_args& a);
 void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a);
@@ -121,6 +124,16 @@ bool dense_umma_applicable(const uzu_dense_linear_args& a);
 
 // tensor-core prefill attention (attention_prefill.cu, opt-in), tried first by uzu_attention_single_pass_encode
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a);
+
+// One decoded row of several sequences, each with a cache of its own (attention.cu): a launch for all of them instead of one per sequence.
+constexpr uint32_t kMaxAttnSequences = 16;
+struct AttnSequences {
+    uint64_t keys[kMaxAttnSequences], values[kMaxAttnSequences];
+    uint32_t prefix[kMaxAttnSequences], position[kMaxAttnSequences];      // cached rows, rotation row; both from dynamic_position[b] where the args have one
+    uint32_t count;
+};
+bool attention_sequences_applicable(const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s);
+void encode_attention_sequences(uzu_command_buffer* cmd, const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s);
 
 // latent attention of a prompt's rows on the tensor pipe (latent_attention_mma.cu)
 bool latent_attention_mma_applicable(const uzu_latent_attention_args& a);

@@ -2899,44 +2899,60 @@ static void encode_batch_step(uzu_engine* e, uzu_command_buffer* cmd, bool dyn) 
             const size_t qkv_row = (size_t)total_heads * D * 2, q_row = (size_t)Hq * D * 2;
             if (A.has_gate) encode_linear(cmd, A.gate, e->hidden_b.ptr(), B, e->gate.ptr());
             encode_linear(cmd, A.qkv, e->hidden_b.ptr(), B, e->qkv.ptr());
-            for (uint32_t b = 0; b < B; ++b) {     // per sequence: q/k norm, RoPE at its own position + KV append, attention over its own cache
-                LayerState& S = e->seqs[b].layers[i];
-                const uint32_t pos = e->seqs[b].context_length;
-                const uint64_t qkv_b = e->qkv.ptr() + b * qkv_row;
-                auto qkn = [&](const Norm& n, uint32_t off, uint32_t cnt) {
-                    if (!n.present || cnt == 0) return;
-                    uzu_qkv_norm_args qa{};
-                    qa.scales = n.scales.ptr(); qa.qkv_output = qkv_b;
-                    qa.batch_size = 1; qa.total_heads = total_heads; qa.head_dim = D;
-                    qa.epsilon = n.cfg.epsilon; qa.scale_offset = n.cfg.scale_offset;
-                    qa.head_offset = off; qa.head_count = cnt; qa.full_layer = n.cfg.full_layer;
-                    qa.in_place = 1; qa.has_scales = n.cfg.has_scale;
-                    uzu_qkv_norm_encode(cmd, &qa);
-                };
-                qkn(A.qnorm, 0, Hq);
-                qkn(A.knorm, Hq, Hkv);
-                uzu_attention_prepare_args pa{};
-                pa.qkv = qkv_b; pa.queries = e->queries.ptr() + b * q_row;
-                pa.keys = S.keys; pa.values = S.values;
-                pa.num_q_heads = Hq; pa.num_kv_heads = Hkv; pa.head_dim = D;
-                pa.kv_token_offset = S.length; pa.batch_dim = 1; pa.has_kv = 1;
-                if (A.rope_index >= 0) {
-                    const RopeCfg& rc = e->ropes[A.rope_index];
-                    pa.has_rope = 1; pa.rope_dim = rc.head_dim;
+            auto qkn = [&](const Norm& n, uint32_t off, uint32_t cnt) {
+                if (!n.present || cnt == 0) return;
+                uzu_qkv_norm_args qa{};
+                qa.scales = n.scales.ptr(); qa.qkv_output = e->qkv.ptr();
+                qa.batch_size = B; qa.total_heads = total_heads; qa.head_dim = D;
+                qa.epsilon = n.cfg.epsilon; qa.scale_offset = n.cfg.scale_offset;
+                qa.head_offset = off; qa.head_count = cnt; qa.full_layer = n.cfg.full_layer;
+                qa.in_place = 1; qa.has_scales = n.cfg.has_scale;
+                uzu_qkv_norm_encode(cmd, &qa);
+            };
+            qkn(A.qnorm, 0, Hq);
+            qkn(A.knorm, Hq, Hkv);
+            // RoPE at a sequence's own position + KV append, attention over its own cache
+            AttnSequences seqs{};
+            seqs.count = B;
+            for (uint32_t b = 0; b < B; ++b) {
+                const LayerState& S = e->seqs[b].layers[i];
+                seqs.keys[b] = S.keys; seqs.values[b] = S.values;
+                seqs.prefix[b] = S.length; seqs.position[b] = e->seqs[b].context_length;
+            }
+            uzu_attention_prepare_args pa{};
+            pa.qkv = e->qkv.ptr(); pa.queries = e->queries.ptr();
+            pa.num_q_heads = Hq; pa.num_kv_heads = Hkv; pa.head_dim = D;
+            pa.batch_dim = B; pa.has_kv = 1;
+            if (A.rope_index >= 0) {
+                pa.has_rope = 1; pa.rope_dim = e->ropes[A.rope_index].head_dim;
+                pa.cosines = e->rope_cos[A.rope_index].ptr(); pa.sines = e->rope_sin[A.rope_index].ptr();
+            }
+            if (dyn) pa.dynamic_position = e->batch_pos.ptr();
+            uzu_attention_args aa{};
+            aa.queries = pa.queries; aa.out = e->attn_out.ptr();
+            aa.gqa_factor = Hq / Hkv; aa.sequence_length = 1;
+            aa.k_head_stride = D; aa.k_seq_stride = Hkv * D; aa.v_head_stride = D; aa.v_seq_stride = Hkv * D;
+            aa.scale = A.has_scale ? A.scale : 1.0f / sqrtf((float)D);
+            aa.num_heads = Hq; aa.suffix_length = 1; aa.head_dim = D; aa.is_causal = A.is_causal;
+            if (dyn) aa.dynamic_position = e->batch_pos.ptr();
+            if (attention_sequences_applicable(pa, aa, seqs)) {
+                encode_attention_sequences(cmd, pa, aa, seqs);
+            } else {
+                for (uint32_t b = 0; b < B; ++b) {
+                    uzu_attention_prepare_args pb = pa;
+                    pb.qkv += b * qkv_row; pb.queries += b * q_row;
+                    pb.keys = seqs.keys[b]; pb.values = seqs.values[b];
+                    pb.kv_token_offset = seqs.prefix[b]; pb.batch_dim = 1;
                     // with a dynamic position the kernel offsets the tables by the device-resident position itself
-                    pa.cosines = e->rope_cos[A.rope_index].ptr() + (dyn ? 0 : (size_t)pos * rc.head_dim * 4);
-                    pa.sines = e->rope_sin[A.rope_index].ptr() + (dyn ? 0 : (size_t)pos * rc.head_dim * 4);
+                    if (dyn) pb.dynamic_position += (uint64_t)b * 4;
+                    else { pb.cosines += (uint64_t)seqs.position[b] * pa.rope_dim * 4; pb.sines += (uint64_t)seqs.position[b] * pa.rope_dim * 4; }
+                    uzu_attention_prepare_encode(cmd, &pb);
+                    uzu_attention_args ab = aa;
+                    ab.queries = pb.queries; ab.keys = pb.keys; ab.values = pb.values; ab.out += b * q_row;
+                    ab.sequence_length = seqs.prefix[b] + 1;
+                    if (dyn) ab.dynamic_position = pb.dynamic_position;
+                    uzu_attention_single_pass_encode(cmd, &ab);
                 }
-                if (dyn) pa.dynamic_position = e->batch_pos.ptr() + (uint64_t)b * 4;
-                uzu_attention_prepare_encode(cmd, &pa);
-                uzu_attention_args aa{};
-                aa.queries = pa.queries; aa.keys = S.keys; aa.values = S.values; aa.out = e->attn_out.ptr() + b * q_row;
-                aa.gqa_factor = Hq / Hkv; aa.sequence_length = S.length + 1;
-                aa.k_head_stride = D; aa.k_seq_stride = Hkv * D; aa.v_head_stride = D; aa.v_seq_stride = Hkv * D;
-                aa.scale = A.has_scale ? A.scale : 1.0f / sqrtf((float)D);
-                aa.num_heads = Hq; aa.suffix_length = 1; aa.head_dim = D; aa.is_causal = A.is_causal;
-                if (dyn) aa.dynamic_position = e->batch_pos.ptr() + (uint64_t)b * 4;
-                uzu_attention_single_pass_encode(cmd, &aa);
             }
             if (A.has_gate) uzu_sigmoid_gate_encode(cmd, e->gate.ptr(), e->attn_out.ptr(), B * Hq * D);
             encode_linear(cmd, A.out, e->attn_out.ptr(), B, e->mixer_out.ptr());
