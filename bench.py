@@ -475,7 +475,7 @@ def speculation_of(eng, step_ms: float, nodes: int = 16, passes: int = 6):
         eng.trie_accept([0], sampled[0])
     pass_ms = float(np.median(ms[1:]))
     return {"supported": True, "nodes": nodes, "pass_ms": pass_ms, "plain_step_ms": step_ms, "break_even_tokens_per_pass": pass_ms / step_ms,
-            "note": "verify half only (no draft model in scope): the pass runs the unfused kernel sequence with the rows GEMV (2..16 rows per weight pass)"}
+            "note": "verify half only (no draft model in scope): the pass runs the unfused kernel sequence with the few-row GEMM (2..32 rows per weight pass)"}
 
 
 def prefill_gemm_of(eng, prefill: int):

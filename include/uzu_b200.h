@@ -204,10 +204,9 @@ typedef struct uzu_fused_linear_args {
 } uzu_fused_linear_args;
 /* Tuning sweeps only (tools/): override the decode GEMV's work split; 0 = heuristic. Process-wide, not thread-safe. */
 UZU_API void uzu_debug_set_qmv_tuning(int warps_per_tile, int k_slices, int ctas_per_sm, int stages);
-/* Prefill path (m >= 64, quantized B, bf16 A): uzu_matmul_encode runs the tcgen05 tensor-core GEMM with an in-kernel dequant stage
- * (csrc/prefill_gemm.cu); UZU_PREFILL_GEMM_MIN_M=<m> moves the threshold, 0 disables it. Probe hook (tools/umma_probe.py only):
- * override the UMMA shared-memory layout (0 = SWIZZLE_128B, 1 = no swizzle; < 0 = built-in default), descriptor words and the
- * instruction descriptor (0 = default), and force the tokens-per-CTA factor mt (0 = heuristic). Process-wide, not thread-safe. */
+/* Quantized B, bf16 A: 2..32 rows run csrc/qmm_rows.cu (mma.sync, groups of 64 and 128), more rows csrc/qmm_scaled.cu (tcgen05, weights as two
+ * exact bf16 planes in tensor memory); UZU_QMM_ROWS=0 / UZU_QMM_SCALED=0 take the kernels for other shapes instead. uzu_debug_set_umma does nothing:
+ * it overrode descriptors of an earlier kernel. */
 UZU_API void uzu_debug_set_umma(int layout, uint32_t desc_hi, uint32_t desc_lbo, uint32_t k_step, uint32_t idesc, int mt);
 UZU_API int uzu_fused_linear_supported(uzu_context* ctx, const uzu_fused_linear_args* args);
 UZU_API void uzu_fused_linear_encode(uzu_command_buffer* cmd, const uzu_fused_linear_args* args);
@@ -316,10 +315,8 @@ typedef struct uzu_attention_args {
 } uzu_attention_args;
 UZU_API void uzu_attention_single_pass_encode(uzu_command_buffer* cmd, const uzu_attention_args* args);
 UZU_API void uzu_attention_two_pass1_encode(uzu_command_buffer* cmd, const uzu_attention_args* args);
-/* Opt-in tensor-core prefill attention (csrc/attention_prefill.cu; suffix >= 16, plain causal / non-causal, head_dim 64 | 128): taken by
- * uzu_attention_single_pass_encode when UZU_PREFILL_ATTN=1 or after uzu_debug_set_prefill_attention(1); -1 = follow the environment.
- * Round 1: probed on hardware against a float64 softmax (profiles/r1_prefill_attention_probe.txt), oracle tests pending -- the default stays
- * the split-KV kernel. */
+/* Tensor-pipe attention of 8 and more query tokens (csrc/attention_prefill.cu; causal, non-causal and tries, head_dim 64 | 128 | 256), taken by
+ * uzu_attention_single_pass_encode; 0 here or UZU_PREFILL_ATTN=0 keeps the split-KV kernel, 1 forces it on, -1 = follow the environment. */
 UZU_API void uzu_debug_set_prefill_attention(int mode);
 /* AttentionTwoPass2Kernel: attention_two_pass.rs:139-149 */
 typedef struct uzu_attention_two_pass2_args {

@@ -67,3 +67,19 @@ def test_epilogue(ctx):
         check(ctx, m, n, k, 4, 64, "zero", d=d, accumulate=True, bias=bias, ab_scale=0.5)
         check(ctx, m, n, k, 8, 64, "symmetric", soft_cap=3.0, bias=bias)
         check(ctx, m, n, k, 4, 64, "symmetric", signed_codes=True)
+
+
+@pytest.mark.parametrize("bits,gs,method", [(4, 64, "zero"), (4, 128, "zero"), (4, 64, "mlx"), (4, 128, "symmetric"), (8, 64, "zero"), (8, 128, "zero"), (8, 64, "symmetric"), (8, 128, "mlx")])
+@pytest.mark.parametrize("m,n,k", [(2, 1700, 2048), (8, 16, 512), (9, 130, 14336), (17, 5000, 1024), (25, 1700, 4096), (32, 4097, 1536), (5, 40, 4096), (8, 28672, 512)])
+def test_few_rows(ctx, m, n, k, bits, gs, method):
+    """The kernel of 2 to 32 rows (qmm_rows.cu): every width of its fragments, one step of k and several slices of it, fewer tiles than CTAs, a ragged tile."""
+    check(ctx, m, n, k, bits, gs, method)
+
+
+def test_few_rows_epilogue(ctx):
+    """Accumulate, bias, scale and signed codes, with and without slices of k."""
+    rng = np.random.default_rng(3)
+    for n, k in ((16 * 160, 512), (48, 4096)):
+        d = rng.uniform(-1, 1, (20, n)).astype(np.float32)
+        check(ctx, 20, n, k, 4, 64, "zero", d=d, accumulate=True, bias=f32_to_bf16(rng.uniform(-1, 1, n).astype(np.float32)), ab_scale=0.5)
+        check(ctx, 20, n, k, 8, 64, "symmetric", signed_codes=True)

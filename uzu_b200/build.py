@@ -26,7 +26,7 @@ COMMON = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-st
 SOURCES = {
     "runtime.cu": [],
     "matmul.cu": [],
-    "prefill_gemm.cu": [],
+    "qmm_rows.cu": [],
     "qmm_scaled.cu": [],
     "tp.cu": [],
     "attention.cu": ["-fmad=false"],

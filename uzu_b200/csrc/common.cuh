@@ -102,14 +102,10 @@ inline void launch(uzu_command_buffer* cmd, const char* what, void (*kernel)(KAr
 }
 #endif
 
-// tcgen05 prefill GEMM (prefill_gemm.cu), dispatched from encode_matmul (matmul.cu)
-bool prefill_gemm_applicable(const uzu_matmul_args& a);
-void encode_prefill_gemm(uzu_command_buffer* cmd, const uzu_matmul_args& a);
-
-// quantised products of 2 .. 48 rows (qmm_rows.cu), dispatched from encode_matmul
+// quantised products of 2 .. 32 rows (qmm_rows.cu), dispatched from encode_matmul
 bool qmm_rows_applicable(uzu_command_buffer* cmd, const uzu_matmul_args& a);
 void encode_qmm_rows(uzu_command_buffer* cmd, const uzu_matmul_args& a);
-// quantised products of two and more rows on tcgen05, group scales applied to partial sums (qmm_scaled.cu), dispatched from encode_matmul
+// quantised products of two and more rows on tcgen05 (qmm_scaled.cu), dispatched from encode_matmul
 bool qmm_scaled_applicable(const uzu_matmul_args& a);
 void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a);
 // the device's word for barrier waits that ran out in a tensor-memory product (dense_umma.cu; 0 = none)

@@ -1,6 +1,5 @@
 // Dense (unquantised) prompt GEMM on the 5th-generation tensor cores: D[m, n] (+)= scale * A[m, k] . W[n, k]^T with A and W bf16 in
-// memory, f32 accumulators in tensor memory, f32 output. The dense counterpart of the quantised prefill GEMM (prefill_gemm.cu): same
-// tile shapes, shared-memory layout and barrier protocol, but the producers have nothing to dequantise -- both operand tiles travel by
+// memory, f32 accumulators in tensor memory, f32 output. Nothing to dequantise: both operand tiles travel by
 // cp.async straight into their swizzled stage, several K blocks ahead, and no thread touches the data.
 //
 //   CTA = 128 tokens x 128 features, K in blocks of 64, 3 stages of (16 KB activation tile + 16 KB weight tile): two CTAs share an SM, so one

@@ -1,4 +1,4 @@
-// Quantised MatmulKernel for two and more activation rows on the 5th-generation tensor cores: D[m, n] = epilogue(A[m, k] * dequant(B[n, k])^T).
+// Quantised MatmulKernel for more than 32 activation rows (qmm_rows.cu; other groups: from 3 rows) on the 5th-generation tensor cores: D[m, n] = epilogue(A[m, k] * dequant(B[n, k])^T).
 // Semantic spec: backends/cpu/kernel/matmul/kernel.rs:164-295 (caller encodable_block/linear/matmul.rs:122-148).
 //
 // Weights are turned in the kernel into TWO bf16 planes, hi = bf16(w) and lo = w - hi. For ZeroPoint / Symmetric weights w = scale * (code - zp) has
@@ -514,10 +514,10 @@ bool qmm_scaled_applicable(const uzu_matmul_args& a) {
     const uint32_t gs = a.b_group_size;
     if (a.k == 0 || a.k > (1u << 18) || a.n == 0 || a.k % 64u != 0 || gs < 32 || (gs & (gs - 1)) != 0 || a.k % gs != 0) return false;
     if ((a.a & 15u) || (a.b & 15u)) return false;            // TMA operands (their pitches are multiples of 32 bytes with k a multiple of 64)
-    // up to 8 rows (MLX: 2) the rows kernel of matmul.cu reads the codes faster: a layer of an 8B model, int4, 8 rows 84 us there, 120 here; 9 rows 142
-    // and 121; int8 128 and 166, 227 and 166; MLX 2 rows 150 and 176, 4 rows 199 and 155. It needs whole 512-nibble steps of k.
+    // two rows with groups of 32 or 256 (64 and 128: qmm_rows.cu): the streaming kernel of matmul.cu, which reads whole 512-nibble steps. A layer of an
+    // 8B model, MLX groups of 32: 2 rows 150 us there, 176 here; 4 rows 199 and 155
     const uint32_t bits = a.b_mode == UZU_QMODE_U4 ? 4 : 8;
-    if (a.m <= (a.b_prologue == UZU_B_SCALE_BIAS_DEQUANT ? 2u : 8u) && a.k * bits % 2048u == 0) return false;
+    if (a.m <= 2 && a.k * bits % 2048u == 0) return false;
     // 17 .. 63 rows over a matrix of at most 2^21 weights (about a megabyte, it stays in L2): launches of 16 rows as before (matmul.cu)
     if (a.m > 16 && a.m < 64 && (uint64_t)a.n * a.k <= (1u << 21)) return false;
     return tensor_map_encoder() != nullptr;
@@ -636,3 +636,6 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
 }
 
 }  // namespace uzu
+
+// The descriptor override of a kernel that is gone; the symbol stays in the interface.
+extern "C" void uzu_debug_set_umma(int, uint32_t, uint32_t, uint32_t, uint32_t, int) {}
