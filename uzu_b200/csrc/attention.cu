@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(256) attention_prepare_kernel(const uzu_attent
     }
 }
 
-// Eight neighbouring channels of a (token, head) per thread, 16-byte accesses; the same arithmetic (1024 tokens x 48 heads of 128 took 53 us a
+// Eight neighbouring channels of a (token, head) per thread, 16-byte accesses; the same arithmetic (1024 tokens x 48 heads of 128: 9.5 us, 53 a
 // channel at a time with a CTA per token and head). SEQS: row b belongs to sequence b, with its own cache, position and query row.
 struct NoSequences {};
 template <bool SEQS>

@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(256) gated_act_mul_kernel(const uzu_gated_act_
     reinterpret_cast<__nv_bfloat16*>(a.fp_out)[(size_t)b * a.gated_dim + j] = f2bf(bf2f(value) * bf2f(activated));
 }
 
-// eight neighbouring elements per thread, 16-byte accesses; the same arithmetic (an element at a time 1024 x 14336 took 62 us).
+// eight neighbouring elements per thread, 16-byte accesses; the same arithmetic (1024 x 14336: 20 us, 62 an element at a time).
 __global__ void __launch_bounds__(256) gated_act_mul_vec_kernel(const uzu_gated_act_mul_args a) {
     pdl_launch_dependents();
     pdl_wait();

@@ -10,8 +10,12 @@
 //           256 bytes of codes per row, with their scales and zero points, by cp.async into a ring of the warp's own.
 //   lane    16 consecutive k of a group of 64 for two rows (g, g + 8 of the tile): 8 or 16 bytes of shared memory each, at pitches that spread a
 //           quarter warp over all banks. The products' k order is the lanes' order, the same for both operands.
-// Bound: the codes' way from HBM, then issue slots: a step of 16 features x 64 k is about @INSTR@ instructions, 100 for 8-bit codes.
-// @MEASURED@
+// Bound: the codes' way from HBM, then issue slots: a step of 16 features x 64 k is about 70 instructions, 130 for 8-bit codes.
+// The linears of a layer of an 8B model (115 MB of 4-bit codes, groups of 64), us, with the kernels before it (9 rows and more: qmm_scaled.cu):
+//   rows      2        8        16        24         32
+//   4 bit  60 (84)  61 (85)  77 (122)  105 (126)  122 (126)      at 40 rows 135 (131): the line is at 32
+//   8 bit  85 (124) 87 (128) 102 (162) 119 (164)  139 (167)
+//   MLX    62 (82)  62 (144) 79 (147)  107 (148)  128 (151)
 #include <cstdlib>
 
 #include "common.cuh"

@@ -518,7 +518,7 @@ bool qmm_scaled_applicable(const uzu_matmul_args& a) {
     // 8B model, MLX groups of 32: 2 rows 150 us there, 176 here; 4 rows 199 and 155
     const uint32_t bits = a.b_mode == UZU_QMODE_U4 ? 4 : 8;
     if (a.m <= 2 && a.k * bits % 2048u == 0) return false;
-    // 17 .. 63 rows over a matrix of at most 2^21 weights (about a megabyte, it stays in L2): launches of 16 rows as before (matmul.cu)
+    // 17 .. 63 rows over a matrix of at most 2^21 weights (about a megabyte, it stays in L2): launches of 16 rows (qmm_rows.cu, or matmul.cu for other groups)
     if (a.m > 16 && a.m < 64 && (uint64_t)a.n * a.k <= (1u << 21)) return false;
     return tensor_map_encoder() != nullptr;
 }
