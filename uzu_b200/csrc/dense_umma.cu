@@ -125,7 +125,7 @@ __global__ void __launch_bounds__(DU_NP + 32, 1) dense_umma_kernel(const DenseUm
     __shared__ uint32_t tmem_slot;
     __shared__ uint32_t gave_up;
 
-    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, z = blockIdx.z;   // (warp: uniform for the compiler too)
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31, z = blockIdx.z;   // (warp: the same in every lane)
     constexpr uint32_t kFeatures = EPI == DuPair ? 64u : 128u;        // output features of a CTA
     const uint32_t n0 = blockIdx.x * kFeatures, m0 = blockIdx.y * 128u;
     uint32_t row_begin = 0, rows = p.m;                               // the group's compact rows

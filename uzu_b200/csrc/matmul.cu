@@ -86,13 +86,12 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 // (code_i, code_{i+4}) of a packed word -> bf16x2 holding (128+code_i, 128+code_{i+4}); exact.
 __device__ __forceinline__ uint32_t nib_pair(uint32_t w, int shift) { return ((w >> shift) & 0x000f000fu) | 0x43004300u; }
 
-// Same, tuned for the decode kernel where the integer ALU pipe is the limiter: the shift is a multiply-high
-// (IMAD.HI runs on the FMA pipe, which is otherwise idle) and (x & mask) | magic is forced into ONE LOP3 by keeping
-// the magic constant in a register (ptxas emits two LOP3 when both constants are immediates).
+// Same, tuned for the decode kernel where the integer ALU pipe is the limiter: the shift can be a multiply-high
+// (on the FMA pipe, which is otherwise idle) and (x & mask) | magic is one lop3 with the magic constant in a register.
 #ifndef UZU_QA_SHIFT_MODE
-#define UZU_QA_SHIFT_MODE 1     // 0: every shift on the FMA pipe (IMAD.HI); 1: plain shifts (ALU pipe); 2: shift by 8 on the ALU pipe, 4 / 12 on FMA.
+#define UZU_QA_SHIFT_MODE 1     // 0: every shift on the FMA pipe (multiply-high); 1: plain shifts (ALU pipe); 2: shift by 8 on the ALU pipe, 4 / 12 on FMA.
                                 // Measured (Llama-3-8B linears, B200): mode 1 is 13-19% faster than mode 0 once the kernel is small
-                                // enough not to stall on instruction fetch (IMAD.HI showed up as dispatch stalls in ncu).
+                                // enough not to stall on instruction fetch (mode 0 showed dispatch stalls in ncu's counters).
 #endif
 __device__ __forceinline__ uint32_t nib_pair_fast(uint32_t w, int shift, uint32_t magic_reg) {
     uint32_t sh;
@@ -1171,7 +1170,7 @@ __global__ void __launch_bounds__(QS_WARPS * 32) qmv_decode_async_kernel(const Q
         auto compute = [&](uint32_t slot, uint32_t c0) {
             const uint4* sw = reinterpret_cast<const uint4*>(ring_base + (size_t)slot * QA_STAGE_BYTES) + lane;
             const uint32_t* swd = reinterpret_cast<const uint32_t*>(ring_base + (size_t)slot * QA_STAGE_BYTES + 4096) + lane;
-            // two independent accumulator fragments halve the dependent HMMA chain (32 MMAs per super-chunk)
+            // two independent accumulator fragments halve the chain of dependent products (32 per super-chunk)
             float d[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #if UZU_QA_ACCS == 4
             float d3[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d4[4] = {0.0f, 0.0f, 0.0f, 0.0f};

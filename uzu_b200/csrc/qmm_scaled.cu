@@ -11,8 +11,8 @@
 //              only: a product that reads both operands from shared memory is capped at half of the tensor rate, and that was the bound of the
 //              kernel before this one (128 x 128 tiles; 1024 rows x 28672 x 4096 in 579 us).
 //   one warp each: TMA of the codes (128 rows x 128 bytes, 128B swizzle), TMA of the activations (NT rows x 128 k a stage), and the products
-//              (tcgen05.mma, 8 a block). What one lane issues stands behind elect.sync, which the compiler knows: behind `lane == 0` it
-//              wrapped every tcgen05 instruction in a loop over the active lanes, and the product warp was the bound.
+//              (tcgen05.mma, 8 a block). What one lane issues stands behind elect.sync: there an instruction takes about 10 clocks to issue, behind
+//              `lane == 0` about 300, and the product warp was the bound.
 //   epilogue   four: finished tiles from tensor memory (a feature per lane, a row per column) to D; next to the following tile's products for NT <= 64
 //              (two accumulators).
 // CTAs stay for several tiles; where the tiles do not fill the chip (few rows, few features) a cluster of up to 8 CTAs shares a tile's k and adds
@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
     __shared__ __align__(8) uint64_t bars[2 * CS + 2 * BS + 2 * AS + 2 * ND];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile uint32_t gave_up;
-    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;     // (known to be uniform)
+    const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;     // (warp: the same in every lane)
     const uint32_t base = (qs_smem(qs_raw) + 1023u) & ~1023u;            // swizzle atoms sit on 1024-byte boundaries
     const uint32_t act0 = base, code0 = base + BS * S::ACT, bar0 = qs_smem(bars);
     auto code_full = [&](uint32_t i) { return bar0 + 8u * i; };
