@@ -1,0 +1,35 @@
+"""Kernels started through `launch()` may run under programmatic dependent launch, beside their predecessor: each has to wait for it (pdl_wait)
+before it touches memory. Read from the sources: no GPU can show a missing wait reliably."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "uzu_b200" / "csrc"
+COOPERATIVE = {"decode_mega_kernel"}      # a cooperative launch: stream-ordered, never a dependent one
+KERNEL = re.compile(r"__global__\s+void\s+(?:__cluster_dims__\([^)]*\)\s*)?(?:__launch_bounds__\([^{;]*?\)\s*)?(\w+)\s*\(")
+
+
+def _body(text, at):
+    """the braces that open behind `at`"""
+    start = text.index("{", text.index(")", at))
+    depth = 0
+    for i in range(start, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[start:i + 1]
+    raise AssertionError("unbalanced braces")
+
+
+def _kernels():
+    for path in sorted(CSRC.glob("*.cu")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in KERNEL.finditer(text):
+            # the stream-ordered form <<<..>>> waits for the kernels before it by itself
+            ordered = re.search(rf"\b{m.group(1)}\s*(<[^;(]*>)?\s*<<<", text)
+            yield pytest.param(_body(text, m.end()), bool(ordered) or m.group(1) in COOPERATIVE, id=f"{path.name}-{m.group(1)}")
+
+
+@pytest.mark.parametrize("body,ordered", list(_kernels()))
+def test_kernel_waits_for_its_predecessor(body, ordered):
+    assert ordered or "pdl_wait();" in body or "griddepcontrol.wait" in body

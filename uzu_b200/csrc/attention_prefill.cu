@@ -58,6 +58,7 @@ __device__ __forceinline__ float pa_remote(uint32_t addr, uint32_t rank) {
 
 template <int D>
 __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(const uzu_attention_args a, const uint32_t splits) {
+    pdl_wait();
     constexpr uint32_t LD = D + 8;                  // padded tile row (elements): 16-byte aligned rows, conflict-free ldmatrix
     constexpr uint32_t TILE = PA_BN * LD * 2;       // bytes
     constexpr uint32_t CH = D / 8;                  // 16-byte chunks per row

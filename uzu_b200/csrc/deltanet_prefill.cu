@@ -202,6 +202,8 @@ constexpr int DP_BLOCK = 8;                // tokens per warp: an input is read 
 // units: q heads, k heads, v heads, then one for the gates
 template <int TAPS>
 __global__ void __launch_bounds__(128) delta_net_conv_kernel(const DeltaScanParams s) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uzu_delta_net_update_args& a = s.p.f.update;
     const uzu_delta_net_conv_update_args& c = s.p.f.conv;
     const uint32_t lane = threadIdx.x & 31, rows = s.p.rows;
@@ -274,6 +276,8 @@ __global__ void __launch_bounds__(128) delta_net_conv_kernel(const DeltaScanPara
 
 // a warp per (token, v head); the blocks behind them move the rolling conv state on by the pass's last inputs, a thread per channel
 __global__ void __launch_bounds__(128) delta_net_gate_kernel(const DeltaScanParams s, uint32_t gate_blocks) {
+    pdl_launch_dependents();
+    pdl_wait();
     const uzu_delta_net_update_args& a = s.p.f.update;
     const uzu_delta_net_conv_update_args& c = s.p.f.conv;
     const uint32_t lane = threadIdx.x & 31, conv_dim = 2 * a.key_dim + a.value_dim;

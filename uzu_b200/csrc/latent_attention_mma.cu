@@ -45,6 +45,8 @@ __device__ __forceinline__ void lm_split3(float x0, float x1, uint32_t (&w)[3]) 
 // NB: most 16-column blocks of a quarter of the rank
 template <int NB>
 __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(const uzu_latent_attention_args a) {
+    pdl_launch_dependents();
+    pdl_wait();
     extern __shared__ __align__(16) uint8_t lm_raw[];
     __shared__ float s_part[4][LM_ROWS];
     const uint32_t width = a.rank + a.rot_dim, ld = width + 8, steps = width / 16, nb = a.rank / 64;
