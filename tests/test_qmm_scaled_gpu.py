@@ -83,3 +83,10 @@ def test_few_rows_epilogue(ctx):
         d = rng.uniform(-1, 1, (20, n)).astype(np.float32)
         check(ctx, 20, n, k, 4, 64, "zero", d=d, accumulate=True, bias=f32_to_bf16(rng.uniform(-1, 1, n).astype(np.float32)), ab_scale=0.5)
         check(ctx, 20, n, k, 8, 64, "symmetric", signed_codes=True)
+
+
+@pytest.mark.parametrize("bits,k", [(4, 512), (4, 1536), (8, 256), (8, 768)])
+@pytest.mark.parametrize("n", [1, 33, 4097])
+def test_few_rows_zero_points_that_end_inside_a_word(ctx, bits, k, n):
+    """Groups of 128 over an odd number of steps: a row's zero points are two bytes modulo four, and so is the array with an odd number of rows."""
+    check(ctx, 7, n, k, bits, 128, "zero")

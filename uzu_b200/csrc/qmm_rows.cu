@@ -19,6 +19,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "qmm_rows_index.h"
 
 namespace uzu {
 
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
     uint32_t magic;
     asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
 
-    auto zp_offset = [&](uint32_t row, uint32_t step) { return row * p.zp_stride + (BITS == 4 ? step * NG / 2 : step * NG); };
+    auto zero_fetch = [&](uint32_t row, uint32_t step) { return qr_zero_fetch(row, step, p.n, p.zp_stride, BITS == 4 ? NG / 2 : NG); };
     auto issue_stage = [&](uint32_t tile, uint32_t step, uint32_t slot) {
         const uint32_t dst = ring_s + slot * S::STAGE;
 #pragma unroll
@@ -109,7 +110,10 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
         const uint32_t at = dst + 16 * PITCH + r * 16u;
         const size_t group = (size_t)row * p.groups + step * NG;
         if (lane < 16) qr_cp_async<SB>(at, p.scales + group);
-        else if (kZero) qr_cp_async<4>(at + 256u, p.second + (zp_offset(row, step) & ~3u));
+        else if (kZero) {
+            const QrZeroFetch z = zero_fetch(row, step);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(at + 256u), "l"(p.second + z.offset), "r"(z.bytes) : "memory");
+        }
         else if (kBias) qr_cp_async<SB>(at + 256u, reinterpret_cast<const __nv_bfloat16*>(p.second) + group);
     };
     // the column's (tile, step) pairs in order, an equal run of them for each warp
@@ -239,8 +243,8 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
                 }
             }
             if (kZero && GS == 128) {                                         // two bytes of a word
-                za[0] >>= (zp_offset(min(tile * 16u + g, p.n - 1u), step) & 3u) * 8u;
-                zb[0] >>= (zp_offset(min(tile * 16u + g + 8u, p.n - 1u), step) & 3u) * 8u;
+                za[0] >>= zero_fetch(min(tile * 16u + g, p.n - 1u), step).shift;
+                zb[0] >>= zero_fetch(min(tile * 16u + g + 8u, p.n - 1u), step).shift;
             }
             const uint4* xrow = xs + (size_t)g * xstride + (size_t)(step - s0) * ITEMS + 2 * t;
 #pragma unroll
