@@ -516,8 +516,11 @@ typedef struct uzu_dense_linear_args {
     uint32_t glu_last_group;
 } uzu_dense_linear_args;
 UZU_API void uzu_dense_linear_encode(uzu_command_buffer* cmd, const uzu_dense_linear_args* args);
-/* 0, or the code of the first bounded barrier wait that ran out inside a tensor-memory dense product (the kernel gives up and returns) */
+/* 0, or the code of the last bounded barrier wait that ran out inside a tensor-memory product, dense or quantised: the kernel gives up and returns, and
+ * the host call that waits for it next (of a command buffer, a context or an engine) fails with UZU_ERROR_CUDA */
 UZU_API unsigned int uzu_debug_dense_umma_error(void);
+/* for tests: stores the word that such a kernel stores. 0 takes it back */
+UZU_API void uzu_debug_set_wait_error(uzu_context* ctx, unsigned int code);
 
 /* RMS norm in `groups` equal consecutive parts of a row: part / sqrt(mean(part^2) + epsilon), whole row times scales.
  * input f32 [rows, in_stride] (first n columns), optional row gather, output f32 [rows, out_stride]. groups = 1 is the plain RMS norm.

@@ -1130,6 +1130,7 @@ extern "C" {
     pub fn uzu_debug_set_delta_prefill(mode: c_int);
     pub fn uzu_dense_linear_encode(cmd: *mut uzu_command_buffer, args: *const uzu_dense_linear_args);
     pub fn uzu_debug_dense_umma_error() -> u32;
+    pub fn uzu_debug_set_wait_error(ctx: *mut uzu_context, code: u32);
     pub fn uzu_group_rms_norm_encode(cmd: *mut uzu_command_buffer, args: *const uzu_group_rms_norm_args);
     pub fn uzu_norm_add_encode(cmd: *mut uzu_command_buffer, args: *const uzu_norm_add_args);
     pub fn uzu_stream_mix_encode(cmd: *mut uzu_command_buffer, args: *const uzu_stream_mix_args);

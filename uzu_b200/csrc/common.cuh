@@ -9,6 +9,7 @@
 #include <string>
 
 #include "../../include/uzu_b200.h"
+#include "wait_errors.h"
 
 namespace uzu {
 
@@ -44,6 +45,7 @@ struct uzu_context {
     float* attn_ws = nullptr;
     size_t attn_ws_bytes = 0;
     unsigned int* attn_counters = nullptr;
+    uzu::WaitErrors wait_errors;
     bool vmm_supported = false;
     size_t vmm_granularity = 0;
     // tensor parallelism (tp.cu): NCCL communicator of this process's rank, created by uzu_context_tp_init
@@ -59,7 +61,7 @@ struct uzu_command_buffer {
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr;
     uzu_status sticky = UZU_OK;
     std::string sticky_msg;
-    uint64_t launches = 0;
+    uint64_t launches = 0, number = 0;      // number: of the context's buffers, when encoding starts
     // Programmatic dependent launch for kernels that opt in (set by the engine)
     bool use_pdl = false;
 
@@ -108,8 +110,8 @@ void encode_qmm_rows(uzu_command_buffer* cmd, const uzu_matmul_args& a);
 // quantised products of two and more rows on tcgen05 (qmm_scaled.cu), dispatched from encode_matmul
 bool qmm_scaled_applicable(const uzu_matmul_args& a);
 void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a);
-// the device's word for barrier waits that ran out in a tensor-memory product (dense_umma.cu; 0 = none)
-unsigned int* umma_error_word();
+// fails with the code of a barrier wait that ran out (0: UZU_OK)
+uzu_status wait_error_status(unsigned int code);
 
 // whether a dense product runs on the kernel that can norm its A rows as it stages them (dense_linear.cu)
 bool dense_rows_takes_norm(const uzu_dense_linear_args& a);
@@ -213,6 +215,12 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // reads) before pdl_wait(). Both are no-ops for a normally launched kernel.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// a barrier wait ran out: tell the host (wait_errors.h)
+__device__ __forceinline__ void report_wait_error(unsigned int* word, unsigned int code) {
+    *reinterpret_cast<volatile unsigned int*>(word) = code;
+    __threadfence_system();
+}
 
 __device__ __forceinline__ uint4 ldg_stream_u4(const void* p) {
     uint4 r;

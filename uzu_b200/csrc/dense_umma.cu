@@ -40,8 +40,6 @@ struct DenseUmmaParams {
     unsigned int* error;
 };
 
-__device__ unsigned int g_dense_umma_error = 0;
-
 constexpr uint32_t DU_TILE_BYTES = 128 * 64 * 2;
 constexpr int DU_STAGES = 3;
 constexpr int DU_NP = 128;
@@ -62,16 +60,16 @@ __device__ __forceinline__ bool du_mbar_try_wait(uint32_t bar, uint32_t parity) 
                  : "memory");
     return ok != 0;
 }
-// false when the phase did not complete within ~1 s (the caller gives up)
+// false when the phase did not complete within ~1 s of the preceding kernel's end (the caller gives up)
 __device__ __forceinline__ bool du_mbar_wait(uint32_t bar, uint32_t parity) {
-    if (du_mbar_try_wait(bar, parity)) return true;
-    uint64_t t0;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+    uint64_t t0 = 0;
     uint32_t spins = 0;
     while (!du_mbar_try_wait(bar, parity)) {
         if ((++spins & 1023u) == 0) {
+            if (!t0) pdl_wait();                                 // the time of a kernel that this one depends on does not count
             uint64_t t1;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+            if (!t0) t0 = t1;
             if (t1 - t0 > 1000000000ull) return false;
         }
     }
@@ -164,7 +162,7 @@ __global__ void __launch_bounds__(DU_NP + 32, 1) dense_umma_kernel(const DenseUm
     const uint32_t nkb = p.k >> 6;
     auto fail = [&](uint32_t code) {
         gave_up = 1;
-        atomicCAS(p.error, 0u, code);
+        report_wait_error(p.error, code);
     };
 
     if (warp < (uint32_t)DU_NP / 32u) {
@@ -376,12 +374,6 @@ bool dense_umma_applicable(const uzu_dense_linear_args& a) {
     return true;
 }
 
-unsigned int* umma_error_word() {
-    void* err = nullptr;
-    cudaGetSymbolAddress(&err, g_dense_umma_error);
-    return (unsigned int*)err;
-}
-
 void encode_dense_umma(uzu_command_buffer* cmd, const uzu_dense_linear_args& a) {
     if (!a.a_bf16) {
         const size_t quads = (size_t)a.m * a.k / 4;
@@ -411,7 +403,7 @@ void encode_dense_umma(uzu_command_buffer* cmd, const uzu_dense_linear_args& a) 
     p.k_step = 2;
     // instruction descriptor (kind::f16): f32 accumulate @ 4, bf16 A @ 7, bf16 B @ 10, both K-major, N >> 3 @ [17,23), M >> 4 @ [24,29)
     p.idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-    p.error = umma_error_word();
+    p.error = cmd->ctx->wait_errors.device_word;
     constexpr size_t smem = (size_t)DU_STAGES * DU_STAGE_BYTES + 1024;
     auto go = [&](auto kernel, std::atomic<uint64_t>& opt_in) {
         opt_in_dynamic_smem(cmd, kernel, (int)smem, opt_in);
@@ -426,10 +418,3 @@ void encode_dense_umma(uzu_command_buffer* cmd, const uzu_dense_linear_args& a) 
 }
 
 }  // namespace uzu
-
-// 0 = every tensor-memory GEMM so far completed its barrier waits; otherwise the code of the first wait that ran out
-extern "C" unsigned int uzu_debug_dense_umma_error(void) {
-    unsigned int v = 0;
-    cudaMemcpyFromSymbol(&v, uzu::g_dense_umma_error, sizeof v);
-    return v;
-}

@@ -641,6 +641,7 @@ struct uzu_engine {
     // scratch arena
     Buf shortcut2;   // fused decode path: the residual ping-pongs between `shortcut` and `shortcut2`
     bool fused_ok = false;
+    uint64_t wait_errors_seen = 0;      // barrier waits that ran out and that this engine's calls have reported
     Buf token_ids, hidden_a, hidden_b, shortcut, qkv, queries, attn_out, gate, fused_up, gated, mixer_out, in_proj, delta_out, delta_scratch, normed_out,
         logits, sampled, seeds, tp_parts, tp_sums, tp_maxs;
     Buf host_ring;        // pinned u32[TOKEN_RING]
@@ -2495,8 +2496,9 @@ static void upload_decode_state(uzu_engine* e) {
     try {                                                              \
         cudaSetDevice(e->ctx->device);                                 \
         __VA_ARGS__;                                                   \
-        return UZU_OK;                                                 \
+        return uzu::wait_error_status(e->ctx->wait_errors.since(e->wait_errors_seen)); \
     } catch (const std::exception& ex) {                               \
+        e->ctx->wait_errors.since(e->wait_errors_seen);                \
         return uzu::fail(UZU_ERROR_INVALID_ARGUMENT, ex.what());       \
     }
 
@@ -2506,6 +2508,7 @@ uzu_status uzu_engine_create(uzu_context* ctx, const char* model_dir, const uzu_
     if (!ctx || !model_dir || !out) return fail(UZU_ERROR_INVALID_ARGUMENT, "uzu_engine_create: null argument");
     auto* e = new uzu_engine();
     e->ctx = ctx;
+    e->wait_errors_seen = ctx->wait_errors.found();
     if (opts) e->opts = *opts;
     if (e->opts.tp_size == 0) e->opts.tp_size = 1;
     e->use_pdl = getenv("UZU_NO_PDL") == nullptr;

@@ -22,7 +22,7 @@
 //
 // Bounds, per block and CTA: the tensor pipe 4 NT cycles; the dequant warps about 230 instructions each, four warps a block. Prompts are bound by the
 // tensor pipe (half of its rate is the most two planes can give), few rows by the codes' way: HBM, then the dequant warps' issue slots.
-// Every barrier wait is bounded (about a second): a wait that runs out sets the error word and the CTA ends its work.
+// Every barrier wait is bounded (about a second): a wait that runs out is reported (wait_errors.h: the call then fails on the host) and the CTA ends its work.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -75,18 +75,19 @@ __device__ __forceinline__ bool qs_try(uint32_t bar, uint32_t parity) {
     asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000u) : "memory");
     return ok != 0;
 }
-// false: the phase did not complete within about a second, or another role of the CTA has given up
+// false: the phase did not complete within about a second of the preceding kernel's end, or another role of the CTA has given up
 __device__ __noinline__ bool qs_wait_long(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up, unsigned int* error, uint32_t code) {
     uint64_t t0 = 0;
     for (uint32_t tries = 0; !qs_try(bar, parity); ++tries) {
         if ((tries & 255u) != 255u) continue;                                // (reading the timer is slow)
         if (*gave_up) return false;
+        if (!t0) pdl_wait();                                                 // the time of a kernel that this one depends on does not count
         uint64_t t1;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
         if (!t0) t0 = t1;
         if (t1 - t0 > 1000000000ull) {
             *gave_up = 1;
-            atomicCAS(error, 0u, code);
+            report_wait_error(error, code);
             return false;
         }
     }
@@ -604,7 +605,7 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     p.ab_scale = (a.d_transform & UZU_D_SCALE) ? a.ab_scale : 1.0f;
     p.soft_cap = a.soft_cap;
     p.plain = !p.d_is_f32 && !p.accumulate && !p.has_soft_cap && !p.bias && p.ab_scale == 1.0f;
-    p.error = umma_error_word();
+    p.error = cmd->ctx->wait_errors.device_word;
     p.m = a.m;
     p.d = (void*)a.d;
     uzu_context* ctx = cmd->ctx;

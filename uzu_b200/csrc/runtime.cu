@@ -56,6 +56,15 @@ uzu_status fail(uzu_status st, const std::string& msg) {
     return st;
 }
 
+static std::atomic<unsigned int> g_last_wait_error{0};
+uzu_status wait_error_status(unsigned int code) {
+    if (!code) return UZU_OK;
+    g_last_wait_error = code;
+    char text[112];
+    snprintf(text, sizeof text, "a barrier wait ran out inside a tensor-memory product (code 0x%x): its results are incomplete", code);
+    return fail(UZU_ERROR_CUDA, text);
+}
+
 static void track_alloc(uzu_context* ctx, size_t bytes) {
     ctx->live_bytes += bytes;
     if (ctx->live_bytes > ctx->peak_bytes) ctx->peak_bytes = ctx->live_bytes;
@@ -137,6 +146,9 @@ uzu_status uzu_context_create(int device_ordinal, uzu_context** out) {
     UZU_CUDA_TRY(cudaMalloc(&ctx->attn_ws, ctx->attn_ws_bytes));
     UZU_CUDA_TRY(cudaMalloc(&ctx->attn_counters, 65536 * sizeof(unsigned int)));
     UZU_CUDA_TRY(cudaMemset(ctx->attn_counters, 0, 65536 * sizeof(unsigned int)));
+    UZU_CUDA_TRY(cudaHostAlloc((void**)&ctx->wait_errors.word, sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable));
+    *ctx->wait_errors.word = 0;
+    UZU_CUDA_TRY(cudaHostGetDevicePointer((void**)&ctx->wait_errors.device_word, ctx->wait_errors.word, 0));
     UZU_CUDA_TRY(cudaMalloc(&ctx->sampling_ws, 64 * 1024));
     UZU_CUDA_TRY(cudaMemset(ctx->sampling_ws, 0, 64 * 1024));
     // VMM support (SparseBuffer)
@@ -169,14 +181,26 @@ void uzu_context_destroy(uzu_context* ctx) {
     cudaFree(ctx->sampling_ws);
     cudaFree(ctx->attn_ws);
     cudaFree(ctx->attn_counters);
+    cudaFreeHost(ctx->wait_errors.word);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
 
 uzu_status uzu_context_synchronize(uzu_context* ctx) {
+    const uint64_t before = ctx->wait_errors.found();
     UZU_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-    return UZU_OK;
+    uint64_t seen = before;
+    return wait_error_status(ctx->wait_errors.since(seen));
 }
+
+// what a kernel does whose wait runs out; 0 takes the word and the last code back
+void uzu_debug_set_wait_error(uzu_context* ctx, unsigned int code) {
+    if (!ctx) return;
+    cudaStreamSynchronize(ctx->stream);
+    __atomic_store_n(ctx->wait_errors.word, code, __ATOMIC_RELEASE);
+    if (!code) g_last_wait_error = 0;
+}
+unsigned int uzu_debug_dense_umma_error(void) { return g_last_wait_error; }
 
 uzu_status uzu_context_peak_memory_usage(uzu_context* ctx, size_t* out_bytes) {
     if (!ctx || !out_bytes) return fail(UZU_ERROR_INVALID_ARGUMENT, "peak_memory_usage: null argument");
@@ -368,6 +392,7 @@ uzu_status uzu_command_buffer_start_encoding(uzu_command_buffer* c) {
     if (!c || c->state != uzu_command_buffer::Initial) return fail(UZU_ERROR_INVALID_ARGUMENT, "start_encoding: not Initial");
     UZU_CUDA_TRY(cudaSetDevice(c->ctx->device));
     UZU_CUDA_TRY(cudaEventRecord(c->ev_begin, c->ctx->stream));
+    c->number = c->ctx->wait_errors.start();
     c->state = uzu_command_buffer::Encoding;
     return UZU_OK;
 }
@@ -411,7 +436,7 @@ uzu_status uzu_command_buffer_wait_until_completed(uzu_command_buffer* c) {
     c->state = uzu_command_buffer::Completed;
     if (e != cudaSuccess) return fail(UZU_ERROR_CUDA, std::string("wait_until_completed: ") + cudaGetErrorString(e));
     if (c->sticky != UZU_OK) return fail(c->sticky, c->sticky_msg);
-    return UZU_OK;
+    return wait_error_status(c->ctx->wait_errors.finished(c->number));
 }
 
 uzu_status uzu_command_buffer_gpu_execution_time(uzu_command_buffer* c, double* out_seconds) {
