@@ -85,3 +85,52 @@ def test_batch_resize_frees_sequences_and_recaptures_the_graph(ctx, tmp_path):
         want2 = run(fresh2, 2)
     for a, c in zip(two, want2):
         assert (a == c).all()
+
+
+LENGTHS = [1, 70, 900, 3000]       # one cached row, two splits of the keys, a launch's worth of them, as many as there are
+
+
+@pytest.fixture(scope="module")
+def uneven(tmp_path_factory):
+    spec = synth.tiny("llama")
+    path = synth.write_model(spec, tmp_path_factory.mktemp("uneven") / "m", seed=44)
+    rng = np.random.default_rng(11)
+    prompts = [rng.integers(0, spec.vocab_size, n) for n in LENGTHS]
+    tokens = rng.integers(0, spec.vocab_size, (3, len(LENGTHS)))
+    refs = [OracleModel(path, max_context=4096) for _ in LENGTHS]
+    for r, p in zip(refs, prompts):
+        r.prefill(p)
+    return spec, path, prompts, tokens, [[r.forward([t[b]]) for b, r in enumerate(refs)] for t in tokens]
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_sequences_of_uneven_lengths(ctx, uneven, graph):
+    """Every sequence's keys are cut by its own length: sequences with one split, a few and the most there are share a launch."""
+    _, path, prompts, tokens, want = uneven
+    with B.Engine(ctx, path, max_context_length=4096, use_cuda_graph=graph) as eng:
+        eng.batch_begin(len(prompts))
+        for b, p in enumerate(prompts):
+            eng.batch_prefill(b, p)
+        for step, toks in enumerate(tokens):
+            eng.batch_step(toks)
+            got = eng.batch_logits()
+            for b in range(len(prompts)):
+                _logit_check(got[b:b + 1], want[step][b], f"{LENGTHS[b]} rows, step {step}")
+
+
+def test_a_sequence_does_not_depend_on_its_neighbours_lengths(ctx, uneven):
+    """The same bits beside short and long neighbours, eager and from a graph."""
+    spec, path, _, tokens, _ = uneven
+    rng = np.random.default_rng(12)
+    prompt = rng.integers(0, spec.vocab_size, 300)
+    results = []
+    for graph in (False, True):
+        for others in ((3, 5), (1500, 40), (64, 3000)):
+            with B.Engine(ctx, path, max_context_length=4096, use_cuda_graph=graph) as eng:
+                eng.batch_begin(3)
+                for b, p in enumerate([prompt] + [rng.integers(0, spec.vocab_size, n) for n in others]):
+                    eng.batch_prefill(b, p)
+                for toks in tokens[:, :3]:
+                    eng.batch_step([int(tokens[0, 0])] + [int(t) for t in toks[1:]])
+                results.append(eng.batch_logits()[0].copy())
+    assert all((r == results[0]).all() for r in results)

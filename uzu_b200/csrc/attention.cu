@@ -264,17 +264,19 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     pdl_launch_dependents();
     pdl_wait();
     uzu_attention_args a = p.a;
-    uint32_t keys_per_split = p.keys_per_split;
+    uint32_t keys_per_split = p.keys_per_split, nsplits = p.nsplits;
     if constexpr (SEQS) {
         const uint32_t b = blockIdx.y;
         a.sequence_length = (a.dynamic_position ? reinterpret_cast<const uint32_t*>(a.dynamic_position)[b] : seqs.prefix[b]) + 1u;
         a.keys = seqs.keys[b];
         a.values = seqs.values[b];
         a.queries += (uint64_t)b * a.num_heads * D * 2u;
-        keys_per_split = ((a.sequence_length + p.nsplits - 1) / p.nsplits + 15u) & ~15u;
+        nsplits = min(p.nsplits, (a.sequence_length + 63u) / 64u);      // by its own length alone, as a launch of its own has it
+        if (blockIdx.z >= nsplits) return;
+        keys_per_split = ((a.sequence_length + nsplits - 1) / nsplits + 15u) & ~15u;
     } else if (a.dynamic_position) {
         a.sequence_length = *reinterpret_cast<const uint32_t*>(a.dynamic_position) + a.suffix_length;
-        keys_per_split = ((a.sequence_length + p.nsplits - 1) / p.nsplits + 15u) & ~15u;   // whole CTA steps per split
+        keys_per_split = ((a.sequence_length + nsplits - 1) / nsplits + 15u) & ~15u;   // whole CTA steps per split
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane / LPK, li = lane % LPK, d0 = li * EPL;
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     __syncthreads();
 
     const uint32_t H = a.num_heads;
-    const bool direct = (p.nsplits == 1) && p.fuse_merge;
+    const bool direct = (nsplits == 1) && p.fuse_merge;
     for (int idx = threadIdx.x; idx < G * D; idx += blockDim.x) {
         const int h = idx / D, d = idx % D;
         float ov = 0.0f;
@@ -480,7 +482,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     if (!p.fuse_merge) {
         // caller-visible two-pass buffers have 32 blocks; blocks this launch did not produce are empty
         if (split == 0) {
-            for (uint32_t blk = p.nsplits + warp; blk < p.nb; blk += ATTN_WARPS)
+            for (uint32_t blk = nsplits + warp; blk < p.nb; blk += ATTN_WARPS)
                 for (int h = 0; h < G; ++h) {
                     const size_t o_off = (size_t)out_row * H + head0 + h;
                     for (int d = lane; d < D; d += 32) p.part_o[(o_off * p.nb + blk) * D + d] = 0.0f;
@@ -495,11 +497,11 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     const uint32_t cidx = out_row * gridDim.x + blockIdx.x;
     if (threadIdx.x == 0) sm_ticket = atomicAdd(&p.counters[cidx], 1u);
     __syncthreads();
-    if (sm_ticket != p.nsplits - 1) return;
+    if (sm_ticket != nsplits - 1) return;
     __threadfence();
     for (int h = warp; h < G; h += ATTN_WARPS) {        // one warp per head: split factors and the global sum
         const size_t o_off = (size_t)out_row * H + head0 + h;
-        const bool has = (uint32_t)lane < p.nsplits;
+        const bool has = (uint32_t)lane < nsplits;
         const float mymax = has ? __ldcg(&p.part_max[o_off * p.nb + lane]) : -INFINITY;
         const float gmax = warp_max(mymax);
         const float f = has ? expf(mymax - gmax) : 0.0f;
@@ -515,9 +517,9 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
         float val = 0.0f;
         float pv[32];                                   // all split partials of this output in flight at once
 #pragma unroll
-        for (uint32_t sp = 0; sp < 32; ++sp) pv[sp] = sp < p.nsplits ? __ldcg(po + (size_t)sp * D) : 0.0f;
+        for (uint32_t sp = 0; sp < 32; ++sp) pv[sp] = sp < nsplits ? __ldcg(po + (size_t)sp * D) : 0.0f;
 #pragma unroll
-        for (uint32_t sp = 0; sp < 32; ++sp) val += sp < p.nsplits ? pv[sp] * sc[h][sp] : 0.0f;
+        for (uint32_t sp = 0; sp < 32; ++sp) val += sp < nsplits ? pv[sp] * sc[h][sp] : 0.0f;
         p.final_out[o_off * D + d] = f2bf(val / sm_lfin[h]);
     }
     if (threadIdx.x == 0) p.counters[cidx] = 0;
@@ -639,15 +641,16 @@ static void dispatch_attn(uzu_command_buffer* cmd, const AttnParams& p, const At
     }
 }
 
-// the rows' keys cut over CTAs, merged by the last CTA of a (row, head group)
-static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& a, const AttnSequences* seqs) {
+// the rows' keys cut over CTAs, merged by the last CTA of a (row, head group). Sequences are cut each by its own length (the kernel; a.sequence_length is
+// the most there is): a long one among short ones would otherwise get as few CTAs as they need, and its bits would depend on its neighbours.
+static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& a, const AttnSequences* seqs, float* workspace) {
     uzu_context* ctx = cmd->ctx;
     const int g = pick_group(a.gqa_factor);
     const uint32_t head_groups = a.num_heads / g, rows = seqs ? seqs->count : a.suffix_length;
     // enough CTAs for ~2 waves, >= 64 keys per split, <= 32 splits, and only for short suffixes (decode)
     uint32_t nsplits = 1;
     if (rows <= 16) {
-        const uint32_t ctas = head_groups * rows;
+        const uint32_t ctas = seqs ? head_groups : head_groups * rows;
         const uint32_t want = (2u * (uint32_t)ctx->sm_count + ctas - 1) / ctas;
         const uint32_t cap = (a.sequence_length + 63) / 64;
         nsplits = std::max(1u, std::min(std::min(want, cap), 32u));
@@ -662,7 +665,7 @@ static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& 
     if (nsplits > 1) {
         const size_t units = (size_t)rows * a.num_heads * nsplits;
         const size_t need = units * (a.head_dim + 2) * sizeof(float);
-        if (need > ctx->attn_ws_bytes) {  // grows outside graph capture only (decode needs < 2 MiB)
+        if (!workspace && need > ctx->attn_ws_bytes) {  // grows outside graph capture only (decode needs < 2 MiB)
             cudaStreamSynchronize(ctx->stream);
             cudaFree(ctx->attn_ws);
             if (cudaMalloc(&ctx->attn_ws, need) != cudaSuccess) {
@@ -677,8 +680,8 @@ static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& 
             cmd->record_error(UZU_ERROR_UNSUPPORTED, "attention_single_pass: too many (token, head group) pairs for the split path");
             return;
         }
-        p.part_o = ctx->attn_ws;
-        p.part_sum = ctx->attn_ws + units * a.head_dim;
+        p.part_o = workspace ? workspace : ctx->attn_ws;
+        p.part_sum = p.part_o + units * a.head_dim;
         p.part_max = p.part_sum + units;
         p.counters = ctx->attn_counters;
     }
@@ -701,16 +704,21 @@ bool attention_sequences_applicable(const uzu_attention_prepare_args& p, const u
            !a.has_sinks && attention_prepare_whole_pieces(p) && !(caches & 15u);
 }
 
-void encode_attention_sequences(uzu_command_buffer* cmd, const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s) {
+size_t attention_sequences_workspace_bytes(uint32_t heads, uint32_t head_dim) {
+    return (size_t)kMaxAttnSequences * heads * 32u * (head_dim + 2u) * sizeof(float);
+}
+
+void encode_attention_sequences(uzu_command_buffer* cmd, const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s, uint32_t longest,
+                                uint64_t workspace) {
     if (!encodable(cmd, "attention_sequences")) return;
-    uzu_attention_args longest = a;                                  // the longest sequence decides on the cut
-    longest.keys = s.keys[0];
-    longest.values = s.values[0];
-    for (uint32_t b = 0; b < s.count; ++b) longest.sequence_length = std::max(longest.sequence_length, s.prefix[b] + 1u);
-    if (!attn_common_checks(cmd, &longest, "attention_sequences")) return;
+    uzu_attention_args most = a;
+    most.keys = s.keys[0];
+    most.values = s.values[0];
+    most.sequence_length = longest;
+    if (!attn_common_checks(cmd, &most, "attention_sequences")) return;
     const uint32_t units = (p.num_q_heads + 2 * p.num_kv_heads) * s.count * (p.head_dim / 8u);
     launch(cmd, "attention_prepare_kernel", attention_prepare_vec_kernel<true>, dim3((units + 255u) / 256u), dim3(256), 0, p, s);
-    encode_attn_rows(cmd, longest, &s);
+    encode_attn_rows(cmd, most, &s, reinterpret_cast<float*>(workspace));
 }
 
 }  // namespace uzu
@@ -761,7 +769,7 @@ void uzu_attention_single_pass_encode(uzu_command_buffer* cmd, const uzu_attenti
     if (!uzu::encodable(cmd, "attention_single_pass")) return;
     if (!uzu::attn_common_checks(cmd, a, "attention_single_pass")) return;
     if (uzu::encode_attention_prefill(cmd, *a)) return;   // the tensor-pipe form (attention_prefill.cu)
-    uzu::encode_attn_rows(cmd, *a, nullptr);
+    uzu::encode_attn_rows(cmd, *a, nullptr, nullptr);
 }
 
 void uzu_attention_two_pass1_encode(uzu_command_buffer* cmd, const uzu_attention_args* a) {

@@ -131,7 +131,10 @@ struct AttnSequences {
     uint32_t count;
 };
 bool attention_sequences_applicable(const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s);
-void encode_attention_sequences(uzu_command_buffer* cmd, const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s);
+size_t attention_sequences_workspace_bytes(uint32_t heads, uint32_t head_dim);      // for kMaxAttnSequences of any length
+// longest: no sequence has more cached rows than that, this step's included (with dynamic positions: at any time the launch is repeated)
+void encode_attention_sequences(uzu_command_buffer* cmd, const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s, uint32_t longest,
+                                uint64_t workspace);
 
 // latent attention of a prompt's rows on the tensor pipe (latent_attention_mma.cu)
 bool latent_attention_mma_applicable(const uzu_latent_attention_args& a);

@@ -661,6 +661,7 @@ struct uzu_engine {
     // multi-sequence batched decode (extension, BASELINE config 4 "batch=8"): independent sequence states sharing one weight pass per step
     struct Sequence { std::vector<LayerState> layers; uint32_t context_length = 0; };
     std::vector<Sequence> seqs;
+    Buf batch_attn;                // partial attention results of a batched step, for sequences of any length (a captured step holds its address)
     Buf batch_pos;                 // device u32[16]: per-sequence prefix lengths (the captured batched step reads positions from here)
     bool batch_pos_valid = false;
     cudaGraphExec_t batch_graph = nullptr;
@@ -2877,8 +2878,9 @@ __global__ void batch_step_end_kernel(uint32_t* pos, uint32_t B, const uint32_t*
     }
 }
 
-// `dyn`: positions come from e->batch_pos on the device (CUDA-graph replay); otherwise from the host-side sequence state
-static void encode_batch_step(uzu_engine* e, uzu_command_buffer* cmd, bool dyn) {
+// `dyn`: positions come from e->batch_pos on the device (CUDA-graph replay); otherwise from the host-side sequence state.
+// `longest`: no sequence has more tokens, this step's included, now or when the graph is replayed
+static void encode_batch_step(uzu_engine* e, uzu_command_buffer* cmd, bool dyn, uint32_t longest) {
     const uint32_t B = (uint32_t)e->seqs.size(), H = e->model_dim;
     if (e->in_emb.w.prologue == UZU_B_FULL_PRECISION) {
         uzu_full_precision_embedding_lookup_encode(cmd, e->token_ids.ptr(), e->in_emb.w.values.ptr(), e->hidden_a.ptr(), B, e->vocab, H, e->input_scale);
@@ -2939,7 +2941,7 @@ static void encode_batch_step(uzu_engine* e, uzu_command_buffer* cmd, bool dyn) 
             aa.num_heads = Hq; aa.suffix_length = 1; aa.head_dim = D; aa.is_causal = A.is_causal;
             if (dyn) aa.dynamic_position = e->batch_pos.ptr();
             if (attention_sequences_applicable(pa, aa, seqs)) {
-                encode_attention_sequences(cmd, pa, aa, seqs);
+                encode_attention_sequences(cmd, pa, aa, seqs, longest, e->batch_attn.ptr());
             } else {
                 for (uint32_t b = 0; b < B; ++b) {
                     uzu_attention_prepare_args pb = pa;
@@ -3005,7 +3007,7 @@ static void capture_batch_graph(uzu_engine* e, uint32_t bucket) {
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) throw std::runtime_error("cudaStreamBeginCapture failed");
     g.c->state = uzu_command_buffer::Encoding;
     g.c->use_pdl = e->use_pdl;
-    encode_batch_step(e, g.c, true);
+    encode_batch_step(e, g.c, true, bucket);
     batch_step_end_kernel<<<1, 32, 0, s>>>((uint32_t*)e->batch_pos.ptr(), B, (const uint32_t*)e->sampled.ptr(), (uint32_t*)e->token_ids.ptr());
     g.c->launches++;
     cudaGraph_t graph = nullptr;
@@ -3043,7 +3045,6 @@ static void run_batch_step(uzu_engine* e, bool chain) {
         }
         const uint32_t bucket = attention_bucket(longest);
         if (!e->batch_graph || e->batch_graph_bucket != bucket || e->batch_graph_B != B) {
-            // the capture encodes with the host-side lengths of THIS step (they pick the KV-split geometry of the bucket)
             capture_batch_graph(e, bucket);
         }
         cudaError_t err = cudaGraphLaunch(e->batch_graph, e->ctx->stream);
@@ -3052,7 +3053,7 @@ static void run_batch_step(uzu_engine* e, bool chain) {
     } else {
         CmdGuard g(e->ctx, "batch step");
         g.c->state = uzu_command_buffer::Encoding;
-        encode_batch_step(e, g.c, false);
+        encode_batch_step(e, g.c, false, longest);
         if (g.c->sticky != UZU_OK) throw std::runtime_error(g.c->sticky_msg);
         e->launches += g.c->launches;
         if (chain) cudaMemcpyAsync((void*)e->token_ids.ptr(), (void*)e->sampled.ptr(), B * 4, cudaMemcpyDeviceToDevice, e->ctx->stream);
@@ -3177,6 +3178,10 @@ uzu_status uzu_engine_batch_begin(uzu_engine* e, uint32_t sequences) {
             e->batch_graph = nullptr;
             e->batch_graph_B = 0;
         }
+        size_t attn_bytes = 0;
+        for (auto& L : e->layers)
+            if (L.is_attention) attn_bytes = std::max(attn_bytes, attention_sequences_workspace_bytes(L.attn.num_heads, L.attn.head_dim));
+        if (attn_bytes && !e->batch_attn.b) e->batch_attn = make_buf(e, attn_bytes, UZU_BUFFER_DEVICE);
         while (e->seqs.size() < sequences) {
             e->seqs.emplace_back();
             alloc_sequence_state(e, e->seqs.back().layers);
