@@ -412,6 +412,43 @@ def test_latent_attention_of_prompt_rows(ctx, T, heads, rank, rot, prefix, windo
     close(bo.numpy(np.float32, (T, heads, rank)), ref.numpy(), 1e-5, "latent attention of prompt rows")
 
 
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("T,heads,rank,rot,prefix,window,row", [(20, 3, 128, 16, 5, 0, 24), (40, 16, 512, 64, 0, 0, 7), (33, 5, 320, 32, 130, 40, 100), (64, 1, 64, 0, 70, 70, 66)])
+def test_latent_rows_that_a_token_does_not_see(ctx, T, heads, rank, rot, prefix, window, row, bad):
+    """A cache row that is not finite reaches the tokens that see it and no other: not those before it, not those whose window has left it behind."""
+    rng = np.random.default_rng(T + row)
+    w, n = rank + rot, prefix + T
+    q = rng.standard_normal((T, heads, w), dtype=np.float32)
+    cache = rng.standard_normal((n, w), dtype=np.float32)
+    outs = []
+    for value in (0.5, bad):
+        cache[row] = value
+        bq, bc, bo = ctx.upload(q), ctx.upload(synth.f32_to_bf16_bits(cache)), ctx.upload(np.zeros((T, heads, rank), np.float32))
+        a = B.LatentAttentionArgs(query=bq.ptr, cache=bc.ptr, out=bo.ptr, rows=T, heads=heads, rank=rank, rot_dim=rot, prefix=prefix, cache_dt=B.DT_BF16, scale=w ** -0.5,
+                                  splits=1, window=window)
+        run(ctx, "uzu_latent_attention_encode", C.byref(a))
+        outs.append(bo.numpy(np.float32, (T, heads, rank)))
+    pos = np.arange(prefix, n)
+    sees = (pos >= row) & ((pos - row < window) if window else True)
+    close(outs[1][~sees], outs[0][~sees], 1e-5, "tokens that do not see the row")
+    assert not np.isfinite(outs[1][sees]).all(axis=(1, 2)).any()
+
+
+def test_latent_queries_beyond_the_largest_bf16_number(ctx):
+    """Their leading part is cut off, not rounded to infinity."""
+    T, heads, rank = 16, 2, 64
+    q = np.zeros((T, heads, rank), np.float32)
+    q[..., 0] = 3.4e38
+    cache = np.random.default_rng(2).standard_normal((T, rank), dtype=np.float32)
+    cache[:, 0] = 2.0 ** -126 * np.arange(T)
+    bq, bc, bo = ctx.upload(q), ctx.upload(synth.f32_to_bf16_bits(cache)), ctx.upload(np.zeros((T, heads, rank), np.float32))
+    a = B.LatentAttentionArgs(query=bq.ptr, cache=bc.ptr, out=bo.ptr, rows=T, heads=heads, rank=rank, cache_dt=B.DT_BF16, scale=1.0, splits=1)
+    run(ctx, "uzu_latent_attention_encode", C.byref(a))
+    rows = t64(synth.st_bits_to_f32(synth.f32_to_bf16_bits(cache)))
+    s = torch.einsum("thw,nw->thn", t64(q), rows).masked_fill(~torch.ones(T, T, dtype=torch.bool).tril()[:, None, :], float("-inf"))
+    close(bo.numpy(np.float32, (T, heads, rank))[..., 1:], (torch.softmax(s, -1) @ rows).numpy()[..., 1:], 1e-5, "queries of 3.4e38")
+
+
 def latent_sizes(heads, dim, rot_dim, rank, dims=None, scaling=None, base=10000.0):
     return {"heads": heads, "dim": dim, "rot_dim": rot_dim, "kv_rank": rank, "scale": 0.3,
             "rot": {"dims": dims or rot_dim, "base": base, "scaling": scaling}}

@@ -8,6 +8,8 @@
 //   ldmatrix.trans from the same key tile (a cache row is key and value). The pipe cuts what it adds to an accumulator off at its last bit, so no
 //   chain is longer than four leading products: they are summed by rounded additions. The first half of the next tile is requested while the second half of
 //   this one is multiplied.
+// A weight of zero does not hide a row that is not finite (0 x NaN), so tiles that some row sees in part are looked over first, and one with infinities or
+// NaN is summed key by key for the rows that see them: no token reaches an earlier one, none from before the window comes back.
 // Bound: mma.sync issue, three products per score and sum. 1024 tokens x 16 heads, rank 512 + 64: 0.26 ms (210 TFLOP/s of the three planes) against 1.99 ms with a token and 8 heads per CTA
 // on the FMA pipe; error against 64 bits 2.3e-7 (3.1e-7 there).
 #include "common.cuh"
@@ -40,6 +42,23 @@ __device__ __forceinline__ void lm_split3(float x0, float x1, uint32_t (&w)[3]) 
     }
 }
 
+// The same for a number of any size: beyond bf16's largest one the leading part is cut off instead of rounded, and an infinity has no rest.
+__device__ __forceinline__ uint32_t lm_leading(float& x) {
+    uint32_t h = __bfloat16_as_ushort(__float2bfloat16_rn(x));
+    if ((h & 0x7F80u) == 0x7F80u && x == x) h = __float_as_uint(x) >> 16;
+    x = fabsf(x) == INFINITY ? 0.0f : x - __uint_as_float(h << 16);
+    return h;
+}
+__device__ __forceinline__ void lm_split3_any(float x0, float x1, uint32_t (&w)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const uint32_t lo = lm_leading(x0);
+        w[i] = lo | lm_leading(x1) << 16;
+    }
+}
+// either half of a word is an infinity or NaN
+__device__ __forceinline__ uint32_t lm_not_finite(uint32_t w) { return (uint32_t)((w & 0x7F80u) == 0x7F80u) | (uint32_t)((w & 0x7F800000u) == 0x7F800000u); }
+
 }  // namespace
 
 // NB: most 16-column blocks of a quarter of the rank
@@ -56,6 +75,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
     const uint32_t total = a.rows * a.heads, row0 = (gridDim.x - 1u - blockIdx.x) * LM_ROWS;      // the rows with the most keys first
     const uint32_t last_t = (min(row0 + LM_ROWS, total) - 1u) / a.heads, nkeys = a.prefix + last_t + 1u;
     const uint32_t first_keys = a.prefix + row0 / a.heads + 1u;
+    const uint32_t last_lo = a.window && nkeys > a.window ? nkeys - a.window : 0u;
     const uint32_t t_begin = (a.window && first_keys > a.window ? first_keys - a.window : 0u) / LM_KEYS, t_end = (nkeys + LM_KEYS - 1) / LM_KEYS;
     const __nv_bfloat16* cache = reinterpret_cast<const __nv_bfloat16*>(a.cache);
 
@@ -79,7 +99,7 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
             float2 x = make_float2(0.0f, 0.0f);
             if (row0 + r < total) x = *reinterpret_cast<const float2*>(q + (size_t)r * width + c);
             uint32_t w[3];
-            lm_split3(x.x, x.y, w);
+            lm_split3_any(x.x, x.y, w);
 #pragma unroll
             for (int p = 0; p < 3; ++p) asm volatile("st.shared.u32 [%0], %1;" ::"r"(sq + p * q_plane + (r * ld + c) * 2), "r"(w[p]) : "memory");
         }
@@ -102,7 +122,21 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
 
     for (uint32_t t = t_begin; t < t_end; ++t) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
+        bool key_by_key = false;
+        if ((t + 1) * LM_KEYS > first_keys || t * LM_KEYS < last_lo) {   // not every row sees the whole tile
+            uint32_t bad = 0;
+            const uint32_t pieces = width / 8;
+            for (uint32_t i = tid; i < 64u * pieces; i += LM_THREADS) {  // (what this thread copied)
+                const uint32_t r = i / pieces, c = i % pieces;
+                uint32_t x[4];
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(sk + (r * ld + c * 8) * 2));
+#pragma unroll
+                for (int j = 0; j < 4; ++j) bad |= lm_not_finite(x[j]);
+            }
+            key_by_key = __syncthreads_or((int)bad) != 0;
+        } else {
+            __syncthreads();
+        }
         // ---- scores of 16 rows x 16 keys ----
         float s[2][4], low[2][4];                                        // [8 keys]: the leading plane | the other two
 #pragma unroll
@@ -182,8 +216,37 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
         }
         __syncthreads();
         // ---- weighted sums of 16 rows x a quarter of the rank ----
+        if (key_by_key) {
+            for (uint32_t k = 0; k < LM_KEYS; ++k) {
+                const uint32_t key = t * LM_KEYS + k;
+                const bool sees_a = key < lim_a && key >= lo_a, sees_b = key < lim_b && key >= lo_b;
+                float w_a = 0.0f, w_b = 0.0f;
 #pragma unroll
-        for (uint32_t half = 0; half < 2; ++half) {
+                for (int p = 2; p >= 0; --p) {
+                    uint16_t ha, hb;
+                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(ha) : "r"(sp + p * p_plane + (lr * LM_PLD + k) * 2));
+                    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(hb) : "r"(sp + p * p_plane + ((lr + 8) * LM_PLD + k) * 2));
+                    w_a += bf16_bits_to_f32(ha);
+                    w_b += bf16_bits_to_f32(hb);
+                }
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    if ((uint32_t)b >= nb) continue;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        uint32_t v;
+                        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(sk + (k * ld + share * (a.rank / 4) + b * 16 + h * 8 + 2 * tq) * 2));
+                        const float v0 = __uint_as_float(v << 16), v1 = __uint_as_float(v & 0xFFFF0000u);
+                        if (sees_a) { o[b][h][0] = fmaf(w_a, v0, o[b][h][0]); o[b][h][1] = fmaf(w_a, v1, o[b][h][1]); }
+                        if (sees_b) { o[b][h][2] = fmaf(w_b, v0, o[b][h][2]); o[b][h][3] = fmaf(w_b, v1, o[b][h][3]); }
+                    }
+                }
+            }
+            __syncthreads();
+            if (t + 1 < t_end) load_half(t + 1, 0);
+        }
+#pragma unroll
+        for (uint32_t half = 0; half < 2 && !key_by_key; ++half) {
             if (half) {
                 __syncthreads();                                         // every warp is done with the tile's first 32 keys
                 if (t + 1 < t_end) load_half(t + 1, 0);
