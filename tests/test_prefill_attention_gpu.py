@@ -84,3 +84,30 @@ def test_rows_of_grouped_heads(ctx, H, Hkv, prefix, suffix, D, trie):
     ref = O.attention_single_pass(q, k, v, **kw)
     got = G.attention_single_pass(ctx, q, k, v, **kw)
     assert_bf16_close(got, ref, max_ulp=1, min_exact=0.95, what="grouped rows vs oracle")
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("H,Hkv,prefix,suffix,D,node", [(8, 2, 5, 40, 128, 39), (8, 2, 0, 70, 256, 3), (4, 4, 63, 8, 64, 5), (8, 2, 700, 9, 256, 4)])
+@pytest.mark.parametrize("trie", [False, True])
+def test_rows_that_a_token_does_not_see(ctx, H, Hkv, prefix, suffix, D, node, trie, bad):
+    """A key or value that is not finite reaches the tokens that see it and no other: not those before it, not another branch of a trie."""
+    rng = np.random.default_rng(H + prefix + suffix)
+    if trie:
+        suffix, node = 16, min(node, 7)
+    n = prefix + suffix
+    q = f32_to_bf16(rng.standard_normal((H, suffix, D)).astype(np.float32))
+    k, v = (rng.standard_normal((n, Hkv * D)).astype(np.float32) for _ in range(2))
+    kw = dict(head_dim=D, gqa_factor=H // Hkv, sequence_length=n, k_head_stride=D, k_seq_stride=Hkv * D, v_head_stride=D, v_seq_stride=Hkv * D,
+              scale=float(D ** -0.5), num_heads=H, suffix_length=suffix, is_causal=True)
+    sees = np.arange(suffix) >= node
+    if trie:                                     # a root, and chains of three nodes each below it
+        heights = [0] + [1 + i % 3 for i in range(suffix - 1)]
+        ends = [max(j for j in range(i, suffix) if all(heights[x] > heights[i] for x in range(i + 1, j + 1))) for i in range(suffix)]
+        kw["trie"] = np.array([[i, ends[i], heights[i]] for i in range(suffix)], dtype=np.uint32)
+        sees = (np.arange(suffix) >= node) & (np.arange(suffix) <= ends[node])
+    finite = G.attention_single_pass(ctx, q, f32_to_bf16(k), f32_to_bf16(v), **kw)
+    k[prefix + node, ::7] = bad
+    v[prefix + node] = bad
+    got = G.attention_single_pass(ctx, q, f32_to_bf16(k), f32_to_bf16(v), **kw)
+    assert_bf16_close(got[~sees], finite[~sees], max_ulp=1, min_exact=0.9, what="tokens that do not see the row")
+    assert not np.isfinite(bf16_to_f32(got[sees])).all(axis=(1, 2)).any()

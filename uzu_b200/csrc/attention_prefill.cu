@@ -11,6 +11,8 @@
 //   * online softmax in f32 registers, row statistics over the 4 lanes of a quad; O is rescaled only when some row's maximum moved;
 //   * O += P V with P split into two bf16 planes (hi = bf16(p), lo = bf16(p - hi)): a single rounded plane would put 2^-9 on every
 //     probability; V fragments come from ldmatrix.trans.
+// A weight of zero does not hide a value that is not finite (0 x NaN): value tiles that some row sees in part are looked over first, and one with infinities
+// or NaN is summed key by key for the rows that see them, so that no token reaches an earlier one or another branch of a trie.
 // The next key tile is requested when S is done (it arrives during P V), the next value tile when P V is done: one buffer each, so that two or
 // three CTAs share an SM and fill one another's waits. Causal tiles past the CTA's last query are never loaded, and tiles every row of a
 // warp sees whole are not masked. CTAs with the most keys start first.
@@ -109,6 +111,7 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
     const uint32_t lim1 = r1 < rows ? (!causal ? seq : a.is_trie ? prefix : prefix + n1 + 1) : 0u;
     const uint32_t w_first = row0 + warp * 16, w_last = w_first + 15;        // every row of the warp sees keys below `whole`
     const uint32_t whole = w_last >= rows ? 0u : (!causal ? seq : a.is_trie ? prefix : prefix + w_first / G + 1);
+    const uint32_t cta_whole = !causal ? seq : a.is_trie ? prefix : prefix + row0 / G + 1;      // every row of the CTA sees keys below it
     const bool trie = causal && a.is_trie;
     const uzu_trie_node* nodes = reinterpret_cast<const uzu_trie_node*>(a.trie);
     auto sees = [&](uint32_t key, uint32_t lim, uint32_t node, bool row_ok) {
@@ -199,28 +202,61 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
         m0 = top0;
         m1 = top1;
         asm volatile("cp.async.wait_group 1;" ::: "memory");        // this tile's values have landed
-        __syncthreads();
-        // ---- O += P V: the S accumulator layout IS the A fragment layout of the next MMA (k = key) ----
+        bool key_by_key = false;
+        if ((t + 1) * PA_BN > cta_whole) {
+            uint32_t bad = 0;
+#pragma unroll 4
+            for (uint32_t c = tid; c < PA_BN * CH; c += 128) {       // (what this thread copied)
+                uint32_t x[4];
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(sv + (c / CH * LD + c % CH * 8) * 2));
 #pragma unroll
-        for (int kt = 0; kt < PA_BN / 16; ++kt) {
-            uint32_t ph[4], pl[4];
-            const float* e0 = s[2 * kt];
-            const float* e1 = s[2 * kt + 1];
-            const float pv[8] = {e0[0], e0[1], e0[2], e0[3], e1[0], e1[1], e1[2], e1[3]};
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {   // a0 = (row, k 2t..): e0[0..1]; a1 = (row + 8): e0[2..3]; a2 = (row, k + 8): e1[0..1]; a3: e1[2..3]
-                const float x = pv[2 * r], y = pv[2 * r + 1];
-                ph[r] = pa_pack(x, y);
-                pl[r] = pa_pack(x - __uint_as_float(ph[r] << 16), y - __uint_as_float(ph[r] & 0xffff0000u));
+                for (int j = 0; j < 4; ++j) bad |= (uint32_t)((x[j] & 0x7F80u) == 0x7F80u) | (uint32_t)((x[j] & 0x7F800000u) == 0x7F800000u);
             }
+            key_by_key = __syncthreads_or((int)bad) != 0;
+        } else {
+            __syncthreads();
+        }
+        if (key_by_key) {
+            float w[PA_BN / 8][4];
 #pragma unroll
-            for (int nd = 0; nd < D / 8; nd += 2) {
-                uint32_t vf[4];
-                pa_ldmatrix_x4_trans(vf, v_addr + kt * 16 * LD * 2 + nd * 16);
-                pa_mma(o[nd], ph, vf[0], vf[1]);
-                pa_mma(o[nd + 1], ph, vf[2], vf[3]);
-                pa_mma(o[nd], pl, vf[0], vf[1]);
-                pa_mma(o[nd + 1], pl, vf[2], vf[3]);
+            for (int nt = 0; nt < PA_BN / 8; ++nt) { w[nt][0] = s[nt][0]; w[nt][1] = s[nt][1]; w[nt][2] = s[nt][2]; w[nt][3] = s[nt][3]; }
+#pragma unroll 1
+            for (uint32_t k = 0; k < PA_BN; ++k) {
+                const uint32_t kg = t * PA_BN + k, holder = (lane & ~3u) | ((k & 7u) >> 1);
+                const float w0 = __shfl_sync(0xffffffffu, w[k >> 3][k & 1u], holder), w1 = __shfl_sync(0xffffffffu, w[k >> 3][2 + (k & 1u)], holder);
+                const bool sees0 = sees(kg, lim0, n0, r0 < rows), sees1 = sees(kg, lim1, n1, r1 < rows);
+#pragma unroll
+                for (int nd = 0; nd < D / 8; ++nd) {
+                    uint32_t v;
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(sv + (k * LD + nd * 8 + 2 * tq) * 2));
+                    const float v0 = __uint_as_float(v << 16), v1 = __uint_as_float(v & 0xffff0000u);
+                    if (sees0) { o[nd][0] = fmaf(w0, v0, o[nd][0]); o[nd][1] = fmaf(w0, v1, o[nd][1]); }
+                    if (sees1) { o[nd][2] = fmaf(w1, v0, o[nd][2]); o[nd][3] = fmaf(w1, v1, o[nd][3]); }
+                }
+            }
+        } else {
+            // ---- O += P V: the S accumulator layout IS the A fragment layout of the next MMA (k = key) ----
+#pragma unroll
+            for (int kt = 0; kt < PA_BN / 16; ++kt) {
+                uint32_t ph[4], pl[4];
+                const float* e0 = s[2 * kt];
+                const float* e1 = s[2 * kt + 1];
+                const float pv[8] = {e0[0], e0[1], e0[2], e0[3], e1[0], e1[1], e1[2], e1[3]};
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {   // a0 = (row, k 2t..): e0[0..1]; a1 = (row + 8): e0[2..3]; a2 = (row, k + 8): e1[0..1]; a3: e1[2..3]
+                    const float x = pv[2 * r], y = pv[2 * r + 1];
+                    ph[r] = pa_pack(x, y);
+                    pl[r] = pa_pack(x - __uint_as_float(ph[r] << 16), y - __uint_as_float(ph[r] & 0xffff0000u));
+                }
+#pragma unroll
+                for (int nd = 0; nd < D / 8; nd += 2) {
+                    uint32_t vf[4];
+                    pa_ldmatrix_x4_trans(vf, v_addr + kt * 16 * LD * 2 + nd * 16);
+                    pa_mma(o[nd], ph, vf[0], vf[1]);
+                    pa_mma(o[nd + 1], ph, vf[2], vf[3]);
+                    pa_mma(o[nd], pl, vf[0], vf[1]);
+                    pa_mma(o[nd + 1], pl, vf[2], vf[3]);
+                }
             }
         }
         __syncthreads();                                            // every warp is done with the value tile
