@@ -435,6 +435,25 @@ def test_sampling_filters_count_values(ctx, V, kw):
         assert np.array_equal(ref, G.unified_sampling(ctx, logits, bitmask=bitmask, **kw))
 
 
+@pytest.mark.parametrize("kw", [dict(top_p=float("nan")), dict(top_p=float("nan"), top_k=7), dict(min_p=-1.0), dict(top_p=-0.5), dict(top_p=0.0), dict(top_p=float("inf"), top_k=3)])
+def test_sampling_filters_outside_their_range(ctx, kw):
+    """Limits that compare with nothing (NaN, the logarithm of a negative min_p) keep every element; limits of zero and below keep none."""
+    rng = np.random.default_rng(5)
+    logits = f32_to_bf16((rng.standard_normal((4, 3000)) * 2).astype(np.float32))
+    seeds = rng.integers(0, 2**63, 4, dtype=np.uint64)
+    assert np.array_equal(O.unified_sampling(logits, seeds=seeds, **kw), G.unified_sampling(ctx, logits, seeds=seeds, **kw))
+
+
+@pytest.mark.parametrize("V", [8 * 65535, 8 * 65535 + 1])
+def test_sampling_filters_at_the_largest_counted_vocabulary(ctx, V):
+    """The last vocabulary whose slices fit 16-bit counts, and the first that walks the candidates. All logits alike: one count takes its whole range."""
+    rng = np.random.default_rng(6)
+    seeds = rng.integers(0, 2**63, 1, dtype=np.uint64)
+    for logits in (np.full((1, V), 0x3F80, np.uint16), f32_to_bf16((rng.standard_normal((1, V)) * 3).astype(np.float32))):
+        for kw in (dict(top_k=5), dict(top_k=50, min_p=0.02, temperature=0.7)):
+            assert np.array_equal(O.unified_sampling(logits, seeds=seeds, **kw), G.unified_sampling(ctx, logits, seeds=seeds, **kw)), kw
+
+
 def test_sampling_filters_rows_without_finite_logits(ctx):
     """Everything masked, infinities of both signs: the candidate walk answers as the oracle does."""
     V = 300

@@ -397,7 +397,7 @@ __global__ void __cluster_dims__(SF_CTAS, 1, 1) __launch_bounds__(SF_THREADS, 1)
             if (a.has_top_k) q = rank0 >= a.top_k ? 0u : min(q, a.top_k - rank0);
             if (a.has_top_p) {                       // element i of this value is kept while mass0 + i e < limit
                 const double room = limit - mass0;
-                if (!(room > 0.0)) q = 0;
+                if (room <= 0.0) q = 0;              // (a top_p that is NaN cuts nothing off)
                 else if (e[j] > 0.0 && room < e[j] * (double)q) q = min(q, (uint32_t)ceil(room / e[j]));
             }
             if (a.has_min_p && key_value(key0 + j) * recip_t < min_p_thr) q = 0;
