@@ -198,16 +198,17 @@ typedef struct uzu_fused_linear_args {
      * 2F row the kernel stores hidden[j] = GatedActMul(up_j, gate_j) (act_type) as bf16 [F] into matmul.d. prologue may be 0. */
     uint32_t epilogue, reserved0;
     /* optional decode-stream copy of matmul.b (unit-major 4608-byte units, built by the engine at load; 0 = none): the decode GEMV then feeds
-     * its shared-memory rings with one TMA bulk copy per stage (UBLKCP) instead of per-lane cp.async. With a stream, prologue 0 + epilogue 0
+     * its shared-memory rings with one TMA bulk copy per stage instead of per-lane cp.async. With a stream, prologue 0 + epilogue 0
      * (a plain GEMV over matmul.a) is accepted too. */
     uint64_t decode_stream;
 } uzu_fused_linear_args;
 /* Tuning sweeps only (tools/): override the decode GEMV's work split; 0 = heuristic. Process-wide, not thread-safe. */
 UZU_API void uzu_debug_set_qmv_tuning(int warps_per_tile, int k_slices, int ctas_per_sm, int stages);
 /* Quantized B, bf16 A: 2..32 rows run csrc/qmm_rows.cu (mma.sync, groups of 64 and 128), more rows csrc/qmm_scaled.cu (tcgen05, weights as two
- * exact bf16 planes in tensor memory); UZU_QMM_ROWS=0 / UZU_QMM_SCALED=0 take the kernels for other shapes instead. uzu_debug_set_umma does nothing:
- * it overrode descriptors of an earlier kernel. */
-UZU_API void uzu_debug_set_umma(int layout, uint32_t desc_hi, uint32_t desc_lbo, uint32_t k_step, uint32_t idesc, int mt);
+ * bf16 planes in tensor memory); UZU_QMM_ROWS=0 / UZU_QMM_SCALED=0 take the kernels for other shapes instead. uzu_debug_set_qmm_tile, for tests: the latter's
+ * rows per tile (16, 32, 64, 128, 192, 256) and CTAs that share a tile's k (1, 2, 4, 8; fewer where k is too short), 0 = the plan's own; returns 0 for
+ * other values. Process-wide, not thread-safe. */
+UZU_API int uzu_debug_set_qmm_tile(int rows, int splits);
 UZU_API int uzu_fused_linear_supported(uzu_context* ctx, const uzu_fused_linear_args* args);
 UZU_API void uzu_fused_linear_encode(uzu_command_buffer* cmd, const uzu_fused_linear_args* args);
 

@@ -1,4 +1,4 @@
-"""Parity of the tcgen05 prefill GEMM (uzu_b200/csrc/prefill_gemm.cu, reached through uzu_matmul_encode for m >= 64) against the
+"""Parity of the quantised products of many rows on tcgen05 (uzu_b200/csrc/qmm_scaled.cu, reached through uzu_matmul_encode for m >= 64) against the
 CPU oracle's MatmulKernel restatement (backends/cpu/kernel/matmul/kernel.rs:164-295). Shapes: the reference's quant dispatch matrix
 (quant_dispatch_test.rs:102-167: bits x group x method) at prefill row counts, ragged m / n tails, and the BASELINE layer shapes
 through size-independent properties. Tolerance: BASELINE rtol 1e-3 / atol 1e-4 on f32 outputs, <= 1 bf16 ulp on bf16 outputs."""
@@ -47,15 +47,15 @@ def test_prefill_gemm_bf16_out(ctx, m, n, k, bits, gs, method):
 
 @pytest.mark.parametrize("mt", [1, 2])
 def test_prefill_gemm_token_tile_variants_agree(ctx, mt):
-    """128- and 256-token CTAs (one / two accumulator tiles sharing the dequantised weight tile) give the same bits."""
+    """Tiles of 128 and 256 tokens give the same bits."""
     m, n, k = 384, 256, 512
     x, w, kw = _quant_case(11, m, n, k, 4, 64, O.QM_ZERO_POINT)
     base = G.matmul(ctx, x, w, m=m, n=n, k=k, d_f32=True, **kw)
-    ctx.lib.uzu_debug_set_umma(-1, 0, 0, 0, 0, mt)
+    assert ctx.lib.uzu_debug_set_qmm_tile(128 * mt, 1)
     try:
         got = G.matmul(ctx, x, w, m=m, n=n, k=k, d_f32=True, **kw)
     finally:
-        ctx.lib.uzu_debug_set_umma(-1, 0, 0, 0, 0, 0)
+        ctx.lib.uzu_debug_set_qmm_tile(0, 0)
     assert (got == base).all()
 
 

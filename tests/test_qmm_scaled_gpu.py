@@ -1,11 +1,11 @@
-"""Quantised products of two and more rows on tcgen05 with group scales applied to partial sums (uzu_b200/csrc/qmm_scaled.cu) against the
-oracle's matmul, at the sizes where its tiles, splits and factor look-ahead can go wrong."""
+"""Quantised products of two and more rows (uzu_b200/csrc/qmm_scaled.cu: tcgen05, weights as bf16 planes in tensor memory; qmm_rows.cu: few rows) against
+the oracle's matmul, at the sizes where tiles, splits and factor look-ahead can go wrong."""
 import numpy as np
 import pytest
 
 from oracle import oracle as O
 from tests import gpu_ops as G
-from tests.util import f32_to_bf16
+from tests.util import assert_bf16_close, f32_to_bf16
 
 pytestmark = [pytest.mark.gpu]
 
@@ -50,6 +50,38 @@ def test_edges(ctx, m, n, k):
     """One k block, odd block counts (a code tile that is not full, fewer blocks than the pipeline is deep), rows at both sides of a tile."""
     check(ctx, m, n, k, 4, 64, "zero")
     check(ctx, m, n, k, 8, 32, "zero")
+
+
+@pytest.fixture
+def tile(ctx):
+    yield ctx.lib.uzu_debug_set_qmm_tile
+    ctx.lib.uzu_debug_set_qmm_tile(0, 0)
+
+
+@pytest.mark.parametrize("bits,gs,method", [(4, 64, "zero"), (8, 32, "mlx"), (4, 128, "mlx")])
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+def test_every_tile_and_split(ctx, tile, splits, bits, gs, method):
+    """Every width of a tile with every number of CTAs that share its k, the last of them with a short share; a width changes no bit."""
+    m, n, k = 150, 200, 61 * 64 if gs < 128 else 30 * 128
+    rng = np.random.default_rng(bits + gs)
+    w, kw = weights(rng, n, k, bits, gs, method)
+    x = f32_to_bf16(rng.uniform(-0.5, 0.5, (m, k)).astype(np.float32))
+    outs = []
+    for rows in (16, 32, 64, 128, 192, 256):
+        assert tile(rows, splits)
+        check(ctx, m, n, k, bits, gs, method)
+        outs.append(G.matmul(ctx, x, w, m=m, n=n, k=k, d_f32=True, **kw))
+    assert all((o == outs[0]).all() for o in outs)
+
+
+@pytest.mark.parametrize("bits,gs,method", [(4, 64, "zero"), (8, 64, "symmetric"), (4, 32, "mlx")])
+@pytest.mark.parametrize("m,n,k", [(3, 130, 512), (21, 1700, 1024), (37, 257, 1024), (77, 384, 512), (150, 1000, 320), (300, 128, 512)])
+def test_bf16_outputs(ctx, m, n, k, bits, gs, method):
+    """The rounded sum stored straight from the accumulators: whole and ragged tiles, rows that are no multiple of 16."""
+    rng = np.random.default_rng(m + n)
+    w, kw = weights(rng, n, k, bits, gs, method)
+    x = f32_to_bf16(rng.uniform(-0.5, 0.5, (m, k)).astype(np.float32))
+    assert_bf16_close(G.matmul(ctx, x, w, m=m, n=n, k=k, **kw), O.matmul(x, w, m=m, n=n, k=k, threads=8, **kw), max_ulp=1, min_exact=0.97, what="bf16 rows")
 
 
 def test_more_tiles_than_the_chip_holds(ctx):

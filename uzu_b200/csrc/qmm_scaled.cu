@@ -556,6 +556,8 @@ QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, ui
     return best;
 }
 
+int g_tile_rows = 0, g_tile_splits = 0;      // uzu_debug_set_qmm_tile; 0: the plan's own
+
 template <int BITS, int NT>
 void qs_launch(uzu_command_buffer* cmd, const CUtensorMap& w, const CUtensorMap& x, const QsParams& p, uint32_t grid) {
     static std::atomic<uint64_t> smem_opt_in{0};
@@ -609,7 +611,12 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     p.m = a.m;
     p.d = (void*)a.d;
     uzu_context* ctx = cmd->ctx;
-    const QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, (uint32_t)ctx->sm_count);
+    QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, (uint32_t)ctx->sm_count);
+    if (g_tile_rows) plan.nt = g_tile_rows;
+    if (g_tile_splits) {
+        plan.splits = (uint32_t)g_tile_splits;
+        while (plan.splits > 1 && (((p.nkb + plan.splits - 1) / plan.splits + 3u) & ~3u) * (plan.splits - 1) >= p.nkb) plan.splits /= 2;      // every rank has some
+    }
     p.splits = plan.splits;
     p.split_kb = p.splits == 1 ? p.nkb : ((p.nkb + p.splits - 1) / p.splits + 3u) & ~3u;
     p.m_tiles = (p.m + plan.nt - 1) / plan.nt;
@@ -638,5 +645,10 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
 
 }  // namespace uzu
 
-// The descriptor override of a kernel that is gone; the symbol stays in the interface.
-extern "C" void uzu_debug_set_umma(int, uint32_t, uint32_t, uint32_t, uint32_t, int) {}
+extern "C" int uzu_debug_set_qmm_tile(int rows, int splits) {
+    const bool known = rows == 0 || rows == 16 || rows == 32 || rows == 64 || rows == 128 || rows == 192 || rows == 256;
+    if (!known || (splits != 0 && splits != 1 && splits != 2 && splits != 4 && splits != 8)) return 0;
+    uzu::g_tile_rows = rows;
+    uzu::g_tile_splits = splits;
+    return 1;
+}
