@@ -1,4 +1,4 @@
-"""The arithmetic claims behind the tensor-core prefill GEMM's dequant stage (uzu_b200/csrc/prefill_gemm.cu), checked
+"""The arithmetic claims behind the weight planes of quantised products on tcgen05 (uzu_b200/csrc/qmm_scaled.cu), checked
 exhaustively in numpy (float64 holds every intermediate exactly, so this is a proof over the enumerated domain, not a sample):
 
   1. ZeroPoint / Symmetric weights: w = scale*(code - zp) (what the reference's `scale*code + corr`, corr = -scale*zp, evaluates to in f32,
