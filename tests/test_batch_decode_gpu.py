@@ -1,8 +1,6 @@
-"""Multi-sequence batched decode (extension API uzu_engine_batch_*, BASELINE config 4 "batch = 8"): B independent sequences sharing one pass
+"""Multi-sequence batched decode (extension API uzu_engine_batch_*): B independent sequences sharing one pass
 over the weights per step, against B independent oracle models (the reference decodes one sequence at a time: N independent reference runs
-are the oracle for an N-sequence batch).
-
-First hardware run: round 2 (3 passed, profiles/r2_first_hardware_run.txt)."""
+are the oracle for an N-sequence batch)."""
 import os
 
 import numpy as np

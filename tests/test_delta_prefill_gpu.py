@@ -1,9 +1,5 @@
-"""Multi-token DeltaNet prefill kernel (uzu_b200/csrc/deltanet_prefill.cu: the m-token recurrence of a layer in ONE launch, state
-resident in shared memory) against the oracle's token-by-token DeltaNet (backends/cpu/kernel/gdn/{conv_update,update}.rs restated in C) and
-against the default path (the parity-tested decode kernel launched once per token inside the batched pass).
-
-First hardware run: round 2 (3 passed, profiles/r2_first_hardware_run.txt); the kernel is now the default hybrid prefill recurrence
-(UZU_DELTA_PREFILL_KERNEL=0 restores one decode-kernel launch per token)."""
+"""Multi-token DeltaNet prefill (uzu_b200/csrc/deltanet_prefill.cu: the m-token recurrence of a layer in one to three launches) against the oracle's token-by-token DeltaNet (backends/cpu/kernel/gdn/{conv_update,update}.rs restated in C) and
+against the decode kernel launched once per token inside the batched pass (UZU_DELTA_PREFILL_KERNEL=0)."""
 import os
 
 import numpy as np

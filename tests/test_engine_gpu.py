@@ -51,7 +51,7 @@ def test_teacher_forced_logits(ctx, tmp_path, kind, quant):
 
 @pytest.mark.parametrize("kind,n", [("qwen-hybrid", 21), ("qwen-hybrid-512", 90)])
 def test_hybrid_batched_prefill_matches_token_stepping(ctx, tmp_path, kind, n):
-    """DeltaNet layers in a multi-token pass: projections batched (tensor-core GEMM for >= 64 rows), the recurrence row by row inside
+    """DeltaNet layers in a multi-token pass: projections batched, the recurrence in a few launches over all rows of
     the pass -- the same function as one pass per token (the oracle restates the m = 1 branch, so it steps)."""
     spec = synth.tiny(kind)
     path = synth.write_model(spec, tmp_path / "m", seed=23)

@@ -43,7 +43,7 @@ def test_quantized_matmul_f32_out(ctx, m, n, k, bits, gs, method):
     assert_f32_close(got, ref, rtol=1e-3, atol=1e-4, what=f"matmul {m}x{n}x{k} int{bits} gs{gs} {method}")
 
 
-# shapes the round-1 review found untested against the oracle: the readout matrices of the BASELINE models and int8 gs64 at Llama-3-8B K
+# the readout matrices of the BASELINE models and int8 gs64 at Llama-3-8B K
 BASELINE_SHAPES = [
     (1, 128256, 4096, 4, 64, "zp"),    # Llama-3-8B readout
     (1, 248320, 1024, 4, 64, "zp"),    # Qwen3.5-0.8B readout
@@ -70,7 +70,7 @@ def test_quantized_matmul_baseline_shapes(ctx, m, n, k, bits, gs, method):
     assert_f32_close(got[:, rows], ref, rtol=1e-3, atol=1e-4, what=f"matmul {m}x{n}x{k} int{bits} gs{gs} {method} (sampled rows)")
 
 
-# rows kernel (qmv_rows_kernel, 2..16 activation rows per weight pass: speculation passes, multi-sequence decode): every quantisation
+# few-row products (qmm_rows_kernel, 2..32 activation rows per weight pass: speculation passes, multi-sequence decode): every quantisation
 # method it instantiates, one and two MMA column blocks, k-slices through the split-k workspace, ragged n, several launches (m > 16)
 ROWS_CASES = [
     (2, 64, 512, 4, 64, "zp"), (3, 4096, 4096, 4, 64, "zp"), (8, 6144, 4096, 4, 64, "zp"), (9, 4096, 4096, 4, 64, "zp"),

@@ -443,7 +443,7 @@ def test_delta_net_update_vs_float64():
     np.testing.assert_allclose(bf16_to_f32(out), ref, rtol=1.5e-2, atol=2e-3)
 
 
-# ---- round 2: float64 twins for the remaining thin spots (conv update, two-pass block merge, sigmoid gate, KV-cache update) ----
+# ---- float64 twins for the remaining thin spots (conv update, two-pass block merge, sigmoid gate, KV-cache update) ----
 
 def test_delta_net_conv_update_vs_float64():
     """gdn/conv_update.rs:8-55: out = silu(bias + sum_t state[t] * w[t] + x * w[last]) rounded to bf16; state shifts left and takes x."""

@@ -67,7 +67,7 @@ def _gpu_count():
         return 0
 
 
-@pytest.mark.skipif(_gpu_count() < 2, reason="needs two GPUs (gpurun --gpus 2)")
+@pytest.mark.skipif(_gpu_count() < 2, reason="needs two GPUs")
 @pytest.mark.parametrize("exchange", ["nccl", "p2p"])
 def test_two_rank_nccl_engine_matches_unsharded_oracle(tmp_path, exchange):
     spec = synth.tiny("llama-512")
@@ -129,10 +129,10 @@ def test_two_rank_nccl_engine_matches_unsharded_oracle(tmp_path, exchange):
     assert d["err"] <= 0.02 * d["scale"] + 1e-3 and len(d["tokens"]) == 12, d
 
 
-@pytest.mark.skipif(_gpu_count() < 2, reason="needs two GPUs (gpurun --gpus 2)")
+@pytest.mark.skipif(_gpu_count() < 2, reason="needs two GPUs")
 def test_two_contexts_on_two_devices_in_one_process():
     """cudaFuncAttributeMaxDynamicSharedMemorySize is per (function, device): a second context on another GPU of the same process must be able to
-    launch the > 48 KB shared-memory GEMV too (round 1 kept a per-process flag: the second device's launches failed)."""
+    launch the > 48 KB shared-memory GEMV too: the opt-in is a property of the device, not of the process."""
     from oracle import oracle as O
     from tests import gpu_ops as G
     rng = np.random.default_rng(3)
