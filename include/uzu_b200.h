@@ -225,7 +225,7 @@ UZU_API uint32_t uzu_context_tp_rank(const uzu_context* ctx);
 /* Optional peer-memory exchange for small (decode) messages -- one kernel pushes the partials to every peer over NVLink, waits, reduces in
  * rank order and rounds (csrc/tp.cu: tp_p2p_all_reduce_kernel). Every rank: export (allocates the exchange buffer, returns a 64-byte CUDA IPC
  * handle), all-gather the handles with the host program, import (handles of all ranks, rank order), then a host-side barrier. After that
- * uzu_tp_all_reduce_encode uses the peer path for count <= capacity_f32 and NCCL otherwise. NOT yet run on hardware (round 1). */
+ * uzu_tp_all_reduce_encode uses the peer path for count <= capacity_f32 and NCCL otherwise. */
 UZU_API uzu_status uzu_tp_p2p_export(uzu_context* ctx, uint32_t capacity_f32, uint8_t* handle_out64);
 UZU_API uzu_status uzu_tp_p2p_import(uzu_context* ctx, const uint8_t* handles_size_x_64);
 /* Row-parallel projection epilogue: sum the f32 partials [count] over the ranks in place (ncclAllReduce on the context stream),
@@ -443,9 +443,8 @@ typedef struct uzu_delta_net_fused_update_args {
 } uzu_delta_net_fused_update_args;
 UZU_API int uzu_delta_net_fused_update_supported(const uzu_delta_net_fused_update_args* args);
 UZU_API void uzu_delta_net_fused_update_encode(uzu_command_buffer* cmd, const uzu_delta_net_fused_update_args* args);
-/* Opt-in (UZU_DELTA_PREFILL_KERNEL=1 or uzu_debug_set_delta_prefill(1); -1 = follow the environment): the engine's batched hybrid prefill runs
- * the m-token DeltaNet recurrence of a layer in ONE launch (csrc/deltanet_prefill.cu: one CTA per v-head, state resident in shared memory)
- * instead of one decode-kernel launch per token. NOT yet run on hardware (round 1). */
+/* Whether the engine's passes of several tokens run the DeltaNet recurrence of a layer in a few launches over all tokens (csrc/deltanet_prefill.cu)
+ * or one decode-kernel launch per token: 1 / 0, -1 = follow UZU_DELTA_PREFILL_KERNEL (default 1). */
 UZU_API void uzu_debug_set_delta_prefill(int mode);
 
 /* ---- Kernels of the parallel-block families (Punilix, Gamanex): 32-bit residual stream, dense (unquantised) weights ------------------- *
@@ -970,15 +969,15 @@ UZU_API uzu_status uzu_engine_forward_rows(uzu_engine* e, uint32_t slot, const u
 /* f32 residual stream (the sum of the streams, if there are several) after every layer run of the last pass (models of the parallel-block
  * family; debug / parity): [num_layer_runs, count, model_dim] */
 UZU_API uzu_status uzu_engine_debug_layer_outputs(uzu_engine* e, uint32_t enable, float* out, uint32_t capacity_floats, uint32_t* out_count);
-/* Multi-sequence batched decode (extension -- the reference decodes ONE sequence; BASELINE config 4 "batch = 8"): `sequences` (<= 16)
+/* Multi-sequence batched decode (extension -- the reference decodes ONE sequence): `sequences` (<= 16)
  * independent sequence states (own KV caches / DeltaNet states / positions) advance by one token per step and share one pass over the
- * weights (every linear runs with m = sequences rows); attention and the DeltaNet recurrence run per sequence. Greedy sampling.
+ * weights (every linear runs with m = sequences rows) and one attention launch per layer; the DeltaNet recurrence runs per sequence. Greedy sampling.
  *   batch_begin        allocate / reset the sequence states (the engine's own single-sequence state is untouched)
  *   batch_prefill      ordinary chunked prefill of `tokens` (HOST) into sequence `sequence`; returns its first sampled token
  *   batch_step         tokens_in[sequences] (HOST) -> one step for all sequences -> tokens_out[sequences] (HOST)
  *   batch_decode_timed `steps` device-chained steps from first_tokens[sequences] between two CUDA events; seconds for all of them
  *   batch_logits       bf16 logits [sequences, vocab] of the last step (parity tests)
- * NOT yet run on hardware (round 1): orchestration of the parity-tested kernels, plain stream-ordered launches (no CUDA graph yet). */
+ * With use_cuda_graph the step is captured once per power of two of the longest sequence and replayed. */
 UZU_API uzu_status uzu_engine_batch_begin(uzu_engine* e, uint32_t sequences);
 UZU_API uzu_status uzu_engine_batch_prefill(uzu_engine* e, uint32_t sequence, const uint32_t* tokens, uint32_t count, uint32_t* out_token);
 UZU_API uzu_status uzu_engine_batch_step(uzu_engine* e, const uint32_t* tokens_in, uint32_t* tokens_out);

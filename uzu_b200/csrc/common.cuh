@@ -120,7 +120,7 @@ bool dense_takes_residual(const uzu_dense_linear_args& a);
 // whether a dense product runs on tcgen05 with its operands in tensor memory (dense_umma.cu)
 bool dense_umma_applicable(const uzu_dense_linear_args& a);
 
-// tensor-core prefill attention (attention_prefill.cu, opt-in), tried first by uzu_attention_single_pass_encode
+// tensor-core prefill attention (attention_prefill.cu), tried first by uzu_attention_single_pass_encode
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a);
 
 // One decoded row of several sequences, each with a cache of its own (attention.cu): a launch for all of them instead of one per sequence.

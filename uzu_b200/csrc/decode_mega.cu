@@ -2,7 +2,7 @@
 // LanguageModelStream::next() (engine/language_model/stream/stream.rs:363-782; op order of encodable_block/{decoder.rs:138-203,
 // transformer.rs:226-329, transformer_layer.rs:194-238}) as a program of phases separated by grid barriers.
 //
-// Why: the per-kernel decode step is launch- and ramp-bound (round 1: 137-197 dependent launches of 4-8 us, each restarting the HBM
+// Why: the per-kernel decode step is launch- and ramp-bound (137-197 dependent launches of 4-8 us, each restarting the HBM
 // stream from empty). Here the weight stream never stops:
 //   * one CTA per SM, MK_NCW consumer warps + 1 producer warp. The producer warp walks the CTA's static schedule of weight units
 //     (16 rows x 512 nibbles = 4608 B incl. per-group coefficients) and feeds per-warp shared-memory rings with cp.async.bulk (TMA bulk
@@ -10,7 +10,7 @@
 //     activations, so while the consumers wait at a barrier / stage the next activation row the rings already hold the next
 //     phase's first units (the whole ring of all SMs is ~22 MB: for Qwen3.5-0.8B that is more than a full layer).
 //   * weights are read from a decode-stream copy built once at load (mega_repack_kernel): unit-major, each unit exactly in the order
-//     the consumer lanes read it (conflict-free LDS.128), so a warp's whole range of a matrix is ONE contiguous byte range of HBM.
+//     the consumer lanes read it (conflict-free 16-byte reads), so a warp's whole range of a matrix is ONE contiguous byte range of HBM.
 //   * work partition = "stream-K": the units of a phase are cut into gridDim * MK_NCW equal contiguous ranges (+-1 unit), one per
 //     consumer warp, regardless of tile boundaries. Every (tile, range) intersection leaves a 16-row partial sum ("piece") in a
 //     small f32 workspace; whoever consumes the matmul output sums a tile's pieces in piece order (deterministic), rounds once to

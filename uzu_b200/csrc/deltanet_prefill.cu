@@ -6,7 +6,7 @@
 //                            without a barrier; 128 CTAs for 16 heads of 128 columns;
 //   delta_net_gate_kernel    RMS norm of each head's row, norm weight, SiLU(z), bf16 store; the rolling conv state moves on here, when all
 //                            readers of the old one are done.
-// Bound: the chain of tokens (about 0.2 us each: a dot product over 128 channels, three shuffles, an update), not bytes. As ONE CTA per
+// Bound: latency of the scan (one warp per scheduler walks the tokens, nothing covers its waits), not bytes. As ONE CTA per
 // head with the state in shared memory and ten barriers per token a 509-token pass of 16 heads took 2.87 ms per layer; an 8-layer prompt
 // (6 such layers) 17.7 ms, 3.05 ms now.
 // Same formulas and rounding points as the single-token kernels (this file is built with -fmad=false like deltanet.cu); sums run in another

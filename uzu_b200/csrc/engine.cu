@@ -658,7 +658,7 @@ struct uzu_engine {
     uint32_t tp_rank = 0, tp_size = 1, vocab_local = 0;
     bool tp_sharded = false;       // the checkpoint is a shard: row-parallel partials in f32 + exchange, vocab-parallel readout
     Buf tp_partial, logits_local, tp_gather;
-    // multi-sequence batched decode (extension, BASELINE config 4 "batch=8"): independent sequence states sharing one weight pass per step
+    // multi-sequence batched decode (extension): independent sequence states sharing one weight pass per step
     struct Sequence { std::vector<LayerState> layers; uint32_t context_length = 0; };
     std::vector<Sequence> seqs;
     Buf batch_attn;                // partial attention results of a batched step, for sequences of any length (a captured step holds its address)
@@ -1490,10 +1490,9 @@ static void encode_attention_mix(uzu_engine* e, uzu_command_buffer* cmd, const L
 static uint64_t encode_delta_net(uzu_engine* e, uzu_command_buffer* cmd, const Layer& L, LayerState& S, uint64_t hidden, const PassCtx& pc) {
     const DeltaNetLayer& D = L.dn;
     const uint32_t m = pc.m;
-    // m > 1 (prefill): the two projections run batched over the m rows (tensor-core GEMM for m >= 64); the recurrence itself -- the
-    // rolling conv state and the delta-rule state update -- is the decode branch (delta_net.rs flat m = 1 path) applied row by row in
-    // token order, so a batched prefill computes exactly what m single-token passes compute. (The reference's chunked-prefill core,
-    // Kernels::DeltaNetChunkedPrefill, evaluates the same recurrence in a different summation order; not restated here.)
+    // m > 1 (prefill): the two projections run batched over the m rows, the recurrence over all of them in a few launches
+    // (deltanet_prefill.cu): the decode branch's formulas (delta_net.rs flat m = 1 path) in token order, with sums in another order. Where that
+    // does not apply the decode kernels run row by row. (The reference's chunked-prefill core, Kernels::DeltaNetChunkedPrefill, is not restated.)
     encode_linear(cmd, D.in_proj, hidden, m, e->in_proj.ptr());
     bool whole_pass = false;
     if (m > 1) {   // the m-token recurrence of this layer in a few launches (deltanet_prefill.cu), state kept on chip across tokens
@@ -2186,7 +2185,7 @@ struct MegaBuilder {
                 prev_kind = op.kind;
                 if (op.kind != MK_GEMV) continue;
                 MkStream d{};
-                // parking the prefetch cursor in front of latency-critical phases was measured (round 2): the KV loads did not get faster,
+                // parking the prefetch cursor in front of latency-critical phases was measured: the KV loads did not get faster,
                 // the phase after them lost its prefetch -> off unless UZU_MEGA_HOLD=1
                 static const bool hold_on = [] { const char* v = getenv("UZU_MEGA_HOLD"); return v && atoi(v) != 0; }();
                 d.hold = (hold_on && (before == MK_ATTN || before == MK_DN_UPDATE)) ? 1u : 0u;
@@ -2604,7 +2603,7 @@ uzu_status uzu_engine_prefill(uzu_engine* e, const uint32_t* tokens, uint32_t co
         if (!tokens || count == 0) throw std::runtime_error("prefill: empty prompt");
         if (sampling) e->sampling = *sampling;
         // chunks of <= 1024 (stream.rs:194-195); only the last chunk's last row is sampled. Hybrid (DeltaNet) models take the same
-        // chunks: projections and MLPs batched, the DeltaNet recurrence row by row inside the pass (encode_delta_net).
+        // chunks: projections and MLPs batched, the DeltaNet recurrence in a few launches over all rows (encode_delta_net).
         // UZU_DELTA_PREFILL_STEPPED=1 restores one pass per token (A/B runs).
         static const bool stepped = getenv("UZU_DELTA_PREFILL_STEPPED") != nullptr;
         const uint32_t step = (stepped && has_delta(e)) ? 1 : MAX_ROWS;
@@ -2857,11 +2856,10 @@ uzu_status uzu_engine_step_host(uzu_engine* e, uint32_t token_in, uint32_t* toke
     });
 }
 
-// ---- multi-sequence batched decode (extension; the reference is single-sequence: batch_dim = tokens of ONE sequence, SURVEY 7 hard part 5) ----
+// ---- multi-sequence batched decode (extension; the reference is single-sequence: batch_dim = tokens of ONE sequence) ----
 // B independent sequences (own KV caches / DeltaNet states / positions) advance by one token per step and share ONE pass over the weights:
-// every linear runs with m = B rows (the m <= 16 GEMV streams the matrix once for all rows), norms / activations / embedding / sampling take
-// B rows, only attention and the DeltaNet recurrence run per sequence (their state is per sequence). Plain stream-ordered launches (no CUDA
-// graph yet). NOT yet run on hardware (written after round 1's GPU budget was spent); orchestration of parity-tested kernels only.
+// every linear runs with m = B rows (qmm_rows.cu reads the matrix once for all of them), norms / activations / embedding / sampling take B rows,
+// attention one launch over all caches; only the DeltaNet recurrence runs per sequence. Eager, or captured into a CUDA graph.
 namespace uzu {
 
 struct SeqSwap {   // RAII: make sequence b the engine's current state for code written against e->state / e->context_length

@@ -5,7 +5,7 @@
 //   general_delta_scan_kernel   passes of >= 4 tokens that bring a scratch: decay, rate * unit key and unit key of all tokens are formed in one
 //                               parallel launch first (general_delta_prepare_kernel), then L lanes own a column and walk the tokens, two dot
 //                               products and an update each, no barrier between tokens; the five vectors of a token come from shared memory,
-//                               a batch of tokens ahead by cp.async. Bound: the chain of tokens.
+//                               a batch of tokens ahead by cp.async. Bound: latency that nothing covers (one warp per scheduler).
 //   general_delta_kernel        the decode step and short passes: a CTA keeps a dim x 32 slice of the state in registers -- warp p owns PART
 //                               key channels, lane c owns column c; partial sums meet in shared memory in warp order (a fixed order: one
 //                               token at a time or several in one launch give the same bits).
@@ -148,8 +148,9 @@ __global__ void __launch_bounds__(128) general_delta_prepare_kernel(const uzu_ge
 }
 
 // The tokens of a pass in order over ready-made vectors (decay in decay_logit, rate * unit key in rate_logit, unit key in `unit`): 4 warps per CTA,
-// 32 / L columns per warp, grid (column blocks, heads). Bound: the chain of a token (dot product over the lane's channels, log2 L shuffles, the
-// update). 1024 tokens, 16 heads of 128: 0.37 ms against 1.70 ms as a CTA per 32 columns with three barriers a token.
+// 32 / L columns per warp, grid (column blocks, heads). Bound: latency. 16 heads of 128 are 512 warps on 592 schedulers, and a warp's 20 shared 16-byte
+// reads and its arithmetic of a token take 375 ns with nothing beside them; the dependent part (dot product over the lane's channels, log2 L shuffles, the
+// update) is about a fifth of that. 1024 tokens, 16 heads of 128: 0.37 ms against 1.70 ms as a CTA per 32 columns with three barriers a token.
 constexpr int GS_WARPS = 4;
 template <int L, int NV>
 constexpr int gs_batch() { return L * NV * 4 <= 128 ? 8 : (L * NV * 4 <= 256 ? 4 : 2); }

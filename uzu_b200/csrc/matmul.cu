@@ -771,8 +771,7 @@ __global__ void __launch_bounds__(QS_WARPS * 32) qmv_stream_kernel(const QmvPara
 // lane unpacks only the two (scale, zero-point) pairs of its own chunk: the affine work drops 4x, the
 // accumulator is zeroed once per 4 KB, and the two register buffers ping-pong without copies.
 // -------------------------------------------------------------------------------------------------
-// (The register-pipelined instance of this specialisation, qmv_decode_kernel, was removed in round 2: it was reachable only through
-// UZU_QMV_REGS after the cp.async variant below replaced it; rows too long for the rings take the streaming kernel above.)
+// (Rows too long for the rings of the cp.async variant below take the streaming kernel above.)
 
 // -------------------------------------------------------------------------------------------------
 // cp.async variant of the decode kernel: the same arithmetic, but the weight stream lands in a per-warp

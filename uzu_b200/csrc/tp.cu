@@ -99,8 +99,7 @@ __global__ void __launch_bounds__(256) tp_interleave_rows_kernel(const uint16_t*
 
 
 // ---- one-shot all-reduce over peer memory (NVLink / NVSwitch P2P), for the 8-32 KB decode messages ----------------------------------
-// NOT yet run on hardware (round 1 had no multi-GPU time): enabled only after uzu_tp_p2p_export / uzu_tp_p2p_import succeeded, and
-// the 2-rank test that covers it is opt-in. NCCL stays the default exchange and the fallback for large (prefill) messages.
+// Enabled only after uzu_tp_p2p_export / uzu_tp_p2p_import succeeded. NCCL stays the default exchange and the fallback for large (prefill) messages.
 //
 // Every rank owns an exchange buffer (cudaMalloc, opened by the peers through CUDA IPC):
 //     data [2 slot sets][P ranks][capacity] f32      partials the peers push into this rank
