@@ -413,7 +413,7 @@ def test_latent_attention_of_prompt_rows(ctx, T, heads, rank, rot, prefix, windo
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
-@pytest.mark.parametrize("T,heads,rank,rot,prefix,window,row", [(20, 3, 128, 16, 5, 0, 24), (40, 16, 512, 64, 0, 0, 7), (33, 5, 320, 32, 130, 40, 100), (64, 1, 64, 0, 70, 70, 66)])
+@pytest.mark.parametrize("T,heads,rank,rot,prefix,window,row", [(20, 3, 128, 16, 5, 0, 24), (40, 16, 512, 64, 0, 0, 7), (33, 5, 320, 32, 130, 40, 100), (64, 1, 64, 0, 70, 40, 66)])
 def test_latent_rows_that_a_token_does_not_see(ctx, T, heads, rank, rot, prefix, window, row, bad):
     """A cache row that is not finite reaches the tokens that see it and no other: not those before it, not those whose window has left it behind."""
     rng = np.random.default_rng(T + row)
