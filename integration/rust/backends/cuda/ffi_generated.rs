@@ -1091,6 +1091,7 @@ extern "C" {
     pub fn uzu_matmul_validate(args: *const uzu_matmul_args) -> c_int;
     pub fn uzu_debug_set_qmv_tuning(warps_per_tile: c_int, k_slices: c_int, ctas_per_sm: c_int, stages: c_int);
     pub fn uzu_debug_set_qmm_tile(rows: c_int, splits: c_int) -> c_int;
+    pub fn uzu_debug_set_umma(layout: c_int, desc_hi: u32, desc_lbo: u32, k_step: u32, idesc: u32, mt: c_int);
     pub fn uzu_fused_linear_supported(ctx: *mut uzu_context, args: *const uzu_fused_linear_args) -> c_int;
     pub fn uzu_fused_linear_encode(cmd: *mut uzu_command_buffer, args: *const uzu_fused_linear_args);
     pub fn uzu_tp_get_unique_id(out128: *mut u8) -> c_int;

@@ -51,11 +51,11 @@ def test_prefill_gemm_token_tile_variants_agree(ctx, mt):
     m, n, k = 384, 256, 512
     x, w, kw = _quant_case(11, m, n, k, 4, 64, O.QM_ZERO_POINT)
     base = G.matmul(ctx, x, w, m=m, n=n, k=k, d_f32=True, **kw)
-    assert ctx.lib.uzu_debug_set_qmm_tile(128 * mt, 1)
+    ctx.lib.uzu_debug_set_umma(-1, 0, 0, 0, 0, mt)
     try:
         got = G.matmul(ctx, x, w, m=m, n=n, k=k, d_f32=True, **kw)
     finally:
-        ctx.lib.uzu_debug_set_qmm_tile(0, 0)
+        ctx.lib.uzu_debug_set_umma(-1, 0, 0, 0, 0, 0)
     assert (got == base).all()
 
 

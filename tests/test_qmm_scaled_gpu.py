@@ -61,7 +61,8 @@ def tile(ctx):
 @pytest.mark.parametrize("bits,gs,method", [(4, 64, "zero"), (8, 32, "mlx"), (4, 128, "mlx")])
 @pytest.mark.parametrize("splits", [1, 2, 4, 8])
 def test_every_tile_and_split(ctx, tile, splits, bits, gs, method):
-    """Every width of a tile with every number of CTAs that share its k, the last of them with a short share; a width changes no bit."""
+    """Every width of a tile with every number of CTAs that share its k, the last of them with a short share. A width changes no bit, except
+    that tiles of up to 64 rows add up chains of two blocks."""
     m, n, k = 150, 200, 61 * 64 if gs < 128 else 30 * 128
     rng = np.random.default_rng(bits + gs)
     w, kw = weights(rng, n, k, bits, gs, method)
@@ -71,7 +72,7 @@ def test_every_tile_and_split(ctx, tile, splits, bits, gs, method):
         assert tile(rows, splits)
         check(ctx, m, n, k, bits, gs, method)
         outs.append(G.matmul(ctx, x, w, m=m, n=n, k=k, d_f32=True, **kw))
-    assert all((o == outs[0]).all() for o in outs)
+    assert all((o == outs[0]).all() for o in outs[:3]) and all((o == outs[3]).all() for o in outs[3:])
 
 
 @pytest.mark.parametrize("bits,gs,method", [(4, 64, "zero"), (8, 64, "symmetric"), (4, 32, "mlx")])

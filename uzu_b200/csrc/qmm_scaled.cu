@@ -49,17 +49,19 @@ namespace {
 
 constexpr uint32_t QS_CODE_TILE = 128 * 128;
 
-template <int NT>
+template <int NT, int PL>
 struct QsShape {
-    static constexpr int DG = NT > 128 ? 3 : 4;                              // dequant groups: a block takes one about 2000 cycles, hardly a third of them issuing
+    static constexpr int DG = NT > 128 || NT == 64 || PL == 3 ? 3 : 4;       // dequant groups: a block takes one about 2000 cycles, hardly a third of them issuing
     static constexpr int ND = NT > 64 ? 1 : 2;                               // accumulators in tensor memory
-    static constexpr int AS = NT > 192 ? 4 : NT > 128 ? 5 : 6;               // weight blocks in tensor memory: 64 columns each (hi, lo)
+    static constexpr int CHAIN = NT > 64 ? 0 : 2;                            // blocks whose products share an accumulator (0: all)
+    static constexpr int AS = NT > 192 || PL == 3 ? 4 : NT > 128 ? 5 : 6;    // weight blocks in tensor memory: 32 columns a plane
     static constexpr int BS = NT > 192 ? 2 : NT > 64 ? 3 : 4;                // activation stages of 128 k
     static constexpr int CS = NT > 64 ? 4 : 8;                               // code tiles
     static constexpr int THREADS = (4 + 4 * DG + 3) * 32;
-    static constexpr uint32_t ACT = NT * 256, A_COL = 512 - 64 * AS;
+    static constexpr uint32_t ACT = NT * 256, COLS = 32 * PL, A_COL = 512 - COLS * AS;
     static constexpr size_t SMEM = (size_t)BS * ACT + (size_t)CS * QS_CODE_TILE + 1024;
     static_assert(ND * NT <= (int)A_COL && DG < AS, "tensor memory columns; a group never waits for its own block");
+    static_assert(CHAIN % 2 == 0 && (CHAIN == 0 || ND == 2), "a chain is whole activation stages; the next one runs while its sums are taken");
     static_assert((size_t)NT * 512 <= (size_t)BS * ACT + (size_t)CS * QS_CODE_TILE, "the split-k exchange reuses the rings");
 };
 
@@ -161,17 +163,23 @@ __device__ __forceinline__ void qs_dequant8(uint32_t q, uint32_t zh2, uint32_t z
     hi[0] = __byte_perm(h[0], h[1], 0x5410); hi[1] = __byte_perm(h[0], h[1], 0x7632);
     lo[0] = __byte_perm(l[0], l[1], 0x5410); lo[1] = __byte_perm(l[0], l[1], 0x7632);
 }
-// MLX: the reference's scale * code + bias in f32, then the two planes
-__device__ __forceinline__ void qs_planes_f32(float w0, float w1, uint32_t& hi, uint32_t& lo) {
-    hi = qs_u(__floats2bfloat162_rn(w0, w1));
-    lo = qs_u(__floats2bfloat162_rn(w0 - __uint_as_float(hi << 16), w1 - __uint_as_float(hi & 0xFFFF0000u)));
+// MLX: the reference's scale * code + bias in f32, then its planes: bf16 of what is left, three hold all of it
+template <int PL>
+__device__ __forceinline__ void qs_planes_f32(float w0, float w1, uint32_t (&plane)[PL][16], uint32_t at) {
+#pragma unroll
+    for (int i = 0; i < PL; ++i) {
+        const uint32_t h = qs_u(__floats2bfloat162_rn(w0, w1));
+        plane[i][at] = h;
+        w0 -= __uint_as_float(h << 16);
+        w1 -= __uint_as_float(h & 0xFFFF0000u);
+    }
 }
 
 }  // namespace
 
-template <int BITS, int NT>
-__global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const QsParams p) {
-    using S = QsShape<NT>;
+template <int BITS, int NT, int PL>
+__global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const QsParams p) {
+    using S = QsShape<NT, PL>;
     constexpr int DG = S::DG, ND = S::ND, AS = S::AS, BS = S::BS, CS = S::CS, DQ_WARPS = 4 * DG;
     constexpr uint32_t kpt = BITS == 4 ? 4u : 2u;                            // k blocks per code tile
     extern __shared__ uint8_t qs_raw[];
@@ -233,41 +241,72 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
                 if (p.d_is_f32) reinterpret_cast<float*>(p.d)[at] = val;
                 else reinterpret_cast<__nv_bfloat16*>(p.d)[at] = f2bf(val);
             };
-            const bool ok = qs_wait(d_full(buf), ph, &gave_up, p.error, 0x101u);
-            qs_fence_after();
-            const uint32_t taddr = tmem + ((warp * 32u) << 16) + buf * NT, columns = min((uint32_t)NT, p.m - t0);
+            const uint32_t columns = min((uint32_t)NT, p.m - t0);
+            bool ok = true;
+            float acc[S::CHAIN ? NT : 1];                                // sums of the chains (CHAIN = 0: they stay in tensor memory until they are stored)
+            if constexpr (S::CHAIN != 0) {
+#pragma unroll
+                for (int c = 0; c < NT; ++c) acc[c] = 0.0f;
+            }
+            auto next = [&]() {
+                qs_fence_before();
+                __syncwarp();
+                if (lane == 0) qs_arrive(d_empty(buf));
+                if (++buf == (uint32_t)ND) { buf = 0; ph ^= 1u; }
+            };
+            for (uint32_t i = 0; i < (S::CHAIN ? nk : 1u) && ok; i += S::CHAIN ? S::CHAIN : 1) {
+                ok = qs_wait(d_full(buf), ph, &gave_up, p.error, 0x101u);
+                qs_fence_after();
+                if constexpr (S::CHAIN != 0) {
+#pragma unroll
+                    for (uint32_t c0 = 0; c0 < (uint32_t)NT; c0 += 16) {
+                        if (c0 >= columns || !ok) continue;
+                        uint32_t v[16];
+                        qs_tmem_ld16(tmem + ((warp * 32u) << 16) + buf * NT + c0, v);
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) acc[c0 + j] += __uint_as_float(v[j]);
+                    }
+                    if (ok) next();
+                }
+            }
+            // f(c0, the sums of columns c0 .. c0 + 15) for the tile's columns
+            auto each16 = [&](auto f) {
+                if constexpr (S::CHAIN != 0) {
+#pragma unroll
+                    for (uint32_t c0 = 0; c0 < (uint32_t)NT; c0 += 16)
+                        if (c0 < columns && ok) f(c0, acc + c0);
+                } else {
+                    for (uint32_t c0 = 0; c0 < columns && ok; c0 += 16) {
+                        uint32_t v[16];
+                        qs_tmem_ld16(tmem + ((warp * 32u) << 16) + buf * NT + c0, v);
+                        f(c0, reinterpret_cast<const float*>(v));
+                    }
+                }
+            };
             if (p.splits == 1 && p.plain && item_n(item) + 128u <= p.n) {
                 // D is the rounded sum: a store per column (64 neighbouring bytes a warp), no more than an address step between them
                 __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.d) + (size_t)t0 * p.n + row;
-                uint32_t c0 = 0;
-                for (; c0 + 16 <= columns && ok; c0 += 16) {
-                    uint32_t v[16];
-                    qs_tmem_ld16(taddr + c0, v);
+                each16([&](uint32_t c0, const float* v) {
+                    if (c0 + 16 <= columns) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j, out += p.n) *out = f2bf(__uint_as_float(v[j]));
-                }
-                if (c0 < columns && ok) {
-                    uint32_t v[16];
-                    qs_tmem_ld16(taddr + c0, v);
+                        for (int j = 0; j < 16; ++j, out += p.n) *out = f2bf(v[j]);
+                    } else {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j, out += p.n)
-                        if (c0 + j < columns) *out = f2bf(__uint_as_float(v[j]));
-                }
+                        for (int j = 0; j < 16; ++j, out += p.n)
+                            if (c0 + j < columns) *out = f2bf(v[j]);
+                    }
+                });
             } else if (p.splits == 1) {
-                for (uint32_t c0 = 0; c0 < columns && ok; c0 += 16) {
-                    uint32_t v[16];
-                    qs_tmem_ld16(taddr + c0, v);
+                each16([&](uint32_t c0, const float* v) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) finish(__uint_as_float(v[j]), t0 + c0 + j);
-                }
+                    for (int j = 0; j < 16; ++j) finish(v[j], t0 + c0 + j);
+                });
             } else {
                 // this CTA's tile to shared memory (the rings are idle: every block has been consumed), then column shares over the cluster
-                for (uint32_t c0 = 0; c0 < columns && ok; c0 += 16) {
-                    uint32_t v[16];
-                    qs_tmem_ld16(taddr + c0, v);
+                each16([&](uint32_t c0, const float* v) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) asm volatile("st.shared.u32 [%0], %1;" ::"r"(base + ((c0 + j) * 128u + f) * 4u), "r"(v[j]) : "memory");
-                }
+                    for (int j = 0; j < 16; ++j) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + ((c0 + j) * 128u + f) * 4u), "f"(v[j]) : "memory");
+                });
                 qs_cluster_sync();
                 for (uint32_t j = rank; j < columns && ok; j += p.splits) {
                     float part[8];
@@ -286,16 +325,13 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
                 }
                 break;                                                   // (one item per cluster)
             }
-            qs_fence_before();
-            __syncwarp();
-            if (lane == 0) qs_arrive(d_empty(buf));
             if (!ok) break;
-            if (++buf == (uint32_t)ND) { buf = 0; ph ^= 1u; }
+            if constexpr (S::CHAIN == 0) next();
         }
     } else if (warp < (uint32_t)(4 + DQ_WARPS)) {
         // ================================ codes -> two bf16 planes in tensor memory ================================
         const uint32_t dg = (warp - 4) >> 2, lw = warp & 3u, r = lw * 32u + lane;
-        const bool mlx = p.method == UZU_QMETHOD_SCALE_BIAS, has_zp = p.method == UZU_QMETHOD_SCALE_ZERO_POINT, halves = p.gshift == 5u;
+        const bool mlx = PL == 3 || p.method == UZU_QMETHOD_SCALE_BIAS, has_zp = p.method == UZU_QMETHOD_SCALE_ZERO_POINT, halves = p.gshift == 5u;
         uint32_t turn = 0, stage = dg, a_ph = 1, slot = 0, c_ph = 0;     // whose block it is; this group's next weight block; code tile
         bool ok = true;
         for (uint32_t item = item0; item < p.items && ok; item += item_step) {
@@ -333,10 +369,10 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
                         f_next[0] = factor(k0);
                         f_next[1] = halves ? factor(k0 + 32u) : f_next[0];
                     }
-                    const uint32_t t_col = tmem + ((lw * 32u) << 16) + S::A_COL + stage * 64u;
+                    const uint32_t t_col = tmem + ((lw * 32u) << 16) + S::A_COL + stage * S::COLS;
 #pragma unroll
                     for (uint32_t h = 0; h < 2; ++h) {                   // 32 k at a time
-                        uint32_t hi[16], lo[16];
+                        uint32_t plane[PL][16], (&hi)[16] = plane[0], (&lo)[16] = plane[1];
                         const uint32_t s1 = f_cur[h] & 0xFFFFu, z = f_cur[h] >> 16, s2 = s1 * 0x00010001u;
                         if constexpr (BITS == 4) {
                             uint32_t q[4];
@@ -350,7 +386,7 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
 #pragma unroll
                                 for (int i = 0; i < 16; ++i) {           // pair i: nibbles 2 (i & 3), + 1 of word i / 4
                                     const uint32_t w = (q[i >> 2] ^ p.xor_mask) >> (8 * (i & 3));
-                                    qs_planes_f32(fmaf(s, (float)(w & 15u), c), fmaf(s, (float)((w >> 4) & 15u), c), hi[i], lo[i]);
+                                    qs_planes_f32<PL>(fmaf(s, (float)(w & 15u), c), fmaf(s, (float)((w >> 4) & 15u), c), plane, i);
                                 }
                             }
                         } else {
@@ -367,7 +403,7 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
 #pragma unroll
                                     for (int i = 0; i < 8; ++i) {
                                         const uint32_t w = (q[i >> 1] ^ p.xor_mask) >> (16 * (i & 1));
-                                        qs_planes_f32(fmaf(s, (float)(w & 255u), c), fmaf(s, (float)((w >> 8) & 255u), c), hi[8 * i2 + i], lo[8 * i2 + i]);
+                                        qs_planes_f32<PL>(fmaf(s, (float)(w & 255u), c), fmaf(s, (float)((w >> 8) & 255u), c), plane, 8 * i2 + i);
                                     }
                                 }
                             }
@@ -377,8 +413,8 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
                             if (!ok) break;
                             qs_fence_after();
                         }
-                        qs_tmem_st16(t_col + h * 16u, hi);
-                        qs_tmem_st16(t_col + 32u + h * 16u, lo);
+#pragma unroll
+                        for (int i = 0; i < PL; ++i) qs_tmem_st16(t_col + 32u * i + h * 16u, plane[i]);
                     }
                     if (!ok) break;
                     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -440,9 +476,11 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
             const uint32_t desc_lo = (act0 >> 4) | (1u << 16);
             uint32_t bs = 0, bs_ph = 0, as = 0, as_ph = 0, buf = 0, d_ph = 1;
             for (uint32_t item = item0; item < p.items && ok; item += item_step) {
-                ok = qs_wait(d_empty(buf), d_ph, &gave_up, p.error, 0x108u);
-                const uint32_t d = tmem + buf * NT;
                 for (uint32_t i = 0; i < nk && ok; i += 2) {
+                    const bool begins = S::CHAIN ? i % (S::CHAIN ? S::CHAIN : 1) == 0 : i == 0, ends = i + 2 >= nk || (S::CHAIN && (i + 2) % (S::CHAIN ? S::CHAIN : 1) == 0);
+                    const uint32_t d = tmem + buf * NT;
+                    if (begins) ok = qs_wait(d_empty(buf), d_ph, &gave_up, p.error, 0x108u);
+                    if (!ok) break;
                     ok = qs_wait(act_full(bs), bs_ph, &gave_up, p.error, 0x106u);
                     if (!ok) break;
 #pragma unroll
@@ -452,11 +490,11 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
                         if (!ok) break;
                         qs_fence_after();
                         if (qs_elect()) {
-                            const uint32_t a_col = tmem + S::A_COL + as * 64u, lo = desc_lo + (bs * S::ACT + half * (S::ACT / 2) >> 4);
+                            const uint32_t a_col = tmem + S::A_COL + as * S::COLS, lo = desc_lo + (bs * S::ACT + half * (S::ACT / 2) >> 4);
 #pragma unroll
                             for (uint32_t kk = 0; kk < 4; ++kk) {
-                                qs_mma(d, a_col + kk * 8u, desc_hi | (lo + kk * 2u), idesc, (i | half | kk) != 0 ? 1u : 0u);
-                                qs_mma(d, a_col + 32u + kk * 8u, desc_hi | (lo + kk * 2u), idesc, 1u);
+#pragma unroll
+                                for (uint32_t pl = 0; pl < (uint32_t)PL; ++pl) qs_mma(d, a_col + 32u * pl + kk * 8u, desc_hi | (lo + kk * 2u), idesc, !begins || (half | kk | pl) != 0 ? 1u : 0u);
                             }
                             qs_commit(a_empty(as));
                         }
@@ -467,11 +505,11 @@ __global__ void __launch_bounds__(QsShape<NT>::THREADS, 1) qmm_scaled_kernel(con
                     if (qs_elect()) qs_commit(act_empty(bs));
                     __syncwarp();
                     if (++bs == (uint32_t)BS) { bs = 0; bs_ph ^= 1u; }
+                    if (!ends) continue;
+                    if (qs_elect()) qs_commit(d_full(buf));
+                    __syncwarp();
+                    if (++buf == (uint32_t)ND) { buf = 0; d_ph ^= 1u; }
                 }
-                if (!ok) break;
-                if (qs_elect()) qs_commit(d_full(buf));
-                __syncwarp();
-                if (++buf == (uint32_t)ND) { buf = 0; d_ph ^= 1u; }
             }
         }
         __syncwarp();
@@ -507,7 +545,8 @@ static bool tensor_map(CUtensorMap* map, CUtensorMapDataType type, uint64_t addr
 
 bool qmm_scaled_applicable(const uzu_matmul_args& a) {
     static const bool off = [] { const char* e = getenv("UZU_QMM_SCALED"); return e && atoi(e) == 0; }();      // 0: the kernels for other shapes (A/B runs)
-    if (off || a.m < 2) return false;
+    static const int min_rows = [] { const char* e = getenv("UZU_PREFILL_GEMM_MIN_M"); return e ? atoi(e) : 2; }();      // fewer rows take the other kernels; 0: all do
+    if (off || min_rows <= 0 || a.m < 2 || a.m < (uint32_t)min_rows) return false;
     if (a.b_prologue == UZU_B_FULL_PRECISION || a.gather_indices || !a.b_transpose) return false;
     if (a.input_dt != UZU_DT_BF16 || a.weights_dt != UZU_DT_BF16) return false;
     if (a.output_dt != UZU_DT_BF16 && a.output_dt != UZU_DT_F32) return false;
@@ -519,8 +558,8 @@ bool qmm_scaled_applicable(const uzu_matmul_args& a) {
     // 8B model, MLX groups of 32: 2 rows 150 us there, 176 here; 4 rows 199 and 155
     const uint32_t bits = a.b_mode == UZU_QMODE_U4 ? 4 : 8;
     if (a.m <= 2 && a.k * bits % 2048u == 0) return false;
-    // 17 .. 63 rows over a matrix of at most 2^21 weights (about a megabyte, it stays in L2): launches of 16 rows (qmm_rows.cu, or matmul.cu for other groups)
-    if (a.m > 16 && a.m < 64 && (uint64_t)a.n * a.k <= (1u << 21)) return false;
+    // 17 .. 63 rows over a matrix of at most 2^21 weights with groups of 64 or 128: launches of 16 rows (qmm_rows.cu)
+    if (a.m > 16 && a.m < 64 && (uint64_t)a.n * a.k <= (1u << 21) && (gs == 64 || gs == 128)) return false;
     return tensor_map_encoder() != nullptr;
 }
 
@@ -530,14 +569,14 @@ struct QsPlan { int nt = 0; uint32_t splits = 1; float cost = 1e30f; };
 
 // Cycles of one CTA per 64 k of a tile, as measured: a product takes about 64 cycles however few its rows are and the product warp's waits come on top
 // (16 rows 850, 128 rows 940), wide tiles run at the tensor pipe (256 rows 1240); MLX and 8-bit codes keep the dequant warps busier than that.
-float qs_block_cycles(int nt, uint32_t bits, bool mlx) {
-    const float products = std::max(850.0f + 0.7f * nt, 4.85f * nt), turn = mlx ? 4000.0f : bits == 4 ? 2000.0f : 2800.0f;
-    return std::max(products, turn / (nt > 128 ? 3.0f : 4.0f));
+float qs_block_cycles(int nt, uint32_t bits, bool mlx, bool three) {
+    const float products = std::max(850.0f + 0.7f * nt, 4.85f * nt) * (three ? 1.5f : 1.0f), turn = mlx ? 4000.0f : bits == 4 ? 2000.0f : 2800.0f;
+    return std::max(products, turn / (nt > 128 || nt == 64 || three ? 3.0f : 4.0f));
 }
 
 // Rows per tile and CTAs per tile: the shortest estimated time over the chip. A wider tile turns its codes once for more rows; a narrower one or a
 // split k fills the chip where tiles are few. Fixed cost per item: filling the pipeline and storing the tile.
-QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, uint32_t sms) {
+QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, bool three, uint32_t sms) {
     QsPlan best;
     const uint32_t n_tiles = (n + 127u) / 128u;
     for (int nt : {16, 32, 64, 128, 192, 256}) {
@@ -547,7 +586,7 @@ QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, ui
         for (uint32_t splits = 1; splits <= 8; splits *= 2) {
             const uint32_t per = ((nkb + splits - 1) / splits + 3u) & ~3u;           // whole code tiles per rank
             if (splits > 1 && (per * (splits - 1) >= nkb || tiles * splits > sms)) break;
-            const float item = (float)std::min(per, nkb) * qs_block_cycles(nt, bits, mlx) + 2500.0f + (nt > 64 ? 12.0f * nt : 0.0f) + (splits > 1 ? 1500.0f + 8.0f * nt : 0.0f);
+            const float item = (float)std::min(per, nkb) * qs_block_cycles(nt, bits, mlx, three) + 2500.0f + (nt > 64 ? 12.0f * nt : 0.0f) + (splits > 1 ? 1500.0f + 8.0f * nt : 0.0f);
             const uint32_t waves = (tiles * splits + sms - 1) / sms;
             const float cost = waves * item;
             if (cost < best.cost) best = {nt, splits, cost};
@@ -558,14 +597,14 @@ QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, ui
 
 int g_tile_rows = 0, g_tile_splits = 0;      // uzu_debug_set_qmm_tile; 0: the plan's own
 
-template <int BITS, int NT>
+template <int BITS, int NT, int PL>
 void qs_launch(uzu_command_buffer* cmd, const CUtensorMap& w, const CUtensorMap& x, const QsParams& p, uint32_t grid) {
     static std::atomic<uint64_t> smem_opt_in{0};
-    opt_in_dynamic_smem(cmd, qmm_scaled_kernel<BITS, NT>, (int)QsShape<NT>::SMEM, smem_opt_in);
+    opt_in_dynamic_smem(cmd, qmm_scaled_kernel<BITS, NT, PL>, (int)QsShape<NT, PL>::SMEM, smem_opt_in);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(QsShape<NT>::THREADS);
-    cfg.dynamicSmemBytes = QsShape<NT>::SMEM;
+    cfg.blockDim = dim3(QsShape<NT, PL>::THREADS);
+    cfg.dynamicSmemBytes = QsShape<NT, PL>::SMEM;
     cfg.stream = cmd->ctx->stream;
     cudaLaunchAttribute attr[2];
     if (cmd->use_pdl) {
@@ -579,7 +618,7 @@ void qs_launch(uzu_command_buffer* cmd, const CUtensorMap& w, const CUtensorMap&
         attr[cfg.numAttrs++].val.clusterDim.z = 1;
     }
     cfg.attrs = attr;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, qmm_scaled_kernel<BITS, NT>, w, x, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, qmm_scaled_kernel<BITS, NT, PL>, w, x, p);
     if (e != cudaSuccess) cmd->record_error(UZU_ERROR_CUDA, std::string("matmul qmm_scaled_kernel: ") + cudaGetErrorString(e));
     cmd->launches++;
 }
@@ -611,7 +650,9 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     p.m = a.m;
     p.d = (void*)a.d;
     uzu_context* ctx = cmd->ctx;
-    QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, (uint32_t)ctx->sm_count);
+    // MLX weights of passes that the kernels before this one summed with the codes as integers keep all their bits; longer ones had two planes always
+    const bool three = p.biases && p.m < 64;
+    QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, three, (uint32_t)ctx->sm_count);
     if (g_tile_rows) plan.nt = g_tile_rows;
     if (g_tile_splits) {
         plan.splits = (uint32_t)g_tile_splits;
@@ -631,12 +672,12 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     auto go = [&](auto bits_c) {
         constexpr int BITS = decltype(bits_c)::value;
         switch (plan.nt) {
-            case 16: qs_launch<BITS, 16>(cmd, mw, mx, p, grid); break;
-            case 32: qs_launch<BITS, 32>(cmd, mw, mx, p, grid); break;
-            case 64: qs_launch<BITS, 64>(cmd, mw, mx, p, grid); break;
-            case 128: qs_launch<BITS, 128>(cmd, mw, mx, p, grid); break;
-            case 192: qs_launch<BITS, 192>(cmd, mw, mx, p, grid); break;
-            default: qs_launch<BITS, 256>(cmd, mw, mx, p, grid); break;
+            case 16: three ? qs_launch<BITS, 16, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 16, 2>(cmd, mw, mx, p, grid); break;
+            case 32: three ? qs_launch<BITS, 32, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 32, 2>(cmd, mw, mx, p, grid); break;
+            case 64: three ? qs_launch<BITS, 64, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 64, 2>(cmd, mw, mx, p, grid); break;
+            case 128: qs_launch<BITS, 128, 2>(cmd, mw, mx, p, grid); break;
+            case 192: qs_launch<BITS, 192, 2>(cmd, mw, mx, p, grid); break;
+            default: qs_launch<BITS, 256, 2>(cmd, mw, mx, p, grid); break;
         }
     };
     if (bits == 4) go(std::integral_constant<int, 4>{});
@@ -644,6 +685,9 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
 }
 
 }  // namespace uzu
+
+// mt: 1, 2: tiles of 128, 256 rows; 0: the plan's own. (The others described operands of an earlier kernel.)
+extern "C" void uzu_debug_set_umma(int, uint32_t, uint32_t, uint32_t, uint32_t, int mt) { uzu::g_tile_rows = mt == 1 ? 128 : mt == 2 ? 256 : 0; }
 
 extern "C" int uzu_debug_set_qmm_tile(int rows, int splits) {
     const bool known = rows == 0 || rows == 16 || rows == 32 || rows == 64 || rows == 128 || rows == 192 || rows == 256;
