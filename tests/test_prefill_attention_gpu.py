@@ -2,8 +2,7 @@
 AttentionSinglePass restatement (backends/cpu/kernel/attention/attention_single_pass.rs:49-126) and the independent float64 softmax of
 tests/unit/encodable_block/attention_test.rs:26-124, on the reference tests' closed-form inputs (attention_single_pass_test.rs:33-78).
 
-First hardware run of these tests: round 2 (7 passed, profiles/r2_first_hardware_run.txt); since then the kernel is the default prefill
-attention for head_dim 64 / 128 (UZU_PREFILL_ATTN=0 restores the split-KV kernel applied per query token)."""
+UZU_PREFILL_ATTN=0 takes the split-KV kernel for every pass."""
 import os
 
 import numpy as np
@@ -61,7 +60,7 @@ def test_prefill_attention_token_major_cache_matches_decode_kernel(prefill_attn)
     assert_bf16_close(got, O.attention_single_pass(q, k, v, **kw), max_ulp=1, min_exact=0.95, what="vs oracle")
 
 
-@pytest.mark.parametrize("H,Hkv,prefix,suffix,D", [(8, 2, 0, 64, 256), (8, 2, 700, 33, 256), (3, 1, 130, 21, 64), (12, 2, 65, 9, 128), (32, 8, 1500, 16, 128), (4, 4, 63, 8, 256), (2, 1, 0, 31, 64)])
+@pytest.mark.parametrize("H,Hkv,prefix,suffix,D", [(8, 2, 0, 64, 256), (8, 2, 700, 33, 256), (3, 1, 130, 21, 64), (12, 2, 65, 9, 128), (32, 8, 1500, 16, 128), (4, 4, 63, 8, 256), (2, 1, 0, 31, 64), (12, 2, 65, 5, 128), (4, 4, 63, 4, 256)])
 @pytest.mark.parametrize("trie", [False, True])
 def test_rows_of_grouped_heads(ctx, H, Hkv, prefix, suffix, D, trie):
     """Rows of (token, head) pairs: tiles that end inside a token's heads, head counts that do not divide a tile, 256 channels, few rows over
@@ -86,11 +85,19 @@ def test_rows_of_grouped_heads(ctx, H, Hkv, prefix, suffix, D, trie):
     assert_bf16_close(got, ref, max_ulp=1, min_exact=0.95, what="grouped rows vs oracle")
 
 
-@pytest.mark.parametrize("bad", [np.nan, np.inf])
-@pytest.mark.parametrize("H,Hkv,prefix,suffix,D,node", [(8, 2, 5, 40, 128, 39), (8, 2, 0, 70, 256, 3), (4, 4, 63, 8, 64, 5), (8, 2, 700, 9, 256, 4)])
+@pytest.mark.parametrize("H,Hkv,prefix,suffix,D", [(8, 2, 0, 64, 256), (8, 2, 700, 33, 256), (3, 1, 130, 21, 64), (12, 2, 65, 9, 128), (12, 2, 65, 5, 128), (4, 4, 63, 8, 256), (2, 1, 0, 31, 64)])
 @pytest.mark.parametrize("trie", [False, True])
-def test_rows_that_a_token_does_not_see(ctx, H, Hkv, prefix, suffix, D, node, trie, bad):
+def test_rows_of_grouped_heads_on_the_tensor_pipe(prefill_attn, H, Hkv, prefix, suffix, D, trie):
+    """The same where the rule would take the split-KV kernel."""
+    test_rows_of_grouped_heads(prefill_attn, H, Hkv, prefix, suffix, D, trie)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("H,Hkv,prefix,suffix,D,node", [(8, 2, 5, 15, 128, 14), (8, 2, 0, 70, 256, 3), (4, 4, 63, 8, 64, 5), (8, 2, 700, 9, 256, 4)])
+@pytest.mark.parametrize("trie", [False, True])
+def test_rows_that_a_token_does_not_see(prefill_attn, H, Hkv, prefix, suffix, D, node, trie, bad):
     """A key or value that is not finite reaches the tokens that see it and no other: not those before it, not another branch of a trie."""
+    ctx = prefill_attn
     rng = np.random.default_rng(H + prefix + suffix)
     if trie:
         suffix, node = 16, min(node, 7)

@@ -9,10 +9,14 @@
 //   * S = Q K^T with mma.sync.m16n8k16 (bf16 x bf16 products are exact, f32 accumulate), Q, K and V fragments by ldmatrix from shared memory
 //     (64 keys x D, rows padded to D + 8: conflict-free);
 //   * online softmax in f32 registers, row statistics over the 4 lanes of a quad; O is rescaled only when some row's maximum moved;
-//   * O += P V with P split into two bf16 planes (hi = bf16(p), lo = bf16(p - hi)): a single rounded plane would put 2^-9 on every
-//     probability; V fragments come from ldmatrix.trans.
+//   * O += P V with P as bf16 planes (bf16(p), then bf16 of what is left): three hold a probability to its last bit. A prompt's passes of 64 and 128
+//     channels have two (16 bits of it); a single plane would put 2^-9 on every probability. V fragments come from ldmatrix.trans. The pipe cuts what it
+//     adds to an accumulator off at its last bit, so with three planes no chain is longer than four products of either sum, and the chains are added by
+//     rounded additions: as many results differ from the correctly rounded ones as on the split-KV kernel (2 in 10000), with two planes and whole chains
+//     it was 20 in 10000.
 // A weight of zero does not hide a value that is not finite (0 x NaN): value tiles that some row sees in part are looked over first, and one with infinities
-// or NaN is summed key by key for the rows that see them, so that no token reaches an earlier one or another branch of a trie.
+// or NaN is summed key by key for the rows that see them, so that no token reaches an earlier one or another branch of a trie (with three planes: the
+// passes that the split-KV kernel served before, which never multiplied what a token does not see).
 // The next key tile is requested when S is done (it arrives during P V), the next value tile when P V is done: one buffer each, so that two or
 // three CTAs share an SM and fill one another's waits. Causal tiles past the CTA's last query are never loaded, and tiles every row of a
 // warp sees whole are not masked. CTAs with the most keys start first.
@@ -58,13 +62,14 @@ __device__ __forceinline__ float pa_remote(uint32_t addr, uint32_t rank) {
     return x;
 }
 
-template <int D>
+template <int D, int PLANES>
 __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(const uzu_attention_args a, const uint32_t splits) {
     pdl_wait();
     constexpr uint32_t LD = D + 8;                  // padded tile row (elements): 16-byte aligned rows, conflict-free ldmatrix
     constexpr uint32_t TILE = PA_BN * LD * 2;       // bytes
     constexpr uint32_t CH = D / 8;                  // 16-byte chunks per row
     constexpr float kLog2e = 1.4426950408889634f;
+    constexpr bool kRounded = PLANES == 3;          // sums of more than four products by rounded additions
     extern __shared__ __align__(16) uint8_t pa_smem[];
     const uint32_t sq = (uint32_t)__cvta_generic_to_shared(pa_smem), sk = sq + TILE, sv = sk + TILE;
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, quad = lane >> 2, tq = lane & 3;
@@ -134,16 +139,38 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
         float s[PA_BN / 8][4];
 #pragma unroll
         for (int nt = 0; nt < PA_BN / 8; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.0f;
+        if constexpr (!kRounded) {
 #pragma unroll
-        for (int ks = 0; ks < D / 16; ++ks) {
-            uint32_t qf[4];
-            pa_ldmatrix_x4(qf, q_addr + ks * 32);
+            for (int ks = 0; ks < D / 16; ++ks) {
+                uint32_t qf[4];
+                pa_ldmatrix_x4(qf, q_addr + ks * 32);
 #pragma unroll
-            for (int nt = 0; nt < PA_BN / 8; nt += 2) {
-                uint32_t kf[4];
-                pa_ldmatrix_x4(kf, k_addr + nt * 8 * LD * 2 + ks * 32);
-                pa_mma(s[nt], qf, kf[0], kf[1]);
-                pa_mma(s[nt + 1], qf, kf[2], kf[3]);
+                for (int nt = 0; nt < PA_BN / 8; nt += 2) {
+                    uint32_t kf[4];
+                    pa_ldmatrix_x4(kf, k_addr + nt * 8 * LD * 2 + ks * 32);
+                    pa_mma(s[nt], qf, kf[0], kf[1]);
+                    pa_mma(s[nt + 1], qf, kf[2], kf[3]);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int k0 = 0; k0 < D / 16; k0 += 4) {
+                uint32_t qf[4][4];
+#pragma unroll
+                for (int ks = 0; ks < 4; ++ks) pa_ldmatrix_x4(qf[ks], q_addr + (k0 + ks) * 32);
+#pragma unroll
+                for (int nt = 0; nt < PA_BN / 8; nt += 2) {
+                    float part[2][4] = {};
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks) {
+                        uint32_t kf[4];
+                        pa_ldmatrix_x4(kf, k_addr + nt * 8 * LD * 2 + (k0 + ks) * 32);
+                        pa_mma(part[0], qf[ks], kf[0], kf[1]);
+                        pa_mma(part[1], qf[ks], kf[2], kf[3]);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) s[nt + (i >> 2)][i & 3] += part[i >> 2][i & 3];
+                }
             }
         }
         __syncthreads();                                            // every warp is done with the key tile
@@ -203,7 +230,7 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
         m1 = top1;
         asm volatile("cp.async.wait_group 1;" ::: "memory");        // this tile's values have landed
         bool key_by_key = false;
-        if ((t + 1) * PA_BN > cta_whole) {
+        if (kRounded && (t + 1) * PA_BN > cta_whole) {
             uint32_t bad = 0;
 #pragma unroll 4
             for (uint32_t c = tid; c < PA_BN * CH; c += 128) {       // (what this thread copied)
@@ -216,14 +243,13 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
         } else {
             __syncthreads();
         }
-        if (key_by_key) {
-            float w[PA_BN / 8][4];
+        if (kRounded && key_by_key) {
 #pragma unroll
-            for (int nt = 0; nt < PA_BN / 8; ++nt) { w[nt][0] = s[nt][0]; w[nt][1] = s[nt][1]; w[nt][2] = s[nt][2]; w[nt][3] = s[nt][3]; }
+            for (int nt = 0; nt < PA_BN / 8; ++nt)
 #pragma unroll 1
-            for (uint32_t k = 0; k < PA_BN; ++k) {
-                const uint32_t kg = t * PA_BN + k, holder = (lane & ~3u) | ((k & 7u) >> 1);
-                const float w0 = __shfl_sync(0xffffffffu, w[k >> 3][k & 1u], holder), w1 = __shfl_sync(0xffffffffu, w[k >> 3][2 + (k & 1u)], holder);
+            for (uint32_t j = 0; j < 8; ++j) {
+                const uint32_t k = nt * 8u + j, kg = t * PA_BN + k, holder = (lane & ~3u) | (j >> 1);
+                const float w0 = __shfl_sync(0xffffffffu, (j & 1u) ? s[nt][1] : s[nt][0], holder), w1 = __shfl_sync(0xffffffffu, (j & 1u) ? s[nt][3] : s[nt][2], holder);
                 const bool sees0 = sees(kg, lim0, n0, r0 < rows), sees1 = sees(kg, lim1, n1, r1 < rows);
 #pragma unroll
                 for (int nd = 0; nd < D / 8; ++nd) {
@@ -236,26 +262,53 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
             }
         } else {
             // ---- O += P V: the S accumulator layout IS the A fragment layout of the next MMA (k = key) ----
+            auto planes = [&](uint32_t (&p)[PLANES][4], int kt) {   // a0 = (row, k 2t..): s[2 kt][0..1]; a1 = (row + 8): [2..3]; a2 = (row, k + 8): s[2 kt + 1][0..1]; a3: [2..3]
 #pragma unroll
-            for (int kt = 0; kt < PA_BN / 16; ++kt) {
-                uint32_t ph[4], pl[4];
-                const float* e0 = s[2 * kt];
-                const float* e1 = s[2 * kt + 1];
-                const float pv[8] = {e0[0], e0[1], e0[2], e0[3], e1[0], e1[1], e1[2], e1[3]};
+                for (int r = 0; r < 4; ++r) {
+                    float x = s[2 * kt + (r >> 1)][2 * (r & 1)], y = s[2 * kt + (r >> 1)][2 * (r & 1) + 1];
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {   // a0 = (row, k 2t..): e0[0..1]; a1 = (row + 8): e0[2..3]; a2 = (row, k + 8): e1[0..1]; a3: e1[2..3]
-                    const float x = pv[2 * r], y = pv[2 * r + 1];
-                    ph[r] = pa_pack(x, y);
-                    pl[r] = pa_pack(x - __uint_as_float(ph[r] << 16), y - __uint_as_float(ph[r] & 0xffff0000u));
+                    for (int i = 0; i < PLANES; ++i) {
+                        p[i][r] = pa_pack(x, y);
+                        x -= __uint_as_float(p[i][r] << 16);
+                        y -= __uint_as_float(p[i][r] & 0xffff0000u);
+                    }
                 }
+            };
+            if constexpr (!kRounded) {
+#pragma unroll
+                for (int kt = 0; kt < PA_BN / 16; ++kt) {
+                    uint32_t p[PLANES][4];
+                    planes(p, kt);
+#pragma unroll
+                    for (int nd = 0; nd < D / 8; nd += 2) {
+                        uint32_t vf[4];
+                        pa_ldmatrix_x4_trans(vf, v_addr + kt * 16 * LD * 2 + nd * 16);
+#pragma unroll
+                        for (int i = 0; i < PLANES; ++i) {
+                            pa_mma(o[nd], p[i], vf[0], vf[1]);
+                            pa_mma(o[nd + 1], p[i], vf[2], vf[3]);
+                        }
+                    }
+                }
+            } else {
+                uint32_t p[PA_BN / 16][PLANES][4];
+#pragma unroll
+                for (int kt = 0; kt < PA_BN / 16; ++kt) planes(p[kt], kt);
 #pragma unroll
                 for (int nd = 0; nd < D / 8; nd += 2) {
-                    uint32_t vf[4];
-                    pa_ldmatrix_x4_trans(vf, v_addr + kt * 16 * LD * 2 + nd * 16);
-                    pa_mma(o[nd], ph, vf[0], vf[1]);
-                    pa_mma(o[nd + 1], ph, vf[2], vf[3]);
-                    pa_mma(o[nd], pl, vf[0], vf[1]);
-                    pa_mma(o[nd + 1], pl, vf[2], vf[3]);
+                    float part[2][4] = {};
+#pragma unroll
+                    for (int kt = 0; kt < PA_BN / 16; ++kt) {
+                        uint32_t vf[4];
+                        pa_ldmatrix_x4_trans(vf, v_addr + kt * 16 * LD * 2 + nd * 16);
+#pragma unroll
+                        for (int i = PLANES - 1; i >= 0; --i) {
+                            pa_mma(part[0], p[kt][i], vf[0], vf[1]);
+                            pa_mma(part[1], p[kt][i], vf[2], vf[3]);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[nd + (i >> 2)][i & 3] += part[i >> 2][i & 3];
                 }
             }
         }
@@ -318,11 +371,11 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
     pa_cluster_sync();                                              // no CTA leaves while another may still read its rows
 }
 
-template <int D>
+template <int D, int PLANES>
 static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a) {
     constexpr size_t smem = (size_t)3 * PA_BN * (D + 8) * sizeof(__nv_bfloat16);
     static std::atomic<uint64_t> smem_opt_in{0};
-    opt_in_dynamic_smem(cmd, attn_prefill_kernel<D>, (int)smem, smem_opt_in);
+    opt_in_dynamic_smem(cmd, attn_prefill_kernel<D, PLANES>, (int)smem, smem_opt_in);
     const uint32_t row_tiles = (a.suffix_length * a.gqa_factor + PA_BM - 1) / PA_BM, kv_heads = a.num_heads / a.gqa_factor;
     const uint32_t key_tiles = (a.sequence_length + PA_BN - 1) / PA_BN, room = (uint32_t)cmd->ctx->sm_count * (D == 256 ? 2u : 3u);
     // split the keys while the chip has room for the CTAs and each keeps two tiles or more
@@ -342,7 +395,7 @@ static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_arg
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_prefill_kernel<D>, a, splits);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_prefill_kernel<D, PLANES>, a, splits);
     if (e != cudaSuccess) cmd->record_error(UZU_ERROR_CUDA, std::string("attn_prefill_kernel: ") + cudaGetErrorString(e));
     cmd->launches++;
 }
@@ -353,16 +406,18 @@ static int g_prefill_attn = -1;   // -1: follow UZU_PREFILL_ATTN, 0 / 1: forced 
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a) {
     static const bool env_enabled = [] { const char* e = getenv("UZU_PREFILL_ATTN"); return !e || atoi(e) != 0; }();   // =0 keeps the split-KV kernel
     if (!(g_prefill_attn < 0 ? env_enabled : g_prefill_attn != 0)) return false;
-    if (a.suffix_length < 8 || a.dynamic_position || a.has_sinks || a.is_kv_cache_ring || a.is_sliding_window) return false;
+    if (g_prefill_attn < 0 && a.suffix_length < 8) return false;
+    if (a.suffix_length < 2 || a.dynamic_position || a.has_sinks || a.is_kv_cache_ring || a.is_sliding_window) return false;
     if (a.is_trie && (!a.is_causal || !a.trie)) return false;
     if (a.head_dim != 64 && a.head_dim != 128 && a.head_dim != 256) return false;
     if (a.gqa_factor == 0 || a.num_heads % a.gqa_factor || (uint64_t)a.suffix_length * a.gqa_factor > 0x7fffffffull) return false;
     if ((a.k_head_stride % 8) || (a.v_head_stride % 8) || (a.k_seq_stride % 8) || (a.v_seq_stride % 8)) return false;   // 16-byte cp.async rows
     if ((a.queries | a.keys | a.values | a.out) & 15u) return false;
     if (a.sequence_length < a.suffix_length) return false;
-    if (a.head_dim == 64) launch_attn_prefill<64>(cmd, a);
-    else if (a.head_dim == 128) launch_attn_prefill<128>(cmd, a);
-    else launch_attn_prefill<256>(cmd, a);
+    const bool long_pass = a.suffix_length >= 16 && !a.is_trie;
+    if (a.head_dim == 64) long_pass ? launch_attn_prefill<64, 2>(cmd, a) : launch_attn_prefill<64, 3>(cmd, a);
+    else if (a.head_dim == 128) long_pass ? launch_attn_prefill<128, 2>(cmd, a) : launch_attn_prefill<128, 3>(cmd, a);
+    else launch_attn_prefill<256, 3>(cmd, a);
     return true;
 }
 
