@@ -14,8 +14,8 @@
 //     for kept elements only. Sums of probabilities are f64 over exact counts: the same whatever the order of the atomics.
 //     Rows whose largest logit is not finite (everything masked, infinities, NaN) walk the candidates one by one instead
 //     (sampling_walk: take the best post-noise element of the current set, accept it if its rank and the mass before it pass, otherwise
-//     shrink the set to the elements ranked before it; metal/kernel/sampling/unified_sampling.metal:154-238), as does a vocabulary
-//     whose slice does not fit 16-bit counts.
+//     shrink the set to the elements ranked before it; metal/kernel/sampling/unified_sampling.metal:154-238), as do small vocabularies
+//     and many rows, where the walk is faster, and a vocabulary whose slice does not fit 16-bit counts.
 #include "common.cuh"
 
 namespace uzu {
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(1024) sampling_argmax_kernel(const uzu_unified
 __device__ __forceinline__ bool ranked_before(float lj, uint32_t j, float lc, uint32_t c) { return lj > lc || (lj == lc && j < c); }
 
 // one CTA of 1024 threads: the candidates of row `row` one by one
-__device__ __noinline__ void sampling_walk(const uzu_unified_sampling_args& a, uint32_t row) {
+__device__ __forceinline__ void sampling_walk(const uzu_unified_sampling_args& a, uint32_t row) {
     __shared__ float redf[32];
     __shared__ unsigned long long redk[32];
     __shared__ unsigned int redc[32];
@@ -231,6 +231,7 @@ __device__ __noinline__ void sampling_walk(const uzu_unified_sampling_args& a, u
 }
 
 __global__ void __launch_bounds__(1024) sampling_walk_kernel(const uzu_unified_sampling_args a) { sampling_walk(a, blockIdx.x); }
+__device__ __noinline__ void sampling_walk_call(const uzu_unified_sampling_args& a, uint32_t row) { sampling_walk(a, row); }
 
 // order-preserving 16-bit key of a bf16 logit; -0 counts as +0 (they compare equal)
 __device__ __forceinline__ uint32_t bf16_key(uint16_t bits) {
@@ -366,7 +367,7 @@ __global__ void __cluster_dims__(SF_CTAS, 1, 1) __launch_bounds__(SF_THREADS, 1)
     const float lmax = key_value(top) * recip_t;
     // not finite, or a temperature that could make different values equal: the general walk
     if (bad || !(fabsf(lmax) < INFINITY) || !(recip_t > 1.52587890625e-5f && recip_t < 65536.0f)) {
-        if (rank == 0) sampling_walk(a, row);
+        if (rank == 0) sampling_walk_call(a, row);
         return;                                      // (uniform over the cluster; no CTA reads another's memory any more)
     }
     // 3. probabilities: f64 sums of counts * exp(l - lmax)
@@ -477,7 +478,12 @@ void uzu_unified_sampling_encode(uzu_command_buffer* cmd, const uzu_unified_samp
     if (a->batch_size == 0) return;
     uzu_context* ctx = cmd->ctx;
     if (a->has_top_k || a->has_top_p || a->has_min_p) {
-        if (a->vocab_size > uzu::SF_CTAS * 65535u) {         // 16-bit counts per slice
+        // us of both forms: counting takes about 18 us for each 15 rows (as many clusters fit the chip at a time), the walk one pass over the row per
+        // candidate, more of them in the unluckiest of several rows. Walk / count: 1 row of 4096 logits 14 / 21, of 16384 34 / 21; 16 rows of 8192 37 / 37, of
+        // 32768 80 / 42; 64 rows of 32768 72 / 104, of 65536 155 / 117.
+        const float count_us = 3.0f + (float)((a->batch_size + 14u) / 15u) * (18.0f + 8e-5f * a->vocab_size);
+        const float walk_us = 9.0f + (a->batch_size == 1 ? 0.0015f : 0.0019f) * a->vocab_size;
+        if (walk_us < count_us || a->vocab_size > uzu::SF_CTAS * 65535u) {      // (16-bit counts per slice)
             uzu::sampling_walk_kernel<<<a->batch_size, 1024, 0, ctx->stream>>>(*a);
             uzu::after_launch(cmd, "sampling_walk_kernel");
             return;
