@@ -383,7 +383,8 @@ def latent_plain(q, kv, uk, norm_w, m, eps, prefix, cache):
 
 
 @pytest.mark.parametrize("T,heads,rank,rot,prefix,window,extra", [(16, 2, 64, 0, 0, 0, False), (33, 3, 128, 16, 0, 0, True), (70, 16, 512, 64, 0, 0, False), (17, 5, 320, 32, 130, 0, False),
-                                                                  (64, 1, 256, 64, 63, 40, True), (100, 8, 192, 16, 200, 1, False)])
+                                                                  (64, 1, 256, 64, 63, 40, True), (100, 8, 192, 16, 200, 1, False),
+                                                                  (16, 2, 64, 0, 40, 0, False), (33, 3, 128, 16, 30, 0, True), (100, 16, 512, 64, 0, 0, False), (80, 1, 256, 64, 63, 40, True)])
 def test_latent_attention_of_prompt_rows(ctx, T, heads, rank, rot, prefix, window, extra):
     """The tensor-pipe form: rows that end inside a token's heads, ranks that leave column blocks of a quarter unused, windows that begin inside a tile,
     sinks and gates; rows behind the last key are NaN. Queries and weights keep f32 precision; the bound: a score
@@ -413,7 +414,7 @@ def test_latent_attention_of_prompt_rows(ctx, T, heads, rank, rot, prefix, windo
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
-@pytest.mark.parametrize("T,heads,rank,rot,prefix,window,row", [(20, 3, 128, 16, 5, 0, 24), (40, 16, 512, 64, 0, 0, 7), (33, 5, 320, 32, 130, 40, 100), (64, 1, 64, 0, 70, 40, 66)])
+@pytest.mark.parametrize("T,heads,rank,rot,prefix,window,row", [(20, 3, 128, 16, 45, 0, 64), (40, 16, 512, 64, 70, 0, 77), (80, 5, 320, 32, 130, 40, 150), (64, 1, 64, 0, 70, 40, 66)])
 def test_latent_rows_that_a_token_does_not_see(ctx, T, heads, rank, rot, prefix, window, row, bad):
     """A cache row that is not finite reaches the tokens that see it and no other: not those before it, not those whose window has left it behind."""
     rng = np.random.default_rng(T + row)
@@ -436,7 +437,7 @@ def test_latent_rows_that_a_token_does_not_see(ctx, T, heads, rank, rot, prefix,
 
 def test_latent_queries_beyond_the_largest_bf16_number(ctx):
     """Their leading part is cut off, not rounded to infinity."""
-    T, heads, rank = 16, 2, 64
+    T, heads, rank = 64, 2, 64
     q = np.zeros((T, heads, rank), np.float32)
     q[..., 0] = 3.4e38
     cache = np.random.default_rng(2).standard_normal((T, rank), dtype=np.float32)

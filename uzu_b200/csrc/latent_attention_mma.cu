@@ -12,6 +12,9 @@
 // NaN is summed key by key for the rows that see them: no token reaches an earlier one, none from before the window comes back.
 // Bound: mma.sync issue, three products per score and sum. 1024 tokens x 16 heads, rank 512 + 64: 0.26 ms (210 TFLOP/s of the three planes) against 1.99 ms with a token and 8 heads per CTA
 // on the FMA pipe; error against 64 bits 2.3e-7 (3.1e-7 there).
+#include <algorithm>
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace uzu {
@@ -42,22 +45,26 @@ __device__ __forceinline__ void lm_split3(float x0, float x1, uint32_t (&w)[3]) 
     }
 }
 
-// The same for a number of any size: beyond bf16's largest one the leading part is cut off instead of rounded, and an infinity has no rest.
+// A number of any size: beyond bf16's largest one the leading part is cut off instead of rounded, and an infinity has no rest.
 __device__ __forceinline__ uint32_t lm_leading(float& x) {
     uint32_t h = __bfloat16_as_ushort(__float2bfloat16_rn(x));
     if ((h & 0x7F80u) == 0x7F80u && x == x) h = __float_as_uint(x) >> 16;
     x = fabsf(x) == INFINITY ? 0.0f : x - __uint_as_float(h << 16);
     return h;
 }
-__device__ __forceinline__ void lm_split3_any(float x0, float x1, uint32_t (&w)[3]) {
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const uint32_t lo = lm_leading(x0);
-        w[i] = lo | lm_leading(x1) << 16;
-    }
-}
 // either half of a word is an infinity or NaN
 __device__ __forceinline__ uint32_t lm_not_finite(uint32_t w) { return (uint32_t)((w & 0x7F80u) == 0x7F80u) | (uint32_t)((w & 0x7F800000u) == 0x7F800000u); }
+// lm_split3 for numbers of any size
+__device__ __forceinline__ void lm_split3_any(float x0, float x1, uint32_t (&w)[3]) {
+    lm_split3(x0, x1, w);
+    if (lm_not_finite(w[0])) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const uint32_t lo = lm_leading(x0);
+            w[i] = lo | lm_leading(x1) << 16;
+        }
+    }
+}
 
 }  // namespace
 
@@ -94,14 +101,23 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
     {   // the query rows as three planes
         const float* q = reinterpret_cast<const float*>(a.query) + (size_t)row0 * width;
         const uint32_t pairs = width / 2;
-        for (uint32_t i = tid; i < LM_ROWS * pairs; i += LM_THREADS) {
-            const uint32_t r = i / pairs, c = i % pairs * 2;
-            float2 x = make_float2(0.0f, 0.0f);
-            if (row0 + r < total) x = *reinterpret_cast<const float2*>(q + (size_t)r * width + c);
-            uint32_t w[3];
-            lm_split3_any(x.x, x.y, w);
+        constexpr int BATCH = 6;                                         // requests in flight
+        for (uint32_t i0 = tid; i0 < LM_ROWS * pairs; i0 += BATCH * LM_THREADS) {
+            float2 x[BATCH];
 #pragma unroll
-            for (int p = 0; p < 3; ++p) asm volatile("st.shared.u32 [%0], %1;" ::"r"(sq + p * q_plane + (r * ld + c) * 2), "r"(w[p]) : "memory");
+            for (int u = 0; u < BATCH; ++u) {
+                const uint32_t i = i0 + u * LM_THREADS, r = i / pairs, c = i % pairs * 2;
+                x[u] = r < LM_ROWS && row0 + r < total ? *reinterpret_cast<const float2*>(q + (size_t)r * width + c) : make_float2(0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int u = 0; u < BATCH; ++u) {
+                const uint32_t i = i0 + u * LM_THREADS, r = i / pairs, c = i % pairs * 2;
+                if (r >= LM_ROWS) break;
+                uint32_t w[3];
+                lm_split3_any(x[u].x, x[u].y, w);
+#pragma unroll
+                for (int p = 0; p < 3; ++p) asm volatile("st.shared.u32 [%0], %1;" ::"r"(sq + p * q_plane + (r * ld + c) * 2), "r"(w[p]) : "memory");
+            }
         }
     }
     float o[NB][2][4];
@@ -120,22 +136,20 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
     const uint32_t p_addr = sp + ((rg * 16 + (lane & 15)) * LM_PLD + (lane >> 4) * 8) * 2;
     const uint32_t v_addr = sk + ((lane & 15) * ld + share * (a.rank / 4) + (lane >> 4) * 8) * 2;
 
-    for (uint32_t t = t_begin; t < t_end; ++t) {
+    auto tile = [&](const uint32_t t, auto part_c) {                     // part: not every row sees the whole tile
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         bool key_by_key = false;
-        if ((t + 1) * LM_KEYS > first_keys || t * LM_KEYS < last_lo) {   // not every row sees the whole tile
+        __syncthreads();
+        if constexpr (decltype(part_c)::value) {
             uint32_t bad = 0;
-            const uint32_t pieces = width / 8;
-            for (uint32_t i = tid; i < 64u * pieces; i += LM_THREADS) {  // (what this thread copied)
-                const uint32_t r = i / pieces, c = i % pieces;
-                uint32_t x[4];
-                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(sk + (r * ld + c * 8) * 2));
+            for (uint32_t r = warp; r < LM_KEYS; r += LM_THREADS / 32)
+                for (uint32_t c = lane; c < a.rank / 8; c += 32) {
+                    uint32_t x[4];
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(x[0]), "=r"(x[1]), "=r"(x[2]), "=r"(x[3]) : "r"(sk + (r * ld + c * 8) * 2));
 #pragma unroll
-                for (int j = 0; j < 4; ++j) bad |= lm_not_finite(x[j]);
-            }
+                    for (int j = 0; j < 4; ++j) bad |= lm_not_finite(x[j]);
+                }
             key_by_key = __syncthreads_or((int)bad) != 0;
-        } else {
-            __syncthreads();
         }
         // ---- scores of 16 rows x 16 keys ----
         float s[2][4], low[2][4];                                        // [8 keys]: the leading plane | the other two
@@ -244,38 +258,43 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
             }
             __syncthreads();
             if (t + 1 < t_end) load_half(t + 1, 0);
-        }
+        } else {
 #pragma unroll
-        for (uint32_t half = 0; half < 2 && !key_by_key; ++half) {
-            if (half) {
-                __syncthreads();                                         // every warp is done with the tile's first 32 keys
-                if (t + 1 < t_end) load_half(t + 1, 0);
-            }
-            uint32_t pf[2][3][4];
-#pragma unroll
-            for (int i = 0; i < 6; ++i) lm_ldmatrix(pf[i / 3][i % 3], p_addr + (i % 3) * p_plane + (half * 2 + i / 3) * 32);
-#pragma unroll
-            for (int b = 0; b < NB; ++b) {
-                if ((uint32_t)b >= nb) continue;
-                float part[2][4];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) part[i >> 2][i & 3] = 0.0f;
-#pragma unroll
-                for (int ks = 0; ks < 2; ++ks) {
-                    uint32_t vf[4];
-                    lm_ldmatrix_trans(vf, v_addr + (half * 2 + ks) * 16 * ld * 2 + b * 32);
-#pragma unroll
-                    for (int p = 2; p >= 0; --p) {
-                        lm_mma(part[0], pf[ks][p], vf[0], vf[1]);
-                        lm_mma(part[1], pf[ks][p], vf[2], vf[3]);
-                    }
+            for (uint32_t half = 0; half < 2; ++half) {
+                if (half) {
+                    __syncthreads();                                         // every warp is done with the tile's first 32 keys
+                    if (t + 1 < t_end) load_half(t + 1, 0);
                 }
+                uint32_t pf[2][3][4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) o[b][i >> 2][i & 3] += part[i >> 2][i & 3];
+                for (int i = 0; i < 6; ++i) lm_ldmatrix(pf[i / 3][i % 3], p_addr + (i % 3) * p_plane + (half * 2 + i / 3) * 32);
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    if ((uint32_t)b >= nb) continue;
+                    float part[2][4];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) part[i >> 2][i & 3] = 0.0f;
+#pragma unroll
+                    for (int ks = 0; ks < 2; ++ks) {
+                        uint32_t vf[4];
+                        lm_ldmatrix_trans(vf, v_addr + (half * 2 + ks) * 16 * ld * 2 + b * 32);
+#pragma unroll
+                        for (int p = 2; p >= 0; --p) {
+                            lm_mma(part[0], pf[ks][p], vf[0], vf[1]);
+                            lm_mma(part[1], pf[ks][p], vf[2], vf[3]);
+                        }
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) o[b][i >> 2][i & 3] += part[i >> 2][i & 3];
+                }
             }
         }
         __syncthreads();
         if (t + 1 < t_end) load_half(t + 1, 1);
+    };
+    for (uint32_t t = t_begin; t < t_end; ++t) {
+        if ((t + 1) * LM_KEYS > first_keys || t * LM_KEYS < last_lo) tile(t, std::true_type{});
+        else tile(t, std::false_type{});
     }
     // a row's weight sum: over the quad's lanes, then over the four shares in order
     l_a += __shfl_xor_sync(0xffffffffu, l_a, 1); l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
@@ -308,9 +327,13 @@ __global__ void __launch_bounds__(LM_THREADS, 1) latent_attention_mma_kernel(con
 
 static size_t latent_mma_smem(uint32_t width) { return ((size_t)3 * LM_ROWS * (width + 8) + (size_t)LM_KEYS * (width + 8) + (size_t)3 * LM_ROWS * LM_PLD) * 2; }
 
-// bf16 rows of whole 16-byte pieces, a rank of whole 64 columns, sixteen tokens and more (fewer are cut into key splits over many CTAs)
+// bf16 rows of whole 16-byte pieces, a rank of whole 64 columns, sixteen tokens and more (fewer are cut into key splits over many CTAs), and enough keys: a
+// tile of 64 costs the same however few are seen, and the FMA kernel takes a CTA per token and 8 heads and two to three keys a microsecond. 16 heads, FMA /
+// this one, us: rank 64, 32 tokens 8.9 / 10.3, 48 tokens 10.9 / 10.3; rank 512, 32 tokens 15 / 25, 96 tokens 50 / 33, 20 tokens behind 100 44 / 33.
 bool latent_attention_mma_applicable(const uzu_latent_attention_args& a) {
     const uint32_t width = a.rank + a.rot_dim;
+    const uint64_t ctas = std::max<uint64_t>((uint64_t)a.rows * ((a.heads + 7) / 8), 148), keys = (uint64_t)(a.window ? std::min(a.prefix, a.window) : a.prefix) + a.rows;
+    if (keys * ctas < (a.rank <= 128 ? 52u : a.heads < 8 ? 112u : 96u) * 148ull) return false;
     if (a.cache_dt != UZU_DT_BF16 || a.dynamic_position || a.splits > 1 || a.rows < 16) return false;
     if (a.rank % 64u || width % 16u || (a.cache & 15u) || (a.query & 7u) || (a.out & 7u)) return false;
     return (uint64_t)a.rows * a.heads < 0x80000000ull && latent_mma_smem(width) <= 225u * 1024u;
