@@ -22,11 +22,12 @@
 // warp sees whole are not masked. CTAs with the most keys start first.
 // Where rows x KV heads do not fill the chip a cluster of up to 8 CTAs shares the keys of a tile and merges its partial results over
 // distributed shared memory in rank order.
-// Bound: shared-memory reads and mma.sync issue. 8 heads of 256 channels (2 KV heads), 1024 rows behind 1024: 0.10 ms against 1.11 ms one query
+// Bound: shared-memory reads and mma.sync issue. 8 heads of 256 channels (2 KV heads), 1024 rows behind 1024: 0.13 ms against 1.11 ms one query
 // token at a time on the split-KV kernel.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
     const uint32_t k_addr = sk + (((lane >> 4) * 8 + (lane & 7)) * LD + ((lane >> 3) & 1) * 8) * 2;
     const uint32_t v_addr = sv + ((lane & 15) * LD + (lane >> 4) * 8) * 2;
 
-    for (uint32_t t = t_begin; t < t_end; ++t) {
+    auto tile_step = [&](const uint32_t t, auto part_c) {           // part: not every row of the CTA sees the whole tile
         asm volatile("cp.async.wait_group 1;" ::: "memory");        // this tile's keys (and the queries) have landed
         __syncthreads();
         // ---- S = Q K^T ----
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
         m1 = top1;
         asm volatile("cp.async.wait_group 1;" ::: "memory");        // this tile's values have landed
         bool key_by_key = false;
-        if (kRounded && (t + 1) * PA_BN > cta_whole) {
+        if constexpr (decltype(part_c)::value) {
             uint32_t bad = 0;
 #pragma unroll 4
             for (uint32_t c = tid; c < PA_BN * CH; c += 128) {       // (what this thread copied)
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
         } else {
             __syncthreads();
         }
-        if (kRounded && key_by_key) {
+        if (decltype(part_c)::value && key_by_key) {
 #pragma unroll
             for (int nt = 0; nt < PA_BN / 8; ++nt)
 #pragma unroll 1
@@ -315,6 +316,10 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
         __syncthreads();                                            // every warp is done with the value tile
         if (t + 1 < t_end) load_tile(sv, vbase, a.v_seq_stride, t + 1);
         else asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (uint32_t t = t_begin; t < t_end; ++t) {
+        if (kRounded && (t + 1) * PA_BN > cta_whole) tile_step(t, std::true_type{});
+        else tile_step(t, std::false_type{});
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1); l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
@@ -371,16 +376,46 @@ __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(con
     pa_cluster_sync();                                              // no CTA leaves while another may still read its rows
 }
 
+// CTAs that share a tile's keys: more while the chip has room for them and each keeps two tiles or more
+static uint32_t pa_splits(const uzu_attention_args& a, uint32_t sms) {
+    const uint32_t row_tiles = (a.suffix_length * a.gqa_factor + PA_BM - 1) / PA_BM, kv_heads = a.num_heads / a.gqa_factor;
+    const uint32_t key_tiles = (a.sequence_length + PA_BN - 1) / PA_BN, room = sms * (a.head_dim == 256 ? 2u : 3u);
+    uint32_t splits = 1;
+    while (splits < 8 && row_tiles * kv_heads * splits * 2 <= room && key_tiles >= splits * 4) splits *= 2;
+    return splits;
+}
+
+static bool pa_two_planes(const uzu_attention_args& a) { return a.suffix_length >= 16 && !a.is_trie && a.head_dim != 256; }
+
+// Whether this kernel is the faster one: both estimates in us, fitted to 1480 sizes (8 to 256 tokens, 0 to 8000 cached rows, 4 to 64 heads in groups of 1 to
+// 8; the choice costs 0.7 % on average). The split-KV kernel pays for every (token, head) and key, this one for whole tiles of 64 x 64. 32 heads of 128 in
+// groups of 4, split-KV / this one: 8 tokens behind 16 rows 6.7 / 13.7, behind 450 23 / 19, behind 2048 48 / 31; 16 tokens behind 16 6.6 / 11.5, behind 1000
+// 41 / 15. 8 heads of 256, 64 tokens alone 10.7 / 27, behind 1000 73 / 28. Fewer than 8 tokens stay with the split-KV kernel: 4 behind 200 take 12.4 / 14.5,
+// behind 1000 19 / 14.5, behind 4096 45 / 37.
+static bool pa_faster(const uzu_attention_args& a, uint32_t sms) {
+    const uint32_t D = a.head_dim, rows = a.suffix_length, keys = a.sequence_length, gq = a.gqa_factor, g = gq % 8 == 0 ? 8 : gq % 4 == 0 ? 4 : gq % 2 == 0 ? 2 : 1;
+    if (rows < 8) return false;
+    const uint32_t ctas = a.num_heads / g * rows;                              // as encode_attn_rows (attention.cu) cuts it
+    const uint32_t nsplits = rows <= 16 ? std::max(1u, std::min(std::min((2 * sms + ctas - 1) / ctas, (keys + 63) / 64), 32u)) : 1u;
+    const float fill = (float)ctas * nsplits / (sms * (D == 128 ? 1.0f : 2.0f));
+    const float waves = D == 128 ? 0.5f * (std::ceil(fill) + std::max(1.0f, fill)) : std::ceil(fill);
+    const float per_key = D == 64 ? 0.0118f + 0.00064f * g * g : D == 128 ? 0.0103f + 0.00081f * g * g : 0.035f + 0.0019f * g * g;
+    const float split = (D == 64 ? 1.0f : D == 128 ? 1.15f : 1.1f) *
+                        ((D == 64 ? 5.5f : 6.2f) + waves * per_key * keys / nsplits + (nsplits == 1 ? 0.0f : D == 64 ? 2.8f : D == 128 ? 4.5f : 6.1f));
+    const bool two = pa_two_planes(a);
+    const uint32_t shares = pa_splits(a, sms), row_tiles = (rows * gq + PA_BM - 1) / PA_BM, key_tiles = (keys + PA_BN - 1) / PA_BN, room = sms * (D == 256 ? 2u : 3u);
+    const uint32_t all = row_tiles * (a.num_heads / gq) * shares, turns = std::max(1u, (all + room - 1) / room), per = (key_tiles + shares - 1) / shares;
+    const float start = D == 64 ? 5.0f : D == 128 ? 8.6f : 14.5f, tile = D == 64 ? (two ? 1.8f : 3.0f) : D == 128 ? (two ? 2.8f : 4.65f) : 7.0f;
+    const float merge = shares == 1 ? 0.0f : D == 64 ? (two ? 4.4f : 2.3f) : D == 128 ? (two ? 1.9f : 0.6f) : -0.7f;
+    return start * (0.5f + 0.5f * turns) + tile * per * turns + merge < split;
+}
+
 template <int D, int PLANES>
 static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a) {
     constexpr size_t smem = (size_t)3 * PA_BN * (D + 8) * sizeof(__nv_bfloat16);
     static std::atomic<uint64_t> smem_opt_in{0};
     opt_in_dynamic_smem(cmd, attn_prefill_kernel<D, PLANES>, (int)smem, smem_opt_in);
-    const uint32_t row_tiles = (a.suffix_length * a.gqa_factor + PA_BM - 1) / PA_BM, kv_heads = a.num_heads / a.gqa_factor;
-    const uint32_t key_tiles = (a.sequence_length + PA_BN - 1) / PA_BN, room = (uint32_t)cmd->ctx->sm_count * (D == 256 ? 2u : 3u);
-    // split the keys while the chip has room for the CTAs and each keeps two tiles or more
-    uint32_t splits = 1;
-    while (splits < 8 && row_tiles * kv_heads * splits * 2 <= room && key_tiles >= splits * 4) splits *= 2;
+    const uint32_t row_tiles = (a.suffix_length * a.gqa_factor + PA_BM - 1) / PA_BM, kv_heads = a.num_heads / a.gqa_factor, splits = pa_splits(a, (uint32_t)cmd->ctx->sm_count);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(row_tiles * splits, kv_heads);
     cfg.blockDim = dim3(128);
@@ -400,13 +435,12 @@ static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_arg
     cmd->launches++;
 }
 
-// true = handled: eight query tokens and more (fewer keep the split-KV kernel, a CTA per token and split, which fills the chip as well), dense prefix, plain mask or a causal trie.
-static int g_prefill_attn = -1;   // -1: follow UZU_PREFILL_ATTN, 0 / 1: forced by uzu_debug_set_prefill_attention
+// true = handled: where it is the faster kernel, for a dense prefix, a plain mask or a causal trie
+static int g_prefill_attn = -1;   // -1: follow UZU_PREFILL_ATTN and the rule, 0: never, 1: wherever it can (uzu_debug_set_prefill_attention)
 
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a) {
     static const bool env_enabled = [] { const char* e = getenv("UZU_PREFILL_ATTN"); return !e || atoi(e) != 0; }();   // =0 keeps the split-KV kernel
     if (!(g_prefill_attn < 0 ? env_enabled : g_prefill_attn != 0)) return false;
-    if (g_prefill_attn < 0 && a.suffix_length < 8) return false;
     if (a.suffix_length < 2 || a.dynamic_position || a.has_sinks || a.is_kv_cache_ring || a.is_sliding_window) return false;
     if (a.is_trie && (!a.is_causal || !a.trie)) return false;
     if (a.head_dim != 64 && a.head_dim != 128 && a.head_dim != 256) return false;
@@ -414,9 +448,10 @@ bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args&
     if ((a.k_head_stride % 8) || (a.v_head_stride % 8) || (a.k_seq_stride % 8) || (a.v_seq_stride % 8)) return false;   // 16-byte cp.async rows
     if ((a.queries | a.keys | a.values | a.out) & 15u) return false;
     if (a.sequence_length < a.suffix_length) return false;
-    const bool long_pass = a.suffix_length >= 16 && !a.is_trie;
-    if (a.head_dim == 64) long_pass ? launch_attn_prefill<64, 2>(cmd, a) : launch_attn_prefill<64, 3>(cmd, a);
-    else if (a.head_dim == 128) long_pass ? launch_attn_prefill<128, 2>(cmd, a) : launch_attn_prefill<128, 3>(cmd, a);
+    if (g_prefill_attn < 0 && !pa_faster(a, (uint32_t)cmd->ctx->sm_count)) return false;
+    const bool two = pa_two_planes(a);
+    if (a.head_dim == 64) two ? launch_attn_prefill<64, 2>(cmd, a) : launch_attn_prefill<64, 3>(cmd, a);
+    else if (a.head_dim == 128) two ? launch_attn_prefill<128, 2>(cmd, a) : launch_attn_prefill<128, 3>(cmd, a);
     else launch_attn_prefill<256, 3>(cmd, a);
     return true;
 }
