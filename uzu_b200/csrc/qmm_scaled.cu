@@ -558,7 +558,10 @@ bool qmm_scaled_applicable(const uzu_matmul_args& a) {
     // 8B model, MLX groups of 32: 2 rows 150 us there, 176 here; 4 rows 199 and 155
     const uint32_t bits = a.b_mode == UZU_QMODE_U4 ? 4 : 8;
     if (a.m <= 2 && a.k * bits % 2048u == 0) return false;
-    // 17 .. 63 rows over a matrix of at most 2^21 weights with groups of 64 or 128: launches of 16 rows (qmm_rows.cu)
+    // MLX with groups of 256: three planes cost more than the streaming kernel up to 8 rows. A layer of an 8B model: 3 rows 130 us there, 168 here; 8 rows
+    // 166 and 169; 9 rows 216 and 170
+    if (a.m <= 8 && bits == 4 && gs == 256 && a.b_prologue == UZU_B_SCALE_BIAS_DEQUANT && a.k * bits % 2048u == 0) return false;
+    // 17 .. 63 rows over a matrix of at most 2^21 weights with groups of 64 or 128: launches of 16 rows (qmm_rows.cu, with the times)
     if (a.m > 16 && a.m < 64 && (uint64_t)a.n * a.k <= (1u << 21) && (gs == 64 || gs == 128)) return false;
     return tensor_map_encoder() != nullptr;
 }
