@@ -2,8 +2,8 @@
 // update.rs:13-144}) applied to the m tokens of a pass, in three launches whatever m is:
 //   delta_net_conv_kernel    causal conv + SiLU (bf16-rounded, like the conv kernel), unit q and k vectors, q scaled by Dk^-0.5, decay and
 //                            beta of all tokens at once into f32 scratch rows (a warp per 8 tokens and head, the conv window in registers);
-//   the gated delta scan     (gated_delta.cu) a value column of the state needs no other column, so 8 lanes own one and walk the tokens
-//                            without a barrier; 128 CTAs for 16 heads of 128 columns;
+//   the gated delta scan     (gated_delta.cu) a value column of the state needs no other column, so a few lanes own one and walk the tokens,
+//                            four at a time; 128 CTAs for 16 heads of 128 columns;
 //   delta_net_gate_kernel    RMS norm of each head's row, norm weight, SiLU(z), bf16 store; the rolling conv state moves on here, when all
 //                            readers of the old one are done.
 // Bound: latency of the scan (one warp per scheduler walks the tokens, nothing covers its waits), not bytes. As ONE CTA per

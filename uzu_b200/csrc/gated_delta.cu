@@ -6,8 +6,10 @@
 // lane part p holds the key channels {4 (i L + p) .. + 3}, NV float4 in registers -- and a token costs two dot products, two shuffle
 // reductions over L lanes and no barrier at all. q and k rows are read from shared memory as float4 with the L parts side by side (128
 // contiguous bytes at L = 8: no bank conflict, the columns of a warp share the read).
+//   gated_delta_block_kernel the tokens of a pass four at a time, keys of 33..128 channels (column_block.cuh).
 //   gated_delta_kernel       the tokens of a pass in order, 4 warps per CTA, grid (column blocks, heads). The prepared q / k / v / decay / beta
-//                            rows arrive by cp.async one batch ahead. An element's arithmetic does not depend on how a prompt is cut.
+//                            rows arrive by cp.async one batch ahead. An element's arithmetic does not depend on how a prompt is cut
+//                            (with blocks of four it does, within rounding).
 //   delta_prepare_kernel     convolution, silu, unit vectors and gates of all tokens of a pass at once, a warp per (a few tokens, head).
 //   gated_delta_step_kernel  one token with everything between the projections in one launch: a cluster of CL CTAs per head, each CTA owning
 //                            vdim / CL columns; the state is requested before the previous kernel's results are waited for; the head's sum
@@ -16,7 +18,7 @@
 // while all CTAs read the other taps - 1 slots, so no ordering between the CTAs is needed (several value heads may share a key head).
 #include <type_traits>
 
-#include "column_scan.cuh"
+#include "column_block.cuh"
 #include "common.cuh"
 
 namespace uzu {
@@ -198,14 +200,26 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const uzu_delta_prep
     }
 }
 
-constexpr int GD_WARPS = 4;
+constexpr int GD_CB_WARPS = 4;
 
 template <int L, int NV>
 constexpr int gd_batch() { return L * NV * 4 <= 256 ? 16 : (L * NV * 4 <= 512 ? 8 : 4); }
 
+// the pass's last inputs of the convolution go to the ring (the launch before the scan was its last reader); all threads of the grid take part
+__device__ __forceinline__ void gd_ring_store(const uzu_delta_prepare_args& a) {
+    const uint32_t channels = 2 * a.kv_heads * a.dim + a.heads * a.vdim, prefix = gd_prefix(a), keep = min(a.rows, a.taps - 1);
+    const uint32_t threads = gridDim.x * gridDim.y * blockDim.x, me = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+    const float* proj = reinterpret_cast<const float*>(a.proj);
+    float* ring = reinterpret_cast<float*>(a.ring);
+    for (uint32_t i = me; i < keep * channels; i += threads) {
+        const uint32_t t = a.rows - keep + i / channels, c = i % channels;
+        ring[(size_t)((prefix + t) % a.taps) * channels + c] = proj[(size_t)t * a.stride + c];
+    }
+}
+
 template <int L, int NV>
-__global__ void __launch_bounds__(GD_WARPS * 32) gated_delta_kernel(const uzu_gated_delta_args ga) {
-    constexpr int ROWF = L * NV * 4, BATCH = gd_batch<L, NV>(), CC = GD_WARPS * (32 / L), U = BATCH < 8 ? BATCH : 8;
+__global__ void __launch_bounds__(GD_CB_WARPS * 32) gated_delta_kernel(const uzu_gated_delta_args ga) {
+    constexpr int ROWF = L * NV * 4, BATCH = gd_batch<L, NV>(), CC = GD_CB_WARPS * (32 / L), U = BATCH < 8 ? BATCH : 8;
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float gd_smem[];
@@ -229,12 +243,12 @@ __global__ void __launch_bounds__(GD_WARPS * 32) gated_delta_kernel(const uzu_ga
         const uint32_t nb = tb < a.rows ? min((uint32_t)BATCH, a.rows - tb) : 0u;
         float* q = qs + buf * BATCH * ROWF;
         float* k = ks + buf * BATCH * ROWF;
-        for (uint32_t i = tid; i < nb * pieces; i += GD_WARPS * 32) {
+        for (uint32_t i = tid; i < nb * pieces; i += GD_CB_WARPS * 32) {
             const uint32_t r = i / pieces, c = (i - r * pieces) * 4;
             gd_cp_async16(q + r * ROWF + c, pq + (size_t)(tb + r) * qk_stride + c);
             gd_cp_async16(k + r * ROWF + c, pk + (size_t)(tb + r) * qk_stride + c);
         }
-        for (uint32_t i = tid; i < nb * CC; i += GD_WARPS * 32) {
+        for (uint32_t i = tid; i < nb * CC; i += GD_CB_WARPS * 32) {
             const uint32_t r = i / CC, c = i % CC;
             if (col0 + c < a.vdim) gd_cp_async4(vs + (buf * BATCH + r) * CC + c, pv + (size_t)(tb + r) * v_stride + c);
         }
@@ -246,23 +260,14 @@ __global__ void __launch_bounds__(GD_WARPS * 32) gated_delta_kernel(const uzu_ga
     };
     if (dim4 < (uint32_t)ROWF) {                     // channels past the head stay zero in both buffers
         const uint32_t tail = ROWF - dim4;
-        for (uint32_t i = tid; i < 2 * BATCH * tail; i += GD_WARPS * 32) {
+        for (uint32_t i = tid; i < 2 * BATCH * tail; i += GD_CB_WARPS * 32) {
             const uint32_t r = i / tail, c = dim4 + i % tail;
             qs[r * ROWF + c] = 0.0f;
             ks[r * ROWF + c] = 0.0f;
         }
     }
     stage(0, 0);
-    {   // the pass's last inputs of the convolution go to the ring (the launch before this one was its last reader)
-        const uint32_t channels = 2 * a.kv_heads * a.dim + a.heads * a.vdim, prefix = gd_prefix(a), keep = min(a.rows, a.taps - 1);
-        const uint32_t threads = gridDim.x * gridDim.y * blockDim.x, me = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + tid;
-        const float* proj = reinterpret_cast<const float*>(a.proj);
-        float* ring = reinterpret_cast<float*>(a.ring);
-        for (uint32_t i = me; i < keep * channels; i += threads) {
-            const uint32_t t = a.rows - keep + i / channels, c = i % channels;
-            ring[(size_t)((prefix + t) % a.taps) * channels + c] = proj[(size_t)t * a.stride + c];
-        }
-    }
+    gd_ring_store(a);
     float4 S[NV];
     float* state = reinterpret_cast<float*>(ga.state) + ((size_t)h * a.vdim + (col_ok ? col : 0u)) * dim4;
 #pragma unroll
@@ -339,6 +344,193 @@ __global__ void __launch_bounds__(GD_WARPS * 32) gated_delta_kernel(const uzu_ga
 }
 
 constexpr int GS_THREADS = 256;
+
+// The same tokens four at a time, keys of 33..128 channels (column_block.cuh). With S the state at a block's start and p_j the product of the decays of
+// its tokens before j, what token j writes is
+//     w_j = beta_j v_j - beta_j g_j p_j (k_j . S) - sum_{i<j} beta_j g_j (g_{i+1} .. g_{j-1}) (k_j . k_i) w_i
+//     o_j = p_{j+1} (q_j . S) + sum_{i<=j} (g_{i+1} .. g_j) (q_j . k_i) w_i,      S' = p_4 S + sum_i (g_{i+1} .. g_3) k_i w_i^T
+// Producer warps (one per block) pass the q and k rows on, form the products k_j . k_i and q_j . k_i and invert the w_i system; consumer warps take the
+// dot products with S, L lanes of four channels per group of Q columns. A decay is at most 1, so no product of them can grow.
+// Bound: the chain dot products -> lane sums -> exchange -> update, about 1150 cycles a block with one consumer warp per scheduler. 509 tokens, 16 heads of
+// 128 x 128: 78 us against 96 us token by token.
+template <int ROWF>
+struct GdBlock {
+    static constexpr int K = 0, R = 4 * ROWF, T = 8 * ROWF, C = T + 12, PO = C + 4, BETA = PO + 4, QS = BETA + 4, OW = QS + 8, V = OW + 16;
+    static constexpr int floats(int columns) { return V + CB_TOKENS * columns; }
+};
+
+template <int L, int NV, int Q>
+__global__ void __launch_bounds__(CB_THREADS, 2) gated_delta_block_kernel(const uzu_gated_delta_args ga) {
+    constexpr int ROWF = L * NV * 4;
+    using F = GdBlock<ROWF>;
+    constexpr int GROUPS = 32 / L, CC = CB_WARPS * GROUPS * Q, U = CB_TOKENS * Q, SPAN = L / U, BLK = F::floats(CC);
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float gd_smem[];
+    float* wbuf = gd_smem + 2 * CB_BLOCKS * BLK;     // [2][CB_WARPS * GROUPS][U], twice each
+    const uzu_delta_prepare_args& a = ga.prep;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t h = blockIdx.y, kvh = h / (a.heads / a.kv_heads), dim4 = (a.dim + 3) & ~3u, col0 = blockIdx.x * CC;
+    const uint32_t steps = (a.rows + CB_BLOCKS * CB_TOKENS - 1) / (CB_BLOCKS * CB_TOKENS);
+    const size_t qk_stride = (size_t)a.kv_heads * dim4, v_stride = (size_t)a.heads * a.vdim;
+    gd_ring_store(a);
+
+    if (warp >= CB_WARPS) {                          // producer of block `which` of every step
+        const uint32_t which = warp - CB_WARPS, ch = 4 * lane;
+        const bool ch_ok = ch < dim4;
+        const float* pq = reinterpret_cast<const float*>(a.q) + (size_t)kvh * dim4 + ch;
+        const float* pk = reinterpret_cast<const float*>(a.k) + (size_t)kvh * dim4 + ch;
+        const float* pv = reinterpret_cast<const float*>(a.v) + (size_t)h * a.vdim + col0 + lane;
+        const float* pg = reinterpret_cast<const float*>(a.decay) + h;
+        const float* pb = reinterpret_cast<const float*>(a.beta) + h;
+        cb_f4 q[CB_TOKENS], k[CB_TOKENS];
+        float v[CB_TOKENS], g[CB_TOKENS], beta[CB_TOKENS];        // a token past the pass changes nothing: g = 1, the others 0
+        auto fetch = [&](uint32_t step) {
+            const uint32_t t0 = (step * CB_BLOCKS + which) * CB_TOKENS;
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j) {
+                const uint32_t t = t0 + j;
+                const bool ok = t < a.rows;
+                q[j] = ok && ch_ok ? cb_load4(pq + t * qk_stride) : cb_set4(0.0f);
+                k[j] = ok && ch_ok ? cb_load4(pk + t * qk_stride) : cb_set4(0.0f);
+                v[j] = ok && lane < CC && col0 + lane < a.vdim ? pv[t * v_stride] : 0.0f;
+                g[j] = ok ? pg[(size_t)t * a.heads] : 1.0f;
+                beta[j] = ok ? pb[(size_t)t * a.heads] : 0.0f;
+            }
+        };
+        auto produce = [&](uint32_t step) {
+            float* B = gd_smem + ((step & 1) * CB_BLOCKS + which) * BLK;
+            if (ch < (uint32_t)ROWF) {
+#pragma unroll
+                for (int j = 0; j < CB_TOKENS; ++j) {
+                    cb_store4(B + F::K + j * ROWF + ch, k[j]);
+                    cb_store4(B + F::R + j * ROWF + ch, q[j]);
+                }
+            }
+            float s[16];                             // [0, 6) k . k below the diagonal, [6, 16) q . k with it
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j)
+#pragma unroll
+                for (int i = 0; i <= j; ++i) {
+                    if (i < j) s[j * (j - 1) / 2 + i] = cb_dot(k[j], k[i]);
+                    s[6 + j * (j + 1) / 2 + i] = cb_dot(q[j], k[i]);
+                }
+            gd_transpose_sum<16, 32>(s, lane);
+            float n[6], t[6];
+#pragma unroll
+            for (int e = 0; e < 6; ++e) n[e] = __shfl_sync(0xffffffffu, s[0], 2 * e);
+            const float g12 = g[1] * g[2], p3 = g[0] * g12;
+            n[0] *= -beta[1] * g[1];
+            n[1] *= -beta[2] * g12;
+            n[2] *= -beta[2] * g[2];
+            n[3] *= -beta[3] * (g12 * g[3]);
+            n[4] *= -beta[3] * (g[2] * g[3]);
+            n[5] *= -beta[3] * g[3];
+            cb_invert(n, t);
+            if (lane == 0) {
+                cb_store_solve(B + F::T, t);
+                const float p1 = g[0], p2 = g[0] * g[1], p4 = p3 * g[3];
+                *reinterpret_cast<float4*>(B + F::PO) = make_float4(p1, p2, p3, p4);
+                *reinterpret_cast<float4*>(B + F::C) = make_float4(-beta[0] * p1, -beta[1] * p2, -beta[2] * p3, -beta[3] * p4);
+                *reinterpret_cast<float4*>(B + F::BETA) = make_float4(beta[0], beta[1], beta[2], beta[3]);
+                const float q0 = g12 * g[3], q1 = g[2] * g[3];
+                *reinterpret_cast<float4*>(B + F::QS) = make_float4(q0, q0, q1, q1);
+                *reinterpret_cast<float4*>(B + F::QS + 4) = make_float4(g[3], g[3], p4, p4);
+            } else if (lane >= 12 && (lane & 1) == 0) {
+                uint32_t j, i;
+                cb_lower(lane / 2 - 6, j, i);
+                float f = 1.0f;                      // g_{i+1} .. g_j
+#pragma unroll
+                for (uint32_t l = 1; l < CB_TOKENS; ++l)
+                    if (l > i && l <= j) f *= g[l];
+                B[F::OW + j * 4 + i] = s[0] * f;
+            }
+            if (lane < CC) {
+#pragma unroll
+                for (int j = 0; j < CB_TOKENS; ++j) B[F::V + j * CC + lane] = v[j];
+            }
+        };
+        fetch(0);
+        produce(0);
+        fetch(1);
+        for (uint32_t step = 0; step < steps; ++step) {
+            __syncthreads();                         // step's blocks are ready, the other buffer is free
+            if (step + 1 < steps) {
+                produce(step + 1);
+                fetch(step + 2);
+            }
+        }
+        return;
+    }
+
+    const uint32_t part = lane % L, group = warp * GROUPS + lane / L, lc = group * Q, col = col0 + lc, ch = 4 * part;
+    const uint32_t idx = part / SPAN, oj = idx / Q, oc = idx % Q;      // after a reduction the lane holds (token, column) oj, oc
+    const bool first = part % SPAN == 0, owner = first && col + oc < a.vdim;
+    cb_f4 S[Q][NV];
+    float* state = reinterpret_cast<float*>(ga.state) + ((size_t)h * a.vdim + col) * dim4 + ch;
+#pragma unroll
+    for (int c = 0; c < Q; ++c)
+#pragma unroll
+        for (int n = 0; n < NV; ++n) S[c][n] = col + c < a.vdim && ch + 4 * L * n < dim4 ? cb_load4(state + (size_t)c * dim4 + 4 * L * n) : cb_set4(0.0f);
+    float* out = reinterpret_cast<float*>(ga.out) + (size_t)h * a.vdim + col + oc;
+    for (uint32_t step = 0; step < steps; ++step) {
+        __syncthreads();
+        const uint32_t t_step = step * CB_BLOCKS * CB_TOKENS, nblocks = min((uint32_t)CB_BLOCKS, (a.rows - t_step + CB_TOKENS - 1) / CB_TOKENS);
+        for (uint32_t b = 0; b < nblocks; ++b) {
+            const float* B = gd_smem + ((step & 1) * CB_BLOCKS + b) * BLK;
+            float* wb = wbuf + ((b & 1) * CB_WARPS * GROUPS + group) * U * 2;
+            cb_f4 k[CB_TOKENS][NV], q[CB_TOKENS][NV];
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j)
+#pragma unroll
+                for (int n = 0; n < NV; ++n) k[j][n] = cb_load4(B + F::K + j * ROWF + ch + 4 * L * n);
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j)
+#pragma unroll
+                for (int n = 0; n < NV; ++n) q[j][n] = cb_load4(B + F::R + j * ROWF + ch + 4 * L * n);
+            float zp[U], op[U];
+            cb_dots<NV, Q>(zp, k, S);
+            const float bv = B[F::BETA + oj] * B[F::V + oj * CC + lc + oc], cj = B[F::C + oj], po = B[F::PO + oj];
+            const cb_f4 qs0 = cb_load4(B + F::QS), qs1 = cb_load4(B + F::QS + 4);
+            gd_transpose_sum<U, L>(zp, part);
+            if (first) {
+                const float r = fmaf(cj, zp[0], bv);
+                *reinterpret_cast<float2*>(wb + 2 * idx) = make_float2(r, r);
+            }
+            __syncwarp();                            // the buffer's next writer is two blocks on, behind another one of these
+            cb_dots<NV, Q>(op, q, S);
+#pragma unroll
+            for (int c = 0; c < Q; ++c)
+#pragma unroll
+                for (int n = 0; n < NV; ++n) S[c][n] = cb_scale(S[c][n], qs1.b);
+            cb_f2 w[CB_TOKENS][Q], y[CB_TOKENS][Q];
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j) cb_load<Q>(y[j], wb + 2 * j * Q);
+            cb_solve<Q>(w, y, B + F::T);
+#pragma unroll
+            for (int c = 0; c < Q; ++c) {            // the last token's write has decayed by nothing
+                y[0][c] = cb_mul2(w[0][c], qs0.a);
+                y[1][c] = cb_mul2(w[1][c], qs0.b);
+                y[2][c] = cb_mul2(w[2][c], qs1.a);
+                y[3][c] = w[3][c];
+            }
+            cb_update<NV, Q>(S, k, y);
+            gd_transpose_sum<U, L>(op, part);
+            float wown[CB_TOKENS];
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j) wown[j] = cb_pick<Q>(w[j], oc);
+            // up to the token itself: a later token's value reaches no earlier one, not even as 0 * x
+            const float o = cb_upto(po * op[0], *reinterpret_cast<const float4*>(B + F::OW + oj * 4), wown, oj + 1);
+            const uint32_t t = t_step + b * CB_TOKENS + oj;
+            if (owner && t < a.rows) out[t * v_stride] = o;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < Q; ++c)
+#pragma unroll
+        for (int n = 0; n < NV; ++n)
+            if (col + c < a.vdim && ch + 4 * L * n < dim4) cb_store4(state + (size_t)c * dim4 + 4 * L * n, S[c][n]);
+}
 
 // CL CTAs (one cluster) per head, ceil(vdim / CL) columns each, GS_THREADS / L columns at a time
 template <int CL, int L, int NV>
@@ -486,12 +678,28 @@ static void by_key_size(uint32_t dim, F&& f) {
 }
 
 void launch_gated_delta_scan(uzu_command_buffer* cmd, const uzu_gated_delta_args& a) {
+    // Four tokens at a time where a key's channels fit the lanes. One column per lane group where two would leave SMs without a CTA.
+    if (a.prep.dim > 32 && a.prep.dim <= 128) {
+        auto blocks = [&](auto nv_c, auto q_c) {
+            constexpr int L = 16, NV = decltype(nv_c)::value, Q = decltype(q_c)::value, GROUPS = CB_WARPS * (32 / L), CC = GROUPS * Q;
+            constexpr size_t smem = ((size_t)2 * CB_BLOCKS * GdBlock<L * NV * 4>::floats(CC) + (size_t)4 * GROUPS * CB_TOKENS * Q) * sizeof(float);
+            static std::atomic<uint64_t> done{0};
+            if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, gated_delta_block_kernel<L, NV, Q>, (int)smem, done);
+            launch(cmd, "gated_delta_kernel", gated_delta_block_kernel<L, NV, Q>, dim3((a.prep.vdim + CC - 1) / CC, a.prep.heads), dim3(CB_THREADS), smem, a);
+        };
+        auto one = std::integral_constant<int, 1>{};
+        auto two = std::integral_constant<int, 2>{};
+        const bool narrow = a.prep.heads * ((a.prep.vdim + 7) / 8) <= 148;
+        if (a.prep.dim <= 64) narrow ? blocks(one, one) : blocks(one, two);
+        else narrow ? blocks(two, one) : blocks(two, two);
+        return;
+    }
     by_key_size(a.prep.dim, [&](auto l_c, auto nv_c) {
-        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GD_WARPS * (32 / L), BATCH = gd_batch<L, NV>();
+        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GD_CB_WARPS * (32 / L), BATCH = gd_batch<L, NV>();
         constexpr size_t smem = ((size_t)4 * BATCH * L * NV * 4 + (size_t)2 * BATCH * CC + 4 * BATCH) * sizeof(float);
         static std::atomic<uint64_t> done{0};
         if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, gated_delta_kernel<L, NV>, (int)smem, done);
-        launch(cmd, "gated_delta_kernel", gated_delta_kernel<L, NV>, dim3((a.prep.vdim + CC - 1) / CC, a.prep.heads), dim3(GD_WARPS * 32), smem, a);
+        launch(cmd, "gated_delta_kernel", gated_delta_kernel<L, NV>, dim3((a.prep.vdim + CC - 1) / CC, a.prep.heads), dim3(GD_CB_WARPS * 32), smem, a);
     });
 }
 

@@ -6,13 +6,14 @@
 //                               parallel launch first (general_delta_prepare_kernel), then L lanes own a column and walk the tokens, two dot
 //                               products and an update each, no barrier between tokens; the five vectors of a token come from shared memory,
 //                               a batch of tokens ahead by cp.async. Bound: latency that nothing covers (one warp per scheduler).
+//   general_delta_block_kernel  the same with four tokens per step, heads of 33..128 channels (column_block.cuh).
 //   general_delta_kernel        the decode step and short passes: a CTA keeps a dim x 32 slice of the state in registers -- warp p owns PART
 //                               key channels, lane c owns column c; partial sums meet in shared memory in warp order (a fixed order: one
 //                               token at a time or several in one launch give the same bits).
 #include <cstdlib>
 #include <type_traits>
 
-#include "column_scan.cuh"
+#include "column_block.cuh"
 #include "common.cuh"
 
 namespace uzu {
@@ -151,13 +152,13 @@ __global__ void __launch_bounds__(128) general_delta_prepare_kernel(const uzu_ge
 // 32 / L columns per warp, grid (column blocks, heads). Bound: latency. 16 heads of 128 are 512 warps on 592 schedulers, and a warp's 20 shared 16-byte
 // reads and its arithmetic of a token take 375 ns with nothing beside them; the dependent part (dot product over the lane's channels, log2 L shuffles, the
 // update) is about a fifth of that. 1024 tokens, 16 heads of 128: 0.37 ms against 1.70 ms as a CTA per 32 columns with three barriers a token.
-constexpr int GS_WARPS = 4;
+constexpr int GS_CB_WARPS = 4;
 template <int L, int NV>
 constexpr int gs_batch() { return L * NV * 4 <= 128 ? 8 : (L * NV * 4 <= 256 ? 4 : 2); }
 
 template <int L, int NV>
-__global__ void __launch_bounds__(GS_WARPS * 32) general_delta_scan_kernel(const uzu_general_delta_args a, uint32_t vec) {
-    constexpr int ROWF = L * NV * 4, BATCH = gs_batch<L, NV>(), CC = GS_WARPS * (32 / L);
+__global__ void __launch_bounds__(GS_CB_WARPS * 32) general_delta_scan_kernel(const uzu_general_delta_args a, uint32_t vec) {
+    constexpr int ROWF = L * NV * 4, BATCH = gs_batch<L, NV>(), CC = GS_CB_WARPS * (32 / L);
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float gs_smem[];
@@ -178,19 +179,19 @@ __global__ void __launch_bounds__(GS_WARPS * 32) general_delta_scan_kernel(const
             const uint32_t pieces = dim / 4;
 #pragma unroll
             for (int w = 0; w < 5; ++w)
-                for (uint32_t i = tid; i < nb * pieces; i += GS_WARPS * 32) {
+                for (uint32_t i = tid; i < nb * pieces; i += GS_CB_WARPS * 32) {
                     const uint32_t r = i / pieces, c = (i - r * pieces) * 4;
                     gd_cp_async16(dst + (r * 5 + w) * ROWF + c, src[w] + (size_t)(tb + r) * stride[w] + c);
                 }
         } else {
 #pragma unroll
             for (int w = 0; w < 5; ++w)
-                for (uint32_t i = tid; i < nb * dim; i += GS_WARPS * 32) {
+                for (uint32_t i = tid; i < nb * dim; i += GS_CB_WARPS * 32) {
                     const uint32_t r = i / dim, c = i - r * dim;
                     gd_cp_async4(dst + (r * 5 + w) * ROWF + c, src[w] + (size_t)(tb + r) * stride[w] + c);
                 }
         }
-        for (uint32_t i = tid; i < nb * CC; i += GS_WARPS * 32) {
+        for (uint32_t i = tid; i < nb * CC; i += GS_CB_WARPS * 32) {
             const uint32_t r = i / CC, c = i % CC;
             if (col0 + c < dim) gd_cp_async4(vs + (buf * BATCH + r) * CC + c, pv + (size_t)(tb + r) * a.v_stride + c);
         }
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32) general_delta_scan_kernel(const
     };
     if (dim < (uint32_t)ROWF) {                      // channels past the head stay zero in both buffers
         const uint32_t tail = ROWF - dim;
-        for (uint32_t i = tid; i < 2 * BATCH * 5 * tail; i += GS_WARPS * 32) vecs[i / tail * ROWF + dim + i % tail] = 0.0f;
+        for (uint32_t i = tid; i < 2 * BATCH * 5 * tail; i += GS_CB_WARPS * 32) vecs[i / tail * ROWF + dim + i % tail] = 0.0f;
     }
     stage(0, 0);
     float4 S[NV];
@@ -275,17 +276,235 @@ __global__ void __launch_bounds__(GS_WARPS * 32) general_delta_scan_kernel(const
     }
 }
 
+// The tokens of a pass four at a time, heads of 33..128 channels whose rows lie on 16-byte boundaries. With S the state at a block's start, P_j the
+// product of the decays of its tokens before j and alpha = rate * unit key:
+//     z_j = u_j . S_j = (u_j P_j) . S + sum_{i<j} -(u_j . (d_{i+1} .. d_{j-1} alpha_i)) z_i + (u_j . (d_{i+1} .. d_{j-1} k_i)) v_i
+//     o_j = (r_j P_{j+1}) . S + sum_{i<=j} the same sums with r_j and one decay more
+//     S' = P_4 S + sum_i (d_{i+1} .. d_3) (k_i v_i^T - alpha_i z_i^T)
+// Producer warps (one per block) form the 17 vectors and the sums over channels, and invert the z_i system; decays are <= 1, so no product of them can
+// grow. Consumer warps: see column_block.cuh; L lanes of four channels per group of Q columns.
+// Bound: the shared-memory reads of a block (34 16-byte vector reads of each of four warps, in bursts) and the chain dot products -> lane sums -> exchange ->
+// update: 1200 cycles a block of which 490 issue. More warps with fewer columns each read more and were slower (291 us), one reduction for both kinds of
+// dot products instead of two was too (235 us). 1024 tokens with their preparation and copies: 16 heads of 128 206 us (386 token by token), 8 heads 0.20 ms
+// (0.39), 32 heads 0.35 ms (0.57), 16 heads of 64 0.15 ms (0.24); 40 tokens 44 us (51), 4 tokens 38 us (38).
+template <int ROWF>
+struct GbBlock {
+    static constexpr int U = 0, A = 4 * ROWF, K = 8 * ROWF, R = 12 * ROWF, P = 16 * ROWF, T = 17 * ROWF, ZK = T + 12, OK = ZK + 16, OA = OK + 16, V = OA + 16;
+    static constexpr int floats(int columns) { return V + 2 * CB_TOKENS * columns; }
+};
+
+template <int L, int NV, int Q>
+__global__ void __launch_bounds__(CB_THREADS, 2) general_delta_block_kernel(const uzu_general_delta_args a) {
+    constexpr int ROWF = L * NV * 4;
+    using F = GbBlock<ROWF>;
+    constexpr int GROUPS = 32 / L, CC = CB_WARPS * GROUPS * Q, U = CB_TOKENS * Q, SPAN = L / U, BLK = F::floats(CC);
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) float gb_smem[];
+    float* zbuf = gb_smem + 2 * CB_BLOCKS * BLK;     // [2][CB_WARPS * GROUPS][U], twice each
+    const uint32_t dim = a.dim, h = blockIdx.y, hc = h * dim, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col0 = blockIdx.x * CC;
+    const uint32_t steps = (a.rows + CB_BLOCKS * CB_TOKENS - 1) / (CB_BLOCKS * CB_TOKENS);
+
+    if (warp >= CB_WARPS) {                          // producer of block `which` of every step
+        const uint32_t which = warp - CB_WARPS, ch = 4 * lane;
+        const bool ch_ok = ch < dim;
+        const uint32_t stride[5] = {a.decay_stride, a.rate_stride, a.heads * dim, a.k_stride, a.r_stride};
+        const float* src[5] = {reinterpret_cast<const float*>(a.decay_logit) + hc + ch, reinterpret_cast<const float*>(a.rate_logit) + hc + ch,
+                               reinterpret_cast<const float*>(a.unit) + hc + ch, reinterpret_cast<const float*>(a.k) + hc + ch, reinterpret_cast<const float*>(a.r) + hc + ch};
+        cb_f4 x[5][CB_TOKENS];                      // d, alpha, u, k, r; a token past the pass changes nothing (d = 1, the others 0)
+        float v[CB_TOKENS];
+        auto fetch = [&](uint32_t step) {
+            const uint32_t t0 = (step * CB_BLOCKS + which) * CB_TOKENS;
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j) {
+                const bool ok = t0 + j < a.rows;
+#pragma unroll
+                for (int w = 0; w < 5; ++w) {
+                    const float none = w == 0 ? 1.0f : 0.0f;
+                    x[w][j] = ok && ch_ok ? cb_load4(src[w] + (size_t)(t0 + j) * stride[w]) : cb_set4(none);
+                }
+                v[j] = ok && lane < CC && col0 + lane < dim ? reinterpret_cast<const float*>(a.v)[(size_t)(t0 + j) * a.v_stride + hc + col0 + lane] : 0.0f;
+            }
+        };
+        auto produce = [&](uint32_t step) {
+            float* B = gb_smem + ((step & 1) * CB_BLOCKS + which) * BLK;
+            const bool in_row = ch < (uint32_t)ROWF;
+            auto put = [&](int off, const cb_f4& y) { if (in_row) cb_store4(B + off + ch, y); };
+            cb_f4 (&d)[CB_TOKENS] = x[0];
+            cb_f4 p = d[0];
+            put(F::U, x[2][0]);
+            put(F::R, cb_mul(x[4][0], p));
+#pragma unroll
+            for (int j = 1; j < CB_TOKENS; ++j) {
+                put(F::U + j * ROWF, cb_mul(x[2][j], p));
+                p = cb_mul(p, d[j]);
+                put(F::R + j * ROWF, cb_mul(x[4][j], p));
+            }
+            put(F::P, p);
+            // sums over the channels: [0, 6) u . -alpha, [6, 12) u . k (strictly lower), [12, 22) r . -alpha, [22, 32) r . k (with the diagonal)
+            float s[32];
+#pragma unroll
+            for (int i = 0; i < CB_TOKENS; ++i) {
+                cb_f4 al = cb_scale(x[1][i], cb_pack(-1.0f, -1.0f)), k = x[3][i];
+#pragma unroll
+                for (int j = i; j < CB_TOKENS; ++j) {
+                    if (j > i) {
+                        s[j * (j - 1) / 2 + i] = cb_dot(x[2][j], al);
+                        s[6 + j * (j - 1) / 2 + i] = cb_dot(x[2][j], k);
+                        al = cb_mul(al, d[j]);
+                        k = cb_mul(k, d[j]);
+                    }
+                    s[12 + j * (j + 1) / 2 + i] = cb_dot(x[4][j], al);
+                    s[22 + j * (j + 1) / 2 + i] = cb_dot(x[4][j], k);
+                }
+                put(F::A + i * ROWF, al);
+                put(F::K + i * ROWF, k);
+            }
+            gd_transpose_sum<32, 32>(s, lane);
+            float n[6], t[6];
+#pragma unroll
+            for (int e = 0; e < 6; ++e) n[e] = __shfl_sync(0xffffffffu, s[0], e);
+            cb_invert(n, t);
+            uint32_t j, i;
+            if (lane == 0) {
+                cb_store_solve(B + F::T, t);
+            } else if (lane >= 6 && lane < 12) {
+                cb_strict(lane - 6, j, i);
+                B[F::ZK + j * 4 + i] = s[0];
+            } else if (lane >= 12) {
+                cb_lower(lane < 22 ? lane - 12 : lane - 22, j, i);
+                B[(lane < 22 ? F::OA : F::OK) + j * 4 + i] = s[0];
+            }
+            if (lane < CC) {
+#pragma unroll
+                for (int j2 = 0; j2 < CB_TOKENS; ++j2) *reinterpret_cast<float2*>(B + F::V + 2 * (j2 * CC + lane)) = make_float2(v[j2], v[j2]);
+            }
+        };
+        fetch(0);
+        produce(0);
+        fetch(1);
+        for (uint32_t step = 0; step < steps; ++step) {
+            __syncthreads();                         // step's blocks are ready, the other buffer is free
+            if (step + 1 < steps) {
+                produce(step + 1);
+                fetch(step + 2);
+            }
+        }
+        return;
+    }
+
+    const uint32_t part = lane % L, group = warp * GROUPS + lane / L, lc = group * Q, col = col0 + lc, ch = 4 * part;
+    const uint32_t idx = part / SPAN, oj = idx / Q, oc = idx % Q;      // after a reduction the lane holds (token, column) oj, oc
+    const bool first = part % SPAN == 0, owner = first && col + oc < dim;
+    cb_f4 S[Q][NV];
+    float* state = reinterpret_cast<float*>(a.state) + (size_t)h * dim * dim + col;
+#pragma unroll
+    for (int c = 0; c < Q; ++c)
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+            const uint32_t cn = ch + 4 * L * n;
+            const float* p = state + (size_t)cn * dim + c;
+            if (col + c < dim && cn < dim) S[c][n] = {cb_pack(p[0], p[dim]), cb_pack(p[2 * dim], p[3 * dim])};
+            else S[c][n] = cb_set4(0.0f);
+        }
+    float* out = reinterpret_cast<float*>(a.out) + hc + col + oc;
+    const uint32_t out_stride = a.heads * dim;
+    for (uint32_t step = 0; step < steps; ++step) {
+        __syncthreads();
+        const uint32_t t_step = step * CB_BLOCKS * CB_TOKENS, nblocks = min((uint32_t)CB_BLOCKS, (a.rows - t_step + CB_TOKENS - 1) / CB_TOKENS);
+        for (uint32_t b = 0; b < nblocks; ++b) {
+            const float* B = gb_smem + ((step & 1) * CB_BLOCKS + b) * BLK;
+            float* zb = zbuf + ((b & 1) * CB_WARPS * GROUPS + group) * U * 2;
+            auto load = [&](cb_f4 (&y)[CB_TOKENS][NV], int off) {
+#pragma unroll
+                for (int j = 0; j < CB_TOKENS; ++j)
+#pragma unroll
+                    for (int n = 0; n < NV; ++n) y[j][n] = cb_load4(B + off + j * ROWF + ch + 4 * L * n);
+            };
+            cb_f4 x[CB_TOKENS][NV];
+            float zp[U], op[U], vown[CB_TOKENS];
+            cb_f2 v[CB_TOKENS][Q];
+            load(x, F::U);
+            cb_dots<NV, Q>(zp, x, S);
+            load(x, F::R);
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j) {
+                vown[j] = B[F::V + 2 * (j * CC + lc + oc)];
+                cb_load<Q>(v[j], B + F::V + 2 * (j * CC + lc));
+            }
+            const float4 zk = *reinterpret_cast<const float4*>(B + F::ZK + oj * 4);
+            gd_transpose_sum<U, L>(zp, part);
+            // the right-hand side of (token, column); a later token's value reaches no earlier one, not even as 0 * x
+            const float r = cb_upto(zp[0], zk, vown, oj);
+            if (first) *reinterpret_cast<float2*>(zb + 2 * idx) = make_float2(r, r);
+            __syncwarp();                            // the buffer's next writer is two blocks on, behind another one of these
+            cb_dots<NV, Q>(op, x, S);
+            load(x, F::K);
+#pragma unroll
+            for (int n = 0; n < NV; ++n) {
+                const cb_f4 p = cb_load4(B + F::P + ch + 4 * L * n);
+#pragma unroll
+                for (int c = 0; c < Q; ++c) S[c][n] = cb_mul(S[c][n], p);
+            }
+            cb_update<NV, Q>(S, x, v);
+            cb_f2 z[CB_TOKENS][Q], rhs[CB_TOKENS][Q];
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j) cb_load<Q>(rhs[j], zb + 2 * j * Q);
+            cb_solve<Q>(z, rhs, B + F::T);
+            load(x, F::A);
+            cb_update<NV, Q>(S, x, z);
+            gd_transpose_sum<U, L>(op, part);
+            float zown[CB_TOKENS];
+#pragma unroll
+            for (int j = 0; j < CB_TOKENS; ++j) zown[j] = cb_pick<Q>(z[j], oc);
+            float o = cb_upto(op[0], *reinterpret_cast<const float4*>(B + F::OK + oj * 4), vown, oj + 1);
+            o = cb_upto(o, *reinterpret_cast<const float4*>(B + F::OA + oj * 4), zown, oj + 1);
+            const uint32_t t = t_step + b * CB_TOKENS + oj;
+            if (owner && t < a.rows) out[(size_t)t * out_stride] = o;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < Q; ++c)
+#pragma unroll
+        for (int n = 0; n < NV; ++n) {
+            const uint32_t cn = ch + 4 * L * n;
+            if (col + c >= dim || cn >= dim) continue;
+            float* p = state + (size_t)cn * dim + c;
+            p[0] = cb_lo(S[c][n].a);
+            p[dim] = cb_hi(S[c][n].a);
+            p[2 * dim] = cb_lo(S[c][n].b);
+            p[3 * dim] = cb_hi(S[c][n].b);
+        }
+}
+
 static void launch_general_delta_scan(uzu_command_buffer* cmd, const uzu_general_delta_args& a) {
     // 16-byte copies where every row of every vector starts on a 16-byte boundary
     const uint32_t vec = !((a.decay_logit | a.rate_logit | a.unit | a.k | a.r) & 15u) &&
                          !((a.decay_stride | a.rate_stride | a.k_stride | a.r_stride | a.dim) & 3u);
     auto go = [&](auto l_c, auto nv_c) {
-        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GS_WARPS * (32 / L), BATCH = gs_batch<L, NV>();
+        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GS_CB_WARPS * (32 / L), BATCH = gs_batch<L, NV>();
         constexpr size_t smem = ((size_t)2 * BATCH * 5 * L * NV * 4 + (size_t)2 * BATCH * CC) * sizeof(float);
         static std::atomic<uint64_t> done{0};
         if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, general_delta_scan_kernel<L, NV>, (int)smem, done);
-        launch(cmd, "general_delta_scan_kernel", general_delta_scan_kernel<L, NV>, dim3((a.dim + CC - 1) / CC, a.heads), dim3(GS_WARPS * 32), smem, a, vec);
+        launch(cmd, "general_delta_scan_kernel", general_delta_scan_kernel<L, NV>, dim3((a.dim + CC - 1) / CC, a.heads), dim3(GS_CB_WARPS * 32), smem, a, vec);
     };
+    // Four tokens at a time wherever a row's channels fit the lanes as float4: faster from 4 tokens on (figures above the kernel). One column per lane group
+    // where two would leave SMs without a CTA.
+    if (vec && a.dim > 32 && a.dim <= 128) {
+        auto blocks = [&](auto nv_c, auto q_c) {
+            constexpr int L = 16, NV = decltype(nv_c)::value, Q = decltype(q_c)::value, GROUPS = CB_WARPS * (32 / L), CC = GROUPS * Q;
+            constexpr size_t smem = ((size_t)2 * CB_BLOCKS * GbBlock<L * NV * 4>::floats(CC) + (size_t)4 * GROUPS * CB_TOKENS * Q) * sizeof(float);
+            static std::atomic<uint64_t> done{0};
+            if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, general_delta_block_kernel<L, NV, Q>, (int)smem, done);
+            launch(cmd, "general_delta_scan_kernel", general_delta_block_kernel<L, NV, Q>, dim3((a.dim + CC - 1) / CC, a.heads), dim3(CB_THREADS), smem, a);
+        };
+        auto one = std::integral_constant<int, 1>{};
+        auto two = std::integral_constant<int, 2>{};
+        const bool narrow = a.heads * ((a.dim + 7) / 8) <= 148;
+        if (a.dim <= 64) narrow ? blocks(one, one) : blocks(one, two);
+        else narrow ? blocks(two, one) : blocks(two, two);
+        return;
+    }
     auto l8 = std::integral_constant<int, 8>{};
     if (a.dim <= 32) go(l8, std::integral_constant<int, 1>{});
     else if (a.dim <= 64) go(l8, std::integral_constant<int, 2>{});
