@@ -75,6 +75,30 @@ constexpr uint32_t SAMPLING_WS_SLOTS = 7168;   // u64 partial keys
 constexpr uint32_t SAMPLING_MAX_BLOCKS = 28;
 constexpr uint32_t SAMPLING_ROWS_PER_LAUNCH = 256;
 
+// rows of whole 16-byte pieces: eight logits per read, their eight mask bits in one word
+static bool sampling_whole_pieces(const uzu_unified_sampling_args& a) { return a.vocab_size % 8u == 0 && !(a.logits & 15u); }
+// eight logits as they count: masked ones are -inf
+__device__ __forceinline__ uint4 masked_piece(const uint16_t* logits, const uint32_t* bitmask, uint32_t i) {
+    uint4 x = *reinterpret_cast<const uint4*>(logits + i);
+    if (bitmask) {
+        const uint32_t on = bitmask[i >> 5] >> (i & 31u);
+        uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (!((on >> (2 * j)) & 1u)) w[j] = (w[j] & 0xFFFF0000u) | 0xFF80u;
+            if (!((on >> (2 * j + 1)) & 1u)) w[j] = (w[j] & 0xFFFFu) | 0xFF800000u;
+        }
+        x = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    return x;
+}
+__device__ __forceinline__ uint16_t piece_bits(const uint4& x, int j) {
+    const uint32_t w = j < 2 ? x.x : j < 4 ? x.y : j < 6 ? x.z : x.w;
+    return (uint16_t)(w >> (16 * (j & 1)));
+}
+
+// VEC: a thread's logits come in one or two 16-byte reads instead of a chain of 2-byte ones. Bound: latency (a read, the block's and the grid's maximum).
+template <bool VEC>
 __global__ void __launch_bounds__(1024) sampling_argmax_kernel(const uzu_unified_sampling_args a, uint32_t row0, unsigned long long* ws,
                                                                unsigned int* tickets) {
     __shared__ unsigned long long red[32];
@@ -87,11 +111,19 @@ __global__ void __launch_bounds__(1024) sampling_argmax_kernel(const uzu_unified
     const float recip_t = a.has_temperature ? 1.0f / a.temperature : 1.0f;
     const uint64_t seed = a.is_stochastic ? reinterpret_cast<const unsigned long long*>(a.seeds)[row] : 0ull;
     unsigned long long best = 0ull;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x) {
-        float v = filtered_logit(a, logits, bitmask, recip_t, i);
+    auto offer = [&](float v, uint32_t i) {
         if (a.is_stochastic) v += gumbel_noise(seed, i, V);
         const unsigned long long k = pack_key(v, i);
         best = k > best ? k : best;
+    };
+    if constexpr (VEC) {
+        for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) * 8u; i < V; i += gridDim.x * blockDim.x * 8u) {
+            const uint4 x = masked_piece(reinterpret_cast<const uint16_t*>(logits), bitmask, i);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) offer(a.has_temperature ? bf16_bits_to_f32(piece_bits(x, j)) * recip_t : bf16_bits_to_f32(piece_bits(x, j)), i + j);
+        }
+    } else {
+        for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x) offer(filtered_logit(a, logits, bitmask, recip_t, i), i);
     }
     best = warp_max_u64(best);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -244,27 +276,32 @@ __device__ __forceinline__ float key_value(uint32_t key) {
 
 constexpr uint32_t SF_CTAS = 8, SF_THREADS = 1024;
 constexpr uint32_t SF_KEYS = 65536, SF_OWNED = SF_KEYS / SF_CTAS, SF_PER = SF_OWNED / SF_THREADS;    // keys per CTA and per thread when they are added up
+constexpr uint32_t SF_PIECES = 4;                    // 16-byte pieces of logits that a thread keeps
 constexpr size_t SF_SMEM = SF_KEYS * sizeof(uint16_t);
 static_assert(SF_PER == 8, "a thread adds up eight neighbouring keys: one 16-byte read per CTA");
 
-// Bound: latency (a few cluster barriers, one pass over a 128 KB count table); the logits are read twice, the second time from L2.
-// 8 rows of 128256 logits, temperature, top-k 50, top-p 0.95: 40 us a call (268 us as one CTA per row walking the candidates).
+// Bound: latency (a few cluster barriers, one pass over a 128 KB count table). VEC: rows of whole 16-byte pieces and at most 262144 logits stay in registers,
+// one read each; otherwise the logits are read twice, two bytes at a time. 8 rows, temperature, top-k 50, top-p 0.95: 34 us at 128256 logits (40 with the
+// two-byte reads), 47 at 248320 (67); 16 rows of 128256 67 us (82).
+template <bool VEC>
 __global__ void __cluster_dims__(SF_CTAS, 1, 1) __launch_bounds__(SF_THREADS, 1) sampling_filtered_kernel(const uzu_unified_sampling_args a) {
     extern __shared__ __align__(16) uint16_t sf_counts[];
     // what the CTAs of the cluster tell one another, slot = the sender
-    __shared__ uint32_t x_top[SF_CTAS], x_n[SF_CTAS], x_edge[SF_CTAS], x_kept[SF_CTAS], x_same[SF_CTAS], x_bad[SF_CTAS];
+    __shared__ uint32_t x_top[SF_CTAS], x_n[SF_CTAS], x_edge[SF_CTAS], x_kept[SF_CTAS], x_bad[SF_CTAS];
     __shared__ double x_mass[SF_CTAS];
     __shared__ unsigned long long x_best[SF_CTAS];
     __shared__ double red_d[32];
     __shared__ uint32_t red_u[32];
     __shared__ unsigned long long red_k[32];
     pdl_launch_dependents();
+    for (uint32_t i = threadIdx.x; i < SF_KEYS / 8; i += SF_THREADS) reinterpret_cast<uint4*>(sf_counts)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
     pdl_wait();
     const uint32_t V = a.vocab_size, row = blockIdx.y, rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint16_t* logits = reinterpret_cast<const uint16_t*>(a.logits) + (size_t)row * V;
     const uint32_t* bitmask = a.has_bitmask ? reinterpret_cast<const uint32_t*>(a.bitmask) + (size_t)row * ((V + 31) / 32) : nullptr;
     const float recip_t = a.has_temperature ? 1.0f / a.temperature : 1.0f;
-    const uint32_t slice = (V + SF_CTAS - 1) / SF_CTAS, lo = min(rank * slice, V), hi = min(lo + slice, V);
+    const uint32_t slice = VEC ? ((V / 8u + SF_CTAS - 1) / SF_CTAS) * 8u : (V + SF_CTAS - 1) / SF_CTAS, lo = min(rank * slice, V), hi = min(lo + slice, V);
     auto masked_bits = [&](uint32_t i) -> uint16_t {
         const bool off = bitmask && ((bitmask[i >> 5] >> (i & 31)) & 1u) == 0u;
         return off ? (uint16_t)0xFF80u : logits[i];
@@ -320,14 +357,27 @@ __global__ void __cluster_dims__(SF_CTAS, 1, 1) __launch_bounds__(SF_THREADS, 1)
     };
 
     // 1. count the values of this CTA's slice
-    for (uint32_t i = tid; i < SF_KEYS / 8; i += SF_THREADS) reinterpret_cast<uint4*>(sf_counts)[i] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
     uint32_t bad = 0;
-    for (uint32_t i = lo + tid; i < hi; i += SF_THREADS) {
-        const uint16_t bits = masked_bits(i);
+    auto count = [&](uint16_t bits) {
         bad |= (uint32_t)((bits & 0x7FFFu) > 0x7F80u) | (uint32_t)(bits == 0x7F80u);       // NaN, +inf
         const uint32_t key = bf16_key(bits);
         atomicAdd(reinterpret_cast<uint32_t*>(sf_counts) + (key >> 1), (key & 1u) ? 0x10000u : 1u);
+    };
+    uint4 x[VEC ? SF_PIECES : 1];
+    if constexpr (VEC) {
+#pragma unroll
+        for (uint32_t v = 0; v < SF_PIECES; ++v) {
+            const uint32_t i = lo + (v * SF_THREADS + tid) * 8u;
+            if (i < hi) x[v] = masked_piece(logits, bitmask, i);
+        }
+#pragma unroll
+        for (uint32_t v = 0; v < SF_PIECES; ++v)
+            if (lo + (v * SF_THREADS + tid) * 8u < hi) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) count(piece_bits(x[v], j));
+            }
+    } else {
+        for (uint32_t i = lo + tid; i < hi; i += SF_THREADS) count(masked_bits(i));
     }
     bad = (uint32_t)__syncthreads_or((int)bad);
     cluster_sync();
@@ -421,9 +471,11 @@ __global__ void __cluster_dims__(SF_CTAS, 1, 1) __launch_bounds__(SF_THREADS, 1)
         if (x_edge[c] > edge) { edge = x_edge[c]; quota = x_kept[c]; }
     // 5. elements of the edge value are kept by rising index: the slices before this CTA's come first
     const uint32_t edge_key = edge - 1;              // (edge = 0: every element is kept)
-    tell_u32(x_same, edge ? (uint32_t)sf_counts[edge_key] : 0u);
-    cluster_sync();
-    for (uint32_t c = 0; c < rank; ++c) quota -= min(quota, x_same[c]);
+    for (uint32_t c = 0; edge && c < rank; ++c) {    // (their tables stay: no CTA leaves before the last barrier)
+        uint16_t same;
+        asm volatile("ld.shared::cluster.u16 %0, [%1];" : "=h"(same) : "r"(remote(sf_counts + edge_key, c)));
+        quota -= min(quota, (uint32_t)same);
+    }
     const uint64_t seed = a.is_stochastic ? reinterpret_cast<const unsigned long long*>(a.seeds)[row] : 0ull;
     unsigned long long best = 0ull;
     auto offer = [&](uint32_t i, uint16_t bits) {
@@ -433,7 +485,40 @@ __global__ void __cluster_dims__(SF_CTAS, 1, 1) __launch_bounds__(SF_THREADS, 1)
         best = k > best ? k : best;
     };
     const bool count_equal = edge != 0 && quota != 0 && quota < sf_counts[edge_key];     // (uniform over the CTA)
-    for (uint32_t i0 = lo; i0 < hi; i0 += SF_THREADS) {
+    if constexpr (VEC) {
+#pragma unroll
+        for (uint32_t v = 0; v < SF_PIECES; ++v) {
+            const uint32_t i = lo + (v * SF_THREADS + tid) * 8u;
+            uint32_t equal = 0, keep = 0;            // a bit per logit of the piece
+            if (i < hi) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint32_t key = bf16_key(piece_bits(x[v], j)) + 1u;
+                    keep |= (uint32_t)(key > edge) << j;
+                    equal |= (uint32_t)(edge != 0 && key == edge) << j;
+                }
+            }
+            if (count_equal) {
+                const uint32_t own = (uint32_t)__popc(equal);
+                uint32_t upto = own;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(0xffffffffu, upto, o); if (lane >= o) upto += t; }
+                __syncthreads();
+                if (lane == 31) red_u[warp] = upto;
+                __syncthreads();
+                const uint32_t w = red_u[lane], all = __reduce_add_sync(0xffffffffu, w);
+                uint32_t left = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u) + upto - own;       // equal ones before this piece
+                left = quota > left ? quota - left : 0u;
+                for (uint32_t m = equal; m && left; m &= m - 1u, --left) keep |= m & (0u - m);
+                quota -= min(quota, all);
+            } else if (quota != 0) keep |= equal;
+            for (; keep; keep &= keep - 1u) {
+                const int j = __ffs(keep) - 1;
+                offer(i + j, piece_bits(x[v], j));
+            }
+        }
+    }
+    for (uint32_t i0 = VEC ? hi : lo; i0 < hi; i0 += SF_THREADS) {
         const uint32_t i = i0 + tid;
         const uint16_t bits = i < hi ? masked_bits(i) : (uint16_t)0xFF80u;
         const uint32_t key = i < hi ? bf16_key(bits) + 1u : 0u;
@@ -488,14 +573,16 @@ void uzu_unified_sampling_encode(uzu_command_buffer* cmd, const uzu_unified_samp
             uzu::after_launch(cmd, "sampling_walk_kernel");
             return;
         }
-        static std::atomic<uint64_t> smem_opt_in{0};
-        uzu::opt_in_dynamic_smem(cmd, uzu::sampling_filtered_kernel, (int)uzu::SF_SMEM, smem_opt_in);
+        const bool pieces = uzu::sampling_whole_pieces(*a) && a->vocab_size <= uzu::SF_CTAS * uzu::SF_THREADS * 8u * uzu::SF_PIECES;
+        const auto kernel = pieces ? uzu::sampling_filtered_kernel<true> : uzu::sampling_filtered_kernel<false>;
+        static std::atomic<uint64_t> smem_opt_in[2];
+        uzu::opt_in_dynamic_smem(cmd, kernel, (int)uzu::SF_SMEM, smem_opt_in[pieces]);
         for (uint32_t row0 = 0; row0 < a->batch_size; row0 += 65535u) {      // (rows are the grid's y axis)
             uzu_unified_sampling_args b = *a;
             b.logits += (uint64_t)row0 * a->vocab_size * 2; b.output += (uint64_t)row0 * 4; b.seeds += a->is_stochastic ? (uint64_t)row0 * 8 : 0;
             b.bitmask += a->has_bitmask ? (uint64_t)row0 * ((a->vocab_size + 31) / 32) * 4 : 0;
             b.batch_size = std::min(65535u, a->batch_size - row0);
-            uzu::launch(cmd, "sampling_filtered_kernel", uzu::sampling_filtered_kernel, dim3(uzu::SF_CTAS, b.batch_size), dim3(uzu::SF_THREADS), uzu::SF_SMEM, b);
+            uzu::launch(cmd, "sampling_filtered_kernel", kernel, dim3(uzu::SF_CTAS, b.batch_size), dim3(uzu::SF_THREADS), uzu::SF_SMEM, b);
         }
         return;
     }
@@ -505,7 +592,7 @@ void uzu_unified_sampling_encode(uzu_command_buffer* cmd, const uzu_unified_samp
     for (uint32_t row0 = 0; row0 < a->batch_size; row0 += uzu::SAMPLING_ROWS_PER_LAUNCH) {
         const uint32_t rows = std::min(uzu::SAMPLING_ROWS_PER_LAUNCH, a->batch_size - row0);
         dim3 grid(nblocks, rows);
-        uzu::launch(cmd, "sampling_argmax_kernel", uzu::sampling_argmax_kernel, grid, dim3(1024), 0, *a, row0, ctx->sampling_ws, tickets);
+        uzu::launch(cmd, "sampling_argmax_kernel", uzu::sampling_whole_pieces(*a) ? uzu::sampling_argmax_kernel<true> : uzu::sampling_argmax_kernel<false>, grid, dim3(1024), 0, *a, row0, ctx->sampling_ws, tickets);
     }
 }
 
