@@ -19,9 +19,16 @@
 // its partial tiles over distributed shared memory in rank order (the same bits every time).
 // (Tried instead: integer codes as one plane, group scales applied to the partial sums as they leave tensor memory. Half the products, but reading
 // 128 x NT partial sums per 64 k costs more than that: 815 us at the size above.)
+// Tiles of up to 64 rows of ZeroPoint / Symmetric weights in groups of 64 and more take ONE plane, the integers code - zp (exact in bf16): half the products,
+// half the stores to tensor memory and no scale in the dequant warps. A chain of at most 128 k inside a group is summed unscaled; the epilogue warps (eight
+// for 64 rows) bring each chain to their sums with one rounded multiply-add by its scale. For wider tiles reading 128 x NT sums per 64 k costs more than the
+// second plane (128 rows: 180 us with two planes, 187 with one). A layer of an 8B model, two planes / integers: 40 rows 153 / 140 us, in groups of 128
+// 160 / 131, 8-bit 201 / 176; 60 rows 170 / 155; groups of 32 187 / 225, so they keep the planes.
 //
 // Bounds, per block and CTA: the tensor pipe 4 NT cycles; the dequant warps about 230 instructions each, four warps a block. Prompts are bound by the
-// tensor pipe (half of its rate is the most two planes can give), few rows by the codes' way: HBM, then the dequant warps' issue slots.
+// tensor pipe (half of its rate is the most two planes can give), few rows by the product
+// warp's way from one block to the next (about 740 cycles, 490 of them outside its waits) and, with one plane, the epilogue's per chain (650); more dequant
+// groups and a product role of one lane changed nothing.
 // Every barrier wait is bounded (about a second): a wait that runs out is reported (wait_errors.h: the call then fails on the host) and the CTA ends its work.
 #include <cuda.h>
 
@@ -41,6 +48,7 @@ struct QsParams {
     unsigned int* error;
     uint32_t m, n, k, groups, zp_stride, gshift, xor_mask, method;
     uint32_t nkb, split_kb, splits, items, m_tiles;
+    uint32_t chain_k;                // PL = 1: k of a chain, 64 or 128: a group or a part of one
     uint32_t d_is_f32, accumulate, has_soft_cap, plain;
     float ab_scale, soft_cap;
 };
@@ -51,17 +59,20 @@ constexpr uint32_t QS_CODE_TILE = 128 * 128;
 
 template <int NT, int PL>
 struct QsShape {
-    static constexpr int DG = NT > 128 || NT == 64 || PL == 3 ? 3 : 4;       // dequant groups: a block takes one about 2000 cycles, hardly a third of them issuing
-    static constexpr int ND = NT > 64 ? 1 : 2;                               // accumulators in tensor memory
+    // PL = 1: the codes as integers; a group's sum is scaled as it leaves tensor memory
+    static constexpr int EW = PL == 1 && NT == 64 ? 8 : 4, EC = NT * 4 / EW;      // epilogue warps and the columns of one
+    // dequant groups: a block takes one about 2000 cycles, hardly a third of them issuing
+    static constexpr int DG = PL == 1 && NT < 64 ? 4 : NT > 128 || NT == 64 || PL == 3 ? 3 : 4;
+    static constexpr int ND = PL == 1 ? 4 : NT > 64 ? 1 : 2;    // accumulators in tensor memory
     static constexpr int CHAIN = NT > 64 ? 0 : 2;                            // blocks whose products share an accumulator (0: all)
-    static constexpr int AS = NT > 192 || PL == 3 ? 4 : NT > 128 ? 5 : 6;    // weight blocks in tensor memory: 32 columns a plane
+    static constexpr int AS = PL == 1 ? 8 : NT > 192 || PL == 3 ? 4 : NT > 128 ? 5 : 6;    // weight blocks in tensor memory: 32 columns a plane
     static constexpr int BS = NT > 192 ? 2 : NT > 64 ? 3 : 4;                // activation stages of 128 k
     static constexpr int CS = NT > 64 ? 4 : 8;                               // code tiles
-    static constexpr int THREADS = (4 + 4 * DG + 3) * 32;
+    static constexpr int THREADS = (EW + 4 * DG + 3) * 32;
     static constexpr uint32_t ACT = NT * 256, COLS = 32 * PL, A_COL = 512 - COLS * AS;
     static constexpr size_t SMEM = (size_t)BS * ACT + (size_t)CS * QS_CODE_TILE + 1024;
     static_assert(ND * NT <= (int)A_COL && DG < AS, "tensor memory columns; a group never waits for its own block");
-    static_assert(CHAIN % 2 == 0 && (CHAIN == 0 || ND == 2), "a chain is whole activation stages; the next one runs while its sums are taken");
+    static_assert(PL == 1 || (CHAIN % 2 == 0 && (CHAIN == 0 || ND == 2)), "a chain is whole activation stages; the next one runs while its sums are taken");
     static_assert((size_t)NT * 512 <= (size_t)BS * ACT + (size_t)CS * QS_CODE_TILE, "the split-k exchange reuses the rings");
 };
 
@@ -163,6 +174,23 @@ __device__ __forceinline__ void qs_dequant8(uint32_t q, uint32_t zh2, uint32_t z
     hi[0] = __byte_perm(h[0], h[1], 0x5410); hi[1] = __byte_perm(h[0], h[1], 0x7632);
     lo[0] = __byte_perm(l[0], l[1], 0x5410); lo[1] = __byte_perm(l[0], l[1], 0x7632);
 }
+// the same codes as integers code - zp, exact in bf16
+__device__ __forceinline__ void qs_integers4(uint32_t q, uint32_t z2, uint32_t* v) {
+    uint32_t d[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) d[p] = qs_u(__hsub2(qs_b2(((q >> (4 * p)) & 0x000F000Fu) | 0x43004300u), qs_b2(z2)));
+    v[0] = __byte_perm(d[0], d[1], 0x5410); v[1] = __byte_perm(d[2], d[3], 0x5410); v[2] = __byte_perm(d[0], d[1], 0x7632); v[3] = __byte_perm(d[2], d[3], 0x7632);
+}
+__device__ __forceinline__ void qs_integers8(uint32_t q, uint32_t zh2, uint32_t zl2, uint32_t* v) {
+    uint32_t d[2];
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const __nv_bfloat162 dl = __hsub2(qs_b2(((q >> (8 * p)) & 0x000F000Fu) | 0x43004300u), qs_b2(zl2));
+        const __nv_bfloat162 dh = __hsub2(qs_b2(((q >> (8 * p + 4)) & 0x000F000Fu) | 0x43004300u), qs_b2(zh2));
+        d[p] = qs_u(__hfma2(qs_b2(0x41804180u), dh, dl));
+    }
+    v[0] = __byte_perm(d[0], d[1], 0x5410); v[1] = __byte_perm(d[0], d[1], 0x7632);
+}
 // MLX: the reference's scale * code + bias in f32, then its planes: bf16 of what is left, three hold all of it
 template <int PL>
 __device__ __forceinline__ void qs_planes_f32(float w0, float w1, uint32_t (&plane)[PL][16], uint32_t at) {
@@ -180,7 +208,7 @@ __device__ __forceinline__ void qs_planes_f32(float w0, float w1, uint32_t (&pla
 template <int BITS, int NT, int PL>
 __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const QsParams p) {
     using S = QsShape<NT, PL>;
-    constexpr int DG = S::DG, ND = S::ND, AS = S::AS, BS = S::BS, CS = S::CS, DQ_WARPS = 4 * DG;
+    constexpr int DG = S::DG, ND = S::ND, AS = S::AS, BS = S::BS, CS = S::CS, DQ_WARPS = 4 * DG, EW = S::EW, EC = S::EC;
     constexpr uint32_t kpt = BITS == 4 ? 4u : 2u;                            // k blocks per code tile
     extern __shared__ uint8_t qs_raw[];
     __shared__ __align__(8) uint64_t bars[2 * CS + 2 * BS + 2 * AS + 2 * ND];
@@ -203,7 +231,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
             for (int i = 0; i < CS; ++i) { qs_init(code_full(i), 1); qs_init(code_empty(i), DQ_WARPS); }
             for (int i = 0; i < BS; ++i) { qs_init(act_full(i), 1); qs_init(act_empty(i), 1); }
             for (int i = 0; i < AS; ++i) { qs_init(a_full(i), 4); qs_init(a_empty(i), 1); }
-            for (int i = 0; i < ND; ++i) { qs_init(d_full(i), 1); qs_init(d_empty(i), 4); }
+            for (int i = 0; i < ND; ++i) { qs_init(d_full(i), 1); qs_init(d_empty(i), EW); }
             gave_up = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -225,12 +253,12 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
     auto item_n = [&](uint32_t item) { return item / p.m_tiles * 128u; };
     auto item_m = [&](uint32_t item) { return item % p.m_tiles * (uint32_t)NT; };
 
-    if (warp < 4) {
+    if (warp < (uint32_t)EW) {
         // ================================ finished tiles ================================
         uint32_t buf = 0, ph = 0;
         pdl_wait();                                                      // D may be read (accumulate) and is written below
         for (uint32_t item = item0; item < p.items; item += item_step) {
-            const uint32_t f = warp * 32u + lane, row = item_n(item) + f, t0 = item_m(item);
+            const uint32_t lanes = (warp & 3u) * 32u, cb = (warp >> 2) * EC, f = lanes + lane, row = item_n(item) + f, t0 = item_m(item);      // cb: this warp's first column
             auto finish = [&](float sum, uint32_t token) {
                 if (token >= p.m || row >= p.n) return;
                 const size_t at = (size_t)token * p.n + row;
@@ -243,10 +271,11 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
             };
             const uint32_t columns = min((uint32_t)NT, p.m - t0);
             bool ok = true;
-            float acc[S::CHAIN ? NT : 1];                                // sums of the chains (CHAIN = 0: they stay in tensor memory until they are stored)
-            if constexpr (S::CHAIN != 0) {
+            constexpr bool kSums = PL == 1 || S::CHAIN != 0;
+            float acc[kSums ? EC : 1];                                   // sums of the chains (else they stay in tensor memory until they are stored)
+            if constexpr (kSums) {
 #pragma unroll
-                for (int c = 0; c < NT; ++c) acc[c] = 0.0f;
+                for (int c = 0; c < EC; ++c) acc[c] = 0.0f;
             }
             auto next = [&]() {
                 qs_fence_before();
@@ -254,6 +283,34 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                 if (lane == 0) qs_arrive(d_empty(buf));
                 if (++buf == (uint32_t)ND) { buf = 0; ph ^= 1u; }
             };
+            if constexpr (PL == 1) {
+                // a chain is a group or a part of one: its exact integer products were summed unscaled; one rounded multiply-add brings it to the sums
+                const uint32_t chains = (nk * 64u + p.chain_k - 1) / p.chain_k, last = p.groups - 1u;
+                const uint16_t* srow = reinterpret_cast<const uint16_t*>(p.scales) + (size_t)min(row, p.n - 1u) * p.groups;
+                auto scale_of = [&](uint32_t i) { return (uint32_t)__ldg(srow + min((kb0 * 64u + i * p.chain_k) >> p.gshift, last)); };
+                uint32_t ahead[4];                                       // scales of the next four chains
+#pragma unroll
+                for (int u = 0; u < 4; ++u) ahead[u] = scale_of(u);
+                for (uint32_t i0 = 0; i0 < chains && ok; i0 += 4) {
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        if (i0 + u >= chains || !ok) continue;
+                        ok = qs_wait(d_full(buf), ph, &gave_up, p.error, 0x101u);
+                        qs_fence_after();
+                        const float scale = __uint_as_float(ahead[u] << 16);
+                        ahead[u] = scale_of(i0 + u + 4);
+#pragma unroll
+                        for (uint32_t c0 = 0; c0 < (uint32_t)EC; c0 += 16) {
+                            if (cb + c0 >= columns || !ok) continue;
+                            uint32_t v[16];
+                            qs_tmem_ld16(tmem + (lanes << 16) + buf * NT + cb + c0, v);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) acc[c0 + j] = fmaf(scale, __uint_as_float(v[j]), acc[c0 + j]);
+                        }
+                        if (ok) next();
+                    }
+                }
+            } else
             for (uint32_t i = 0; i < (S::CHAIN ? nk : 1u) && ok; i += S::CHAIN ? S::CHAIN : 1) {
                 ok = qs_wait(d_full(buf), ph, &gave_up, p.error, 0x101u);
                 qs_fence_after();
@@ -271,10 +328,10 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
             }
             // f(c0, the sums of columns c0 .. c0 + 15) for the tile's columns
             auto each16 = [&](auto f) {
-                if constexpr (S::CHAIN != 0) {
+                if constexpr (kSums) {
 #pragma unroll
-                    for (uint32_t c0 = 0; c0 < (uint32_t)NT; c0 += 16)
-                        if (c0 < columns && ok) f(c0, acc + c0);
+                    for (uint32_t c0 = 0; c0 < (uint32_t)EC; c0 += 16)
+                        if (cb + c0 < columns && ok) f(cb + c0, acc + c0);
                 } else {
                     for (uint32_t c0 = 0; c0 < columns && ok; c0 += 16) {
                         uint32_t v[16];
@@ -285,7 +342,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
             };
             if (p.splits == 1 && p.plain && item_n(item) + 128u <= p.n) {
                 // D is the rounded sum: a store per column (64 neighbouring bytes a warp), no more than an address step between them
-                __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.d) + (size_t)t0 * p.n + row;
+                __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.d) + (size_t)(t0 + cb) * p.n + row;
                 each16([&](uint32_t c0, const float* v) {
                     if (c0 + 16 <= columns) {
 #pragma unroll
@@ -308,7 +365,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                     for (int j = 0; j < 16; ++j) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + ((c0 + j) * 128u + f) * 4u), "f"(v[j]) : "memory");
                 });
                 qs_cluster_sync();
-                for (uint32_t j = rank; j < columns && ok; j += p.splits) {
+                for (uint32_t j = rank + p.splits * (warp >> 2); j < columns && ok; j += p.splits * (EW / 4)) {
                     float part[8];
 #pragma unroll
                     for (uint32_t q = 0; q < 8; ++q) {
@@ -326,11 +383,11 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                 break;                                                   // (one item per cluster)
             }
             if (!ok) break;
-            if constexpr (S::CHAIN == 0) next();
+            if constexpr (!kSums) next();
         }
-    } else if (warp < (uint32_t)(4 + DQ_WARPS)) {
+    } else if (warp < (uint32_t)(EW + DQ_WARPS)) {
         // ================================ codes -> two bf16 planes in tensor memory ================================
-        const uint32_t dg = (warp - 4) >> 2, lw = warp & 3u, r = lw * 32u + lane;
+        const uint32_t dg = (warp - EW) >> 2, lw = warp & 3u, r = lw * 32u + lane;
         const bool mlx = PL == 3 || p.method == UZU_QMETHOD_SCALE_BIAS, has_zp = p.method == UZU_QMETHOD_SCALE_ZERO_POINT, halves = p.gshift == 5u;
         uint32_t turn = 0, stage = dg, a_ph = 1, slot = 0, c_ph = 0;     // whose block it is; this group's next weight block; code tile
         bool ok = true;
@@ -345,7 +402,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                 uint32_t c = BITS == 4 ? 8u : 128u;
                 if (mlx) c = crow[g];
                 else if (has_zp) c = BITS == 4 ? (uint32_t)(zrow[g >> 1] >> (4u * (g & 1u))) & 15u : (uint32_t)zrow[g];
-                return (uint32_t)srow[g] | c << 16;
+                return (PL == 1 ? 0u : (uint32_t)srow[g]) | c << 16;
             };
             auto first_block = [&]() -> uint32_t { return (dg + DG - turn) % DG; };      // blocks until this group's turn
             uint32_t f_next[2];
@@ -372,13 +429,16 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                     const uint32_t t_col = tmem + ((lw * 32u) << 16) + S::A_COL + stage * S::COLS;
 #pragma unroll
                     for (uint32_t h = 0; h < 2; ++h) {                   // 32 k at a time
-                        uint32_t plane[PL][16], (&hi)[16] = plane[0], (&lo)[16] = plane[1];
+                        uint32_t plane[PL][16], (&hi)[16] = plane[0], (&lo)[16] = plane[PL > 1 ? 1 : 0];
                         const uint32_t s1 = f_cur[h] & 0xFFFFu, z = f_cur[h] >> 16, s2 = s1 * 0x00010001u;
                         if constexpr (BITS == 4) {
                             uint32_t q[4];
                             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(line + (((j * 2 + h) ^ (r & 7u)) << 4)));
-                            if (!mlx) {
-                                const uint32_t z2 = (0x4300u | z) * 0x00010001u;      // bf16 128 + zp
+                            const uint32_t z2 = (0x4300u | z) * 0x00010001u;      // bf16 128 + zp
+                            if constexpr (PL == 1) {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) qs_integers4(q[i] ^ p.xor_mask, z2, hi + 4 * i);
+                            } else if (!mlx) {
 #pragma unroll
                                 for (int i = 0; i < 4; ++i) qs_dequant4(q[i] ^ p.xor_mask, z2, s2, hi + 4 * i, lo + 4 * i);
                             } else {
@@ -394,8 +454,11 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                             for (uint32_t i2 = 0; i2 < 2; ++i2) {
                                 uint32_t q[4];
                                 asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(line + (((j * 4 + h * 2 + i2) ^ (r & 7u)) << 4)));
-                                if (!mlx) {
-                                    const uint32_t zh2 = (0x4300u | (z >> 4)) * 0x00010001u, zl2 = (0x4300u | (z & 15u)) * 0x00010001u;
+                                const uint32_t zh2 = (0x4300u | (z >> 4)) * 0x00010001u, zl2 = (0x4300u | (z & 15u)) * 0x00010001u;
+                                if constexpr (PL == 1) {
+#pragma unroll
+                                    for (int i = 0; i < 4; ++i) qs_integers8(q[i] ^ p.xor_mask, zh2, zl2, hi + 8 * i2 + 2 * i);
+                                } else if (!mlx) {
 #pragma unroll
                                     for (int i = 0; i < 4; ++i) qs_dequant8(q[i] ^ p.xor_mask, zh2, zl2, s2, hi + 8 * i2 + 2 * i, lo + 8 * i2 + 2 * i);
                                 } else {
@@ -432,7 +495,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
         }
         if (p.splits > 1) qs_cluster_sync();
     } else {
-        const uint32_t role = warp - (4 + DQ_WARPS);
+        const uint32_t role = warp - (EW + DQ_WARPS);
         bool ok = true;
         if (role == 0) {
             // ================================ codes by TMA (they depend on no kernel) ================================
@@ -476,6 +539,35 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
             const uint32_t desc_lo = (act0 >> 4) | (1u << 16);
             uint32_t bs = 0, bs_ph = 0, as = 0, as_ph = 0, buf = 0, d_ph = 1;
             for (uint32_t item = item0; item < p.items && ok; item += item_step) {
+                if constexpr (PL == 1) {
+                    const bool pairs = p.chain_k == 128u;                // a chain is two blocks or one
+                    for (uint32_t i = 0; i < nk && ok; i += 2) {
+                        ok = qs_wait(act_full(bs), bs_ph, &gave_up, p.error, 0x106u);
+#pragma unroll
+                        for (uint32_t half = 0; half < 2; ++half) {
+                            if (i + half >= nk || !ok) continue;
+                            const bool begins = !pairs || half == 0, ends = !pairs || half == 1 || i + half + 1 >= nk;
+                            ok = qs_wait(a_full(as), as_ph, &gave_up, p.error, 0x107u);
+                            if (begins && ok) ok = qs_wait(d_empty(buf), d_ph, &gave_up, p.error, 0x108u);
+                            if (!ok) break;
+                            qs_fence_after();
+                            if (qs_elect()) {
+                                const uint32_t d = tmem + buf * NT, a_col = tmem + S::A_COL + as * S::COLS, lo = desc_lo + (bs * S::ACT + half * (S::ACT / 2) >> 4);
+#pragma unroll
+                                for (uint32_t kk = 0; kk < 4; ++kk) qs_mma(d, a_col + kk * 8u, desc_hi | (lo + kk * 2u), idesc, !begins || kk != 0 ? 1u : 0u);
+                                qs_commit(a_empty(as));
+                                if (ends) qs_commit(d_full(buf));
+                            }
+                            __syncwarp();
+                            if (++as == (uint32_t)AS) { as = 0; as_ph ^= 1u; }
+                            if (ends && ++buf == (uint32_t)ND) { buf = 0; d_ph ^= 1u; }
+                        }
+                        if (!ok) break;
+                        if (qs_elect()) qs_commit(act_empty(bs));
+                        __syncwarp();
+                        if (++bs == (uint32_t)BS) { bs = 0; bs_ph ^= 1u; }
+                    }
+                } else
                 for (uint32_t i = 0; i < nk && ok; i += 2) {
                     const bool begins = S::CHAIN ? i % (S::CHAIN ? S::CHAIN : 1) == 0 : i == 0, ends = i + 2 >= nk || (S::CHAIN && (i + 2) % (S::CHAIN ? S::CHAIN : 1) == 0);
                     const uint32_t d = tmem + buf * NT;
@@ -572,14 +664,15 @@ struct QsPlan { int nt = 0; uint32_t splits = 1; float cost = 1e30f; };
 
 // Cycles of one CTA per 64 k of a tile, as measured: a product takes about 64 cycles however few its rows are and the product warp's waits come on top
 // (16 rows 850, 128 rows 940), wide tiles run at the tensor pipe (256 rows 1240); MLX and 8-bit codes keep the dequant warps busier than that.
-float qs_block_cycles(int nt, uint32_t bits, bool mlx, bool three) {
+float qs_block_cycles(int nt, uint32_t bits, bool mlx, bool three, bool integers) {
+    if (integers) return bits == 4 ? 700.0f + 0.7f * nt : 760.0f + 0.7f * nt;
     const float products = std::max(850.0f + 0.7f * nt, 4.85f * nt) * (three ? 1.5f : 1.0f), turn = mlx ? 4000.0f : bits == 4 ? 2000.0f : 2800.0f;
     return std::max(products, turn / (nt > 128 || nt == 64 || three ? 3.0f : 4.0f));
 }
 
 // Rows per tile and CTAs per tile: the shortest estimated time over the chip. A wider tile turns its codes once for more rows; a narrower one or a
 // split k fills the chip where tiles are few. Fixed cost per item: filling the pipeline and storing the tile.
-QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, bool three, uint32_t sms) {
+QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, bool three, bool integers, uint32_t sms) {
     QsPlan best;
     const uint32_t n_tiles = (n + 127u) / 128u;
     for (int nt : {16, 32, 64, 128, 192, 256}) {
@@ -589,7 +682,7 @@ QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, bo
         for (uint32_t splits = 1; splits <= 8; splits *= 2) {
             const uint32_t per = ((nkb + splits - 1) / splits + 3u) & ~3u;           // whole code tiles per rank
             if (splits > 1 && (per * (splits - 1) >= nkb || tiles * splits > sms)) break;
-            const float item = (float)std::min(per, nkb) * qs_block_cycles(nt, bits, mlx, three) + 2500.0f + (nt > 64 ? 12.0f * nt : 0.0f) + (splits > 1 ? 1500.0f + 8.0f * nt : 0.0f);
+            const float item = (float)std::min(per, nkb) * qs_block_cycles(nt, bits, mlx, three, integers && nt < 128) + 2500.0f + (nt > 64 ? 12.0f * nt : 0.0f) + (splits > 1 ? 1500.0f + 8.0f * nt : 0.0f);
             const uint32_t waves = (tiles * splits + sms - 1) / sms;
             const float cost = waves * item;
             if (cost < best.cost) best = {nt, splits, cost};
@@ -654,8 +747,9 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     p.d = (void*)a.d;
     uzu_context* ctx = cmd->ctx;
     // MLX weights of passes that the kernels before this one summed with the codes as integers keep all their bits; longer ones had two planes always
-    const bool three = p.biases && p.m < 64;
-    QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, three, (uint32_t)ctx->sm_count);
+    const bool three = p.biases && p.m < 64, integers = !p.biases && a.b_group_size >= 64;      // (integers: tiles of up to 64 rows)
+    p.chain_k = std::min(a.b_group_size, 128u);
+    QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, three, integers, (uint32_t)ctx->sm_count);
     if (g_tile_rows) plan.nt = g_tile_rows;
     if (g_tile_splits) {
         plan.splits = (uint32_t)g_tile_splits;
@@ -675,9 +769,9 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     auto go = [&](auto bits_c) {
         constexpr int BITS = decltype(bits_c)::value;
         switch (plan.nt) {
-            case 16: three ? qs_launch<BITS, 16, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 16, 2>(cmd, mw, mx, p, grid); break;
-            case 32: three ? qs_launch<BITS, 32, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 32, 2>(cmd, mw, mx, p, grid); break;
-            case 64: three ? qs_launch<BITS, 64, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 64, 2>(cmd, mw, mx, p, grid); break;
+            case 16: integers ? qs_launch<BITS, 16, 1>(cmd, mw, mx, p, grid) : three ? qs_launch<BITS, 16, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 16, 2>(cmd, mw, mx, p, grid); break;
+            case 32: integers ? qs_launch<BITS, 32, 1>(cmd, mw, mx, p, grid) : three ? qs_launch<BITS, 32, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 32, 2>(cmd, mw, mx, p, grid); break;
+            case 64: integers ? qs_launch<BITS, 64, 1>(cmd, mw, mx, p, grid) : three ? qs_launch<BITS, 64, 3>(cmd, mw, mx, p, grid) : qs_launch<BITS, 64, 2>(cmd, mw, mx, p, grid); break;
             case 128: qs_launch<BITS, 128, 2>(cmd, mw, mx, p, grid); break;
             case 192: qs_launch<BITS, 192, 2>(cmd, mw, mx, p, grid); break;
             default: qs_launch<BITS, 256, 2>(cmd, mw, mx, p, grid); break;
