@@ -570,6 +570,32 @@ __global__ void decode_step_end_kernel(DecodeState* st, const uint32_t* sampled,
 
 using namespace uzu;
 
+namespace uzu {
+
+// A captured step, for contexts up to `bucket`. An engine keeps a few: sequences that are restored, or prompts of other lengths, go back and forth over a
+// bucket's edge, and a capture costs as much as a step (decoding 16 tokens from 500 on and again from a snapshot: 5.74 ms a time with one graph).
+struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    uint32_t bucket = 0, sequences = 1;
+    uint64_t launches = 0;
+    uzu_sampling_method sampling{};     // baked into the captured sampling launch (seed excluded: it lives in DecodeState)
+    const void* workspace = nullptr;    // the attention workspace whose address was captured
+};
+constexpr size_t MAX_STEP_GRAPHS = 4;
+
+// room for one more; the stream is idle
+static void drop_oldest_step_graph(std::vector<StepGraph>& graphs) {
+    if (graphs.size() < MAX_STEP_GRAPHS) return;
+    cudaGraphExecDestroy(graphs.front().exec);
+    graphs.erase(graphs.begin());
+}
+static void drop_step_graphs(std::vector<StepGraph>& graphs) {
+    for (StepGraph& g : graphs) cudaGraphExecDestroy(g.exec);
+    graphs.clear();
+}
+
+}  // namespace uzu
+
 struct uzu_engine {
     uzu_context* ctx = nullptr;
     uzu_engine_options opts{};
@@ -664,19 +690,13 @@ struct uzu_engine {
     Buf batch_attn;                // partial attention results of a batched step, for sequences of any length (a captured step holds its address)
     Buf batch_pos;                 // device u32[16]: per-sequence prefix lengths (the captured batched step reads positions from here)
     bool batch_pos_valid = false;
-    cudaGraphExec_t batch_graph = nullptr;
-    uint32_t batch_graph_bucket = 0, batch_graph_B = 0;
-    uint64_t batch_graph_launches = 0;
+    std::vector<uzu::StepGraph> batch_graphs;
     // streaming
     uzu_sampling_method sampling{};
     uint32_t steps_issued = 0, steps_returned = 0;
     cudaEvent_t step_events[2] = {nullptr, nullptr};
     // CUDA graph of one decode step
-    cudaGraphExec_t graph_exec = nullptr;
-    uint32_t graph_bucket = 0;
-    bool graph_stochastic = false;
-    uzu_sampling_method graph_sampling{};   // the method baked into the captured sampling launch (seed excluded: it lives in DecodeState)
-    uint64_t graph_launches_per_step = 0;
+    std::vector<uzu::StepGraph> decode_graphs;
     bool use_pdl = true;   // programmatic dependent launch between the kernels of a decode step (UZU_NO_PDL=1 disables)
     uint64_t launches = 0;
     uzu_model_info info{};
@@ -2396,11 +2416,11 @@ static uint32_t attention_bucket(uint32_t seq) {
 }
 
 // Capture one decode step (m = 1, positions from DecodeState) into a CUDA graph.
-static void capture_decode_graph(uzu_engine* e) {
-    if (e->graph_exec) { cudaGraphExecDestroy(e->graph_exec); e->graph_exec = nullptr; }
+static StepGraph& capture_decode_graph(uzu_engine* e) {
     cudaStream_t s = e->ctx->stream;
     CmdGuard g(e->ctx, "decode-graph");
     cudaStreamSynchronize(s);
+    drop_oldest_step_graph(e->decode_graphs);
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) throw std::runtime_error("cudaStreamBeginCapture failed");
     g.c->state = uzu_command_buffer::Encoding;   // events are not recorded inside a capture
     g.c->use_pdl = e->use_pdl;
@@ -2423,19 +2443,22 @@ static void capture_decode_graph(uzu_engine* e) {
         if (graph) cudaGraphDestroy(graph);
         throw std::runtime_error(std::string("decode graph capture failed: ") + (g.c->sticky != UZU_OK ? g.c->sticky_msg : cudaGetErrorString(err)));
     }
-    err = cudaGraphInstantiate(&e->graph_exec, graph, 0);
+    StepGraph made;
+    err = cudaGraphInstantiate(&made.exec, graph, 0);
     cudaGraphDestroy(graph);
     if (err != cudaSuccess) throw std::runtime_error(std::string("cudaGraphInstantiate: ") + cudaGetErrorString(err));
-    e->graph_launches_per_step = g.c->launches;
-    e->graph_bucket = attention_bucket(e->context_length + 1);
-    e->graph_stochastic = e->sampling.kind == UZU_SAMPLING_STOCHASTIC;
-    e->graph_sampling = e->sampling;
+    made.launches = g.c->launches;
+    made.bucket = attention_bucket(e->context_length + 1);
+    made.sampling = e->sampling;
+    made.workspace = e->ctx->attn_ws;
+    e->decode_graphs.push_back(made);
+    return e->decode_graphs.back();
 }
 
 // The captured graph passes temperature / top-k / top-p / min-p by value: it is only valid for the method it was captured with.
-static bool graph_sampling_matches(const uzu_engine* e) {
-    const uzu_sampling_method &a = e->graph_sampling, &b = e->sampling;
-    return a.kind == b.kind && a.has_temperature == b.has_temperature && (!a.has_temperature || a.temperature == b.temperature) &&
+static bool graph_matches(const uzu_engine* e, const StepGraph& g) {
+    const uzu_sampling_method &a = g.sampling, &b = e->sampling;
+    return g.bucket == attention_bucket(e->context_length + 1) && g.workspace == e->ctx->attn_ws && a.kind == b.kind && a.has_temperature == b.has_temperature && (!a.has_temperature || a.temperature == b.temperature) &&
            a.has_top_k == b.has_top_k && (!a.has_top_k || a.top_k == b.top_k) && a.has_top_p == b.has_top_p && (!a.has_top_p || a.top_p == b.top_p) &&
            a.has_min_p == b.has_min_p && (!a.has_min_p || a.min_p == b.min_p);
 }
@@ -2450,11 +2473,11 @@ static void issue_decode_step(uzu_engine* e, uint64_t dev_out, uint32_t dev_out_
     if (mega_usable(e)) {
         launch_mega_step(e, dev_out, dev_out_base_step);
     } else if (e->opts.use_cuda_graph && !dev_out) {
-        if (!e->graph_exec || e->graph_bucket != attention_bucket(e->context_length + 1) || !graph_sampling_matches(e))
-            capture_decode_graph(e);
-        cudaError_t err = cudaGraphLaunch(e->graph_exec, s);
+        auto kept = std::find_if(e->decode_graphs.begin(), e->decode_graphs.end(), [&](const StepGraph& g) { return graph_matches(e, g); });
+        const StepGraph& g = kept != e->decode_graphs.end() ? *kept : capture_decode_graph(e);
+        cudaError_t err = cudaGraphLaunch(g.exec, s);
         if (err != cudaSuccess) throw std::runtime_error(std::string("cudaGraphLaunch: ") + cudaGetErrorString(err));
-        e->launches += e->graph_launches_per_step;
+        e->launches += g.launches;
     } else {
         CmdGuard g(e->ctx, "decode");
         g.c->state = uzu_command_buffer::Encoding;
@@ -2537,8 +2560,8 @@ void uzu_engine_destroy(uzu_engine* e) {
     if (!e) return;
     cudaSetDevice(e->ctx->device);
     cudaStreamSynchronize(e->ctx->stream);
-    if (e->graph_exec) cudaGraphExecDestroy(e->graph_exec);
-    if (e->batch_graph) cudaGraphExecDestroy(e->batch_graph);
+    drop_step_graphs(e->decode_graphs);
+    drop_step_graphs(e->batch_graphs);
     for (auto& S : e->state) {
         if (S.k_sparse) uzu_sparse_buffer_destroy(S.k_sparse);
         if (S.v_sparse) uzu_sparse_buffer_destroy(S.v_sparse);
@@ -2996,12 +3019,12 @@ static void encode_batch_step(uzu_engine* e, uzu_command_buffer* cmd, bool dyn, 
 
 // Capture one batched step (positions from e->batch_pos) into a CUDA graph: ~740 launches per step for Llama-3-8B x 8 sequences, which
 // the host cannot issue eagerly faster than ~22 ms; replayed as a graph the step is bound by the GPU again.
-static void capture_batch_graph(uzu_engine* e, uint32_t bucket) {
-    if (e->batch_graph) { cudaGraphExecDestroy(e->batch_graph); e->batch_graph = nullptr; }
+static StepGraph& capture_batch_graph(uzu_engine* e, uint32_t bucket) {
     const uint32_t B = (uint32_t)e->seqs.size();
     cudaStream_t s = e->ctx->stream;
     CmdGuard g(e->ctx, "batch-graph");
     cudaStreamSynchronize(s);
+    drop_oldest_step_graph(e->batch_graphs);
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) throw std::runtime_error("cudaStreamBeginCapture failed");
     g.c->state = uzu_command_buffer::Encoding;
     g.c->use_pdl = e->use_pdl;
@@ -3014,12 +3037,16 @@ static void capture_batch_graph(uzu_engine* e, uint32_t bucket) {
         if (graph) cudaGraphDestroy(graph);
         throw std::runtime_error(std::string("batch graph capture failed: ") + (g.c->sticky != UZU_OK ? g.c->sticky_msg : cudaGetErrorString(err)));
     }
-    err = cudaGraphInstantiate(&e->batch_graph, graph, 0);
+    StepGraph made;
+    err = cudaGraphInstantiate(&made.exec, graph, 0);
     cudaGraphDestroy(graph);
     if (err != cudaSuccess) throw std::runtime_error(std::string("cudaGraphInstantiate (batch): ") + cudaGetErrorString(err));
-    e->batch_graph_launches = g.c->launches;
-    e->batch_graph_bucket = bucket;
-    e->batch_graph_B = B;
+    made.launches = g.c->launches;
+    made.bucket = bucket;
+    made.sequences = B;
+    made.workspace = e->ctx->attn_ws;
+    e->batch_graphs.push_back(made);
+    return e->batch_graphs.back();
 }
 
 // one step for all sequences; the sampled tokens are chained into token_ids on the device (next step's inputs)
@@ -3042,12 +3069,12 @@ static void run_batch_step(uzu_engine* e, bool chain) {
             e->batch_pos_valid = true;
         }
         const uint32_t bucket = attention_bucket(longest);
-        if (!e->batch_graph || e->batch_graph_bucket != bucket || e->batch_graph_B != B) {
-            capture_batch_graph(e, bucket);
-        }
-        cudaError_t err = cudaGraphLaunch(e->batch_graph, e->ctx->stream);
+        auto kept = std::find_if(e->batch_graphs.begin(), e->batch_graphs.end(),
+                                 [&](const StepGraph& g) { return g.bucket == bucket && g.sequences == B && g.workspace == e->ctx->attn_ws; });
+        const StepGraph& g = kept != e->batch_graphs.end() ? *kept : capture_batch_graph(e, bucket);
+        cudaError_t err = cudaGraphLaunch(g.exec, e->ctx->stream);
         if (err != cudaSuccess) throw std::runtime_error(std::string("cudaGraphLaunch (batch): ") + cudaGetErrorString(err));
-        e->launches += e->batch_graph_launches;
+        e->launches += g.launches;
     } else {
         CmdGuard g(e->ctx, "batch step");
         g.c->state = uzu_command_buffer::Encoding;
@@ -3071,7 +3098,7 @@ static void run_batch_step(uzu_engine* e, bool chain) {
 uzu_status uzu_engine_slot_acquire(uzu_engine* e, uint32_t* out_slot) {
     UZU_ENGINE_TRY({
         if (!out_slot) throw std::runtime_error("slot_acquire: null output");
-        if (e->batch_graph) throw std::runtime_error("slot_acquire: a batched decode is active");
+        if (!e->batch_graphs.empty()) throw std::runtime_error("slot_acquire: a batched decode is active");
         e->slot_used.resize(e->seqs.size(), 0);
         uint32_t slot = 0;
         while (slot < e->slot_used.size() && e->slot_used[slot]) ++slot;
@@ -3170,12 +3197,8 @@ uzu_status uzu_engine_batch_begin(uzu_engine* e, uint32_t sequences) {
         if (e->sampling.kind == UZU_SAMPLING_STOCHASTIC) throw std::runtime_error("batch decode samples greedily (per-row seeds are not wired yet)");
         if (e->logits_rows < sequences) throw std::runtime_error("batch_begin: logits scratch too small");
         cudaStreamSynchronize(e->ctx->stream);
-        if (e->seqs.size() != sequences && e->batch_graph) {
-            // the captured batched step holds the addresses of every sequence's state: a different set of sequences needs a new capture
-            cudaGraphExecDestroy(e->batch_graph);
-            e->batch_graph = nullptr;
-            e->batch_graph_B = 0;
-        }
+        // a captured batched step holds the addresses of every sequence's state: a different set of sequences needs new captures
+        if (e->seqs.size() != sequences) drop_step_graphs(e->batch_graphs);
         size_t attn_bytes = 0;
         for (auto& L : e->layers)
             if (L.is_attention) attn_bytes = std::max(attn_bytes, attention_sequences_workspace_bytes(L.attn.num_heads, L.attn.head_dim));
