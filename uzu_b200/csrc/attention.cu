@@ -276,6 +276,9 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
         keys_per_split = ((a.sequence_length + nsplits - 1) / nsplits + 15u) & ~15u;
     } else if (a.dynamic_position) {
         a.sequence_length = *reinterpret_cast<const uint32_t*>(a.dynamic_position) + a.suffix_length;
+        // by its own length too: a captured step serves every length up to a bound, and its bits must not depend on the length it was captured at
+        nsplits = min(p.nsplits, (a.sequence_length + 63u) / 64u);
+        if (blockIdx.z >= nsplits) return;
         keys_per_split = ((a.sequence_length + nsplits - 1) / nsplits + 15u) & ~15u;   // whole CTA steps per split
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

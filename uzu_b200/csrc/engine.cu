@@ -1431,6 +1431,7 @@ struct PassCtx {
 };
 
 // q/k norms, RoPE + KV append, attention core, optional sigmoid gate: everything between the qkv and the out projections
+static uint32_t attention_bucket(uint32_t seq);
 static void encode_attention_mix(uzu_engine* e, uzu_command_buffer* cmd, const Layer& L, LayerState& S, const PassCtx& pc, bool with_gate);
 
 static uint64_t encode_attention(uzu_engine* e, uzu_command_buffer* cmd, const Layer& L, LayerState& S, uint64_t hidden, const PassCtx& pc) {
@@ -1484,7 +1485,7 @@ static void encode_attention_mix(uzu_engine* e, uzu_command_buffer* cmd, const L
     uzu_attention_args aa{};
     aa.queries = e->queries.ptr(); aa.keys = S.keys; aa.values = S.values;
     aa.gqa_factor = Hq / Hkv;
-    aa.sequence_length = prefix + m;
+    aa.sequence_length = pc.dynamic ? attention_bucket(prefix + m) : prefix + m;   // (the most a captured step may meet; the kernel cuts by the length it finds)
     aa.k_head_stride = D; aa.k_seq_stride = Hkv * D; aa.v_head_stride = D; aa.v_seq_stride = Hkv * D;
     aa.scale = A.has_scale ? A.scale : 1.0f / sqrtf((float)D);
     aa.num_heads = Hq; aa.suffix_length = m; aa.head_dim = D; aa.is_causal = A.is_causal;
@@ -1607,8 +1608,6 @@ static void encode_readout_tail(uzu_engine* e, uzu_command_buffer* cmd, uint32_t
     if (e->has_logit_scale || e->has_logit_soft_cap)
         uzu_logit_transform_encode(cmd, e->logits.ptr(), rows * e->vocab, e->has_logit_scale ? e->logit_scale : 1.0f, e->logit_soft_cap, e->has_logit_soft_cap);
 }
-
-static uint32_t attention_bucket(uint32_t seq);
 
 #include "engine_parallel_block.inl"
 
@@ -1800,7 +1799,7 @@ static void encode_decoder_fused(uzu_engine* e, uzu_command_buffer* cmd, const P
             }
             uzu_attention_args aa{};
             aa.queries = e->queries.ptr(); aa.keys = St.keys; aa.values = St.values; aa.out = e->attn_out.ptr();
-            aa.gqa_factor = Hq / Hkv; aa.sequence_length = St.length + 1;
+            aa.gqa_factor = Hq / Hkv; aa.sequence_length = attention_bucket(St.length + 1);   // the most; the kernel reads its own
             aa.k_head_stride = D; aa.k_seq_stride = Hkv * D; aa.v_head_stride = D; aa.v_seq_stride = Hkv * D;
             aa.scale = A.has_scale ? A.scale : 1.0f / sqrtf((float)D);
             aa.num_heads = Hq; aa.suffix_length = 1; aa.head_dim = D; aa.is_causal = A.is_causal; aa.dynamic_position = dyn;
@@ -2975,7 +2974,7 @@ static void encode_batch_step(uzu_engine* e, uzu_command_buffer* cmd, bool dyn, 
                     uzu_attention_prepare_encode(cmd, &pb);
                     uzu_attention_args ab = aa;
                     ab.queries = pb.queries; ab.keys = pb.keys; ab.values = pb.values; ab.out += b * q_row;
-                    ab.sequence_length = seqs.prefix[b] + 1;
+                    ab.sequence_length = dyn ? longest : seqs.prefix[b] + 1;
                     if (dyn) ab.dynamic_position = pb.dynamic_position;
                     uzu_attention_single_pass_encode(cmd, &ab);
                 }
