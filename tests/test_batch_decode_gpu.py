@@ -132,3 +132,24 @@ def test_a_sequence_does_not_depend_on_its_neighbours_lengths(ctx, uneven):
                     eng.batch_step([int(tokens[0, 0])] + [int(t) for t in toks[1:]])
                 results.append(eng.batch_logits()[0].copy())
     assert all((r == results[0]).all() for r in results)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_a_batch_samples_greedily_whatever_the_engines_own_sequence_does(ctx, tmp_path, graph):
+    """The engine's own sequence takes a stochastic method after batch_begin: prompts and steps of the batch still return their largest logit, from steps
+    captured before the change, while it lasts and after it."""
+    spec = synth.tiny("llama-512")
+    path = synth.write_model(spec, tmp_path / "m", seed=41)
+    rng = np.random.default_rng(10)
+    hot = B.Engine.sampling(seed=7, temperature=50.0)
+    prompts = [rng.integers(0, spec.vocab_size, 60) for _ in range(3)]
+    largest = lambda logits: [int(t) for t in bf16_to_f32(logits).argmax(-1)]
+    with B.Engine(ctx, path, max_context_length=512, use_cuda_graph=graph) as eng:
+        eng.batch_begin(3)
+        for sampling in (None, hot, B.Engine.sampling()):
+            eng.prefill(prompts[0], sampling)
+            for b, p in enumerate(prompts):
+                assert eng.batch_prefill(b, p) == largest(eng.last_logits())[-1]
+            for step in range(40):                  # lengths that share a captured step and lengths that do not
+                got = eng.batch_step([1, 2, 3])
+                assert got == largest(eng.batch_logits()), (step, sampling)

@@ -2329,8 +2329,7 @@ static void launch_mega_step(uzu_engine* e, uint64_t dev_out, uint32_t dev_out_b
     e->launches += 1;
 }
 
-static void encode_sampling(uzu_engine* e, uzu_command_buffer* cmd, uint32_t rows) {
-    const uzu_sampling_method& s = e->sampling;
+static void encode_sampling(uzu_engine* e, uzu_command_buffer* cmd, uint32_t rows, const uzu_sampling_method& s) {
     uzu_unified_sampling_args sa{};
     sa.logits = e->logits.ptr();
     sa.output = e->sampled.ptr();
@@ -2345,6 +2344,14 @@ static void encode_sampling(uzu_engine* e, uzu_command_buffer* cmd, uint32_t row
         sa.has_min_p = s.has_min_p; sa.min_p = s.min_p;
     }
     uzu_unified_sampling_encode(cmd, &sa);
+}
+
+// Sequences of a batch sample greedily whatever method the engine's own sequence has taken since batch_begin: there are no seeds for their rows, and a
+// captured batched step would keep the method of the moment.
+static uzu_sampling_method batch_sampling() {
+    uzu_sampling_method s{};
+    s.kind = UZU_SAMPLING_GREEDY;
+    return s;
 }
 
 static bool has_delta(const uzu_engine* e) {
@@ -2381,8 +2388,8 @@ static uint64_t prng_derive(uint64_t seed, uint64_t index) {
     return h;
 }
 
-// one non-graph pass over `count` host tokens; optionally samples the last row
-static void run_pass(uzu_engine* e, const uint32_t* tokens, uint32_t count, uint32_t row_begin, uint32_t row_end, bool sample_last) {
+// one non-graph pass over `count` host tokens; samples the last row by `sampling`, if any
+static void run_pass(uzu_engine* e, const uint32_t* tokens, uint32_t count, uint32_t row_begin, uint32_t row_end, const uzu_sampling_method* sampling) {
     if (count == 0 || count > MAX_ROWS) throw std::runtime_error("pass size must be in 1..1024");
     if (e->trie_pending) throw std::runtime_error("a speculation pass is pending: uzu_engine_trie_accept first");
     if (e->context_length + count > e->max_context + MAX_ROWS || e->context_length + count > e->rope_positions)
@@ -2395,14 +2402,14 @@ static void run_pass(uzu_engine* e, const uint32_t* tokens, uint32_t count, uint
     PassCtx pc;
     pc.m = count;
     encode_decoder(e, g.c, pc, row_begin, row_end);
-    if (sample_last) {
-        if (e->sampling.kind == UZU_SAMPLING_STOCHASTIC) {
+    if (sampling) {
+        if (sampling->kind == UZU_SAMPLING_STOCHASTIC) {
             // seed of the sampled row = PRng::derive(absolute index of its input token) (stream.rs:252-254)
-            uint64_t seed = prng_derive(e->sampling.seed, (uint64_t)e->context_length + count - 1);
+            uint64_t seed = prng_derive(sampling->seed, (uint64_t)e->context_length + count - 1);
             cudaMemcpyAsync((void*)e->seeds.ptr(), &seed, 8, cudaMemcpyHostToDevice, e->ctx->stream);
             cudaStreamSynchronize(e->ctx->stream);
         }
-        encode_sampling(e, g.c, 1);
+        encode_sampling(e, g.c, 1, *sampling);
     }
     run_cmd_to_completion(e, g.c);
     accept(e, count);
@@ -2432,7 +2439,7 @@ static StepGraph& capture_decode_graph(uzu_engine* e) {
     pc.dynamic = true;
     if (e->fused_ok) encode_decoder_fused(e, g.c, pc);
     else encode_decoder(e, g.c, pc, 0, 1);
-    encode_sampling(e, g.c, 1);
+    encode_sampling(e, g.c, 1, e->sampling);
     decode_step_end_kernel<<<1, 1, 0, s>>>((DecodeState*)e->decode_state.ptr(), (const uint32_t*)e->sampled.ptr(), (uint32_t*)e->token_ids.ptr(),
                                            (volatile uint32_t*)e->host_ring.ptr(), nullptr, 0);
     g.c->launches++;
@@ -2490,7 +2497,7 @@ static void issue_decode_step(uzu_engine* e, uint64_t dev_out, uint32_t dev_out_
         pc.dynamic = true;
         if (e->fused_ok) encode_decoder_fused(e, g.c, pc);
         else encode_decoder(e, g.c, pc, 0, 1);
-        encode_sampling(e, g.c, 1);
+        encode_sampling(e, g.c, 1, e->sampling);
         decode_step_end_kernel<<<1, 1, 0, s>>>((DecodeState*)e->decode_state.ptr(), (const uint32_t*)e->sampled.ptr(), (uint32_t*)e->token_ids.ptr(),
                                                (volatile uint32_t*)e->host_ring.ptr(), (uint32_t*)dev_out, dev_out_base_step);
         g.c->launches++;
@@ -2632,7 +2639,7 @@ uzu_status uzu_engine_prefill(uzu_engine* e, const uint32_t* tokens, uint32_t co
         for (uint32_t s0 = 0; s0 < count; s0 += step) {
             const uint32_t n = std::min(step, count - s0);
             const bool last = s0 + n == count;
-            run_pass(e, tokens + s0, n, last ? n - 1 : 0, last ? n : 0, last);
+            run_pass(e, tokens + s0, n, last ? n - 1 : 0, last ? n : 0, last ? &e->sampling : nullptr);
         }
         uint32_t tok = 0;
         cudaMemcpy(&tok, (void*)e->sampled.ptr(), 4, cudaMemcpyDeviceToHost);
@@ -2687,7 +2694,7 @@ uzu_status uzu_engine_decode_device(uzu_engine* e, uint32_t steps, uint64_t out_
 uzu_status uzu_engine_forward(uzu_engine* e, const uint32_t* tokens, uint32_t count, uint32_t row_begin, uint32_t row_end, uint16_t* out_logits) {
     UZU_ENGINE_TRY({
         if (row_end > count || row_begin > row_end || row_end - row_begin > e->logits_rows) throw std::runtime_error("forward: bad row range (<= 16 rows)");
-        run_pass(e, tokens, count, row_begin, row_end, false);
+        run_pass(e, tokens, count, row_begin, row_end, nullptr);
         if (out_logits && row_end > row_begin)
             cudaMemcpy(out_logits, (void*)e->logits.ptr(), (size_t)(row_end - row_begin) * e->vocab * 2, cudaMemcpyDeviceToHost);
     });
@@ -2746,7 +2753,7 @@ uzu_status uzu_engine_trie_pass(uzu_engine* e, const uint32_t* tokens, const uzu
         pc.m = count;
         pc.trie = e->trie_nodes.ptr();
         encode_decoder(e, g.c, pc, 0, count);        // logits for every node (stream.rs:640: Some(0..batch_dim.size()))
-        encode_sampling(e, g.c, count);
+        encode_sampling(e, g.c, count, e->sampling);
         uzu_command_buffer_encode_copy(g.c, e->sampled.ptr(), e->host_trie.ptr() + MAX_TRIE * (8 + sizeof(uzu_trie_node)) + MAX_TRIE * 4, count * 4);
         run_cmd_to_completion(e, g.c);
         if (out_tokens) memcpy(out_tokens, h_sampled, count * 4);
@@ -3013,7 +3020,7 @@ static void encode_batch_step(uzu_engine* e, uzu_command_buffer* cmd, bool dyn, 
     encode_linear(cmd, e->out_emb, e->normed_out.ptr(), B, e->logits.ptr());
     if (e->has_logit_scale || e->has_logit_soft_cap)
         uzu_logit_transform_encode(cmd, e->logits.ptr(), B * e->vocab, e->has_logit_scale ? e->logit_scale : 1.0f, e->logit_soft_cap, e->has_logit_soft_cap);
-    encode_sampling(e, cmd, B);
+    encode_sampling(e, cmd, B, batch_sampling());
 }
 
 // Capture one batched step (positions from e->batch_pos) into a CUDA graph: ~740 launches per step for Llama-3-8B x 8 sequences, which
@@ -3141,7 +3148,7 @@ uzu_status uzu_engine_forward_rows(uzu_engine* e, uint32_t slot, const uint32_t*
         uint32_t next = 0;
         for (uint32_t s0 = 0; s0 < count; s0 += MAX_ROWS) {
             const uint32_t n = std::min(MAX_ROWS, count - s0);
-            run_pass(e, tokens + s0, n, 0, 0, false);
+            run_pass(e, tokens + s0, n, 0, 0, nullptr);
             while (next < nrows && rows[next] < s0 + n) {     // contiguous runs of wanted rows, at most logits_rows at a time
                 uint32_t end = next + 1;
                 while (end < nrows && rows[end] == rows[end - 1] + 1 && rows[end] < s0 + n && end - next < e->logits_rows) ++end;
@@ -3242,10 +3249,11 @@ uzu_status uzu_engine_batch_prefill(uzu_engine* e, uint32_t sequence, const uint
         uint32_t tok = 0;
         {
             SeqSwap sw(e, sequence);    // the ordinary chunked prefill, against this sequence's state
+            const uzu_sampling_method greedy = batch_sampling();
             for (uint32_t s0 = 0; s0 < count; s0 += MAX_ROWS) {
                 const uint32_t n = std::min(MAX_ROWS, count - s0);
                 const bool last = s0 + n == count;
-                run_pass(e, tokens + s0, n, last ? n - 1 : 0, last ? n : 0, last);
+                run_pass(e, tokens + s0, n, last ? n - 1 : 0, last ? n : 0, last ? &greedy : nullptr);
             }
             cudaMemcpy(&tok, (void*)e->sampled.ptr(), 4, cudaMemcpyDeviceToHost);
         }
