@@ -988,6 +988,7 @@ UZU_API uzu_status uzu_engine_batch_decode_timed(uzu_engine* e, const uint32_t* 
 UZU_API uzu_status uzu_engine_batch_logits(uzu_engine* e, uint16_t* out_logits);
 UZU_API uint32_t uzu_engine_batch_context_length(const uzu_engine* e, uint32_t sequence);
 UZU_API uint64_t uzu_engine_launch_count(const uzu_engine* e);   /* kernels launched (incl. graph nodes replayed) */
+UZU_API uint64_t uzu_engine_debug_step_captures(const uzu_engine* e);   /* for tests: decode steps and batched steps captured into a CUDA graph so far */
 /* Measurement helpers (bench.py). All time with CUDA events recorded on the engine's stream.
  *  decode_timed: `steps` device-chained decode passes between two events; returns seconds.
  *  step_host:    one decode pass fed from and read back to HOST memory: token_in is copied host->device from pinned

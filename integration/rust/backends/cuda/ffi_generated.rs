@@ -1189,6 +1189,7 @@ extern "C" {
     pub fn uzu_engine_batch_logits(e: *mut uzu_engine, out_logits: *mut u16) -> c_int;
     pub fn uzu_engine_batch_context_length(e: *const uzu_engine, sequence: u32) -> u32;
     pub fn uzu_engine_launch_count(e: *const uzu_engine) -> u64;
+    pub fn uzu_engine_debug_step_captures(e: *const uzu_engine) -> u64;
     pub fn uzu_engine_decode_timed(e: *mut uzu_engine, steps: u32, out_seconds: *mut f64) -> c_int;
     pub fn uzu_engine_step_host(e: *mut uzu_engine, token_in: u32, token_out: *mut u32) -> c_int;
     pub fn uzu_engine_decode_mode(e: *const uzu_engine) -> c_int;

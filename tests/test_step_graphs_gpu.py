@@ -1,5 +1,5 @@
-"""Decode steps that go back and forth over the context lengths at which another captured step is taken (64, 128, ..): what is read back is what a fresh
-engine gives, for more lengths than an engine keeps captured steps, and after a change of the sampling method."""
+"""Captured decode steps. Steps that go back and forth over the context lengths at which another one is taken (64, 128, ..), a change of the sampling method
+and batches of other lengths and numbers of sequences: what is read back is what a fresh engine gives, and steps are captured no more often than they have to."""
 import ctypes as C
 import dataclasses
 
@@ -94,3 +94,86 @@ def test_attention_at_a_device_position_is_cut_by_that_position(ctx, heads, grou
             cmd.encode("uzu_attention_single_pass_encode", C.byref(a))
         results.append(out.numpy(np.uint16, (heads * dim,)))
     assert np.array_equal(results[1], results[0]) and np.array_equal(results[2], results[0])
+
+
+def test_an_engine_keeps_the_steps_it_used_last(ctx, tmp_path):
+    """Four of them: going back and forth over three ranges captures each once; five ranges in turn do not fit; a range in use survives others that come and go."""
+    spec = synth.tiny("llama")
+    path = synth.write_model(spec, tmp_path / "m", seed=3)
+    prompt = np.random.default_rng(6).integers(0, spec.vocab_size, 1100)
+    with B.Engine(ctx, path, max_context_length=2048, use_cuda_graph=True) as eng:
+        eng.set_persistent_decode(False)
+
+        def captures(*lengths):
+            before = eng.step_captures
+            for n in lengths:
+                eng.reset()
+                eng.prefill(prompt[:n])
+                eng.step_host(1)
+            return eng.step_captures - before
+        assert captures(40, 100, 200) == 3
+        assert captures(200, 40, 100, 40, 200) == 0
+        assert captures(400) == 1                             # the fourth
+        assert captures(800) == 1 and captures(100) == 1      # the fifth takes the place of the one used longest ago
+        assert captures(800, 100, 200, 400) == 0
+        assert captures(40, 800, 100, 200, 400) == 5          # five in turn: always the next one is gone
+
+
+@pytest.mark.parametrize("kind", ["llama-512", "qwen-hybrid-512"])
+def test_a_change_of_the_sampling_method(ctx, tmp_path, kind):
+    """The method is part of a captured step: ids after greedy, two stochastic methods and greedy again at the same lengths are those of fresh engines, and a
+    method that comes back finds its step."""
+    spec = synth.tiny(kind)
+    path = synth.write_model(spec, tmp_path / "m", seed=3)
+    prompt = np.random.default_rng(7).integers(0, spec.vocab_size, 50)
+    methods = [B.Engine.sampling(), B.Engine.sampling(seed=5, temperature=3.0, top_k=40), B.Engine.sampling(seed=5, temperature=30.0), B.Engine.sampling(seed=9, temperature=30.0)]
+
+    def ids(eng, method):
+        return [eng.prefill(prompt, method)] + [eng.step_host(tok) for tok in range(10)]
+
+    def fresh(method):
+        with B.Engine(ctx, path, max_context_length=512, use_cuda_graph=True) as eng:
+            eng.set_persistent_decode(False)
+            return ids(eng, method)
+    ref = [fresh(m) for m in methods]
+    assert ref[0] != ref[1] != ref[2] != ref[3]
+    with B.Engine(ctx, path, max_context_length=512, use_cuda_graph=True) as eng:
+        eng.set_persistent_decode(False)
+        before = eng.step_captures
+        for i in (0, 1, 2, 0, 3, 1, 0, 2):
+            eng.reset()
+            assert ids(eng, methods[i]) == ref[i], i
+        assert eng.step_captures - before == 3                # a seed is no part of it: methods 2 and 3 share a step
+
+
+@pytest.mark.parametrize("kind", ["llama-512", "qwen-hybrid-512"])
+def test_batches_that_come_back_to_a_length(ctx, tmp_path, kind):
+    """Kept batched steps over batch_begin: the same count of sequences keeps them, at other prompt lengths too; another count drops them."""
+    spec = synth.tiny(kind)
+    path = synth.write_model(spec, tmp_path / "m", seed=3)
+    prompt = np.random.default_rng(8).integers(0, spec.vocab_size, 300)
+
+    def batch(eng, lengths):
+        eng.batch_begin(len(lengths))
+        for b, n in enumerate(lengths):
+            eng.batch_prefill(b, prompt[b:b + n])
+        out = []
+        for tok in range(4):
+            out.append((eng.batch_step([tok + b for b in range(len(lengths))]), eng.batch_logits()))
+        return out
+
+    def fresh(lengths):
+        with B.Engine(ctx, path, max_context_length=512, use_cuda_graph=True) as eng:
+            return batch(eng, lengths)
+    shapes = [(60, 20, 62), (120, 126, 5), (250, 7, 9)]       # the longest goes over 64, over 128, stays below 256
+    ref = {s: fresh(s) for s in shapes + [(60, 20)]}
+    with B.Engine(ctx, path, max_context_length=512, use_cuda_graph=True) as eng:
+        def captures(s):
+            before = eng.step_captures
+            for (ids, logits), (want, want_logits) in zip(batch(eng, s), ref[s]):
+                assert ids == want and np.array_equal(logits, want_logits), s
+            return eng.step_captures - before
+        assert [captures(s) for s in shapes] == [2, 1, 0]     # 64 and 128, then 256
+        assert [captures(s) for s in shapes] == [0, 0, 0]
+        assert captures((60, 20)) == 1                        # below 64 only
+        assert captures(shapes[0]) == 2

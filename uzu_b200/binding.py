@@ -282,7 +282,7 @@ uzu_tensor_add_bias_encode uzu_tensor_add_swap_encode uzu_unified_sampling_encod
 uzu_delta_net_update_encode uzu_engine_create uzu_engine_destroy uzu_engine_info uzu_engine_reset uzu_engine_context_length
 uzu_engine_snapshot uzu_engine_restore uzu_engine_prefill uzu_engine_next uzu_engine_flush uzu_engine_decode_device
 uzu_engine_forward uzu_engine_batch_begin uzu_engine_batch_prefill uzu_engine_batch_step uzu_engine_batch_decode_timed
-uzu_engine_batch_logits uzu_engine_batch_context_length uzu_engine_launch_count uzu_engine_decode_timed uzu_engine_step_host
+uzu_engine_batch_logits uzu_engine_batch_context_length uzu_engine_launch_count uzu_engine_debug_step_captures uzu_engine_decode_timed uzu_engine_step_host
 uzu_delta_net_fused_update_supported uzu_delta_net_fused_update_encode uzu_engine_time_linears uzu_engine_time_prefill_linears uzu_engine_time_linears_select uzu_debug_set_qmv_tuning uzu_debug_set_delta_prefill uzu_debug_set_prefill_attention uzu_debug_set_umma uzu_debug_set_qmm_tile uzu_tp_get_unique_id uzu_context_tp_init uzu_context_tp_destroy uzu_context_tp_size
 uzu_context_tp_rank uzu_tp_p2p_export uzu_tp_p2p_import uzu_tp_all_reduce_encode uzu_tp_all_gather_encode uzu_fused_linear_supported uzu_fused_linear_encode
 uzu_engine_decode_mode uzu_engine_decode_mode_reason uzu_engine_set_decode_mode uzu_engine_last_logits uzu_engine_debug_decode_trace
@@ -392,6 +392,7 @@ def load() -> C.CDLL:
         "uzu_engine_decode_device": (C.c_int, [vp, u32, u64]),
         "uzu_engine_forward": (C.c_int, [vp, C.POINTER(u32), u32, u32, u32, C.POINTER(C.c_uint16)]),
         "uzu_engine_launch_count": (u64, [vp]),
+        "uzu_engine_debug_step_captures": (u64, [vp]),
         "uzu_engine_batch_begin": (C.c_int, [vp, u32]),
         "uzu_engine_batch_prefill": (C.c_int, [vp, u32, C.POINTER(u32), u32, C.POINTER(u32)]),
         "uzu_engine_batch_step": (C.c_int, [vp, C.POINTER(u32), C.POINTER(u32)]),
@@ -739,6 +740,10 @@ class Engine:
     @property
     def launch_count(self):
         return self.lib.uzu_engine_launch_count(self.h)
+
+    @property
+    def step_captures(self):
+        return self.lib.uzu_engine_debug_step_captures(self.h)
 
     def decode_timed(self, steps: int) -> float:
         t = C.c_double()

@@ -572,8 +572,9 @@ using namespace uzu;
 
 namespace uzu {
 
-// A captured step, for contexts up to `bucket`. An engine keeps a few: sequences that are restored, or prompts of other lengths, go back and forth over a
-// bucket's edge, and a capture costs as much as a step (decoding 16 tokens from 500 on and again from a snapshot: 5.74 ms a time with one graph).
+// A captured step, for contexts up to `bucket`. An engine keeps the few that it used last, the last one at the end: sequences that are restored, or prompts of
+// other lengths, go back and forth over a bucket's edge, and a capture costs as much as a step (decoding 16 tokens from 500 on and again from a snapshot:
+// 5.80 ms a time with one graph, 5.18 with these; an answer that crosses each length once gains nothing).
 struct StepGraph {
     cudaGraphExec_t exec = nullptr;
     uint32_t bucket = 0, sequences = 1;
@@ -583,8 +584,16 @@ struct StepGraph {
 };
 constexpr size_t MAX_STEP_GRAPHS = 4;
 
+// the kept step that `matches`, now the one used last, or nothing
+template <typename F>
+static StepGraph* find_step_graph(std::vector<StepGraph>& graphs, F&& matches) {
+    const auto kept = std::find_if(graphs.begin(), graphs.end(), matches);
+    if (kept == graphs.end()) return nullptr;
+    std::rotate(kept, kept + 1, graphs.end());
+    return &graphs.back();
+}
 // room for one more; the stream is idle
-static void drop_oldest_step_graph(std::vector<StepGraph>& graphs) {
+static void make_room_for_step_graph(std::vector<StepGraph>& graphs) {
     if (graphs.size() < MAX_STEP_GRAPHS) return;
     cudaGraphExecDestroy(graphs.front().exec);
     graphs.erase(graphs.begin());
@@ -697,6 +706,7 @@ struct uzu_engine {
     cudaEvent_t step_events[2] = {nullptr, nullptr};
     // CUDA graph of one decode step
     std::vector<uzu::StepGraph> decode_graphs;
+    uint64_t step_captures = 0;    // of both kinds, ever
     bool use_pdl = true;   // programmatic dependent launch between the kernels of a decode step (UZU_NO_PDL=1 disables)
     uint64_t launches = 0;
     uzu_model_info info{};
@@ -2426,7 +2436,7 @@ static StepGraph& capture_decode_graph(uzu_engine* e) {
     cudaStream_t s = e->ctx->stream;
     CmdGuard g(e->ctx, "decode-graph");
     cudaStreamSynchronize(s);
-    drop_oldest_step_graph(e->decode_graphs);
+    make_room_for_step_graph(e->decode_graphs);
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) throw std::runtime_error("cudaStreamBeginCapture failed");
     g.c->state = uzu_command_buffer::Encoding;   // events are not recorded inside a capture
     g.c->use_pdl = e->use_pdl;
@@ -2458,6 +2468,7 @@ static StepGraph& capture_decode_graph(uzu_engine* e) {
     made.sampling = e->sampling;
     made.workspace = e->ctx->attn_ws;
     e->decode_graphs.push_back(made);
+    ++e->step_captures;
     return e->decode_graphs.back();
 }
 
@@ -2479,8 +2490,8 @@ static void issue_decode_step(uzu_engine* e, uint64_t dev_out, uint32_t dev_out_
     if (mega_usable(e)) {
         launch_mega_step(e, dev_out, dev_out_base_step);
     } else if (e->opts.use_cuda_graph && !dev_out) {
-        auto kept = std::find_if(e->decode_graphs.begin(), e->decode_graphs.end(), [&](const StepGraph& g) { return graph_matches(e, g); });
-        const StepGraph& g = kept != e->decode_graphs.end() ? *kept : capture_decode_graph(e);
+        const StepGraph* kept = find_step_graph(e->decode_graphs, [&](const StepGraph& g) { return graph_matches(e, g); });
+        const StepGraph& g = kept ? *kept : capture_decode_graph(e);
         cudaError_t err = cudaGraphLaunch(g.exec, s);
         if (err != cudaSuccess) throw std::runtime_error(std::string("cudaGraphLaunch: ") + cudaGetErrorString(err));
         e->launches += g.launches;
@@ -2797,6 +2808,7 @@ uzu_status uzu_engine_trie_accept(uzu_engine* e, const uint32_t* accepted_indice
 }
 
 uint64_t uzu_engine_launch_count(const uzu_engine* e) { return e ? e->launches : 0; }
+uint64_t uzu_engine_debug_step_captures(const uzu_engine* e) { return e ? e->step_captures : 0; }
 
 // ---- persistent decode kernel controls (extension) ----
 int uzu_engine_decode_mode(const uzu_engine* e) { return e && e->mega.ok ? 1 : 0; }
@@ -3030,7 +3042,7 @@ static StepGraph& capture_batch_graph(uzu_engine* e, uint32_t bucket) {
     cudaStream_t s = e->ctx->stream;
     CmdGuard g(e->ctx, "batch-graph");
     cudaStreamSynchronize(s);
-    drop_oldest_step_graph(e->batch_graphs);
+    make_room_for_step_graph(e->batch_graphs);
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) throw std::runtime_error("cudaStreamBeginCapture failed");
     g.c->state = uzu_command_buffer::Encoding;
     g.c->use_pdl = e->use_pdl;
@@ -3052,6 +3064,7 @@ static StepGraph& capture_batch_graph(uzu_engine* e, uint32_t bucket) {
     made.sequences = B;
     made.workspace = e->ctx->attn_ws;
     e->batch_graphs.push_back(made);
+    ++e->step_captures;
     return e->batch_graphs.back();
 }
 
@@ -3075,9 +3088,8 @@ static void run_batch_step(uzu_engine* e, bool chain) {
             e->batch_pos_valid = true;
         }
         const uint32_t bucket = attention_bucket(longest);
-        auto kept = std::find_if(e->batch_graphs.begin(), e->batch_graphs.end(),
-                                 [&](const StepGraph& g) { return g.bucket == bucket && g.sequences == B && g.workspace == e->ctx->attn_ws; });
-        const StepGraph& g = kept != e->batch_graphs.end() ? *kept : capture_batch_graph(e, bucket);
+        const StepGraph* kept = find_step_graph(e->batch_graphs, [&](const StepGraph& g) { return g.bucket == bucket && g.sequences == B && g.workspace == e->ctx->attn_ws; });
+        const StepGraph& g = kept ? *kept : capture_batch_graph(e, bucket);
         cudaError_t err = cudaGraphLaunch(g.exec, e->ctx->stream);
         if (err != cudaSuccess) throw std::runtime_error(std::string("cudaGraphLaunch (batch): ") + cudaGetErrorString(err));
         e->launches += g.launches;
