@@ -9,7 +9,7 @@ from tests.util import f32_to_bf16
 pytestmark = [pytest.mark.gpu]
 
 
-@pytest.mark.parametrize("V", [32768, 65544, 262144, 262152])       # one piece per thread, a ragged second one, the most that is kept, one piece too many
+@pytest.mark.parametrize("V", [32768, 65528, 65536, 65544, 262144, 262152])       # too few pieces, one for every thread, a ragged second one, the most that is kept, one piece too many
 @pytest.mark.parametrize("kw", [dict(top_k=37), dict(top_p=0.9, temperature=0.7), dict(min_p=0.05, top_k=3000)])
 def test_filters(ctx, V, kw):
     """Values on a grid, so that the kept set ends inside a group of equals spread over threads, pieces and CTAs; masked entries among them."""
@@ -21,7 +21,7 @@ def test_filters(ctx, V, kw):
         assert np.array_equal(O.unified_sampling(logits, seeds=seeds, bitmask=bitmask, **kw), G.unified_sampling(ctx, logits, seeds=seeds, bitmask=bitmask, **kw))
 
 
-@pytest.mark.parametrize("V", [8, 8184, 8192, 8200, 229384])       # a piece, the edges of a block, more than one piece per thread
+@pytest.mark.parametrize("V", [8, 8184, 8192, 8200, 229376, 229384, 248320, 458752, 458760])       # a piece, the edges of a block, one and two pieces per thread and what is left over
 def test_greedy_and_gumbel(ctx, V):
     rng = np.random.default_rng(V)
     logits = f32_to_bf16((np.round(rng.standard_normal((3, V)) * 8) / 4).astype(np.float32))

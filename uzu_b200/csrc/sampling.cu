@@ -97,7 +97,10 @@ __device__ __forceinline__ uint16_t piece_bits(const uint4& x, int j) {
     return (uint16_t)(w >> (16 * (j & 1)));
 }
 
-// VEC: a thread's logits come in one or two 16-byte reads instead of a chain of 2-byte ones. Bound: latency (a read, the block's and the grid's maximum).
+// VEC: a thread's logits come in one or two 16-byte reads instead of a chain of 2-byte ones. Bound: latency (a read, the block's and the grid's maximum;
+// with seeds the noise of a thread's logits, one behind another). With seeds a short rest behind whole rounds of pieces is dealt out singly: 1 row of 248320
+// logits, 18944 of them such a rest, 12.4 us (as without VEC) against 16.5 with a second piece for some threads, 8 rows 20.6 against 24.6 (22.6 without VEC).
+// A rest of six logits a thread and more is as well off as pieces: 400000 logits 16.4 us both ways, 16 rows 51.5 singly, 43.1 as pieces.
 template <bool VEC>
 __global__ void __launch_bounds__(1024) sampling_argmax_kernel(const uzu_unified_sampling_args a, uint32_t row0, unsigned long long* ws,
                                                                unsigned int* tickets) {
@@ -117,11 +120,14 @@ __global__ void __launch_bounds__(1024) sampling_argmax_kernel(const uzu_unified
         best = k > best ? k : best;
     };
     if constexpr (VEC) {
-        for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) * 8u; i < V; i += gridDim.x * blockDim.x * 8u) {
+        const uint32_t threads = gridDim.x * blockDim.x, me = blockIdx.x * blockDim.x + threadIdx.x, rest = V % (threads * 8u);
+        const uint32_t whole = a.is_stochastic && V > rest && rest <= threads * 5u ? V - rest : V;
+        for (uint32_t i = me * 8u; i < whole; i += threads * 8u) {
             const uint4 x = masked_piece(reinterpret_cast<const uint16_t*>(logits), bitmask, i);
 #pragma unroll
             for (int j = 0; j < 8; ++j) offer(a.has_temperature ? bf16_bits_to_f32(piece_bits(x, j)) * recip_t : bf16_bits_to_f32(piece_bits(x, j)), i + j);
         }
+        for (uint32_t i = whole + me; i < V; i += threads) offer(filtered_logit(a, logits, bitmask, recip_t, i), i);
     } else {
         for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < V; i += gridDim.x * blockDim.x) offer(filtered_logit(a, logits, bitmask, recip_t, i), i);
     }
@@ -280,8 +286,9 @@ constexpr uint32_t SF_PIECES = 4;                    // 16-byte pieces of logits
 constexpr size_t SF_SMEM = SF_KEYS * sizeof(uint16_t);
 static_assert(SF_PER == 8, "a thread adds up eight neighbouring keys: one 16-byte read per CTA");
 
-// Bound: latency (a few cluster barriers, one pass over a 128 KB count table). VEC: rows of whole 16-byte pieces and at most 262144 logits stay in registers,
-// one read each; otherwise the logits are read twice, two bytes at a time. 8 rows, temperature, top-k 50, top-p 0.95: 34 us at 128256 logits (40 with the
+// Bound: latency (a few cluster barriers, one pass over a 128 KB count table). VEC: rows of whole 16-byte pieces, one for every thread and at most four (65536
+// to 262144 logits), stay in registers, one read each; otherwise the logits are read twice, two bytes at a time. Below that some threads would count eight
+// logits and others none: 1 row of 32768, top-k 50, 21.5 us without VEC and 22.9 with it, 8 rows of 8192 20.6 and 24.6, 1 row of 65536 26.7 and 25.0. 8 rows, temperature, top-k 50, top-p 0.95: 34 us at 128256 logits (40 with the
 // two-byte reads), 47 at 248320 (67); 16 rows of 128256 67 us (82).
 template <bool VEC>
 __global__ void __cluster_dims__(SF_CTAS, 1, 1) __launch_bounds__(SF_THREADS, 1) sampling_filtered_kernel(const uzu_unified_sampling_args a) {
@@ -573,7 +580,8 @@ void uzu_unified_sampling_encode(uzu_command_buffer* cmd, const uzu_unified_samp
             uzu::after_launch(cmd, "sampling_walk_kernel");
             return;
         }
-        const bool pieces = uzu::sampling_whole_pieces(*a) && a->vocab_size <= uzu::SF_CTAS * uzu::SF_THREADS * 8u * uzu::SF_PIECES;
+        constexpr uint32_t piece_each = uzu::SF_CTAS * uzu::SF_THREADS * 8u;
+        const bool pieces = uzu::sampling_whole_pieces(*a) && a->vocab_size >= piece_each && a->vocab_size <= piece_each * uzu::SF_PIECES;
         const auto kernel = pieces ? uzu::sampling_filtered_kernel<true> : uzu::sampling_filtered_kernel<false>;
         static std::atomic<uint64_t> smem_opt_in[2];
         uzu::opt_in_dynamic_smem(cmd, kernel, (int)uzu::SF_SMEM, smem_opt_in[pieces]);
