@@ -6,10 +6,10 @@
 // lane part p holds the key channels {4 (i L + p) .. + 3}, NV float4 in registers -- and a token costs two dot products, two shuffle
 // reductions over L lanes and no barrier at all. q and k rows are read from shared memory as float4 with the L parts side by side (128
 // contiguous bytes at L = 8: no bank conflict, the columns of a warp share the read).
-//   gated_delta_block_kernel the tokens of a pass four at a time, keys of 33..128 channels (column_block.cuh).
+//   gated_delta_block_kernel the tokens of a longer pass four at a time, keys of 33..128 channels (column_block.cuh). Sums in another order than token by
+//                            token: how a prompt is cut shows in an element's last bits.
 //   gated_delta_kernel       the tokens of a pass in order, 4 warps per CTA, grid (column blocks, heads). The prepared q / k / v / decay / beta
-//                            rows arrive by cp.async one batch ahead. An element's arithmetic does not depend on how a prompt is cut
-//                            (with blocks of four it does, within rounding).
+//                            rows arrive by cp.async one batch ahead. Passes that all go this way give the same bits however they are cut.
 //   delta_prepare_kernel     convolution, silu, unit vectors and gates of all tokens of a pass at once, a warp per (a few tokens, head).
 //   gated_delta_step_kernel  one token with everything between the projections in one launch: a cluster of CL CTAs per head, each CTA owning
 //                            vdim / CL columns; the state is requested before the previous kernel's results are waited for; the head's sum
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(128) delta_prepare_kernel(const uzu_delta_prep
     }
 }
 
-constexpr int GD_CB_WARPS = 4;
+constexpr int GD_WARPS = 4;
 
 template <int L, int NV>
 constexpr int gd_batch() { return L * NV * 4 <= 256 ? 16 : (L * NV * 4 <= 512 ? 8 : 4); }
@@ -218,8 +218,8 @@ __device__ __forceinline__ void gd_ring_store(const uzu_delta_prepare_args& a) {
 }
 
 template <int L, int NV>
-__global__ void __launch_bounds__(GD_CB_WARPS * 32) gated_delta_kernel(const uzu_gated_delta_args ga) {
-    constexpr int ROWF = L * NV * 4, BATCH = gd_batch<L, NV>(), CC = GD_CB_WARPS * (32 / L), U = BATCH < 8 ? BATCH : 8;
+__global__ void __launch_bounds__(GD_WARPS * 32) gated_delta_kernel(const uzu_gated_delta_args ga) {
+    constexpr int ROWF = L * NV * 4, BATCH = gd_batch<L, NV>(), CC = GD_WARPS * (32 / L), U = BATCH < 8 ? BATCH : 8;
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float gd_smem[];
@@ -243,12 +243,12 @@ __global__ void __launch_bounds__(GD_CB_WARPS * 32) gated_delta_kernel(const uzu
         const uint32_t nb = tb < a.rows ? min((uint32_t)BATCH, a.rows - tb) : 0u;
         float* q = qs + buf * BATCH * ROWF;
         float* k = ks + buf * BATCH * ROWF;
-        for (uint32_t i = tid; i < nb * pieces; i += GD_CB_WARPS * 32) {
+        for (uint32_t i = tid; i < nb * pieces; i += GD_WARPS * 32) {
             const uint32_t r = i / pieces, c = (i - r * pieces) * 4;
             gd_cp_async16(q + r * ROWF + c, pq + (size_t)(tb + r) * qk_stride + c);
             gd_cp_async16(k + r * ROWF + c, pk + (size_t)(tb + r) * qk_stride + c);
         }
-        for (uint32_t i = tid; i < nb * CC; i += GD_CB_WARPS * 32) {
+        for (uint32_t i = tid; i < nb * CC; i += GD_WARPS * 32) {
             const uint32_t r = i / CC, c = i % CC;
             if (col0 + c < a.vdim) gd_cp_async4(vs + (buf * BATCH + r) * CC + c, pv + (size_t)(tb + r) * v_stride + c);
         }
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(GD_CB_WARPS * 32) gated_delta_kernel(const uzu
     };
     if (dim4 < (uint32_t)ROWF) {                     // channels past the head stay zero in both buffers
         const uint32_t tail = ROWF - dim4;
-        for (uint32_t i = tid; i < 2 * BATCH * tail; i += GD_CB_WARPS * 32) {
+        for (uint32_t i = tid; i < 2 * BATCH * tail; i += GD_WARPS * 32) {
             const uint32_t r = i / tail, c = dim4 + i % tail;
             qs[r * ROWF + c] = 0.0f;
             ks[r * ROWF + c] = 0.0f;
@@ -677,9 +677,14 @@ static void by_key_size(uint32_t dim, F&& f) {
     else f(std::integral_constant<int, 32>{}, std::integral_constant<int, 8>{});
 }
 
+// Blocks of four tokens for keys of 33..128 channels from the pass length on at which they are no slower. One column per lane group while such CTAs have an SM
+// each (8 heads of 128 x 128, 1024 tokens: 105 us, 144 with two columns); more of them share an SM's issue slots and shared memory, and two columns per
+// lane group are faster in half the CTAs (16 heads 144 us, 158 with one). Token by token / blocks, us: one column, 8 heads of 128, 3 tokens 4.8 / 5.2, 12 tokens
+// 6.3 / 6.3, 24 tokens 8.4 / 7.3; two columns, 16 heads of 128, 2 tokens 4.2 / 6.3, 16 tokens 6.8 / 7.2, 36 tokens 11.3 / 10.4; 32 heads of 128, 9 tokens 6.4 / 8.3, 33 tokens
+// 12.5 / 13.4, 36 tokens 14.1 / 13.5.
 void launch_gated_delta_scan(uzu_command_buffer* cmd, const uzu_gated_delta_args& a) {
-    // Four tokens at a time where a key's channels fit the lanes. One column per lane group where two would leave SMs without a CTA.
-    if (a.prep.dim > 32 && a.prep.dim <= 128) {
+    const bool one_column = a.prep.heads * ((a.prep.vdim + 7) / 8) <= (uint32_t)cmd->ctx->sm_count;
+    if (a.prep.dim > 32 && a.prep.dim <= 128 && a.prep.rows >= (one_column ? 12u : 36u)) {
         auto blocks = [&](auto nv_c, auto q_c) {
             constexpr int L = 16, NV = decltype(nv_c)::value, Q = decltype(q_c)::value, GROUPS = CB_WARPS * (32 / L), CC = GROUPS * Q;
             constexpr size_t smem = ((size_t)2 * CB_BLOCKS * GdBlock<L * NV * 4>::floats(CC) + (size_t)4 * GROUPS * CB_TOKENS * Q) * sizeof(float);
@@ -689,17 +694,16 @@ void launch_gated_delta_scan(uzu_command_buffer* cmd, const uzu_gated_delta_args
         };
         auto one = std::integral_constant<int, 1>{};
         auto two = std::integral_constant<int, 2>{};
-        const bool narrow = a.prep.heads * ((a.prep.vdim + 7) / 8) <= 148;
-        if (a.prep.dim <= 64) narrow ? blocks(one, one) : blocks(one, two);
-        else narrow ? blocks(two, one) : blocks(two, two);
+        if (a.prep.dim <= 64) one_column ? blocks(one, one) : blocks(one, two);
+        else one_column ? blocks(two, one) : blocks(two, two);
         return;
     }
     by_key_size(a.prep.dim, [&](auto l_c, auto nv_c) {
-        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GD_CB_WARPS * (32 / L), BATCH = gd_batch<L, NV>();
+        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GD_WARPS * (32 / L), BATCH = gd_batch<L, NV>();
         constexpr size_t smem = ((size_t)4 * BATCH * L * NV * 4 + (size_t)2 * BATCH * CC + 4 * BATCH) * sizeof(float);
         static std::atomic<uint64_t> done{0};
         if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, gated_delta_kernel<L, NV>, (int)smem, done);
-        launch(cmd, "gated_delta_kernel", gated_delta_kernel<L, NV>, dim3((a.prep.vdim + CC - 1) / CC, a.prep.heads), dim3(GD_CB_WARPS * 32), smem, a);
+        launch(cmd, "gated_delta_kernel", gated_delta_kernel<L, NV>, dim3((a.prep.vdim + CC - 1) / CC, a.prep.heads), dim3(GD_WARPS * 32), smem, a);
     });
 }
 

@@ -6,7 +6,7 @@
 //                               parallel launch first (general_delta_prepare_kernel), then L lanes own a column and walk the tokens, two dot
 //                               products and an update each, no barrier between tokens; the five vectors of a token come from shared memory,
 //                               a batch of tokens ahead by cp.async. Bound: latency that nothing covers (one warp per scheduler).
-//   general_delta_block_kernel  the same with four tokens per step, heads of 33..128 channels (column_block.cuh).
+//   general_delta_block_kernel  the same for passes of ten and more tokens, four per step, heads of 33..128 channels (column_block.cuh).
 //   general_delta_kernel        the decode step and short passes: a CTA keeps a dim x 32 slice of the state in registers -- warp p owns PART
 //                               key channels, lane c owns column c; partial sums meet in shared memory in warp order (a fixed order: one
 //                               token at a time or several in one launch give the same bits).
@@ -152,13 +152,13 @@ __global__ void __launch_bounds__(128) general_delta_prepare_kernel(const uzu_ge
 // 32 / L columns per warp, grid (column blocks, heads). Bound: latency. 16 heads of 128 are 512 warps on 592 schedulers, and a warp's 20 shared 16-byte
 // reads and its arithmetic of a token take 375 ns with nothing beside them; the dependent part (dot product over the lane's channels, log2 L shuffles, the
 // update) is about a fifth of that. 1024 tokens, 16 heads of 128: 0.37 ms against 1.70 ms as a CTA per 32 columns with three barriers a token.
-constexpr int GS_CB_WARPS = 4;
+constexpr int GS_WARPS = 4;
 template <int L, int NV>
 constexpr int gs_batch() { return L * NV * 4 <= 128 ? 8 : (L * NV * 4 <= 256 ? 4 : 2); }
 
 template <int L, int NV>
-__global__ void __launch_bounds__(GS_CB_WARPS * 32) general_delta_scan_kernel(const uzu_general_delta_args a, uint32_t vec) {
-    constexpr int ROWF = L * NV * 4, BATCH = gs_batch<L, NV>(), CC = GS_CB_WARPS * (32 / L);
+__global__ void __launch_bounds__(GS_WARPS * 32) general_delta_scan_kernel(const uzu_general_delta_args a, uint32_t vec) {
+    constexpr int ROWF = L * NV * 4, BATCH = gs_batch<L, NV>(), CC = GS_WARPS * (32 / L);
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) float gs_smem[];
@@ -179,19 +179,19 @@ __global__ void __launch_bounds__(GS_CB_WARPS * 32) general_delta_scan_kernel(co
             const uint32_t pieces = dim / 4;
 #pragma unroll
             for (int w = 0; w < 5; ++w)
-                for (uint32_t i = tid; i < nb * pieces; i += GS_CB_WARPS * 32) {
+                for (uint32_t i = tid; i < nb * pieces; i += GS_WARPS * 32) {
                     const uint32_t r = i / pieces, c = (i - r * pieces) * 4;
                     gd_cp_async16(dst + (r * 5 + w) * ROWF + c, src[w] + (size_t)(tb + r) * stride[w] + c);
                 }
         } else {
 #pragma unroll
             for (int w = 0; w < 5; ++w)
-                for (uint32_t i = tid; i < nb * dim; i += GS_CB_WARPS * 32) {
+                for (uint32_t i = tid; i < nb * dim; i += GS_WARPS * 32) {
                     const uint32_t r = i / dim, c = i - r * dim;
                     gd_cp_async4(dst + (r * 5 + w) * ROWF + c, src[w] + (size_t)(tb + r) * stride[w] + c);
                 }
         }
-        for (uint32_t i = tid; i < nb * CC; i += GS_CB_WARPS * 32) {
+        for (uint32_t i = tid; i < nb * CC; i += GS_WARPS * 32) {
             const uint32_t r = i / CC, c = i % CC;
             if (col0 + c < dim) gd_cp_async4(vs + (buf * BATCH + r) * CC + c, pv + (size_t)(tb + r) * a.v_stride + c);
         }
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(GS_CB_WARPS * 32) general_delta_scan_kernel(co
     };
     if (dim < (uint32_t)ROWF) {                      // channels past the head stay zero in both buffers
         const uint32_t tail = ROWF - dim;
-        for (uint32_t i = tid; i < 2 * BATCH * 5 * tail; i += GS_CB_WARPS * 32) vecs[i / tail * ROWF + dim + i % tail] = 0.0f;
+        for (uint32_t i = tid; i < 2 * BATCH * 5 * tail; i += GS_WARPS * 32) vecs[i / tail * ROWF + dim + i % tail] = 0.0f;
     }
     stage(0, 0);
     float4 S[NV];
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(GS_CB_WARPS * 32) general_delta_scan_kernel(co
 // Bound: the shared-memory reads of a block (34 16-byte vector reads of each of four warps, in bursts) and the chain dot products -> lane sums -> exchange ->
 // update: 1200 cycles a block of which 490 issue. More warps with fewer columns each read more and were slower (291 us), one reduction for both kinds of
 // dot products instead of two was too (235 us). 1024 tokens with their preparation and copies: 16 heads of 128 206 us (386 token by token), 8 heads 0.20 ms
-// (0.39), 32 heads 0.35 ms (0.57), 16 heads of 64 0.15 ms (0.24); 40 tokens 44 us (51), 4 tokens 38 us (38).
+// (0.39), 32 heads 0.35 ms (0.57), 16 heads of 64 0.15 ms (0.24); 40 tokens 44 us (51).
 template <int ROWF>
 struct GbBlock {
     static constexpr int U = 0, A = 4 * ROWF, K = 8 * ROWF, R = 12 * ROWF, P = 16 * ROWF, T = 17 * ROWF, ZK = T + 12, OK = ZK + 16, OA = OK + 16, V = OA + 16;
@@ -482,15 +482,17 @@ static void launch_general_delta_scan(uzu_command_buffer* cmd, const uzu_general
     const uint32_t vec = !((a.decay_logit | a.rate_logit | a.unit | a.k | a.r) & 15u) &&
                          !((a.decay_stride | a.rate_stride | a.k_stride | a.r_stride | a.dim) & 3u);
     auto go = [&](auto l_c, auto nv_c) {
-        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GS_CB_WARPS * (32 / L), BATCH = gs_batch<L, NV>();
+        constexpr int L = decltype(l_c)::value, NV = decltype(nv_c)::value, CC = GS_WARPS * (32 / L), BATCH = gs_batch<L, NV>();
         constexpr size_t smem = ((size_t)2 * BATCH * 5 * L * NV * 4 + (size_t)2 * BATCH * CC) * sizeof(float);
         static std::atomic<uint64_t> done{0};
         if (smem > 48 * 1024) opt_in_dynamic_smem(cmd, general_delta_scan_kernel<L, NV>, (int)smem, done);
-        launch(cmd, "general_delta_scan_kernel", general_delta_scan_kernel<L, NV>, dim3((a.dim + CC - 1) / CC, a.heads), dim3(GS_CB_WARPS * 32), smem, a, vec);
+        launch(cmd, "general_delta_scan_kernel", general_delta_scan_kernel<L, NV>, dim3((a.dim + CC - 1) / CC, a.heads), dim3(GS_WARPS * 32), smem, a, vec);
     };
-    // Four tokens at a time wherever a row's channels fit the lanes as float4: faster from 4 tokens on (figures above the kernel). One column per lane group
-    // where two would leave SMs without a CTA.
-    if (vec && a.dim > 32 && a.dim <= 128) {
+    // Four tokens at a time wherever a row's channels fit the lanes as float4, from ten tokens on. With the preparation, token by token / blocks, us: 16 heads of
+    // 128, 5 tokens 10.4 / 11.5, 10 tokens 12.5 / 12.5, 16 tokens 15.0 / 12.8; 64 heads of 64, 9 tokens 11.6 / 12.5, 10 tokens 12.5 / 12.5, 64 tokens 27.8 / 23.7.
+    // One column per lane group while such CTAs have an SM each (8 heads of 128, 1024 tokens: 166 us, 178 with two columns); more of them share an SM's issue
+    // slots and shared memory, and two columns per lane group are faster in half the CTAs (10 heads 179 us, 272 with one; 16 heads 183, 273).
+    if (vec && a.dim > 32 && a.dim <= 128 && a.rows >= 10) {
         auto blocks = [&](auto nv_c, auto q_c) {
             constexpr int L = 16, NV = decltype(nv_c)::value, Q = decltype(q_c)::value, GROUPS = CB_WARPS * (32 / L), CC = GROUPS * Q;
             constexpr size_t smem = ((size_t)2 * CB_BLOCKS * GbBlock<L * NV * 4>::floats(CC) + (size_t)4 * GROUPS * CB_TOKENS * Q) * sizeof(float);
@@ -500,9 +502,9 @@ static void launch_general_delta_scan(uzu_command_buffer* cmd, const uzu_general
         };
         auto one = std::integral_constant<int, 1>{};
         auto two = std::integral_constant<int, 2>{};
-        const bool narrow = a.heads * ((a.dim + 7) / 8) <= 148;
-        if (a.dim <= 64) narrow ? blocks(one, one) : blocks(one, two);
-        else narrow ? blocks(two, one) : blocks(two, two);
+        const bool one_column = a.heads * ((a.dim + 7) / 8) <= (uint32_t)cmd->ctx->sm_count;
+        if (a.dim <= 64) one_column ? blocks(one, one) : blocks(one, two);
+        else one_column ? blocks(two, one) : blocks(two, two);
         return;
     }
     auto l8 = std::integral_constant<int, 8>{};
