@@ -174,19 +174,22 @@ __device__ __forceinline__ void qs_dequant8(uint32_t q, uint32_t zh2, uint32_t z
     hi[0] = __byte_perm(h[0], h[1], 0x5410); hi[1] = __byte_perm(h[0], h[1], 0x7632);
     lo[0] = __byte_perm(l[0], l[1], 0x5410); lo[1] = __byte_perm(l[0], l[1], 0x7632);
 }
-// the same codes as integers code - zp, exact in bf16
+// The same codes as integers code - zp, exact in bf16, times 2^-11 (bytes: 2^-15): a chain of 128 of them then adds up to no more than the largest
+// activation, so an unscaled sum is never out of range where the product is in range. The nibble lies behind the bits of 2^-4 (2^-8) instead of 128.0.
+template <int BITS> constexpr uint32_t qs_base = BITS == 4 ? 0x3D80u : 0x3B80u;
+template <int BITS> constexpr float qs_unit = BITS == 4 ? 2048.0f : 32768.0f;      // 1 / the integers' factor
 __device__ __forceinline__ void qs_integers4(uint32_t q, uint32_t z2, uint32_t* v) {
     uint32_t d[4];
 #pragma unroll
-    for (int p = 0; p < 4; ++p) d[p] = qs_u(__hsub2(qs_b2(((q >> (4 * p)) & 0x000F000Fu) | 0x43004300u), qs_b2(z2)));
+    for (int p = 0; p < 4; ++p) d[p] = qs_u(__hsub2(qs_b2(((q >> (4 * p)) & 0x000F000Fu) | qs_base<4> * 0x00010001u), qs_b2(z2)));
     v[0] = __byte_perm(d[0], d[1], 0x5410); v[1] = __byte_perm(d[2], d[3], 0x5410); v[2] = __byte_perm(d[0], d[1], 0x7632); v[3] = __byte_perm(d[2], d[3], 0x7632);
 }
 __device__ __forceinline__ void qs_integers8(uint32_t q, uint32_t zh2, uint32_t zl2, uint32_t* v) {
     uint32_t d[2];
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
-        const __nv_bfloat162 dl = __hsub2(qs_b2(((q >> (8 * p)) & 0x000F000Fu) | 0x43004300u), qs_b2(zl2));
-        const __nv_bfloat162 dh = __hsub2(qs_b2(((q >> (8 * p + 4)) & 0x000F000Fu) | 0x43004300u), qs_b2(zh2));
+        const __nv_bfloat162 dl = __hsub2(qs_b2(((q >> (8 * p)) & 0x000F000Fu) | qs_base<8> * 0x00010001u), qs_b2(zl2));
+        const __nv_bfloat162 dh = __hsub2(qs_b2(((q >> (8 * p + 4)) & 0x000F000Fu) | qs_base<8> * 0x00010001u), qs_b2(zh2));
         d[p] = qs_u(__hfma2(qs_b2(0x41804180u), dh, dl));
     }
     v[0] = __byte_perm(d[0], d[1], 0x5410); v[1] = __byte_perm(d[0], d[1], 0x7632);
@@ -310,6 +313,8 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                         if (ok) next();
                     }
                 }
+#pragma unroll
+                for (int c = 0; c < EC; ++c) acc[c] *= qs_unit<BITS>;
             } else
             for (uint32_t i = 0; i < (S::CHAIN ? nk : 1u) && ok; i += S::CHAIN ? S::CHAIN : 1) {
                 ok = qs_wait(d_full(buf), ph, &gave_up, p.error, 0x101u);
@@ -434,7 +439,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                         if constexpr (BITS == 4) {
                             uint32_t q[4];
                             asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(line + (((j * 2 + h) ^ (r & 7u)) << 4)));
-                            const uint32_t z2 = (0x4300u | z) * 0x00010001u;      // bf16 128 + zp
+                            const uint32_t z2 = ((PL == 1 ? qs_base<4> : 0x4300u) | z) * 0x00010001u;      // bf16 128 + zp
                             if constexpr (PL == 1) {
 #pragma unroll
                                 for (int i = 0; i < 4; ++i) qs_integers4(q[i] ^ p.xor_mask, z2, hi + 4 * i);
@@ -454,7 +459,8 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                             for (uint32_t i2 = 0; i2 < 2; ++i2) {
                                 uint32_t q[4];
                                 asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]) : "r"(line + (((j * 4 + h * 2 + i2) ^ (r & 7u)) << 4)));
-                                const uint32_t zh2 = (0x4300u | (z >> 4)) * 0x00010001u, zl2 = (0x4300u | (z & 15u)) * 0x00010001u;
+                                constexpr uint32_t base = PL == 1 ? qs_base<8> : 0x4300u;
+                                const uint32_t zh2 = (base | (z >> 4)) * 0x00010001u, zl2 = (base | (z & 15u)) * 0x00010001u;
                                 if constexpr (PL == 1) {
 #pragma unroll
                                     for (int i = 0; i < 4; ++i) qs_integers8(q[i] ^ p.xor_mask, zh2, zl2, hi + 8 * i2 + 2 * i);
