@@ -3,7 +3,8 @@
 //
 // mma.sync.m16n8k16 with 16 output features as M and 8 activation rows as N: here it is the better pipe than tcgen05, whose products cost the same for
 // 8 rows as for 64. Codes become bf16 INTEGERS code - zp in registers (exact: nibbles behind the bits of 128.0, one subtraction; bytes as two nibbles
-// and one fma), sums of a group are f32, and a group's scale is one f32 fma per sum. Nothing of a weight is rounded.
+// and one fma), sums of a group are f32, and a group's scale is one f32 fma per sum. Nothing of a weight is rounded. The integers enter times 2^-11 (bytes
+// 2^-15) and a finished sum is brought back: a group's sum is no larger than the largest activation, so it is in range where the product is.
 //   CTA     12 warps, one CTA per SM, pinned to a slice of k whose activations it keeps in shared memory in fragment order; slices of a tile meet in
 //           the split-k workspace, added in slice order by whoever comes last (the same bits every time).
 //   warp    an equal run of the CTA's (16 features, step of k) pairs; a tile that several warps share meets in shared memory, in order. Steps are
@@ -45,6 +46,8 @@ constexpr int QR_WARPS = 12, QR_STAGES = 2;
 template <int BITS>
 struct QrShape {
     static constexpr uint32_t CODES = BITS == 4 ? 512 : 256, PITCH = BITS == 4 ? 288 : 320, STAGE = 16 * PITCH + 512;
+    static constexpr float DOWN = BITS == 4 ? 1.0f / 2048.0f : 1.0f / 32768.0f, UP = 1.0f / DOWN;            // the integers' factor
+    static constexpr uint32_t MAGIC = BITS == 4 ? 0x3D803D80u : 0x3B803B80u;                                 // bf16 128 DOWN, twice
 };
 
 template <int BYTES>
@@ -57,7 +60,7 @@ __device__ __forceinline__ void qr_mma(float (&d)[4], uint32_t a0, uint32_t a1, 
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// nibbles 0 and 4 of w as bf16 128 + nibble
+// nibbles 0 and 4 of w as bf16 128 + nibble, times the integers' factor
 __device__ __forceinline__ uint32_t qr_nibbles(uint32_t w, uint32_t magic) {
     uint32_t r;
     asm("lop3.b32 %0, %1, 0x000f000f, %2, 0xEA;" : "=r"(r) : "r"(w), "r"(magic));
@@ -72,7 +75,7 @@ __device__ __forceinline__ uint32_t qr_mad16(uint32_t a, uint32_t b) {          
     const __nv_bfloat162 r = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&a), *reinterpret_cast<const __nv_bfloat162*>(&sixteen), *reinterpret_cast<const __nv_bfloat162*>(&b));
     return *reinterpret_cast<const uint32_t*>(&r);
 }
-// Four codes of a byte word less the zero point: (0, 2) and (1, 3). lo, hi: 128 + the zero point's nibbles
+// Four codes of a byte word less the zero point: (0, 2) and (1, 3). lo, hi: 128 + the zero point's nibbles, times the factor
 __device__ __forceinline__ void qr_bytes(uint32_t w, uint32_t lo, uint32_t hi, uint32_t magic, uint32_t& p02, uint32_t& p13) {
     p02 = qr_mad16(qr_sub(qr_nibbles(w >> 4, magic), hi), qr_sub(qr_nibbles(w, magic), lo));
     p13 = qr_mad16(qr_sub(qr_nibbles(w >> 12, magic), hi), qr_sub(qr_nibbles(w >> 8, magic), lo));
@@ -90,13 +93,13 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
     const uint32_t tile_begin = (uint32_t)((uint64_t)column * p.tiles / columns), tile_end = (uint32_t)((uint64_t)(column + 1) * p.tiles / columns);
     const uint32_t xstride = p.slice_steps * ITEMS + 1;                       // odd: the rows of a fragment read fall on all banks
     uint4* xs = reinterpret_cast<uint4*>(qr_smem);                            // [MROWS][xstride]
-    float* sx = reinterpret_cast<float*>(xs + (size_t)MROWS * xstride);       // [slice_steps * NG][MROWS]: sums of the groups' activations (ScaleBias)
+    float* sx = reinterpret_cast<float*>(xs + (size_t)MROWS * xstride);       // [slice_steps * NG][MROWS]: sums of the groups' activations, times the factor (ScaleBias)
     float* turns = sx + (kBias ? (size_t)p.slice_steps * NG * MROWS : 0), *turn = turns + warp * 128;      // [8][16] of each warp
     float4* heads = reinterpret_cast<float4*>(turns + QR_WARPS * 128);        // [warps][MB][32]: what a warp adds to a tile that another one began
     uint8_t* ring = reinterpret_cast<uint8_t*>(heads + (p.whole ? 0 : QR_WARPS * MB * 32)) + (size_t)warp * QR_STAGES * S::STAGE;
     const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
     uint32_t magic;
-    asm volatile("mov.b32 %0, 0x43004300;" : "=r"(magic));
+    asm volatile("mov.b32 %0, %1;" : "=r"(magic) : "n"(S::MAGIC));
 
     auto zero_fetch = [&](uint32_t row, uint32_t step) { return qr_zero_fetch(row, step, p.n, p.zp_stride, BITS == 4 ? NG / 2 : NG); };
     auto issue_stage = [&](uint32_t tile, uint32_t step, uint32_t slot) {
@@ -159,7 +162,7 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
                     const uint32_t e[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
                     float sum = 0.0f;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) sum += __uint_as_float(e[i] << 16) + __uint_as_float(e[i] & 0xffff0000u);
+                    for (int i = 0; i < 4; ++i) sum += fmaf(S::DOWN, __uint_as_float(e[i] << 16), S::DOWN * __uint_as_float(e[i] & 0xffff0000u));
 #pragma unroll
                     for (uint32_t o_ = 1; o_ < GS / 8; o_ <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o_);
                     if (li % (GS / 8) == 0) sx[(size_t)(li / (GS / 8)) * MROWS + r] = sum;
@@ -206,7 +209,7 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
                 const uint32_t o = lane + 32u * i, row = (uint32_t)c * 8u + o / 16u, feature = tile * 16u + o % 16u;
                 if (row >= p.m || feature >= p.n) continue;
                 const size_t idx = (size_t)row * p.n + feature;
-                float v = p.ab_scale * turn[o];
+                float v = p.ab_scale * (S::UP * turn[o]);
                 if (p.accumulate) v += p.d_is_f32 ? reinterpret_cast<const float*>(p.d)[idx] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.d)[idx]);
                 if (p.bias) v += __bfloat162float(p.bias[feature]);
                 if (p.has_soft_cap) v = p.soft_cap * tanhf(v / p.soft_cap);
@@ -252,7 +255,7 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
                 float d[MB][4];
 #pragma unroll
                 for (int c = 0; c < MB; ++c) d[c][0] = d[c][1] = d[c][2] = d[c][3] = 0.0f;
-                uint32_t lo_a, lo_b, hi_a = magic, hi_b = magic;              // 128 + the zero point (its nibbles)
+                uint32_t lo_a, lo_b, hi_a = magic, hi_b = magic;              // 128 + the zero point (its nibbles), times the factor
                 if (kZero) {
                     const uint32_t z1 = za[0] >> (gq * BITS), z2 = zb[0] >> (gq * BITS);
                     lo_a = magic + (z1 & 15u) * 0x00010001u;
@@ -261,8 +264,8 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
                 } else if (kBias) {
                     lo_a = lo_b = magic;
                 } else {
-                    lo_a = lo_b = BITS == 4 ? 0x43084308u : magic;
-                    hi_a = hi_b = 0x43084308u;
+                    lo_a = lo_b = BITS == 4 ? S::MAGIC + 0x00080008u : magic;
+                    hi_a = hi_b = S::MAGIC + 0x00080008u;
                 }
 #pragma unroll
                 for (int part = 0; part < GS / 64; ++part) {
