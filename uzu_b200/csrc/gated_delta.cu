@@ -351,7 +351,7 @@ constexpr int GS_THREADS = 256;
 //     o_j = p_{j+1} (q_j . S) + sum_{i<=j} (g_{i+1} .. g_j) (q_j . k_i) w_i,      S' = p_4 S + sum_i (g_{i+1} .. g_3) k_i w_i^T
 // Producer warps (one per block) pass the q and k rows on, form the products k_j . k_i and q_j . k_i and invert the w_i system; consumer warps take the
 // dot products with S, L lanes of four channels per group of Q columns. A decay is at most 1, so no product of them can grow.
-// Bound: the chain dot products -> lane sums -> exchange -> update, about 1150 cycles a block with one consumer warp per scheduler. 509 tokens, 16 heads of
+// Bound: the chain dot products -> lane sums -> exchange -> update, 1200 cycles a block with one consumer warp per scheduler, which issues 420. 509 tokens, 16 heads of
 // 128 x 128: 78 us against 96 us token by token.
 template <int ROWF>
 struct GdBlock {

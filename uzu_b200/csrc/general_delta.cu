@@ -284,7 +284,7 @@ __global__ void __launch_bounds__(GS_WARPS * 32) general_delta_scan_kernel(const
 // Producer warps (one per block) form the 17 vectors and the sums over channels, and invert the z_i system; decays are <= 1, so no product of them can
 // grow. Consumer warps: see column_block.cuh; L lanes of four channels per group of Q columns.
 // Bound: the shared-memory reads of a block (34 16-byte vector reads of each of four warps, in bursts) and the chain dot products -> lane sums -> exchange ->
-// update: 1200 cycles a block of which 490 issue. More warps with fewer columns each read more and were slower (291 us), one reduction for both kinds of
+// update: 1350 cycles a block, of which a scheduler issues 510 (16 heads of 128). More warps with fewer columns each read more and were slower (291 us), one reduction for both kinds of
 // dot products instead of two was too (235 us). 1024 tokens with their preparation and copies: 16 heads of 128 206 us (386 token by token), 8 heads 0.20 ms
 // (0.39), 32 heads 0.35 ms (0.57), 16 heads of 64 0.15 ms (0.24); 40 tokens 44 us (51).
 template <int ROWF>

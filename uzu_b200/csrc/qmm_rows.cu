@@ -12,11 +12,13 @@
 //   lane    16 consecutive k of a group of 64 for two rows (g, g + 8 of the tile): 8 or 16 bytes of shared memory each, at pitches that spread a
 //           quarter warp over all banks. The products' k order is the lanes' order, the same for both operands.
 // Bound: the codes' way from HBM, then issue slots: a step of 16 features x 64 k is about 70 instructions, 130 for 8-bit codes.
-// The linears of a layer of an 8B model (115 MB of 4-bit codes, groups of 64), us, with the kernels before it (9 rows and more: qmm_scaled.cu):
-//   rows      2        8        16        24         32
-//   4 bit  60 (84)  61 (85)  77 (122)  105 (126)  122 (126)      at 40 rows 135 (131): the line is at 32
-//   8 bit  85 (124) 87 (128) 102 (162) 119 (164)  139 (167)
-//   MLX    62 (82)  62 (144) 79 (147)  107 (148)  128 (151)
+// The linears of a layer of an 8B model (115 MB of 4-bit codes, groups of 64), us, with the kernels that took these rows before it (2 and 8 rows) or would take
+// them without it (qmm_scaled.cu):
+//   rows            2        8        16         24         32
+//   4 bit        60 (84)  61 (85)  76 (118)   102 (129)  123 (131)      at 40 rows 135 (135): the line is at 32
+//     groups 128          59 (112) 75 (114)   99 (116)   119 (118)
+//   8 bit        85 (124) 88 (128) 105 (142)  121 (151)  146 (152)
+//   MLX          62 (82)  65 (144) 81 (173)   108 (176)  130 (177)
 #include <cstdlib>
 
 #include "common.cuh"

@@ -26,9 +26,9 @@
 // 160 / 131, 8-bit 201 / 176; 60 rows 170 / 155; groups of 32 187 / 225, so they keep the planes.
 //
 // Bounds, per block and CTA: the tensor pipe 4 NT cycles; the dequant warps about 230 instructions each, four warps a block. Prompts are bound by the
-// tensor pipe (half of its rate is the most two planes can give), few rows by the product
-// warp's way from one block to the next (about 740 cycles, 490 of them outside its waits) and, with one plane, the epilogue's per chain (650); more dequant
-// groups and a product role of one lane changed nothing.
+// tensor pipe (half of its rate is the most two planes can give), few rows by the way of a
+// block through its roles (28672 x 4096 at 40 rows: 1000 cycles per 64 k with fill and drain, issue slots 56 % used, tensor pipe 10 %); more dequant groups
+// and a product role of one lane changed nothing.
 // Every barrier wait is bounded (about a second): a wait that runs out is reported (wait_errors.h: the call then fails on the host) and the CTA ends its work.
 #include <cuda.h>
 
