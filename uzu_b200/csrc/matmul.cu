@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(QS_WARPS * 32) qmv_stream_kernel(const QmvPara
 // -------------------------------------------------------------------------------------------------
 // cp.async variant of the decode kernel: the same arithmetic, but the weight stream lands in a per-warp
 // shared-memory ring (QA_STAGES super-chunks deep) instead of registers. Measured on B200: with the
-// GEMV access pattern the HBM pipe needs >100 KB in flight per SM to reach ~6 TB/s (tools/bw_probe.cu);
+// GEMV access pattern the HBM pipe needs >100 KB in flight per SM to reach ~6 TB/s;
 // registers can hold ~8 KB per warp, the ring holds QA_STAGES-1 x 4.5 KB per warp with no register cost,
 // each lane consuming exactly the bytes it copied (no cross-thread synchronisation on the ring).
 // -------------------------------------------------------------------------------------------------
