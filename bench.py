@@ -1,11 +1,11 @@
 #!/usr/bin/env python
-"""bench.py -- decode tokens/s of the uzu transformer decode hot path on B200 (BASELINE.json metric).
+"""bench.py -- decode tokens/s of the uzu transformer decode hot path on B200 (the reference's headline metric).
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--workload NAME] [--impl ours|reference] [--tp P]
 
 A "step" is one decoded token: one full forward pass (all layers + readout + sampling) at batch 1 over the synthetic uzu-format
 checkpoint of the workload, starting right after a `prefill`-token prompt. Default workload = the configuration the "at 1/2/4/8 B200"
-metric is quoted on: BASELINE.json configs[2], Llama-3-8B int4, prefill 2048, decode 256. The N = 1 run adds configs[1]
+metric is quoted on: Llama-3-8B int4, prefill 2048, decode 256. The N = 1 run adds the smaller model's line
 (Qwen3.5-0.8B int4, prefill 512, decode 128) as `config.secondary` with its own value / e2e / roofline / parity.
 
   value      decode tokens/s with everything resident in HBM: K device-chained steps (the sampled token is fed back on the device)
@@ -23,7 +23,7 @@ metric is quoted on: BASELINE.json configs[2], Llama-3-8B int4, prefill 2048, de
              host cores, single worker thread like the reference (rank 0, N = 1 only).
   --impl reference   times the same CPU restatement on the host threads the cgroup really grants (the reference itself is Rust and
              cannot be built here: no rustc/cargo in the image).
-Multi-GPU: the BASELINE models that fit one GPU run as independent replicas (weak scaling, no collective on the path). At N >= 2 the
+Multi-GPU: the models that fit one GPU run as independent replicas (weak scaling, no collective on the path). At N >= 2 the
 run also shards ONE copy of the model over the N ranks (uzu_b200/tp.py: attention head / FFN column / vocabulary row; two all-reduces
 per layer + one all-gather of the logits) and reports it under `config.tp` for both exchanges (NCCL, one-kernel peer memory).
 `--tp P` (with --gpus P) makes that sharded model the headline instead: value = tokens/s of the single replica, "strong".
@@ -447,7 +447,7 @@ def roofline_of(eng, workload: str, prefill: int, K: int, seconds: float):
 
 def speculation_of(eng, step_ms: float, nodes: int = 16, passes: int = 6):
     """Cost of one speculation pass (uzu_engine_trie_pass over a linearized trie of `nodes` nodes: one sweep over the weights, logits + a
-    sampled token for every node; SURVEY 8f-4) next to the plain decode step of the timed run. Wall clock around the synchronous call,
+    sampled token for every node) next to the plain decode step of the timed run. Wall clock around the synchronous call,
     which ends with the D2H read of the sampled ids like the stream's speculation loop. `break_even_tokens_per_pass` = pass / step: a
     proposer has to get more than that many tokens accepted per pass for speculation to pay on this GPU."""
     if not eng.speculation_supported:
@@ -569,13 +569,13 @@ def run_ours(args, rank: int, world: int, local_rank: int):
         except Exception as ex:  # the baseline must not take the measurement down
             line["cpu_baseline"] = {"value": None, "unit": "tokens/s", "cores": threads, "kind": "port", "sample": f"failed: {ex}"}
     eng.close()
-    # ---- secondary line (N = 1): BASELINE.json configs[1], Qwen3.5-0.8B int4 prefill 512 / decode 128 ----
+    # ---- secondary line (N = 1): Qwen3.5-0.8B int4 prefill 512 / decode 128 ----
     if world == 1 and tp == 1 and not args.no_secondary and workload != SECONDARY:
         try:
             line["config"]["secondary"] = secondary_line(B, ctx, args, local_rank)
         except Exception as ex:
             line["config"]["secondary"] = {"error": str(ex)[:300]}
-    # ---- tensor-parallel sub-measurement (N >= 2): the same model sharded over the N ranks (SURVEY 8e) ----
+    # ---- tensor-parallel sub-measurement (N >= 2): the same model sharded over the N ranks ----
     if world > 1 and tp == 1 and not args.no_tp_sub:
         sub = {}
         # the one-kernel peer-memory exchange has run on hardware at 2 ranks only: larger groups need UZU_BENCH_TP_P2P=1
@@ -837,7 +837,7 @@ def main():
     ap.add_argument("--warmup", type=int, default=8)
     ap.add_argument("--impl", choices=["ours", "reference"], default="ours")
     ap.add_argument("--workload", default="llama3-8b-int4", choices=sorted(WORKLOADS))
-    ap.add_argument("--no-secondary", action="store_true", help="skip the Qwen3.5-0.8B int4 line (BASELINE configs[1]) that the default N = 1 run adds under config.secondary")
+    ap.add_argument("--no-secondary", action="store_true", help="skip the Qwen3.5-0.8B int4 line that the default N = 1 run adds under config.secondary")
     ap.add_argument("--no-tp-sub", action="store_true", help="N >= 2: skip the tensor-parallel sub-measurement reported under config.tp")
     ap.add_argument("--no-persistent", action="store_true", help="use the per-kernel decode path instead of the persistent whole-token kernel (A/B)")
     ap.add_argument("--prefill", type=int, default=0)

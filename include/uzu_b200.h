@@ -2,12 +2,12 @@
  * uzu_b200.h -- C ABI of libuzu_b200.so: a B200 (sm_100a) CUDA backend for uzu's transformer
  * decode hot path.
  *
- * This is the drop-in boundary (SURVEY.md section 8b). The reference has no FFI: its backends are
+ * This is the drop-in boundary. The reference has no FFI: its backends are
  * Rust types implementing the `Backend` / `Context` / `CommandBuffer*` / `DenseBuffer` /
  * `SparseBuffer` / `Kernels` / `<Name>Kernel` traits of crates/backend-uzu. A `backends/cuda`
- * Rust module implements those traits by calling the entry points below one-to-one
- * (INTEGRATION.md shows the binding); each declaration cites the trait item it replaces.
- * Paths are relative to /root/reference/crates/backend-uzu/src/.
+ * Rust module implements those traits by calling the entry points below one-to-one;
+ * each declaration cites the trait item it replaces.
+ * Paths are relative to crates/backend-uzu/src/ of the reference.
  *
  * Conventions
  *   - plain C: opaque handles, raw device pointers (Buffer::gpu_ptr() + byte offset) and sizes;
@@ -215,7 +215,7 @@ UZU_API void uzu_debug_set_umma(int layout, uint32_t desc_hi, uint32_t desc_lbo,
 UZU_API int uzu_fused_linear_supported(uzu_context* ctx, const uzu_fused_linear_args* args);
 UZU_API void uzu_fused_linear_encode(uzu_command_buffer* cmd, const uzu_fused_linear_args* args);
 
-/* ---- Tensor parallelism (extension; the reference is single-device, SURVEY.md 8e) -------------------------------------------
+/* ---- Tensor parallelism (extension; the reference is single-device) -------------------------------------------
  * One process per GPU. Rank 0 creates a 128-byte NCCL unique id, the host program distributes it (bench.py: torch.distributed
  * broadcast), every rank calls uzu_context_tp_init on its context. The engine then loads the checkpoint shard written by
  * uzu_b200/tp.py (config.json "tensor_parallel" block) and inserts the two exchange steps below. NCCL is dlopen'ed at first use
@@ -339,7 +339,7 @@ typedef struct uzu_kv_cache_update_args {
 } uzu_kv_cache_update_args;
 UZU_API void uzu_kv_cache_update_encode(uzu_command_buffer* cmd, const uzu_kv_cache_update_args* args);
 
-/* ActivationTransformKernel (Mirai RHT, SURVEY 8f-3): backends/cpu/kernel/activation_transform/activation_transform.rs:44-63 (declaration
+/* ActivationTransformKernel (Mirai RHT): backends/cpu/kernel/activation_transform/activation_transform.rs:44-63 (declaration
  * order), semantics :64-136 and mod.rs:9-44; ops = gpu_types ActivationTransformOp. InputRht: out = H32 (s o x) per 32-wide stripe,
  * OutputRht: out = s o (H32 x), H32 = Sylvester Walsh-Hadamard / sqrt(32), s = rht_factors (i32 +-1, [element_count]). Quantize ops run
  * the InputRht transform and emit symmetric int8 codes per activation group (divisor = max|t| / 127), the f32 divisors and -- with
@@ -375,7 +375,7 @@ typedef struct uzu_gated_act_mul_args {
     uint64_t fp_out;
     uint32_t gated_dim, batch_dim, value_offset, value_row_stride;
     uint32_t act_type;             /* uzu_activation_type */
-    uint32_t interleaved;          /* Quantize ops / Hadamard: unsupported (SURVEY 8f-3) */
+    uint32_t interleaved;          /* Quantize ops / Hadamard: unsupported */
 } uzu_gated_act_mul_args;
 UZU_API void uzu_gated_act_mul_encode(uzu_command_buffer* cmd, const uzu_gated_act_mul_args* args);
 
@@ -423,7 +423,7 @@ UZU_API void uzu_unified_sampling_encode(uzu_command_buffer* cmd, const uzu_unif
 
 /* DeltaNetConvUpdateKernel / DeltaNetUpdateKernel (Qwen3.5 hybrid layers, decode branch):
  * backends/cpu/kernel/gdn/conv_update.rs:8-20, update.rs:13-30; parameter/state dtypes are f32 as
- * the engine allocates them and Metal declares them (SURVEY.md row a11). */
+ * the engine allocates them and Metal declares them. */
 typedef struct uzu_delta_net_conv_update_args {
     uint64_t conv_weight, bias /* optional(has_bias) */, in_out, state;
     uint32_t kernel_size, conv_dim, state_stride, has_bias;
@@ -1006,7 +1006,7 @@ UZU_API const char* uzu_engine_decode_mode_reason(const uzu_engine* e);
 UZU_API uzu_status uzu_engine_set_decode_mode(uzu_engine* e, int persistent);
 UZU_API uzu_status uzu_engine_last_logits(uzu_engine* e, uint16_t* out_logits);
 
-/* Speculative (trie) decode, the verify half (SURVEY 8f-4). Replaces what LanguageModelStream::generate does between "propose a trie" and
+/* Speculative (trie) decode, the verify half. Replaces what LanguageModelStream::generate does between "propose a trie" and
  * "accept a path" (engine/language_model/stream/stream.rs:550-657 and :436-520): the host (trie.rs, unchanged) linearizes the proposal into
  * `count` <= 16 nodes -- token ids, gpu_types::trie::TrieNode {trie_start, trie_end, height} from FlatTrie::token_subtrie_ranges
  * (trie.rs:211-222) and per-node seeds (token_seeds, :224-226; NULL = PRng::derive(context + height)) -- and

@@ -16,7 +16,7 @@ impl ActivationKernel for CudaActivationKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, in_place: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("Activation: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("Activation: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'input, 'output, 'encoder>(&self, input: Option<impl BufferArg<'input, Cuda>>, output: impl BufferArgMut<'output, Cuda>, n: u32, act_type: crate::backends::common::gpu_types::activation_type::ActivationType, encoder: &'encoder mut Encoder<Cuda>) {
@@ -61,7 +61,7 @@ impl AncestorAttentionKernel for CudaAncestorAttentionKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, HEAD_DIM: u32, num_heads: u32) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("AncestorAttention: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("AncestorAttention: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'prefix_kv, 'node_kv, 'current_qkv, 'cosines, 'sines, 'node_metadata, 'ancestor_indices, 'ancestor_counts, 'node_indices, 'output, 'encoder>(&self, prefix_kv: impl BufferArg<'prefix_kv, Cuda>, node_kv: impl BufferArgMut<'node_kv, Cuda>, current_qkv: impl BufferArg<'current_qkv, Cuda>, cosines: impl BufferArg<'cosines, Cuda>, sines: impl BufferArg<'sines, Cuda>, node_metadata: impl BufferArg<'node_metadata, Cuda>, ancestor_indices: impl BufferArg<'ancestor_indices, Cuda>, ancestor_counts: impl BufferArg<'ancestor_counts, Cuda>, node_indices: impl BufferArg<'node_indices, Cuda>, output: impl BufferArgMut<'output, Cuda>, rows: u32, prefix_length: u32, ancestor_stride: u32, node_capacity: u32, max_depth: u32, scale: f32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -75,7 +75,7 @@ impl AttentionFallbackScatterScoresKernel for CudaAttentionFallbackScatterScores
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, is_kv_cache_ring: bool, is_causal: bool, is_trie: bool, is_sliding_window: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("AttentionFallbackScatterScores: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("AttentionFallbackScatterScores: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'group_scores, 'scores, 'trie, 'encoder>(&self, group_scores: impl BufferArg<'group_scores, Cuda>, scores: impl BufferArgMut<'scores, Cuda>, ring_params: Option<crate::backends::common::gpu_types::ring::RingParams>, trie: Option<impl BufferArg<'trie, Cuda>>, sliding_window_size: Option<u32>, group_index: u32, gqa_factor: u32, sequence_length: u32, suffix_length: u32, total_elements: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -89,7 +89,7 @@ impl AttentionFallbackScatterValuesKernel for CudaAttentionFallbackScatterValues
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("AttentionFallbackScatterValues: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("AttentionFallbackScatterValues: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'group_output, 'out, 'encoder>(&self, group_output: impl BufferArg<'group_output, Cuda>, out: impl BufferArgMut<'out, Cuda>, group_index: u32, gqa_factor: u32, suffix_length: u32, num_heads: u32, head_dim: u32, total_elements: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -251,7 +251,7 @@ impl BuildTreeGramKernel for CudaBuildTreeGramKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, USE_MXU: bool, use_h0: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("BuildTreeGram: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("BuildTreeGram: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'q, 'k, 'trie, 'prefix, 'beta, 'h0, 'h0_idx, 'a_packed, 'qkd, 'a_inv, 'kh0, 'encoder>(&self, q: impl BufferArg<'q, Cuda>, k: impl BufferArg<'k, Cuda>, trie: impl BufferArg<'trie, Cuda>, prefix: impl BufferArg<'prefix, Cuda>, beta: impl BufferArg<'beta, Cuda>, h0: Option<impl BufferArg<'h0, Cuda>>, h0_idx: Option<impl BufferArg<'h0_idx, Cuda>>, a_packed: impl BufferArgMut<'a_packed, Cuda>, qkd: impl BufferArgMut<'qkd, Cuda>, a_inv: impl BufferArgMut<'a_inv, Cuda>, kh0: Option<impl BufferArgMut<'kh0, Cuda>>, scale: f32, batch_size: u32, tree_size: u32, k_heads: u32, value_heads: u32, head_k_dim: u32, head_v_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -265,7 +265,7 @@ impl BuildTreeOutKernel for CudaBuildTreeOutKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, QKT: DataType, OutputT: DataType, use_mxu: bool, transposed_h0: bool, use_h0: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("BuildTreeOut: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("BuildTreeOut: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'q, 'prefix, 'qkd, 'u, 'h0, 'h0_indices, 'o, 'encoder>(&self, q: impl BufferArg<'q, Cuda>, prefix: impl BufferArg<'prefix, Cuda>, qkd: impl BufferArg<'qkd, Cuda>, u: impl BufferArg<'u, Cuda>, h0: Option<impl BufferArg<'h0, Cuda>>, h0_indices: Option<impl BufferArg<'h0_indices, Cuda>>, o: impl BufferArgMut<'o, Cuda>, scale: f32, batch_size: u32, tree_size: u32, qk_heads: u32, value_heads: u32, head_k_dim: u32, head_v_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -279,7 +279,7 @@ impl BuildTreePrefixKernel for CudaBuildTreePrefixKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("BuildTreePrefix: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("BuildTreePrefix: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'trie, 'log_decay, 'prefix, 'encoder>(&self, trie: impl BufferArg<'trie, Cuda>, log_decay: impl BufferArg<'log_decay, Cuda>, prefix: impl BufferArgMut<'prefix, Cuda>, batch_size: u32, tree_size: u32, value_heads: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -293,7 +293,7 @@ impl ContextRingUpdateKernel for CudaContextRingUpdateKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("ContextRingUpdate: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("ContextRingUpdate: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'input, 'context_ring, 'encoder>(&self, input: impl BufferArg<'input, Cuda>, context_ring: impl BufferArgMut<'context_ring, Cuda>, suffix_repetition_length: u32, input_length: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -307,7 +307,7 @@ impl Conv1dDecodeKernel for CudaConv1dDecodeKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, has_bias: bool, state_in_place: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("Conv1dDecode: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("Conv1dDecode: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'x, 'w, 'b, 'state, 'x_out, 'b_out, 'c_out, 'next_state, 'encoder>(&self, x: impl BufferArg<'x, Cuda>, w: impl BufferArg<'w, Cuda>, b: Option<impl BufferArg<'b, Cuda>>, state: Option<impl BufferArg<'state, Cuda>>, x_out: impl BufferArgMut<'x_out, Cuda>, b_out: impl BufferArgMut<'b_out, Cuda>, c_out: impl BufferArgMut<'c_out, Cuda>, next_state: impl BufferArgMut<'next_state, Cuda>, kernel_size: u32, row_stride: u32, state_stride: u32, num_channels: u32, suffix_len: u32, inner_dim: u32, proj_dim: u32, activation_type: crate::backends::common::gpu_types::activation_type::ActivationType, encoder: &'encoder mut Encoder<Cuda>) {
@@ -321,7 +321,7 @@ impl Conv1dPackKernel for CudaConv1dPackKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, StateT: DataType, InputT: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("Conv1dPack: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("Conv1dPack: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'state_in, 'x, 'padded, 'encoder>(&self, state_in: impl BufferArg<'state_in, Cuda>, x: impl BufferArg<'x, Cuda>, padded: impl BufferArgMut<'padded, Cuda>, state_stride: u32, row_stride: u32, suffix_len: u32, num_channels: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -335,7 +335,7 @@ impl Conv1dScanKernel for CudaConv1dScanKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, has_bias: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("Conv1dScan: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("Conv1dScan: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'padded, 'w, 'b, 'x_out, 'b_out, 'c_out, 'state_out, 'encoder>(&self, padded: impl BufferArg<'padded, Cuda>, w: impl BufferArg<'w, Cuda>, b: Option<impl BufferArg<'b, Cuda>>, x_out: impl BufferArgMut<'x_out, Cuda>, b_out: impl BufferArgMut<'b_out, Cuda>, c_out: impl BufferArgMut<'c_out, Cuda>, state_out: impl BufferArgMut<'state_out, Cuda>, suffix_len: u32, kernel_size: u32, row_stride: u32, state_stride: u32, num_channels: u32, inner_dim: u32, proj_dim: u32, activation_type: crate::backends::common::gpu_types::activation_type::ActivationType, encoder: &'encoder mut Encoder<Cuda>) {
@@ -349,7 +349,7 @@ impl ConvTreeScanKernel for CudaConvTreeScanKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, kernel_size: u32, has_bias: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("ConvTreeScan: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("ConvTreeScan: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'in_proj, 'conv_weight, 'bias, 'base_state, 'parents, 'out_proj, 'suffix_state, 'encoder>(&self, in_proj: impl BufferArg<'in_proj, Cuda>, conv_weight: impl BufferArg<'conv_weight, Cuda>, bias: Option<impl BufferArg<'bias, Cuda>>, base_state: impl BufferArg<'base_state, Cuda>, parents: impl BufferArg<'parents, Cuda>, out_proj: impl BufferArgMut<'out_proj, Cuda>, suffix_state: impl BufferArgMut<'suffix_state, Cuda>, suffix_len: u32, total_proj_dim: u32, conv_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -363,7 +363,7 @@ impl DeltaNetConvScanKernel for CudaDeltaNetConvScanKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, has_bias: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("DeltaNetConvScan: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("DeltaNetConvScan: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'conv_padded, 'conv_weight, 'bias, 'in_proj, 'state_out, 'encoder>(&self, conv_padded: impl BufferArg<'conv_padded, Cuda>, conv_weight: impl BufferArg<'conv_weight, Cuda>, bias: Option<impl BufferArg<'bias, Cuda>>, in_proj: impl BufferArgMut<'in_proj, Cuda>, state_out: impl BufferArgMut<'state_out, Cuda>, suffix_len: u32, kernel_size: u32, row_stride: u32, state_stride: u32, conv_dim: u32, out_stride: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -403,7 +403,7 @@ impl DeltaNetNormGateKernel for CudaDeltaNetNormGateKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("DeltaNetNormGate: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("DeltaNetNormGate: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'in_out, 'in_proj, 'norm_weight, 'encoder>(&self, in_out: impl BufferArgMut<'in_out, Cuda>, in_proj: impl BufferArg<'in_proj, Cuda>, norm_weight: impl BufferArg<'norm_weight, Cuda>, num_v_heads: u32, head_v_dim: u32, value_dim: u32, conv_dim: u32, total_proj_dim: u32, norm_epsilon: f32, suffix_len: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -417,7 +417,7 @@ impl DeltaNetPrefillKernel for CudaDeltaNetPrefillKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, HEAD_K_DIM: u32) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("DeltaNetPrefill: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("DeltaNetPrefill: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'q_norm, 'k_norm, 'beta_buf, 'decay_buf, 'in_proj, 'state, 'out, 'encoder>(&self, q_norm: impl BufferArg<'q_norm, Cuda>, k_norm: impl BufferArg<'k_norm, Cuda>, beta_buf: impl BufferArg<'beta_buf, Cuda>, decay_buf: impl BufferArg<'decay_buf, Cuda>, in_proj: impl BufferArg<'in_proj, Cuda>, state: impl BufferArgMut<'state, Cuda>, out: impl BufferArgMut<'out, Cuda>, num_v_heads: u32, num_k_heads: u32, head_v_dim: u32, key_dim: u32, value_dim: u32, suffix_len: u32, num_dv_groups: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -431,7 +431,7 @@ impl DeltaNetPrefillPrepKernel for CudaDeltaNetPrefillPrepKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, QKT: DataType, HEAD_K_DIM: u32, write_log_decay: bool, write_compact_v: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("DeltaNetPrefillPrep: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("DeltaNetPrefillPrep: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'in_proj, 'a_log, 'dt_bias, 'q_norm_out, 'k_norm_out, 'compact_v_out, 'beta_out, 'decay_out, 'encoder>(&self, in_proj: impl BufferArg<'in_proj, Cuda>, a_log: impl BufferArg<'a_log, Cuda>, dt_bias: impl BufferArg<'dt_bias, Cuda>, q_norm_out: impl BufferArgMut<'q_norm_out, Cuda>, k_norm_out: impl BufferArgMut<'k_norm_out, Cuda>, compact_v_out: Option<impl BufferArgMut<'compact_v_out, Cuda>>, beta_out: impl BufferArgMut<'beta_out, Cuda>, decay_out: impl BufferArgMut<'decay_out, Cuda>, num_v_heads: u32, num_k_heads: u32, key_dim: u32, value_dim: u32, suffix_len: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -560,7 +560,7 @@ impl MoeBlockBasesFromPartialsKernel for CudaMoeBlockBasesFromPartialsKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeBlockBasesFromPartials: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeBlockBasesFromPartials: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'partials, 'block_bases, 'block_alloc, 'encoder>(&self, partials: impl BufferArg<'partials, Cuda>, block_bases: impl BufferArgMut<'block_bases, Cuda>, block_alloc: impl BufferArgMut<'block_alloc, Cuda>, e_input: u32, num_blocks: u32, num_tiles: u32, capacity_per_expert: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -574,7 +574,7 @@ impl MoeBuildTileMapKernel for CudaMoeBuildTileMapKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeBuildTileMap: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeBuildTileMap: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'offsets, 'tile_row_offsets, 'tile_counts, 'tile_map, 'encoder>(&self, offsets: impl BufferArg<'offsets, Cuda>, tile_row_offsets: impl BufferArg<'tile_row_offsets, Cuda>, tile_counts: impl BufferArg<'tile_counts, Cuda>, tile_map: impl BufferArgMut<'tile_map, Cuda>, e: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -588,7 +588,7 @@ impl MoeCountsOffsetsFusedKernel for CudaMoeCountsOffsetsFusedKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeCountsOffsetsFused: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeCountsOffsetsFused: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'topk_ids, 'offsets, 'sum_k_out, 'partials, 'encoder>(&self, topk_ids: impl BufferArg<'topk_ids, Cuda>, offsets: impl BufferArgMut<'offsets, Cuda>, sum_k_out: impl BufferArgMut<'sum_k_out, Cuda>, partials: impl BufferArgMut<'partials, Cuda>, t_input: u32, e_input: u32, k_input: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -602,7 +602,7 @@ impl MoeExpertsDecodeDownFused2DKernel for CudaMoeExpertsDecodeDownFused2DKernel
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, AccumT: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeExpertsDecodeDownFused2D: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeExpertsDecodeDownFused2D: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'hidden, 'row_expert_map, 'w2_all, 'down_biases, 'y_out, 'encoder>(&self, hidden: impl BufferArg<'hidden, Cuda>, row_expert_map: impl BufferArg<'row_expert_map, Cuda>, w2_all: impl BufferArg<'w2_all, Cuda>, down_biases: impl BufferArg<'down_biases, Cuda>, y_out: impl BufferArgMut<'y_out, Cuda>, total_rows: u32, d_model: u32, d_ff: u32, e: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -616,7 +616,7 @@ impl MoeExpertsDecodePassAKernel for CudaMoeExpertsDecodePassAKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, gating_sel: u32) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeExpertsDecodePassA: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeExpertsDecodePassA: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'x_perm, 'expert_offsets, 'w13_all, 'hidden_out, 'up_biases, 'tile_map, '__dsl_indirect_dispatch_buffer, 'encoder>(&self, x_perm: impl BufferArg<'x_perm, Cuda>, expert_offsets: impl BufferArg<'expert_offsets, Cuda>, w13_all: impl BufferArg<'w13_all, Cuda>, hidden_out: impl BufferArgMut<'hidden_out, Cuda>, up_biases: impl BufferArg<'up_biases, Cuda>, d_model: u32, d_ff: u32, e: u32, gate_clip_min: f32, gate_clip_max: f32, up_clip_min: f32, up_clip_max: f32, silu_alpha: f32, tile_map: impl BufferArg<'tile_map, Cuda>, __dsl_indirect_dispatch_buffer: impl BufferArg<'__dsl_indirect_dispatch_buffer, Cuda>, encoder: &'encoder mut Encoder<Cuda>) {
@@ -630,7 +630,7 @@ impl MoeExpertsPrefillPassAKernel for CudaMoeExpertsPrefillPassAKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, gating_sel: u32) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeExpertsPrefillPassA: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeExpertsPrefillPassA: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'x_perm, 'expert_offsets, 'w13_all, 'up_biases, 'hidden_out, 'tile_map, '__dsl_indirect_dispatch_buffer, 'encoder>(&self, x_perm: impl BufferArg<'x_perm, Cuda>, expert_offsets: impl BufferArg<'expert_offsets, Cuda>, w13_all: impl BufferArg<'w13_all, Cuda>, up_biases: impl BufferArg<'up_biases, Cuda>, hidden_out: impl BufferArgMut<'hidden_out, Cuda>, d_model: u32, d_ff: u32, e: u32, gate_clip_min: f32, gate_clip_max: f32, up_clip_min: f32, up_clip_max: f32, silu_alpha: f32, tile_map: impl BufferArg<'tile_map, Cuda>, __dsl_indirect_dispatch_buffer: impl BufferArg<'__dsl_indirect_dispatch_buffer, Cuda>, encoder: &'encoder mut Encoder<Cuda>) {
@@ -644,7 +644,7 @@ impl MoeExpertsPrefillPassBKernel for CudaMoeExpertsPrefillPassBKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeExpertsPrefillPassB: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeExpertsPrefillPassB: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'hidden, 'expert_offsets, 'w2_all, 'down_biases, 'output, 'tile_map, '__dsl_indirect_dispatch_buffer, 'encoder>(&self, hidden: impl BufferArg<'hidden, Cuda>, expert_offsets: impl BufferArg<'expert_offsets, Cuda>, w2_all: impl BufferArg<'w2_all, Cuda>, down_biases: impl BufferArg<'down_biases, Cuda>, output: impl BufferArgMut<'output, Cuda>, d_model: u32, d_ff: u32, e: u32, tile_map: impl BufferArg<'tile_map, Cuda>, __dsl_indirect_dispatch_buffer: impl BufferArg<'__dsl_indirect_dispatch_buffer, Cuda>, encoder: &'encoder mut Encoder<Cuda>) {
@@ -658,7 +658,7 @@ impl MoeFinalizeKernel for CudaMoeFinalizeKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeFinalize: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeFinalize: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'tok2row, 'probs, 'y_partial, 'y, 'encoder>(&self, tok2row: impl BufferArg<'tok2row, Cuda>, probs: impl BufferArg<'probs, Cuda>, y_partial: impl BufferArg<'y_partial, Cuda>, y: impl BufferArgMut<'y, Cuda>, t_count: u32, d_model: u32, k_input: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -672,7 +672,7 @@ impl MoeGatherXPerm1DKernel for CudaMoeGatherXPerm1DKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeGatherXPerm1D: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeGatherXPerm1D: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'x, 'bucketed_ids, 'x_perm, 'sumk_buf, 'encoder>(&self, x: impl BufferArg<'x, Cuda>, bucketed_ids: impl BufferArg<'bucketed_ids, Cuda>, x_perm: impl BufferArgMut<'x_perm, Cuda>, sumk_buf: impl BufferArg<'sumk_buf, Cuda>, d_model: u32, t: u32, k: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -686,7 +686,7 @@ impl MoeGatherXPerm2DKernel for CudaMoeGatherXPerm2DKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeGatherXPerm2D: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeGatherXPerm2D: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'x, 'bucketed_ids, 'x_perm, 'sumk_buf, 'encoder>(&self, x: impl BufferArg<'x, Cuda>, bucketed_ids: impl BufferArg<'bucketed_ids, Cuda>, x_perm: impl BufferArgMut<'x_perm, Cuda>, sumk_buf: impl BufferArg<'sumk_buf, Cuda>, d_model: u32, t: u32, k: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -700,7 +700,7 @@ impl MoePassABuildRowMapKernel for CudaMoePassABuildRowMapKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoePassABuildRowMap: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoePassABuildRowMap: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'expert_offsets, 'row_expert_map, 'encoder>(&self, expert_offsets: impl BufferArg<'expert_offsets, Cuda>, row_expert_map: impl BufferArgMut<'row_expert_map, Cuda>, total_rows: u32, e: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -714,7 +714,7 @@ impl MoePassABuildTileMapKernel for CudaMoePassABuildTileMapKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoePassABuildTileMap: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoePassABuildTileMap: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'expert_offsets, 'tile_offsets, 'row_expert_map, 'tile_map, 'encoder>(&self, expert_offsets: impl BufferArg<'expert_offsets, Cuda>, tile_offsets: impl BufferArg<'tile_offsets, Cuda>, row_expert_map: impl BufferArg<'row_expert_map, Cuda>, tile_map: impl BufferArgMut<'tile_map, Cuda>, total_rows: u32, h_blocks: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -728,7 +728,7 @@ impl MoePassATileCountsKernel for CudaMoePassATileCountsKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoePassATileCounts: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoePassATileCounts: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'expert_offsets, 'tile_counts, 'encoder>(&self, expert_offsets: impl BufferArg<'expert_offsets, Cuda>, tile_counts: impl BufferArgMut<'tile_counts, Cuda>, e: u32, h_blocks: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -742,7 +742,7 @@ impl MoePassATileScanKernel for CudaMoePassATileScanKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoePassATileScan: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoePassATileScan: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'tile_counts, 'tile_offsets, 'total_tiles, 'encoder>(&self, tile_counts: impl BufferArg<'tile_counts, Cuda>, tile_offsets: impl BufferArgMut<'tile_offsets, Cuda>, total_tiles: impl BufferArgMut<'total_tiles, Cuda>, e: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -756,7 +756,7 @@ impl MoePassAWriteDispatchArgsKernel for CudaMoePassAWriteDispatchArgsKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoePassAWriteDispatchArgs: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoePassAWriteDispatchArgs: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'total_tiles, 'dispatch_args, 'encoder>(&self, total_tiles: impl BufferArg<'total_tiles, Cuda>, dispatch_args: impl BufferArgMut<'dispatch_args, Cuda>, num_tiles_y: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -770,7 +770,7 @@ impl MoeRouterTopKKernel for CudaMoeRouterTopKKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, ScalarT: DataType, has_biases: bool, has_router_scales: bool, has_per_expert_scales: bool, has_router_input_scale: bool, normalize_router_input: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeRouterTopK: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeRouterTopK: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'input, 'weight, 'bias, 'router_scale, 'per_expert_scale, 'topk_ids, 'topk_probs, 'encoder>(&self, input: impl BufferArg<'input, Cuda>, weight: impl BufferArg<'weight, Cuda>, bias: Option<impl BufferArg<'bias, Cuda>>, router_scale: Option<impl BufferArg<'router_scale, Cuda>>, per_expert_scale: Option<impl BufferArg<'per_expert_scale, Cuda>>, topk_ids: impl BufferArgMut<'topk_ids, Cuda>, topk_probs: impl BufferArgMut<'topk_probs, Cuda>, t: u32, d_model: u32, e: u32, k: u32, renorm: bool, router_norm_epsilon: Option<f32>, router_input_scale: Option<f32>, encoder: &'encoder mut Encoder<Cuda>) {
@@ -784,7 +784,7 @@ impl MoeScatterBucketsMapKernel for CudaMoeScatterBucketsMapKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeScatterBucketsMap: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeScatterBucketsMap: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'topk_ids, 'topk_probs, 'offsets, 'block_bases, 'block_alloc, 'out_ids, 'out_probs, 'tok2row, 'encoder>(&self, topk_ids: impl BufferArg<'topk_ids, Cuda>, topk_probs: impl BufferArg<'topk_probs, Cuda>, offsets: impl BufferArg<'offsets, Cuda>, block_bases: impl BufferArg<'block_bases, Cuda>, block_alloc: impl BufferArg<'block_alloc, Cuda>, out_ids: impl BufferArgMut<'out_ids, Cuda>, out_probs: impl BufferArgMut<'out_probs, Cuda>, t: u32, e: u32, k: u32, num_blocks: u32, num_tiles: u32, tok2row: impl BufferArgMut<'tok2row, Cuda>, encoder: &'encoder mut Encoder<Cuda>) {
@@ -798,7 +798,7 @@ impl MoeTileCountsKernel for CudaMoeTileCountsKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeTileCounts: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeTileCounts: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'offsets, 'tile_counts, 'encoder>(&self, offsets: impl BufferArg<'offsets, Cuda>, tile_counts: impl BufferArgMut<'tile_counts, Cuda>, e: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -812,7 +812,7 @@ impl MoeTileScanKernel for CudaMoeTileScanKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeTileScan: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeTileScan: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'tile_counts, 'tile_row_offsets, 'total_tiles_buf, 'encoder>(&self, tile_counts: impl BufferArg<'tile_counts, Cuda>, tile_row_offsets: impl BufferArgMut<'tile_row_offsets, Cuda>, total_tiles_buf: impl BufferArgMut<'total_tiles_buf, Cuda>, e: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -826,7 +826,7 @@ impl MoeWriteDispatchArgsKernel for CudaMoeWriteDispatchArgsKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("MoeWriteDispatchArgs: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("MoeWriteDispatchArgs: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'total_tiles_buf, 'dispatch_args, 'encoder>(&self, total_tiles_buf: impl BufferArg<'total_tiles_buf, Cuda>, dispatch_args: impl BufferArgMut<'dispatch_args, Cuda>, num_tiles_n: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -881,7 +881,7 @@ impl PoolingMeanKernel for CudaPoolingMeanKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("PoolingMean: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("PoolingMean: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'input, 'output, 'encoder>(&self, input: impl BufferArg<'input, Cuda>, output: impl BufferArgMut<'output, Cuda>, seq_len: u32, hidden_dim: u32, batch_size: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -959,7 +959,7 @@ impl RepetitionPenaltyKernel for CudaRepetitionPenaltyKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("RepetitionPenalty: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("RepetitionPenalty: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'original_logits, 'logits_copy, 'context_ring, 'token_ids, 'encoder>(&self, original_logits: impl BufferArg<'original_logits, Cuda>, logits_copy: impl BufferArgMut<'logits_copy, Cuda>, context_ring: impl BufferArg<'context_ring, Cuda>, token_ids: impl BufferArg<'token_ids, Cuda>, repetition_penalty: f32, suffix_repetition_length: u32, vocab_size: u32, sampling_start: u32, sampling_length: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -973,7 +973,7 @@ impl SSDPrefillKernel for CudaSSDPrefillKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("SSDPrefill: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("SSDPrefill: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'x, 'dt_raw, 'b, 'c, 'd, 'z, 'state, 'y, 'encoder>(&self, x: impl BufferArg<'x, Cuda>, dt_raw: impl BufferArg<'dt_raw, Cuda>, b: impl BufferArg<'b, Cuda>, c: impl BufferArg<'c, Cuda>, d: impl BufferArg<'d, Cuda>, z: impl BufferArg<'z, Cuda>, state: impl BufferArgMut<'state, Cuda>, y: impl BufferArgMut<'y, Cuda>, suffix_len: u32, group_size: u32, state_size: u32, x_strides: &[u32; 3], dt_strides: &[u32; 2], cb_strides: &[u32; 3], state_strides: &[u32; 3], num_heads: u32, head_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -987,7 +987,7 @@ impl SSDPrefill64Kernel for CudaSSDPrefill64Kernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("SSDPrefill64: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("SSDPrefill64: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'x, 'dt_raw, 'b, 'c, 'd, 'z, 'state, 'y, 'encoder>(&self, x: impl BufferArg<'x, Cuda>, dt_raw: impl BufferArg<'dt_raw, Cuda>, b: impl BufferArg<'b, Cuda>, c: impl BufferArg<'c, Cuda>, d: impl BufferArg<'d, Cuda>, z: impl BufferArg<'z, Cuda>, state: impl BufferArgMut<'state, Cuda>, y: impl BufferArgMut<'y, Cuda>, suffix_len: u32, group_size: u32, state_size: u32, x_strides: &[u32; 3], dt_strides: &[u32; 2], cb_strides: &[u32; 3], state_strides: &[u32; 3], num_heads: u32, head_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1001,7 +1001,7 @@ impl SSDUpdateKernel for CudaSSDUpdateKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, state_in_place: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("SSDUpdate: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("SSDUpdate: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'x, 'dt_raw, 'b, 'c, 'd, 'z, 'state, 'y, 'next_state, 'encoder>(&self, x: impl BufferArg<'x, Cuda>, dt_raw: impl BufferArg<'dt_raw, Cuda>, b: impl BufferArg<'b, Cuda>, c: impl BufferArg<'c, Cuda>, d: impl BufferArg<'d, Cuda>, z: impl BufferArg<'z, Cuda>, state: Option<impl BufferArg<'state, Cuda>>, y: impl BufferArgMut<'y, Cuda>, next_state: impl BufferArgMut<'next_state, Cuda>, group_size: u32, state_size: u32, x_strides: &[u32; 3], dt_strides: &[u32; 2], cb_strides: &[u32; 3], state_strides: &[u32; 4], b_size: u32, h_size: u32, dh_size: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1015,7 +1015,7 @@ impl ShortConvDecodeKernel for CudaShortConvDecodeKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, WeightT: DataType, has_bias: bool, state_in_place: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("ShortConvDecode: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("ShortConvDecode: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'in_proj, 'w, 'b, 'state, 'out, 'next_state, 'encoder>(&self, in_proj: impl BufferArg<'in_proj, Cuda>, w: impl BufferArg<'w, Cuda>, b: Option<impl BufferArg<'b, Cuda>>, state: Option<impl BufferArg<'state, Cuda>>, out: impl BufferArgMut<'out, Cuda>, next_state: impl BufferArgMut<'next_state, Cuda>, suffix_len: u32, kernel_size: u32, in_proj_stride: u32, state_stride: u32, model_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1029,7 +1029,7 @@ impl ShortConvPackKernel for CudaShortConvPackKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("ShortConvPack: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("ShortConvPack: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'state_in, 'in_proj, 'padded, 'encoder>(&self, state_in: impl BufferArg<'state_in, Cuda>, in_proj: impl BufferArg<'in_proj, Cuda>, padded: impl BufferArgMut<'padded, Cuda>, state_stride: u32, suffix_len: u32, in_proj_stride: u32, model_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1043,7 +1043,7 @@ impl ShortConvPrefillKernel for CudaShortConvPrefillKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, WeightT: DataType, has_bias: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("ShortConvPrefill: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("ShortConvPrefill: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'padded, 'in_proj, 'w, 'b, 'out, 'state_out, 'encoder>(&self, padded: impl BufferArg<'padded, Cuda>, in_proj: impl BufferArg<'in_proj, Cuda>, w: impl BufferArg<'w, Cuda>, b: Option<impl BufferArg<'b, Cuda>>, out: impl BufferArgMut<'out, Cuda>, state_out: impl BufferArgMut<'state_out, Cuda>, suffix_len: u32, kernel_size: u32, in_proj_stride: u32, state_stride: u32, model_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1057,7 +1057,7 @@ impl ShortConvTrieKernel for CudaShortConvTrieKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, WeightT: DataType, has_bias: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("ShortConvTrie: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("ShortConvTrie: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'in_proj, 'w, 'b, 'base_state, 'parents, 'out, 'suffix_state, 'encoder>(&self, in_proj: impl BufferArg<'in_proj, Cuda>, w: impl BufferArg<'w, Cuda>, b: Option<impl BufferArg<'b, Cuda>>, base_state: impl BufferArg<'base_state, Cuda>, parents: impl BufferArg<'parents, Cuda>, out: impl BufferArgMut<'out, Cuda>, suffix_state: impl BufferArgMut<'suffix_state, Cuda>, suffix_len: u32, kernel_size: u32, in_proj_stride: u32, state_stride: u32, model_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1087,7 +1087,7 @@ impl SoftmaxKernel for CudaSoftmaxKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, has_sinks: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("Softmax: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("Softmax: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'values, 'sinks, 'encoder>(&self, values: impl BufferArgMut<'values, Cuda>, sinks: Option<impl BufferArg<'sinks, Cuda>>, row_length: u32, outer_dim: u32, batch_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1101,7 +1101,7 @@ impl SplitInProjKernel for CudaSplitInProjKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("SplitInProj: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("SplitInProj: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'input, 'conv_out, 'z_out, 'dt_out, 'z_bias, 'encoder>(&self, input: impl BufferArg<'input, Cuda>, conv_out: impl BufferArgMut<'conv_out, Cuda>, z_out: impl BufferArgMut<'z_out, Cuda>, dt_out: impl BufferArgMut<'dt_out, Cuda>, z_bias: impl BufferArg<'z_bias, Cuda>, suffix_length: u32, total_dim: u32, conv_dim: u32, inner_dim: u32, num_heads: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1115,7 +1115,7 @@ impl StateAdvanceKernel for CudaStateAdvanceKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, HEAD_K_DIM: u32, num_v_heads: u32, num_k_heads: u32) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("StateAdvance: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("StateAdvance: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'k_norm, 'v, 'log_decay_buf, 'beta_buf, 'accepted_indices, 'state, 'encoder>(&self, k_norm: impl BufferArg<'k_norm, Cuda>, v: impl BufferArg<'v, Cuda>, log_decay_buf: impl BufferArg<'log_decay_buf, Cuda>, beta_buf: impl BufferArg<'beta_buf, Cuda>, accepted_indices: impl BufferArg<'accepted_indices, Cuda>, state: impl BufferArgMut<'state, Cuda>, accepted_len: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1194,7 +1194,7 @@ impl TreeUpdateSolveKernel for CudaTreeUpdateSolveKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext, T: DataType, BV: u32, use_h0: bool) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("TreeUpdateSolve: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("TreeUpdateSolve: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'kh0, 'v, 'prefix, 'beta, 'a_packed, 'a_inv, 'h0_idx, 'u, 'encoder>(&self, kh0: Option<impl BufferArg<'kh0, Cuda>>, v: impl BufferArg<'v, Cuda>, prefix: impl BufferArg<'prefix, Cuda>, beta: impl BufferArg<'beta, Cuda>, a_packed: impl BufferArg<'a_packed, Cuda>, a_inv: impl BufferArg<'a_inv, Cuda>, h0_idx: Option<impl BufferArg<'h0_idx, Cuda>>, u: impl BufferArgMut<'u, Cuda>, batch_size: u32, tree_size: u32, value_heads: u32, head_v_dim: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1242,7 +1242,7 @@ impl WeaverFrontierInsertChildrenKernel for CudaWeaverFrontierInsertChildrenKern
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("WeaverFrontierInsertChildren: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("WeaverFrontierInsertChildren: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'packed_tree, 'node_metadata, 'node_valid, 'child_ids, 'child_logprobs, 'frontier, 'encoder>(&self, packed_tree: impl BufferArg<'packed_tree, Cuda>, node_metadata: impl BufferArg<'node_metadata, Cuda>, node_valid: impl BufferArg<'node_valid, Cuda>, child_ids: impl BufferArg<'child_ids, Cuda>, child_logprobs: impl BufferArg<'child_logprobs, Cuda>, frontier: impl BufferArgMut<'frontier, Cuda>, frontier_capacity: u32, tree_slot_count: u32, node_count: u32, expand_width: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1256,7 +1256,7 @@ impl WeaverFrontierSelectKernel for CudaWeaverFrontierSelectKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("WeaverFrontierSelect: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("WeaverFrontierSelect: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'frontier, 'packed_tree, 'slot_ancestors, 'node_token_ids, 'node_metadata, 'node_ancestor_indices, 'node_valid, 'candidate_pool_ids, 'candidate_pool_logits, 'node_candidate_ids, 'node_candidate_logits, 'encoder>(&self, frontier: impl BufferArgMut<'frontier, Cuda>, packed_tree: impl BufferArgMut<'packed_tree, Cuda>, slot_ancestors: impl BufferArgMut<'slot_ancestors, Cuda>, node_token_ids: impl BufferArgMut<'node_token_ids, Cuda>, node_metadata: impl BufferArgMut<'node_metadata, Cuda>, node_ancestor_indices: impl BufferArgMut<'node_ancestor_indices, Cuda>, node_valid: impl BufferArgMut<'node_valid, Cuda>, candidate_pool_ids: impl BufferArg<'candidate_pool_ids, Cuda>, candidate_pool_logits: impl BufferArg<'candidate_pool_logits, Cuda>, node_candidate_ids: impl BufferArgMut<'node_candidate_ids, Cuda>, node_candidate_logits: impl BufferArgMut<'node_candidate_logits, Cuda>, frontier_capacity: u32, tree_slot_count: u32, node_count: u32, batch_start_slot: u32, ancestor_stride: u32, max_depth: u32, lookahead_count: u32, candidate_depth_count: u32, candidates_per_depth: u32, encoder: &'encoder mut Encoder<Cuda>) {
@@ -1270,7 +1270,7 @@ impl WeaverTopChildrenKernel for CudaWeaverTopChildrenKernel {
     type Backend = Cuda;
     #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]
     fn new(context: &CudaContext) -> Result<Self, CudaError> {
-        Err(CudaError::NotSupported("WeaverTopChildren: outside the CUDA decode hot path (SURVEY 8 scope)"))
+        Err(CudaError::NotSupported("WeaverTopChildren: outside the CUDA decode hot path"))
     }
     #[allow(unused_variables, clippy::too_many_arguments)]
     fn encode<'residual_logits, 'candidate_logits, 'candidate_ids, 'depth_seeds, 'node_metadata, 'output_token_ids, 'output_model_logprobs, 'encoder>(&self, residual_logits: impl BufferArg<'residual_logits, Cuda>, candidate_logits: impl BufferArg<'candidate_logits, Cuda>, candidate_ids: impl BufferArg<'candidate_ids, Cuda>, depth_seeds: impl BufferArg<'depth_seeds, Cuda>, node_metadata: impl BufferArg<'node_metadata, Cuda>, output_token_ids: impl BufferArgMut<'output_token_ids, Cuda>, output_model_logprobs: impl BufferArgMut<'output_model_logprobs, Cuda>, rows: u32, candidates: u32, expand_width: u32, vocab_size: u32, encoder: &'encoder mut Encoder<Cuda>) {

@@ -94,7 +94,7 @@ class OracleModel:
     """`tp_reduce` / `tp_gather`: the two exchange steps of a tensor-parallel shard written by uzu_b200.tp.shard_checkpoint
     (config.json carries a "tensor_parallel" block): f32 partial sums [m, H] of the row-parallel out / down projections are summed
     over ranks (all-reduce) and rounded to bf16 once; the vocab-parallel readout's [rows, V/P] logits are concatenated (all-gather).
-    The reference has no tensor parallelism; the 1-rank model is the oracle for the P-rank one (SURVEY 8e)."""
+    The reference has no tensor parallelism; the 1-rank model is the oracle for the P-rank one."""
 
     def __init__(self, path, threads: int = 1, max_context: int = 4096, tp_reduce=None, tp_gather=None):
         path = Path(path)

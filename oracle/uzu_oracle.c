@@ -1,16 +1,16 @@
 /*
  * uzu_oracle.c -- CPU restatement of the uzu reference CPU backend for the transformer
- * decode hot path (SURVEY.md section 8c).
+ * decode hot path.
  *
  * THIS IS TEST INFRASTRUCTURE. Only tests/, __graft_entry__.smoke() and bench.py's
  * cpu_baseline / --impl reference legs may load it. The product (libuzu_b200.so) never
  * links, loads or calls anything in oracle/.
  *
  * The reference (trymirai/uzu @ 9670da1) is Rust; no Rust toolchain exists in this image, so
- * the reference itself cannot be compiled or run here (DESIGN.md "Oracle"). Every function
+ * the reference itself cannot be compiled or run here. Every function
  * below restates one reference CPU kernel loop-for-loop, with the same accumulation order and
  * the same rounding points, and cites the file:line it follows (paths relative to
- * /root/reference/crates/backend-uzu/src/).
+ * crates/backend-uzu/src/ of the reference).
  *
  * Pinning status: the reference tests hold NO stored outputs for this path except the
  * `unit_interval` endpoints (tests/unit/encodable_block/sampling/gumbel_test.rs:7-12), which
@@ -315,7 +315,7 @@ ORACLE_API void oracle_qkv_norm(bf16_t* qkv, const float* scales, int batch_size
 
 /* ------------------------------------------------------------------------------------------
  * RoPE tables: encodable_block/mixer/attention/rope.rs:13-114 (host f32 math).
- * kind: 0 unscaled, 1 linear, 2 llama3. (YaRN / LongRoPE: not in any BASELINE config.)
+ * kind: 0 unscaled, 1 linear, 2 llama3. (YaRN / LongRoPE: not in any measured model's config.)
  * ---------------------------------------------------------------------------------------- */
 typedef struct {
     int kind;
@@ -694,7 +694,7 @@ ORACLE_API void oracle_tensor_add_swap(bf16_t* skip, bf16_t* main_, int length) 
 }
 
 /* ------------------------------------------------------------------------------------------
- * ActivationTransform (Mirai RHT, SURVEY 8f-3): backends/cpu/kernel/activation_transform/
+ * ActivationTransform (Mirai RHT): backends/cpu/kernel/activation_transform/
  * {activation_transform.rs:44-136, mod.rs:31-44}. 32-point Walsh-Hadamard per stripe in f32
  * (butterflies stride 1,2,4,8,16: lower = a+b, upper = a-b; then * 1/sqrt(32)); InputRht multiplies
  * by the +-1 factors before the transform, OutputRht after. Quantize ops: symmetric int8 per
@@ -901,10 +901,10 @@ ORACLE_API void oracle_unified_sampling(const oracle_sampling_args* p) {
 }
 
 /* ------------------------------------------------------------------------------------------
- * DeltaNet decode (Qwen3.5 hybrid layers; SURVEY.md 8(f)-1): backends/cpu/kernel/gdn/
+ * DeltaNet decode (Qwen3.5 hybrid layers): backends/cpu/kernel/gdn/
  * conv_update.rs:8-55 and update.rs:13-144, with the parameter/state element types the engine
- * actually allocates and Metal declares (f32 a_log/dt_bias/norm_weight/state; SURVEY.md row
- * a11 documents the reference CPU kernel's mistyped pointers).
+ * actually allocates and Metal declares (f32 a_log/dt_bias/norm_weight/state; the reference CPU
+ * kernel's pointers have another type).
  * ---------------------------------------------------------------------------------------- */
 ORACLE_API void oracle_delta_net_conv_update(const float* conv_weight, const float* bias, bf16_t* in_out, float* state,
                                              int kernel_size, int conv_dim, int state_stride) {

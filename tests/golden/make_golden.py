@@ -1,7 +1,7 @@
 """Regenerates tests/golden/*.npz with the CPU oracle (run from the repo root: python tests/golden/make_golden.py).
 
 These are ORACLE-generated regression vectors (the reference stores no outputs for this path and cannot be run
-here -- see DESIGN.md section 2): they freeze the oracle's behaviour and give the GPU tests fixed targets that do
+here): they freeze the oracle's behaviour and give the GPU tests fixed targets that do
 not depend on the oracle library being rebuilt."""
 import sys
 import tempfile

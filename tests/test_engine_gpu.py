@@ -369,7 +369,7 @@ def test_delta_net_fused_conv_update_matches_two_kernels(ctx):
 
 
 def test_real_qwen35_0p8b_dims_both_decode_paths(ctx, tmp_path):
-    """BASELINE configs[1] at its REAL dimensions (Qwen3.5-0.8B hybrid: 18 DeltaNet + 6 attention layers, model_dim 1024, vocabulary
+    """The small hybrid model at its REAL dimensions (Qwen3.5-0.8B: 18 DeltaNet + 6 attention layers, model_dim 1024, vocabulary
     248320, int4 gs64), not a toy: a short prompt, then decode steps under teacher forcing through BOTH decode paths (per-kernel CUDA-graph
     path and the persistent whole-token kernel) against the CPU oracle. Greedy token ids must match wherever the oracle's top-2 gap is
     not a near-tie; logits within the bf16 output budget."""

@@ -1,8 +1,8 @@
 """Parity of every CUDA kernel (called through the C ABI) against the CPU oracle on the same seeded inputs.
-Shapes follow the reference's own kernel tests (tests/unit/backends/common/kernel/**) plus the BASELINE
+Shapes follow the reference's own kernel tests (tests/unit/backends/common/kernel/**) plus the measured
 layer shapes. Integer / index outputs are compared bit-exactly; bf16 outputs of kernels whose f32 summation
 order necessarily differs from the sequential CPU loop are held to <= 1 bf16 ulp with >= 97 % identical bits,
-and to rtol 1e-3 / atol 1e-4 on f32 outputs (BASELINE.json north_star tolerance)."""
+and to rtol 1e-3 / atol 1e-4 on f32 outputs."""
 import numpy as np
 import pytest
 
@@ -23,7 +23,7 @@ def _quant_case(seed, m, n, k, bits, gs, method, scale_lo=0.01, scale_hi=0.3):
     return x, packed, dict(scales=scales, zero_points=zp, biases=biases, method=method, bits=bits, group_size=gs)
 
 
-# quant_dispatch_test.rs:102-167 matrix (shape x group x method) + decode shapes of the BASELINE models
+# quant_dispatch_test.rs:102-167 matrix (shape x group x method) + decode shapes of the measured models
 QUANT_CASES = [
     (1, 64, 128, 4, 64, "zp"), (1, 48, 256, 4, 32, "mlx"), (1, 2048, 4096, 4, 64, "zp"), (4, 64, 4096, 4, 128, "sym"),
     (8, 2048, 128, 4, 64, "mlx"), (1, 11, 512, 8, 64, "zp"), (3, 100, 1024, 8, 32, "mlx"), (2, 64, 2048, 8, 128, "sym"),
@@ -43,8 +43,8 @@ def test_quantized_matmul_f32_out(ctx, m, n, k, bits, gs, method):
     assert_f32_close(got, ref, rtol=1e-3, atol=1e-4, what=f"matmul {m}x{n}x{k} int{bits} gs{gs} {method}")
 
 
-# the readout matrices of the BASELINE models and int8 gs64 at Llama-3-8B K
-BASELINE_SHAPES = [
+# the readout matrices of the measured models and int8 gs64 at Llama-3-8B K
+MODEL_SHAPES = [
     (1, 128256, 4096, 4, 64, "zp"),    # Llama-3-8B readout
     (1, 248320, 1024, 4, 64, "zp"),    # Qwen3.5-0.8B readout
     (1, 6144, 4096, 8, 64, "zp"),      # Llama-3-8B int8 qkv
@@ -53,7 +53,7 @@ BASELINE_SHAPES = [
 ]
 
 
-@pytest.mark.parametrize("m,n,k,bits,gs,method", BASELINE_SHAPES)
+@pytest.mark.parametrize("m,n,k,bits,gs,method", MODEL_SHAPES)
 def test_quantized_matmul_baseline_shapes(ctx, m, n, k, bits, gs, method):
     """Full matrices on the GPU; the oracle (scalar C) checks a seeded sample of 2048 output rows -- restating the loop on a row subset is the
     same function on those rows."""
@@ -166,7 +166,7 @@ def test_matmul_invalid_arguments_are_sticky_errors(ctx):
 
 
 def test_matmul_linearity_full_size(ctx):
-    """Size-independent property at a BASELINE shape (Llama-3-8B up projection 28672 x 4096 int4):
+    """Size-independent property at a model's shape (Llama-3-8B up projection 28672 x 4096 int4):
     f32 outputs are linear in the activation, A(x1 + x2) == A x1 + A x2 up to f32 rounding, and the
     zero vector maps to exactly zero."""
     n, k = 28672, 4096
@@ -237,7 +237,7 @@ def test_attention_prepare_bit_exact(ctx):
 ATTN_CASES = [  # H, Hkv, seq, suffix, D, causal
     (4, 4, 16, 1, 64, False), (8, 2, 40, 4, 128, True), (4, 1, 64, 8, 64, True), (32, 8, 700, 1, 128, True),
     (8, 2, 1500, 1, 256, True), (64, 8, 300, 2, 128, True), (6, 2, 90, 3, 128, True), (3, 1, 50, 1, 64, True),
-    (32, 8, 2304, 1, 128, True),      # Llama-3-8B decode at the end of BASELINE config 3 (prefill 2048 + decode 256)
+    (32, 8, 2304, 1, 128, True),      # Llama-3-8B decode at the end of the benchmark (prefill 2048 + decode 256)
 ]
 
 
@@ -291,7 +291,7 @@ def test_gated_act_mul(ctx):
     rng = np.random.default_rng(15)
     up = f32_to_bf16(rng.standard_normal((3, 2 * 3584)).astype(np.float32) * 3)
     # SiLU: expf differs by <= 1 f32 ulp between CUDA and glibc. GELU: 1 + tanh / 1 + erf cancel for negative gates, so the
-    # libm difference is amplified before the bf16 rounding (transcendental parity is unpinned in the reference, SURVEY 8c)
+    # libm difference is amplified before the bf16 rounding (transcendental parity is unpinned in the reference)
     for act, min_exact in ((O.ACT_SILU, 0.995), (O.ACT_GELU_APPROX, 0.95), (O.ACT_GELU_EXACT, 0.95)):
         assert_bf16_close(G.gated_act_mul(ctx, up, 3584, act), O.gated_act_mul(up, 3584, act), max_ulp=1, min_exact=min_exact,
                           what=f"gated_act_mul act={act}")

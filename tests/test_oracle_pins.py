@@ -507,7 +507,7 @@ def test_sigmoid_gate_and_kv_cache_update_closed_forms():
     assert (keys == ek).all() and (values == ev).all()
 
 
-# ---- Mirai RHT (SURVEY 8f-3): ActivationTransform + the matmul's output-RHT epilogue ------------------------------------------
+# ---- Mirai RHT: ActivationTransform + the matmul's output-RHT epilogue ------------------------------------------
 
 def _rht_case(batch, channels):
     # the reference's own test inputs (tests/unit/backends/common/kernel/activation_transform_test.rs:64-76)

@@ -67,7 +67,7 @@ def test_int8_planes_are_exact_and_match_the_kernel_order():
 
 def test_single_plane_would_miss_the_parity_budget():
     """Why two planes: one rounded bf16 plane carries up to 2^-9 relative error per weight, i.e. ~1e-3 of a dot product's rms -- the
-    whole rtol the north_star allows."""
+    whole rtol the tests allow."""
     s, w, hi, lo, _ = _check(4)
     rel = np.abs(lo[w != 0] / w[w != 0])
     assert rel.max() > 1.5e-3 and rel.max() <= 2.0 ** -8

@@ -1,7 +1,7 @@
 """Parity of the quantised products of many rows on tcgen05 (uzu_b200/csrc/qmm_scaled.cu, reached through uzu_matmul_encode for m >= 64) against the
 CPU oracle's MatmulKernel restatement (backends/cpu/kernel/matmul/kernel.rs:164-295). Shapes: the reference's quant dispatch matrix
-(quant_dispatch_test.rs:102-167: bits x group x method) at prefill row counts, ragged m / n tails, and the BASELINE layer shapes
-through size-independent properties. Tolerance: BASELINE rtol 1e-3 / atol 1e-4 on f32 outputs, <= 1 bf16 ulp on bf16 outputs."""
+(quant_dispatch_test.rs:102-167: bits x group x method) at prefill row counts, ragged m / n tails, and the models' layer shapes
+through size-independent properties. Tolerance: rtol 1e-3 / atol 1e-4 on f32 outputs, <= 1 bf16 ulp on bf16 outputs."""
 import numpy as np
 import pytest
 
@@ -86,7 +86,7 @@ def test_prefill_gemm_rows_match_decode_gemv(ctx):
 
 
 def test_prefill_gemm_linearity_full_size(ctx):
-    """Size-independent properties at a BASELINE shape (Llama-3-8B qkv 6144 x 4096 int4, m = 512): zero rows map to exact zeros,
+    """Size-independent properties at a model's shape (Llama-3-8B qkv 6144 x 4096 int4, m = 512): zero rows map to exact zeros,
     A(x1 + x2) == A x1 + A x2, and a sample of outputs matches the oracle."""
     m, n, k = 512, 6144, 4096
     rng = np.random.default_rng(15)

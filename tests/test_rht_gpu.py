@@ -1,4 +1,4 @@
-"""Mirai RHT path on the GPU (SURVEY 8f-3): ActivationTransform (uzu_b200/csrc/activation_transform.cu), the matmul's output-RHT epilogue
+"""Mirai RHT path on the GPU: ActivationTransform (uzu_b200/csrc/activation_transform.cu), the matmul's output-RHT epilogue
 and a HybridSpec checkpoint through the engine, against the oracle (oracle_activation_transform, pinned by float64 twins in
 tests/test_oracle_pins.py). Reference: backends/cpu/kernel/activation_transform/*.rs, cpu/kernel/matmul/kernel.rs:297-303,
 encodable_block/linear/rht_wrapper.rs; shapes and inputs of tests/unit/backends/common/kernel/activation_transform_test.rs."""

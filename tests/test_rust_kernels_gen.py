@@ -1,4 +1,4 @@
-"""The generated kernel trait impls (integration/rust/backends/cuda/kernel/generated.rs, tools/gen_rust_kernels.py; SURVEY 8f-2) cannot be
+"""The generated kernel trait impls (integration/rust/backends/cuda/kernel/generated.rs, tools/gen_rust_kernels.py) cannot be
 compiled here (no rustc), so they are checked structurally: current with the kernel table + header, one impl per reference `#[kernel]`,
 every covered kernel's struct literal names exactly the fields of its C struct in header order, the C ABI registers every struct the Rust
 start-up check asks about, and -- when the reference checkout is present (build container only) -- the committed table is what

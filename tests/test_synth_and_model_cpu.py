@@ -36,7 +36,7 @@ def test_config_schema_matches_reference_structs(tmp_path):
 
 
 def test_bytes_per_token_formula():
-    # SURVEY.md 8(d): Llama-3-8B int4 gs64 zero-point = 4.046 GB of weights per decoded token
+    # Llama-3-8B int4 gs64 zero-point = 4.046 GB of weights per decoded token
     s = synth.llama3_8b()
     def mat(n, k, bits=4, gs=64):
         g = -(-k // gs)

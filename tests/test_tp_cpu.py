@@ -1,4 +1,4 @@
-"""Tensor-parallel sharding (uzu_b200/tp.py, SURVEY 8e) on CPU: the P-rank oracle (shards + all-reduce / all-gather hooks) against the
+"""Tensor-parallel sharding (uzu_b200/tp.py) on CPU: the P-rank oracle (shards + all-reduce / all-gather hooks) against the
 1-rank oracle on the same synthetic checkpoint. The reference has no tensor parallelism, so the unsharded model IS the oracle; the f32
 partial sums are added in a different order than the sequential k loop, hence bf16-ulp (not bit) agreement. One test runs the ranks as
 threads in lockstep, one as two real processes over torch.distributed gloo (the host-side path of `bench.py --tp 2`)."""
@@ -116,7 +116,7 @@ def test_two_rank_oracle_matches_unsharded(tmp_path, kind, quant):
 
 
 def test_eight_rank_oracle_with_llama3_head_geometry(tmp_path):
-    """BASELINE config 5's split (TP = 8) on a small model with Llama-3's head geometry ratios: 8 kv heads -> one per rank, q heads 4 per
+    """An eight-way split on a small model with Llama-3's head geometry ratios: 8 kv heads -> one per rank, q heads 4 per
     kv head, FFN columns and vocabulary in 8 slices, every K shard an even number of quantisation groups. The 8 rank oracles (threads,
     lockstep exchange) must reproduce the unsharded logits."""
     from uzu_b200.synth import LLAMA3_ROPE, ModelSpec
@@ -199,7 +199,7 @@ def test_nccl_is_resolved_at_run_time():
 @pytest.mark.parametrize("preset,kw,sizes", [("llama3-8b", dict(bits=4), (2, 4, 8)), ("llama3-8b", dict(bits=8), (2, 4, 8)),
                                               ("llama3-70b", dict(bits=4), (2, 4, 8))])
 def test_baseline_models_are_shardable_shape_only(preset, kw, sizes):
-    """Llama-3-8B / 70B (BASELINE configs 3-5) at TP 2 / 4 / 8: whole heads, whole groups, whole zero-point bytes on every rank --
+    """Llama-3-8B / 70B at TP 2 / 4 / 8: whole heads, whole groups, whole zero-point bytes on every rank --
     checked from config + quantisation specs alone (no 35 GB of weights needed)."""
     spec = synth.PRESETS[preset](layers=2, **kw)
     cfg = synth.build_config(spec)

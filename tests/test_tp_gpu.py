@@ -1,4 +1,4 @@
-"""Tensor-parallel path of the engine on the GPU (SURVEY 8e). With one GPU the whole TP data path except the NCCL calls is exercised
+"""Tensor-parallel path of the engine on the GPU. With one GPU the whole TP data path except the NCCL calls is exercised
 through a size-1 shard: row-parallel projections emit f32 partials that uzu_tp_all_reduce rounds to bf16 once, the readout goes through
 uzu_tp_all_gather. With >= 2 GPUs two ranks (one process per GPU, NCCL) run the sharded model against the unsharded oracle."""
 import ctypes as C

@@ -1,4 +1,4 @@
-"""Speculative (trie) decode on the GPU (SURVEY 8f-4): uzu_engine_trie_pass / uzu_engine_trie_accept against the oracle's speculation pass
+"""Speculative (trie) decode on the GPU: uzu_engine_trie_pass / uzu_engine_trie_accept against the oracle's speculation pass
 (oracle/model.py forward(trie=) + accept, itself checked against flat passes in tests/test_trie_cpu.py) and against the engine's own
 plain decode: whatever a proposer suggests, the verified output is what token-by-token decode produces
 (engine/language_model/stream/stream.rs:550-657, trie.rs:262-296, mixer/attention/state.rs:174-237, mask.rs:21-29)."""

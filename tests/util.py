@@ -24,7 +24,7 @@ def bf16_ulp_distance(a_bits, b_bits):
 def assert_bf16_close(got_bits, ref_bits, *, max_ulp=1, min_exact=0.97, atol=1e-4, what=""):
     """bf16 outputs of a kernel whose f32 summation order differs from the oracle's:
     every element within `max_ulp` bf16 steps of the oracle (or within atol in value), and at least
-    `min_exact` of them bit-identical. BASELINE's rtol=1e-3 is below bf16's own 2^-8 rounding step, so it is
+    `min_exact` of them bit-identical. An rtol of 1e-3 is below bf16's own 2^-8 rounding step, so it is
     asserted on f32 outputs (see assert_f32_close) and as this ulp bound on bf16 ones."""
     got_bits, ref_bits = np.asarray(got_bits), np.asarray(ref_bits)
     assert got_bits.shape == ref_bits.shape, (got_bits.shape, ref_bits.shape)
@@ -39,7 +39,7 @@ def assert_bf16_close(got_bits, ref_bits, *, max_ulp=1, min_exact=0.97, atol=1e-
 
 
 def assert_f32_close(got, ref, *, rtol=1e-3, atol=1e-4, what=""):
-    """BASELINE tolerance (rtol 1e-3 / atol 1e-4) on f32 outputs. atol is taken relative to the output scale
+    """The tolerance (rtol 1e-3 / atol 1e-4) on f32 outputs. atol is taken relative to the output scale
     (rms of the reference, floor 1): an absolute 1e-4 on outputs of magnitude 100 would be 1e-6 relative, below the
     f32 accumulation noise of the *reference's own* 2048-term sequential sum."""
     got, ref = np.asarray(got, dtype=np.float32), np.asarray(ref, dtype=np.float32)

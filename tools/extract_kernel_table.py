@@ -2,7 +2,7 @@
 """Extract the kernel declaration table the reference's build scripts walk (build/cpu/compiler.rs:176-330: every `#[kernel(Name)]` fn under
 src/backends/cpu/kernel/**, its `#[variants]` generics, its arguments with `#[optional(..)]` / `#[specialize]`) into
 integration/rust/kernel_table.json, so that tools/gen_rust_kernels.py can emit the `impl <Name>Kernel for Cuda<Name>Kernel` blocks
- on a machine that has neither the reference checkout nor a Rust toolchain.
+on a machine that has neither the reference checkout nor a Rust toolchain.
 
     python tools/extract_kernel_table.py [/root/reference]
 

@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Generate integration/rust/backends/cuda/kernel/generated.rs: one `impl <Name>Kernel for Cuda<Name>Kernel` per `#[kernel]` of the
-reference (SURVEY 8f-2) -- what a `build/cuda/compiler.rs` arm would emit next to build/cpu/compiler.rs:176-613.
+reference -- what a `build/cuda/compiler.rs` arm would emit next to build/cpu/compiler.rs:176-613.
 
 Inputs: integration/rust/kernel_table.json (the declaration table, tools/extract_kernel_table.py) and include/uzu_b200.h (the C ABI).
 For the kernels this backend implements, `new` stores the generics / `#[specialize]` block and `encode` fills `uzu_<name>_args` (or the
@@ -143,7 +143,7 @@ def gen_kernel(k, cfg, structs, funcs) -> list[str]:
                 f"impl {name}Kernel for {sname} {{", "    type Backend = Cuda;",
                 "    #[allow(non_snake_case, unused_variables, clippy::too_many_arguments)]",
                 f"    fn new({new_sig}) -> Result<Self, CudaError> {{",
-                f"        Err(CudaError::NotSupported(\"{name}: outside the CUDA decode hot path (SURVEY 8 scope)\"))", "    }",
+                f"        Err(CudaError::NotSupported(\"{name}: outside the CUDA decode hot path\"))", "    }",
                 "    #[allow(unused_variables, clippy::too_many_arguments)]",
                 f"    fn encode<{', '.join(lifetimes)}>(&self, {enc_sig}) {{",
                 f"        unreachable!(\"{sname} cannot be constructed\")", "    }", "}", ""]

@@ -1,4 +1,4 @@
-"""Print the handful of ncu metrics used in DESIGN.md / profiles/ from a .ncu-rep (first kernel): python tools/ncu_brief.py file.ncu-rep"""
+"""Print the handful of ncu metrics that the notes and profiles/ use from a .ncu-rep (first kernel): python tools/ncu_brief.py file.ncu-rep"""
 import csv, subprocess, sys, io
 raw = subprocess.run(["ncu", "-i", sys.argv[1], "--page", "raw", "--csv"], capture_output=True, text=True).stdout
 r = list(csv.reader(io.StringIO(raw)))

@@ -1,6 +1,6 @@
 """ctypes binding of libuzu_b200.so (include/uzu_b200.h) for tests and bench.py.
 
-This is the kind of stub a host-language binding adds (INTEGRATION.md): structs mirrored field for field
+This is the kind of stub a host-language binding adds: structs mirrored field for field
 (verified at import against uzu_abi_struct_size), opaque handles, status codes turned into exceptions.
 There is no fallback: a missing library raises at load(), a missing GPU raises at Context().
 """

@@ -1,4 +1,4 @@
-// ActivationTransformKernel (Mirai RHT, SURVEY 8f-3): crates/backend-uzu/src/backends/cpu/kernel/activation_transform/
+// ActivationTransformKernel (Mirai RHT): crates/backend-uzu/src/backends/cpu/kernel/activation_transform/
 // {activation_transform.rs:44-136, mod.rs:9-44}; callers encodable_block/linear/rht_wrapper.rs:214-297 (input RHT of a HybridSpec linear)
 // and the matmul's output-RHT epilogue (cpu/kernel/matmul/kernel.rs:297-303, matmul.cu: UZU_D_RHT).
 //

@@ -239,7 +239,7 @@ __device__ __forceinline__ uint32_t mk_range_of(uint64_t u, uint64_t U, uint64_t
 // Two-level partition of a phase with U units. Level 1: the units are cut into geff = min(gridDim, U) equal contiguous CTA ranges
 // (boundaries floor(c * U / geff)): every SM pulls the same number of bytes. Level 2: a CTA's range is cut into min(NCW, length) equal
 // contiguous warp ranges. Contiguous warps of ONE CTA therefore share the tiles that straddle warp boundaries: their partial sums meet in
-// shared memory (fixed warp order) and a tile leaves one piece per CTA that touches it -- at most two for every BASELINE shape -- instead
+// shared memory (fixed warp order) and a tile leaves one piece per CTA that touches it -- at most two for every matrix of the measured models -- instead
 // of one per warp (the first version: up to ten pieces per tile, i.e. ten dependent L2 round trips in the consumer's staging).
 __device__ __forceinline__ void mk_my_range(uint32_t cta, uint32_t warp, uint32_t ncw, uint32_t U, uint32_t& geff, uint32_t& ub, uint32_t& ue) {
     geff = min(gridDim.x, U);

@@ -1,8 +1,8 @@
-// DeltaNet decode kernels for Qwen3.5 hybrid layers (SURVEY.md 8(f)-1):
+// DeltaNet decode kernels for Qwen3.5 hybrid layers:
 //   DeltaNetConvUpdate  backends/cpu/kernel/gdn/conv_update.rs:8-55   (1-token causal conv + SiLU, f32 rolling state)
 //   DeltaNetUpdate      backends/cpu/kernel/gdn/update.rs:13-144      (gated delta rule over S[Hv, Dv, Dk] + RMSNorm * SiLU(z))
 // Parameter / state dtypes are f32 (what the engine allocates and Metal declares; the reference CPU
-// kernel's `*const T` typing of these buffers is the bug documented in SURVEY.md row a11).
+// kernel's `*const T` typing of these buffers does not fit what is allocated).
 // State traffic: Hv*Dv*Dk*4 B read + written per layer per token (2 MB for Qwen3.5-0.8B).
 #include "common.cuh"
 

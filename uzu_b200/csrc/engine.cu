@@ -851,7 +851,7 @@ static RopeCfg parse_rope(const Json& j) {
         r.original_context_length = j.at("original_context_length").u32();
         r.low = (float)j.at("low_frequency_factor").number();
         r.high = (float)j.at("high_frequency_factor").number();
-    } else throw std::runtime_error("unsupported RoPE config " + ty + " (YaRN / LongRoPE are outside the BASELINE configs)");
+    } else throw std::runtime_error("unsupported RoPE config " + ty + " (YaRN / LongRoPE are not built)");
     return r;
 }
 
@@ -960,7 +960,7 @@ static void load_language_model_config(uzu_engine* e, const Json& cfg, const std
     e->hidden_dim = tr.at("hidden_dim").u32();
     e->vocab = dec.at("vocab_size").u32();
     if (!dec.at("ple_model_config").is_null() || !dec.at("embedding_norm_config").is_null())
-        throw std::runtime_error("PLE / embedding norm are outside this backend's scope (SURVEY 2.1)");
+        throw std::runtime_error("PLE / embedding norm are outside this backend's scope");
     ParameterLoader pl(dir + "/model.safetensors");
     const uint32_t H = e->model_dim, V = e->vocab;
     // tensor-parallel shard (uzu_b200/tp.py): narrower heads / hidden_dim come from the shard's own config; the block says which rank
@@ -1079,7 +1079,7 @@ static void load_language_model_config(uzu_engine* e, const Json& cfg, const std
             stb += 2ull * D.num_heads * D.value_head_dim * D.head_dim * 4;
             n_dn++;
         } else {
-            throw std::runtime_error("mixer " + mty + " is outside this backend's scope (SURVEY 2.1)");
+            throw std::runtime_error("mixer " + mty + " is outside this backend's scope");
         }
         const Json& mlp = lc.at("mlp_config");
         if (mlp.type_tag() != "DenseMLPConfig") throw std::runtime_error("only DenseMLPConfig is supported");
@@ -2712,7 +2712,7 @@ uzu_status uzu_engine_forward(uzu_engine* e, const uint32_t* tokens, uint32_t co
 }
 
 
-// ---- speculation pass over a trie (SURVEY 8f-4): the verify half of the stream's speculative decode (stream.rs:550-657) ----
+// ---- speculation pass over a trie: the verify half of the stream's speculative decode (stream.rs:550-657) ----
 // The proposer (a draft model / n-gram lookup) and the trie bookkeeping (trie.rs: linearize, accept) stay on the host side of the boundary;
 // the backend runs Decoder::encode over the linearized nodes (positions = context + height, attention masked by subtrie range, one sampled
 // token per node) and later compacts the KV rows of the accepted path (TransformerState::encode_accept).

@@ -1,4 +1,4 @@
-// Tensor-parallel exchange steps (SURVEY 8e; extension -- the reference is single-device): one process per GPU, NCCL over NVLink.
+// Tensor-parallel exchange steps (extension -- the reference is single-device): one process per GPU, NCCL over NVLink.
 //
 //   uzu_tp_all_reduce_encode : f32 partial sums [count] of a row-parallel projection (out / down) are summed over the ranks with
 //                              ncclAllReduce on the context's stream, then rounded to bf16 ONCE (the unsharded kernel's single

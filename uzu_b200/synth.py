@@ -1,8 +1,8 @@
 """Synthetic uzu-format checkpoints (config.json + model.safetensors) for tests and benchmarks.
 
 There is no network in the build/bench environment, so real checkpoints cannot be fetched; this
-module emits seeded random weights in exactly the on-disk layout the reference engine loads
-(SURVEY.md Appendix A): config.json follows crates/backend-uzu/src/config/** (abstract-config
+module emits seeded random weights in exactly the on-disk layout the reference engine loads:
+config.json follows crates/backend-uzu/src/config/** (abstract-config
 variants carry a "type" tag, every Option field is present as null), tensor keys follow
 encodable_block/{embedding,transformer_layer,mixer/attention/mod,mixer/delta_net,mlp/mod}.rs and
 per-matrix quantisation specs are JSON strings under `<prefix>.spec` in the safetensors
@@ -33,7 +33,7 @@ class QuantSpec:
     bits: int = 4
     group_size: int = 64
     symmetric: bool = False    # IntSpec.is_symmetric
-    rht: bool = False          # HybridSpec: 32-wide input/output randomized Hadamard around this quantization (Mirai RHT, SURVEY 8f-3)
+    rht: bool = False          # HybridSpec: 32-wide input/output randomized Hadamard around this quantization (Mirai RHT)
 
     def spec_json(self, layout: str) -> dict:
         if self.rht:
@@ -257,7 +257,7 @@ def write_model(spec: ModelSpec, path, seed: int = 0) -> Path:
 
 
 # ---------------------------------------------------------------------------------------------
-# presets
+# presets of the measured models
 # ---------------------------------------------------------------------------------------------
 LLAMA3_ROPE = {"type": "LlamaRoPEConfig", "base": 500000.0, "max_sequence_length": 8192, "head_dim": 128,
                "scaling_factor": 8.0, "original_context_length": 8192, "low_frequency_factor": 1.0,

@@ -1,4 +1,4 @@
-"""Tensor-parallel sharding of a uzu-format checkpoint (SURVEY.md 8e; nothing in the reference to mirror: uzu is single-device).
+"""Tensor-parallel sharding of a uzu-format checkpoint (nothing in the reference to mirror: uzu is single-device).
 
 `shard_checkpoint(model_dir, out_dir, rank, size)` writes the checkpoint rank `rank` of `size` loads: an ordinary uzu checkpoint of a
 *narrower* model (num_heads / num_groups / hidden_dim divided by `size`, model_dim unchanged) plus a `"tensor_parallel"` block in
@@ -13,8 +13,8 @@ config.json that tells the engine where the exchange steps are:
     scale and the RoPE tables are replicated. A tied embedding is untied in the shard (full table for the lookup + its row slice).
 
 Quantisation groups run along K, so K shards must be whole groups (and whole zero-point bytes for 4-bit): checked here.
-The KV cache of a rank holds its Hkv/P heads only; attention is rank-local. DeltaNet layers are not sharded (the BASELINE config
-that needs TP, Llama-3-70B, has none): such checkpoints are rejected.
+The KV cache of a rank holds its Hkv/P heads only; attention is rank-local. DeltaNet layers are not sharded (Llama-3-70B,
+the model that needs them cut, has none): such checkpoints are rejected.
 """
 from __future__ import annotations
 
