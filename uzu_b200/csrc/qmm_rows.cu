@@ -38,7 +38,7 @@ struct QrParams {
     uint32_t m, n, k, row_bytes, groups, zp_stride, xor_mask;
     uint32_t steps, slice_steps, slices, tiles, whole;      // steps of k: all, of a slice; whole: tiles are not shared by warps
     uint32_t d_is_f32, accumulate, has_soft_cap;
-    float ab_scale, soft_cap;
+    float ab_scale, soft_cap;        // ab_scale brings the integers' factor back
 };
 
 namespace {
@@ -48,7 +48,7 @@ constexpr int QR_WARPS = 12, QR_STAGES = 2;
 template <int BITS>
 struct QrShape {
     static constexpr uint32_t CODES = BITS == 4 ? 512 : 256, PITCH = BITS == 4 ? 288 : 320, STAGE = 16 * PITCH + 512;
-    static constexpr float DOWN = BITS == 4 ? 1.0f / 2048.0f : 1.0f / 32768.0f, UP = 1.0f / DOWN;            // the integers' factor
+    static constexpr float DOWN = BITS == 4 ? 1.0f / 2048.0f : 1.0f / 32768.0f;                              // the integers' factor
     static constexpr uint32_t MAGIC = BITS == 4 ? 0x3D803D80u : 0x3B803B80u;                                 // bf16 128 DOWN, twice
 };
 
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(QR_WARPS * 32, 1) qmm_rows_kernel(const QrPara
                 const uint32_t o = lane + 32u * i, row = (uint32_t)c * 8u + o / 16u, feature = tile * 16u + o % 16u;
                 if (row >= p.m || feature >= p.n) continue;
                 const size_t idx = (size_t)row * p.n + feature;
-                float v = p.ab_scale * (S::UP * turn[o]);
+                float v = p.ab_scale * turn[o];
                 if (p.accumulate) v += p.d_is_f32 ? reinterpret_cast<const float*>(p.d)[idx] : __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p.d)[idx]);
                 if (p.bias) v += __bfloat162float(p.bias[feature]);
                 if (p.has_soft_cap) v = p.soft_cap * tanhf(v / p.soft_cap);
@@ -447,7 +447,7 @@ void encode_qmm_rows(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
         p.d_is_f32 = a.output_dt == UZU_DT_F32;
         p.accumulate = (a.d_transform & UZU_D_ACCUMULATE) != 0;
         p.has_soft_cap = (a.d_transform & UZU_D_SOFT_CAP) != 0;
-        p.ab_scale = (a.d_transform & UZU_D_SCALE) ? a.ab_scale : 1.0f;
+        p.ab_scale = ((a.d_transform & UZU_D_SCALE) ? a.ab_scale : 1.0f) / (bits == 4 ? QrShape<4>::DOWN : QrShape<8>::DOWN);
         p.soft_cap = a.soft_cap;
         const uint32_t grid = std::min(p.tiles, (uint32_t)cmd->ctx->sm_count / p.slices) * p.slices;
         if (bits == 4) a.b_group_size == 64 ? qr_method<4, 64>(cmd, p, a.b_prologue, grid, plan.smem) : qr_method<4, 128>(cmd, p, a.b_prologue, grid, plan.smem);
