@@ -33,3 +33,12 @@ def _kernels():
 @pytest.mark.parametrize("body,ordered", list(_kernels()))
 def test_kernel_waits_for_its_predecessor(body, ordered):
     assert ordered or "pdl_wait();" in body or "griddepcontrol.wait" in body
+
+
+def test_copies_and_fills_are_ordered_with_the_contexts_stream():
+    """The stream of a context does not wait for the legacy stream. A fill or a copy on the device that goes to the latter returns before it is done, so that a kernel
+    launched next may not see it."""
+    for path in sorted(CSRC.iterdir()):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        assert not re.search(r"\bcudaMemset\s*\(", text), path.name
+        assert not re.search(r"\bcudaMemcpy\s*\([^;]*cudaMemcpyDeviceToDevice", text), path.name

@@ -2556,6 +2556,7 @@ uzu_status uzu_engine_create(uzu_context* ctx, const char* model_dir, const uzu_
         cudaSetDevice(ctx->device);
         load_model(e, model_dir);
         create_state_and_scratch(e);
+        cudaStreamSynchronize(cudaStreamLegacy);     // uploads from pageable memory may still be on their way; the engine's stream does not wait for them
         reset_state(e);
         e->fused_ok = !e->parallel_block && e->opts.fused_decode && getenv("UZU_NO_FUSED") == nullptr && fused_decode_supported(e);
         if (e->parallel_block) e->mega.why = "the persistent decode kernel does not cover the parallel-block family";
@@ -2655,7 +2656,7 @@ uzu_status uzu_engine_prefill(uzu_engine* e, const uint32_t* tokens, uint32_t co
         uint32_t tok = 0;
         cudaMemcpy(&tok, (void*)e->sampled.ptr(), 4, cudaMemcpyDeviceToHost);
         // the sampled token becomes the next input, chained on the device
-        cudaMemcpy((void*)e->token_ids.ptr(), (void*)e->sampled.ptr(), 4, cudaMemcpyDeviceToDevice);
+        cudaMemcpyAsync((void*)e->token_ids.ptr(), (void*)e->sampled.ptr(), 4, cudaMemcpyDeviceToDevice, e->ctx->stream);
         e->steps_issued = e->steps_returned = 0;
         upload_decode_state(e);
         if (out_token) *out_token = tok;
@@ -2820,7 +2821,7 @@ uzu_status uzu_engine_set_decode_mode(uzu_engine* e, int persistent) {
         else if (!e->mega.ok) {
             if (e->mega.ops.empty() || !e->mega.ops_dev.b) throw std::runtime_error("persistent decode kernel not available: " + e->mega.why);
             *(volatile unsigned int*)uzu_buffer_cpu_ptr(e->mega.error_flag.b) = 0u;
-            cudaMemset((void*)e->mega.barrier.ptr(), 0, 256);
+            cudaMemsetAsync((void*)e->mega.barrier.ptr(), 0, 256, e->ctx->stream);
             e->mega.barrier_base = 0;
             e->mega.ok = true;
         }

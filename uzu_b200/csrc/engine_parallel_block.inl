@@ -1366,7 +1366,7 @@ static void create_parallel_block_scratch(uzu_engine* e) {
     P.pair_weight_compact = dev(R * top * 4);
     P.route_scratch = dev(R * top * 2);
     P.attn_tickets = dev((size_t)kSplitRows * tickets * 4);
-    cudaMemset((void*)P.attn_tickets.ptr(), 0, (size_t)kSplitRows * tickets * 4);
+    cudaMemsetAsync((void*)P.attn_tickets.ptr(), 0, (size_t)kSplitRows * tickets * 4, e->ctx->stream);
     P.operand_bf16 = dev(R * kmax * 2);     // bf16 copy of a prompt pass's activation rows for the tensor-memory products
     P.proj = dev(R * proj * 4);
     P.lat = dev(R * lat * 4);

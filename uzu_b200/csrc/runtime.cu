@@ -141,16 +141,16 @@ uzu_status uzu_context_create(int device_ordinal, uzu_context** out) {
     ctx->splitk_counter_count = 1u << 16;
     UZU_CUDA_TRY(cudaMalloc(&ctx->splitk_ws, ctx->splitk_ws_bytes));
     UZU_CUDA_TRY(cudaMalloc(&ctx->splitk_counters, ctx->splitk_counter_count * sizeof(unsigned int)));
-    UZU_CUDA_TRY(cudaMemset(ctx->splitk_counters, 0, ctx->splitk_counter_count * sizeof(unsigned int)));
+    UZU_CUDA_TRY(cudaMemsetAsync(ctx->splitk_counters, 0, ctx->splitk_counter_count * sizeof(unsigned int), ctx->stream));
     ctx->attn_ws_bytes = 8u << 20;
     UZU_CUDA_TRY(cudaMalloc(&ctx->attn_ws, ctx->attn_ws_bytes));
     UZU_CUDA_TRY(cudaMalloc(&ctx->attn_counters, 65536 * sizeof(unsigned int)));
-    UZU_CUDA_TRY(cudaMemset(ctx->attn_counters, 0, 65536 * sizeof(unsigned int)));
+    UZU_CUDA_TRY(cudaMemsetAsync(ctx->attn_counters, 0, 65536 * sizeof(unsigned int), ctx->stream));
     UZU_CUDA_TRY(cudaHostAlloc((void**)&ctx->wait_errors.word, sizeof(unsigned int), cudaHostAllocMapped | cudaHostAllocPortable));
     *ctx->wait_errors.word = 0;
     UZU_CUDA_TRY(cudaHostGetDevicePointer((void**)&ctx->wait_errors.device_word, ctx->wait_errors.word, 0));
     UZU_CUDA_TRY(cudaMalloc(&ctx->sampling_ws, 64 * 1024));
-    UZU_CUDA_TRY(cudaMemset(ctx->sampling_ws, 0, 64 * 1024));
+    UZU_CUDA_TRY(cudaMemsetAsync(ctx->sampling_ws, 0, 64 * 1024, ctx->stream));
     // VMM support (SparseBuffer)
     int vmm = 0;
     CUdevice cu_dev;

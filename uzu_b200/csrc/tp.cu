@@ -259,7 +259,8 @@ uzu_status uzu_tp_p2p_export(uzu_context* ctx, uint32_t capacity_f32, uint8_t* h
     const size_t bytes = tp_p2p_bytes(ctx->tp_size, capacity_f32);
     cudaError_t e = cudaMalloc(&st->local, bytes);
     if (e != cudaSuccess) { delete st; return fail(UZU_ERROR_OUT_OF_MEMORY, std::string("tp_p2p_export: ") + cudaGetErrorString(e)); }
-    cudaMemset(st->local, 0, bytes);
+    cudaMemsetAsync(st->local, 0, bytes, ctx->stream);
+    cudaStreamSynchronize(ctx->stream);              // no peer learns of it before it is zero
     cudaIpcMemHandle_t h;
     e = cudaIpcGetMemHandle(&h, st->local);
     if (e != cudaSuccess) { cudaFree(st->local); delete st; return fail(UZU_ERROR_CUDA, std::string("cudaIpcGetMemHandle: ") + cudaGetErrorString(e)); }
