@@ -314,7 +314,8 @@ typedef struct uzu_attention_args {
     uint32_t head_dim;             /* HEAD_DIM variant: 64 | 128 | 256 */
     uint32_t has_sinks, is_kv_cache_ring, is_causal, is_trie, is_sliding_window;
     /* Extension for CUDA-graph replay (0 = reference semantics): device u32* holding the prefix length P; when set,
-     * sequence_length is read as P + suffix_length and `sequence_length` is only a sizing hint for the KV split. */
+     * sequence_length is read as P + suffix_length and `sequence_length` is the most it may be: the keys are cut by the length that is
+     * found, into no more parts than that most allows (a smaller one costs time, not keys). */
     uint64_t dynamic_position;
 } uzu_attention_args;
 UZU_API void uzu_attention_single_pass_encode(uzu_command_buffer* cmd, const uzu_attention_args* args);
