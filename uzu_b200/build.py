@@ -38,6 +38,7 @@ SOURCES = {
     "deltanet.cu": ["-fmad=false"],
     "deltanet_prefill.cu": ["-fmad=false"],
     "decode_mega.cu": [],
+    "decode_linear.cu": [],
     "dense_linear.cu": [],
     "dense_umma.cu": [],
     "residual_f32.cu": [],

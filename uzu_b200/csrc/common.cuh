@@ -110,6 +110,12 @@ void encode_qmm_rows(uzu_command_buffer* cmd, const uzu_matmul_args& a);
 // quantised products of two and more rows on tcgen05 (qmm_scaled.cu), dispatched from encode_matmul
 bool qmm_scaled_applicable(const uzu_matmul_args& a);
 void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a);
+// one row times a matrix in the decode-stream layout (decode_linear.cu), for calls that uzu_fused_linear_supported accepts
+bool decode_linear_applicable(const uzu_fused_linear_args& f);
+void encode_decode_linear(uzu_command_buffer* cmd, const uzu_fused_linear_args& f);
+// uzu_fused_linear_supported / _encode, 8-bit weights with a decode stream as well
+bool fused_linear_supported(uzu_context* ctx, const uzu_fused_linear_args* args);
+void encode_fused_linear(uzu_command_buffer* cmd, const uzu_fused_linear_args* args);
 // fails with the code of a barrier wait that ran out (0: UZU_OK)
 uzu_status wait_error_status(unsigned int code);
 

@@ -1684,30 +1684,41 @@ static bool any_rht(const uzu_engine* e) {
     return e->out_emb.rht();
 }
 
+static void encode_fused(uzu_command_buffer* cmd, const uzu_fused_linear_args& f) {
+    if (!encodable(cmd, "fused_linear")) return;
+    if (fused_linear_supported(cmd->ctx, &f)) encode_fused_linear(cmd, &f);
+    else cmd->record_error(UZU_ERROR_UNSUPPORTED, "fused_linear: shape / format not covered by the fused decode kernel");
+}
+
+// (8-bit weights only where every fused linear has its decode-stream copy)
 static bool fused_decode_supported(uzu_engine* e) {
     const uint32_t mask = fuse_mask();
     if (any_rht(e)) return false;   // RHT linears take the unfused sequence (input transform, GEMV, output transform)
     for (auto& L : e->layers) {
         if (L.pre_mixer.cfg.subtract_mean || L.pre_mlp.cfg.subtract_mean || !L.pre_mixer.cfg.has_scale || !L.pre_mlp.cfg.has_scale) return false;
         std::vector<uzu_fused_linear_args> fs;
+        auto add = [&](uzu_fused_linear_args f, const Linear& l) {
+            f.decode_stream = g_stream_lookup(e->mega.stream_of, l);
+            fs.push_back(f);
+        };
         const uint64_t x = e->hidden_a.ptr(), s0 = e->shortcut.ptr(), s1 = e->shortcut2.ptr();
         if (mask & 1u) {
             if (L.is_attention) {
-                if (L.attn.has_gate) fs.push_back(fused_norm_args(L.attn.gate, L.pre_mixer, x, s0, s1, true, e->gate.ptr()));
-                fs.push_back(fused_norm_args(L.attn.qkv, L.pre_mixer, x, s0, s1, true, e->qkv.ptr()));
+                if (L.attn.has_gate) add(fused_norm_args(L.attn.gate, L.pre_mixer, x, s0, s1, true, e->gate.ptr()), L.attn.gate);
+                add(fused_norm_args(L.attn.qkv, L.pre_mixer, x, s0, s1, true, e->qkv.ptr()), L.attn.qkv);
             } else {
-                fs.push_back(fused_norm_args(L.dn.in_proj, L.pre_mixer, x, s0, s1, true, e->in_proj.ptr()));
+                add(fused_norm_args(L.dn.in_proj, L.pre_mixer, x, s0, s1, true, e->in_proj.ptr()), L.dn.in_proj);
             }
         }
         if (L.is_attention && L.attn.has_gate && (mask & 4u)) {
             uzu_fused_linear_args g{};
             g.matmul = linear_args(L.attn.out, 0, 1, e->mixer_out.ptr());
             g.prologue = 3; g.sg_attn = e->attn_out.ptr(); g.sg_gate = e->gate.ptr();
-            fs.push_back(g);
+            add(g, L.attn.out);
         }
-        if (mask & 3u) fs.push_back(fused_up_args(e, L, (mask & 1u) != 0, s0, s1));
+        if (mask & 3u) add(fused_up_args(e, L, (mask & 1u) != 0, s0, s1), L.up);
         for (auto& f : fs)
-            if (!uzu_fused_linear_supported(e->ctx, &f)) return false;
+            if (!fused_linear_supported(e->ctx, &f)) return false;
     }
     return true;
 }
@@ -1719,8 +1730,8 @@ static void encode_decode_gemv(uzu_engine* e, uzu_command_buffer* cmd, const Lin
         uzu_fused_linear_args f{};
         f.matmul = linear_args(lin, x, 1, d);
         f.decode_stream = stream;
-        if (uzu_fused_linear_supported(e->ctx, &f)) {
-            uzu_fused_linear_encode(cmd, &f);
+        if (fused_linear_supported(e->ctx, &f)) {
+            encode_fused(cmd, f);
             return;
         }
     }
@@ -1759,7 +1770,7 @@ static void encode_decoder_fused(uzu_engine* e, uzu_command_buffer* cmd, const P
             if (fuse_norm) {
                 auto f = fused_norm_args(lin, L.pre_mixer, e->hidden_a.ptr(), S[cur], wrote ? 0 : S[cur ^ 1], add, d);
                 f.decode_stream = g_stream_lookup(e->mega.stream_of, lin);
-                uzu_fused_linear_encode(cmd, &f);
+                encode_fused(cmd, f);
                 wrote = true;
             } else {
                 encode_linear(cmd, lin, e->hidden_b.ptr(), 1, d);
@@ -1819,7 +1830,7 @@ static void encode_decoder_fused(uzu_engine* e, uzu_command_buffer* cmd, const P
                 g.matmul = linear_args(A.out, 0, 1, e->mixer_out.ptr());
                 g.prologue = 3; g.sg_attn = e->attn_out.ptr(); g.sg_gate = e->gate.ptr();
                 g.decode_stream = g_stream_lookup(e->mega.stream_of, A.out);
-                uzu_fused_linear_encode(cmd, &g);
+                encode_fused(cmd, g);
             } else {
                 if (A.has_gate) uzu_sigmoid_gate_encode(cmd, e->gate.ptr(), e->attn_out.ptr(), Hq * D);
                 encode_decode_gemv(e, cmd, A.out, e->attn_out.ptr(), e->mixer_out.ptr());
@@ -1850,7 +1861,7 @@ static void encode_decoder_fused(uzu_engine* e, uzu_command_buffer* cmd, const P
         if (fuse_norm || fuse_gated) {
             auto fu = fused_up_args(e, L, fuse_norm, S[cur], S[cur ^ 1]);
             fu.decode_stream = g_stream_lookup(e->mega.stream_of, L.up);
-            uzu_fused_linear_encode(cmd, &fu);
+            encode_fused(cmd, fu);
         } else {
             encode_linear(cmd, L.up, e->hidden_b.ptr(), 1, e->fused_up.ptr());
         }
@@ -2558,10 +2569,10 @@ uzu_status uzu_engine_create(uzu_context* ctx, const char* model_dir, const uzu_
         create_state_and_scratch(e);
         cudaStreamSynchronize(cudaStreamLegacy);     // uploads from pageable memory may still be on their way; the engine's stream does not wait for them
         reset_state(e);
-        e->fused_ok = !e->parallel_block && e->opts.fused_decode && getenv("UZU_NO_FUSED") == nullptr && fused_decode_supported(e);
         if (e->parallel_block) e->mega.why = "the persistent decode kernel does not cover the parallel-block family";
         if (e->opts.fused_decode && !e->parallel_block) {                   // the persistent decode kernel is the fused path's next step: one launch per token
             build_mega(e);
+            e->fused_ok = getenv("UZU_NO_FUSED") == nullptr && fused_decode_supported(e);
             calibrate_decode_path(e);
         }
         check(uzu_context_synchronize(ctx));
@@ -3356,7 +3367,7 @@ uzu_status uzu_engine_time_linears_select(uzu_engine* e, uint32_t iters, uint32_
                     f.matmul = linear_args(L.up, e->hidden_b.ptr(), 1, e->gated.ptr());
                     f.epilogue = 1; f.act_type = L.act;
                     f.decode_stream = g_stream_lookup(e->mega.stream_of, L.up);
-                    uzu_fused_linear_encode(g.c, &f);
+                    encode_fused(g.c, f);
                 }
                 if (select & 8u) encode_decode_gemv(e, g.c, L.down, e->gated.ptr(), e->hidden_a.ptr());
                 if ((select & 64u) && L.is_attention) {     // attention mix at the current context (rewrites the same KV row each time)
