@@ -66,11 +66,8 @@ __global__ void __launch_bounds__(256) attention_prepare_kernel(const uzu_attent
 }
 
 // Eight neighbouring channels of a (token, head) per thread, 16-byte accesses; the same arithmetic (1024 tokens x 48 heads of 128: 9.5 us, 53 a
-// channel at a time with a CTA per token and head). SEQS: row b belongs to sequence b, with its own cache, position and query row.
-struct NoSequences {};
-template <bool SEQS>
-__global__ void __launch_bounds__(256) attention_prepare_vec_kernel(const uzu_attention_prepare_args a,
-                                                                    const __grid_constant__ std::conditional_t<SEQS, AttnSequences, NoSequences> seqs) {
+// channel at a time with a CTA per token and head).
+__global__ void __launch_bounds__(256) attention_prepare_vec_kernel(const uzu_attention_prepare_args a) {
     pdl_launch_dependents();
     pdl_wait();
     const uint32_t total_heads = a.has_kv ? a.num_q_heads + 2 * a.num_kv_heads : a.num_q_heads, chunks = a.head_dim / 8u;
@@ -80,19 +77,11 @@ __global__ void __launch_bounds__(256) attention_prepare_vec_kernel(const uzu_at
     const __nv_bfloat16* head = reinterpret_cast<const __nv_bfloat16*>(a.qkv) + ((size_t)b * total_heads + h) * a.head_dim;
     const bool is_query = !a.has_kv || h < a.num_q_heads, is_key = a.has_kv && h >= a.num_q_heads && h < a.num_q_heads + a.num_kv_heads;
     uint32_t row = a.kv_token_offset, rope_row = b;
-    uint64_t keys = a.keys, values = a.values;
-    if constexpr (SEQS) {
-        row = a.dynamic_position ? reinterpret_cast<const uint32_t*>(a.dynamic_position)[b] : seqs.prefix[b];
-        rope_row = a.dynamic_position ? row : seqs.position[b];
-        keys = seqs.keys[b];
-        values = seqs.values[b];
-    } else {
-        if (a.dynamic_position) {
-            row = *reinterpret_cast<const uint32_t*>(a.dynamic_position);
-            rope_row += row;
-        }
-        row += b;
+    if (a.dynamic_position) {
+        row = *reinterpret_cast<const uint32_t*>(a.dynamic_position);
+        rope_row += row;
     }
+    row += b;
     uint4 v = *reinterpret_cast<const uint4*>(head + d);
     if (a.has_rope && d < a.rope_dim && (is_query || is_key)) {
         const uint32_t half = a.rope_dim / 2;                       // (a multiple of 8: a chunk lies in one half)
@@ -115,9 +104,9 @@ __global__ void __launch_bounds__(256) attention_prepare_vec_kernel(const uzu_at
         }
     }
     __nv_bfloat16* dst;
-    if (is_query) dst = reinterpret_cast<__nv_bfloat16*>(a.queries) + (SEQS ? (size_t)b * a.num_q_heads + h : (size_t)h * a.batch_dim + b) * a.head_dim;
-    else if (is_key) dst = reinterpret_cast<__nv_bfloat16*>(keys) + ((size_t)row * a.num_kv_heads + (h - a.num_q_heads)) * a.head_dim;
-    else dst = reinterpret_cast<__nv_bfloat16*>(values) + ((size_t)row * a.num_kv_heads + (h - a.num_q_heads - a.num_kv_heads)) * a.head_dim;
+    if (is_query) dst = reinterpret_cast<__nv_bfloat16*>(a.queries) + ((size_t)h * a.batch_dim + b) * a.head_dim;
+    else if (is_key) dst = reinterpret_cast<__nv_bfloat16*>(a.keys) + ((size_t)row * a.num_kv_heads + (h - a.num_q_heads)) * a.head_dim;
+    else dst = reinterpret_cast<__nv_bfloat16*>(a.values) + ((size_t)row * a.num_kv_heads + (h - a.num_q_heads - a.num_kv_heads)) * a.head_dim;
     *reinterpret_cast<uint4*>(dst + d) = v;
 }
 
@@ -247,9 +236,8 @@ constexpr int ATTN_UNROLL = 2;      // key rows per lane group per round (one mo
 // loaded ATTN_UNROLL at a time with no dependency between them; (2) chunk max / exp / sum per head; (3) o += p.V with the V
 // rows streamed the same way. The running (m, l, o) is rescaled only once per chunk, so the key loop has no serial
 // softmax chain (the first version of this kernel updated (m, l, o) per key and spent most of its time waiting on loads).
-// SEQS: grid y is a sequence with one query row and a cache of its own instead of a query row.
-template <int D, int G, bool SEQS>
-__global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnParams p, const __grid_constant__ std::conditional_t<SEQS, AttnSequences, NoSequences> seqs) {
+template <int D, int G>
+__global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnParams p) {
     constexpr int EPL = (D >= 128 && G < 8) ? 16 : 8;    // elements per lane (q and o live in registers: 2 * G * EPL floats)
     constexpr int CH = (G >= 8) ? ATTN_CHUNK / 2 : ATTN_CHUNK;   // scores [G][CH] + partial outputs stay under the 48 KB static limit
     constexpr int LPK = D / EPL;              // lanes per key row
@@ -265,16 +253,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     pdl_wait();
     uzu_attention_args a = p.a;
     uint32_t keys_per_split = p.keys_per_split, nsplits = p.nsplits;
-    if constexpr (SEQS) {
-        const uint32_t b = blockIdx.y;
-        a.sequence_length = (a.dynamic_position ? reinterpret_cast<const uint32_t*>(a.dynamic_position)[b] : seqs.prefix[b]) + 1u;
-        a.keys = seqs.keys[b];
-        a.values = seqs.values[b];
-        a.queries += (uint64_t)b * a.num_heads * D * 2u;
-        nsplits = min(p.nsplits, (a.sequence_length + 63u) / 64u);      // by its own length alone, as a launch of its own has it
-        if (blockIdx.z >= nsplits) return;
-        keys_per_split = ((a.sequence_length + nsplits - 1) / nsplits + 15u) & ~15u;
-    } else if (a.dynamic_position) {
+    if (a.dynamic_position) {
         a.sequence_length = *reinterpret_cast<const uint32_t*>(a.dynamic_position) + a.suffix_length;
         // by its own length too: a captured step serves every length up to a bound, and its bits must not depend on the length it was captured at
         nsplits = min(p.nsplits, (a.sequence_length + 63u) / 64u);
@@ -283,7 +262,7 @@ __global__ void __launch_bounds__(ATTN_WARPS * 32) attn_split_kernel(const AttnP
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int sub = lane / LPK, li = lane % LPK, d0 = li * EPL;
-    const uint32_t head0 = blockIdx.x * G, out_row = blockIdx.y, qs = SEQS ? 0u : blockIdx.y, split = blockIdx.z;
+    const uint32_t head0 = blockIdx.x * G, out_row = blockIdx.y, qs = blockIdx.y, split = blockIdx.z;
     const uint32_t kvh = head0 / a.gqa_factor;
 
     const uint32_t prefix_length = a.sequence_length - a.suffix_length;
@@ -588,20 +567,19 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(const __nv_bfloat16* 
 // host dispatch
 // ---------------------------------------------------------------------------------------------------
 template <int D, int G>
-static void launch_attn(uzu_command_buffer* cmd, const AttnParams& p, const AttnSequences* seqs, uint32_t head_groups) {
-    dim3 grid(head_groups, seqs ? seqs->count : p.a.suffix_length, p.nsplits);
-    if (seqs) launch(cmd, "attn_split_kernel", attn_split_kernel<D, G, true>, grid, dim3(ATTN_WARPS * 32), 0, p, *seqs);
-    else launch(cmd, "attn_split_kernel", attn_split_kernel<D, G, false>, grid, dim3(ATTN_WARPS * 32), 0, p, NoSequences{});
+static void launch_attn(uzu_command_buffer* cmd, const AttnParams& p, uint32_t head_groups) {
+    dim3 grid(head_groups, p.a.suffix_length, p.nsplits);
+    launch(cmd, "attn_split_kernel", attn_split_kernel<D, G>, grid, dim3(ATTN_WARPS * 32), 0, p);
 }
 
 template <int D>
-static void launch_attn_g(uzu_command_buffer* cmd, const AttnParams& p, const AttnSequences* seqs, int g) {
+static void launch_attn_g(uzu_command_buffer* cmd, const AttnParams& p, int g) {
     const uint32_t H = p.a.num_heads;
     switch (g) {
-        case 8: launch_attn<D, 8>(cmd, p, seqs, H / 8); break;
-        case 4: launch_attn<D, 4>(cmd, p, seqs, H / 4); break;
-        case 2: launch_attn<D, 2>(cmd, p, seqs, H / 2); break;
-        default: launch_attn<D, 1>(cmd, p, seqs, H); break;
+        case 8: launch_attn<D, 8>(cmd, p, H / 8); break;
+        case 4: launch_attn<D, 4>(cmd, p, H / 4); break;
+        case 2: launch_attn<D, 2>(cmd, p, H / 2); break;
+        default: launch_attn<D, 1>(cmd, p, H); break;
     }
 }
 
@@ -636,24 +614,23 @@ static int pick_group(uint32_t gqa) {
     return 1;
 }
 
-static void dispatch_attn(uzu_command_buffer* cmd, const AttnParams& p, const AttnSequences* seqs, int g) {
+static void dispatch_attn(uzu_command_buffer* cmd, const AttnParams& p, int g) {
     switch (p.a.head_dim) {
-        case 64: launch_attn_g<64>(cmd, p, seqs, g); break;
-        case 128: launch_attn_g<128>(cmd, p, seqs, g); break;
-        default: launch_attn_g<256>(cmd, p, seqs, g); break;
+        case 64: launch_attn_g<64>(cmd, p, g); break;
+        case 128: launch_attn_g<128>(cmd, p, g); break;
+        default: launch_attn_g<256>(cmd, p, g); break;
     }
 }
 
-// the rows' keys cut over CTAs, merged by the last CTA of a (row, head group). Sequences are cut each by its own length (the kernel; a.sequence_length is
-// the most there is): a long one among short ones would otherwise get as few CTAs as they need, and its bits would depend on its neighbours.
-static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& a, const AttnSequences* seqs, float* workspace) {
+// the rows' keys cut over CTAs, merged by the last CTA of a (row, head group)
+static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& a) {
     uzu_context* ctx = cmd->ctx;
     const int g = pick_group(a.gqa_factor);
-    const uint32_t head_groups = a.num_heads / g, rows = seqs ? seqs->count : a.suffix_length;
+    const uint32_t head_groups = a.num_heads / g, rows = a.suffix_length;
     // enough CTAs for ~2 waves, >= 64 keys per split, <= 32 splits, and only for short suffixes (decode)
     uint32_t nsplits = 1;
     if (rows <= 16) {
-        const uint32_t ctas = seqs ? head_groups : head_groups * rows;
+        const uint32_t ctas = head_groups * rows;
         const uint32_t want = (2u * (uint32_t)ctx->sm_count + ctas - 1) / ctas;
         const uint32_t cap = (a.sequence_length + 63) / 64;
         nsplits = std::max(1u, std::min(std::min(want, cap), 32u));
@@ -668,7 +645,7 @@ static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& 
     if (nsplits > 1) {
         const size_t units = (size_t)rows * a.num_heads * nsplits;
         const size_t need = units * (a.head_dim + 2) * sizeof(float);
-        if (!workspace && need > ctx->attn_ws_bytes) {  // grows outside graph capture only (decode needs < 2 MiB)
+        if (need > ctx->attn_ws_bytes) {  // grows outside graph capture only (decode needs < 2 MiB)
             cudaStreamSynchronize(ctx->stream);
             cudaFree(ctx->attn_ws);
             if (cudaMalloc(&ctx->attn_ws, need) != cudaSuccess) {
@@ -683,12 +660,12 @@ static void encode_attn_rows(uzu_command_buffer* cmd, const uzu_attention_args& 
             cmd->record_error(UZU_ERROR_UNSUPPORTED, "attention_single_pass: too many (token, head group) pairs for the split path");
             return;
         }
-        p.part_o = workspace ? workspace : ctx->attn_ws;
+        p.part_o = ctx->attn_ws;
         p.part_sum = p.part_o + units * a.head_dim;
         p.part_max = p.part_sum + units;
         p.counters = ctx->attn_counters;
     }
-    dispatch_attn(cmd, p, seqs, g);
+    dispatch_attn(cmd, p, g);
 }
 
 // whole 16-byte pieces of every row, and of each half of the rotated channels
@@ -696,32 +673,6 @@ static bool attention_prepare_whole_pieces(const uzu_attention_prepare_args& a) 
     const uint64_t total_heads = a.has_kv ? a.num_q_heads + 2 * a.num_kv_heads : a.num_q_heads;
     return a.head_dim % 8u == 0 && (!a.has_rope || (a.rope_dim % 16u == 0 && !((a.cosines | a.sines) & 15u))) && total_heads * a.batch_dim * (a.head_dim / 8u) < 0x80000000ull &&
            !((a.qkv | a.queries) & 15u);
-}
-
-// Plain causal rows on caches of whole 16-byte pieces. 8 sequences x 32 heads of 128 at 200 cached rows, a layer: 19 us -- 132 us as a prepare and
-// an attention launch per sequence.
-bool attention_sequences_applicable(const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s) {
-    uint64_t caches = 0;
-    for (uint32_t b = 0; b < s.count; ++b) caches |= s.keys[b] | s.values[b];
-    return s.count && s.count <= kMaxAttnSequences && p.batch_dim == s.count && p.has_kv && a.suffix_length == 1 && !a.is_trie && !a.is_kv_cache_ring && !a.is_sliding_window &&
-           !a.has_sinks && attention_prepare_whole_pieces(p) && !(caches & 15u);
-}
-
-size_t attention_sequences_workspace_bytes(uint32_t heads, uint32_t head_dim) {
-    return (size_t)kMaxAttnSequences * heads * 32u * (head_dim + 2u) * sizeof(float);
-}
-
-void encode_attention_sequences(uzu_command_buffer* cmd, const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s, uint32_t longest,
-                                uint64_t workspace) {
-    if (!encodable(cmd, "attention_sequences")) return;
-    uzu_attention_args most = a;
-    most.keys = s.keys[0];
-    most.values = s.values[0];
-    most.sequence_length = longest;
-    if (!attn_common_checks(cmd, &most, "attention_sequences")) return;
-    const uint32_t units = (p.num_q_heads + 2 * p.num_kv_heads) * s.count * (p.head_dim / 8u);
-    launch(cmd, "attention_prepare_kernel", attention_prepare_vec_kernel<true>, dim3((units + 255u) / 256u), dim3(256), 0, p, s);
-    encode_attn_rows(cmd, most, &s, reinterpret_cast<float*>(workspace));
 }
 
 }  // namespace uzu
@@ -740,7 +691,7 @@ void uzu_attention_prepare_encode(uzu_command_buffer* cmd, const uzu_attention_p
     if (a->batch_dim == 0 || total_heads == 0) return;
     if (uzu::attention_prepare_whole_pieces(*a) && !((a->has_kv ? a->keys | a->values : 0u) & 15u)) {
         const uint32_t units = total_heads * a->batch_dim * (a->head_dim / 8u);
-        uzu::launch(cmd, "attention_prepare_kernel", uzu::attention_prepare_vec_kernel<false>, dim3((units + 255u) / 256u), dim3(256), 0, *a, uzu::NoSequences{});
+        uzu::launch(cmd, "attention_prepare_kernel", uzu::attention_prepare_vec_kernel, dim3((units + 255u) / 256u), dim3(256), 0, *a);
         return;
     }
     dim3 grid(total_heads, a->batch_dim);
@@ -772,7 +723,7 @@ void uzu_attention_single_pass_encode(uzu_command_buffer* cmd, const uzu_attenti
     if (!uzu::encodable(cmd, "attention_single_pass")) return;
     if (!uzu::attn_common_checks(cmd, a, "attention_single_pass")) return;
     if (uzu::encode_attention_prefill(cmd, *a)) return;   // the tensor-pipe form (attention_prefill.cu)
-    uzu::encode_attn_rows(cmd, *a, nullptr, nullptr);
+    uzu::encode_attn_rows(cmd, *a);
 }
 
 void uzu_attention_two_pass1_encode(uzu_command_buffer* cmd, const uzu_attention_args* a) {
@@ -797,7 +748,7 @@ void uzu_attention_two_pass1_encode(uzu_command_buffer* cmd, const uzu_attention
     p.nsplits = std::max(1u, std::min(std::min(want, cap), 32u));
     p.nb = 32;  // TOTAL_BLOCKS_COUNT (attention_two_pass.rs:10)
     p.keys_per_split = p.nsplits > 1 ? (((a->sequence_length + p.nsplits - 1) / p.nsplits + 15u) & ~15u) : a->sequence_length;
-    uzu::dispatch_attn(cmd, p, nullptr, g);
+    uzu::dispatch_attn(cmd, p, g);
 }
 
 void uzu_attention_two_pass2_encode(uzu_command_buffer* cmd, const uzu_attention_two_pass2_args* a) {

@@ -129,18 +129,18 @@ bool dense_umma_applicable(const uzu_dense_linear_args& a);
 // tensor-core prefill attention (attention_prefill.cu), tried first by uzu_attention_single_pass_encode
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a);
 
-// One decoded row of several sequences, each with a cache of its own (attention.cu): a launch for all of them instead of one per sequence.
+// One decoded row a sequence, each with a cache of its own (decode_attention.cu): rotation, cache and attention in one launch for all of them.
 constexpr uint32_t kMaxAttnSequences = 16;
 struct AttnSequences {
     uint64_t keys[kMaxAttnSequences], values[kMaxAttnSequences];
     uint32_t prefix[kMaxAttnSequences], position[kMaxAttnSequences];      // cached rows, rotation row; both from dynamic_position[b] where the args have one
     uint32_t count;
 };
-bool attention_sequences_applicable(const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s);
-size_t attention_sequences_workspace_bytes(uint32_t heads, uint32_t head_dim);      // for kMaxAttnSequences of any length
-// longest: no sequence has more cached rows than that, this step's included (with dynamic positions: at any time the launch is repeated)
-void encode_attention_sequences(uzu_command_buffer* cmd, const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s, uint32_t longest,
-                                uint64_t workspace);
+bool decode_attention_applicable(const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s);
+// longest: no sequence has more cached rows than that, this step's included (with dynamic positions: at any time the launch is repeated). All rows before this
+// step's, and the positions, were written before the first kernel of the step could start.
+void encode_decode_attention(uzu_command_buffer* cmd, const uzu_attention_prepare_args& a, const uzu_qk_norm_config* q_norm, const uzu_qk_norm_config* k_norm, float scale, uint64_t out,
+                             const AttnSequences& s, uint32_t longest);
 
 // latent attention of a prompt's rows on the tensor pipe (latent_attention_mma.cu)
 bool latent_attention_mma_applicable(const uzu_latent_attention_args& a);

@@ -696,7 +696,6 @@ struct uzu_engine {
     // multi-sequence batched decode (extension): independent sequence states sharing one weight pass per step
     struct Sequence { std::vector<LayerState> layers; uint32_t context_length = 0; };
     std::vector<Sequence> seqs;
-    Buf batch_attn;                // partial attention results of a batched step, for sequences of any length (a captured step holds its address)
     Buf batch_pos;                 // device u32[16]: per-sequence prefix lengths (the captured batched step reads positions from here)
     bool batch_pos_valid = false;
     std::vector<uzu::StepGraph> batch_graphs;
@@ -1662,8 +1661,9 @@ static uzu_fused_linear_args fused_norm_args(const Linear& l, const Norm& n, uin
 //   bit 2: SigmoidGate -> prologue of the attention out projection
 //   bit 3: QKVNorm(q) + QKVNorm(k) + AttentionPrepare -> one launch
 //   bit 4: DeltaNetConvUpdate -> inside DeltaNetUpdate (one k head per v head only)
+//   bit 5: QKVNorm, AttentionPrepare and attention -> one launch
 static uint32_t fuse_mask() {
-    static const uint32_t m = [] { const char* v = getenv("UZU_FUSE_MASK"); return v ? (uint32_t)atoi(v) : 31u; }();
+    static const uint32_t m = [] { const char* v = getenv("UZU_FUSE_MASK"); return v ? (uint32_t)atoi(v) : 63u; }();
     return m;
 }
 
@@ -1741,7 +1741,7 @@ static void encode_decode_gemv(uzu_engine* e, uzu_command_buffer* cmd, const Lin
 static void encode_decoder_fused(uzu_engine* e, uzu_command_buffer* cmd, const PassCtx& pc) {
     const uint32_t H = e->model_dim;
     const uint32_t mask = fuse_mask();
-    const bool fuse_norm = (mask & 1u) != 0, fuse_gated = (mask & 2u) != 0, fuse_sigmoid = (mask & 4u) != 0, fuse_qknorm = (mask & 8u) != 0, fuse_conv = (mask & 16u) != 0;
+    const bool fuse_norm = (mask & 1u) != 0, fuse_gated = (mask & 2u) != 0, fuse_sigmoid = (mask & 4u) != 0, fuse_qknorm = (mask & 8u) != 0, fuse_conv = (mask & 16u) != 0, fuse_attention = (mask & 32u) != 0;
     // embedding lookup (embedding.rs:345-372)
     if (e->in_emb.w.prologue == UZU_B_FULL_PRECISION) {
         uzu_full_precision_embedding_lookup_encode(cmd, e->token_ids.ptr(), e->in_emb.w.values.ptr(), e->hidden_a.ptr(), 1, e->vocab, H, e->input_scale);
@@ -1792,15 +1792,27 @@ static void encode_decoder_fused(uzu_engine* e, uzu_command_buffer* cmd, const P
                 pa.cosines = e->rope_cos[A.rope_index].ptr(); pa.sines = e->rope_sin[A.rope_index].ptr();
             }
             pa.dynamic_position = dyn;
-            if (fuse_qknorm && (A.qnorm.present || A.knorm.present) && D <= 256) {
+            uzu_attention_args aa{};
+            aa.queries = e->queries.ptr(); aa.keys = St.keys; aa.values = St.values; aa.out = e->attn_out.ptr();
+            aa.gqa_factor = Hq / Hkv; aa.sequence_length = attention_bucket(St.length + 1);   // the most; the kernel reads its own
+            aa.k_head_stride = D; aa.k_seq_stride = Hkv * D; aa.v_head_stride = D; aa.v_seq_stride = Hkv * D;
+            aa.scale = A.has_scale ? A.scale : 1.0f / sqrtf((float)D);
+            aa.num_heads = Hq; aa.suffix_length = 1; aa.head_dim = D; aa.is_causal = A.is_causal; aa.dynamic_position = dyn;
+            auto cfg = [](const Norm& nm) {
+                uzu_qk_norm_config c{};
+                c.present = nm.present; c.scales = nm.scales.ptr(); c.epsilon = nm.cfg.epsilon; c.scale_offset = nm.cfg.scale_offset;
+                c.full_layer = nm.cfg.full_layer; c.has_scales = nm.cfg.has_scale;
+                return c;
+            };
+            AttnSequences seq{};
+            seq.count = 1; seq.keys[0] = St.keys; seq.values[0] = St.values;
+            const bool one_launch = fuse_attention && decode_attention_applicable(pa, aa, seq);
+            if (one_launch) {
+                const uzu_qk_norm_config qn = cfg(A.qnorm), kn = cfg(A.knorm);
+                encode_decode_attention(cmd, pa, &qn, &kn, aa.scale, aa.out, seq, aa.sequence_length);
+            } else if (fuse_qknorm && (A.qnorm.present || A.knorm.present) && D <= 256) {
                 uzu_attention_prepare_norm_args pn{};
                 pn.prepare = pa;
-                auto cfg = [](const Norm& nm) {
-                    uzu_qk_norm_config c{};
-                    c.present = nm.present; c.scales = nm.scales.ptr(); c.epsilon = nm.cfg.epsilon; c.scale_offset = nm.cfg.scale_offset;
-                    c.full_layer = nm.cfg.full_layer; c.has_scales = nm.cfg.has_scale;
-                    return c;
-                };
                 pn.q_norm = cfg(A.qnorm); pn.k_norm = cfg(A.knorm);
                 uzu_attention_prepare_norm_encode(cmd, &pn);
             } else {
@@ -1818,13 +1830,7 @@ static void encode_decoder_fused(uzu_engine* e, uzu_command_buffer* cmd, const P
                 qkn(A.knorm, Hq, Hkv);
                 uzu_attention_prepare_encode(cmd, &pa);
             }
-            uzu_attention_args aa{};
-            aa.queries = e->queries.ptr(); aa.keys = St.keys; aa.values = St.values; aa.out = e->attn_out.ptr();
-            aa.gqa_factor = Hq / Hkv; aa.sequence_length = attention_bucket(St.length + 1);   // the most; the kernel reads its own
-            aa.k_head_stride = D; aa.k_seq_stride = Hkv * D; aa.v_head_stride = D; aa.v_seq_stride = Hkv * D;
-            aa.scale = A.has_scale ? A.scale : 1.0f / sqrtf((float)D);
-            aa.num_heads = Hq; aa.suffix_length = 1; aa.head_dim = D; aa.is_causal = A.is_causal; aa.dynamic_position = dyn;
-            uzu_attention_single_pass_encode(cmd, &aa);
+            if (!one_launch) uzu_attention_single_pass_encode(cmd, &aa);
             if (A.has_gate && fuse_sigmoid && !e->tp_sharded) {
                 uzu_fused_linear_args g{};
                 g.matmul = linear_args(A.out, 0, 1, e->mixer_out.ptr());
@@ -2991,8 +2997,8 @@ static void encode_batch_step(uzu_engine* e, uzu_command_buffer* cmd, bool dyn, 
             aa.scale = A.has_scale ? A.scale : 1.0f / sqrtf((float)D);
             aa.num_heads = Hq; aa.suffix_length = 1; aa.head_dim = D; aa.is_causal = A.is_causal;
             if (dyn) aa.dynamic_position = e->batch_pos.ptr();
-            if (attention_sequences_applicable(pa, aa, seqs)) {
-                encode_attention_sequences(cmd, pa, aa, seqs, longest, e->batch_attn.ptr());
+            if (decode_attention_applicable(pa, aa, seqs)) {
+                encode_decode_attention(cmd, pa, nullptr, nullptr, aa.scale, aa.out, seqs, longest);
             } else {
                 for (uint32_t b = 0; b < B; ++b) {
                     uzu_attention_prepare_args pb = pa;
@@ -3229,10 +3235,6 @@ uzu_status uzu_engine_batch_begin(uzu_engine* e, uint32_t sequences) {
         cudaStreamSynchronize(e->ctx->stream);
         // a captured batched step holds the addresses of every sequence's state: a different set of sequences needs new captures
         if (e->seqs.size() != sequences) drop_step_graphs(e->batch_graphs);
-        size_t attn_bytes = 0;
-        for (auto& L : e->layers)
-            if (L.is_attention) attn_bytes = std::max(attn_bytes, attention_sequences_workspace_bytes(L.attn.num_heads, L.attn.head_dim));
-        if (attn_bytes && !e->batch_attn.b) e->batch_attn = make_buf(e, attn_bytes, UZU_BUFFER_DEVICE);
         while (e->seqs.size() < sequences) {
             e->seqs.emplace_back();
             alloc_sequence_state(e, e->seqs.back().layers);
