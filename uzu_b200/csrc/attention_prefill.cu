@@ -65,6 +65,7 @@ __device__ __forceinline__ float pa_remote(uint32_t addr, uint32_t rank) {
 
 template <int D, int PLANES>
 __global__ void __launch_bounds__(128, D == 256 ? 2 : 3) attn_prefill_kernel(const uzu_attention_args a, const uint32_t splits) {
+    pdl_launch_dependents();
     pdl_wait();
     constexpr uint32_t LD = D + 8;                  // padded tile row (elements): 16-byte aligned rows, conflict-free ldmatrix
     constexpr uint32_t TILE = PA_BN * LD * 2;       // bytes
@@ -422,12 +423,17 @@ static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_arg
     cfg.dynamicSmemBytes = smem;
     cfg.stream = cmd->ctx->stream;
     cudaLaunchAttribute attr[1];
+    cfg.attrs = attr;
     if (splits > 1) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = splits;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    else if (cmd->use_pdl) {      // (not clusters: started beside the last CTAs of the kernel before, they share SMs that others leave idle, 31 us -> 44 for 16 rows and 2048 keys)
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 1;
     }
     const cudaError_t e = cudaLaunchKernelEx(&cfg, attn_prefill_kernel<D, PLANES>, a, splits);

@@ -1535,6 +1535,8 @@ static uint64_t encode_delta_net(uzu_engine* e, uzu_command_buffer* cmd, const L
         f0.update.value_dim = D.value_dim; f0.update.norm_epsilon = D.norm_epsilon; f0.update.head_k_dim = D.head_dim;
         whole_pass = encode_delta_net_prefill(cmd, f0, m, D.total_proj_dim, D.value_dim, e->delta_scratch.ptr());
     }
+    const bool pdl = cmd->use_pdl;
+    if (m > 1) cmd->use_pdl = false;      // row by row: the update kernel reads its state, which the row before it writes, ahead of its wait
     for (uint32_t t = 0; t < m && !whole_pass; ++t) {
         const uint64_t row = e->in_proj.ptr() + (size_t)t * D.total_proj_dim * 2;
         uzu_delta_net_fused_update_args fa{};
@@ -1553,6 +1555,7 @@ static uint64_t encode_delta_net(uzu_engine* e, uzu_command_buffer* cmd, const L
             uzu_delta_net_update_encode(cmd, &ua);
         }
     }
+    cmd->use_pdl = pdl;
     encode_linear(cmd, D.out_proj, e->delta_out.ptr(), m, e->mixer_out.ptr());
     return e->mixer_out.ptr();
 }
@@ -2425,6 +2428,7 @@ static void run_pass(uzu_engine* e, const uint32_t* tokens, uint32_t count, uint
     memcpy(uzu_buffer_cpu_ptr(e->host_tokens.b), tokens, count * 4);
     CmdGuard g(e->ctx, "pass");
     check(uzu_command_buffer_start_encoding(g.c));
+    g.c->use_pdl = e->use_pdl && !e->parallel_block;      // (those models' layers may run several times in a pass, and their kernels read states ahead of their wait)
     uzu_command_buffer_encode_copy(g.c, e->host_tokens.ptr(), e->token_ids.ptr(), count * 4);
     PassCtx pc;
     pc.m = count;
@@ -2769,6 +2773,7 @@ uzu_status uzu_engine_trie_pass(uzu_engine* e, const uint32_t* tokens, const uzu
             h_seeds[i] = seeds ? seeds[i] : prng_derive(e->sampling.seed, (uint64_t)e->context_length + nodes[i].height);
         CmdGuard g(e->ctx, "trie pass");
         check(uzu_command_buffer_start_encoding(g.c));
+        g.c->use_pdl = e->use_pdl;
         uzu_command_buffer_encode_copy(g.c, e->host_trie.ptr() + MAX_TRIE * (8 + sizeof(uzu_trie_node)), e->token_ids.ptr(), count * 4);
         uzu_command_buffer_encode_copy(g.c, e->host_trie.ptr() + MAX_TRIE * 8, e->trie_nodes.ptr(), count * sizeof(uzu_trie_node));
         uzu_command_buffer_encode_copy(g.c, e->host_trie.ptr(), e->seeds.ptr(), count * 8);
