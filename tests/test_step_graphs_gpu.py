@@ -177,3 +177,27 @@ def test_batches_that_come_back_to_a_length(ctx, tmp_path, kind):
         assert [captures(s) for s in shapes] == [0, 0, 0]
         assert captures((60, 20)) == 1                        # below 64 only
         assert captures(shapes[0]) == 2
+
+
+@pytest.mark.parametrize("mode", [True, False])
+@pytest.mark.parametrize("lookahead", [1, 257])
+def test_fed_steps_behind_steps_in_flight(ctx, tmp_path, mode, lookahead):
+    """A fed step after steps that nobody waited for (their tokens land in the ring that it reads): alone, and behind a reset that counts from zero again."""
+    spec = synth.tiny("llama", layers=1)
+    path = synth.write_model(spec, tmp_path / "m", seed=11)
+    prompt = np.arange(9) * 5 % spec.vocab_size
+    with B.Engine(ctx, path, max_context_length=1024, use_cuda_graph=mode) as eng:
+        eng.prefill(prompt)
+        eng.decode_device(lookahead)
+        ctx.synchronize()
+        want = eng.step_host(3)
+        eng.reset()
+        again = eng.step_host(7)
+        eng.prefill(prompt)
+        eng.reset()
+        eng.prefill(prompt)
+        eng.decode_device(lookahead)
+        assert eng.step_host(3) == want
+        eng.decode_device(lookahead - 1)
+        eng.reset()
+        assert eng.step_host(7) == again
