@@ -321,7 +321,8 @@ typedef struct uzu_attention_args {
 UZU_API void uzu_attention_single_pass_encode(uzu_command_buffer* cmd, const uzu_attention_args* args);
 UZU_API void uzu_attention_two_pass1_encode(uzu_command_buffer* cmd, const uzu_attention_args* args);
 /* Tensor-pipe attention of 8 and more query tokens (csrc/attention_prefill.cu; causal, non-causal and tries, head_dim 64 | 128 | 256), taken by
- * uzu_attention_single_pass_encode; 0 here or UZU_PREFILL_ATTN=0 keeps the split-KV kernel, 1 forces it on, -1 = follow the environment. */
+ * uzu_attention_single_pass_encode; 0 here or UZU_PREFILL_ATTN=0 keeps the split-KV kernel, 1 forces the mma.sync kernel on, 2 the tcgen05 one
+ * (csrc/attention_umma.cu), -1 = follow the environment. */
 UZU_API void uzu_debug_set_prefill_attention(int mode);
 /* AttentionTwoPass2Kernel: attention_two_pass.rs:139-149 */
 typedef struct uzu_attention_two_pass2_args {

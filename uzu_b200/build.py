@@ -31,6 +31,7 @@ SOURCES = {
     "tp.cu": [],
     "attention.cu": ["-fmad=false"],
     "attention_prefill.cu": [],
+    "attention_umma.cu": [],
     "decode_attention.cu": [],
     "norm.cu": ["-fmad=false"],
     "elementwise.cu": ["-fmad=false"],

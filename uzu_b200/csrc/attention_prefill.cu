@@ -388,15 +388,21 @@ static uint32_t pa_splits(const uzu_attention_args& a, uint32_t sms) {
 
 static bool pa_two_planes(const uzu_attention_args& a) { return a.suffix_length >= 16 && !a.is_trie && a.head_dim != 256; }
 
-// Whether this kernel is the faster one: both estimates in us, fitted to 1480 sizes (8 to 256 tokens, 0 to 8000 cached rows, 4 to 64 heads in groups of 1 to
-// 8; the choice costs 0.7 % on average). The split-KV kernel pays for every (token, head) and key, this one for whole tiles of 64 x 64. 32 heads of 128 in
+// Which kernel takes a call. Estimates in us of this one and the split-KV kernel, fitted to 1480 sizes (8 to 256 tokens, 0 to 8000 cached rows, 4 to 64 heads in groups
+// of 1 to 8; the choice costs 0.7 % on average). The split-KV kernel pays for every (token, head) and key, this one for whole tiles of 64 x 64. 32 heads of 128 in
 // groups of 4, split-KV / this one: 8 tokens behind 16 rows 6.7 / 13.7, behind 450 23 / 19, behind 2048 48 / 31; 16 tokens behind 16 6.6 / 11.5, behind 1000
 // 41 / 15. 8 heads of 256, 64 tokens alone 10.7 / 27, behind 1000 73 / 28. Fewer than 8 tokens stay with the split-KV kernel: 4 behind 200 take 12.4 / 14.5,
 // behind 1000 19 / 14.5, behind 4096 45 / 37.
-static bool pa_faster(const uzu_attention_args& a, uint32_t sms) {
+// The tcgen05 kernel (attention_umma.cu) walks the keys in CTAs of 128 rows that share nothing: the chip has to be filled by the rows. Fitted to 720 sizes (16 to 1024
+// tokens, 0 to 6000 cached rows), within 10 % for nine in ten, so that it is taken where it is the faster by a sixth. This one / that one: 32 heads of 128 in groups
+// of 4, 64 tokens behind 100 16.4 / 13.4, behind 1100 20.4 / 25.9 (its keys are split, that one's not), 256 behind 1100 42.9 / 28.7, 1024 behind 1100 167 / 48; of 64,
+// 1024 behind 1100 92 / 43; 8 heads of 256 in groups of 4, 256 behind 1100 38.2 / 38.7, 400 57 / 41, 1024 128 / 53. In place of the split-KV kernel, whose weights
+// are f32, it has to have three planes: 8 heads of 256, 100 tokens behind 100 21.7 / 16.5.
+enum class PaKernel { Split, Mma, Umma };
+static PaKernel pa_choose(const uzu_attention_args& a, uint32_t sms) {
     const uint32_t D = a.head_dim, rows = a.suffix_length, keys = a.sequence_length, gq = a.gqa_factor, g = gq % 8 == 0 ? 8 : gq % 4 == 0 ? 4 : gq % 2 == 0 ? 2 : 1;
-    if (rows < 8) return false;
-    const uint32_t ctas = a.num_heads / g * rows;                              // as encode_attn_rows (attention.cu) cuts it
+    if (rows < 8) return PaKernel::Split;
+    const uint32_t kv_heads = a.num_heads / gq, ctas = a.num_heads / g * rows;      // as encode_attn_rows (attention.cu) cuts it
     const uint32_t nsplits = rows <= 16 ? std::max(1u, std::min(std::min((2 * sms + ctas - 1) / ctas, (keys + 63) / 64), 32u)) : 1u;
     const float fill = (float)ctas * nsplits / (sms * (D == 128 ? 1.0f : 2.0f));
     const float waves = D == 128 ? 0.5f * (std::ceil(fill) + std::max(1.0f, fill)) : std::ceil(fill);
@@ -405,10 +411,17 @@ static bool pa_faster(const uzu_attention_args& a, uint32_t sms) {
                         ((D == 64 ? 5.5f : 6.2f) + waves * per_key * keys / nsplits + (nsplits == 1 ? 0.0f : D == 64 ? 2.8f : D == 128 ? 4.5f : 6.1f));
     const bool two = pa_two_planes(a);
     const uint32_t shares = pa_splits(a, sms), row_tiles = (rows * gq + PA_BM - 1) / PA_BM, key_tiles = (keys + PA_BN - 1) / PA_BN, room = sms * (D == 256 ? 2u : 3u);
-    const uint32_t all = row_tiles * (a.num_heads / gq) * shares, turns = std::max(1u, (all + room - 1) / room), per = (key_tiles + shares - 1) / shares;
+    const uint32_t all = row_tiles * kv_heads * shares, turns = std::max(1u, (all + room - 1) / room), per = (key_tiles + shares - 1) / shares;
     const float start = D == 64 ? 5.0f : D == 128 ? 8.6f : 14.5f, tile = D == 64 ? (two ? 1.8f : 3.0f) : D == 128 ? (two ? 2.8f : 4.65f) : 7.0f;
     const float merge = shares == 1 ? 0.0f : D == 64 ? (two ? 4.4f : 2.3f) : D == 128 ? (two ? 1.9f : 0.6f) : -0.7f;
-    return start * (0.5f + 0.5f * turns) + tile * per * turns + merge < split;
+    const float mma = start * (0.5f + 0.5f * turns) + tile * per * turns + merge;
+    const bool split_is_faster = mma >= split;
+    if (!attn_umma_applicable(a) || (split_is_faster && (two || rows <= 16))) return split_is_faster ? PaKernel::Split : PaKernel::Mma;
+    const uint32_t u_ctas = (rows * gq + 127) / 128 * kv_heads * (D == 256 ? 2u : 1u), u_sm = D == 256 || (D == 128 && !two) ? 1u : 2u, u_turns = std::max(1u, (u_ctas + sms * u_sm - 1) / (sms * u_sm));
+    const float u_tile = (D == 64 ? 0.73f : D == 128 ? 0.81f : 1.27f) * u_turns + (u_sm == 2 && u_ctas > sms ? (D == 64 ? 0.24f : 0.33f) : 0.0f);
+    const float umma = (D == 64 ? 4.0f + 4.0f * u_turns : 9.7f) + u_tile * key_tiles * (D != 256 && !two ? 1.3f : 1.0f);
+    if (1.2f * umma < std::min(mma, split)) return PaKernel::Umma;
+    return split_is_faster ? PaKernel::Split : PaKernel::Mma;
 }
 
 template <int D, int PLANES>
@@ -442,7 +455,7 @@ static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_arg
 }
 
 // true = handled: where it is the faster kernel, for a dense prefix, a plain mask or a causal trie
-static int g_prefill_attn = -1;   // -1: follow UZU_PREFILL_ATTN and the rule, 0: never, 1: wherever it can (uzu_debug_set_prefill_attention)
+static int g_prefill_attn = -1;   // -1: follow UZU_PREFILL_ATTN and the rule, 0: never, 1: wherever it can, 2: the tcgen05 kernel wherever that can (uzu_debug_set_prefill_attention)
 
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a) {
     static const bool env_enabled = [] { const char* e = getenv("UZU_PREFILL_ATTN"); return !e || atoi(e) != 0; }();   // =0 keeps the split-KV kernel
@@ -454,8 +467,13 @@ bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args&
     if ((a.k_head_stride % 8) || (a.v_head_stride % 8) || (a.k_seq_stride % 8) || (a.v_seq_stride % 8)) return false;   // 16-byte cp.async rows
     if ((a.queries | a.keys | a.values | a.out) & 15u) return false;
     if (a.sequence_length < a.suffix_length) return false;
-    if (g_prefill_attn < 0 && !pa_faster(a, (uint32_t)cmd->ctx->sm_count)) return false;
     const bool two = pa_two_planes(a);
+    PaKernel kernel = g_prefill_attn == 1 ? PaKernel::Mma : g_prefill_attn == 2 ? PaKernel::Umma : pa_choose(a, (uint32_t)cmd->ctx->sm_count);
+    if (kernel == PaKernel::Umma) {
+        if (attn_umma_applicable(a) && encode_attn_umma(cmd, a, two ? 2u : 3u)) return true;
+        kernel = g_prefill_attn == 2 ? PaKernel::Split : PaKernel::Mma;
+    }
+    if (kernel == PaKernel::Split) return false;
     if (a.head_dim == 64) two ? launch_attn_prefill<64, 2>(cmd, a) : launch_attn_prefill<64, 3>(cmd, a);
     else if (a.head_dim == 128) two ? launch_attn_prefill<128, 2>(cmd, a) : launch_attn_prefill<128, 3>(cmd, a);
     else launch_attn_prefill<256, 3>(cmd, a);

@@ -129,6 +129,10 @@ bool dense_umma_applicable(const uzu_dense_linear_args& a);
 // tensor-core prefill attention (attention_prefill.cu), tried first by uzu_attention_single_pass_encode
 bool encode_attention_prefill(uzu_command_buffer* cmd, const uzu_attention_args& a);
 
+// the same on tcgen05 (attention_umma.cu), for calls that encode_attention_prefill takes; planes: bf16 planes of a weight, 2 or 3. false: not encoded
+bool attn_umma_applicable(const uzu_attention_args& a);
+bool encode_attn_umma(uzu_command_buffer* cmd, const uzu_attention_args& a, uint32_t planes);
+
 // One decoded row a sequence, each with a cache of its own (decode_attention.cu): rotation, cache and attention in one launch for all of them.
 constexpr uint32_t kMaxAttnSequences = 16;
 struct AttnSequences {
