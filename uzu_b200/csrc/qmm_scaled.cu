@@ -206,10 +206,49 @@ __device__ __forceinline__ void qs_planes_f32(float w0, float w1, uint32_t (&pla
     }
 }
 
+__device__ __forceinline__ void qs_finish(const QsParams& p, float sum, uint32_t token, uint32_t row) {
+    if (token >= p.m || row >= p.n) return;
+    const size_t at = (size_t)token * p.n + row;
+    float val = __fmul_rn(p.ab_scale, sum);                                  // separate roundings, like the reference
+    if (p.accumulate) val = __fadd_rn(val, p.d_is_f32 ? reinterpret_cast<const float*>(p.d)[at] : bf2f(reinterpret_cast<const __nv_bfloat16*>(p.d)[at]));
+    if (p.bias) val = __fadd_rn(val, bf2f(p.bias[row]));
+    if (p.has_soft_cap) val = __fmul_rn(p.soft_cap, tanhf(__fdiv_rn(val, p.soft_cap)));
+    if (p.d_is_f32) reinterpret_cast<float*>(p.d)[at] = val;
+    else reinterpret_cast<__nv_bfloat16*>(p.d)[at] = f2bf(val);
+}
+// Columns `first`, `first` + step, .. of a tile whose partial sums lie in the shared memory of a cluster's CTAs, at `own` in each (this thread's feature, 512 bytes a
+// column), added in rank order. (Not part of the kernel's body: there it cost the tiles that share nothing a tenth of their time.)
+__device__ __noinline__ void qs_exchange(const QsParams& params, uint32_t own, uint32_t first, uint32_t step, uint32_t columns, uint32_t t0, uint32_t row) {
+    const QsParams p = params;                                               // (in registers: read again for each column, 7 us at 256 columns)
+    uint32_t remote[8];
+#pragma unroll
+    for (uint32_t q = 0; q < 8; ++q) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote[q]) : "r"(own), "r"(min(q, p.splits - 1u)));
+    for (uint32_t j0 = first; j0 < columns; j0 += 4 * step) {
+        float part[4][8];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            const uint32_t at = min(j0 + u * step, columns - 1u) * 512u;
+#pragma unroll
+            for (uint32_t q = 0; q < 8; ++q) {
+                part[u][q] = 0.0f;
+                if (q < p.splits) asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part[u][q]) : "r"(remote[q] + at) : "memory");
+            }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            if (j0 + u * step >= columns) continue;
+            float sum = part[u][0];
+#pragma unroll
+            for (int q = 1; q < 8; ++q) sum += part[u][q];
+            qs_finish(p, sum, t0 + j0 + u * step, row);
+        }
+    }
+}
+
 }  // namespace
 
 template <int BITS, int NT, int PL>
-__global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const QsParams p) {
+__global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ QsParams p) {
     using S = QsShape<NT, PL>;
     constexpr int DG = S::DG, ND = S::ND, AS = S::AS, BS = S::BS, CS = S::CS, DQ_WARPS = 4 * DG, EW = S::EW, EC = S::EC;
     constexpr uint32_t kpt = BITS == 4 ? 4u : 2u;                            // k blocks per code tile
@@ -262,16 +301,6 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
         pdl_wait();                                                      // D may be read (accumulate) and is written below
         for (uint32_t item = item0; item < p.items; item += item_step) {
             const uint32_t lanes = (warp & 3u) * 32u, cb = (warp >> 2) * EC, f = lanes + lane, row = item_n(item) + f, t0 = item_m(item);      // cb: this warp's first column
-            auto finish = [&](float sum, uint32_t token) {
-                if (token >= p.m || row >= p.n) return;
-                const size_t at = (size_t)token * p.n + row;
-                float val = __fmul_rn(p.ab_scale, sum);                  // separate roundings, like the reference
-                if (p.accumulate) val = __fadd_rn(val, p.d_is_f32 ? reinterpret_cast<const float*>(p.d)[at] : bf2f(reinterpret_cast<const __nv_bfloat16*>(p.d)[at]));
-                if (p.bias) val = __fadd_rn(val, bf2f(p.bias[row]));
-                if (p.has_soft_cap) val = __fmul_rn(p.soft_cap, tanhf(__fdiv_rn(val, p.soft_cap)));
-                if (p.d_is_f32) reinterpret_cast<float*>(p.d)[at] = val;
-                else reinterpret_cast<__nv_bfloat16*>(p.d)[at] = f2bf(val);
-            };
             const uint32_t columns = min((uint32_t)NT, p.m - t0);
             bool ok = true;
             constexpr bool kSums = PL == 1 || S::CHAIN != 0;
@@ -361,30 +390,14 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
             } else if (p.splits == 1) {
                 each16([&](uint32_t c0, const float* v) {
 #pragma unroll
-                    for (int j = 0; j < 16; ++j) finish(v[j], t0 + c0 + j);
+                    for (int j = 0; j < 16; ++j) qs_finish(p, v[j], t0 + c0 + j, row);
                 });
             } else {
-                // this CTA's tile to shared memory (the rings are idle: every block has been consumed), then column shares over the cluster
+                // this CTA's tile to shared memory (the rings are idle: every block has been consumed); below, column shares over the cluster
                 each16([&](uint32_t c0, const float* v) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) asm volatile("st.shared.f32 [%0], %1;" ::"r"(base + ((c0 + j) * 128u + f) * 4u), "f"(v[j]) : "memory");
                 });
-                qs_cluster_sync();
-                for (uint32_t j = rank + p.splits * (warp >> 2); j < columns && ok; j += p.splits * (EW / 4)) {
-                    float part[8];
-#pragma unroll
-                    for (uint32_t q = 0; q < 8; ++q) {
-                        uint32_t remote;
-                        part[q] = 0.0f;
-                        if (q >= p.splits) continue;
-                        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(base + (j * 128u + f) * 4u), "r"(q));
-                        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(part[q]) : "r"(remote) : "memory");
-                    }
-                    float sum = part[0];
-#pragma unroll
-                    for (int q = 1; q < 8; ++q) sum += part[q];
-                    finish(sum, t0 + j);
-                }
                 break;                                                   // (one item per cluster)
             }
             if (!ok) break;
@@ -499,7 +512,6 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                 if (++slot == (uint32_t)CS) { slot = 0; c_ph ^= 1u; }
             }
         }
-        if (p.splits > 1) qs_cluster_sync();
     } else {
         const uint32_t role = warp - (EW + DQ_WARPS);
         bool ok = true;
@@ -611,10 +623,18 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
             }
         }
         __syncwarp();
-        if (p.splits > 1) qs_cluster_sync();
     }
-    // no CTA of a cluster leaves while another may still read its tile
-    if (p.splits > 1) qs_cluster_sync();
+    if (p.splits > 1) {
+        // A rank's columns of the tile: the partial sums of all ranks in rank order. The warps that turned codes help, and loads of four columns are in flight (the
+        // epilogue warps alone, a column at a time, took 25 us for 256 columns of two ranks).
+        qs_cluster_sync();
+        if (warp < (uint32_t)(EW + DQ_WARPS)) {
+            if (warp >= (uint32_t)EW) pdl_wait();                        // (the epilogue's have waited: D may be read)
+            const uint32_t f = (warp & 3u) * 32u + lane, t0 = item_m(item0);
+            qs_exchange(p, base + f * 4u, rank + p.splits * (warp >> 2), p.splits * ((EW + DQ_WARPS) / 4), min((uint32_t)NT, p.m - t0), t0, item_n(item0) + f);
+        }
+        qs_cluster_sync();      // no CTA of a cluster leaves while another may still read its tile
+    }
     qs_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -668,29 +688,37 @@ namespace {
 
 struct QsPlan { int nt = 0; uint32_t splits = 1; float cost = 1e30f; };
 
-// Cycles of one CTA per 64 k of a tile, as measured: a product takes about 64 cycles however few its rows are and the product warp's waits come on top
-// (16 rows 850, 128 rows 940), wide tiles run at the tensor pipe (256 rows 1240); MLX and 8-bit codes keep the dequant warps busier than that.
-float qs_block_cycles(int nt, uint32_t bits, bool mlx, bool three, bool integers) {
-    if (integers) return bits == 4 ? 700.0f + 0.7f * nt : 760.0f + 0.7f * nt;
-    const float products = std::max(850.0f + 0.7f * nt, 4.85f * nt) * (three ? 1.5f : 1.0f), turn = mlx ? 4000.0f : bits == 4 ? 2000.0f : 2800.0f;
-    return std::max(products, turn / (nt > 128 || nt == 64 || three ? 3.0f : 4.0f));
-}
+// The plan's estimate in us: 5 for a launch; for each turn of the chip, what filling the pipeline and storing a tile of that many rows take, and 64 k as often as a CTA
+// has them; where CTAs share a tile's k, their exchange. Fitted to 3500 times of 13 matrices (512 x 1024 to 28672 x 4096) with 5 to 1024 rows, within 4 % for half of
+// them and 12 % for nine in ten; its choices cost 1 % over the best tile and split of each. (The estimate before it, in cycles, took splits for cheap and turns for
+// all alike: 21 % over the best, 38.8 us for 13.6 at 256 rows x 7168 x 1024.)
+struct QsCost { float fill, integers4, integers8, planes4, planes8, mlx4, mlx8, three4, three8; };
+constexpr int QS_TILES[6] = {16, 32, 64, 128, 192, 256};
+constexpr QsCost QS_COST[6] = {{0.5f, 0.342f, 0.448f, 0.472f, 0.624f, 0.516f, 0.522f, 0.603f, 0.574f}, {0.5f, 0.361f, 0.479f, 0.483f, 0.636f, 0.543f, 0.535f, 0.617f, 0.587f},
+                               {0.9f, 0.376f, 0.487f, 0.491f, 0.646f, 0.539f, 0.561f, 0.659f, 0.629f}, {2.0f, 0.0f, 0.0f, 0.395f, 0.558f, 0.502f, 0.520f, 0.0f, 0.0f},
+                               {1.7f, 0.0f, 0.0f, 0.494f, 0.591f, 0.511f, 0.536f, 0.0f, 0.0f}, {3.2f, 0.0f, 0.0f, 0.558f, 0.588f, 0.584f, 0.569f, 0.0f, 0.0f}};
 
 // Rows per tile and CTAs per tile: the shortest estimated time over the chip. A wider tile turns its codes once for more rows; a narrower one or a
-// split k fills the chip where tiles are few. Fixed cost per item: filling the pipeline and storing the tile.
-QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, bool three, bool integers, uint32_t sms) {
+// split k fills the chip where tiles are few. (Clusters leave SMs idle whose neighbours are taken: of 148, 144 work in pairs, 132 in fours and 112 in eights.)
+QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, bool three, bool integers, bool halves, uint32_t sms) {
     QsPlan best;
     const uint32_t n_tiles = (n + 127u) / 128u;
-    for (int nt : {16, 32, 64, 128, 192, 256}) {
+    for (int i = 0; i < 6; ++i) {
+        const int nt = QS_TILES[i];
+        const QsCost& c = QS_COST[i];
         if (nt > 16 && m <= (uint32_t)nt / 2) break;
-        if (nt < 128 && m > 2u * nt) continue;
+        if (nt < 64 && m > 2u * nt) continue;
+        if (nt >= 128 && three) break;                                       // (three planes: fewer than 64 rows)
+        const float block = integers && nt < 128 ? (bits == 4 ? c.integers4 : c.integers8) : three ? (bits == 4 ? c.three4 : c.three8) : mlx ? (bits == 4 ? c.mlx4 : c.mlx8) : bits == 4 ? c.planes4 : c.planes8;
+        const float two_factors = mlx && halves ? (nt == 256 ? 0.015f : 0.055f) : 0.0f;      // groups of 32
         const uint32_t tiles = n_tiles * ((m + nt - 1) / nt);
         for (uint32_t splits = 1; splits <= 8; splits *= 2) {
             const uint32_t per = ((nkb + splits - 1) / splits + 3u) & ~3u;           // whole code tiles per rank
-            if (splits > 1 && (per * (splits - 1) >= nkb || tiles * splits > sms)) break;
-            const float item = (float)std::min(per, nkb) * qs_block_cycles(nt, bits, mlx, three, integers && nt < 128) + 2500.0f + (nt > 64 ? 12.0f * nt : 0.0f) + (splits > 1 ? 1500.0f + 8.0f * nt : 0.0f);
-            const uint32_t waves = (tiles * splits + sms - 1) / sms;
-            const float cost = waves * item;
+            const uint32_t room = splits == 1 ? sms : splits == 2 ? sms * 36 / 37 : splits == 4 ? sms * 33 / 37 : sms * 28 / 37;
+            if (splits > 1 && (per * (splits - 1) >= nkb || tiles * splits > room)) break;
+            const uint32_t turns = (tiles * splits + room - 1) / room;
+            const float exchange = splits == 1 ? 0.0f : (splits == 2 ? 2.3f : splits == 4 ? 1.7f : 4.5f) + 0.01f * nt;
+            const float cost = 5.2f + turns * (c.fill + (block + two_factors) * std::min(per, nkb)) + exchange;
             if (cost < best.cost) best = {nt, splits, cost};
         }
     }
@@ -755,7 +783,7 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     // MLX weights of passes that the kernels before this one summed with the codes as integers keep all their bits; longer ones had two planes always
     const bool three = p.biases && p.m < 64, integers = !p.biases && a.b_group_size >= 64;      // (integers: tiles of up to 64 rows)
     p.chain_k = std::min(a.b_group_size, 128u);
-    QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, three, integers, (uint32_t)ctx->sm_count);
+    QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, three, integers, a.b_group_size == 32, (uint32_t)ctx->sm_count);
     if (g_tile_rows) plan.nt = g_tile_rows;
     if (g_tile_splits) {
         plan.splits = (uint32_t)g_tile_splits;
