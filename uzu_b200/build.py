@@ -28,6 +28,7 @@ SOURCES = {
     "matmul.cu": [],
     "qmm_rows.cu": [],
     "qmm_scaled.cu": [],
+    "qmm_wide.cu": [],
     "tp.cu": [],
     "attention.cu": ["-fmad=false"],
     "attention_prefill.cu": [],
