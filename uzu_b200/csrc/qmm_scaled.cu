@@ -554,7 +554,7 @@ QsPlan qs_plan(uint32_t m, uint32_t n, uint32_t nkb, uint32_t bits, bool mlx, bo
         const int nt = QS_TILES[i];
         const QsCost& c = QS_COST[i];
         if (nt > 16 && m <= (uint32_t)nt / 2) break;
-        if (nt < 64 && m > 2u * nt) continue;
+        if (nt < 128 && m > 2u * nt) continue;                              // (up to 64 rows sum in another order: the widest of them up to twice its rows)
         if (nt >= 128 && three) break;                                       // (three planes: fewer than 64 rows)
         const float block = integers && nt < 128 ? (bits == 4 ? c.integers4 : c.integers8) : three ? (bits == 4 ? c.three4 : c.three8) : mlx ? (bits == 4 ? c.mlx4 : c.mlx8) : bits == 4 ? c.planes4 : c.planes8;
         const float two_factors = mlx && halves ? (nt == 256 ? 0.015f : 0.055f) : 0.0f;      // groups of 32
