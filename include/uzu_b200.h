@@ -197,8 +197,8 @@ typedef struct uzu_fused_linear_args {
     /* epilogue 1: the matmul's n = 2F rows are [up | gate] (DenseMlp's fused up projection, mlp/dense.rs:32-48); instead of the
      * 2F row the kernel stores hidden[j] = GatedActMul(up_j, gate_j) (act_type) as bf16 [F] into matmul.d. prologue may be 0. */
     uint32_t epilogue, reserved0;
-    /* optional decode-stream copy of matmul.b (unit-major 4608-byte units, built by the engine at load; 0 = none): the decode GEMV then feeds
-     * its shared-memory rings with one TMA bulk copy per stage instead of per-lane cp.async. With a stream, prologue 0 + epilogue 0
+    /* optional decode-stream copy of matmul.b (unit-major 4608-byte units, built by the engine at load; 0 = none): the product of one row then runs on
+     * integer tensor instructions (csrc/decode_linear.cu), its codes fetched by bulk copies. With a stream, prologue 0 + epilogue 0
      * (a plain GEMV over matmul.a) is accepted too. */
     uint64_t decode_stream;
 } uzu_fused_linear_args;

@@ -1811,7 +1811,7 @@ bool fused_linear_supported(uzu_context* ctx, const uzu_fused_linear_args* args)
         if (!m.a) m.a = m.d;
         if (validate(&m)) return false;
     }
-    // prologue 0 + epilogue 0 = a plain GEMV: only meaningful through this entry point when it brings a decode stream (TMA-fed rings)
+    // prologue 0 + epilogue 0 = a plain GEMV: only meaningful through this entry point when it brings a decode stream (decode_linear.cu)
     if (args->matmul.d_transform & UZU_D_RHT) return false;   // the output transform needs the whole row first: unfused sequence
     if (args->prologue > 3 || args->prologue == 2 || args->epilogue > 1 || (args->prologue == 0 && args->epilogue == 0 && !args->decode_stream)) return false;
     if (args->prologue == 3 && args->epilogue) return false;
