@@ -114,7 +114,15 @@ __device__ __forceinline__ void au_st16(uint32_t taddr, const uint32_t (&v)[16])
                  "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
                  : "memory");
 }
-__device__ __forceinline__ void au_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// nothing that uses what was asked for is done before the wait
+__device__ __forceinline__ void au_wait_ld(uint32_t (&v)[32]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]),
+                   "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]), "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]),
+                   "+r"(v[22]), "+r"(v[23]), "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
+                 :
+                 : "memory");
+}
 __device__ __forceinline__ void au_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ uint32_t au_pack(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
@@ -224,7 +232,7 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
             au_fence_after();
             uint32_t raw[32];
             au_ld32(s_col + side * 32u, raw);
-            au_wait_ld();
+            au_wait_ld(raw);
             float2 s[16];
             const bool part = (i + 1) * AU_KEYS > whole;                     // (rows past the last one sum what nobody reads)
             const uint32_t key0 = i * AU_KEYS + side * 32u;
@@ -259,7 +267,7 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
                 for (uint32_t c = side * (S::OUT / 2); c < (side + 1) * (S::OUT / 2); c += 32) {
                     uint32_t v[32];
                     au_ld32(tmem + lanes + S::O_COL + c, v);
-                    au_wait_ld();
+                    au_wait_ld(v);
 #pragma unroll
                     for (uint32_t j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * factor);
                     au_st32(tmem + lanes + S::O_COL + c, v);
@@ -387,7 +395,7 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
     auto read_o = [&](uint32_t c, float (&v)[32]) {
         uint32_t raw[32];
         au_ld32(tmem + ((warp & 3u) << 21) + S::O_COL + c, raw);
-        au_wait_ld();
+        au_wait_ld(raw);
 #pragma unroll
         for (uint32_t j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
     };

@@ -18,7 +18,7 @@
 // CTAs stay for several tiles; where the tiles do not fill the chip (few rows, few features) a cluster of up to 8 CTAs shares a tile's k and adds
 // its partial tiles over distributed shared memory in rank order (the same bits every time).
 // (Tried instead: integer codes as one plane, group scales applied to the partial sums as they leave tensor memory. Half the products, but reading
-// 128 x NT partial sums per 64 k costs more than that: 815 us at the size above.)
+// 128 x NT partial sums per 64 k costs more than that: 815 us at the size above. With eight warps for the sums, chains of 128 k and 4-bit codes it pays: qmm_wide.cu.)
 // Tiles of up to 64 rows of ZeroPoint / Symmetric weights in groups of 64 and more take ONE plane, the integers code - zp (exact in bf16): half the products,
 // half the stores to tensor memory and no scale in the dequant warps. A chain of at most 128 k inside a group is summed unscaled; the epilogue warps (eight
 // for 64 rows) bring each chain to their sums with one rounded multiply-add by its scale. For wider tiles reading 128 x NT sums per 64 k costs more than the
