@@ -42,3 +42,15 @@ def test_copies_and_fills_are_ordered_with_the_contexts_stream():
         text = re.sub(r"//[^\n]*", "", path.read_text())
         assert not re.search(r"\bcudaMemset\s*\(", text), path.name
         assert not re.search(r"\bcudaMemcpy\s*\([^;]*cudaMemcpyDeviceToDevice", text), path.name
+
+
+def test_the_first_launch_of_a_buffer_waits_for_the_buffer_before():
+    """Kernels read ahead of their wait what earlier steps left behind (a decoded row's position, cached rows, recurrent states), and a dependent launch orders nothing
+    before its wait: every launch asks the buffer whether it may be one, and the first one may not."""
+    struct = re.search(r"struct uzu_command_buffer \{.*?\n\};", (CSRC / "common.cuh").read_text(), re.S).group(0)
+    assert re.search(r"bool dependent\(\) const \{ return use_pdl && launches > 0; \}", struct)
+    for path in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh"), *CSRC.glob("*.inl")]):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(r"= cudaLaunchAttributeProgrammaticStreamSerialization", text):
+            guard = text.rfind("if (", 0, m.start())
+            assert text[guard:].startswith("if (cmd->dependent())") and "}" not in text[guard:m.start()], path.name

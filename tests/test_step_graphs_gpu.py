@@ -201,3 +201,20 @@ def test_fed_steps_behind_steps_in_flight(ctx, tmp_path, mode, lookahead):
         eng.decode_device(lookahead - 1)
         eng.reset()
         assert eng.step_host(7) == again
+
+
+@pytest.mark.parametrize("kind", ["llama-512", "qwen-hybrid-512"])
+def test_chained_steps_without_a_graph(ctx, tmp_path, kind):
+    """Steps that follow one another on the device alone, launch by launch as in captured ones: a step's first kernel stands behind the whole step before it. The products of
+    these models have fewer tiles than the chip has room for."""
+    spec = synth.tiny(kind)
+    path = synth.write_model(spec, tmp_path / "m", seed=5)
+    prompt = np.random.default_rng(6).integers(0, spec.vocab_size, 60)
+    logits = []
+    for graph in (True, False):
+        with B.Engine(ctx, path, max_context_length=1024, use_cuda_graph=graph) as eng:
+            eng.set_persistent_decode(False)
+            eng.prefill(prompt)
+            eng.decode_device(300)
+            logits.append(eng.last_logits().copy())
+    assert np.array_equal(*logits)

@@ -444,7 +444,7 @@ static void launch_attn_prefill(uzu_command_buffer* cmd, const uzu_attention_arg
         attr[0].val.clusterDim.z = 1;
         cfg.numAttrs = 1;
     }
-    else if (cmd->use_pdl) {      // (not clusters: started beside the last CTAs of the kernel before, they share SMs that others leave idle, 31 us -> 44 for 16 rows and 2048 keys)
+    else if (cmd->dependent()) {      // (not clusters: started beside the last CTAs of the kernel before, they share SMs that others leave idle, 31 us -> 44 for 16 rows and 2048 keys)
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 1;

@@ -482,7 +482,7 @@ static void launch_attn_umma(uzu_command_buffer* cmd, const AuParams& p, const C
     cfg.stream = cmd->ctx->stream;
     cudaLaunchAttribute attr[1];
     cfg.attrs = attr;
-    if (cmd->use_pdl) {
+    if (cmd->dependent()) {
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 1;

@@ -64,6 +64,10 @@ struct uzu_command_buffer {
     uint64_t launches = 0, number = 0;      // number: of the context's buffers, when encoding starts
     // Programmatic dependent launch for kernels that opt in (set by the engine)
     bool use_pdl = false;
+    // Whether the next launch may start beside its predecessor. A buffer's first one does not: a dependent launch may start when the last kernel of the buffer before
+    // has no CTA left, and only its wait makes that kernel's writes visible, so kernels behind it that read ahead of their own wait (a decoded row's position, rows of
+    // the cache, recurrent states) would read them unordered. Behind an ordinary first launch all that earlier buffers wrote is there.
+    bool dependent() const { return use_pdl && launches > 0; }
 
     void record_error(uzu_status st, const std::string& msg) {
         if (sticky == UZU_OK) {
@@ -92,7 +96,7 @@ inline void launch(uzu_command_buffer* cmd, const char* what, void (*kernel)(KAr
     cfg.dynamicSmemBytes = smem;
     cfg.stream = cmd->ctx->stream;
     cudaLaunchAttribute attr[1];
-    if (cmd->use_pdl) {
+    if (cmd->dependent()) {
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
@@ -142,7 +146,7 @@ struct AttnSequences {
 };
 bool decode_attention_applicable(const uzu_attention_prepare_args& p, const uzu_attention_args& a, const AttnSequences& s);
 // longest: no sequence has more cached rows than that, this step's included (with dynamic positions: at any time the launch is repeated). All rows before this
-// step's, and the positions, were written before the first kernel of the step could start.
+// step's, and the positions, were written before the buffer's first kernel, an ordinary launch, could start.
 void encode_decode_attention(uzu_command_buffer* cmd, const uzu_attention_prepare_args& a, const uzu_qk_norm_config* q_norm, const uzu_qk_norm_config* k_norm, float scale, uint64_t out,
                              const AttnSequences& s, uint32_t longest);
 

@@ -7,8 +7,8 @@
 //   * A warp takes tiles of 16 keys. Scores and the weighted sum are products on mma.sync: the heads of a key head are rows 0..7 of the product, the exact f32
 //     probabilities three bf16 planes, two of them in rows g and g + 8 of one product and the third in a second one. Keys go from memory to registers in the
 //     order of the product's B operand (channels are permuted alike in the query), values are paired by PRMT; neither passes through shared memory.
-//   * The first tile of a warp is read before the kernel waits for its predecessor: every row before this step's is there already (kept by earlier steps, whose last
-//     kernel is an ordinary launch).
+//   * The position and a warp's first tile are read before the kernel waits for its predecessor: what earlier steps wrote is there already, since a step's first
+//     kernel is an ordinary launch (uzu_command_buffer::dependent).
 //   * A cluster of up to eight CTAs shares a key head's keys, each 128 and more; the parts meet in distributed shared memory, in rank order.
 // From the end of the projection, Llama-3-8B at 2048 tokens: 18.5 us a layer before, 8.6 now; Qwen3.5-0.8B at 500 (heads of 256, normed): 22, 10.8. What is left are some
 // 2000 instructions of eight warps, one after another, and the trips to the row, to distributed shared memory and back.
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
     float* all_ml = weights + DA_WARPS * G;                                               // [ranks][G][2]: of the cluster
     float* slices = all_ml + ((p.ranks * G * 2 + 3u) & ~3u);                               // [ranks][slice]: this rank's outputs, of every rank
 
-    // (a word that only the last kernel of a step writes, an ordinary launch: it is there before any kernel of this step starts)
+    // (a word that only the last kernel of a step writes: it is there before the second kernel of this step starts, since the first is an ordinary launch)
     // (asm: of a plain load and the parameter the compiler makes one load from either address, and a parameter has none that such a load may take)
     uint32_t position = seqs.prefix[b], rope_row = seqs.position[b];
     if (p.positions) {
@@ -382,7 +382,7 @@ static void launch_decode_attention(uzu_command_buffer* cmd, const DecodeAttnPar
     attr[0].val.clusterDim.x = p.ranks;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
     cfg.numAttrs = 1;
-    if (cmd->use_pdl) {
+    if (cmd->dependent()) {
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs = 2;

@@ -584,7 +584,7 @@ void qs_launch(uzu_command_buffer* cmd, const CUtensorMap& w, const CUtensorMap&
     cfg.dynamicSmemBytes = QsShape<NT, PL>::SMEM;
     cfg.stream = cmd->ctx->stream;
     cudaLaunchAttribute attr[2];
-    if (cmd->use_pdl) {
+    if (cmd->dependent()) {
         attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }

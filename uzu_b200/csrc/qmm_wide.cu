@@ -407,7 +407,7 @@ static void qw_launch(uzu_command_buffer* cmd, const CUtensorMap& mw, const CUte
     cfg.dynamicSmemBytes = QW_SMEM;
     cfg.stream = cmd->ctx->stream;
     cudaLaunchAttribute attr[1];
-    if (cmd->use_pdl) {
+    if (cmd->dependent()) {
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
