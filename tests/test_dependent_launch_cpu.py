@@ -54,3 +54,12 @@ def test_the_first_launch_of_a_buffer_waits_for_the_buffer_before():
         for m in re.finditer(r"= cudaLaunchAttributeProgrammaticStreamSerialization", text):
             guard = text.rfind("if (", 0, m.start())
             assert text[guard:].startswith("if (cmd->dependent())") and "}" not in text[guard:m.start()], path.name
+
+
+@pytest.mark.parametrize("body", [pytest.param(p.values[0], id=p.id) for p in _kernels() if "tcgen05.alloc" in p.values[0]])
+def test_tensor_memory_is_taken_before_dependents_may_start(body):
+    """A dependent's CTA beside this one could take the tensor memory that this one still waits for, and wait itself for this kernel's end. One thread's call lets
+    dependents start: it stands behind the barrier that every warp passes once the memory is there."""
+    if "pdl_launch_dependents" in body:
+        taken = body.index("tcgen05.alloc")
+        assert body.index("__syncthreads", taken) < body.index("pdl_launch_dependents") < body.index("tcgen05.dealloc")

@@ -145,11 +145,11 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(qs_smem(&tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    pdl_launch_dependents();
     qs_fence_before();
     __syncthreads();
     qs_fence_after();
     const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();      // (not before this CTA has its tensor memory: a dependent's CTA that took it would wait for this one)
 
     // this CTA's work: items blockIdx.x / splits, then in steps of the grid; the k blocks of its rank
     const uint32_t rank = p.splits > 1 ? blockIdx.x % p.splits : 0u, item0 = blockIdx.x / p.splits, item_step = gridDim.x / p.splits;

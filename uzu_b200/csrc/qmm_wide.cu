@@ -136,11 +136,11 @@ __global__ void __launch_bounds__(QW_THREADS, 1) qmm_wide_kernel(const __grid_co
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(qs_smem(&tmem_slot)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    pdl_launch_dependents();
     qs_fence_before();
     __syncthreads();
     qs_fence_after();
     const uint32_t tmem = tmem_slot;
+    pdl_launch_dependents();      // (not before this CTA has its tensor memory: a dependent's CTA that took it would wait for this one)
     // neighbouring items share their weights: the row tiles of a feature tile are in flight together
     auto item_n = [&](uint32_t item) { return item / p.m_tiles * 128u; };
     auto item_m = [&](uint32_t item) { return item % p.m_tiles * w.width; };
