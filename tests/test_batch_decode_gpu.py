@@ -153,3 +153,22 @@ def test_a_batch_samples_greedily_whatever_the_engines_own_sequence_does(ctx, tm
             for step in range(40):                  # lengths that share a captured step and lengths that do not
                 got = eng.batch_step([1, 2, 3])
                 assert got == largest(eng.batch_logits()), (step, sampling)
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_more_slots_than_a_batched_step_takes(ctx, tmp_path, graph):
+    """Sequence slots lie in the batch's list, and there may be 64 of them: a batched step over more than 16 is refused before anything is written."""
+    spec = synth.tiny("llama", layers=1)
+    path = synth.write_model(spec, tmp_path / "m", seed=42)
+    with B.Engine(ctx, path, max_context_length=64, use_cuda_graph=graph) as eng:
+        slots = [eng.slot_acquire() for _ in range(17)]
+        eng._batch = 17
+        for call in (lambda: eng.batch_step([1] * 17), eng.batch_logits, lambda: eng.batch_decode_timed([1] * 17, 2)):
+            with pytest.raises(B.UzuError, match="at most 16"):
+                call()
+        for s in slots:
+            eng.slot_release(s)
+        eng.batch_begin(2)
+        firsts = [eng.batch_prefill(b, [3, 1, 4]) for b in range(2)]
+        got = eng.batch_step(firsts)
+        assert firsts[0] == firsts[1] and got[0] == got[1]

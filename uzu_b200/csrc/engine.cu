@@ -2618,6 +2618,7 @@ static void upload_decode_state(uzu_engine* e, bool set_token, uint64_t token_fr
 
 static void set_tokens(uzu_engine* e, const uint32_t* tokens, uint32_t count) {
     TokenValues v{};
+    if (count > sizeof v.t / sizeof v.t[0]) throw std::runtime_error("at most 16 tokens of a step");
     memcpy(v.t, tokens, count * 4);
     set_tokens_kernel<<<1, 32, 0, e->ctx->stream>>>((uint32_t*)e->token_ids.ptr(), v, count);
 }
@@ -3158,6 +3159,14 @@ static StepGraph& capture_batch_graph(uzu_engine* e, uint32_t bucket) {
     return e->batch_graphs.back();
 }
 
+// Sequences of a batched step: batch_begin makes at most 16, but sequence slots lie in the same list, up to 64 of them.
+static uint32_t batch_sequences(const uzu_engine* e, const char* what) {
+    const size_t n = e->seqs.size();
+    if (n == 0) throw std::runtime_error(std::string(what) + ": batch_begin first");
+    if (n > 16) throw std::runtime_error(std::string(what) + ": at most 16 sequences (" + std::to_string(n) + " sequence slots are there)");
+    return (uint32_t)n;
+}
+
 // one step for all sequences; the sampled tokens are chained into token_ids on the device (next step's inputs)
 static void run_batch_step(uzu_engine* e, bool chain) {
     const uint32_t B = (uint32_t)e->seqs.size();
@@ -3366,8 +3375,8 @@ uzu_status uzu_engine_batch_prefill(uzu_engine* e, uint32_t sequence, const uint
 
 uzu_status uzu_engine_batch_step(uzu_engine* e, const uint32_t* tokens_in, uint32_t* tokens_out) {
     UZU_ENGINE_TRY({
-        const uint32_t B = (uint32_t)e->seqs.size();
-        if (B == 0 || !tokens_in) throw std::runtime_error("batch_step: batch_begin first / null tokens");
+        const uint32_t B = batch_sequences(e, "batch_step");
+        if (!tokens_in) throw std::runtime_error("batch_step: null tokens");
         uint32_t* said = (uint32_t*)uzu_buffer_cpu_ptr(e->host_tokens.b) + MAX_ROWS + 16;
         set_tokens(e, tokens_in, B);
         run_batch_step(e, false);
@@ -3380,8 +3389,8 @@ uzu_status uzu_engine_batch_step(uzu_engine* e, const uint32_t* tokens_in, uint3
 
 uzu_status uzu_engine_batch_decode_timed(uzu_engine* e, const uint32_t* first_tokens, uint32_t steps, double* out_seconds) {
     UZU_ENGINE_TRY({
-        const uint32_t B = (uint32_t)e->seqs.size();
-        if (B == 0 || !first_tokens || steps == 0) throw std::runtime_error("batch_decode_timed: batch_begin first / null tokens / zero steps");
+        const uint32_t B = batch_sequences(e, "batch_decode_timed");
+        if (!first_tokens || steps == 0) throw std::runtime_error("batch_decode_timed: null tokens / zero steps");
         cudaStream_t s = e->ctx->stream;
         uint32_t* staging = (uint32_t*)uzu_buffer_cpu_ptr(e->host_tokens.b);
         memcpy(staging, first_tokens, B * 4);
@@ -3404,9 +3413,10 @@ uzu_status uzu_engine_batch_decode_timed(uzu_engine* e, const uint32_t* first_to
 
 uzu_status uzu_engine_batch_logits(uzu_engine* e, uint16_t* out_logits) {
     UZU_ENGINE_TRY({
-        if (e->seqs.empty() || !out_logits) throw std::runtime_error("batch_logits: batch_begin first / null output");
+        const uint32_t B = batch_sequences(e, "batch_logits");
+        if (!out_logits) throw std::runtime_error("batch_logits: null output");
         cudaStreamSynchronize(e->ctx->stream);
-        cudaMemcpy(out_logits, (void*)e->logits.ptr(), e->seqs.size() * (size_t)e->vocab * 2, cudaMemcpyDeviceToHost);
+        cudaMemcpy(out_logits, (void*)e->logits.ptr(), B * (size_t)e->vocab * 2, cudaMemcpyDeviceToHost);
     });
 }
 
