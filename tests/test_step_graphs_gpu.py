@@ -218,3 +218,31 @@ def test_chained_steps_without_a_graph(ctx, tmp_path, kind):
             eng.decode_device(300)
             logits.append(eng.last_logits().copy())
     assert np.array_equal(*logits)
+
+
+def test_engines_of_two_threads_on_one_core(tmp_path):
+    """A fed step watches for its token in host memory; another engine's thread on the same core comes to its turn all the same."""
+    import os
+    import threading
+    spec = synth.tiny("llama", layers=1)
+    path = synth.write_model(spec, tmp_path / "m", seed=12)
+    out = {}
+
+    def run(name, core=None):
+        if core is not None:
+            os.sched_setaffinity(0, {core})      # (of this thread)
+        with B.Context(0) as own, B.Engine(own, path, max_context_length=1024) as eng:
+            eng.set_persistent_decode(False)
+            token, out[name] = eng.prefill(np.arange(5)), []
+            for _ in range(200):
+                token = eng.step_host(token)
+                out[name].append(token)
+
+    core = min(os.sched_getaffinity(0))
+    for names, where in ((["alone"], None), (["a", "b"], core)):
+        threads = [threading.Thread(target=run, args=(n, where)) for n in names]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(60)
+    assert len(out["alone"]) == 200 and out["a"] == out["b"] == out["alone"]

@@ -31,6 +31,7 @@
 #include <memory>
 #include <set>
 #include <sstream>
+#include <thread>
 #include <vector>
 
 #include "common.cuh"
@@ -2975,8 +2976,11 @@ uzu_status uzu_engine_step_host(uzu_engine* e, uint32_t token_in, uint32_t* toke
         set_tokens(e, &token_in, 1);
         issue_decode_step(e, 0, 0);
         cudaError_t err = cudaErrorNotReady;
-        for (uint32_t i = 1; *place == 0xFFFFFFFFu && err == cudaErrorNotReady; ++i)
+        for (uint32_t i = 1; *place == 0xFFFFFFFFu && err == cudaErrorNotReady; ++i) {
+            __builtin_ia32_pause();
+            if (i % 64 == 0) std::this_thread::yield();      // (engines on few cores: the thread that has something to encode comes first)
             if (i % 1024 == 0) err = cudaStreamQuery(s);
+        }
         if (err != cudaErrorNotReady && err != cudaSuccess) throw std::runtime_error(std::string("step_host: ") + cudaGetErrorString(err));
         const uint32_t tok = *place;
         e->ring_busy = false;
