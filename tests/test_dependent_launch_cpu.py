@@ -63,3 +63,12 @@ def test_tensor_memory_is_taken_before_dependents_may_start(body):
     if "pdl_launch_dependents" in body:
         taken = body.index("tcgen05.alloc")
         assert body.index("__syncthreads", taken) < body.index("pdl_launch_dependents") < body.index("tcgen05.dealloc")
+
+
+def test_scores_are_not_written_over_weights_that_products_still_read():
+    """attention_umma.cu: scores that go where weights of an earlier tile were wait for that tile's products, or go elsewhere. (Only products of the same shape into the
+    same sum are in order by themselves.)"""
+    text = re.sub(r"//[^\n]*", "", (CSRC / "attention_umma.cu").read_text())
+    issue = text[text.index("if (i + 1 < tiles)"):text.index("au_commit(o_done)")]
+    over = "tmem + s * 64u + pl * 32u" in issue                        # weights in the columns of scores
+    assert not over or issue.index("au_wait(o_done") < issue.index("scores(i + 1)")

@@ -370,7 +370,11 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
         if (ok) scores(0);
         for (uint32_t i = 0; i < tiles && ok; ++i) {
             const uint32_t s = i & 1u;
-            if (i + 1 < tiles) scores(i + 1);
+            if (i + 1 < tiles) {
+                // (they go where the weights of tile i - 1 are: products of another shape and sum are not in order with those that read them)
+                if (i) ok = au_wait(o_done, (i - 1) & 1u, &gave_up, p.error, 0x506u);
+                if (ok) scores(i + 1);
+            }
             if (ok) ok = au_wait(p_full(s), i >> 1 & 1u, &gave_up, p.error, 0x509u);
             if (ok) ok = au_wait(v_full(s), i >> 1 & 1u, &gave_up, p.error, 0x50au);
             if (!ok) break;
