@@ -5,7 +5,7 @@ import pytest
 
 from tests import gpu_ops as G
 from tests import test_prefill_attention_gpu as P
-from tests.util import bf16_to_f32, f32_to_bf16
+from tests.util import bf16_to_f32, f32_to_bf16, off_the_rounding
 
 pytestmark = [pytest.mark.gpu]
 
@@ -61,3 +61,24 @@ def test_against_64_bits(umma, H, Hkv, prefix, suffix, D, causal, grows):
     got = bf16_to_f32(got).astype(np.float64).reshape(want.shape)
     # one rounding to bf16, 2^-9 of a result on average and 2^-8 at most; weights of 16 bits and scores in f32 (2^-22 of up to 60 in the exponent) add 2^-16 of the values' size, about 5
     assert (np.abs(got - want) <= 2.0 ** -8 * np.abs(want) + 5 * 2.0 ** -14).all(), np.abs(got - want).max()
+
+
+@pytest.mark.parametrize("H,Hkv,prefix,suffix,D,before", [(8, 2, 1500, 512, 256, 0), (8, 2, 64, 64, 256, 0), (32, 8, 1100, 256, 128, 1), (32, 8, 600, 512, 64, 1)])
+def test_no_further_off_than_the_kernel_before(ctx, H, Hkv, prefix, suffix, D, before):
+    """Results that are not the correctly rounded ones: with three planes no more than of the split-KV kernel, whose weights and sums are f32 (0), with two no more than of
+    the mma.sync kernel, which has as many (1). (Sums of all keys in tensor memory, which cuts off what it adds, had half as many again and more.)"""
+    rng = np.random.default_rng(D + suffix)
+    n, off, count = prefix + suffix, [0, 0], 0
+    while count < 1 << 20:
+        q, k, v = (f32_to_bf16(rng.standard_normal(s).astype(np.float32)) for s in ((H, suffix, D), (n, Hkv * D), (n, Hkv * D)))
+        want = _reference(q, k, v, H, Hkv, prefix, suffix, D, True, D ** -0.5)
+        count += want.size
+        for i, mode in enumerate((before, 2)):
+            ctx.lib.uzu_debug_set_prefill_attention(mode)
+            try:
+                got = G.attention_single_pass(ctx, q, k, v, head_dim=D, gqa_factor=H // Hkv, sequence_length=n, k_head_stride=D, k_seq_stride=Hkv * D, v_head_stride=D,
+                                              v_seq_stride=Hkv * D, scale=float(D ** -0.5), num_heads=H, suffix_length=suffix)
+            finally:
+                ctx.lib.uzu_debug_set_prefill_attention(-1)
+            off[i] += off_the_rounding(got, want)
+    assert off[1] <= off[0] + 4 * sum(off) ** 0.5, off      # (four standard deviations of the two counts)

@@ -48,3 +48,16 @@ def assert_f32_close(got, ref, *, rtol=1e-3, atol=1e-4, what=""):
     tol = atol * scale + rtol * np.abs(ref)
     bad = err > tol
     assert not bad.any(), f"{what}: {bad.sum()} / {bad.size} elements outside rtol={rtol} atol={atol}; max err {err.max()}"
+
+
+def off_the_rounding(got, want64):
+    """how many bf16 results are not the 64-bit ones rounded once"""
+    return int((np.asarray(got, np.uint16).reshape(want64.shape) != f32_to_bf16_of_f64(want64)).sum())
+
+
+def f32_to_bf16_of_f64(x):
+    """64-bit numbers rounded once to bf16 (by way of f32 a second rounding could turn a tie)"""
+    down = np.ascontiguousarray(x, np.float32)
+    down = np.where(np.abs(down.astype(np.float64)) > np.abs(x), np.nextafter(down, np.float32(0)), down).view(np.uint32)      # towards zero
+    down = np.where((down & 0xFFFF == 0x8000) & (np.abs(down.view(np.float32).astype(np.float64)) < np.abs(x)), down + 1, down)  # (just above a tie: sticky)
+    return ((down + 0x7FFF + ((down >> 16) & 1)) >> 16).astype(np.uint16)

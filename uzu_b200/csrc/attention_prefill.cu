@@ -394,10 +394,10 @@ static bool pa_two_planes(const uzu_attention_args& a) { return a.suffix_length 
 // 41 / 15. 8 heads of 256, 64 tokens alone 10.7 / 27, behind 1000 73 / 28. Fewer than 8 tokens stay with the split-KV kernel: 4 behind 200 take 12.4 / 14.5,
 // behind 1000 19 / 14.5, behind 4096 45 / 37.
 // The tcgen05 kernel (attention_umma.cu) walks the keys in CTAs of 128 rows that share nothing: the chip has to be filled by the rows. Fitted to 720 sizes (16 to 1024
-// tokens, 0 to 6000 cached rows), within 10 % for nine in ten, so that it is taken where it is the faster by a sixth. This one / that one: 32 heads of 128 in groups
-// of 4, 64 tokens behind 100 16.4 / 13.4, behind 1100 20.4 / 25.9 (its keys are split, that one's not), 256 behind 1100 42.9 / 28.7, 1024 behind 1100 167 / 48; of 64,
-// 1024 behind 1100 92 / 43; 8 heads of 256 in groups of 4, 256 behind 1100 38.2 / 38.7, 400 57 / 41, 1024 128 / 53. In place of the split-KV kernel, whose weights
-// are f32, it has to have three planes: 8 heads of 256, 100 tokens behind 100 21.7 / 16.5.
+// tokens, 0 to 6000 cached rows), within 10 % for nine in ten, so that it is taken where it is the faster by a sixth (none of the 720 is then slower). This one / that
+// one: 32 heads of 128 in groups of 4, 64 tokens behind 100 16.2 / 12.3, behind 1100 20.3 / 27.2 (its keys are split, that one's not), 256 behind 1100 44.1 / 30.7, 1024
+// behind 1100 168 / 74; of 64, 1024 behind 1100 92 / 53; 8 heads of 256 in groups of 4, 256 behind 1100 38.4 / 38.2, 400 58 / 41, 1024 128 / 52. In place of the
+// split-KV kernel, whose weights are f32, it has to have three planes: 8 heads of 256, 100 tokens behind 100 21.6 / 16.4.
 enum class PaKernel { Split, Mma, Umma };
 static PaKernel pa_choose(const uzu_attention_args& a, uint32_t sms) {
     const uint32_t D = a.head_dim, rows = a.suffix_length, keys = a.sequence_length, gq = a.gqa_factor, g = gq % 8 == 0 ? 8 : gq % 4 == 0 ? 4 : gq % 2 == 0 ? 2 : 1;
@@ -417,9 +417,10 @@ static PaKernel pa_choose(const uzu_attention_args& a, uint32_t sms) {
     const float mma = start * (0.5f + 0.5f * turns) + tile * per * turns + merge;
     const bool split_is_faster = mma >= split;
     if (!attn_umma_applicable(a) || (split_is_faster && (two || rows <= 16))) return split_is_faster ? PaKernel::Split : PaKernel::Mma;
-    const uint32_t u_ctas = (rows * gq + 127) / 128 * kv_heads * (D == 256 ? 2u : 1u), u_sm = D == 256 || (D == 128 && !two) ? 1u : 2u, u_turns = std::max(1u, (u_ctas + sms * u_sm - 1) / (sms * u_sm));
-    const float u_tile = (D == 64 ? 0.73f : D == 128 ? 0.81f : 1.27f) * u_turns + (u_sm == 2 && u_ctas > sms ? (D == 64 ? 0.24f : 0.33f) : 0.0f);
-    const float umma = (D == 64 ? 4.0f + 4.0f * u_turns : 9.7f) + u_tile * key_tiles * (D != 256 && !two ? 1.3f : 1.0f);
+    const uint32_t u_ctas = (rows * gq + 127) / 128 * kv_heads * (D == 256 ? 2u : 1u), u_room = sms * (D == 64 ? 2u : 1u), u_turns = std::max(1u, (u_ctas + u_room - 1) / u_room);
+    const float u_start = D == 64 ? 19.7f - 12.3f * u_turns : D == 128 ? 11.4f - 2.4f * u_turns : 16.3f - 5.5f * u_turns;
+    const float u_tile = (D == 64 ? 1.03f : D == 128 ? 0.97f : 1.2f) * u_turns + (D == 64 && u_ctas > sms ? 0.26f : 0.0f);
+    const float umma = u_start + u_tile * key_tiles * (D != 256 && !two ? 1.1f : 1.0f);
     if (1.2f * umma < std::min(mma, split)) return PaKernel::Umma;
     return split_is_faster ? PaKernel::Split : PaKernel::Mma;
 }

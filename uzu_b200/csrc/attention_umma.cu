@@ -3,19 +3,23 @@
 // What bounded the kernel before it (attention_prefill.cu, still the one for what this does not take): mma.sync has a quarter of this pipe's rate, and its four warps
 // reached a third of that. Here a CTA has 128 rows, (token, head) pairs of a key head, two threads of eight softmax warps each, one warp that copies and one that issues:
 //   copy    keys and values by TMA, 64 keys a stage, two stages, 64 channels a block of 128-byte swizzled rows (keys past the last are not read: zeros).
-//   issue   S = Q K^T into tensor memory (two tiles of 64 columns in turn), then O += P V with P as operand A there: two or three bf16 planes, as many as the kernel
+//   issue   S = Q K^T into tensor memory, 64 columns for every 64 channels, then a tile's P V with P as operand A there: two or three bf16 planes, as many as the kernel
 //           before has, so that the f32 weights are exact to 16 bits or whole. Values are operand B as they lie (N-major).
-//   softmax a thread reads 32 of its row's 64 scores, the two tell each other their maxima, and it writes its planes over them. O stays in tensor memory: it is
-//           rescaled only where a row's maximum has grown by more than 2^8, so that weights reach 256 at most; sums and the division are f32.
-// Up to 128 channels two CTAs share an SM, one's products run beside the other's softmax. Of 256 channels a CTA sums one half (grid z), so that the prompts of few
-// heads fill the chip. What bounds it now: a product of 128 x 64 x 16 takes the pipe 50 cycles (32 at its rate) and of 128 x 128 x 16 58, a tile of 256 channels 815
-// for the scores and 700 for the values of 2250 in all, the rest waits for keys and softmax; tiles of 128 keys fill the pipe better, but the 64 scores
-// of a thread spilled, and that was slower.
-// 1024 tokens behind 1100 rows, before -> now: 8 heads of 256 in groups of 4 128 -> 53 us, 32 of 128 167 -> 48, 32 of 64 92 -> 43.
+//   softmax a thread reads 32 of its row's 64 scores, the two tell each other their maxima, and it writes its planes. The tile before is added to O, half of it in each
+//           thread's registers; it is rescaled only where a row's maximum has grown by more than 2^8, so that weights reach 256 at most.
+// The pipe cuts what it adds to an accumulator off at its last bit. So no chain is longer than 64 channels or the products of a tile, the smallest plane first, and the
+// chains are added by rounded additions: with three planes 1.4 to 2.1 results in 10000 are off the correct rounding (split-KV, all f32, 1.8 to 4.7; mma.sync 2.3 to 2.9;
+// 33 with whole chains in tensor memory), with two 24 to 25 (mma.sync 23 to 30, whole chains 29 to 31).
+// Of 64 channels two CTAs share an SM, one's products run beside the other's softmax (and a thread spills 370 bytes for it); of more, the sums take the registers. Of 256
+// channels a CTA sums one half (grid z), so that the prompts of few heads fill the chip. What bounds it now: the softmax warps' way through a tile, 1900 cycles of 128
+// channels and 2300 of 256 (exponentials 750, planes 300, the waits for scores, for the tile before and for stores 140 each); products take 860 and 1500 of them. Four
+// threads a row instead of two changed nothing.
+// 1024 tokens behind 1100 rows, before -> now: 8 heads of 256 in groups of 4 128 -> 52 us, 32 of 128 168 -> 74, 32 of 64 92 -> 53 (with O in tensor memory, two CTAs an
+// SM: 53, 48, 43).
 // (Accumulators start at multiples of 128 columns, scores at multiples of 64. A form with score tiles 96 columns apart, 256 channels a CTA and clusters that shared the
 // keys of a row tile ended in an illegal memory access whose cause was not found; none of the three is built.)
-// A value that is not finite behind a mask would make NaN of a weight of zero: tiles that some row does not see whole are looked over, and a CTA that met one
-// computes its rows again key by key.
+// A value that is not finite makes NaN of a weight of zero, in whole or in one of its planes: a row whose sums are not finite, its weights being so, is computed again
+// key by key, each only where it is seen.
 // Every barrier wait is bounded (wait_errors.h).
 #include <cuda.h>
 
@@ -38,15 +42,20 @@ template <int D, int PLANES>
 struct AuShape {
     static constexpr uint32_t OUT = D < 128 ? D : 128;                       // channels of O that a CTA sums
     static constexpr uint32_t Q_BLOCK = AU_ROWS * 128, KV_BLOCK = AU_KEYS * 128, Q = D / 64 * Q_BLOCK, K = D / 64 * KV_BLOCK, V = OUT / 64 * KV_BLOCK;
-    static constexpr uint32_t CTAS = D == 256 || (D == 128 && PLANES == 3) ? 1 : 2;      // of an SM
-    // tensor memory: two score tiles of 64 columns, two planes over each; O; the third planes
-    static constexpr uint32_t COLUMNS = CTAS == 1 ? 512 : 256, O_COL = 128, THIRD = D == 64 ? 192 : 256;
+    static constexpr uint32_t CTAS = D == 64 ? 2 : 1;      // of an SM
+    // tensor memory: scores, 64 columns for every 64 channels; a tile's products; the planes of its weights
+    static constexpr uint32_t COLUMNS = 512 / CTAS, O_COL = 256 / CTAS;
+    static constexpr __host__ __device__ uint32_t plane(uint32_t i) { return CTAS == 1 ? 384 + 32 * i : i < 2 ? 64 + 32 * i : 192; }
     static constexpr size_t SMEM = Q + 2 * K + 2 * V + 1024;
 };
 
 __device__ __forceinline__ uint32_t au_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void au_init(uint32_t bar, uint32_t count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory"); }
-__device__ __forceinline__ void au_arrive(uint32_t bar) { asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(bar) : "memory"); }
+// (a whole warp, for all its lanes)
+__device__ __forceinline__ void au_arrive(uint32_t bar) {
+    __syncwarp();
+    if ((threadIdx.x & 31u) == 0) asm volatile("{ .reg .b64 st; mbarrier.arrive.shared::cta.b64 st, [%0]; }" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ bool au_try(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000u) : "memory");
@@ -101,14 +110,6 @@ __device__ __forceinline__ void au_ld32(uint32_t taddr, uint32_t (&v)[32]) {
         : "r"(taddr)
         : "memory");
 }
-__device__ __forceinline__ void au_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]),
-        "r"(v[31])
-        : "memory");
-}
 __device__ __forceinline__ void au_st16(uint32_t taddr, const uint32_t (&v)[16]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
                  "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
@@ -146,15 +147,48 @@ __device__ __forceinline__ float au_exp2(float x) {      // 2 ulp, as exp2f; wei
 }
 __device__ __forceinline__ float au_lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float au_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+struct AuRow {
+    const __nv_bfloat16 *query, *keys, *values;
+    __nv_bfloat16* out;
+    const uzu_trie_node* nodes;      // null: no trie
+    uint64_t k_stride, v_stride;
+    uint32_t token, lim, prefix, kend;
+    float scale2;
+};
+// 32 channels of a row key by key, each key only where it is seen: slow, for sums of values that are not finite
+template <int D>
+__device__ __noinline__ void au_row_by_key(const AuRow r) {
+#pragma unroll 1
+    for (uint32_t c = 0; c < 32; c += 16) {
+        float o[16], most = -INFINITY, total = 0.0f;
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j) o[j] = 0.0f;
+#pragma unroll 1
+        for (uint32_t key = 0; key < r.kend; ++key) {
+            if (key >= r.lim && !(r.nodes && key >= r.prefix && r.token >= r.nodes[key - r.prefix].trie_start && r.token <= r.nodes[key - r.prefix].trie_end)) continue;
+            float s = 0.0f;
+            for (uint32_t d = 0; d < D; ++d) s = fmaf(bf2f(r.query[d]), bf2f(r.keys[key * r.k_stride + d]), s);
+            s *= r.scale2;
+            const float next = fmaxf(most, s), from = next == -INFINITY ? 0.0f : next, keep = exp2f(most - from), w = exp2f(s - from);
+            total = total * keep + w;
+            most = next;
+#pragma unroll
+            for (uint32_t j = 0; j < 16; ++j) o[j] = fmaf(w, bf2f(r.values[key * r.v_stride + c + j]), o[j] * keep);
+        }
+        const float inv = total > 0.0f ? 1.0f / total : 0.0f;
+#pragma unroll
+        for (uint32_t j = 0; j < 16; ++j) r.out[c + j] = f2bf(o[j] * inv);
+    }
+}
 }  // namespace
 
 template <int D, int PLANES>
 __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const AuParams p) {
     using S = AuShape<D, PLANES>;
     extern __shared__ uint8_t au_raw[];
-    __shared__ __align__(8) uint64_t bars[14];
+    __shared__ __align__(8) uint64_t bars[13];
     __shared__ uint32_t tmem_slot;
-    __shared__ volatile uint32_t gave_up, not_finite;
+    __shared__ volatile uint32_t gave_up;
     __shared__ float row_max[2][2][AU_ROWS], row_sum[2][AU_ROWS];      // [tile][side][row]: what the two threads of a row tell each other
     const uzu_attention_args& a = p.a;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -165,9 +199,7 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
     auto k_empty = [&](uint32_t s) { return bar0 + 8u * (3 + s); };
     auto v_full = [&](uint32_t s) { return bar0 + 8u * (5 + s); };
     auto v_empty = [&](uint32_t s) { return bar0 + 8u * (7 + s); };
-    auto s_full = [&](uint32_t s) { return bar0 + 8u * (9 + s); };
-    auto p_full = [&](uint32_t s) { return bar0 + 8u * (11 + s); };
-    const uint32_t o_done = bar0 + 8u * 13;
+    const uint32_t s_full = bar0 + 8u * 9, s_empty = bar0 + 8u * 10, p_full = bar0 + 8u * 11, o_done = bar0 + 8u * 12;
 
     const uint32_t G = a.gqa_factor, m = a.suffix_length, seq = a.sequence_length, prefix = seq - m, rows = m * G, half = blockIdx.z * S::OUT;      // half: the first of this CTA's channels
     const uint32_t row0 = (gridDim.x - 1u - blockIdx.x) * AU_ROWS, kvh = blockIdx.y;      // the rows with the most keys first
@@ -178,13 +210,12 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
 
     if (warp == 0) {
         if (lane == 0) {
-            au_init(q_full, AU_SOFT);
+            au_init(q_full, AU_SOFT / 32);
             for (uint32_t s = 0; s < 2; ++s) {
-                au_init(k_full(s), 1); au_init(k_empty(s), 1); au_init(v_full(s), 1); au_init(v_empty(s), 1); au_init(s_full(s), 1); au_init(p_full(s), AU_SOFT);
+                au_init(k_full(s), 1); au_init(k_empty(s), 1); au_init(v_full(s), 1); au_init(v_empty(s), 1);
             }
-            au_init(o_done, 1);
+            au_init(s_full, 1); au_init(s_empty, AU_SOFT / 32); au_init(p_full, AU_SOFT / 32); au_init(o_done, 1);
             gave_up = 0;
-            not_finite = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
         __syncwarp();
@@ -209,7 +240,22 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
     };
     const float scale2 = a.scale * 1.4426950408889634f;
     float top = -INFINITY, sum = 0.0f;                                   // of the row: what its weights are relative to (in units of ln 2), their sum
+    constexpr uint32_t MINE = S::OUT / 2;                                // columns of this thread
+    float acc[MINE];
+#pragma unroll
+    for (uint32_t j = 0; j < MINE; ++j) acc[j] = 0.0f;
     bool ok = true;
+    // a tile's products to the sums, by rounded additions (its weights are relative to the row's maximum at that time)
+    auto add_tile = [&]() {
+#pragma unroll
+        for (uint32_t c = 0; c < MINE; c += 32) {
+            uint32_t v[32];
+            au_ld32(tmem + ((warp & 3u) << 21) + S::O_COL + side * MINE + c, v);
+            au_wait_ld(v);
+#pragma unroll
+            for (uint32_t j = 0; j < 32; ++j) acc[c + j] += __uint_as_float(v[j]);
+        }
+    };
 
     if (warp < 8) {
         // ================================ softmax ================================
@@ -226,18 +272,25 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
         const uint32_t lanes = (warp & 3u) << 21, pair = 1u + (warp & 3u);      // pair: the barrier of the two warps of 32 rows
         auto leave = [&]() { asm volatile("bar.arrive %0, 64;" ::"r"(pair) : "memory"); };      // a wait ran out: the other warp is not left waiting
         for (uint32_t i = 0; i < tiles; ++i) {
-            const uint32_t b = i & 1u, s_col = tmem + lanes + b * 64u;
-            if (ok) ok = au_wait(s_full(b), i >> 1 & 1u, &gave_up, p.error, 0x501u);
+            if (ok) ok = au_wait(s_full, i & 1u, &gave_up, p.error, 0x501u);
             if (!ok) { leave(); break; }
             au_fence_after();
-            uint32_t raw[32];
-            au_ld32(s_col + side * 32u, raw);
-            au_wait_ld(raw);
             float2 s[16];
+#pragma unroll
+            for (uint32_t c = 0; c < D / 64; ++c) {                          // the sums over 64 channels each
+                uint32_t raw[32];
+                au_ld32(tmem + lanes + c * 64u + side * 32u, raw);
+                au_wait_ld(raw);
+#pragma unroll
+                for (uint32_t j = 0; j < 16; ++j) {
+                    const float2 x = make_float2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]));
+                    s[j] = c ? au_add2(s[j], x) : x;
+                }
+            }
+            au_fence_before();
+            au_arrive(s_empty);
             const bool part = (i + 1) * AU_KEYS > whole;                     // (rows past the last one sum what nobody reads)
             const uint32_t key0 = i * AU_KEYS + side * 32u;
-#pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) s[j] = make_float2(__uint_as_float(raw[2 * j]), __uint_as_float(raw[2 * j + 1]));
             if (part) {
 #pragma unroll
                 for (uint32_t j = 0; j < 16; ++j) {
@@ -250,29 +303,12 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
             for (uint32_t j = 0; j < 16; ++j) mosts[j & 3u] = fmaxf(mosts[j & 3u], fmaxf(s[j].x, s[j].y));
             float most = fmaxf(fmaxf(mosts[0], mosts[1]), fmaxf(mosts[2], mosts[3]));
             row_max[i & 1u][side][lr] = most;
-            au_fence_before();                                               // (the weights of either side lie over scores of both)
             asm volatile("bar.sync %0, 64;" ::"r"(pair) : "memory");
             if (gave_up) { ok = false; leave(); break; }
-            au_fence_after();
             most = scale2 * fmaxf(most, row_max[i & 1u][side ^ 1u][lr]);     // (the scale is positive)
             // the maximum moves when it has grown by 2^8; from -inf (nothing seen yet) always
             const bool moves = most > top + 8.0f || (top == -INFINITY && most != -INFINITY);
-            if (i && __any_sync(0xffffffffu, moves)) {
-                const float factor = moves ? exp2f(top - most) : 1.0f;      // (exp2(-inf - most) = 0)
-                ok = au_wait(o_done, (i - 1) & 1u, &gave_up, p.error, 0x502u);
-                if (!ok) { leave(); break; }
-                au_fence_after();
-                sum *= factor;
-#pragma unroll 1
-                for (uint32_t c = side * (S::OUT / 2); c < (side + 1) * (S::OUT / 2); c += 32) {
-                    uint32_t v[32];
-                    au_ld32(tmem + lanes + S::O_COL + c, v);
-                    au_wait_ld(v);
-#pragma unroll
-                    for (uint32_t j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * factor);
-                    au_st32(tmem + lanes + S::O_COL + c, v);
-                }
-            }
+            const float factor = moves ? exp2f(top - most) : 1.0f;          // (exp2(-inf - most) = 0)
             if (moves) top = most;
             const float from = top == -INFINITY ? 0.0f : top;
             const float2 scale_2 = make_float2(scale2, scale2), from_2 = make_float2(-from, -from), minus = make_float2(-1.0f, -1.0f);
@@ -283,7 +319,17 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
                 s[j] = make_float2(au_exp2(x.x), au_exp2(x.y));
                 sums[j & 1u] = au_add2(sums[j & 1u], s[j]);
             }
-            sum += (sums[0].x + sums[0].y) + (sums[1].x + sums[1].y);
+            sum = sum * factor + ((sums[0].x + sums[0].y) + (sums[1].x + sums[1].y));
+            if (i) {                                                         // the tile before is done, its weights' place free
+                ok = au_wait(o_done, (i - 1) & 1u, &gave_up, p.error, 0x502u);
+                if (!ok) { leave(); break; }
+                au_fence_after();
+                add_tile();
+                if (__any_sync(0xffffffffu, moves)) {
+#pragma unroll
+                    for (uint32_t j = 0; j < MINE; ++j) acc[j] *= factor;
+                }
+            }
 #pragma unroll
             for (uint32_t pl = 0; pl < (uint32_t)PLANES; ++pl) {
                 uint32_t w[16];
@@ -292,28 +338,16 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
                     w[j] = au_pack(s[j].x, s[j].y);
                     if (pl + 1 < (uint32_t)PLANES) s[j] = au_fma2(make_float2(au_lo(w[j]), au_hi(w[j])), minus, s[j]);
                 }
-                au_st16((pl == 2 ? tmem + lanes + S::THIRD + b * 32u : s_col + 32u * pl) + 16u * side, w);
-            }
-            if (part) {      // a value that is not finite? (a row of its own for each thread, as the copy wrote them)
-                ok = au_wait(v_full(i & 1u), i >> 1 & 1u, &gave_up, p.error, 0x503u);
-                if (!ok) { leave(); break; }
-                const uint4* v = reinterpret_cast<const uint4*>(base_p + S::Q + 2 * S::K + (i & 1u) * S::V);
-                uint32_t bad = 0;
-#pragma unroll 4
-                for (uint32_t c = tid; c < S::V / 16; c += AU_SOFT) {
-                    const uint4 x = v[c];
-                    auto odd = [](uint32_t w) { return (uint32_t)((w & 0x7F80u) == 0x7F80u) | (uint32_t)((w & 0x7F800000u) == 0x7F800000u); };
-                    bad |= odd(x.x) | odd(x.y) | odd(x.z) | odd(x.w);
-                }
-                if (bad) not_finite = 1;
+                au_st16(tmem + lanes + S::plane(pl) + 16u * side, w);
             }
             au_wait_st();
             au_fence_before();
-            au_arrive(p_full(b));
+            au_arrive(p_full);
         }
         if (ok) {
             ok = au_wait(o_done, (tiles - 1) & 1u, &gave_up, p.error, 0x502u);
             au_fence_after();
+            if (ok) add_tile();
         }
         row_sum[side][lr] = sum;
     } else if (warp == 8) {
@@ -352,15 +386,16 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
         auto scores = [&](uint32_t i) {
             const uint32_t s = i & 1u;
             ok = au_wait(k_full(s), i >> 1 & 1u, &gave_up, p.error, 0x507u);
+            if (ok && i) ok = au_wait(s_empty, (i - 1) & 1u, &gave_up, p.error, 0x506u);
             if (!ok) return;
             au_fence_after();
             if (au_elect()) {
 #pragma unroll
-                for (uint32_t kk = 0; kk < D / 16; ++kk) {
+                for (uint32_t kk = 0; kk < D / 16; ++kk) {                   // 64 channels a sum
                     const uint32_t qa = q0 + (kk >> 2) * S::Q_BLOCK + (kk & 3u) * 32u, ka = k0 + s * S::K + (kk >> 2) * S::KV_BLOCK + (kk & 3u) * 32u;
-                    au_mma_ss(tmem + s * 64u, desc_hi | (1u << 16) | (qa >> 4), desc_hi | (1u << 16) | (ka >> 4), idesc_s, kk != 0);
+                    au_mma_ss(tmem + (kk >> 2) * 64u, desc_hi | (1u << 16) | (qa >> 4), desc_hi | (1u << 16) | (ka >> 4), idesc_s, (kk & 3u) != 0);
                 }
-                au_commit(s_full(s));
+                au_commit(s_full);
                 au_commit(k_empty(s));
             }
             __syncwarp();
@@ -370,22 +405,16 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
         if (ok) scores(0);
         for (uint32_t i = 0; i < tiles && ok; ++i) {
             const uint32_t s = i & 1u;
-            if (i + 1 < tiles) {
-                // (they go where the weights of tile i - 1 are: products of another shape and sum are not in order with those that read them)
-                if (i) ok = au_wait(o_done, (i - 1) & 1u, &gave_up, p.error, 0x506u);
-                if (ok) scores(i + 1);
-            }
-            if (ok) ok = au_wait(p_full(s), i >> 1 & 1u, &gave_up, p.error, 0x509u);
+            if (i + 1 < tiles) scores(i + 1);
+            if (ok) ok = au_wait(p_full, i & 1u, &gave_up, p.error, 0x509u);
             if (ok) ok = au_wait(v_full(s), i >> 1 & 1u, &gave_up, p.error, 0x50au);
             if (!ok) break;
             au_fence_after();
             if (au_elect()) {
 #pragma unroll
-                for (uint32_t kk = 0; kk < AU_KEYS / 16; ++kk) {
-                    const uint32_t va = v0 + s * S::V + kk * 2048u;
-#pragma unroll
-                    for (uint32_t pl = 0; pl < (uint32_t)PLANES; ++pl)
-                        au_mma_ts(tmem + S::O_COL, (pl == 2 ? tmem + S::THIRD + s * 32u : tmem + s * 64u + pl * 32u) + kk * 8u, desc_hi | ((uint64_t)(S::KV_BLOCK >> 4) << 16) | (va >> 4), idesc_o, (i | kk | pl) != 0);
+                for (uint32_t n = 0; n < (uint32_t)PLANES * (AU_KEYS / 16); ++n) {      // the smallest plane first
+                    const uint32_t pl = PLANES - 1 - n / (AU_KEYS / 16), kk = n % (AU_KEYS / 16), va = v0 + s * S::V + kk * 2048u;
+                    au_mma_ts(tmem + S::O_COL, tmem + S::plane(pl) + kk * 8u, desc_hi | ((uint64_t)(S::KV_BLOCK >> 4) << 16) | (va >> 4), idesc_o, n != 0);
                 }
                 au_commit(v_empty(s));
                 au_commit(o_done);
@@ -395,54 +424,38 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
     }
 
     // ---- the rows: out[token, head, d] = O / sum, rounded once ----
-    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out) + ((size_t)(row < rows ? token : 0u) * a.num_heads + kvh * G + (row < rows ? row % G : 0u)) * D + half;
-    auto read_o = [&](uint32_t c, float (&v)[32]) {
-        uint32_t raw[32];
-        au_ld32(tmem + ((warp & 3u) << 21) + S::O_COL + c, raw);
-        au_wait_ld(raw);
-#pragma unroll
-        for (uint32_t j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
-    };
-    auto store = [&](uint32_t c, const float (&v)[32], float inv) {
-#pragma unroll
-        for (uint32_t j = 0; j < 32; j += 8)
-            *reinterpret_cast<uint4*>(out + c + j) = make_uint4(au_pack(v[j] * inv, v[j + 1] * inv), au_pack(v[j + 2] * inv, v[j + 3] * inv), au_pack(v[j + 4] * inv, v[j + 5] * inv),
-                                                                au_pack(v[j + 6] * inv, v[j + 7] * inv));
-    };
-    __syncthreads();      // (not_finite, gave_up; no copy or product is under way)
+    __syncthreads();      // (gave_up and the sums; no copy or product is under way)
     ok = !gave_up;
-    if (warp < 8 && ok && !not_finite) {
+    if (warp < 8 && ok) {
+        const uint32_t head = kvh * G + (row < rows ? row % G : 0u), at = row < rows ? token : 0u;
+        __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out) + ((size_t)at * a.num_heads + head) * D + half + side * MINE;
         const float both = row_sum[0][lr] + row_sum[1][lr], inv = both > 0.0f ? 1.0f / both : 0.0f;
-#pragma unroll 1
-        for (uint32_t c = side * (S::OUT / 2); c < (side + 1) * (S::OUT / 2); c += 32) {
-            float v[32];
-            read_o(c, v);
-            if (row < rows) store(c, v, inv);
-        }
-    }
-    if (not_finite && ok && warp < 8 && row < rows) {      // key by key, 16 channels at a time: slow, and each key only where it is seen
-        const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(a.queries) + ((size_t)(kvh * G + row % G) * m + token) * D;
-        const __nv_bfloat16 *keys = reinterpret_cast<const __nv_bfloat16*>(a.keys) + (size_t)kvh * a.k_head_stride, *values = reinterpret_cast<const __nv_bfloat16*>(a.values) + (size_t)kvh * a.v_head_stride + half;
-#pragma unroll 1
-        for (uint32_t c = side * (S::OUT / 2); c < (side + 1) * (S::OUT / 2); c += 16) {
-            float o[16], most = -INFINITY, total = 0.0f;
 #pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) o[j] = 0.0f;
-#pragma unroll 1
-            for (uint32_t key = 0; key < kend; ++key) {
-                if (!sees(key)) continue;
-                float s = 0.0f;
-                for (uint32_t d = 0; d < D; ++d) s = fmaf(bf2f(q[d]), bf2f(keys[(size_t)key * a.k_seq_stride + d]), s);
-                s *= scale2;
-                const float next = fmaxf(most, s), from = next == -INFINITY ? 0.0f : next, keep = exp2f(most - from), w = exp2f(s - from);
-                total = total * keep + w;
-                most = next;
+        for (uint32_t c = 0; c < MINE; c += 32) {
+            const float* v = acc + c;
+            bool finite = true;
 #pragma unroll
-                for (uint32_t j = 0; j < 16; ++j) o[j] = fmaf(w, bf2f(values[(size_t)key * a.v_seq_stride + c + j]), o[j] * keep);
+            for (uint32_t j = 0; j < 32; ++j) finite &= fabsf(v[j]) < INFINITY;
+            if (row < rows) {
+                if (finite || !(both < INFINITY)) {
+#pragma unroll
+                    for (uint32_t j = 0; j < 32; j += 8)
+                        *reinterpret_cast<uint4*>(out + c + j) = make_uint4(au_pack(v[j] * inv, v[j + 1] * inv), au_pack(v[j + 2] * inv, v[j + 3] * inv),
+                                                                            au_pack(v[j + 4] * inv, v[j + 5] * inv), au_pack(v[j + 6] * inv, v[j + 7] * inv));
+                } else {
+                    AuRow r;
+                    r.query = reinterpret_cast<const __nv_bfloat16*>(a.queries) + ((size_t)head * m + token) * D;
+                    r.keys = reinterpret_cast<const __nv_bfloat16*>(a.keys) + (size_t)kvh * a.k_head_stride;
+                    r.values = reinterpret_cast<const __nv_bfloat16*>(a.values) + (size_t)kvh * a.v_head_stride + half + side * MINE + c;
+                    r.out = out + c;
+                    r.nodes = trie ? nodes : nullptr;
+                    r.k_stride = a.k_seq_stride; r.v_stride = a.v_seq_stride;
+                    r.token = token; r.lim = lim; r.prefix = prefix; r.kend = kend;
+                    r.scale2 = scale2;
+                    au_row_by_key<D>(r);
+                }
             }
-            const float inv = total > 0.0f ? 1.0f / total : 0.0f;
-#pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) out[c + j] = f2bf(o[j] * inv);
+            __syncwarp();
         }
     }
     au_fence_before();
