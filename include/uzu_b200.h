@@ -324,6 +324,9 @@ UZU_API void uzu_attention_two_pass1_encode(uzu_command_buffer* cmd, const uzu_a
  * uzu_attention_single_pass_encode; 0 here or UZU_PREFILL_ATTN=0 keeps the split-KV kernel, 1 forces the mma.sync kernel on, 2 the tcgen05 one
  * (csrc/attention_umma.cu), -1 = follow the environment. */
 UZU_API void uzu_debug_set_prefill_attention(int mode);
+/* For tests: one decoded row as the engine's steps encode it (csrc/decode_attention.cu): normed, rotated, appended to the cache behind prepare.kv_token_offset
+ * rows (attention->keys / values) and attended over it; 0 where that kernel does not take the call, and nothing is encoded. */
+UZU_API int uzu_debug_decode_attention_encode(uzu_command_buffer* cmd, const uzu_attention_prepare_norm_args* prepare, const uzu_attention_args* attention);
 /* AttentionTwoPass2Kernel: attention_two_pass.rs:139-149 */
 typedef struct uzu_attention_two_pass2_args {
     uint64_t partials, sums, maxs, out;

@@ -1110,6 +1110,7 @@ extern "C" {
     pub fn uzu_attention_single_pass_encode(cmd: *mut uzu_command_buffer, args: *const uzu_attention_args);
     pub fn uzu_attention_two_pass1_encode(cmd: *mut uzu_command_buffer, args: *const uzu_attention_args);
     pub fn uzu_debug_set_prefill_attention(mode: c_int);
+    pub fn uzu_debug_decode_attention_encode(cmd: *mut uzu_command_buffer, prepare: *const uzu_attention_prepare_norm_args, attention: *const uzu_attention_args) -> c_int;
     pub fn uzu_attention_two_pass2_encode(cmd: *mut uzu_command_buffer, args: *const uzu_attention_two_pass2_args);
     pub fn uzu_kv_cache_update_encode(cmd: *mut uzu_command_buffer, args: *const uzu_kv_cache_update_args);
     pub fn uzu_activation_transform_encode(cmd: *mut uzu_command_buffer, args: *const uzu_activation_transform_args);

@@ -7,6 +7,9 @@
 //   * A warp takes tiles of 16 keys. Scores and the weighted sum are products on mma.sync: the heads of a key head are rows 0..7 of the product, the exact f32
 //     probabilities three bf16 planes, two of them in rows g and g + 8 of one product and the third in a second one. Keys go from memory to registers in the
 //     order of the product's B operand (channels are permuted alike in the query), values are paired by PRMT; neither passes through shared memory.
+//   * The pipe cuts what it adds to an accumulator off at its last bit: a chain is 32 channels of a score or one tile's products, the smallest plane first, and chains
+//     are added by rounded additions. As many results are off the correct rounding as on the split-KV kernel, all f32 (1 to 2.5 in 10000); with whole chains up to twice
+//     as many, in the same time.
 //   * The position and a warp's first tile are read before the kernel waits for its predecessor: what earlier steps wrote is there already, since a step's first
 //     kernel is an ordinary launch (uzu_command_buffer::dependent).
 //   * A cluster of up to eight CTAs shares a key head's keys, each 128 and more; the parts meet in distributed shared memory, in rank order.
@@ -58,7 +61,7 @@ __device__ __forceinline__ void da_store_remote(uint32_t addr, float v) { asm vo
 template <int D, bool FEW>
 __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const __grid_constant__ DecodeAttnParams p, const __grid_constant__ AttnSequences seqs) {
     constexpr uint32_t KB = D / 32, VB = D / 64, PER = D / 32;      // 16-byte blocks of a lane: of a key, of a value; elements of a lane of a row
-    constexpr bool kRoomy = D <= 128;                                // registers for the query and for values beside keys; else values are asked for into L2
+    constexpr bool kRoomy = D <= 128;                                // registers for values beside keys; else values are asked for into L2, and read half by half
     extern __shared__ __align__(16) uint8_t da_raw[];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t rank = blockIdx.x, kv_head = blockIdx.y / p.groups, head0 = kv_head * (p.num_heads / p.num_kv_heads) + blockIdx.y % p.groups * p.heads, b = blockIdx.z, G = p.heads;
@@ -84,7 +87,8 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
     const __nv_bfloat16* keys = reinterpret_cast<const __nv_bfloat16*>(seqs.keys[b]) + (size_t)kv_head * D;
     const __nv_bfloat16* values = reinterpret_cast<const __nv_bfloat16*>(seqs.values[b]) + (size_t)kv_head * D;
 
-    uint4 kk[2][KB], vv[4][VB];
+    constexpr uint32_t VR = kRoomy ? VB : VB / 2;                    // blocks of a value that are read at a time
+    uint4 kk[2][KB], vv[4][VR];
     // keys g and g + 8 of a tile, channels 32 i + 8 t; values 2t, 2t + 1, 2t + 8 and 2t + 9, channels 64 i + 8 g. The new token's come from shared memory.
     auto read_keys = [&](uint32_t tile) {
 #pragma unroll
@@ -95,19 +99,20 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
             for (uint32_t i = 0; i < KB; ++i) kk[n][i] = key < length ? *reinterpret_cast<const uint4*>(src + i * 32) : make_uint4(0, 0, 0, 0);
         }
     };
-    auto read_values = [&](uint32_t tile) {
+    auto read_values = [&](uint32_t tile, uint32_t from, uint32_t count) {
 #pragma unroll
         for (uint32_t n = 0; n < 4; ++n) {
             const uint32_t key = tile * 16 + 2 * t + (n & 1u) + (n >> 1) * 8;
             const __nv_bfloat16* src = (key == position ? rows + (G + 1) * D : values + (size_t)key * p.kv_stride) + g * 8;
 #pragma unroll
-            for (uint32_t i = 0; i < VB; ++i) vv[n][i] = key < length ? *reinterpret_cast<const uint4*>(src + i * 64) : make_uint4(0, 0, 0, 0);
+            for (uint32_t i = 0; i < VB; ++i)
+                if (i >= from && i < from + count) vv[n][i % VR] = key < length ? *reinterpret_cast<const uint4*>(src + i * 64) : make_uint4(0, 0, 0, 0);
         }
     };
     const bool early = first < last_tile;      // (the last tile may hold the new key)
     if (early) {
         read_keys(first);
-        if constexpr (kRoomy) read_values(first);
+        if constexpr (kRoomy) read_values(first, 0, VR);
         else if (lane < 16) {
 #pragma unroll
             for (uint32_t i = 0; i < D; i += 64) asm volatile("prefetch.global.L2 [%0];" ::"l"(values + (size_t)(first * 16 + lane) * p.kv_stride + i));
@@ -191,8 +196,8 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
     // ---- a warp's tiles ----
     const uint32_t head = FEW ? g & 3u : g;      // of this lane's rows
     auto query = [&](uint32_t i) { return head < G ? *reinterpret_cast<const uint4*>(rows + head * D + i * 32 + t * 8) : make_uint4(0, 0, 0, 0); };
-    uint4 q[kRoomy ? KB : 1];
-    if constexpr (kRoomy) {
+    uint4 q[D == 64 ? KB : 1];
+    if constexpr (D == 64) {
 #pragma unroll
         for (uint32_t i = 0; i < KB; ++i) q[i] = query(i);
     }
@@ -202,23 +207,25 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
     for (uint32_t i = 0; i < VB * 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.0f;
     if (!early && first < tiles) {
         read_keys(first);
-        if constexpr (kRoomy) read_values(first);
+        if constexpr (kRoomy) read_values(first, 0, VR);
     }
     for (uint32_t tile = first; tile < tiles; tile += step) {
-        float s[2][4];
-        s[0][0] = s[0][1] = s[0][2] = s[0][3] = s[1][0] = s[1][1] = s[1][2] = s[1][3] = 0.0f;
+        float s[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
 #pragma unroll
         for (uint32_t i = 0; i < KB; ++i) {
             uint4 qi;
-            if constexpr (kRoomy) qi = q[i];
+            if constexpr (D == 64) qi = q[i];
             else qi = query(i);
 #pragma unroll
             for (uint32_t n = 0; n < 2; ++n) {
-                da_mma(s[n], qi.x, 0, qi.y, 0, kk[n][i].x, kk[n][i].y);
-                da_mma(s[n], qi.z, 0, qi.w, 0, kk[n][i].z, kk[n][i].w);
+                float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                da_mma(part, qi.x, 0, qi.y, 0, kk[n][i].x, kk[n][i].y);
+                da_mma(part, qi.z, 0, qi.w, 0, kk[n][i].z, kk[n][i].w);
+                s[n][0] += part[0];
+                s[n][1] += part[1];
             }
         }
-        if constexpr (!kRoomy) read_values(tile);
+        if constexpr (!kRoomy) read_values(tile, 0, VR);
         else if (tile + step < tiles) read_keys(tile + step);
         float pr[4];      // keys 2t, 2t + 1, 2t + 8, 2t + 9
 #pragma unroll
@@ -233,10 +240,6 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
         for (uint32_t n = 0; n < 4; ++n) {
             pr[n] = da_weight(pr[n], m);
             l += pr[n];                                     // (this lane's keys; the quad's meet at the end)
-        }
-        if (__any_sync(0xffffffffu, factor != 1.0f)) {
-#pragma unroll
-            for (uint32_t i = 0; i < VB * 8; ++i) { o[i][0] *= factor; o[i][1] *= factor; o[i][2] *= factor; o[i][3] *= factor; }
         }
         uint32_t plane[3][2];
 #pragma unroll
@@ -255,13 +258,17 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
 #pragma unroll
             for (uint32_t j = 0; j < 8; ++j) {
                 const uint32_t sel = j & 1u ? 0x7632u : 0x5410u;
-                const uint32_t b0 = __byte_perm(da_word(vv[0][i], j / 2), da_word(vv[1][i], j / 2), sel), b1 = __byte_perm(da_word(vv[2][i], j / 2), da_word(vv[3][i], j / 2), sel);
-                da_mma(o[i * 8 + j], a[0], a[1], a[2], a[3], b0, b1);
-                if constexpr (!FEW) da_mma(o[i * 8 + j], plane[2][0], 0, plane[2][1], 0, b0, b1);
+                const uint32_t b0 = __byte_perm(da_word(vv[0][i % VR], j / 2), da_word(vv[1][i % VR], j / 2), sel), b1 = __byte_perm(da_word(vv[2][i % VR], j / 2), da_word(vv[3][i % VR], j / 2), sel);
+                float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                if constexpr (!FEW) da_mma(part, plane[2][0], 0, plane[2][1], 0, b0, b1);
+                da_mma(part, a[0], a[1], a[2], a[3], b0, b1);
+#pragma unroll
+                for (uint32_t c = 0; c < 4; ++c) o[i * 8 + j][c] = fmaf(o[i * 8 + j][c], factor, part[c]);
             }
+            if (i + VR < VB) read_values(tile, i + VR, 1);
         }
         if (tile + step < tiles) {
-            if constexpr (kRoomy) read_values(tile + step);
+            if constexpr (kRoomy) read_values(tile + step, 0, VR);
             else read_keys(tile + step);
         }
     }
@@ -438,3 +445,14 @@ void encode_decode_attention(uzu_command_buffer* cmd, const uzu_attention_prepar
 }
 
 }  // namespace uzu
+
+extern "C" int uzu_debug_decode_attention_encode(uzu_command_buffer* cmd, const uzu_attention_prepare_norm_args* p, const uzu_attention_args* a) {
+    if (!cmd || !p || !a || a->sequence_length <= p->prepare.kv_token_offset) return 0;
+    uzu::AttnSequences s{};
+    s.count = 1;
+    s.keys[0] = a->keys; s.values[0] = a->values;
+    s.prefix[0] = s.position[0] = p->prepare.kv_token_offset;
+    if (!uzu::decode_attention_applicable(p->prepare, *a, s)) return 0;
+    uzu::encode_decode_attention(cmd, p->prepare, &p->q_norm, &p->k_norm, a->scale, a->out, s, a->sequence_length);
+    return 1;
+}
