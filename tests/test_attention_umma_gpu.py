@@ -82,3 +82,22 @@ def test_no_further_off_than_the_kernel_before(ctx, H, Hkv, prefix, suffix, D, b
                 ctx.lib.uzu_debug_set_prefill_attention(-1)
             off[i] += off_the_rounding(got, want)
     assert off[1] <= off[0] + 4 * sum(off) ** 0.5, off      # (four standard deviations of the two counts)
+
+
+@pytest.mark.parametrize("H,Hkv,prefix,suffix,D", [(8, 2, 130, 70, 256), (32, 8, 200, 40, 128), (8, 2, 100, 15, 128), (3, 1, 70, 33, 64)])
+def test_values_that_are_not_finite(umma, H, Hkv, prefix, suffix, D):
+    """An infinity that a row sees comes out as one, in its channel, and rows that do not see it have none of it."""
+    rng, n, c = np.random.default_rng(prefix), prefix + suffix, 9
+    q, k, v = (f32_to_bf16(rng.standard_normal(s).astype(np.float32)) for s in ((H, suffix, D), (n, Hkv, D), (n, Hkv, D)))
+    kw = dict(head_dim=D, gqa_factor=H // Hkv, sequence_length=n, k_head_stride=D, k_seq_stride=Hkv * D, v_head_stride=D, v_seq_stride=Hkv * D, scale=float(D ** -0.5), num_heads=H,
+              suffix_length=suffix)
+    want = bf16_to_f32(G.attention_single_pass(umma, q, k, v, **kw)).copy()
+    v[5, 0, c] = f32_to_bf16(np.array([-np.inf], np.float32))[0]
+    v[prefix + 7, Hkv - 1, c + 1] = f32_to_bf16(np.array([np.inf], np.float32))[0]
+    per = H // Hkv
+    want[:, :per, c] = -np.inf
+    want[7:, H - per:, c + 1] = np.inf
+    got = bf16_to_f32(G.attention_single_pass(umma, q, k, v, **kw))
+    odd = ~np.isfinite(want)
+    assert np.array_equal(got[odd], want[odd])
+    assert (np.abs(got[~odd] - want[~odd]) <= 2.0 ** -7 * np.abs(want[~odd]) + 1e-5).all()      # sums in another order, two planes of a weight: a neighbour at most, 2^-7 off

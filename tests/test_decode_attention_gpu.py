@@ -79,3 +79,24 @@ def test_no_further_off_than_sums_in_f32(ctx, heads, groups, dim, n):
         off[0] += off_the_rounding(before, want)
         off[1] += off_the_rounding(got, want)
     assert off[1] <= off[0] + 4 * sum(off) ** 0.5, off      # (four standard deviations of the two counts)
+
+
+@pytest.mark.parametrize("heads,groups,dim,n", [(8, 2, 64, 700), (12, 2, 128, 40), (4, 1, 128, 2300), (8, 2, 256, 300), (12, 1, 256, 300)])
+def test_values_that_are_not_finite(ctx, heads, groups, dim, n):
+    """An infinity that a row sees comes out as one, and only in its channel, as sums in f32 give it: among the cached rows and as the new one."""
+    rng, per = np.random.default_rng(n), heads // groups
+    qkv = f32_to_bf16(rng.standard_normal((heads + 2 * groups, dim)).astype(np.float32))
+    k, v = (f32_to_bf16(rng.standard_normal((n, groups, dim)).astype(np.float32)) for _ in range(2))
+    clean, _, _ = _row(ctx, qkv, k.reshape(n, -1), v.reshape(n, -1), heads, groups, dim)
+    want = bf16_to_f32(clean).copy()
+    bad = {3: [np.inf], 5: [-np.inf], 6: [np.inf, -np.inf], dim - 1: [np.nan]}          # of the last key head: a channel's values, each of another key
+    for c, values in bad.items():
+        for i, x in enumerate(values):
+            v[(7 * c + 11 * i) % (n - 1), groups - 1, c] = f32_to_bf16(np.array([x], np.float32))[0]
+        want[heads - per:, c] = values[0] if len(values) == 1 else np.nan
+    qkv[heads + 2 * groups - 1, 8] = f32_to_bf16(np.array([np.inf], np.float32))[0]
+    want[heads - per:, 8] = np.inf
+    got = bf16_to_f32(_row(ctx, qkv, k.reshape(n, -1), v.reshape(n, -1), heads, groups, dim)[0])
+    odd = ~np.isfinite(want)
+    assert np.array_equal(got[odd], want[odd], equal_nan=True)
+    assert (np.abs(got[~odd] - want[~odd]) <= 2.0 ** -7 * np.abs(want[~odd]) + 1e-6).all()      # sums in another order: a neighbour at most, 2^-7 off

@@ -13,6 +13,7 @@
 //   * The position and a warp's first tile are read before the kernel waits for its predecessor: what earlier steps wrote is there already, since a step's first
 //     kernel is an ordinary launch (uzu_command_buffer::dependent).
 //   * A cluster of up to eight CTAs shares a key head's keys, each 128 and more; the parts meet in distributed shared memory, in rank order.
+// (Heads of 256 spill 110 to 160 bytes a thread.)
 // From the end of the projection, Llama-3-8B at 2048 tokens: 18.5 us a layer before, 8.6 now; Qwen3.5-0.8B at 500 (heads of 256, normed): 22, 10.8. What is left are some
 // 2000 instructions of eight warps, one after another, and the trips to the row, to distributed shared memory and back.
 #include <algorithm>
@@ -53,6 +54,36 @@ __device__ __forceinline__ uint32_t da_remote(const void* p, uint32_t rank) {
     return a;
 }
 __device__ __forceinline__ void da_store_remote(uint32_t addr, float v) { asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory"); }
+
+// a warp's tiles of one head, key by key in f32: its sums to `out`, the maximum and the sum of the weights returned (not part of the kernel's body: its registers)
+template <int D>
+__device__ __noinline__ float2 da_key_by_key(const __nv_bfloat16* query, const __nv_bfloat16* fresh, const __nv_bfloat16* keys, const __nv_bfloat16* values, uint32_t stride, uint32_t position,
+                                             uint32_t first, uint32_t step, float scale, float* out) {
+    const uint32_t lane = threadIdx.x & 31;
+    float acc[D / 32], most = -INFINITY, total = 0.0f;
+#pragma unroll
+    for (uint32_t i = 0; i < D / 32; ++i) acc[i] = 0.0f;
+#pragma unroll 1
+    for (uint32_t tile = first; tile * 16 <= position; tile += step) {
+#pragma unroll 1
+        for (uint32_t key = tile * 16; key <= min(tile * 16 + 15, position); ++key) {
+            const __nv_bfloat16* k = (key == position ? fresh : keys + (size_t)key * stride) + lane;
+            const __nv_bfloat16* v = (key == position ? fresh + D : values + (size_t)key * stride) + lane;
+            float score = 0.0f;
+            for (uint32_t i = 0; i < D / 32; ++i) score = fmaf(bf2f(query[lane + 32 * i]), bf2f(k[32 * i]), score);
+            score = scale * warp_sum(score);
+            const float next = fmaxf(most, score), keep = da_weight(most, next), weight = da_weight(score, next);
+            total = total * keep + weight;
+            most = next;
+#pragma unroll
+            for (uint32_t i = 0; i < D / 32; ++i) acc[i] = fmaf(weight, bf2f(v[32 * i]), acc[i] * keep);
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (uint32_t i = 0; i < D / 32; ++i) out[lane + 32 * i] = acc[i];
+    return make_float2(most, total);
+}
 
 }  // namespace
 
@@ -278,6 +309,7 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
     // ---- the warps' parts ----
     if (first < tiles) {
         float* dst = parts + (warp * G + head) * D;
+        float probe = 0.0f;      // stays zero while everything is finite
 #pragma unroll
         for (uint32_t i = 0; i < VB; ++i) {
 #pragma unroll
@@ -289,9 +321,20 @@ __global__ void __launch_bounds__(DA_THREADS, 1) decode_attention_kernel(const _
                     if constexpr (FEW) v[j] += __shfl_xor_sync(0xffffffffu, v[j], 16);
                 }
                 if (g < G) {
+#pragma unroll
+                    for (uint32_t j = 0; j < 8; ++j) probe = fmaf(v[j], 0.0f, probe);
                     *reinterpret_cast<float4*>(dst + 64 * i + 16 * t + 8 * c) = make_float4(v[0], v[1], v[2], v[3]);
                     *reinterpret_cast<float4*>(dst + 64 * i + 16 * t + 8 * c + 4) = make_float4(v[4], v[5], v[6], v[7]);
                 }
+            }
+        }
+        // A value that is not finite makes NaN of a weight's plane that is zero. Where sums are not finite and weights are, the warp's keys are taken one after another
+        // in f32, and what is not finite comes out as the products make it.
+        if (!__all_sync(0xffffffffu, probe == 0.0f)) {
+            for (uint32_t h = 0; h < G; ++h) {
+                if (!(__shfl_sync(0xffffffffu, l, h * 4) < INFINITY)) continue;
+                const float2 ml = da_key_by_key<D>(rows + h * D, rows + G * D, keys, values, p.kv_stride, position, first, step, p.scale, parts + (warp * G + h) * D);
+                if (g == h) { m = ml.x; l = ml.y; }
             }
         }
     }
