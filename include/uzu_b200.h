@@ -203,12 +203,14 @@ typedef struct uzu_fused_linear_args {
     uint64_t decode_stream;
 } uzu_fused_linear_args;
 /* Tuning sweeps only (tools/): override the decode GEMV's work split; 0 = heuristic. Process-wide, not thread-safe. */
+/* for tests: as the engine's steps encode it, 8-bit weights with a decode stream as well; 0 where it is not supported, and nothing is encoded */
+UZU_API int uzu_debug_fused_linear_encode(uzu_command_buffer* cmd, const uzu_fused_linear_args* args);
 UZU_API void uzu_debug_set_qmv_tuning(int warps_per_tile, int k_slices, int ctas_per_sm, int stages);
 /* Quantized B, bf16 A: 2..32 rows run csrc/qmm_rows.cu (mma.sync, groups of 64 and 128), more rows csrc/qmm_scaled.cu (tcgen05, weights as two
  * bf16 planes in tensor memory); UZU_QMM_ROWS=0 / UZU_QMM_SCALED=0 take the kernels for other shapes instead;
  * UZU_PREFILL_GEMM_MIN_M=<m> does so for fewer rows than that, 0 for all. uzu_debug_set_qmm_tile, for tests: the latter's
  * rows per tile (16, 32, 64, 128, 192, 256) and CTAs that share a tile's k (1, 2, 4, 8; fewer where k is too short), 0 = the plan's own; splits -1: the
- * kernel of csrc/qmm_wide.cu with tiles of that many rows (a multiple of 16 up to 256); returns 0 for other values. Process-wide, not thread-safe. */
+ * kernel of csrc/qmm_wide.cu with tiles of that many rows (a multiple of 16 up to 256), an error of the call where that cannot run; returns 0 for other values. Process-wide, not thread-safe. */
 UZU_API int uzu_debug_set_qmm_tile(int rows, int splits);
 /* the same for tiles of mt x 128 rows (1, 2); the other arguments are not used */
 UZU_API void uzu_debug_set_umma(int layout, uint32_t desc_hi, uint32_t desc_lbo, uint32_t k_step, uint32_t idesc, int mt);

@@ -1089,6 +1089,7 @@ extern "C" {
     pub fn uzu_command_buffer_launch_count(cmd: *const uzu_command_buffer) -> u64;
     pub fn uzu_matmul_encode(cmd: *mut uzu_command_buffer, args: *const uzu_matmul_args);
     pub fn uzu_matmul_validate(args: *const uzu_matmul_args) -> c_int;
+    pub fn uzu_debug_fused_linear_encode(cmd: *mut uzu_command_buffer, args: *const uzu_fused_linear_args) -> c_int;
     pub fn uzu_debug_set_qmv_tuning(warps_per_tile: c_int, k_slices: c_int, ctas_per_sm: c_int, stages: c_int);
     pub fn uzu_debug_set_qmm_tile(rows: c_int, splits: c_int) -> c_int;
     pub fn uzu_debug_set_umma(layout: c_int, desc_hi: u32, desc_lbo: u32, k_step: u32, idesc: u32, mt: c_int);

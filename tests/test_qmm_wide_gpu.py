@@ -7,6 +7,7 @@ from tests import gpu_ops as G
 from tests.test_qmm_integer_codes_gpu import ENDS, check_ends
 from tests.test_qmm_scaled_gpu import check, weights
 from tests.util import assert_bf16_close, f32_to_bf16
+from uzu_b200.binding import UzuError
 
 pytestmark = [pytest.mark.gpu]
 
@@ -50,3 +51,10 @@ def test_epilogue(ctx, width):
     w, kw = weights(rng, n, k, 4, 128, "zero")
     x = f32_to_bf16(rng.uniform(-0.5, 0.5, (m, k)).astype(np.float32))
     assert_bf16_close(G.matmul(ctx, x, w, m=m, n=n, k=k, **kw), O.matmul(x, w, m=m, n=n, k=k, threads=8, **kw), max_ulp=1, min_exact=0.97, what="bf16 rows")
+
+
+@pytest.mark.parametrize("bits,gs,method", [(4, 64, "zero"), (8, 128, "zero"), (4, 128, "mlx")])
+def test_what_it_does_not_take(ctx, width, bits, gs, method):
+    """(so that no test above runs another kernel unseen)"""
+    with pytest.raises(UzuError, match="qmm_wide"):
+        check(ctx, 100, 128, 512, bits, gs, method)

@@ -291,7 +291,7 @@ uzu_activation_transform_validate uzu_dense_linear_encode uzu_group_rms_norm_enc
 uzu_unary_f32_encode uzu_residual_add_encode uzu_logit_cap_f32_encode uzu_table_route_encode uzu_routed_combine_encode
 uzu_general_delta_encode uzu_head_norm_gate_encode uzu_latent_prepare_encode uzu_latent_attention_encode
 uzu_silu_glu_encode uzu_topk_route_encode uzu_routed_combine_gated_encode uzu_sigmoid_attention_prepare_encode uzu_sigmoid_attention_encode
-uzu_engine_slot_acquire uzu_engine_slot_release uzu_engine_forward_rows uzu_engine_debug_layer_outputs uzu_debug_dense_umma_error uzu_debug_set_wait_error uzu_debug_decode_attention_encode
+uzu_engine_slot_acquire uzu_engine_slot_release uzu_engine_forward_rows uzu_engine_debug_layer_outputs uzu_debug_dense_umma_error uzu_debug_set_wait_error uzu_debug_decode_attention_encode uzu_debug_fused_linear_encode
 uzu_min_gru_encode uzu_retention_encode uzu_window_attention_prepare_encode uzu_window_attention_encode
 uzu_exp_gates_encode uzu_norm_add_encode uzu_token_gate_encode uzu_embedding_f32_scaled_encode uzu_rows_to_bf16_encode
 uzu_side_step_encode uzu_side_attention_encode uzu_embedding_f32_position_encode uzu_glu_encode uzu_stream_mix_encode uzu_delta_prepare_encode uzu_gated_delta_encode uzu_gated_delta_step_encode""".split()
@@ -415,6 +415,7 @@ def load() -> C.CDLL:
         "uzu_debug_set_qmv_tuning": (None, [C.c_int, C.c_int, C.c_int, C.c_int]),
         "uzu_debug_set_prefill_attention": (None, [C.c_int]),
         "uzu_debug_set_delta_prefill": (None, [C.c_int]),
+        "uzu_debug_fused_linear_encode": (C.c_int, [vp, C.POINTER(FusedLinearArgs)]),
         "uzu_debug_decode_attention_encode": (C.c_int, [vp, C.POINTER(AttentionPrepareNormArgs), C.POINTER(AttentionArgs)]),
         "uzu_debug_set_qmm_tile": (C.c_int, [C.c_int, C.c_int]),
         "uzu_debug_set_umma": (None, [C.c_int, C.c_uint32, C.c_uint32, C.c_uint32, C.c_uint32, C.c_int]),

@@ -6,8 +6,10 @@
 // by memory (asking for its weights ahead of time, into L2, changed nothing).
 //   * Codes stay integers: a word of eight nibbles is two registers of bytes (three instructions; bf16 pairs 128 + code took seven), 8-bit codes are taken as they
 //     lie, and products run on mma.sync u8 x s8, which has the rate of bf16 per instruction at twice the depth. The row is a 28-bit fixed-point number per element,
-//     scaled by the largest exponent of its quantisation group, in four digits of seven bits: one column of the product per digit. The sums are exact; what a digit
-//     cut off at 2^-26 of the group's largest element loses is below the rounding of sums in f32. A group's two halves of columns keep two groups apart.
+//     scaled by the largest exponent of its quantisation group, in four digits of seven bits: one column of the product per digit. A group's two halves of columns
+//     keep two groups apart. The integer sums are exact; a pair of digits' sum has up to 24 bits with 4-bit codes, exact in f32 too, and up to 28 with bytes, rounded to
+//     24. What a digit cut off at 2^-26 of the group's largest element loses is below the rounding of sums in f32. A row with an infinity or a NaN makes NaN of
+//     every output: codes and the zero point, which multiplies the row's sum, are taken apart.
 //   * A CTA has 16 warps and whole 16-row tiles; its units lie one behind another in memory and the warps take them in turn, so that each SM reads one
 //     contiguous range. A warp copies a unit to registers as soon as it has landed and asks for the next one at once: 74 to 147 KB an SM are on their way. The first
 //     half of that is asked for before the kernel waits for its predecessor, the second half behind the row, whose reads would otherwise stand in line for it.

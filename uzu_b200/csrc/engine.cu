@@ -757,7 +757,7 @@ struct uzu_engine {
         uint32_t nstreams = 0;
         uint64_t stream_bytes = 0;
         uint64_t barrier_base = 0;       // arrivals the monotonic grid-barrier counter has seen before the next launch
-        std::map<uint64_t, uint64_t> stream_of;   // weight values pointer -> decode-stream copy (also feeds the per-kernel path's TMA GEMV)
+        std::map<uint64_t, uint64_t> stream_of;   // weight values pointer -> decode-stream copy (decode_linear.cu reads it in the per-kernel path)
     } mega;
 };
 
@@ -1787,7 +1787,7 @@ static bool fused_decode_supported(uzu_engine* e) {
     return true;
 }
 
-// a plain m = 1 GEMV of the decode step: through the TMA-fed stream variant when the linear has a decode-stream copy
+// a plain m = 1 GEMV of the decode step: decode_linear.cu where the linear has a decode-stream copy
 static void encode_decode_gemv(uzu_engine* e, uzu_command_buffer* cmd, const Linear& lin, uint64_t x, uint64_t d) {
     const uint64_t stream = e->tp_sharded ? 0 : g_stream_lookup(e->mega.stream_of, lin);
     if (stream) {

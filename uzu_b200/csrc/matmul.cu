@@ -1881,6 +1881,12 @@ int uzu_fused_linear_supported(uzu_context* ctx, const uzu_fused_linear_args* ar
     return args && args->matmul.b_mode == UZU_QMODE_U4 && uzu::fused_linear_supported(ctx, args) ? 1 : 0;
 }
 
+int uzu_debug_fused_linear_encode(uzu_command_buffer* cmd, const uzu_fused_linear_args* args) {
+    if (!cmd || !args || !uzu::encodable(cmd, "fused_linear") || !uzu::fused_linear_supported(cmd->ctx, args)) return 0;
+    uzu::encode_fused_linear(cmd, args);
+    return 1;
+}
+
 void uzu_fused_linear_encode(uzu_command_buffer* cmd, const uzu_fused_linear_args* args) {
     if (!uzu::encodable(cmd, "fused_linear")) return;
     if (!uzu_fused_linear_supported(cmd->ctx, args)) {

@@ -631,8 +631,13 @@ void encode_qmm_scaled(uzu_command_buffer* cmd, const uzu_matmul_args& a) {
     const bool three = p.biases && p.m < 64, integers = !p.biases && a.b_group_size >= 64;      // (integers: tiles of up to 64 rows)
     p.chain_k = std::min(a.b_group_size, 128u);
     QsPlan plan = qs_plan(p.m, a.n, p.nkb, bits, p.biases != nullptr, three, integers, a.b_group_size == 32, (uint32_t)ctx->sm_count);
+    const bool wide_can = integers && bits == 4 && p.chain_k == 128u && !p.has_soft_cap;
+    if (g_wide && !wide_can) {
+        cmd->record_error(UZU_ERROR_UNSUPPORTED, "matmul: the kernel asked for (qmm_wide.cu) does not take this call");
+        return;
+    }
     // one plane of integers for wide tiles: 4-bit codes in groups of 128 and more (qmm_wide.cu, with the times of both kernels)
-    if (integers && bits == 4 && p.chain_k == 128u && !p.has_soft_cap && (g_wide || (p.m > 64 && !g_tile_rows && !g_tile_splits))) {
+    if (wide_can && (g_wide || (p.m > 64 && !g_tile_rows && !g_tile_splits))) {
         const QwPlan wide = qw_plan(p.m, a.n, p.nkb, (uint32_t)ctx->sm_count);
         if (g_wide || wide.cost < plan.cost) return encode_qmm_wide(cmd, a, p, g_wide ? (uint32_t)g_wide : wide.width);
     }
