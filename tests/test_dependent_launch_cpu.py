@@ -72,3 +72,10 @@ def test_scores_are_not_written_over_weights_that_products_still_read():
     issue = text[text.index("if (i + 1 < tiles)"):text.index("au_commit(o_done)")]
     over = "tmem + s * 64u + pl * 32u" in issue                        # weights in the columns of scores
     assert not over or issue.index("au_wait(o_done") < issue.index("scores(i + 1)")
+
+
+@pytest.mark.parametrize("body", [pytest.param(p.values[0], id=p.id) for p in _kernels() if "tcgen05.alloc" in p.values[0]])
+def test_products_in_flight_are_waited_for_before_tensor_memory_is_given_back(body):
+    """Also where a wait ran out: the role that issues products then commits what it has issued and waits, with a limit, for that."""
+    end = body.index("tcgen05.dealloc")
+    assert re.search(r"(_commit\(last_products\);\s*\}?\s*__syncwarp\(\);\s*\w+_settle\(last_products, 0\)|\(accum_bar\)[^;]*;\s*__syncwarp\(\);\s*if \(!ok\)\s*for \([^)]*try_wait\(accum_bar, 0\))", body[:end])

@@ -61,6 +61,10 @@ __device__ __forceinline__ bool au_try(uint32_t bar, uint32_t parity) {
     asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3; selp.u32 %0, 1, 0, p; }" : "=r"(ok) : "r"(bar), "r"(parity), "r"(20000u) : "memory");
     return ok != 0;
 }
+// after a wait that ran out: what is in flight ends before the CTA does
+__device__ __forceinline__ void au_settle(uint32_t bar, uint32_t parity) {
+    for (uint32_t n = 0; n < 4096 && !au_try(bar, parity); ++n) {}
+}
 // false: the phase did not complete within about a second, or another role of the CTA has given up
 __device__ __noinline__ bool au_wait_long(uint32_t bar, uint32_t parity, volatile uint32_t* gave_up, unsigned int* error, uint32_t code) {
     uint64_t t0, t1;
@@ -186,7 +190,7 @@ template <int D, int PLANES>
 __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const AuParams p) {
     using S = AuShape<D, PLANES>;
     extern __shared__ uint8_t au_raw[];
-    __shared__ __align__(8) uint64_t bars[13];
+    __shared__ __align__(8) uint64_t bars[14];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile uint32_t gave_up;
     __shared__ float row_max[2][2][AU_ROWS], row_sum[2][AU_ROWS];      // [tile][side][row]: what the two threads of a row tell each other
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
     auto k_empty = [&](uint32_t s) { return bar0 + 8u * (3 + s); };
     auto v_full = [&](uint32_t s) { return bar0 + 8u * (5 + s); };
     auto v_empty = [&](uint32_t s) { return bar0 + 8u * (7 + s); };
-    const uint32_t s_full = bar0 + 8u * 9, s_empty = bar0 + 8u * 10, p_full = bar0 + 8u * 11, o_done = bar0 + 8u * 12;
+    const uint32_t s_full = bar0 + 8u * 9, s_empty = bar0 + 8u * 10, p_full = bar0 + 8u * 11, o_done = bar0 + 8u * 12, last_products = bar0 + 8u * 13;
 
     const uint32_t G = a.gqa_factor, m = a.suffix_length, seq = a.sequence_length, prefix = seq - m, rows = m * G, half = blockIdx.z * S::OUT;      // half: the first of this CTA's channels
     const uint32_t row0 = (gridDim.x - 1u - blockIdx.x) * AU_ROWS, kvh = blockIdx.y;      // the rows with the most keys first
@@ -214,7 +218,7 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
             for (uint32_t s = 0; s < 2; ++s) {
                 au_init(k_full(s), 1); au_init(k_empty(s), 1); au_init(v_full(s), 1); au_init(v_empty(s), 1);
             }
-            au_init(s_full, 1); au_init(s_empty, AU_SOFT / 32); au_init(p_full, AU_SOFT / 32); au_init(o_done, 1);
+            au_init(s_full, 1); au_init(s_empty, AU_SOFT / 32); au_init(p_full, AU_SOFT / 32); au_init(o_done, 1); au_init(last_products, 1);
             gave_up = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -371,10 +375,9 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
             if (ok) { copy(i, false); asked_v += ok; }
         }
         if (!ok) {      // copies that are on their way end before the CTA does
-            auto settle = [&](uint32_t bar, uint32_t i) { for (uint32_t n = 0; n < 4096 && !au_try(bar, i >> 1 & 1u); ++n) {} };
             for (uint32_t n = 1; n <= 2; ++n) {
-                if (asked_k >= n) settle(k_full((asked_k - n) & 1u), asked_k - n);
-                if (asked_v >= n) settle(v_full((asked_v - n) & 1u), asked_v - n);
+                if (asked_k >= n) au_settle(k_full((asked_k - n) & 1u), (asked_k - n) >> 1 & 1u);
+                if (asked_v >= n) au_settle(v_full((asked_v - n) & 1u), (asked_v - n) >> 1 & 1u);
             }
         }
     } else {
@@ -420,6 +423,11 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
                 au_commit(o_done);
             }
             __syncwarp();
+        }
+        if (!ok) {
+            if (au_elect()) au_commit(last_products);
+            __syncwarp();
+            au_settle(last_products, 0);                                 // none in flight when tensor memory is given back
         }
     }
 

@@ -304,9 +304,11 @@ __global__ void __launch_bounds__(DU_NP + 32, 1) dense_umma_kernel(const DenseUm
     } else {
         // ================================ MMA issuer ================================
         uint32_t s = 0, parity = 0;
+        bool ok = true;
         for (uint32_t kb = 0; kb < nkb; ++kb) {
             if (__any_sync(0xffffffffu, !du_mbar_wait(full_bar(s), parity))) {
                 if (lane == 0) fail(3);
+                ok = false;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -330,6 +332,8 @@ __global__ void __launch_bounds__(DU_NP + 32, 1) dense_umma_kernel(const DenseUm
         }
         if (du_elect()) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(accum_bar) : "memory");
         __syncwarp();
+        if (!ok)
+            for (uint32_t n = 0; n < 4096 && !du_mbar_try_wait(accum_bar, 0); ++n) {}      // none in flight when tensor memory is given back
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
     constexpr int DG = S::DG, ND = S::ND, AS = S::AS, BS = S::BS, CS = S::CS, DQ_WARPS = 4 * DG, EW = S::EW, EC = S::EC;
     constexpr uint32_t kpt = BITS == 4 ? 4u : 2u;                            // k blocks per code tile
     extern __shared__ uint8_t qs_raw[];
-    __shared__ __align__(8) uint64_t bars[2 * CS + 2 * BS + 2 * AS + 2 * ND];
+    __shared__ __align__(8) uint64_t bars[2 * CS + 2 * BS + 2 * AS + 2 * ND + 1];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile uint32_t gave_up;
     const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;     // (warp: the same in every lane)
@@ -131,6 +131,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
     auto a_empty = [&](uint32_t i) { return bar0 + 8u * (2 * CS + 2 * BS + AS + i); };
     auto d_full = [&](uint32_t i) { return bar0 + 8u * (2 * CS + 2 * BS + 2 * AS + i); };
     auto d_empty = [&](uint32_t i) { return bar0 + 8u * (2 * CS + 2 * BS + 2 * AS + ND + i); };
+    const uint32_t last_products = bar0 + 8u * (2 * CS + 2 * BS + 2 * AS + 2 * ND);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -138,6 +139,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
             for (int i = 0; i < BS; ++i) { qs_init(act_full(i), 1); qs_init(act_empty(i), 1); }
             for (int i = 0; i < AS; ++i) { qs_init(a_full(i), 4); qs_init(a_empty(i), 1); }
             for (int i = 0; i < ND; ++i) { qs_init(d_full(i), 1); qs_init(d_empty(i), EW); }
+            qs_init(last_products, 1);
             gave_up = 0;
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -381,7 +383,7 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
         bool ok = true;
         if (role == 0) {
             // ================================ codes by TMA (they depend on no kernel) ================================
-            uint32_t slot = 0, ph = 1;
+            uint32_t slot = 0, ph = 1, asked = 0;
             for (uint32_t item = item0; item < p.items && ok; item += item_step) {
                 const uint32_t y = item_n(item), x0 = kb0 / kpt * 128u;
                 for (uint32_t tile = 0; tile < tiles; ++tile) {
@@ -392,12 +394,15 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                         qs_tma_2d(code0 + slot * QS_CODE_TILE, &map_w, x0 + tile * 128u, y, code_full(slot));
                     }
                     __syncwarp();
+                    ++asked;
                     if (++slot == (uint32_t)CS) { slot = 0; ph ^= 1u; }
                 }
             }
+            if (!ok)
+                for (uint32_t n = asked > (uint32_t)CS ? asked - CS : 0; n < asked; ++n) qs_settle(code_full(n % CS), n / CS & 1u);
         } else if (role == 1) {
             // ================================ activations by TMA, 128 k a stage ================================
-            uint32_t slot = 0, ph = 1;
+            uint32_t slot = 0, ph = 1, asked = 0;
             pdl_wait();
             for (uint32_t item = item0; item < p.items && ok; item += item_step) {
                 const uint32_t y = item_m(item);
@@ -410,9 +415,12 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                         qs_tma_2d(act0 + slot * S::ACT + S::ACT / 2, &map_x, (kb0 + i + 1) * 64u, y, act_full(slot));
                     }
                     __syncwarp();
+                    ++asked;
                     if (++slot == (uint32_t)BS) { slot = 0; ph ^= 1u; }
                 }
             }
+            if (!ok)
+                for (uint32_t n = asked > (uint32_t)BS ? asked - BS : 0; n < asked; ++n) qs_settle(act_full(n % BS), n / BS & 1u);
         } else {
             // ================================ products ================================
             // shared-memory descriptor: K-major SWIZZLE_128B, 1024 bytes between 8-row groups, +32 bytes per 16 k
@@ -484,6 +492,11 @@ __global__ void __launch_bounds__(QsShape<NT, PL>::THREADS, 1) qmm_scaled_kernel
                     __syncwarp();
                     if (++buf == (uint32_t)ND) { buf = 0; d_ph ^= 1u; }
                 }
+            }
+            if (!ok) {
+                if (qs_elect()) qs_commit(last_products);
+                __syncwarp();
+                qs_settle(last_products, 0);                             // none in flight when tensor memory is given back
             }
         }
         __syncwarp();

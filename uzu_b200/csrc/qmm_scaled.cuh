@@ -59,6 +59,10 @@ __device__ __forceinline__ bool qs_wait(uint32_t bar, uint32_t parity, volatile 
     if (__all_sync(0xffffffffu, qs_try(bar, parity))) return true;
     return __all_sync(0xffffffffu, qs_wait_long(bar, parity, gave_up, error, code));
 }
+// after a wait that ran out: what is in flight ends before the CTA does
+__device__ __forceinline__ void qs_settle(uint32_t bar, uint32_t parity) {
+    for (uint32_t n = 0; n < 4096 && !qs_try(bar, parity); ++n) {}
+}
 __device__ __forceinline__ void qs_tma_2d(uint32_t dst, const CUtensorMap* map, uint32_t x, uint32_t y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
                  : "memory");

@@ -69,10 +69,6 @@ __device__ __forceinline__ bool qw_wait_long(uint32_t bar, uint32_t parity, vola
 __device__ __forceinline__ bool qw_wait(uint32_t ready, uint32_t bar, uint32_t parity, volatile uint32_t* gave_up, unsigned int* error, uint32_t code) {
     return __all_sync(0xffffffffu, ready) || qw_wait_long(bar, parity, gave_up, error, code);
 }
-// after a wait that ran out: what is in flight ends before the CTA does
-__device__ __forceinline__ void qw_settle(uint32_t bar, uint32_t parity) {
-    for (uint32_t n = 0; n < 4096 && !qs_try(bar, parity); ++n) {}
-}
 __device__ __forceinline__ void qw_ld32(uint32_t taddr, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
@@ -313,7 +309,7 @@ __global__ void __launch_bounds__(QW_THREADS, 1) qmm_wide_kernel(const __grid_co
                 }
             }
             if (!ok)
-                for (uint32_t n = asked > QW_CODES ? asked - QW_CODES : 0; n < asked; ++n) qw_settle(code_full(n % QW_CODES), n / QW_CODES & 1u);
+                for (uint32_t n = asked > QW_CODES ? asked - QW_CODES : 0; n < asked; ++n) qs_settle(code_full(n % QW_CODES), n / QW_CODES & 1u);
         } else if (role == 1) {
             // ================================ activations by TMA, 64 k a stage ================================
             uint32_t slot = 0, ph = 1, asked = 0;
@@ -333,7 +329,7 @@ __global__ void __launch_bounds__(QW_THREADS, 1) qmm_wide_kernel(const __grid_co
                 }
             }
             if (!ok)
-                for (uint32_t n = asked > QW_ACTS ? asked - QW_ACTS : 0; n < asked; ++n) qw_settle(act_full(n % QW_ACTS), n / QW_ACTS & 1u);
+                for (uint32_t n = asked > QW_ACTS ? asked - QW_ACTS : 0; n < asked; ++n) qs_settle(act_full(n % QW_ACTS), n / QW_ACTS & 1u);
         } else if (role - 2 < halves) {
             // ================================ products: a warp for each half ================================
             // shared-memory descriptor: K-major SWIZZLE_128B, 1024 bytes between 8-row groups, +32 bytes per 16 k
@@ -372,7 +368,7 @@ __global__ void __launch_bounds__(QW_THREADS, 1) qmm_wide_kernel(const __grid_co
             }
             if (qs_elect()) qs_commit(last_products);
             __syncwarp();
-            qw_settle(last_products, 0);                                 // none in flight when tensor memory is given back
+            qs_settle(last_products, 0);                                 // none in flight when tensor memory is given back
         }
         __syncwarp();
     }
