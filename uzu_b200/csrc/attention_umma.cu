@@ -10,7 +10,7 @@
 // The pipe cuts what it adds to an accumulator off at its last bit. So no chain is longer than 64 channels or the products of a tile, the smallest plane first, and the
 // chains are added by rounded additions: with three planes 1.4 to 2.1 results in 10000 are off the correct rounding (split-KV, all f32, 1.8 to 4.7; mma.sync 2.3 to 2.9;
 // 33 with whole chains in tensor memory), with two 24 to 25 (mma.sync 23 to 30, whole chains 29 to 31).
-// Of 64 channels two CTAs share an SM, one's products run beside the other's softmax (and a thread spills 370 bytes for it); of more, the sums take the registers. Of 256
+// Of 64 channels two CTAs share an SM, one's products run beside the other's softmax (and a thread spills 360 bytes for it); of more, the sums take the registers. Of 256
 // channels a CTA sums one half (grid z), so that the prompts of few heads fill the chip. What bounds it now: the softmax warps' way through a tile, 1900 cycles of 128
 // channels and 2300 of 256 (exponentials 750, planes 300, the waits for scores, for the tile before and for stores 140 each); products take 860 and 1500 of them. Four
 // threads a row instead of two changed nothing.
@@ -19,7 +19,7 @@
 // (Accumulators start at multiples of 128 columns, scores at multiples of 64. A form with score tiles 96 columns apart, 256 channels a CTA and clusters that shared the
 // keys of a row tile ended in an illegal memory access whose cause was not found; none of the three is built.)
 // A value that is not finite makes NaN of a weight of zero, in whole or in one of its planes: a row whose sums are not finite, its weights being so, is computed again
-// key by key, each only where it is seen.
+// key by key, each only where it is seen (1024 tokens behind 1024 rows with nothing but infinities: 5 ms of 64 channels, 10 of 128 and 256).
 // Every barrier wait is bounded (wait_errors.h).
 #include <cuda.h>
 
@@ -159,30 +159,44 @@ struct AuRow {
     uint32_t token, lim, prefix, kend;
     float scale2;
 };
-// 32 channels of a row key by key, each key only where it is seen: slow, for sums of values that are not finite
-template <int D>
+// some channels of a row key by key, each key only where it is seen: for sums of values that are not finite (a warp's rows share their keys, so that its lanes read alike)
+template <int D, uint32_t CHANNELS>
 __device__ __noinline__ void au_row_by_key(const AuRow r) {
-#pragma unroll 1
-    for (uint32_t c = 0; c < 32; c += 16) {
-        float o[16], most = -INFINITY, total = 0.0f;
+    float o[CHANNELS], most = -INFINITY, total = 0.0f;
 #pragma unroll
-        for (uint32_t j = 0; j < 16; ++j) o[j] = 0.0f;
+    for (uint32_t j = 0; j < CHANNELS; ++j) o[j] = 0.0f;
 #pragma unroll 1
-        for (uint32_t key = 0; key < r.kend; ++key) {
-            if (key >= r.lim && !(r.nodes && key >= r.prefix && r.token >= r.nodes[key - r.prefix].trie_start && r.token <= r.nodes[key - r.prefix].trie_end)) continue;
-            float s = 0.0f;
-            for (uint32_t d = 0; d < D; ++d) s = fmaf(bf2f(r.query[d]), bf2f(r.keys[key * r.k_stride + d]), s);
-            s *= r.scale2;
-            const float next = fmaxf(most, s), from = next == -INFINITY ? 0.0f : next, keep = exp2f(most - from), w = exp2f(s - from);
-            total = total * keep + w;
-            most = next;
+    for (uint32_t key = 0; key < r.kend; ++key) {
+        if (key >= r.lim && !(r.nodes && key >= r.prefix && r.token >= r.nodes[key - r.prefix].trie_start && r.token <= r.nodes[key - r.prefix].trie_end)) continue;
+        const uint4 *q = reinterpret_cast<const uint4*>(r.query), *k = reinterpret_cast<const uint4*>(r.keys + key * r.k_stride), *v = reinterpret_cast<const uint4*>(r.values + key * r.v_stride);
+        float s = 0.0f;
+#pragma unroll 4
+        for (uint32_t d = 0; d < D / 8; ++d) {
+            const uint4 x = q[d], y = k[d];
+            const uint32_t xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
 #pragma unroll
-            for (uint32_t j = 0; j < 16; ++j) o[j] = fmaf(w, bf2f(r.values[key * r.v_stride + c + j]), o[j] * keep);
+            for (uint32_t i = 0; i < 4; ++i) s = fmaf(au_hi(xs[i]), au_hi(ys[i]), fmaf(au_lo(xs[i]), au_lo(ys[i]), s));
         }
-        const float inv = total > 0.0f ? 1.0f / total : 0.0f;
+        s *= r.scale2;
+        const float next = fmaxf(most, s), from = next == -INFINITY ? 0.0f : next, keep = exp2f(most - from), w = exp2f(s - from);
+        total = total * keep + w;
+        most = next;
 #pragma unroll
-        for (uint32_t j = 0; j < 16; ++j) r.out[c + j] = f2bf(o[j] * inv);
+        for (uint32_t j = 0; j < CHANNELS; j += 8) {
+            const uint4 y = v[j / 8];
+            const uint32_t ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                o[j + 2 * i] = fmaf(w, au_lo(ys[i]), o[j + 2 * i] * keep);
+                o[j + 2 * i + 1] = fmaf(w, au_hi(ys[i]), o[j + 2 * i + 1] * keep);
+            }
+        }
     }
+    const float inv = total > 0.0f ? 1.0f / total : 0.0f;
+#pragma unroll
+    for (uint32_t j = 0; j < CHANNELS; j += 8)
+        *reinterpret_cast<uint4*>(r.out + j) = make_uint4(au_pack(o[j] * inv, o[j + 1] * inv), au_pack(o[j + 2] * inv, o[j + 3] * inv), au_pack(o[j + 4] * inv, o[j + 5] * inv),
+                                                          au_pack(o[j + 6] * inv, o[j + 7] * inv));
 }
 }  // namespace
 
@@ -438,32 +452,25 @@ __global__ void __launch_bounds__(AU_THREADS, AuShape<D, PLANES>::CTAS) attn_umm
         const uint32_t head = kvh * G + (row < rows ? row % G : 0u), at = row < rows ? token : 0u;
         __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(a.out) + ((size_t)at * a.num_heads + head) * D + half + side * MINE;
         const float both = row_sum[0][lr] + row_sum[1][lr], inv = both > 0.0f ? 1.0f / both : 0.0f;
+        bool finite = true;
 #pragma unroll
-        for (uint32_t c = 0; c < MINE; c += 32) {
-            const float* v = acc + c;
-            bool finite = true;
+        for (uint32_t j = 0; j < MINE; ++j) finite &= fabsf(acc[j]) < INFINITY;
+        if (row < rows && (finite || !(both < INFINITY))) {
 #pragma unroll
-            for (uint32_t j = 0; j < 32; ++j) finite &= fabsf(v[j]) < INFINITY;
-            if (row < rows) {
-                if (finite || !(both < INFINITY)) {
-#pragma unroll
-                    for (uint32_t j = 0; j < 32; j += 8)
-                        *reinterpret_cast<uint4*>(out + c + j) = make_uint4(au_pack(v[j] * inv, v[j + 1] * inv), au_pack(v[j + 2] * inv, v[j + 3] * inv),
-                                                                            au_pack(v[j + 4] * inv, v[j + 5] * inv), au_pack(v[j + 6] * inv, v[j + 7] * inv));
-                } else {
-                    AuRow r;
-                    r.query = reinterpret_cast<const __nv_bfloat16*>(a.queries) + ((size_t)head * m + token) * D;
-                    r.keys = reinterpret_cast<const __nv_bfloat16*>(a.keys) + (size_t)kvh * a.k_head_stride;
-                    r.values = reinterpret_cast<const __nv_bfloat16*>(a.values) + (size_t)kvh * a.v_head_stride + half + side * MINE + c;
-                    r.out = out + c;
-                    r.nodes = trie ? nodes : nullptr;
-                    r.k_stride = a.k_seq_stride; r.v_stride = a.v_seq_stride;
-                    r.token = token; r.lim = lim; r.prefix = prefix; r.kend = kend;
-                    r.scale2 = scale2;
-                    au_row_by_key<D>(r);
-                }
-            }
-            __syncwarp();
+            for (uint32_t j = 0; j < MINE; j += 8)
+                *reinterpret_cast<uint4*>(out + j) = make_uint4(au_pack(acc[j] * inv, acc[j + 1] * inv), au_pack(acc[j + 2] * inv, acc[j + 3] * inv),
+                                                                au_pack(acc[j + 4] * inv, acc[j + 5] * inv), au_pack(acc[j + 6] * inv, acc[j + 7] * inv));
+        } else if (row < rows) {
+            AuRow r;
+            r.query = reinterpret_cast<const __nv_bfloat16*>(a.queries) + ((size_t)head * m + token) * D;
+            r.keys = reinterpret_cast<const __nv_bfloat16*>(a.keys) + (size_t)kvh * a.k_head_stride;
+            r.values = reinterpret_cast<const __nv_bfloat16*>(a.values) + (size_t)kvh * a.v_head_stride + half + side * MINE;
+            r.out = out;
+            r.nodes = trie ? nodes : nullptr;
+            r.k_stride = a.k_seq_stride; r.v_stride = a.v_seq_stride;
+            r.token = token; r.lim = lim; r.prefix = prefix; r.kend = kend;
+            r.scale2 = scale2;
+            au_row_by_key<D, MINE>(r);
         }
     }
     au_fence_before();
