@@ -60,7 +60,10 @@ def _run(ctx, n, k, group, method, x, ops, gated=False, bits=4, fused=None):
                             d=out.ptr, b_prologue={"zero": B.B_SCALE_ZERO_POINT, "symmetric": B.B_SCALE_SYMMETRIC, "mlx": B.B_SCALE_BIAS}[method], b_mode=B.QMODE_U4 if bits == 4 else B.QMODE_U8,
                             b_group_size=group, b_transpose=1, ab_scale=1.0, m=1, n=n, k=k, weights_dt=B.DT_BF16, input_dt=B.DT_BF16, output_dt=B.DT_BF16 if gated else B.DT_F32)
     with ctx.command_buffer("decode-linear") as cmd:
-        assert ctx.lib.uzu_debug_fused_linear_encode(cmd.h, C.byref(a)) == 1
+        if bits == 4:
+            cmd.encode("uzu_fused_linear_encode", C.byref(a))
+        else:                    # (that entry takes 4-bit weights only)
+            assert ctx.lib.uzu_debug_fused_linear_encode(cmd.h, C.byref(a)) == 1
     got = bf16_to_f32(out.numpy(np.uint16, (n // 2,))) if gated else out.numpy(np.float32, (n,))
     return (got, fields["shortcut_out"].numpy(np.uint16, (k,))) if fused and "shortcut_out" in fused else got
 
